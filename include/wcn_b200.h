@@ -380,6 +380,20 @@ int wcn_conv_fwd(int algo, const void* feats, int64_t num_in, int64_t feats_ld, 
 int wcn_row_reduce(const void* feats, int64_t num_in, const int32_t* nbr, int64_t num_out, int32_t num_offsets,
                    int32_t channels, int dtype, int op, void* out, int32_t* dev_status, void* stream);
 
+/* The same, leaving what its gradient needs (each may be NULL): `arg` [num_out, channels] of arg_bytes = 1 (at most
+ * 255 offsets) or 2 bytes per element (min, max: the first offset that attained the result, all ones where there is
+ * none) and `count` [num_out] (mean: neighbours of the row, at least 1). */
+int wcn_row_reduce_train(const void* feats, int64_t num_in, const int32_t* nbr, int64_t num_out, int32_t num_offsets,
+                         int32_t channels, int dtype, int op, void* out, void* arg, int32_t arg_bytes, float* count,
+                         int32_t* dev_status, void* stream);
+
+/* Gradient of a pooling with respect to its features, over the transposed table nbr_t [num_offsets, num_in]:
+ * grad_in[i, :] = sum over the offsets k with m = nbr_t[k*num_in + i] >= 0 of grad_out[m, :] (divided by count[m] when
+ * `count` is given; where arg[m] == k only, when `arg` is given).  fp32 accumulation in order of k. */
+int wcn_row_reduce_backward(const void* grad_out, int64_t num_out, const int32_t* nbr_t, int64_t num_in,
+                            int32_t num_offsets, int32_t channels, int dtype, const void* arg, int32_t arg_bytes,
+                            const float* count, void* grad_in, int32_t* dev_status, void* stream);
+
 /* Convolution in which every output row has exactly one (input row, kernel offset) pair, run from the
  * INPUT side on the tensor cores: a 1x1x1 convolution (optionally writing through a row permutation)
  * and a transposed convolution whose window equals its stride (2x2x2, stride 2).  For input row j and

@@ -99,3 +99,37 @@ def test_reduce_and_stride_convolution():
     assert y.tensor_stride == (2, 2, 2)
     assert rel_l2(y.feature_tensor.cpu().numpy(), want) < 1e-4
     check_device_status(DEV)
+
+
+@pytest.mark.parametrize("reduction", ["max", "min", "mean", "sum"])
+@pytest.mark.parametrize("dtype,c,ksize", [(torch.float32, 4, 2), (torch.float32, 7, 3), (torch.float16, 8, 2),
+                                           (torch.bfloat16, 24, 3), (torch.float16, 9, 2), (torch.float16, 8, 7)])
+def test_pooling_gradients_of_every_width(reduction, dtype, c, ksize):
+    """The gradient kernel at whole and odd channel counts, at windows of 8, 27 and 343 offsets (one and two bytes per
+    arg-extremum), overlapping or not, with ties, against the reduction's definition over the kernel map."""
+    coords, x, vox = _scene(1500, c, 63, dtype)
+    x = (x * 2).round() / 2  # many equal values: the first offset takes the gradient
+    xg = x.to(DEV).requires_grad_(True)
+    out = sparse_reduce(vox.replace(batched_features=xg), kernel_size=ksize, stride=2, reduction=reduction).feature_tensor
+    g = torch.randn(out.shape, generator=torch.Generator().manual_seed(64)).to(dtype)
+    (got,) = torch.autograd.grad(out, [xg], g.to(DEV))
+    ref_c, _ = km.stride_coords(coords, (2, 2, 2))
+    i, o, f, _ = km.generate_kernel_map(coords, ref_c, (2, 2, 2), (ksize,) * 3)
+    k = np.repeat(np.arange(len(f) - 1), np.diff(f))
+    want = np.zeros((len(coords), c))
+    count = np.bincount(o, minlength=len(ref_c))
+    xs, gs = x.double().numpy(), g.double().numpy()
+    if reduction in ("max", "min"):
+        s = 1.0 if reduction == "max" else -1.0
+        top = np.full((len(ref_c), c), -np.inf)
+        at = np.full((len(ref_c), c), -1)
+        for p in np.argsort(k, kind="stable"):
+            beyond = s * xs[i[p]] > top[o[p]]
+            top[o[p]][beyond] = s * xs[i[p]][beyond]
+            at[o[p]][beyond] = i[p]
+        for ch in range(c):
+            np.add.at(want[:, ch], at[:, ch], gs[:, ch])
+    else:
+        np.add.at(want, i, gs[o] / (count[o][:, None] if reduction == "mean" else 1.0))
+    check_device_status(DEV)
+    assert rel_l2(got.double().cpu().numpy(), want) < {torch.float32: 1e-6, torch.float16: 1e-3, torch.bfloat16: 8e-3}[dtype]

@@ -97,18 +97,30 @@ class IntSearchResult:
         self._compact()
         return self._offsets
 
+    def _kept(self) -> dict:
+        """Where the tables derived from the neighbour table are kept.  A transposed view keeps its own with the
+        map it was swapped from, so every layer's backward pass over one map shares one transposed table (and its
+        tile order) and they live as long as the map."""
+        fwd = self._forward
+        if fwd is None:
+            return self.__dict__.setdefault("_derived", {})
+        return fwd.__dict__.setdefault("_derived", {}).setdefault(("transposed", self._num_out), {})
+
     def neighbor_table(self, num_out: int) -> Tensor:
         """``nbr[K, num_out]`` int32 on the maps' device."""
         if self._nbr is not None:
             assert self._num_out == num_out, f"kernel map was built for {self._num_out} outputs, got {num_out}"
             return self._nbr
-        if self._in_maps is None:  # a transposed view whose table has not been asked for yet
-            fwd = self._forward
+        fwd = self._forward
+        if fwd is not None and fwd._nbr is not None:  # a transposed view whose table has not been asked for yet
             assert self._num_out == num_out, f"kernel map was built for {self._num_out} outputs, got {num_out}"
-            dev = fwd._nbr.device
-            nbr_t = torch.empty((self._num_offsets, num_out), dtype=torch.int32, device=dev)
-            check(lib().wcn_nbr_transpose(ptr(fwd._nbr), fwd._num_offsets, fwd._num_out, num_out, ptr(nbr_t),
-                                          stream_ptr(dev)), "wcn_nbr_transpose")
+            nbr_t = self._kept().get("nbr")
+            if nbr_t is None:
+                dev = fwd._nbr.device
+                nbr_t = torch.empty((self._num_offsets, num_out), dtype=torch.int32, device=dev)
+                check(lib().wcn_nbr_transpose(ptr(fwd._nbr), fwd._num_offsets, fwd._num_out, num_out, ptr(nbr_t),
+                                              stream_ptr(dev)), "wcn_nbr_transpose")
+                self._kept()["nbr"] = nbr_t
             self._nbr = nbr_t
             return nbr_t
         dev = self._in_maps.device
@@ -129,34 +141,36 @@ class IntSearchResult:
         scan), and the convolution kernels skip the empty ones.  Built once per map, so every
         layer that shares the map shares the order."""
         if self._tiled is None:
+            self._tiled = self._kept().get("tiled")
+        if self._tiled is None:
             nbr = self.neighbor_table(num_out)
             dev = nbr.device
             tiled = torch.empty_like(nbr)
             rows = torch.empty(num_out, dtype=torch.int32, device=dev)
             check(lib().wcn_kmap_tile_order(ptr(nbr), num_out, self._num_offsets, ptr(rows), ptr(tiled),
                                             stream_ptr(dev)), "wcn_kmap_tile_order")
-            self._tiled = (tiled, rows)
+            self._tiled = self._kept()["tiled"] = (tiled, rows)
         assert self._tiled[0].shape[1] == num_out
         return self._tiled
 
     def tile_masks(self, num_out: int, tiled: bool = False) -> Tensor:
         """Per 128 consecutive rows of the neighbour table (the tiled one with ``tiled``), the set of
         offsets (bit k) that have any neighbour there; ``int32 [ceil(num_out / 128)]``, built once."""
-        store = self.__dict__.setdefault("_tile_masks", {})
-        if tiled not in store:
+        store, key = self._kept(), ("masks", tiled)
+        if key not in store:
             nbr = self.tiled_neighbor_table(num_out)[0] if tiled else self.neighbor_table(num_out)
             masks = torch.empty((num_out + 127) // 128, dtype=torch.int32, device=nbr.device)
             check(lib().wcn_kmap_tile_masks(ptr(nbr), num_out, self._num_offsets, ptr(masks), stream_ptr(nbr.device)),
                   "wcn_kmap_tile_masks")
-            store[tiled] = masks
-        return store[tiled]
+            store[key] = masks
+        return store[key]
 
     def swapped(self, num_in: Optional[int] = None) -> "IntSearchResult":
         """The map with inputs and outputs exchanged (transposed convolution,
         warpconvnet/nn/functional/sparse_conv.py:1934-1938)."""
-        if self._forward is not None and self._in_maps is None and (num_in is None or int(num_in) == self._forward._num_out):
+        if self._forward is not None and (num_in is None or int(num_in) == self._forward._num_out):
             return self._forward  # exchanging a transposed view back gives the map it came from
-        if self._offsets is None and self._nbr is not None and (num_in or self._num_in) is not None:
+        if self._nbr is not None and (num_in or self._num_in) is not None:
             # Both forms of the view come from this map when first asked for: the compact one by exchanging
             # in and out, the dense one by transposing the table (a layer that runs from the input side,
             # sparse_conv_rows_fused, needs neither: it reads this map's own table).

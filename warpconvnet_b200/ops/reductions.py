@@ -31,6 +31,7 @@ class REDUCTIONS(Enum):
 
 
 _NATIVE_OP = {REDUCTIONS.MIN: 0, REDUCTIONS.MAX: 1, REDUCTIONS.SUM: 2, REDUCTIONS.MEAN: 3, REDUCTIONS.MUL: 4}
+_EXTREMA = (_NATIVE_OP[REDUCTIONS.MIN], _NATIVE_OP[REDUCTIONS.MAX])
 
 
 def _native_reduce(features: Tensor, nbr: Tensor, op: int) -> Tensor:
@@ -44,45 +45,65 @@ def _native_reduce(features: Tensor, nbr: Tensor, op: int) -> Tensor:
 
 
 class _RowReduce(torch.autograd.Function):
-    """``wcn_row_reduce`` with a backward pass.
-
-    sum / mean: ``dX[i] = sum over (k, m) with nbr[k][m] == i of dY[m] (/ count[m])`` — the same
-    kernel over the transposed table.  max / min: the gradient of output row m goes, per channel,
-    to the first neighbour (ascending offset) whose value equals the result, as ``segment_csr``'s
-    arg-extremum does.  mul has no backward here."""
+    """``wcn_row_reduce`` with a backward pass: sum and mean send the output gradient (over the number of
+    neighbours) to every neighbour, max and min send it, per channel, to the first neighbour (ascending
+    offset) that attained the result, as ``segment_csr``'s arg-extremum does.  The forward kernel leaves
+    that offset (or the counts) behind; mul has no backward here."""
 
     @staticmethod
     def forward(ctx, features: Tensor, kernel_map: IntSearchResult, num_out: int, op: int) -> Tensor:
         x = features.contiguous()
-        out = _native_reduce(x, kernel_map.neighbor_table(num_out), op)
-        ctx.kernel_map, ctx.num_out, ctx.op = kernel_map, num_out, op
-        ctx.save_for_backward(x, out)
+        nbr = kernel_map.neighbor_table(num_out)
+        K, M, C, dev = nbr.shape[0], num_out, x.shape[1], x.device
+        out = torch.empty((M, C), dtype=x.dtype, device=dev)
+        arg = count = None
+        if op in _EXTREMA:
+            arg = torch.empty((M, C), dtype=torch.uint8 if K <= 255 else torch.int16, device=dev)
+        elif op == _NATIVE_OP[REDUCTIONS.MEAN]:
+            count = torch.empty(M, dtype=torch.float32, device=dev)
+        check(lib().wcn_row_reduce_train(ptr(x), x.shape[0], ptr(nbr), M, K, C, dtype_code(x.dtype), op, ptr(out),
+                                         ptr(arg), arg.element_size() if arg is not None else 0, ptr(count),
+                                         ptr(device_status(dev)), stream_ptr(dev)), "wcn_row_reduce_train")
+        ctx.kernel_map, ctx.num_in, ctx.op = kernel_map, x.shape[0], op
+        ctx.save_for_backward(arg, count)
         return out
 
     @staticmethod
     def backward(ctx, grad_out: Tensor):
-        x, out = ctx.saved_tensors
-        km, M, op = ctx.kernel_map, ctx.num_out, ctx.op
+        if ctx.op == _NATIVE_OP[REDUCTIONS.MUL]:
+            raise NotImplementedError("the 'mul' reduction has no backward pass")
+        arg, count = ctx.saved_tensors
+        return _RowReduceBackward.apply(grad_out, ctx.kernel_map, ctx.num_in, arg, count), None, None, None
+
+
+class _RowReduceBackward(torch.autograd.Function):
+    """The gradient of :class:`_RowReduce`, linear in the output gradient and differentiable with respect to it."""
+
+    @staticmethod
+    def forward(ctx, grad_out: Tensor, kernel_map: IntSearchResult, num_in: int, arg, count) -> Tensor:
         g = grad_out.contiguous()
-        nbr = km.neighbor_table(M)
-        if op in (_NATIVE_OP[REDUCTIONS.SUM], _NATIVE_OP[REDUCTIONS.MEAN]):
-            if op == _NATIVE_OP[REDUCTIONS.MEAN]:
-                count = (nbr >= 0).sum(0).clamp_(min=1).to(g.dtype)
-                g = (g / count.unsqueeze(1)).contiguous()
-            nbr_t = km.swapped(num_in=x.shape[0]).neighbor_table(x.shape[0])
-            return _native_reduce(g, nbr_t, _NATIVE_OP[REDUCTIONS.SUM]), None, None, None
-        if op in (_NATIVE_OP[REDUCTIONS.MAX], _NATIVE_OP[REDUCTIONS.MIN]):
-            gx = torch.zeros_like(x)
-            taken = torch.zeros_like(out, dtype=torch.bool)
-            for k in range(nbr.shape[0]):
-                rows = nbr[k].long()
-                have = rows >= 0
-                src = rows.clamp(min=0)
-                hit = have.unsqueeze(1) & (x[src] == out) & ~taken
-                gx.index_add_(0, src, torch.where(hit, g, torch.zeros_like(g)))
-                taken |= hit
-            return gx, None, None, None
-        raise NotImplementedError("the 'mul' reduction has no backward pass")
+        M, C, dev = g.shape[0], g.shape[1], g.device
+        nbr_t = kernel_map.swapped(num_in=num_in).neighbor_table(num_in)
+        gx = torch.empty((num_in, C), dtype=g.dtype, device=dev)
+        check(lib().wcn_row_reduce_backward(ptr(g), M, ptr(nbr_t), num_in, nbr_t.shape[0], C, dtype_code(g.dtype),
+                                            ptr(arg), arg.element_size() if arg is not None else 0, ptr(count),
+                                            ptr(gx), ptr(device_status(dev)), stream_ptr(dev)),
+              "wcn_row_reduce_backward")
+        ctx.kernel_map, ctx.num_out = kernel_map, M
+        ctx.save_for_backward(arg, count)
+        return gx
+
+    @staticmethod
+    def backward(ctx, gg: Tensor):
+        arg, count = ctx.saved_tensors
+        nbr = ctx.kernel_map.neighbor_table(ctx.num_out)
+        if arg is None:
+            total = _native_reduce(gg.contiguous(), nbr, _NATIVE_OP[REDUCTIONS.SUM])
+            return (total if count is None else (total / count.unsqueeze(1)).to(gg.dtype)), None, None, None, None
+        at = arg.long() & (255 if arg.dtype == torch.uint8 else 65535)
+        rows = nbr.long().gather(0, at.clamp(max=nbr.shape[0] - 1))
+        live = (at < nbr.shape[0]) & (rows >= 0)
+        return gg.gather(0, rows.clamp(min=0)) * live, None, None, None, None
 
 
 def neighbor_reduction(features: Tensor, kernel_map: IntSearchResult, num_out: int,
