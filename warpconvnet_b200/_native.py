@@ -1,4 +1,4 @@
-"""ctypes binding of ``csrc/libwcn_b200.so`` (declared in ``include/wcn_b200.h``).
+"""Binding of ``csrc/libwcn_b200.so`` (declared in ``include/wcn_b200.h``).
 
 The library is the only compute back-end of this package: when it is missing
 or cannot be loaded, every operation raises; there is no CPU or eager fallback.
@@ -7,6 +7,7 @@ PyTorch is used for device memory and streams only.
 from __future__ import annotations
 
 import ctypes
+import importlib.util
 import os
 from collections import Counter
 from typing import Optional
@@ -15,6 +16,7 @@ import torch
 
 _HERE = os.path.dirname(os.path.abspath(__file__))
 LIB_PATH = os.path.join(_HERE, "csrc", "libwcn_b200.so")
+FASTCALL_PATH = os.path.join(_HERE, "csrc", "_fastcall.so")
 
 WCN_F32, WCN_F16, WCN_BF16 = 0, 1, 2
 CONV_AUTO, CONV_SIMT, CONV_TCGEN05 = 0, 1, 2
@@ -80,26 +82,22 @@ KERNELS_PER_CALL = {
 LAUNCH_COUNTS: Counter = Counter()
 
 
-class _CountingLib:
-    """Attribute access returns the C function wrapped so that calls are counted."""
+class _Library:
+    """The C functions as attributes.  Those that take only integers and pointers go through the ``_fastcall``
+    extension (csrc/fastcall.c): a 26-argument call costs 0.3 us there and 3.5 us through ctypes, which for a small
+    layer is as much as its launch.  It also counts the kernels they launch."""
 
-    def __init__(self, handle):
-        self._handle = handle
-        self._wrapped = {}
-
-    def __getattr__(self, name):
-        fn = self._wrapped.get(name)
-        if fn is None:
-            raw = getattr(self._handle, name)
-            n = KERNELS_PER_CALL.get(name, 0)
-            if n:
-                def fn(*args, _raw=raw, _name=name, _n=n):
-                    LAUNCH_COUNTS[_name] += _n
-                    return _raw(*args)
-            else:
-                fn = raw
-            self._wrapped[name] = fn
-        return fn
+    def __init__(self, handle, bind):
+        for name, argtypes in SIGNATURES.items():
+            fn = getattr(handle, name)
+            fn.argtypes, fn.restype = argtypes, ctypes.c_int
+            if all(t in (_c_i32, _c_i64, _c_vp) for t in argtypes):
+                fn = bind(ctypes.cast(fn, ctypes.c_void_p).value, len(argtypes), name, LAUNCH_COUNTS,
+                          KERNELS_PER_CALL.get(name))
+            setattr(self, name, fn)
+        handle.wcn_status_string.argtypes, handle.wcn_status_string.restype = [ctypes.c_int], ctypes.c_char_p
+        handle.wcn_brick_usable_flag.argtypes, handle.wcn_brick_usable_flag.restype = [ctypes.c_void_p], ctypes.c_void_p
+        self.wcn_status_string, self.wcn_brick_usable_flag = handle.wcn_status_string, handle.wcn_brick_usable_flag
 
 
 def launches_total() -> int:
@@ -114,23 +112,19 @@ def lib():
     """The loaded library; raises NativeLibraryError when it is not built."""
     global _lib
     if _lib is None:
-        if not os.path.isfile(LIB_PATH):
-            raise NativeLibraryError(
-                f"{LIB_PATH} is missing: build it with `python -m warpconvnet_b200.csrc.build` "
-                "(nvcc, sm_100a). This package has no fallback path.")
+        for path in (LIB_PATH, FASTCALL_PATH):
+            if not os.path.isfile(path):
+                raise NativeLibraryError(
+                    f"{path} is missing: build it with `python -m warpconvnet_b200.csrc.build` "
+                    "(nvcc, sm_100a). This package has no fallback path.")
         try:
             handle = ctypes.CDLL(LIB_PATH)
-        except OSError as e:  # pragma: no cover
-            raise NativeLibraryError(f"cannot load {LIB_PATH}: {e}") from e
-        for name, argtypes in SIGNATURES.items():
-            fn = getattr(handle, name)
-            fn.argtypes = argtypes
-            fn.restype = ctypes.c_int
-        handle.wcn_status_string.argtypes = [ctypes.c_int]
-        handle.wcn_status_string.restype = ctypes.c_char_p
-        handle.wcn_brick_usable_flag.argtypes = [ctypes.c_void_p]
-        handle.wcn_brick_usable_flag.restype = ctypes.c_void_p
-        _lib = _CountingLib(handle)
+            spec = importlib.util.spec_from_file_location("_fastcall", FASTCALL_PATH)
+            fastcall = importlib.util.module_from_spec(spec)
+            spec.loader.exec_module(fastcall)
+        except (OSError, ImportError) as e:  # pragma: no cover
+            raise NativeLibraryError(f"cannot load the native library: {e}") from e
+        _lib = _Library(handle, fastcall.bind)
     return _lib
 
 

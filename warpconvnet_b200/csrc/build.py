@@ -1,16 +1,19 @@
-"""Build libwcn_b200.so in this folder with nvcc for sm_100a (no other architecture).
+"""Build libwcn_b200.so in this folder with nvcc for sm_100a (no other architecture), and the _fastcall.so extension
+through which Python calls it.
 
 Usage: ``python -m warpconvnet_b200.csrc.build [--force] [--verbose]``
 """
 import os
 import subprocess
 import sys
+import sysconfig
 
 HERE = os.path.dirname(os.path.abspath(__file__))
 SOURCES = ["api.cu", "hash_kmap.cu", "brick_kmap.cu", "conv_explicit.cu", "row_reduce.cu", "conv_simt.cu", "conv_tcgen05.cu",
            "conv_wgrad_tcgen05.cu", "conv_rows_tcgen05.cu"]
 HEADERS = ["wcn_common.cuh", "tcgen05_common.cuh", os.path.join("..", "..", "include", "wcn_b200.h")]
 LIB = os.path.join(HERE, "libwcn_b200.so")
+FASTCALL_SOURCE, FASTCALL = os.path.join(HERE, "fastcall.c"), os.path.join(HERE, "_fastcall.so")
 NVCC_FLAGS = ["-gencode", "arch=compute_100a,code=sm_100a", "-lineinfo", "-O3", "-std=c++17",
               "-Xcompiler", "-fPIC", "--use_fast_math=false"]
 
@@ -30,7 +33,14 @@ def needs_build():
     return any(os.path.getmtime(d) > t for d in deps)
 
 
+def build_fastcall(force=False):
+    if force or not os.path.isfile(FASTCALL) or os.path.getmtime(FASTCALL_SOURCE) > os.path.getmtime(FASTCALL):
+        subprocess.check_call([os.environ.get("CC", "gcc"), "-O2", "-shared", "-fPIC", "-I" + sysconfig.get_paths()["include"],
+                               FASTCALL_SOURCE, "-o", FASTCALL])
+
+
 def build(force=False, verbose=False, ptxas_info=False):
+    build_fastcall(force)
     if not force and not needs_build():
         return LIB
     flags = [f for f in NVCC_FLAGS if not f.startswith("--use_fast_math")]

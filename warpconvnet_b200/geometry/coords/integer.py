@@ -61,6 +61,14 @@ class IntCoords(Coords):
         self._shared = other._shared
         return self
 
+    def labelled(self, tensor_stride: Tuple[int, ...]) -> "IntCoords":
+        """The same rows (and their derived data) under another tensor stride."""
+        new = object.__new__(IntCoords)
+        new.offsets, new.batched_tensor, new._shared = self.offsets, self.batched_tensor, self._shared
+        new.voxel_size = new.voxel_origin = None
+        new.tensor_stride = tensor_stride
+        return new
+
     @property
     def batch_indexed_coordinates(self) -> Tensor:
         """[N, 4] (batch, x, y, z); built once per set of rows."""

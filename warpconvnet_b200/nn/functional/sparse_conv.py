@@ -360,7 +360,7 @@ def _prepared_rows_weight(weight: Tensor, dtype: torch.dtype):
         width = -(-c_out // 16) * 16
         dc = dtype_code(dtype)
         yes = ctypes.c_int32(0)
-        check(lib().wcn_conv_rows_supported(K, c_in, width, dc, dc, ctypes.byref(yes)), "wcn_conv_rows_supported")
+        check(lib().wcn_conv_rows_supported(K, c_in, width, dc, dc, ctypes.addressof(yes)), "wcn_conv_rows_supported")
         if yes.value:
             w = weight.detach().to(dtype=dtype)
             if width != c_out:
@@ -940,13 +940,163 @@ def spatially_sparse_conv(
             if own and out_ic.tensor_stride is None:
                 out_ic.tensor_stride = out_tensor_stride  # the cached set is labelled once
             else:  # same rows under another stride label: a view that shares the derived data
-                out_ic = IntCoords(out_ic.batched_tensor, offsets=out_ic.offsets,
-                                   tensor_stride=out_tensor_stride).share_derived(out_ic)
+                out_ic = out_ic.labelled(out_tensor_stride)
         return input_sparse_tensor._derive(out, out_ic)
     out_ic = IntCoords(out_coords[:, 1:], offsets=out_offsets if out_offsets.device.type == "cpu" else out_offsets.cpu())
     out_ic._bcoords = out_coords
     return input_sparse_tensor.replace(batched_coordinates=out_ic, batched_features=out,
                                        tensor_stride=out_tensor_stride)
+
+
+# --------------------------------------------------------------------------- layers in inference
+#
+# A small layer takes the GPU 10-20 us; deriving its launch from the arguments of spatially_sparse_conv takes
+# Python twice that.  What does not change between two calls of a layer is resolved once: the weights and the folded
+# epilogue in a launch record kept with the weight tensor, the tables of a coordinate set and a window with that
+# coordinate set (where the coordinate set's other derived data lives).
+
+
+class _LayerRecord:
+    """The launch records of one (weight, bias, epilogue vectors, dtype), current while none of them is written.
+    (It is kept with the weight tensor, so it holds none itself.)"""
+
+    __slots__ = ("w_version", "w_ptr", "vectors", "versions", "conv", "rows")
+
+    def __init__(self, weight, bias, scale, shift, relu, dtype):
+        ep = _merge_bias(ConvEpilogue(scale=scale, shift=shift), bias)
+        self.w_version, self.w_ptr = weight._version, weight.data_ptr()
+        self.vectors = (bias, scale, shift)
+        self.versions = tuple(t._version if t is not None else 0 for t in self.vectors)
+        self.conv = FusedConvLaunch(weight, dtype, ep.scale, ep.shift, relu=relu)
+        self.rows = None  # FusedRowsLaunch, made by the first layer call that can use one
+
+    def current(self, weight, bias, scale, shift) -> bool:
+        b, sc, sh = self.vectors
+        v = self.versions
+        return (b is bias and sc is scale and sh is shift and weight._version == self.w_version
+                and weight.data_ptr() == self.w_ptr and (b is None or b._version == v[0])
+                and (sc is None or sc._version == v[1]) and (sh is None or sh._version == v[2]))
+
+    def rows_launch(self, weight) -> "FusedRowsLaunch":
+        if self.rows is None:
+            c = self.conv
+            self.rows = FusedRowsLaunch(weight, c.dtype, c.scale, c.shift, relu=c.relu)
+        return self.rows
+
+
+def _layer_record(weight, bias, scale, shift, relu, dtype) -> _LayerRecord:
+    store = weight.__dict__.setdefault("_wcn_layer", {})
+    rec = store.get((dtype, relu))
+    if rec is None or not rec.current(weight, bias, scale, shift):
+        rec = store[(dtype, relu)] = _LayerRecord(weight, bias, scale, shift, relu, dtype)
+    return rec
+
+
+@dataclass
+class _LayerTables:
+    """What a layer of one window reads of a coordinate set: neighbour table (with its row order), or for layers
+    with one pair per output row also the destination rows of the input-side kernel."""
+
+    num_in: int
+    num_out: int
+    nbr: Optional[Tensor]
+    out_rows: Optional[Tensor]
+    one_pair: bool = False
+    dst: Optional[Tensor] = None
+    coords: Optional[IntCoords] = None  # strided layers: the output coordinates
+
+
+def _layer_tables(x: Voxels, kernel_size, stride, dilation, transposed: bool, target: Optional[Voxels]) -> _LayerTables:
+    n = x.batched_coordinates.batched_tensor.shape[0]
+    if all(k == 1 for k in kernel_size) and all(s == 1 for s in stride):
+        return _LayerTables(n, n, _identity_map(n, x.device).neighbor_table(n), None, True)
+    out_coords, _, km = generate_output_coords_and_kernel_map(x, kernel_size, dilation, stride, False, transposed, target)
+    m = out_coords.shape[0]
+    if transposed and getattr(km, "_one_pair", False) and km._forward is not None:
+        return _LayerTables(n, m, None, None, True, km._forward.neighbor_table(n))
+    if TILE_ORDER_MIN_OFFSETS <= len(km) <= 32 and m >= TILE_ORDER_MIN_ROWS:
+        nbr, out_rows = km.tiled_neighbor_table(m)
+    else:
+        nbr, out_rows = km.neighbor_table(m), None
+    strided = strided_coordinates(x.batched_coordinates, stride) if any(s != 1 for s in stride) and not transposed else None
+    return _LayerTables(n, m, nbr, out_rows, coords=strided)
+
+
+_NATIVE_ALGOS = (SPARSE_CONV_FWD_ALGO_MODE.AUTO, SPARSE_CONV_FWD_ALGO_MODE.IMPLICIT_GEMM,
+                 SPARSE_CONV_FWD_ALGO_MODE.CUTLASS_IMPLICIT_GEMM)
+_NATIVE_DTYPES = (torch.float32, torch.float16, torch.bfloat16)
+
+
+def run_layer(layer, x: Voxels, target: Optional[Voxels], epilogue: Optional[ConvEpilogue]) -> Optional[Voxels]:
+    """``layer`` (a :class:`SpatiallySparseConv`) on ``x`` without gradients, from its launch record and the
+    coordinate set's tables; None when the call is one that only :func:`spatially_sparse_conv` takes."""
+    if type(x) is not Voxels or layer.generative or torch.is_autocast_enabled():
+        return None
+    feats, weight, ic = x.batched_features.batched_tensor, layer.weight, x.batched_coordinates
+    dtype = feats.dtype
+    if (not feats.is_cuda or dtype not in _NATIVE_DTYPES or feats.stride(1) != 1 or feats.shape[0] == 0
+            or (weight.dtype != dtype and _min_dtype(dtype, weight.dtype) != dtype) or weight.device != feats.device
+            or layer.compute_dtype not in (None, dtype) or layer.order != POINT_ORDERING.RANDOM
+            or layer.stride_mode != STRIDED_CONV_MODE.STRIDE_ONLY or weight.shape[1] != feats.shape[1]):
+        return None
+    scale = shift = residual = out = None
+    relu = False
+    if epilogue is not None:
+        if epilogue.out_rows is not None:
+            return None
+        scale, shift, residual, out, relu = (epilogue.scale, epilogue.shift, epilogue.residual, epilogue.out, epilogue.relu)
+        if residual is not None and (residual.dtype != dtype or residual.dim() != 2 or residual.stride(1) != 1):
+            return None
+    elif layer.fwd_algo not in _NATIVE_ALGOS:
+        return None
+    kernel_size, stride = layer.kernel_size, layer.stride
+    transposed = layer.transposed
+    key = ("layer", kernel_size, stride, layer.dilation, transposed)
+    ones = (1,) * len(kernel_size)
+    if transposed:
+        # only back onto the set these coordinates are the strided ones of: its tables live with that set
+        if target is None:
+            return None
+        holder = target.batched_coordinates
+        parent = holder._shared.get(("strided", stride))
+        if (parent is None or parent._shared is not ic._shared or ic.tensor_stride is None
+                or not any(o < i for o, i in zip(holder.tensor_stride or ones, ic.tensor_stride))):
+            return None
+    elif target is not None:
+        return None
+    else:
+        holder = ic
+    tables = holder._shared.get(key)
+    if tables is None:
+        tables = holder._shared[key] = _layer_tables(x, kernel_size, stride, layer.dilation, transposed, target)
+    m, c_out = tables.num_out, weight.shape[2]
+    if m == 0 or tables.num_in != feats.shape[0]:
+        return None
+    if out is not None and (out.dtype != dtype or out.shape != (m, c_out) or out.stride(1) != 1 or out.device != feats.device):
+        return None
+    if residual is not None and residual.shape != (m, c_out):
+        return None
+    rec = _layer_record(weight, layer.bias, scale, shift, relu, dtype)
+    if x._extra_attributes.get("_cache") is None:
+        x._extra_attributes["_cache"] = IntSearchCache()  # shared by everything derived from x, as after any convolution
+    if tables.one_pair and rec.rows_launch(weight).takes(feats):
+        y = rec.rows(feats, tables.dst, m, residual, out)
+    elif tables.nbr is None:
+        return None
+    else:
+        y = rec.conv(feats, tables.nbr, tables.out_rows, m, residual, out)
+    if transposed:
+        return x._derive(y, holder)
+    if kernel_size == ones and stride == ones:
+        return x._derive(y)
+    ts = ic.tensor_stride or ones
+    if stride == ones:
+        out_ic, out_ts = ic, ts
+    else:
+        out_ic, out_ts = tables.coords, tuple(o * s for o, s in zip(stride, ts))
+        if out_ic.tensor_stride is None:
+            out_ic.tensor_stride = out_ts  # the cached set is labelled once
+    return x._derive(y, out_ic if out_ic.tensor_stride == out_ts else out_ic.labelled(out_ts))
 
 
 def _merge_bias(epilogue: Optional[ConvEpilogue], bias: Optional[Tensor]) -> Optional[ConvEpilogue]:

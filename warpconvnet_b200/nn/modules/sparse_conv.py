@@ -18,7 +18,7 @@ from ...geometry.coords.ops.serialization import POINT_ORDERING
 from ...geometry.types.voxels import Voxels
 from ...utils.ntuple import ntuple
 from ..functional.sparse_conv import (SPARSE_CONV_BWD_ALGO_MODE, SPARSE_CONV_FWD_ALGO_MODE, STRIDED_CONV_MODE,
-                                      ConvEpilogue, spatially_sparse_conv)
+                                      ConvEpilogue, run_layer, spatially_sparse_conv)
 from .base_module import BaseSpatialModule
 
 
@@ -87,6 +87,10 @@ class SpatiallySparseConv(BaseSpatialModule):
 
     def forward(self, input_sparse_tensor: Voxels, output_spatially_sparse_tensor: Optional[Voxels] = None,
                 epilogue: Optional[ConvEpilogue] = None):
+        if not torch.is_grad_enabled():
+            y = run_layer(self, input_sparse_tensor, output_spatially_sparse_tensor, epilogue)
+            if y is not None:
+                return y
         return spatially_sparse_conv(
             input_sparse_tensor=input_sparse_tensor, weight=self.weight, kernel_size=self.kernel_size,
             stride=self.stride, kernel_dilation=self.dilation, bias=self.bias,
