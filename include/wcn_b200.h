@@ -419,8 +419,8 @@ int wcn_conv_rows_fwd(const void* feats, int64_t num_in, int64_t feats_ld, const
  *   grad_weight[k] += feats[nbr[k*M + m], :]^T (outer) grad_out[m, :]   over rows m with nbr >= 0
  * feats / grad_out share `dtype` (f16 or bf16), fp32 accumulation on the tensor cores; the partial
  * sums of different row ranges are added with atomics, so the last bits vary from run to run.
- * Needs c_in % 32 == 0, c_out % 32 == 0, c_out <= 256; else WCN_ERR_UNSUPPORTED_CONFIG (callers fall
- * back to a GEMM per offset).  (`nbr`, `out_rows`) is the pair wcn_conv_fwd takes: the plain table
+ * Needs c_in % 32 == 0, c_out % 32 == 0, c_out <= 256; else WCN_ERR_UNSUPPORTED_CONFIG (callers
+ * take wcn_conv_wgrad_pairs).  (`nbr`, `out_rows`) is the pair wcn_conv_fwd takes: the plain table
  * with out_rows NULL, or the tiled one with its row order (grad_out is then read at out_rows[s]);
  * `tile_masks` (from wcn_kmap_tile_masks on the same table, or NULL) lets the kernel skip the 128-row
  * steps in which the offsets of a CTA have no neighbour.
@@ -430,6 +430,15 @@ int wcn_conv_rows_fwd(const void* feats, int64_t num_in, int64_t feats_ld, const
 int wcn_conv_wgrad(const void* feats, int64_t num_in, const void* grad_out, const int32_t* nbr,
                    const int32_t* out_rows, const uint32_t* tile_masks, int64_t num_out, int32_t num_offsets, int32_t c_in, int32_t c_out, int dtype,
                    float* grad_weight, int32_t* dev_status, void* stream);
+
+/* The same gradient on the FP32 pipes, for any dtype and widths (fp32 tensors, a 3-channel stem): grad_weight is
+ * written, not accumulated into, from partial sums of row ranges added in order (the same bits on every run).
+ * `workspace`: wcn_conv_wgrad_pairs_workspace_bytes bytes (0: none needed). */
+int wcn_conv_wgrad_pairs_workspace_bytes(int64_t num_out, int32_t num_offsets, int32_t c_in, int32_t c_out, int64_t* bytes);
+int wcn_conv_wgrad_pairs(const void* feats, int64_t num_in, const void* grad_out, const int32_t* nbr,
+                         const int32_t* out_rows, int64_t num_out, int32_t num_offsets, int32_t c_in, int32_t c_out,
+                         int dtype, float* grad_weight, void* workspace, int64_t workspace_bytes, int32_t* dev_status,
+                         void* stream);
 
 /* ------------------------------------------------------------------ self test */
 

@@ -580,3 +580,54 @@ def test_minkunet_matches_oracle(dtype):
     # 5 3x3x3 maps + 4 down maps + the transposed views the output-side kernel needed (a layer run from the
     # input side reads the down map itself)
     assert len(out.cache) == 13 if dtype == torch.float32 else 9 <= len(out.cache) <= 13
+
+
+@pytest.mark.parametrize("ksize,n,c_in,c_out", [(3, 1, 4, 4), (3, 63, 32, 32), (3, 65, 36, 60), (3, 3000, 160, 132), (3, 20000, 32, 32),
+                                                (5, 700, 64, 96), (1, 5000, 96, 128), (3, 12000, 64, 64), (3, 9500, 128, 20)])
+def test_fp32_kernel_matches_the_fp32_pipe_kernel(ksize, n, c_in, c_out):
+    """Both tile heights, every column tile, with and without offset groups, remainders of rows, columns and channel
+    slices, more offsets than are listed at a time; the order of the rows does not matter."""
+    from warpconvnet_b200 import generate_kernel_map
+    g = torch.Generator().manual_seed(n + c_in)
+    e = max(4, int((n * 6) ** (1 / 3)) + 1)
+    cells = torch.randperm(e ** 3, generator=g)[:n]
+    bc = torch.stack([torch.zeros_like(cells), cells // (e * e), cells // e % e, cells % e], 1).int().to(DEV)
+    km_ = generate_kernel_map(bc, bc, (1, 1, 1), (ksize,) * 3)
+    K = ksize ** 3
+    x = torch.randn(n, c_in, generator=g).to(DEV)
+    w = torch.randn(K, c_in, c_out, generator=g).to(DEV)
+    ep = ConvEpilogue(scale=torch.rand(c_out, generator=g).to(DEV), shift=torch.randn(c_out, generator=g).to(DEV),
+                      residual=torch.randn(n, c_out, generator=g).to(DEV), relu=True)
+    for epilogue in (None, ep):
+        got = sparse_conv_fused(x, w, km_, n, epilogue)
+        ref = sparse_conv_fused(x, w, km_, n, epilogue, algo=CONV_SIMT)
+        assert rel_l2(got.cpu().numpy(), ref.cpu().numpy()) < 1e-6
+        if 8 <= ksize ** 3 <= 32:
+            assert torch.equal(got, sparse_conv_fused(x, w, km_, n, epilogue, tile_order=False))
+            assert torch.equal(got, sparse_conv_fused(x, w, km_, n, epilogue, tile_order=True))
+    check_device_status(DEV)
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.float16, torch.bfloat16])
+@pytest.mark.parametrize("ksize,n,c_in,c_out", [(3, 5000, 3, 32), (3, 1025, 8, 64), (2, 4000, 48, 20), (3, 3000, 64, 64),
+                                                (3, 700, 33, 31), (5, 600, 5, 96), (1, 40, 130, 70)])
+def test_pair_weight_gradient_matches_definition(dtype, ksize, n, c_in, c_out):
+    from warpconvnet_b200 import generate_kernel_map
+    from warpconvnet_b200.nn.functional.sparse_conv import sparse_conv_wgrad
+    g = torch.Generator().manual_seed(n + c_out)
+    e = max(4, int((n * 5) ** (1 / 3)) + 1)
+    cells = torch.randperm(e ** 3, generator=g)[:n]
+    bc = torch.stack([torch.zeros_like(cells), cells // (e * e), cells // e % e, cells % e], 1).int().to(DEV)
+    km_ = generate_kernel_map(bc, bc, (1, 1, 1), (ksize,) * 3)
+    x = torch.randn(n, c_in, generator=g).to(dtype).to(DEV)
+    dy = torch.randn(n, c_out, generator=g).to(dtype).to(DEV)
+    got = sparse_conv_wgrad(x, dy, km_, n)
+    again = sparse_conv_wgrad(x, dy, km_, n)
+    if dtype == torch.float32 or c_in % 32 or c_out % 32:
+        assert torch.equal(got, again)
+    want = torch.zeros(ksize ** 3, c_in, c_out, dtype=torch.float64, device=DEV)
+    for k in range(ksize ** 3):
+        i, o = km_[k]
+        want[k] = x[i.long()].double().T @ dy[o.long()].double()
+    check_device_status(DEV)
+    assert rel_l2(got.cpu().numpy(), want.cpu().numpy()) < 1e-6

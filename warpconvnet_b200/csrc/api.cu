@@ -19,6 +19,13 @@ int wcn_conv_narrow_out_fwd(const void* feats, int64_t num_in, int64_t feats_ld,
                             int dtype, const float* scale, const float* shift, const void* residual,
                             int64_t residual_ld, int relu, void* out, int64_t out_ld, int out_dtype,
                             int32_t* dev_status, cudaStream_t st);
+// conv_fp32.cu
+bool wcn_conv_fp32_supported(int c_in, int c_out, int dtype, int out_dtype, const void* feats, int64_t feats_ld,
+                             const void* weight, const void* out, int64_t out_ld, const void* residual, int64_t residual_ld);
+int wcn_conv_fp32_fwd(const void* feats, int64_t num_in, int64_t feats_ld, const void* weight, const int32_t* nbr,
+                      const int32_t* out_rows, int64_t M, int K, int c_in, int c_out, const float* scale,
+                      const float* shift, const void* residual, int64_t residual_ld, int relu, void* out,
+                      int64_t out_ld, int sms, int32_t* dev_status, cudaStream_t st);
 // conv_tcgen05.cu
 bool wcn_conv_tcgen05_supported(int K, int c_in, int c_out, int dtype, int out_dtype);
 int64_t wcn_conv_tcgen05_packed_bytes(int K, int c_in, int c_out);
@@ -126,6 +133,10 @@ extern "C" int wcn_conv_fwd(int algo, const void* feats, int64_t num_in, int64_t
                                            out_dtype, dev_status, st);
     if (rc != WCN_ERR_UNSUPPORTED_CONFIG) return rc;
   }
+  if (algo == WCN_CONV_AUTO && num_in > 0 &&
+      wcn_conv_fp32_supported(c_in, c_out, dtype, out_dtype, feats, feats_ld, weight, out, out_ld, residual, residual_ld))
+    return wcn_conv_fp32_fwd(feats, num_in, feats_ld, weight, nbr, out_rows, num_out, num_offsets, c_in, c_out, scale, shift,
+                             residual, residual_ld, relu, out, out_ld, wcn_num_sms(), dev_status, st);
   return wcn_conv_simt_fwd(feats, num_in, feats_ld, weight, nbr, out_rows, num_out, num_offsets, c_in, c_out, dtype,
                            scale, shift, residual, residual_ld, relu, out, out_ld, out_dtype, dev_status, st);
 }

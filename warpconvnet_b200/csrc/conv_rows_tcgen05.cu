@@ -502,7 +502,7 @@ int wcn_conv_rows_tcgen05_fwd(const void* feats, int64_t num_in, int64_t feats_l
                              CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
   if (rc != CUDA_SUCCESS) return WCN_ERR_UNSUPPORTED_CONFIG;
 
-  const int sms = num_sms();
+  const int sms = wcn_num_sms();
   const unsigned grid = (unsigned)(p.units < sms ? p.units : sms);
   const bool bf = dtype == WCN_BF16;
 #define WCN_ROWS_CASE(BKV, BFV, TOV) return launch_rows<BKV, BFV, TOV>(map, p, smem, grid, st)

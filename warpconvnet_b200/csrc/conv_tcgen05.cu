@@ -755,7 +755,7 @@ constexpr int MAX_SLICES = 16;
 // slices); otherwise the output columns are divided among CTAs, each re-gathering the rows,
 // which stay in L2 (split_k < 0 forces -split_k column blocks).
 bool plan_launch(ConvTcParams& p, int bk, int split_k, size_t* smem, dim3* grid) {
-  const int sms = num_sms();
+  const int sms = wcn_num_sms();
   const int64_t tiles = (p.M + BLOCK_M - 1) / BLOCK_M;
   int S = 1;
   if (split_k >= 2) {

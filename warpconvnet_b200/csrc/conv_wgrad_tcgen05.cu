@@ -238,7 +238,7 @@ int launch_wgrad(WgradParams& p, cudaStream_t st) {
   p.cols = cols;
   // enough CTAs for a few waves, but at least four steps each so the set-up cost stays small
   const int64_t total_steps = (p.M + WG_ROWS - 1) / WG_ROWS;
-  int64_t ranges = (4 * (int64_t)num_sms() + groups - 1) / groups;
+  int64_t ranges = (4 * (int64_t)wcn_num_sms() + groups - 1) / groups;
   if (ranges > (total_steps + 3) / 4) ranges = (total_steps + 3) / 4;
   if (ranges < 1) ranges = 1;
   p.steps_per_cta = (int)((total_steps + ranges - 1) / ranges);

@@ -189,17 +189,4 @@ template <int RB> __device__ __forceinline__ uint64_t smem_desc_mn(uint32_t addr
   return d;
 }
 
-// Multiprocessors of the current device (cached per device).
-inline int num_sms() {
-  static int cached[64] = {};
-  int dev = 0;
-  if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return 148;
-  if (!cached[dev]) {
-    int n = 0;
-    if (cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || n <= 0) n = 148;
-    cached[dev] = n;
-  }
-  return cached[dev];
-}
-
 }  // namespace

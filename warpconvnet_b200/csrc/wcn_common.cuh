@@ -114,3 +114,16 @@ static inline int wcn_dtype_size(int dtype) { return dtype == WCN_F32 ? 4 : 2; }
 __device__ __forceinline__ void wcn_report_bounds(int32_t* dev_status) {
   if (dev_status) atomicCAS(dev_status, 0, (int)WCN_ERR_BOUNDS);
 }
+
+// Multiprocessors of the current device (cached per device).
+static inline int wcn_num_sms() {
+  static int cached[64] = {};
+  int dev = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return 148;
+  if (!cached[dev]) {
+    int n = 0;
+    if (cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || n <= 0) n = 148;
+    cached[dev] = n;
+  }
+  return cached[dev];
+}

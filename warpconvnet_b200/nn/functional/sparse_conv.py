@@ -41,6 +41,9 @@ from ...utils.ntuple import ntuple
 from ...utils.type_cast import _maybe_cast, _min_dtype
 
 
+_NATIVE_DTYPES = (torch.float32, torch.float16, torch.bfloat16)
+
+
 class STRIDED_CONV_MODE(enum.Enum):
     REDUCE_AND_STRIDE = "reduce_and_stride"
     STRIDE_ONLY = "stride_only"
@@ -714,14 +717,14 @@ def _cached_bricks(voxels: Optional[Voxels], coords: Tensor):
 
 def sparse_conv_wgrad(in_features: Tensor, grad_output: Tensor, kernel_map: IntSearchResult,
                       num_out_coords: int, tile_order: bool = False) -> Optional[Tensor]:
-    """``dW[k] = X[in_k]^T @ dY[out_k]`` for every kernel offset in one launch on the tensor cores
-    (fp16 / bf16 operands, fp32 result ``[K, C_in, C_out]``), or None when the shape is not one the
-    native kernel takes (the caller then uses a GEMM per offset)."""
+    """``dW[k] = X[in_k]^T @ dY[out_k]`` for every kernel offset, fp32 result ``[K, C_in, C_out]``: one launch on the
+    tensor cores for fp16 / bf16 widths that are multiples of 32 (output width at most 256), the pair kernel on the FP32
+    pipes for fp32 and all other widths.  None when the operands are in no native dtype (the caller then uses a
+    GEMM per offset)."""
     require_cuda(in_features, "in_features")
     x, g = in_features.contiguous(), grad_output.contiguous()
     K, c_in, c_out = len(kernel_map), x.shape[1], g.shape[1]
-    if (x.dtype not in (torch.float16, torch.bfloat16) or g.dtype != x.dtype or c_in % 32 or c_out % 32
-            or c_out > 256 or K > 32 or x.shape[0] == 0 or num_out_coords == 0):
+    if x.dtype not in _NATIVE_DTYPES or g.dtype != x.dtype or x.shape[0] == 0 or num_out_coords == 0:
         return None
     dev = x.device
     tiled = bool(tile_order)
@@ -729,6 +732,14 @@ def sparse_conv_wgrad(in_features: Tensor, grad_output: Tensor, kernel_map: IntS
         nbr, out_rows = kernel_map.tiled_neighbor_table(num_out_coords)
     else:
         nbr, out_rows = kernel_map.neighbor_table(num_out_coords), None
+    if x.dtype == torch.float32 or c_in % 32 or c_out % 32 or c_out > 256 or K > 32:
+        gw = torch.empty((K, c_in, c_out), dtype=torch.float32, device=dev)
+        nbytes = query_bytes("wcn_conv_wgrad_pairs_workspace_bytes", num_out_coords, K, c_in, c_out)
+        ws = torch.empty(nbytes, dtype=torch.uint8, device=dev) if nbytes else None
+        check(lib().wcn_conv_wgrad_pairs(ptr(x), x.shape[0], ptr(g), ptr(nbr), ptr(out_rows), num_out_coords, K, c_in,
+                                         c_out, dtype_code(x.dtype), ptr(gw), ptr(ws), nbytes, ptr(device_status(dev)),
+                                         stream_ptr(dev)), "wcn_conv_wgrad_pairs")
+        return gw
     masks = kernel_map.tile_masks(num_out_coords, tiled) if K > 1 else None  # steps without neighbours are skipped
     gw = torch.zeros((K, c_in, c_out), dtype=torch.float32, device=dev)
     check(lib().wcn_conv_wgrad(ptr(x), x.shape[0], ptr(g), ptr(nbr), ptr(out_rows), ptr(masks), num_out_coords, K,
@@ -755,8 +766,7 @@ class _SparseConvFunction(torch.autograd.Function):
     dW_k = X[in_k]^T @ dY[out_k], a GEMM per offset.  With the implicit algorithms (the reference's
     AD gather-scatter with the maps swapped and W^T, and its trAB gather / split-K kernels,
     :472-480, 591-604): dX is ONE launch of the forward kernel over the transposed neighbour table
-    with the weights transposed, dW ONE launch of the tensor-core weight-gradient kernel (shapes it
-    does not take fall back to the per-offset GEMMs)."""
+    with the weights transposed, dW ONE launch of a weight-gradient kernel."""
 
     @staticmethod
     def forward(ctx, in_features, weight, kernel_map, num_out_coords, algo, compute_dtype, epilogue,
@@ -777,8 +787,9 @@ class _SparseConvFunction(torch.autograd.Function):
         dt = ctx.compute_dtype if ctx.compute_dtype is not None else x.dtype
         xc, wc, gc = x.to(dt), w.to(dt), grad_output.contiguous().to(dt)
         need_gx, need_gw = ctx.needs_input_grad[0], ctx.needs_input_grad[1]
-        native_dx = (need_gx and ctx.bwd_algo != SPARSE_CONV_BWD_ALGO_MODE.EXPLICIT_GEMM and gc.is_cuda
-                     and dt in (torch.float32, torch.float16, torch.bfloat16) and x.shape[0] > 0)
+        native = (ctx.bwd_algo != SPARSE_CONV_BWD_ALGO_MODE.EXPLICIT_GEMM and gc.is_cuda and dt in _NATIVE_DTYPES
+                  and x.shape[0] > 0)
+        native_dx = native and need_gx
         gx = None
         if native_dx:
             with torch.no_grad():
@@ -787,7 +798,7 @@ class _SparseConvFunction(torch.autograd.Function):
         elif need_gx:
             gx = torch.zeros_like(xc)
         gw = None
-        if need_gw and native_dx:  # the implicit algorithms: one tensor-core launch when the shape allows
+        if need_gw and native:
             with torch.no_grad():
                 gw = sparse_conv_wgrad(xc.detach(), gc.detach(), km, gc.shape[0])
         native_dw = gw is not None
@@ -1024,7 +1035,6 @@ def _layer_tables(x: Voxels, kernel_size, stride, dilation, transposed: bool, ta
 
 _NATIVE_ALGOS = (SPARSE_CONV_FWD_ALGO_MODE.AUTO, SPARSE_CONV_FWD_ALGO_MODE.IMPLICIT_GEMM,
                  SPARSE_CONV_FWD_ALGO_MODE.CUTLASS_IMPLICIT_GEMM)
-_NATIVE_DTYPES = (torch.float32, torch.float16, torch.bfloat16)
 
 
 def run_layer(layer, x: Voxels, target: Optional[Voxels], epilogue: Optional[ConvEpilogue]) -> Optional[Voxels]:
