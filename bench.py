@@ -285,6 +285,8 @@ def install_conv_profiler(profile):
     plan uses) so that each call of a step is recorded for replay."""
     import warpconvnet_b200.nn.functional.sparse_conv as F
     from warpconvnet_b200._native import query_bytes, dtype_code
+    from warpconvnet_b200.examples.mink_unet import _LaunchPlan
+    _LaunchPlan.use_program = False  # single launches are recorded: the same kernels, one call each
     orig = F.sparse_conv_fused
     orig_launch = F.FusedConvLaunch.__call__
     orig_rows = F.FusedRowsLaunch.__call__
@@ -318,6 +320,7 @@ def install_conv_profiler(profile):
         F.sparse_conv_fused = orig
         F.FusedConvLaunch.__call__ = orig_launch
         F.FusedRowsLaunch.__call__ = orig_rows
+        _LaunchPlan.use_program = True
     return restore
 
 

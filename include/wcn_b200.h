@@ -440,6 +440,86 @@ int wcn_conv_wgrad_pairs(const void* feats, int64_t num_in, const void* grad_out
                          int dtype, float* grad_weight, void* workspace, int64_t workspace_bytes, int32_t* dev_status,
                          void* stream);
 
+/* ------------------------------------------------------------------ Morton order, pyramid, maps of all levels */
+
+/* Rows of a batch of voxel sets in Morton order, one cooperative launch:
+ *   perm [n] int64      sorted row -> caller's row, stable by (batch item, code)
+ *   codes [n] int64     Morton code of the caller's rows about the corner
+ *   rows [n, 4] int32   sorted (batch, x, y, z), 16-byte aligned
+ *   info [8] int32      [0..2] the corner: the per-axis minimum rounded down to a multiple of 16; [3] bits per axis of
+ *                       the codes; [4] 1 when no two positions share a code (extent below 2^21)
+ *   feats_sorted        rows of feat_row_bytes (even; feats NULL: none) in sorted order
+ * `offsets` is a HOST array [batches + 1] of row offsets; at most 255 batch items (else WCN_ERR_UNSUPPORTED_CONFIG).
+ * Replaces the per-batch argsort of warpconvnet/coords/ops/serialization.py:60-254 behind Voxels.sort
+ * (geometry/types/voxels.py:255-267). */
+int wcn_morton_sort_workspace_bytes(int64_t n, int64_t* bytes);
+int wcn_morton_sort(const int32_t* coords, int64_t n, const int64_t* offsets, int32_t batches, int64_t* codes,
+                    int64_t* perm, int32_t* rows, int32_t* info, const void* feats, void* feats_sorted,
+                    int32_t feat_row_bytes, void* workspace, int32_t* dev_status, void* stream);
+
+/* The coarser levels of rows sorted by wcn_morton_sort: level l (1..levels, at most 4) holds the distinct rows of
+ * floor(row / 2^l) in first-occurrence order, as wcn_unique_emit gives them.
+ *   out [levels, n, 4], first [levels, n]   rows of each level and, per row, its first row on the level below
+ *   counts [24]   [0..6] distinct cells of 2^s voxels about the corner, [7] non-zero when two rows are equal,
+ *                 [8 + 4 l ..] the corner of level l + 1 (a copy in 16-byte steps)
+ *   host          HOST-mapped (pinned) int64 [levels * (batches + 1) + 2]: row offsets of every level, then 1 when the
+ *                 levels are usable (rows distinct, codes whole), then the device status word.  Written by the kernel:
+ *                 valid once the stream has passed it.
+ * Replaces stride_coords level by level (warpconvnet/geometry/coords/ops/stride.py:17-54). */
+int wcn_pyramid_workspace_bytes(int64_t n, int64_t* bytes);
+int wcn_pyramid(const int32_t* rows, int64_t n, const int32_t* info, const int64_t* offsets, int32_t batches,
+                int32_t levels, int32_t* out, int32_t* first, int32_t* counts, int64_t* host, void* workspace,
+                const int32_t* dev_status, void* stream);
+
+/* One level of wcn_level_maps. */
+typedef struct {
+  const int32_t* rows;        /* [n, 4] of wcn_morton_sort (level 0) or wcn_pyramid */
+  int64_t n;
+  void* bricks;               /* wcn_level_brick_bytes(n) bytes of scratch, 32-byte aligned */
+  int32_t* order;             /* [n] slot -> row of the tile order; NULL: slots are rows */
+  int32_t* nbr;               /* [27, n] 3x3x3 neighbour table, slots in tile order */
+  int32_t* child;             /* [8, n] row of the level below at each 2x2x2 offset, -1 where none; NULL: not wanted */
+  const int32_t* first_child; /* [n] of wcn_pyramid (child only) */
+  const int32_t* rows_below;  /* [n_below, 4] (child only) */
+  int64_t n_below;
+  int64_t level;              /* 0..4 */
+} wcn_level;
+
+/* 3x3x3 maps in tile order and children tables of up to five levels, a launch per stage for all of them.  The rows must
+ * be what wcn_pyramid called usable.  (nbr, order) is a pair for wcn_conv_fwd, child the [8, n] table of the 2x2x2
+ * stride-2 convolution and of wcn_conv_rows_fwd on the way back up.
+ * Replaces generate_kernel_map per layer geometry (warpconvnet/geometry/coords/search/torch_discrete.py:365-466). */
+int wcn_level_brick_bytes(int64_t n, int64_t* bytes);
+int wcn_level_maps(const wcn_level* levels, int32_t num_levels, const int32_t* info, const int32_t* counts, void* stream);
+
+/* ------------------------------------------------------------------ a network as one call */
+
+/* One convolution of wcn_net_run: columns [src_col, src_col + c_in) of buffer src to columns [dst_col, ..) of buffer dst,
+ * + columns [res_col, ..) of buffer res (res < 0: none). */
+typedef struct {
+  int32_t kind;        /* 0: wcn_conv_fwd over table `table`; 1: wcn_conv_rows_fwd, dst_rows = nbr of `table` (-1: identity) */
+  int32_t table;
+  int32_t level_in, level_out;
+  int32_t num_offsets, c_in, c_out, c_out_packed, relu;
+  int32_t src, src_col, dst, dst_col, res, res_col;
+  int32_t reserved;
+  const void* weight;
+  const void* packed;
+  const float* scale;
+  const float* shift;
+} wcn_net_op;
+typedef struct { void* data; int64_t ld; } wcn_net_buffer;                       /* rows of ld elements */
+typedef struct { const int32_t* nbr; const int32_t* out_rows; } wcn_net_table;
+
+/* Enqueues the convolutions in order, all tensors of one 16-bit dtype.  `rows` are the row counts per level;
+ * `workspace` of wcn_net_workspace_bytes serves the offset slices of every op in turn.  *launches receives the kernels
+ * enqueued.  The reference runs the same layers from Python, one module at a time
+ * (warpconvnet/nn/modules/sequential.py:14-62, examples/mink_unet.py:212-413). */
+int wcn_net_workspace_bytes(const wcn_net_op* ops, int32_t num_ops, const int64_t* rows, int dtype, int64_t* bytes);
+int wcn_net_run(const wcn_net_op* ops, int32_t num_ops, const int64_t* rows, const wcn_net_buffer* buffers,
+                const wcn_net_table* tables, int dtype, void* workspace, int64_t workspace_bytes, int32_t* launches,
+                int32_t* dev_status, void* stream);
+
 /* ------------------------------------------------------------------ self test */
 
 /* Checks the library's bounded device-side waits: launches one small kernel that waits, with a

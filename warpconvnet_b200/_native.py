@@ -63,11 +63,34 @@ SIGNATURES = {
     "wcn_conv_workspace_bytes": [_c_i32, _c_i64, _c_i32, _c_i32, _c_i32, _c_i32, _c_i32, _c_i32, _p_i64],
     "wcn_conv_fwd": [_c_i32, _c_vp, _c_i64, _c_i64, _c_vp, _c_vp, _c_vp, _c_vp, _c_i64, _c_i32, _c_i32, _c_i32, _c_i32,
                      _c_vp, _c_vp, _c_vp, _c_i64, _c_i32, _c_vp, _c_i64, _c_i32, _c_i32, _c_vp, _c_i64, _c_vp, _c_vp],
+    "wcn_morton_sort_workspace_bytes": [_c_i64, _p_i64],
+    "wcn_morton_sort": [_c_vp, _c_i64, _c_vp, _c_i32, _c_vp, _c_vp, _c_vp, _c_vp, _c_vp, _c_vp, _c_i32, _c_vp, _c_vp, _c_vp],
+    "wcn_pyramid_workspace_bytes": [_c_i64, _p_i64],
+    "wcn_pyramid": [_c_vp, _c_i64, _c_vp, _c_vp, _c_i32, _c_i32, _c_vp, _c_vp, _c_vp, _c_vp, _c_vp, _c_vp, _c_vp],
+    "wcn_level_brick_bytes": [_c_i64, _p_i64],
+    "wcn_level_maps": [_c_vp, _c_i32, _c_vp, _c_vp, _c_vp],
+    "wcn_net_workspace_bytes": [_c_vp, _c_i32, _c_vp, _c_i32, _p_i64],
+    "wcn_net_run": [_c_vp, _c_i32, _c_vp, _c_vp, _c_vp, _c_i32, _c_vp, _c_i64, _c_vp, _c_vp, _c_vp],
     "wcn_selftest_bounded_wait": [_c_i64, _c_vp, _c_vp, _c_vp],
     "wcn_conv_rows_supported": [_c_i32, _c_i32, _c_i32, _c_i32, _c_i32, _c_vp],
     "wcn_conv_rows_fwd": [_c_vp, _c_i64, _c_i64, _c_vp, _c_vp, _c_i64, _c_i32, _c_i32, _c_i32, _c_i32, _c_i32, _c_vp, _c_vp,
                           _c_vp, _c_i64, _c_i32, _c_vp, _c_i64, _c_i32, _c_vp, _c_vp],
 }
+
+
+
+class Level(ctypes.Structure):
+    """``wcn_level``"""
+    _fields_ = [("rows", _c_vp), ("n", _c_i64), ("bricks", _c_vp), ("order", _c_vp), ("nbr", _c_vp), ("child", _c_vp),
+                ("first_child", _c_vp), ("rows_below", _c_vp), ("n_below", _c_i64), ("level", _c_i64)]
+
+
+class NetOp(ctypes.Structure):
+    """``wcn_net_op``"""
+    _fields_ = [(f, _c_i32) for f in ("kind", "table", "level_in", "level_out", "num_offsets", "c_in", "c_out", "c_out_packed",
+                                      "relu", "src", "src_col", "dst", "dst_col", "res", "res_col", "reserved")] + [
+        (f, _c_vp) for f in ("weight", "packed", "scale", "shift")]
+
 
 _lib = None
 
@@ -79,7 +102,7 @@ KERNELS_PER_CALL = {
     "wcn_kmap_tile_order": 3, "wcn_conv_wgrad": 1, "wcn_conv_wgrad_pairs": 2, "wcn_kmap_tile_masks": 1, "wcn_row_reduce": 1, "wcn_row_reduce_train": 1, "wcn_row_reduce_backward": 1, "wcn_kmap_search_self": 1, "wcn_kmap_search_dilated": 1, "wcn_kmap_count": 1,
     "wcn_gather_rows": 1, "wcn_scatter_add_rows": 1, "wcn_conv_pack_weight": 1, "wcn_conv_fwd": 1,
     "wcn_selftest_bounded_wait": 1, "wcn_brick_build": 3, "wcn_kmap_search_bricks": 1,
-    "wcn_conv_rows_fwd": 1,
+    "wcn_conv_rows_fwd": 1, "wcn_morton_sort": 1, "wcn_pyramid": 2, "wcn_level_maps": 5,
 }
 LAUNCH_COUNTS: Counter = Counter()
 

@@ -4,6 +4,7 @@
 // compaction, no host synchronisation inside the library.
 #include <atomic>
 
+#include "tile_order.cuh"
 #include "wcn_common.cuh"
 
 namespace {
@@ -347,8 +348,6 @@ __global__ void nbr_transpose_kernel(const int32_t* __restrict__ nbr_fwd, int64_
 // tile local.  Windows of 16384 rows (tables of more than 4096 rows) leave 7-9 % fewer (tile,
 // offset) pairs than windows of 4096 on room scans (11.1 / 13.0 / 16.5 offsets per tile at 2, 4 and
 // 8 cm against 11.9 / 14.1 / 18.2).
-constexpr int kTileWindowSmall = 4096, kTileWindowLarge = 16384;
-constexpr int kTileOrderThreads = 1024;
 constexpr int kTileCopyOffsets = 3;  // offsets per block of the permuted copy
 
 // Pass 1: presence mask of every output row (one thread per row, all loads in flight).
@@ -360,20 +359,8 @@ __global__ void kmap_row_mask_kernel(const int32_t* __restrict__ nbr, int64_t M,
   for (int k = 0; k < 32; ++k) v[k] = k < K ? __ldg(&nbr[(int64_t)k * M + m]) : -1;
   uint32_t mask = 0;
   if (K == 27) {
-    // Sort key of a 3x3x3 window: the centre in bit 0, then the 6 face, 12 edge and 8 corner offsets, so that
-    // the rarest offsets are the most significant bits and rows that share them end up in the same tiles
-    // (2-4 % fewer (tile, offset) pairs than offsets in index order).  Only the order of the rows depends on it.
 #pragma unroll
-    for (int k = 0; k < 27; ++k) {
-      const int ax = (k / 9 != 1) + ((k / 3) % 3 != 1) + (k % 3 != 1);   // 0 centre, 1 face, 2 edge, 3 corner
-      int pos = 0;   // offsets of a lower class, and earlier ones of the same class, come first
-#pragma unroll
-      for (int q = 0; q < 27; ++q) {
-        const int aq = (q / 9 != 1) + ((q / 3) % 3 != 1) + (q % 3 != 1);
-        pos += (aq < ax) || (aq == ax && q < k);
-      }
-      mask |= (uint32_t)(v[k] >= 0) << pos;
-    }
+    for (int k = 0; k < 27; ++k) mask |= (uint32_t)(v[k] >= 0) << presence_bit27(k);
   } else {
 #pragma unroll
     for (int k = 0; k < 32; ++k) mask |= (uint32_t)(v[k] >= 0) << k;
@@ -400,91 +387,12 @@ __global__ void kmap_tile_mask_kernel(const int32_t* __restrict__ nbr, int64_t M
   if (threadIdx.x == 0) masks[blockIdx.x] = part[0] | part[1] | part[2] | part[3];
 }
 
-// Pass 2: one block per window sorts its rows by (mask, row) and replaces the masks by the row
-// order.  Stable least-significant-digit radix sort of the permutation, 7 bits per pass
-// (ceil(K / 7) passes): a warp owns 128 consecutive positions, ranks equal digits with
-// match_any (lane order = position order, so the sort is stable and deterministic), the
-// per-(digit, warp) counts are scanned digit-major by the block, and rows scatter to their place.
-constexpr int kDigitBits = 7, kDigits = 1 << kDigitBits;
-
+// Pass 2: one block per window sorts its rows by (mask, row) and replaces the masks by the row order.
 template <int kTileWindow>
 __global__ void __launch_bounds__(kTileOrderThreads)
 kmap_window_sort_kernel(int32_t* __restrict__ rows_io, int64_t M, int K) {
   extern __shared__ __align__(16) uint8_t sort_smem[];
-  uint32_t* mask_s = reinterpret_cast<uint32_t*>(sort_smem);                       // mask of local row r (never moves)
-  uint16_t (*perm_s)[kTileWindow] = reinterpret_cast<uint16_t (*)[kTileWindow]>(mask_s + kTileWindow);  // current / next order
-  uint16_t* cnt = reinterpret_cast<uint16_t*>(perm_s + 2);                         // [digit][warp] counts, then start positions
-  uint32_t* warp_sums = reinterpret_cast<uint32_t*>(cnt + kDigits * 32);
-  constexpr int kBatches = kTileWindow / kTileOrderThreads;                        // rows per thread
-  const int64_t base = (int64_t)blockIdx.x * kTileWindow;
-  const int n = (int)min((int64_t)kTileWindow, M - base);
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  for (int i = threadIdx.x; i < kTileWindow; i += kTileOrderThreads) {
-    mask_s[i] = i < n ? (uint32_t)rows_io[base + i] : 0xFFFFFFFFu;  // padding sorts last (ties: stable)
-    perm_s[0][i] = (uint16_t)i;
-  }
-  int cur = 0;
-  const int passes = (K + kDigitBits - 1) / kDigitBits;
-  for (int pass = 0; pass < passes; ++pass) {
-    const int shift = pass * kDigitBits;
-    for (int i = threadIdx.x; i < kDigits * 32; i += kTileOrderThreads) cnt[i] = 0;
-    __syncthreads();
-    // rank inside (warp, digit); positions of a warp: warp * (32 * kBatches) + batch*32 + lane
-    uint16_t row[kBatches];
-    int dig[kBatches], rank[kBatches];
-#pragma unroll
-    for (int b = 0; b < kBatches; ++b) {
-      row[b] = perm_s[cur][warp * (32 * kBatches) + b * 32 + lane];
-      dig[b] = (int)((mask_s[row[b]] >> shift) & (kDigits - 1));
-      const unsigned same = __match_any_sync(0xFFFFFFFFu, dig[b]);
-      const int r = __popc(same & ((1u << lane) - 1u));
-      const int leader = __ffs(same) - 1;
-      int before = 0;
-      if (r == 0) {  // the first lane of each digit updates the warp's count
-        before = cnt[dig[b] * 32 + warp];
-        cnt[dig[b] * 32 + warp] = (uint16_t)(before + __popc(same));
-      }
-      before = __shfl_sync(0xFFFFFFFFu, before, leader);
-      rank[b] = before + r;
-      __syncwarp();  // the next batch reads the counts written here
-    }
-    __syncthreads();
-    // exclusive scan of the counts in (digit, warp) order: 4 consecutive entries per thread
-    {
-      constexpr int kPer = kDigits * 32 / kTileOrderThreads;
-      uint32_t v[kPer], sum = 0;
-#pragma unroll
-      for (int j = 0; j < kPer; ++j) { v[j] = cnt[threadIdx.x * kPer + j]; sum += v[j]; }
-      uint32_t incl = sum;
-#pragma unroll
-      for (int d = 1; d < 32; d <<= 1) {
-        const uint32_t o = __shfl_up_sync(0xFFFFFFFFu, incl, d);
-        if (lane >= d) incl += o;
-      }
-      if (lane == 31) warp_sums[warp] = incl;
-      __syncthreads();
-      if (warp == 0) {
-        const uint32_t w = warp_sums[lane];
-        uint32_t wi = w;
-#pragma unroll
-        for (int d = 1; d < 32; d <<= 1) {
-          const uint32_t o = __shfl_up_sync(0xFFFFFFFFu, wi, d);
-          if (lane >= d) wi += o;
-        }
-        warp_sums[lane] = wi - w;
-      }
-      __syncthreads();
-      uint32_t run = warp_sums[warp] + incl - sum;
-#pragma unroll
-      for (int j = 0; j < kPer; ++j) { cnt[threadIdx.x * kPer + j] = (uint16_t)run; run += v[j]; }
-    }
-    __syncthreads();
-#pragma unroll
-    for (int b = 0; b < kBatches; ++b) perm_s[cur ^ 1][cnt[dig[b] * 32 + warp] + rank[b]] = row[b];
-    cur ^= 1;
-    __syncthreads();
-  }
-  for (int i = threadIdx.x; i < n; i += kTileOrderThreads) rows_io[base + i] = (int32_t)(base + perm_s[cur][i]);
+  sort_window<kTileWindow>(rows_io, M, K, blockIdx.x, sort_smem);
 }
 
 // Pass 3: nbr_tiled[k][s] = nbr[k][out_rows[s]]; a block stages one window of one offset in
@@ -541,7 +449,7 @@ inline unsigned grid_for(int64_t n) { return (unsigned)((n + kThreads - 1) / kTh
 template <int W>
 int tile_order_windows(const int32_t* nbr, int64_t num_out, int num_offsets, int32_t* out_rows, int32_t* nbr_tiled,
                        cudaStream_t st) {
-  constexpr size_t sort_bytes = (size_t)W * 4 + 2 * (size_t)W * 2 + kDigits * 32 * 2 + 32 * 4;
+  constexpr size_t sort_bytes = sort_window_bytes<W>();
   constexpr size_t permute_bytes = (size_t)W * 4 + (size_t)W * 2;
   static bool configured[64] = {};
   int dev = 0;

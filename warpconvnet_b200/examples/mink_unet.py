@@ -9,15 +9,19 @@ one fused kernel.
 """
 from __future__ import annotations
 
+import ctypes
 import operator
 from typing import Optional, Union
 
 import torch
 import torch.nn as nn
 
+from .._native import LAUNCH_COUNTS, NetOp, check, device_status, dtype_code, lib, ptr, query_bytes, stream_ptr
 from ..geometry.types.voxels import Voxels
 from ..geometry.coords.search.cache import IntSearchCache
+from ..geometry.coords.search.level_maps import LevelMaps
 from ..geometry.coords.search.search_results import IntSearchResult
+from ..nn.functional import sparse_conv
 from ..nn.functional.sparse_conv import (STRIDED_CONV_MODE, TILE_ORDER_MIN_OFFSETS, TILE_ORDER_MIN_ROWS, ConvEpilogue,
                                          FusedConvLaunch, FusedRowsLaunch, _identity_map, _implicit_gemm_forward_logic, _merge_bias,
                                          generate_output_coords_and_kernel_map, prefetch_strided_coordinates)
@@ -222,7 +226,10 @@ class _LaunchPlan:
     and one foreign call per convolution remain, instead of the ``Module`` -> ``Sequential`` ->
     ``spatially_sparse_conv`` stack for each of the 60-odd layers.  The numbers are those of the
     module-by-module path (same kernels, same epilogues, same buffers without concatenation
-    copies), and the kernel maps land in the input's shared cache under the same keys."""
+    copies), and the kernel maps land in the input's shared cache under the same keys.  For inputs that
+    ``Voxels.sort`` has ordered the records themselves become one foreign call (:class:`_Program`)."""
+
+    use_program = True  # False: always layer by layer, e.g. to time single launches
 
     def __init__(self, model: "MinkUNetBase", dtype: torch.dtype, device: torch.device):
         self.dtype, self.device = dtype, device
@@ -264,6 +271,7 @@ class _LaunchPlan:
         head_shift = head.bias.detach().float() if head.bias is not None else None
         self.head = FusedConvLaunch(head.weight, dtype, None, head_shift)
         self.head_rows = FusedRowsLaunch(head.weight, dtype, None, head_shift)
+        self._program = None
 
     def current(self, dtype, device) -> bool:
         """True while no parameter or buffer has been written or re-allocated since the plan was made
@@ -287,6 +295,17 @@ class _LaunchPlan:
         return x
 
     def run(self, x: Voxels, restore_order: bool):
+        if self.use_program and x.batched_coordinates._shared.get("morton_info") is not None:
+            if self._program is None:
+                self._program = _Program(self)
+            if self._program.usable:
+                done = self._program.run(x, restore_order)
+                if done is not None:
+                    return done
+        return self._run_layers(x, restore_order)
+
+    def _run_layers(self, x: Voxels, restore_order: bool):
+        """Layer by layer over any coordinate set (unsorted rows, repeated voxels, fp32)."""
         P, dtype, dev = self.planes, self.dtype, self.device
         ics = [x.batched_coordinates] + prefetch_strided_coordinates(x, [2, 2, 2, 2])
         n = [ic.batched_tensor.shape[0] for ic in ics]
@@ -361,6 +380,140 @@ class _LaunchPlan:
         if self.head_rows.takes(cur):
             return x._derive(self.head_rows(cur, None, n[0]))
         return x._derive(self.head(cur, _identity_map(n[0], dev).neighbor_table(n[0]), None, n[0]))
+
+
+class _Program:
+    """The launch records of a plan as an op list for ``wcn_net_run``: per forward, one call computes the coordinate
+    pyramid, one all kernel maps, one enqueues every convolution; activations live in one allocation.  The numbers are
+    those of the layer-by-layer path (same kernels, same order of sums)."""
+
+    IN, OUT, TEMP = 0, 5, 6          # buffers: input, joined skip buffers of levels 0..3 (1..4), logits, 4 per level
+    CHILD, IDENTITY, PERM = 5, 9, 10  # tables: 3x3x3 of levels 0..4, children (level -> level + 1), 1x1x1, sort permutation
+
+    def __init__(self, plan: "_LaunchPlan"):
+        P, init = plan.planes, plan.init_dim
+        self.dtype, self.device = plan.dtype, plan.device
+        self.joined_width = [P[7] + init, P[6] + P[0], P[5] + P[1], P[4] + P[2]]
+        skip_col = [P[7], P[6], P[5], P[4]]
+        ops, width = [], {}
+
+        def emit(kind, rec, level_in, level_out, table, src, dst, res=(-1, 0), relu=None):
+            width[dst[0]] = max(width.get(dst[0], 0), dst[1] + rec.c_out)
+            ops.append((kind, rec, level_in, level_out, table, src, dst, res, rec.relu if relu is None else relu))
+
+        def temp(level, i):
+            return self.TEMP + 4 * level + i
+
+        def stage(blocks, level, src, out=None):
+            for i, (c1, c2, proj) in enumerate(blocks):
+                identity = src
+                if proj is not None:
+                    identity = (temp(level, 0), 0)
+                    if proj[1].usable:
+                        emit(1, proj[1], level, level, -1, src, identity)
+                    else:  # weights of one offset too large for the input-side kernel
+                        emit(0, proj[0], level, level, self.IDENTITY, src, identity)
+                mid = (temp(level, 1), 0)
+                emit(0, c1, level, level, level, src, mid)
+                dst = (temp(level, 3 if src[0] == temp(level, 2) else 2), 0)
+                if out is not None and i == len(blocks) - 1:
+                    dst = out
+                emit(0, c2, level, level, level, mid, dst, identity)
+                src = dst
+            return src
+
+        emit(0, plan.stem, 0, 0, self.IDENTITY, (self.IN, 0), (1, skip_col[0]))
+        cur = (1, skip_col[0])
+        for level in range(4):
+            down = (temp(level + 1, 2), 0)
+            emit(0, plan.down[level], level, level + 1, self.CHILD + level, cur, down)
+            cur = stage(plan.enc[level], level + 1, down, (level + 2, skip_col[level + 1]) if level < 3 else None)
+        for i, level in enumerate((3, 2, 1, 0)):
+            emit(1, plan.up[i][1], level + 1, level, self.CHILD + level, cur, (level + 1, 0))
+            cur = stage(plan.dec[i], level, (level + 1, 0))
+        emit(1, plan.head_rows, 0, 0, -1, cur, (self.OUT, 0))
+
+        half = plan.dtype in (torch.float16, torch.bfloat16)
+        self.usable = half and all((rec.usable if kind == 1 else rec.packed is not None or rec is plan.stem)
+                                   and all(c % 8 == 0 for c in (src[1], dst[1], res[1]))
+                                   for kind, rec, _, _, _, src, dst, res, _ in ops)
+        self.usable = self.usable and all(w % 8 == 0 for b, w in width.items() if b != self.OUT) \
+            and all(w % 8 == 0 for w in self.joined_width)
+        if not self.usable:
+            return
+        self._records = [op[1] for op in ops]  # keep the weights they point to
+        self.ops = (NetOp * len(ops))()
+        for o, (kind, rec, level_in, level_out, table, src, dst, res, relu) in zip(self.ops, ops):
+            o.kind, o.table, o.level_in, o.level_out = kind, table, level_in, level_out
+            o.num_offsets, o.c_in, o.c_out, o.relu = rec.K, rec.c_in, rec.c_out, int(relu)
+            o.c_out_packed = rec.c_pack if kind == 1 else rec.c_out
+            (o.src, o.src_col), (o.dst, o.dst_col), (o.res, o.res_col) = src, dst, res
+            o.weight = None if kind == 1 else rec._w_ptr
+            o.packed, o.scale, o.shift = rec._packed_ptr, rec._scale_ptr, rec._shift_ptr
+        self.classes = plan.head_rows.c_out
+        # activations besides the joined buffer of level 0, which the stem needs before the coarser sizes are known
+        self.arena = [(1 + l, l, self.joined_width[l]) for l in (1, 2, 3)]
+        self.arena += [(b, (b - self.TEMP) // 4, w) for b, w in sorted(width.items()) if b >= self.TEMP]
+        self.dtype_code = dtype_code(plan.dtype)
+
+    def run(self, x: Voxels, restore_order: bool):
+        dev, dtype = self.device, self.dtype
+        feats = x.feature_tensor
+        if feats.stride(1) != 1:
+            feats = feats.contiguous()
+        ic = x.batched_coordinates
+        perm = x.extra_attributes.get("perm") if restore_order else None
+        assert not restore_order or perm is not None, "restore_order needs the permutation that Voxels.sort records"
+        n0 = feats.shape[0]
+        lib_, status, stream = lib(), ptr(device_status(dev)), stream_ptr(dev)
+        maps = LevelMaps(ic, sparse_conv.TILE_ORDER_MIN_ROWS)
+        buffers = (ctypes.c_int64 * (2 * (self.TEMP + 20)))()
+        tables = (ctypes.c_int64 * 22)()
+        rows = (ctypes.c_int64 * 5)(n0, 0, 0, 0, 0)
+        launches = ctypes.c_int32(0)
+        joined0 = torch.empty((n0, self.joined_width[0]), dtype=dtype, device=dev)
+        identity = _identity_map(n0, dev).neighbor_table(n0)
+        buffers[0], buffers[1] = feats.data_ptr(), feats.stride(0)
+        buffers[2], buffers[3] = joined0.data_ptr(), self.joined_width[0]
+        tables[2 * self.IDENTITY] = identity.data_ptr()
+        ops, count = ctypes.addressof(self.ops), len(self.ops)
+
+        def enqueue(first, n, ws, ws_bytes):
+            check(lib_.wcn_net_run(ops + first * ctypes.sizeof(NetOp), n, ctypes.addressof(rows), ctypes.addressof(buffers),
+                                   ctypes.addressof(tables), self.dtype_code, ws, ws_bytes, ctypes.addressof(launches), status,
+                                   stream), "wcn_net_run")
+            LAUNCH_COUNTS["wcn_net_run"] += launches.value
+
+        enqueue(0, 1, None, 0)  # the stem runs while the host waits for the sizes of the coarser levels
+        if maps.finish() is None:
+            return None
+        for l in range(5):
+            rows[l] = maps.n[l]
+            tables[2 * l], tables[2 * l + 1] = maps.nbr[l].data_ptr(), ptr(maps.order[l]) or 0
+            if l < 4:
+                tables[2 * (self.CHILD + l)] = maps.child[l].data_ptr()
+        ws_bytes = query_bytes("wcn_net_workspace_bytes", ops, count, ctypes.addressof(rows), self.dtype_code)
+        total, places = -(-ws_bytes // 256) * 256, []
+        for b, level, w in self.arena:
+            places.append((b, w, total))
+            total += -(-2 * maps.n[level] * w // 256) * 256
+        arena = torch.empty(total, dtype=torch.uint8, device=dev)
+        base = arena.data_ptr()
+        for b, w, at in places:
+            buffers[2 * b], buffers[2 * b + 1] = base + at, w
+        out = torch.empty((n0, self.classes), dtype=dtype, device=dev)
+        buffers[2 * self.OUT], buffers[2 * self.OUT + 1] = out.data_ptr(), self.classes
+        if restore_order:  # sorted row j is original row perm[j]: each row of logits is written at its original place
+            dst = perm.to(torch.int32)
+            tables[2 * self.PERM] = dst.data_ptr()
+            enqueue(1, count - 2, base, ws_bytes)
+            last = NetOp.from_buffer_copy(self.ops[count - 1])
+            last.table = self.PERM
+            ops, count = ctypes.addressof(last), 1
+            enqueue(0, 1, None, 0)
+            return out
+        enqueue(1, count - 1, base, ws_bytes)
+        return x._derive(out)
 
 
 class MinkUNet18(MinkUNetBase):

@@ -1,0 +1,147 @@
+"""Coordinate pyramid and kernel maps of a natively sorted ``Voxels``, all levels at once.
+
+An addition to the reference's structures, for coordinate sets that ``Voxels.sort`` has put in Morton order: the
+coarser levels come from comparing neighbouring rows (:func:`morton_pyramid`), and the 3x3x3 maps in tile order with
+the stride-2 child tables of a whole U-Net from one launch per stage (:class:`LevelMaps`).  The row counts are written
+by the kernel into pinned memory; :meth:`PyramidBuild.finish` is the one point where the host waits, and it waits for
+the small pyramid kernels only: whatever was enqueued behind them keeps the device busy meanwhile.
+"""
+from __future__ import annotations
+
+import ctypes
+from typing import List, Optional
+
+import torch
+from torch import Tensor
+
+from ...._native import Level, check, device_status, lib, ptr, query_bytes, raise_for_status, stream_ptr
+from ..integer import IntCoords
+from .search_results import IntSearchResult
+
+PYRAMID_LEVELS = 4
+
+
+class PyramidBuild:
+    """The four stride-2 levels below a sorted coordinate set, enqueued on the current stream."""
+
+    def __init__(self, ic: IntCoords):
+        info = ic._shared["morton_info"]
+        rows = ic._shared["bcoords"]
+        dev = rows.device
+        n = rows.shape[0]
+        offsets = ic.offsets if ic.offsets.dtype == torch.int64 and ic.offsets.is_contiguous() else ic.offsets.to(torch.int64).contiguous()
+        self.ic, self.rows, self.info, self.n, self.device = ic, rows, info, n, dev
+        self.batches = len(offsets) - 1
+        self.out = torch.empty((PYRAMID_LEVELS, n, 4), dtype=torch.int32, device=dev)
+        self.first = torch.empty((PYRAMID_LEVELS, n), dtype=torch.int32, device=dev)
+        self.counts = torch.empty(24, dtype=torch.int32, device=dev)
+        self.host = torch.empty(PYRAMID_LEVELS * (self.batches + 1) + 2, dtype=torch.int64, pin_memory=True)
+        ws = torch.empty(query_bytes("wcn_pyramid_workspace_bytes", n), dtype=torch.uint8, device=dev)
+        check(lib().wcn_pyramid(ptr(rows), n, ptr(info), ptr(offsets), self.batches, PYRAMID_LEVELS, ptr(self.out),
+                                ptr(self.first), ptr(self.counts), ptr(self.host), ptr(ws), ptr(device_status(dev)),
+                                stream_ptr(dev)), "wcn_pyramid")
+        self._done = torch.cuda.Event()
+        self._done.record(torch.cuda.current_stream(dev))
+
+    def finish(self) -> Optional[List[IntCoords]]:
+        """Waits for the counts; the levels' coordinates, or None when the rows are not what the pyramid needs
+        (repeated voxels, an extent of 2^21 or more)."""
+        self._done.synchronize()
+        host = self.host.tolist()
+        nb = self.batches + 1
+        raise_for_status(host[-1], self.device)
+        if not host[-2]:
+            return None
+        levels = []
+        for l in range(PYRAMID_LEVELS):
+            offs = host[l * nb:(l + 1) * nb]
+            rows = self.out[l, :offs[-1]]
+            c = object.__new__(IntCoords)
+            c.offsets = torch.tensor(offs, dtype=torch.int64)
+            c.offsets.__dict__["_wcn_tuple"] = tuple(offs)  # the form kernel-map cache keys want
+            c.batched_tensor = rows[:, 1:]
+            c.voxel_size = c.voxel_origin = c.tensor_stride = None
+            c._shared = {"bcoords": rows, "morton_origin": self.counts[8 + 4 * l:11 + 4 * l]}
+            levels.append(c)
+        return levels
+
+
+def link_levels(ic: IntCoords, levels: List[IntCoords]) -> None:
+    """Leaves the levels where :func:`strided_coordinates` looks for them."""
+    for c in levels:
+        ic._shared[("strided", (2, 2, 2))] = c
+        ic = c
+
+
+def morton_pyramid(ic: IntCoords) -> bool:
+    """Computes and links the stride-2 levels of a natively sorted set; False when it is none (or not usable)."""
+    if ic._shared.get("morton_info") is None:
+        return False
+    levels = PyramidBuild(ic).finish()
+    if levels is None:
+        ic._shared["morton_info"] = None
+        return False
+    link_levels(ic, levels)
+    return True
+
+
+# 3x3x3 tables of at least this many rows are put in tile order.
+TILE_ORDER_ROWS = 1024
+
+
+class LevelMaps:
+    """Tables of levels 0..4: :meth:`begin` enqueues the pyramid and level 0, :meth:`finish` the other levels."""
+
+    def __init__(self, ic: IntCoords, tile_order_rows: int = TILE_ORDER_ROWS):
+        self.build = PyramidBuild(ic)
+        self.min_rows = tile_order_rows
+        n = self.build.n
+        self.n = [n]
+        self.rows = [self.build.rows]
+        self.nbr, self.order, self.child = [], [], []
+        self._bricks = []
+        self._enqueue(range(1))
+
+    def _enqueue(self, which) -> None:
+        b = self.build
+        levels = (Level * len(which))()
+        for slot, l in zip(levels, which):
+            n = self.n[l]
+            nbr = torch.empty((27, n), dtype=torch.int32, device=b.device)
+            order = torch.empty(n, dtype=torch.int32, device=b.device) if n >= self.min_rows else None
+            bricks = torch.empty(query_bytes("wcn_level_brick_bytes", n), dtype=torch.uint8, device=b.device)
+            self.nbr.append(nbr)
+            self.order.append(order)
+            self._bricks.append(bricks)
+            slot.rows, slot.n, slot.level = self.rows[l].data_ptr(), n, l
+            slot.bricks, slot.order, slot.nbr = bricks.data_ptr(), ptr(order), nbr.data_ptr()
+            if l:
+                child = torch.empty((8, n), dtype=torch.int32, device=b.device)
+                self.child.append(child)
+                slot.child, slot.first_child = child.data_ptr(), b.first[l - 1].data_ptr()
+                slot.rows_below, slot.n_below = self.rows[l - 1].data_ptr(), self.n[l - 1]
+        check(lib().wcn_level_maps(ctypes.addressof(levels), len(which), ptr(b.info), ptr(b.counts), stream_ptr(b.device)),
+              "wcn_level_maps")
+
+    def finish(self) -> Optional[List[IntCoords]]:
+        """The coordinates of levels 1..4 (None: not usable); their maps are enqueued and every level's maps left with
+        its coordinates, where layers of those geometries find them."""
+        b = self.build
+        levels = b.finish()
+        if levels is None:
+            b.ic._shared["morton_info"] = None
+            return None
+        link_levels(b.ic, levels)
+        for c in levels:
+            self.rows.append(c._shared["bcoords"])
+            self.n.append(self.rows[-1].shape[0])
+        self._enqueue(range(1, PYRAMID_LEVELS + 1))
+        self._bricks = None
+        for l, c in enumerate([b.ic] + levels):
+            if self.order[l] is not None:
+                c._shared[("kmap", (3, 3, 3), (1, 1, 1))] = IntSearchResult.from_tiled_table(self.nbr[l], self.order[l], self.n[l], 13)
+            else:
+                c._shared[("kmap", (3, 3, 3), (1, 1, 1))] = IntSearchResult.from_neighbor_table(self.nbr[l], self.n[l], None, 13)
+            if l < PYRAMID_LEVELS:
+                c._shared[("kmap", (2, 2, 2), (2, 2, 2))] = IntSearchResult.from_neighbor_table(self.child[l], self.n[l], None, None)
+        return levels

@@ -54,6 +54,25 @@ class IntSearchResult:
         self._tiled = None
         return self
 
+    @classmethod
+    def from_tiled_table(cls, tiled: Tensor, out_rows: Tensor, num_in: int,
+                         identity_map_index: Optional[int] = None) -> "IntSearchResult":
+        """A map that is known by its tile-ordered table (``tiled_neighbor_table``); the plain table is
+        made from it when something asks."""
+        self = cls.from_neighbor_table(tiled, num_in, None, identity_map_index)
+        self._nbr = None
+        self._tiled = (tiled, out_rows)
+        return self
+
+    def _plain(self) -> Tensor:
+        """The plain neighbour table of a map made dense."""
+        if self._nbr is None:
+            tiled, rows = self._tiled
+            nbr = torch.empty_like(tiled)
+            nbr[:, rows.long()] = tiled
+            self._nbr = nbr
+        return self._nbr
+
     def _compact(self):
         if self._offsets is not None:
             return
@@ -62,7 +81,7 @@ class IntSearchResult:
             fwd = self._forward
             self._in_maps, self._out_maps, self._offsets = fwd.out_maps, fwd.in_maps, fwd.offsets
             return
-        nbr, K, M = self._nbr, self._num_offsets, self._num_out
+        nbr, K, M = self._plain(), self._num_offsets, self._num_out
         dev = nbr.device
         ws = self._workspace
         if ws is None:  # searched without hit counts: count now
@@ -111,14 +130,18 @@ class IntSearchResult:
         if self._nbr is not None:
             assert self._num_out == num_out, f"kernel map was built for {self._num_out} outputs, got {num_out}"
             return self._nbr
+        if self._forward is None and self._tiled is not None:
+            assert self._num_out == num_out, f"kernel map was built for {self._num_out} outputs, got {num_out}"
+            return self._plain()
         fwd = self._forward
-        if fwd is not None and fwd._nbr is not None:  # a transposed view whose table has not been asked for yet
+        if fwd is not None and (fwd._nbr is not None or fwd._tiled is not None):  # a transposed view whose table has not been asked for yet
             assert self._num_out == num_out, f"kernel map was built for {self._num_out} outputs, got {num_out}"
             nbr_t = self._kept().get("nbr")
             if nbr_t is None:
-                dev = fwd._nbr.device
+                table = fwd._plain()
+                dev = table.device
                 nbr_t = torch.empty((self._num_offsets, num_out), dtype=torch.int32, device=dev)
-                check(lib().wcn_nbr_transpose(ptr(fwd._nbr), fwd._num_offsets, fwd._num_out, num_out, ptr(nbr_t),
+                check(lib().wcn_nbr_transpose(ptr(table), fwd._num_offsets, fwd._num_out, num_out, ptr(nbr_t),
                                               stream_ptr(dev)), "wcn_nbr_transpose")
                 self._kept()["nbr"] = nbr_t
             self._nbr = nbr_t
@@ -170,7 +193,8 @@ class IntSearchResult:
         warpconvnet/nn/functional/sparse_conv.py:1934-1938)."""
         if self._forward is not None and (num_in is None or int(num_in) == self._forward._num_out):
             return self._forward  # exchanging a transposed view back gives the map it came from
-        if self._nbr is not None and (num_in or self._num_in) is not None:
+        if (self._nbr is not None or (self._forward is None and self._tiled is not None)) \
+                and (num_in or self._num_in) is not None:
             # Both forms of the view come from this map when first asked for: the compact one by exchanging
             # in and out, the dense one by transposing the table (a layer that runs from the input side,
             # sparse_conv_rows_fused, needs neither: it reads this map's own table).
@@ -237,4 +261,6 @@ class IntSearchResult:
     def device(self):
         if self._nbr is not None:
             return self._nbr.device
+        if self._tiled is not None:
+            return self._tiled[0].device
         return self._in_maps.device if self._in_maps is not None else self._forward.device

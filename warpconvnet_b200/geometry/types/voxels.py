@@ -8,6 +8,7 @@ from typing import List, Optional, Tuple, Union
 import torch
 from torch import Tensor
 
+from ..._native import check, device_status, lib, ptr, query_bytes, stream_ptr
 from ..base.geometry import Geometry
 from ..coords.integer import IntCoords
 from ..coords.ops.batch_index import offsets_from_batch_index
@@ -79,6 +80,10 @@ class Voxels(Geometry):
         if ordering == self.ordering:
             return self
         assert isinstance(ordering, POINT_ORDERING), f"Invalid ordering: {ordering}"
+        if ordering == POINT_ORDERING.MORTON_XYZ and type(self) is Voxels:
+            done = self._sort_native()
+            if done is not None:
+                return done
         origin = None
         coords = self.coordinate_tensor
         if ordering == POINT_ORDERING.MORTON_XYZ and coords.is_cuda and coords.shape[0] > 0 and coords.shape[1] == 3:
@@ -96,6 +101,44 @@ class Voxels(Geometry):
             sorted_coords.morton_origin = origin
         return self.__class__(batched_coordinates=sorted_coords,
                               batched_features=CatFeatures(self.feature_tensor[res.perm], self.offsets), **kwargs)
+
+    def _sort_native(self) -> Optional["Voxels"]:
+        """The Morton sort in one launch (int32 coordinates on a CUDA device, at most 255 batch items), or None."""
+        coords, n = self.coordinate_tensor, self.coordinate_tensor.shape[0]
+        if not coords.is_cuda or coords.dtype != torch.int32 or n == 0 or coords.shape[1] != 3 or len(self.offsets) > 256:
+            return None
+        dev = coords.device
+        coords = coords.contiguous()
+        offsets = self.offsets
+        off64 = offsets if offsets.dtype == torch.int64 and offsets.is_contiguous() else offsets.to(torch.int64).contiguous()
+        feats = self.feature_tensor
+        row_bytes = feats.shape[1] * feats.element_size()
+        # narrow rows ride along; wide ones (and ones with a gradient) are gathered by torch
+        inline = (not (torch.is_grad_enabled() and feats.requires_grad) and feats.is_cuda and feats.is_contiguous()
+                  and 0 < row_bytes <= 32 and row_bytes % 2 == 0)
+        sorted_feats = torch.empty_like(feats) if inline else None
+        codes = torch.empty(n, dtype=torch.int64, device=dev)
+        perm = torch.empty(n, dtype=torch.int64, device=dev)
+        rows = torch.empty((n, 4), dtype=torch.int32, device=dev)
+        info = torch.empty(8, dtype=torch.int32, device=dev)
+        ws = torch.empty(query_bytes("wcn_morton_sort_workspace_bytes", n), dtype=torch.uint8, device=dev)
+        check(lib().wcn_morton_sort(ptr(coords), n, ptr(off64), len(off64) - 1, ptr(codes), ptr(perm), ptr(rows), ptr(info),
+                                    ptr(feats) if inline else None, ptr(sorted_feats), row_bytes if inline else 0, ptr(ws),
+                                    ptr(device_status(dev)), stream_ptr(dev)), "wcn_morton_sort")
+        new = object.__new__(Voxels)
+        ic = object.__new__(IntCoords)
+        ic.offsets, ic.batched_tensor, ic.tensor_stride = offsets, rows[:, 1:], self.tensor_stride
+        ic.voxel_size = ic.voxel_origin = None
+        ic._shared = {"bcoords": rows, "morton_origin": info[:3], "morton_info": info}
+        new.batched_coordinates = ic
+        f = object.__new__(CatFeatures)
+        f.batched_tensor, f.offsets = (sorted_feats if inline else feats[perm]), offsets
+        new.batched_features = f
+        attrs = self.extra_attributes
+        attrs.update(ordering=POINT_ORDERING.MORTON_XYZ, code=codes, perm=perm)  # sorted = original[perm]
+        attrs.pop("_cache", None)  # cached maps index the old row order
+        new._extra_attributes = attrs
+        return new
 
     def unique(self) -> "Voxels":
         """One voxel per distinct coordinate, keeping its first occurrence (voxels.py:269-276)."""

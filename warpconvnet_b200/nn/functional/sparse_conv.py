@@ -33,6 +33,7 @@ from ...geometry.coords.integer import IntCoords
 from ...geometry.coords.ops.serialization import POINT_ORDERING, encode
 from ...geometry.coords.ops.expand import expand_coords
 from ...geometry.coords.ops.stride import stride_coords
+from ...geometry.coords.search.level_maps import morton_pyramid
 from ...geometry.coords.search.cache import IntSearchCache, IntSearchCacheKey
 from ...geometry.coords.search.search_results import IntSearchResult
 from ...geometry.coords.search.torch_discrete import generate_kernel_map
@@ -577,6 +578,8 @@ def generate_output_coords_and_kernel_map(input_sparse_tensor: Voxels, kernel_si
         fwd = None
         if cache is not None:
             fwd = cache.get(key_for(False, out_offsets, input_sparse_tensor.offsets))
+        if fwd is None and output_spatially_sparse_tensor is not None:
+            fwd = _level_map(output_spatially_sparse_tensor, kernel_size, kernel_dilation, stride, in_coords)
         if fwd is None:
             # forward map: table on the (fine) output coordinates, (coarse) inputs * stride as queries
             fwd = _generate_kernel_map_nd(out_coords, in_coords, stride, kernel_size, kernel_dilation,
@@ -591,14 +594,27 @@ def generate_output_coords_and_kernel_map(input_sparse_tensor: Voxels, kernel_si
                                 and parent is not None
                                 and parent._shared is input_sparse_tensor.batched_coordinates._shared)
     else:
-        kernel_map = _generate_kernel_map_nd(in_coords, out_coords, stride, kernel_size, kernel_dilation,
-                                             hashtable=_cached_table(input_sparse_tensor, in_coords),
-                                             bricks=_cached_bricks(input_sparse_tensor, in_coords))
+        kernel_map = _level_map(input_sparse_tensor, kernel_size, kernel_dilation, stride, out_coords)
+        if kernel_map is None:
+            kernel_map = _generate_kernel_map_nd(in_coords, out_coords, stride, kernel_size, kernel_dilation,
+                                                 hashtable=_cached_table(input_sparse_tensor, in_coords),
+                                                 bricks=_cached_bricks(input_sparse_tensor, in_coords))
 
     if input_sparse_tensor.cache is None:
         input_sparse_tensor._extra_attributes["_cache"] = IntSearchCache()
     input_sparse_tensor.cache.put(key, kernel_map)
     return out_coords, out_offsets, kernel_map
+
+
+def _level_map(fine: Voxels, kernel_size, kernel_dilation, stride, coarse_rows: Tensor) -> Optional[IntSearchResult]:
+    """The map of this window that :class:`LevelMaps` left with the coordinates of ``fine`` (from ``fine`` to its own
+    rows or to its strided rows), or None."""
+    shared = fine.batched_coordinates._shared
+    km = shared.get(("kmap", tuple(kernel_size), tuple(stride)))
+    if km is None or any(d != 1 for d in kernel_dilation):
+        return None
+    rows = shared["bcoords"] if all(s == 1 for s in stride) else shared[("strided", tuple(stride))]._shared["bcoords"]
+    return km if rows.data_ptr() == coarse_rows.data_ptr() and rows.shape == coarse_rows.shape else None
 
 
 def strided_coordinates(coords: IntCoords, stride: Tuple[int, ...]) -> IntCoords:
@@ -609,6 +625,8 @@ def strided_coordinates(coords: IntCoords, stride: Tuple[int, ...]) -> IntCoords
     stride = tuple(int(s) for s in stride)
     key = ("strided", stride)
     hit = coords._shared.get(key)
+    if hit is None and stride == (2, 2, 2) and morton_pyramid(coords):
+        hit = coords._shared[key]
     if hit is None:
         bc = coords.batch_indexed_coordinates
         if bc.dtype != torch.int32:
@@ -656,6 +674,8 @@ def prefetch_strided_coordinates(voxels: Voxels, strides) -> List[IntCoords]:
     nd = voxels.num_spatial_dims
     level = voxels.batched_coordinates
     steps = [ntuple(s, ndim=nd) for s in strides]
+    if steps and steps[0] == (2, 2, 2) and ("strided", steps[0]) not in level._shared:
+        morton_pyramid(level)
     bc = level.batch_indexed_coordinates
     if (nd == 3 and bc.is_cuda and bc.dtype == torch.int32 and 0 < bc.shape[0] <= PYRAMID_ONE_SYNC_MAX_ROWS
             and steps and ("strided", steps[0]) not in level._shared):
