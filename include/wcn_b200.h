@@ -321,11 +321,9 @@ int wcn_conv_packed_weight_bytes(int algo, int32_t num_offsets, int32_t c_in, in
 int wcn_conv_pack_weight(int algo, const void* weight, int32_t num_offsets, int32_t c_in,
                          int32_t c_out, int dtype, void* packed, void* stream);
 
-/* Bytes of `workspace` wcn_conv_fwd needs for this problem on the current device (0: none).  Only
- * the tensor-core kernel uses one, when it divides the kernel offsets of a row block among several
- * CTAs (see split_k below): S * num_out * c_out fp32 partial sums.
- * Replaces the cudaMalloc inside the reference's split-K launcher
- * (warpconvnet/csrc/implicit_gemm_split_k.cu:254-258). */
+/* Bytes of `workspace` wcn_conv_fwd needs for this problem: 0 in this version (the slices of split_k are added through
+ * distributed shared memory), so NULL may be passed.
+ * (warpconvnet/csrc/implicit_gemm_split_k.cu:254-258 allocates its partial sums inside the call.) */
 int wcn_conv_workspace_bytes(int algo, int64_t num_out, int32_t num_offsets, int32_t c_in, int32_t c_out,
                              int dtype, int out_dtype, int32_t split_k, int64_t* bytes);
 
@@ -347,14 +345,12 @@ int wcn_conv_workspace_bytes(int algo, int64_t num_out, int32_t num_offsets, int
  * algo WCN_CONV_TCGEN05 needs dtype f16/bf16, c_in % 32 == 0, c_out % 16 == 0, 16 <= c_out <= 256
  * and `packed_weight` from wcn_conv_pack_weight; WCN_CONV_AUTO picks it when those hold and
  * packed_weight is not NULL, else the SIMT kernel.
- * split_k: the tensor-core kernel may divide the kernel offsets of a 128-row block among S CTAs
- * (slice s owns offsets [s*K/S, (s+1)*K/S)), each leaving fp32 partial sums in `workspace`, which
- * a second kernel adds in slice order before the epilogue: for problems with fewer row blocks
- * than multiprocessors.  0 = the library decides, 1 = never, 2..16 = that many slices; a negative
- * value divides the OUTPUT COLUMNS into -split_k blocks instead (a tuning aid).  `workspace` must
- * hold wcn_conv_workspace_bytes(...) for the same arguments (NULL / 0 when that is 0).  Results
- * are the same bits on every run for a given S; different S round differently (fp32 sums are
- * grouped by slice).
+ * split_k: the tensor-core kernel may divide the kernel offsets of a 128-row block among the S CTAs of a cluster (slice s
+ * owns the offsets k with k % S == s), whose fp32 sums are added in slice order before the epilogue: for problems with
+ * fewer row blocks than multiprocessors.  0 = the library decides, 1 = never, 2.. = that many slices (at most 8); a
+ * negative value divides the OUTPUT COLUMNS into -split_k blocks instead (a tuning aid).  `workspace` must hold
+ * wcn_conv_workspace_bytes(...) for the same arguments (NULL / 0 when that is 0).  Results are the same bits on every run
+ * for a given S; different S round differently (fp32 sums are grouped by slice).
  * Replaces implicit_gemm (warpconvnet/csrc/warpconvnet_pybind.cpp:732-837,
  * warpconvnet/csrc/implicit_gemm.cu:44-267) and cutlass_gemm_AD_gather_scatter with its
  * split_k_slices argument (warpconvnet_pybind.cpp:396-509,
@@ -511,14 +507,11 @@ typedef struct {
 typedef struct { void* data; int64_t ld; } wcn_net_buffer;                       /* rows of ld elements */
 typedef struct { const int32_t* nbr; const int32_t* out_rows; } wcn_net_table;
 
-/* Enqueues the convolutions in order, all tensors of one 16-bit dtype.  `rows` are the row counts per level;
- * `workspace` of wcn_net_workspace_bytes serves the offset slices of every op in turn.  *launches receives the kernels
- * enqueued.  The reference runs the same layers from Python, one module at a time
+/* Enqueues the convolutions in order, all tensors of one 16-bit dtype; `rows` are the row counts per level.  Weights,
+ * scales and tables must have been written before the call (its launches overlap and read them early).  The reference runs the same layers from Python, one module at a time
  * (warpconvnet/nn/modules/sequential.py:14-62, examples/mink_unet.py:212-413). */
-int wcn_net_workspace_bytes(const wcn_net_op* ops, int32_t num_ops, const int64_t* rows, int dtype, int64_t* bytes);
 int wcn_net_run(const wcn_net_op* ops, int32_t num_ops, const int64_t* rows, const wcn_net_buffer* buffers,
-                const wcn_net_table* tables, int dtype, void* workspace, int64_t workspace_bytes, int32_t* launches,
-                int32_t* dev_status, void* stream);
+                const wcn_net_table* tables, int dtype, int32_t* dev_status, void* stream);
 
 /* ------------------------------------------------------------------ self test */
 

@@ -29,18 +29,18 @@ int wcn_conv_fp32_fwd(const void* feats, int64_t num_in, int64_t feats_ld, const
 // conv_tcgen05.cu
 bool wcn_conv_tcgen05_supported(int K, int c_in, int c_out, int dtype, int out_dtype);
 int64_t wcn_conv_tcgen05_packed_bytes(int K, int c_in, int c_out);
-int64_t wcn_conv_tcgen05_workspace_bytes(int64_t M, int K, int c_in, int c_out, int split_k);
 int wcn_conv_tcgen05_pack(const void* weight, int K, int c_in, int c_out, void* packed, cudaStream_t st);
 int wcn_conv_tcgen05_fwd(const void* feats, int64_t num_in, int64_t feats_ld, const void* packed, const int32_t* nbr,
                          const int32_t* out_rows, int64_t M, int K, int c_in, int c_out, int dtype,
                          const float* scale, const float* shift, const void* residual, int64_t residual_ld, int relu,
-                         void* out, int64_t out_ld, int out_dtype, int split_k, void* workspace,
-                         int64_t workspace_bytes, int32_t* dev_status, cudaStream_t st);
+                         void* out, int64_t out_ld, int out_dtype, int split_k, int32_t* dev_status, cudaStream_t st);
 // conv_wgrad_tcgen05.cu
 bool wcn_conv_wgrad_tcgen05_supported(int K, int c_in, int c_out, int dtype);
 int wcn_conv_wgrad_tcgen05(const void* feats, int64_t num_in, const void* grad_out, const int32_t* nbr,
                            const int32_t* out_rows, const uint32_t* tile_masks, int64_t M, int K, int c_in, int c_out, int dtype,
                            float* grad_weight, int32_t* dev_status, cudaStream_t st);
+
+thread_local bool wcn_overlap_launches = false;
 
 extern "C" int wcn_version(void) { return 100; }
 
@@ -87,9 +87,8 @@ static bool conv_takes_tcgen05(int algo, bool tc_ok, const void* packed_weight, 
 extern "C" int wcn_conv_workspace_bytes(int algo, int64_t num_out, int32_t num_offsets, int32_t c_in, int32_t c_out,
                                         int dtype, int out_dtype, int32_t split_k, int64_t* bytes) {
   if (!bytes || num_out < 0 || num_offsets <= 0 || c_in <= 0 || c_out <= 0) return WCN_ERR_INVALID_PARAMETERS;
-  *bytes = 0;
-  if (algo == WCN_CONV_SIMT || !wcn_conv_tcgen05_supported(num_offsets, c_in, c_out, dtype, out_dtype)) return WCN_OK;
-  *bytes = wcn_conv_tcgen05_workspace_bytes(num_out, num_offsets, c_in, c_out, split_k);
+  *bytes = 0;  // no kernel of this version keeps partial sums in global memory
+  (void)algo; (void)dtype; (void)out_dtype; (void)split_k;
   return WCN_OK;
 }
 
@@ -109,13 +108,14 @@ extern "C" int wcn_conv_fwd(int algo, const void* feats, int64_t num_in, int64_t
   if (feats_ld < c_in || out_ld < c_out || residual_ld < c_out) return WCN_ERR_INVALID_PARAMETERS;
   if (num_out == 0) return WCN_OK;
   if (!nbr || !out || (num_in > 0 && !feats)) return WCN_ERR_INVALID_PARAMETERS;
+  (void)workspace; (void)workspace_bytes;
   cudaStream_t st = wcn_stream(stream);
   const bool tc_ok = wcn_conv_tcgen05_supported(num_offsets, c_in, c_out, dtype, out_dtype);
   if (conv_takes_tcgen05(algo, tc_ok, packed_weight, dev_status, num_in)) {
     if (!tc_ok) return WCN_ERR_UNSUPPORTED_CONFIG;
     return wcn_conv_tcgen05_fwd(feats, num_in, feats_ld, packed_weight, nbr, out_rows, num_out, num_offsets, c_in,
                                 c_out, dtype, scale, shift, residual, residual_ld, relu, out, out_ld, out_dtype,
-                                split_k, workspace, workspace_bytes, dev_status, st);
+                                split_k, dev_status, st);
   }
   if (algo != WCN_CONV_SIMT && algo != WCN_CONV_AUTO) return WCN_ERR_INVALID_PARAMETERS;
   if (!weight) return WCN_ERR_INVALID_PARAMETERS;

@@ -173,7 +173,9 @@ conv_rows_tcgen05_kernel(const __grid_constant__ CUtensorMap feats_map, const Ro
 
   if (tid == 0) ctl->skip = *(volatile int32_t*)p.dev_status;
   __syncthreads();
+  launch_dependents();
   if (ctl->skip == (int)WCN_ERR_WAIT_EXPIRED) {
+    wait_for_primary();
     // A kernel on this status word gave up earlier: compute nothing and mark this launch's rows.
     const TO nan = wcn_from_float<TO>(__int_as_float(0x7FC00000));
     for (UnitCursor c = first; c.chunk < p.nchunks; c.advance(grid, tiles)) {
@@ -221,6 +223,7 @@ conv_rows_tcgen05_kernel(const __grid_constant__ CUtensorMap feats_map, const Ro
     if (lane == 0) {
       Ring ra{0, 0, p.stages};
       int bbuf = 0, bphase = 0, cur_chunk = -1;
+      bool waited = false;
       int issued = 0;  // row-tile copies issued (for the drain below)
       for (UnitCursor c = first; c.chunk < p.nchunks && ok; c.advance(grid, tiles)) {
         if (c.chunk != cur_chunk) {
@@ -234,6 +237,10 @@ conv_rows_tcgen05_kernel(const __grid_constant__ CUtensorMap feats_map, const Ro
             for (int o = 0; o < qc; ++o)
               bulk_copy_g2s(b_base + (uint32_t)(bbuf * B_BUF + s * B_SLICE + o * B_TILE),
                             p.wpacked + ((int64_t)(k0 + o) * KB + s) * B_TILE, (uint32_t)B_TILE, fullb);
+        }
+        if (!waited) {  // the feature rows are the previous launch's; the weights were there before
+          wait_for_primary();
+          waited = true;
         }
         const int row0 = c.tile * BLOCK_M;
         for (int s = 0; s < KB; ++s) {
@@ -301,6 +308,9 @@ conv_rows_tcgen05_kernel(const __grid_constant__ CUtensorMap feats_map, const Ro
     // TMEM lanes 32*(warp % 4).. belong to this warp.  The two warps of a lane quarter take
     // alternate units: what an epilogue pays per unit besides the data (barrier round trip, table
     // lookup, loop control) then overlaps between the two, and four accumulator sets keep both fed.
+    wait_for_primary();
+    // (a launch that overlaps the one before it may have started before that one failed)
+    const bool poison = *(volatile const int32_t*)p.dev_status == (int)WCN_ERR_WAIT_EXPIRED;
     const int ew = warp - EPI_WARP0, quarter = warp & 3, half = ew >> 2;
     const bool affine = p.scale != nullptr || p.shift != nullptr;
     const int pieces = p.c_out >> 4;
@@ -318,6 +328,10 @@ conv_rows_tcgen05_kernel(const __grid_constant__ CUtensorMap feats_map, const Ro
       if (p.relu) {
 #pragma unroll
         for (int i = 0; i < 16; ++i) y[i] = fmaxf(y[i], 0.f);
+      }
+      if (poison) {
+#pragma unroll
+        for (int i = 0; i < 16; ++i) y[i] = __int_as_float(0x7FC00000);
       }
       store_piece<TO>(orow, c0, y, p.c_store, p.vec);
     };
@@ -444,8 +458,7 @@ int launch_rows(const CUtensorMap& map, const RowsParams& p, size_t smem, unsign
       return WCN_ERR_EXECUTION;
     configured[dev] = true;
   }
-  kern<<<grid, THREADS, smem, st>>>(map, p);
-  return cudaGetLastError() == cudaSuccess ? WCN_OK : WCN_ERR_EXECUTION;
+  return wcn_launch(kern, dim3(grid), dim3(THREADS), smem, st, 1, map, p);
 }
 
 }  // namespace

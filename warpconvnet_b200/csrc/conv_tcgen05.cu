@@ -21,11 +21,15 @@
 //    (folded BatchNorm or bias), residual add and ReLU, convert and store every
 //    output row exactly once.  No atomics, bit-reproducible.
 //
-// Problems with fewer 128-row tiles than multiprocessors divide the kernel offsets of a tile
-// among S CTAs ("split-K over kernel offsets": slice s owns the offsets [s*K/S, (s+1)*K/S)).
-// Each CTA then leaves its fp32 accumulators in a caller-supplied workspace [S][M][C_out] and a
-// second kernel adds the S slices in slice order and runs the epilogue; still no atomics and the
-// same bits on every run.
+// Problems with fewer 128-row tiles than multiprocessors divide the kernel offsets of a tile among the S CTAs of a
+// cluster ("split-K over kernel offsets": slice s owns the offsets k with k % S == s, which deals the frequent central
+// ones evenly).  Each CTA leaves its fp32 accumulators in its shared memory, where the ring was, and adds 1 / S of the
+// rows over all slices through distributed shared memory, in slice order, with the epilogue behind it: no workspace, no
+// second kernel, no atomics and the same bits on every run.
+//
+// Launches of one network overlap (programmatic dependent launch): everything up to the first read of a feature row -
+// barriers, tensor memory, neighbour tables, weight slices, all written before the network's first launch - runs while
+// the previous layer finishes.
 //
 // Every wait is bounded: a wait that runs out stores WCN_ERR_WAIT_EXPIRED in the
 // device status word, the other waits notice it and the CTA leaves through the
@@ -39,6 +43,7 @@ constexpr int BLOCK_M = 128;
 constexpr int MAX_G = 2;              // sub-tiles per supertile (one per MMA issuer)
 constexpr int MAX_RING = 12;          // slots per ring
 constexpr int MAX_OFFSETS = 27;
+constexpr int MAX_SLICES = 8;         // CTAs of a (portable) cluster
 constexpr int EPI_THREADS = 128;      // warps 0..3: TMEM lane quarter = warp index
 constexpr int IDX_THREADS = 128;      // warps 4..7: neighbour-table staging
 constexpr int GATHER_WARP0 = 8;       // warps 8..15: row gathers
@@ -50,7 +55,7 @@ constexpr int THREADS = 608;
 
 struct ConvTcParams {
   const char* feats;
-  bool wide_out, wide_partial, wide_res;   // rows of `out` / the slice workspace / `residual` start on 32-byte boundaries
+  bool wide_out, wide_res;   // rows of `out` / `residual` start on 32-byte boundaries
   const char* wpacked;
   const int32_t* nbr;
   const int32_t* out_rows;  // slot -> output row, or null for the identity
@@ -72,16 +77,29 @@ struct ConvTcParams {
   int kbc;          // channel slices per ring slot (a slot holds kbc K-major tiles side by side)
   int64_t supertiles;
   int S;            // offset slices per supertile (split-K over kernel offsets); 1 = none
-  int64_t units;    // supertiles * S work units, walked by the persistent CTAs
-  float* partial;   // [S][M][c_out] fp32 accumulators of the slices (S > 1)
+  int64_t units;    // supertiles * S work units, walked by the persistent CTAs (S > 1: one each)
 };
 
-// Offsets of slice s of S: bits [s*K/S, (s+1)*K/S).
-__device__ __forceinline__ uint32_t slice_mask(int s, int S, int K) {
+// Offsets of slice s of S: the k with k % S == s.
+__device__ __forceinline__ uint32_t slice_mask(int s, int S) {
   if (S <= 1) return 0xFFFFFFFFu;
-  const int lo = (s * K) / S, hi = ((s + 1) * K) / S;
-  const uint32_t upto_hi = hi >= 32 ? 0xFFFFFFFFu : ((1u << hi) - 1u);
-  return upto_hi & ~((1u << lo) - 1u);
+  uint32_t m = 0;
+  for (int k = s; k < 32; k += S) m |= 1u << k;
+  return m;
+}
+
+__device__ __forceinline__ void cluster_meet() {
+  asm volatile("barrier.cluster.arrive.release;\n\tbarrier.cluster.wait.acquire;" ::: "memory");
+}
+__device__ __forceinline__ float4 ld_cluster(uint32_t addr, uint32_t rank) {
+  float4 v;
+  asm volatile(
+      "{\n\t.reg .b32 r;\n\tmapa.shared::cluster.u32 r, %4, %5;\n\t"
+      "ld.shared::cluster.v4.f32 {%0, %1, %2, %3}, [r];\n\t}"
+      : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w)
+      : "r"(addr), "r"(rank)
+      : "memory");
+  return v;
 }
 
 // 32 bytes in one request: a whole sector per lane.  Every thread of the epilogue writes its own row,
@@ -191,7 +209,8 @@ struct Control {
   uint32_t mask_acc[2][MAX_G];    // index warps' scratch while building the masks
   uint32_t tmem_holder;
   int skip;
-  float sc[256], sh[256];         // this CTA's columns of the epilogue scale / shift (1 / 0 when absent)
+  int failed;                     // S > 1: the status word once every CTA of the cluster is done
+  __align__(16) float sc[256], sh[256];         // this CTA's columns of the epilogue scale / shift (1 / 0 when absent)
 };
 
 // ------------------------------------------------------------------ kernel
@@ -226,10 +245,13 @@ conv_tcgen05_kernel(const ConvTcParams p) {
 
   if (tid == 0) ctl->skip = *(volatile int32_t*)p.dev_status;  // an earlier launch on this status word failed
   __syncthreads();
+  launch_dependents();
+  bool ok = true;
   if (ctl->skip == (int)WCN_ERR_WAIT_EXPIRED) {
     // Nothing is computed after a kernel on this status word gave up.  The rows this CTA would have
-    // produced are filled with NaN so that the failure cannot pass for data (with offset slices
-    // the second kernel does the same).
+    // produced are filled with NaN so that the failure cannot pass for data (the CTAs of a cluster go on to the
+    // meeting points at the end, which do the same).
+    wait_for_primary();
     if (p.S == 1) {
       const TO nan = wcn_from_float<TO>(__int_as_float(0x7FC00000));
       for (int64_t st = blockIdx.x; st < p.supertiles; st += gridDim.x) {
@@ -241,8 +263,9 @@ conv_tcgen05_kernel(const ConvTcParams p) {
           reinterpret_cast<TO*>(p.out)[m * p.out_ld + n0 + (int)(i % BN)] = nan;
         }
       }
+      return;
     }
-    return;
+    ok = false;  // no role does any work
   }
 
   if (tid == 0) {
@@ -269,7 +292,6 @@ conv_tcgen05_kernel(const ConvTcParams p) {
   tc_fence_after();
   const uint32_t tmem_base = ctl->tmem_holder;
 
-  bool ok = true;
   if (warp >= 4 && warp < GATHER_WARP0) {
     // ================================================================ index warps
     // Stage the neighbour table of a supertile (one supertile ahead of the copies):
@@ -283,7 +305,7 @@ conv_tcgen05_kernel(const ConvTcParams p) {
     bool bad = false;
     for (int64_t wu = blockIdx.x; wu < p.units && ok; wu += gridDim.x) {
       const int64_t st = p.S > 1 ? wu / p.S : wu;
-      const uint32_t kmask = slice_mask((int)(wu - st * p.S), p.S, K);
+      const uint32_t kmask = slice_mask((int)(wu - st * p.S), p.S);
       const int64_t m0 = st * G * BLOCK_M;
       if (!mbar_wait(bar(&ctl->info_empty[ib]), iphase ^ 1, p.dev_status)) { ok = false; break; }
       int32_t* dst = rows_idx + ib * IDX_INTS;
@@ -375,6 +397,7 @@ conv_tcgen05_kernel(const ConvTcParams p) {
     __syncwarp();
   } else if (warp >= GATHER_WARP0 && warp < MMA_WARP) {
     // ================================================================ gather warps
+    wait_for_primary();  // the feature rows are the previous launch's
     const int gwarp = warp - GATHER_WARP0;
     constexpr int ROWS_PER_WARP = BLOCK_M / (GATHER_THREADS / 32);  // 16
     constexpr int NJ = ROWS_PER_WARP / RPI;                          // copy instructions per warp per A slot
@@ -567,6 +590,9 @@ conv_tcgen05_kernel(const ConvTcParams p) {
     __syncwarp();
   } else {
     // ================================================================ epilogue (warps 0..3)
+    wait_for_primary();
+    // (a launch that overlaps the one before it may have started before that one failed)
+    const bool poison = *(volatile const int32_t*)p.dev_status == (int)WCN_ERR_WAIT_EXPIRED;
     int ib = 0, iphase = 0, ab = 0, aphase = 0;
     const bool affine = p.scale != nullptr || p.shift != nullptr;
     // One 16-column piece of this thread's row: affine, residual, ReLU, convert, store.
@@ -592,9 +618,13 @@ conv_tcgen05_kernel(const ConvTcParams p) {
 #pragma unroll
         for (int i = 0; i < 16; ++i) y[i] = fmaxf(y[i], 0.f);
       }
+      if (poison) {
+#pragma unroll
+        for (int i = 0; i < 16; ++i) y[i] = __int_as_float(0x7FC00000);
+      }
       OutVec<TO>::store(orow + c0, y, p.wide_out);
     };
-    const bool sliced = p.S > 1;  // leave raw fp32 sums for the reduction kernel instead of finishing rows
+    const bool sliced = p.S > 1;  // leave raw fp32 sums in shared memory instead of finishing rows
     // This thread's output rows in the two sub-tiles of a unit.  With rows in tile order they come from
     // `out_rows`, and a load issued when its value is needed costs the epilogue a full memory latency per
     // sub-tile (the gather keeps the memory system busy): the rows of the next unit are read while this one
@@ -609,7 +639,7 @@ conv_tcgen05_kernel(const ConvTcParams p) {
     };
     int32_t next_rows[MAX_G];
     if ((int64_t)blockIdx.x < p.units) unit_rows(blockIdx.x, next_rows);
-    for (int64_t wu = blockIdx.x; wu < p.units; wu += gridDim.x) {
+    for (int64_t wu = blockIdx.x; wu < p.units && ok; wu += gridDim.x) {
       const int64_t st = sliced ? wu / p.S : wu;
       int32_t rows[MAX_G];
 #pragma unroll
@@ -636,8 +666,8 @@ conv_tcgen05_kernel(const ConvTcParams p) {
         const uint32_t trow = tmem_base + ((uint32_t)(warp * 32) << 16) + (uint32_t)((ab * G + g) * p.cols);
         TO* orow = reinterpret_cast<TO*>(p.out) + m * p.out_ld + n0;
         const TO* rrow = p.residual ? reinterpret_cast<const TO*>(p.residual) + m * p.res_ld + n0 : nullptr;
-        // slice wu % S of this row block: [S][M][c_out] fp32, rows in table order (a slice owns all columns)
-        float* prow = sliced ? p.partial + (((wu - st * p.S) * p.M + slot) * p.c_out) : nullptr;
+        // this slice's sums of the row, where the ring was (every slot has been consumed)
+        float* prow = reinterpret_cast<float*>(gen) + tid * (BN + 4);
 #pragma unroll 1
         for (int c0 = 0; c0 < BN; c0 += 32) {  // two TMEM loads in flight per wait (BN is a multiple of 16)
           const bool two = c0 + 16 < BN;
@@ -653,9 +683,12 @@ conv_tcgen05_kernel(const ConvTcParams p) {
 #pragma unroll
             for (int i = 0; i < 16; ++i) y0[i] = y1[i] = 0.f;
           }
-          if (live && sliced) {
-            OutVec<float>::store(prow + c0, y0, p.wide_partial);
-            if (two) OutVec<float>::store(prow + c0 + 16, y1, p.wide_partial);
+          if (sliced) {
+#pragma unroll
+            for (int q = 0; q < 4; ++q) {
+              *reinterpret_cast<float4*>(prow + c0 + 4 * q) = make_float4(y0[4 * q], y0[4 * q + 1], y0[4 * q + 2], y0[4 * q + 3]);
+              if (two) *reinterpret_cast<float4*>(prow + c0 + 16 + 4 * q) = make_float4(y1[4 * q], y1[4 * q + 1], y1[4 * q + 2], y1[4 * q + 3]);
+            }
           } else if (live) {
             finish16(y0, c0, orow, rrow);
             if (two) finish16(y1, c0 + 16, orow, rrow);
@@ -666,6 +699,49 @@ conv_tcgen05_kernel(const ConvTcParams p) {
       mbar_arrive(bar(&ctl->acc_empty[ab]));   // accumulator set may be overwritten
       if (++ab == NBUF) { ab = 0; aphase ^= 1; }
     }
+  }
+  if (p.S > 1) {
+    // ================================================================ the cluster adds its slices
+    __syncwarp();
+    cluster_meet();  // every slice's sums are in its CTA's shared memory
+    if (tid == 0) ctl->failed = *(volatile const int32_t*)p.dev_status == (int)WCN_ERR_WAIT_EXPIRED;
+    __syncthreads();
+    const int64_t st = blockIdx.x / p.S;
+    const int rank = (int)(blockIdx.x - st * p.S), per_row = BN / 4;
+    const int r0 = rank * BLOCK_M / p.S, r1 = (rank + 1) * BLOCK_M / p.S;
+    for (int i = tid; i < (r1 - r0) * per_row; i += THREADS) {
+      const int r = r0 + i / per_row, c = (i % per_row) * 4;
+      const int64_t slot = st * BLOCK_M + r;
+      if (slot >= p.M) break;  // rows ascend with i
+      const int64_t m = p.out_rows ? (int64_t)__ldg(&p.out_rows[slot]) : slot;
+      const uint32_t at = base + (uint32_t)(r * (BN + 4) + c) * 4u;
+      float4 v[MAX_SLICES];
+#pragma unroll
+      for (int s = 0; s < MAX_SLICES; ++s)
+        if (s < p.S) v[s] = ld_cluster(at, (uint32_t)s);
+      float y[4] = {v[0].x, v[0].y, v[0].z, v[0].w};
+#pragma unroll
+      for (int s = 1; s < MAX_SLICES; ++s) {
+        if (s < p.S) {
+          y[0] = __fadd_rn(y[0], v[s].x); y[1] = __fadd_rn(y[1], v[s].y);
+          y[2] = __fadd_rn(y[2], v[s].z); y[3] = __fadd_rn(y[3], v[s].w);
+        }
+      }
+      __align__(16) TO o[4];
+      const TO* rrow = p.residual ? reinterpret_cast<const TO*>(p.residual) + m * p.res_ld + n0 + c : nullptr;
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        y[j] = fmaf(y[j], ctl->sc[c + j], ctl->sh[c + j]);  // (1 and 0 when there is no affine step)
+        if (rrow) y[j] += wcn_to_float<TO>(rrow[j]);
+        if (p.relu) y[j] = fmaxf(y[j], 0.f);
+        if (ctl->failed) y[j] = __int_as_float(0x7FC00000);
+        o[j] = wcn_from_float<TO>(y[j]);
+      }
+      TO* dst = reinterpret_cast<TO*>(p.out) + m * p.out_ld + n0 + c;
+      if (sizeof(TO) == 4) *reinterpret_cast<uint4*>(dst) = *reinterpret_cast<const uint4*>(o);
+      else *reinterpret_cast<uint2*>(dst) = *reinterpret_cast<const uint2*>(o);
+    }
+    cluster_meet();  // no CTA leaves while another may read its sums
   }
   tc_fence_before();
   __syncthreads();
@@ -693,90 +769,48 @@ __global__ void pack_weight_kernel(const T* __restrict__ w, T* __restrict__ pack
   packed[tile + off_bytes / 2 + within] = w[i];
 }
 
-// Second pass of a convolution whose kernel offsets were divided among S CTAs per row block:
-// adds the S fp32 slices of every output element in slice order (fixed, so the result has the
-// same bits on every run) and runs the epilogue.  One thread owns four consecutive columns
-// of one table row, so the slices are read and the rows written in full lines.
-template <typename TO>
-__global__ void conv_slice_reduce_kernel(const float* __restrict__ partial, int S, int64_t M, int c_out,
-                                         const int32_t* __restrict__ out_rows, const float* __restrict__ scale,
-                                         const float* __restrict__ shift, const TO* __restrict__ residual,
-                                         int64_t res_ld, int relu, TO* __restrict__ out, int64_t out_ld,
-                                         const int32_t* __restrict__ dev_status) {
-  const int quads = c_out >> 2;
-  const int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (t >= M * quads) return;
-  const int64_t slot = t / quads;
-  const int c = (int)(t - slot * quads) * 4;
-  const int64_t m = out_rows ? (int64_t)__ldg(&out_rows[slot]) : slot;
-  float y[4];
-  if (*dev_status == (int)WCN_ERR_WAIT_EXPIRED) {  // the first pass did not run (or gave up): no data to finish
-    y[0] = y[1] = y[2] = y[3] = __int_as_float(0x7FC00000);
-  } else {
-    const float4* src = reinterpret_cast<const float4*>(partial + slot * c_out + c);
-    const int64_t slice = M * (int64_t)c_out / 4;
-    float4 acc = __ldcg(src);
-    for (int s = 1; s < S; ++s) {
-      const float4 v = __ldcg(src + s * slice);
-      acc.x = __fadd_rn(acc.x, v.x); acc.y = __fadd_rn(acc.y, v.y);
-      acc.z = __fadd_rn(acc.z, v.z); acc.w = __fadd_rn(acc.w, v.w);
-    }
-    y[0] = acc.x; y[1] = acc.y; y[2] = acc.z; y[3] = acc.w;
-    if (scale || shift) {  // the recipe of the one-pass epilogue: one fused multiply-add
-#pragma unroll
-      for (int i = 0; i < 4; ++i)
-        y[i] = fmaf(y[i], scale ? __ldg(&scale[c + i]) : 1.f, shift ? __ldg(&shift[c + i]) : 0.f);
-    }
-    if (residual) {
-      const TO* r = residual + m * res_ld + c;
-#pragma unroll
-      for (int i = 0; i < 4; ++i) y[i] += wcn_to_float<TO>(r[i]);
-    }
-    if (relu) {
-#pragma unroll
-      for (int i = 0; i < 4; ++i) y[i] = fmaxf(y[i], 0.f);
-    }
-  }
-  __align__(16) TO o[4];
-#pragma unroll
-  for (int i = 0; i < 4; ++i) o[i] = wcn_from_float<TO>(y[i]);
-  TO* dst = out + m * out_ld + c;
-  if (sizeof(TO) == 4) *reinterpret_cast<uint4*>(dst) = *reinterpret_cast<const uint4*>(o);
-  else *reinterpret_cast<uint2*>(dst) = *reinterpret_cast<const uint2*>(o);
-}
-
 inline int pick_bk(int c_in) { return c_in % 64 == 0 ? 64 : 32; }
 
-constexpr int MAX_SLICES = 16;
+// Launch geometry.  A problem with fewer 128-row tiles than multiprocessors cannot occupy the GPU with one CTA per tile:
+// its kernel offsets are divided among S CTAs of a cluster and its output columns among blocks of their own (which gather
+// the rows again), whichever combination of the two moves the fewest bytes through one multiprocessor (split_k: 0 =
+// decide here, 1 = columns only, >= 2 = that many slices, at most eight; < 0 = -split_k column blocks).
+//
+// The model: a CTA reads n_off * (A + B) bytes, A = its 128 rows, B = its columns' weights at one offset, from L2 at the
+// ~100 KB/us one multiprocessor sustains; of K offsets about 0.6 K have a neighbour in a tile; adding the slices
+// costs about 1.5 us.  Clusters of S fit 8 * floor(18 / S) times (eight GPCs of at least 18 multiprocessors), and CTAs
+// beyond what fits wait for a second wave.
+void pick_split(const ConvTcParams& p, int64_t tiles, int split_k, int* slices, int* blocks) {
+  const int sms = wcn_num_sms();
+  *slices = *blocks = 1;
+  double best = 1e30;
+  for (int S = 1; S <= MAX_SLICES && S <= p.K; ++S) {
+    if (split_k == 1 && S > 1) break;
+    const int64_t fit = S == 1 ? sms : (int64_t)S * (18 / S) * 8 * sms / 148;
+    for (int nb = 1; nb <= 8; nb *= 2) {
+      if (p.c_out % (16 * nb) != 0 || (nb > 1 && p.c_out / nb < 32)) break;
+      const int64_t ctas = tiles * S * nb;
+      if (ctas > fit && ctas > tiles) continue;
+      const double off = (p.K > 2 ? 0.6 * p.K : p.K) / S;
+      const double bytes = (off < 1 ? 1 : off) * 2.0 * p.c_in * (BLOCK_M + p.c_out / nb);
+      const double us = bytes / 100e3 + (S > 1 ? 1.5 : 0.0);
+      if (us < best) { best = us; *slices = S; *blocks = nb; }
+    }
+  }
+}
 
-// Launch geometry.  A problem with fewer 128-row tiles than multiprocessors cannot occupy the
-// GPU with one CTA per tile.  With a 3x3x3-sized window there is enough work per tile to divide
-// its kernel offsets among S CTAs (split_k: 0 = decide here, 1 = never, >= 2 = that many
-// slices); otherwise the output columns are divided among CTAs, each re-gathering the rows,
-// which stay in L2 (split_k < 0 forces -split_k column blocks).
 bool plan_launch(ConvTcParams& p, int bk, int split_k, size_t* smem, dim3* grid) {
   const int sms = wcn_num_sms();
   const int64_t tiles = (p.M + BLOCK_M - 1) / BLOCK_M;
-  int S = 1;
+  int S = 1, split = 1;
   if (split_k >= 2) {
-    S = split_k;
-  } else if (split_k == 0 && p.K >= 9 && tiles * 2 <= sms) {
-    S = (int)(sms / tiles);
-    if (S > 8) S = 8;
-  }
-  if (S > p.K) S = p.K;
-  if (S > MAX_SLICES) S = MAX_SLICES;
-  int split = 1;
-  if (S == 1) {
-    if (split_k < 0) {
-      split = -split_k;
-      if (split > 16 || p.c_out % (16 * split) != 0) return false;
-    } else {
-      // Column blocks only while they at least double the CTAs that fit: with more than half as many
-      // tiles as multiprocessors one full-width CTA per tile is faster (measured: 147 tiles,
-      // 128 -> 128 channels, 39 us whole against 59 us in two column blocks).
-      while (tiles * split * 2 <= sms && p.c_out % (16 * split * 2) == 0 && p.c_out / (split * 2) >= 32 && split < 8) split *= 2;
-    }
+    S = split_k < MAX_SLICES ? split_k : MAX_SLICES;
+    if (S > p.K) S = p.K;
+  } else if (split_k < 0) {
+    split = -split_k;
+    if (split > 16 || p.c_out % (16 * split) != 0) return false;
+  } else if (tiles * 2 <= sms) {
+    pick_split(p, tiles, split_k, &S, &split);
   }
   p.S = S;
   p.block_n = p.c_out / split;
@@ -786,7 +820,7 @@ bool plan_launch(ConvTcParams& p, int bk, int split_k, size_t* smem, dim3* grid)
   // Two sub-tiles per supertile (one per issuer).  Four were used for narrow outputs once, to share a weight
   // slice among more rows; narrow layers have tiny weights, and the two extra staged tables (55 KB) are worth
   // more as row slots: 3x3x3 C = 32 / 64 layers measured 11 % faster with two.
-  int g = 2;
+  int g = S > 1 ? 1 : 2;
   while (g > 1 && ((tiles + g - 1) / g) * split * S < 2 * (int64_t)sms) g /= 2;
   const size_t a_unit = (size_t)BLOCK_M * bk * 2, b_unit = (size_t)p.block_n * bk * 2;
   const size_t limit = 226 * 1024;  // the kernels opt in to this much dynamic shared memory
@@ -827,10 +861,12 @@ bool plan_launch(ConvTcParams& p, int bk, int split_k, size_t* smem, dim3* grid)
   while (sb < 6 && fixed + sa * a_stage + (sb + 1) * b_stage <= limit) ++sb;
   p.sa = sa;
   p.sb = sb;
+  // the sums of a slice take the place of the rings
+  if (S > 1 && sa * a_stage + sb * b_stage < (size_t)BLOCK_M * (p.block_n + 4) * 4) return false;
   *smem = fixed + sa * a_stage + sb * b_stage;
   int64_t gx = p.units;
   const int64_t cap = sms / split > 0 ? sms / split : 1;
-  if (gx > cap) gx = cap;
+  if (gx > cap && S == 1) gx = cap;
   *grid = dim3((unsigned)gx, (unsigned)split);
   return true;
 }
@@ -848,29 +884,14 @@ int launch_kbc(const ConvTcParams& p, size_t smem, dim3 grid, cudaStream_t st) {
     }
     configured[dev] = true;
   }
-  kern<<<grid, THREADS, smem, st>>>(p);
-  if (cudaGetLastError() != cudaSuccess) return WCN_ERR_EXECUTION;
-  if (p.S > 1) {
-    const int64_t threads = p.M * (p.c_out >> 2);
-    conv_slice_reduce_kernel<TO><<<(unsigned)((threads + 255) / 256), 256, 0, st>>>(
-        p.partial, p.S, p.M, p.c_out, p.out_rows, p.scale, p.shift, reinterpret_cast<const TO*>(p.residual), p.res_ld,
-        p.relu, reinterpret_cast<TO*>(p.out), p.out_ld, p.dev_status);
-    if (cudaGetLastError() != cudaSuccess) return WCN_ERR_EXECUTION;
-  }
-  return WCN_OK;
+  return wcn_launch(kern, grid, dim3(THREADS), smem, st, (unsigned)p.S, p);
 }
 
 template <int BK, bool BF16, typename TO>
-int launch_tc(ConvTcParams& p, int split_k, void* workspace, int64_t workspace_bytes, cudaStream_t st) {
+int launch_tc(ConvTcParams& p, int split_k, cudaStream_t st) {
   size_t smem = 0;
   dim3 grid;
   if (!plan_launch(p, BK, split_k, &smem, &grid)) return WCN_ERR_UNSUPPORTED_CONFIG;
-  if (p.S > 1) {
-    const int64_t need = (int64_t)p.S * p.M * p.c_out * (int64_t)sizeof(float);
-    if (!workspace || workspace_bytes < need || (reinterpret_cast<uintptr_t>(workspace) & 15))
-      return WCN_ERR_INVALID_PARAMETERS;
-    p.partial = reinterpret_cast<float*>(workspace);
-  }
   // SPAN: the whole C_in is one slice and a ring slot holds KBC consecutive active offsets; otherwise a
   // slot holds KBC channel slices of one offset.  A compile-time choice, so that every role's loop
   // carries only the form it runs.
@@ -922,16 +943,6 @@ bool wcn_conv_tcgen05_supported(int K, int c_in, int c_out, int dtype, int out_d
 
 int64_t wcn_conv_tcgen05_packed_bytes(int K, int c_in, int c_out) { return (int64_t)K * c_in * c_out * 2; }
 
-// Bytes of slice workspace wcn_conv_tcgen05_fwd needs for this problem (0: one pass).
-int64_t wcn_conv_tcgen05_workspace_bytes(int64_t M, int K, int c_in, int c_out, int split_k) {
-  ConvTcParams p = {};
-  p.M = M; p.K = K; p.c_in = c_in; p.c_out = c_out;
-  size_t smem = 0;
-  dim3 grid;
-  if (M <= 0 || !plan_launch(p, pick_bk(c_in), split_k, &smem, &grid) || p.S <= 1) return 0;
-  return (int64_t)p.S * M * c_out * (int64_t)sizeof(float);
-}
-
 int wcn_conv_tcgen05_pack(const void* weight, int K, int c_in, int c_out, void* packed, cudaStream_t st) {
   const int64_t total = (int64_t)K * c_in * c_out;
   if (total == 0) return WCN_OK;
@@ -943,8 +954,7 @@ int wcn_conv_tcgen05_pack(const void* weight, int K, int c_in, int c_out, void* 
 int wcn_conv_tcgen05_fwd(const void* feats, int64_t num_in, int64_t feats_ld, const void* packed, const int32_t* nbr,
                          const int32_t* out_rows, int64_t M, int K, int c_in, int c_out, int dtype,
                          const float* scale, const float* shift, const void* residual, int64_t residual_ld, int relu,
-                         void* out, int64_t out_ld, int out_dtype, int split_k, void* workspace,
-                         int64_t workspace_bytes, int32_t* dev_status, cudaStream_t st) {
+                         void* out, int64_t out_ld, int out_dtype, int split_k, int32_t* dev_status, cudaStream_t st) {
   if (!wcn_conv_tcgen05_supported(K, c_in, c_out, dtype, out_dtype)) return WCN_ERR_UNSUPPORTED_CONFIG;
   if (!dev_status || !packed || num_in <= 0 || num_in >= 0x7FFFFFFFll || M >= 0x7FFFFFFFll) return WCN_ERR_INVALID_PARAMETERS;
   const int64_t osz = out_dtype == WCN_F32 ? 4 : 2;
@@ -961,11 +971,10 @@ int wcn_conv_tcgen05_fwd(const void* feats, int64_t num_in, int64_t feats_ld, co
   p.dev_status = dev_status;
   p.wide_out = (reinterpret_cast<uintptr_t>(out) & 31) == 0 && (out_ld * osz) % 32 == 0;
   p.wide_res = residual && (reinterpret_cast<uintptr_t>(residual) & 31) == 0 && (residual_ld * osz) % 32 == 0;
-  p.wide_partial = (reinterpret_cast<uintptr_t>(workspace) & 31) == 0;   // its rows are c_out fp32 values: 64-byte multiples
   const int bk = pick_bk(c_in);
   const bool bf = dtype == WCN_BF16;
 #define WCN_TC_CASE(BKV, BFV, TO) \
-  if (bk == BKV && bf == BFV) return launch_tc<BKV, BFV, TO>(p, split_k, workspace, workspace_bytes, st);
+  if (bk == BKV && bf == BFV) return launch_tc<BKV, BFV, TO>(p, split_k, st);
   if (out_dtype == WCN_F32) {
     WCN_TC_CASE(64, false, float) WCN_TC_CASE(64, true, float) WCN_TC_CASE(32, false, float) WCN_TC_CASE(32, true, float)
   } else if (bf) {

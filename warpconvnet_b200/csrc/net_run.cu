@@ -16,26 +16,14 @@ bool valid(const wcn_net_op& o) {
 
 }  // namespace
 
-extern "C" int wcn_net_workspace_bytes(const wcn_net_op* ops, int32_t num_ops, const int64_t* rows, int dtype, int64_t* bytes) {
-  if (!ops || num_ops < 0 || !rows || !bytes || (dtype != WCN_F16 && dtype != WCN_BF16)) return WCN_ERR_INVALID_PARAMETERS;
-  *bytes = 0;
-  for (int i = 0; i < num_ops; ++i) {
-    const wcn_net_op& o = ops[i];
-    if (!valid(o)) return WCN_ERR_INVALID_PARAMETERS;
-    if (o.kind != 0 || !o.packed) continue;
-    int64_t need = 0;
-    const int rc = wcn_conv_workspace_bytes(WCN_CONV_AUTO, rows[o.level_out], o.num_offsets, o.c_in, o.c_out, dtype, dtype, 0, &need);
-    if (rc != WCN_OK) return rc;
-    if (need > *bytes) *bytes = need;
-  }
-  return WCN_OK;
-}
-
 extern "C" int wcn_net_run(const wcn_net_op* ops, int32_t num_ops, const int64_t* rows, const wcn_net_buffer* buffers,
-                           const wcn_net_table* tables, int dtype, void* workspace, int64_t workspace_bytes,
-                           int32_t* launches, int32_t* dev_status, void* stream) {
+                           const wcn_net_table* tables, int dtype, int32_t* dev_status, void* stream) {
   if (!ops || num_ops < 0 || !rows || !buffers || !tables || (dtype != WCN_F16 && dtype != WCN_BF16)) return WCN_ERR_INVALID_PARAMETERS;
-  int count = 0;
+  // The first launch waits for everything before it (tables among it); the ones after it overlap with their
+  // predecessors.
+  struct Overlap {
+    ~Overlap() { wcn_overlap_launches = false; }
+  } until_return;
   for (int i = 0; i < num_ops; ++i) {
     const wcn_net_op& o = ops[i];
     if (!valid(o)) return WCN_ERR_INVALID_PARAMETERS;
@@ -52,19 +40,12 @@ extern "C" int wcn_net_run(const wcn_net_op* ops, int32_t num_ops, const int64_t
                              o.c_out_packed, o.c_out, dtype, o.scale, o.shift, res, res_ld, o.relu, dst, out.ld, dtype, dev_status,
                              stream);
     } else {
-      int64_t need = 0;
-      if (o.packed) {
-        rc = wcn_conv_workspace_bytes(WCN_CONV_AUTO, n_out, o.num_offsets, o.c_in, o.c_out, dtype, dtype, 0, &need);
-        if (rc != WCN_OK) return rc;
-      }
       rc = wcn_conv_fwd(WCN_CONV_AUTO, src, n_in, in.ld, o.weight, o.packed, tables[o.table].nbr, tables[o.table].out_rows, n_out,
                         o.num_offsets, o.c_in, o.c_out, dtype, o.scale, o.shift, res, res_ld, o.relu, dst, out.ld, dtype, 0,
-                        need ? workspace : nullptr, need ? workspace_bytes : 0, dev_status, stream);
-      count += need ? 1 : 0;
+                        nullptr, 0, dev_status, stream);
     }
     if (rc != WCN_OK) return rc;
-    ++count;
+    wcn_overlap_launches = true;
   }
-  if (launches) *launches = count;
   return WCN_OK;
 }

@@ -127,3 +127,39 @@ static inline int wcn_num_sms() {
   }
   return cached[dev];
 }
+
+// ------------------------------------------------------------------ launches that overlap
+//
+// While it is set (by wcn_net_run, from its second op on), the kernels that take part start as soon as every block of
+// the launch before them has: they may read what was written before the network's first launch at once, and wait with
+// wait_for_primary() before they touch anything the launch before them reads or writes.
+extern thread_local bool wcn_overlap_launches;
+
+#ifdef __CUDACC__
+__device__ __forceinline__ void launch_dependents() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+__device__ __forceinline__ void wait_for_primary() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+
+template <typename K, typename... A>
+static inline int wcn_launch(K kernel, dim3 grid, dim3 block, size_t smem, cudaStream_t st, unsigned cluster, const A&... args) {
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = grid; cfg.blockDim = block; cfg.dynamicSmemBytes = smem; cfg.stream = st;
+  cudaLaunchAttribute attr[2];
+  if (cluster > 1) {
+    attr[cfg.numAttrs].id = cudaLaunchAttributeClusterDimension;
+    attr[cfg.numAttrs].val.clusterDim.x = cluster;
+    attr[cfg.numAttrs].val.clusterDim.y = attr[cfg.numAttrs].val.clusterDim.z = 1;
+    ++cfg.numAttrs;
+  }
+  if (wcn_overlap_launches) {
+    attr[cfg.numAttrs].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[cfg.numAttrs].val.programmaticStreamSerializationAllowed = 1;
+    ++cfg.numAttrs;
+  }
+  cfg.attrs = attr;
+  if (cudaLaunchKernelEx(&cfg, kernel, args...) != cudaSuccess) {
+    (void)cudaGetLastError();
+    return WCN_ERR_EXECUTION;
+  }
+  return WCN_OK;
+}
+#endif

@@ -16,7 +16,7 @@ from typing import Optional, Union
 import torch
 import torch.nn as nn
 
-from .._native import LAUNCH_COUNTS, NetOp, check, device_status, dtype_code, lib, ptr, query_bytes, stream_ptr
+from .._native import LAUNCH_COUNTS, NetOp, check, device_status, dtype_code, lib, ptr, stream_ptr
 from ..geometry.types.voxels import Voxels
 from ..geometry.coords.search.cache import IntSearchCache
 from ..geometry.coords.search.level_maps import LevelMaps
@@ -470,7 +470,6 @@ class _Program:
         buffers = (ctypes.c_int64 * (2 * (self.TEMP + 20)))()
         tables = (ctypes.c_int64 * 22)()
         rows = (ctypes.c_int64 * 5)(n0, 0, 0, 0, 0)
-        launches = ctypes.c_int32(0)
         joined0 = torch.empty((n0, self.joined_width[0]), dtype=dtype, device=dev)
         identity = _identity_map(n0, dev).neighbor_table(n0)
         buffers[0], buffers[1] = feats.data_ptr(), feats.stride(0)
@@ -478,13 +477,12 @@ class _Program:
         tables[2 * self.IDENTITY] = identity.data_ptr()
         ops, count = ctypes.addressof(self.ops), len(self.ops)
 
-        def enqueue(first, n, ws, ws_bytes):
+        def enqueue(first, n):
             check(lib_.wcn_net_run(ops + first * ctypes.sizeof(NetOp), n, ctypes.addressof(rows), ctypes.addressof(buffers),
-                                   ctypes.addressof(tables), self.dtype_code, ws, ws_bytes, ctypes.addressof(launches), status,
-                                   stream), "wcn_net_run")
-            LAUNCH_COUNTS["wcn_net_run"] += launches.value
+                                   ctypes.addressof(tables), self.dtype_code, status, stream), "wcn_net_run")
+            LAUNCH_COUNTS["wcn_net_run"] += n
 
-        enqueue(0, 1, None, 0)  # the stem runs while the host waits for the sizes of the coarser levels
+        enqueue(0, 1)  # the stem runs while the host waits for the sizes of the coarser levels
         if maps.finish() is None:
             return None
         for l in range(5):
@@ -492,8 +490,7 @@ class _Program:
             tables[2 * l], tables[2 * l + 1] = maps.nbr[l].data_ptr(), ptr(maps.order[l]) or 0
             if l < 4:
                 tables[2 * (self.CHILD + l)] = maps.child[l].data_ptr()
-        ws_bytes = query_bytes("wcn_net_workspace_bytes", ops, count, ctypes.addressof(rows), self.dtype_code)
-        total, places = -(-ws_bytes // 256) * 256, []
+        total, places = 0, []
         for b, level, w in self.arena:
             places.append((b, w, total))
             total += -(-2 * maps.n[level] * w // 256) * 256
@@ -506,13 +503,13 @@ class _Program:
         if restore_order:  # sorted row j is original row perm[j]: each row of logits is written at its original place
             dst = perm.to(torch.int32)
             tables[2 * self.PERM] = dst.data_ptr()
-            enqueue(1, count - 2, base, ws_bytes)
+            enqueue(1, count - 2)
             last = NetOp.from_buffer_copy(self.ops[count - 1])
             last.table = self.PERM
             ops, count = ctypes.addressof(last), 1
-            enqueue(0, 1, None, 0)
+            enqueue(0, 1)
             return out
-        enqueue(1, count - 1, base, ws_bytes)
+        enqueue(1, count - 1)
         return x._derive(out)
 
 

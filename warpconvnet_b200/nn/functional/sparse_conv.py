@@ -27,7 +27,7 @@ import numpy as np
 import torch
 from torch import Tensor
 
-from ..._native import (CONV_AUTO, CONV_SIMT, CONV_TCGEN05, LAUNCH_COUNTS, check, device_status, dtype_code, lib, ptr,
+from ..._native import (CONV_AUTO, CONV_SIMT, CONV_TCGEN05, check, device_status, dtype_code, lib, ptr,
                         query_bytes, require_cuda, stream_ptr)
 from ...geometry.coords.integer import IntCoords
 from ...geometry.coords.ops.serialization import POINT_ORDERING, encode
@@ -196,22 +196,6 @@ def _row_view(t: Tensor) -> Tensor:
     return t if t.dim() == 2 and t.stride(1) == 1 and t.stride(0) >= t.shape[1] else t.contiguous()
 
 
-_workspace_bytes_cache: dict = {}
-
-
-def _conv_workspace(algo: int, num_out: int, K: int, c_in: int, c_out: int, dtype_c: int, out_dtype_c: int,
-                    split_k: int, dev: torch.device) -> Optional[Tensor]:
-    """Scratch for the offset-sliced tensor-core convolution (None when the launch is one pass)."""
-    key = (algo, num_out, K, c_in, c_out, dtype_c, out_dtype_c, split_k, dev.index)
-    nbytes = _workspace_bytes_cache.get(key)
-    if nbytes is None:
-        nbytes = query_bytes("wcn_conv_workspace_bytes", algo, num_out, K, c_in, c_out, dtype_c, out_dtype_c, split_k)
-        if len(_workspace_bytes_cache) > 4096:
-            _workspace_bytes_cache.clear()
-        _workspace_bytes_cache[key] = nbytes
-    return torch.empty(nbytes, dtype=torch.uint8, device=dev) if nbytes else None
-
-
 def sparse_conv_fused(in_features: Tensor, weight: Tensor, kernel_map: IntSearchResult, num_out_coords: int,
                       epilogue: Optional[ConvEpilogue] = None, out_dtype: Optional[torch.dtype] = None,
                       algo: int = CONV_AUTO, tile_order: Optional[bool] = None, split_k: int = 0) -> Tensor:
@@ -220,7 +204,7 @@ def sparse_conv_fused(in_features: Tensor, weight: Tensor, kernel_map: IntSearch
     output rows grouped by neighbour pattern (``IntSearchResult.tiled_neighbor_table``;
     same numbers, fewer (tile, offset) pairs to compute); None = by size.  ``split_k``
     (the reference's ``split_k_slices``): 0 lets the library divide the kernel offsets of
-    small problems among CTAs, 1 forbids it, 2..16 asks for that many slices.  Features,
+    small problems among CTAs, 1 forbids it, 2 and more ask for that many slices (at most 8).  Features,
     residual and ``epilogue.out`` may be column blocks of wider matrices."""
     require_cuda(in_features, "in_features")
     x = _row_view(in_features)
@@ -279,15 +263,11 @@ def sparse_conv_fused(in_features: Tensor, weight: Tensor, kernel_map: IntSearch
         assert tuple(residual.shape) == (num_out_coords, c_out), \
             f"residual {tuple(residual.shape)} != output {(num_out_coords, c_out)}"
     dc, odc = dtype_code(x.dtype), dtype_code(out_dtype)
-    ws = _conv_workspace(algo, num_out_coords, K, c_in, c_out, dc, odc, split_k, dev) if packed is not None else None
     check(lib().wcn_conv_fwd(algo, ptr(x), x.shape[0], x.stride(0), ptr(w), ptr(packed), ptr(nbr), ptr(out_rows),
                              num_out_coords, K, c_in, c_out, dc, ptr(scale), ptr(shift), ptr(residual),
                              residual.stride(0) if residual is not None else 0, int(ep.relu), ptr(out),
-                             out.stride(0), odc, split_k, ptr(ws), ws.numel() if ws is not None else 0,
-                             ptr(device_status(dev)), stream_ptr(dev)),
+                             out.stride(0), odc, split_k, None, 0, ptr(device_status(dev)), stream_ptr(dev)),
           "wcn_conv_fwd")
-    if ws is not None:
-        LAUNCH_COUNTS["wcn_conv_fwd"] += 1  # the offset-sliced form is two kernels: slices, then their sum + epilogue
     return out
 
 
@@ -304,7 +284,7 @@ class FusedConvLaunch:
     neighbour table (tiled, with its ``out_rows``, or plain with ``out_rows=None``)."""
 
     __slots__ = ("weight", "packed", "scale", "shift", "relu", "K", "c_in", "c_out", "dtype", "device", "_dc",
-                 "_w_ptr", "_packed_ptr", "_scale_ptr", "_shift_ptr", "_status_ptr", "_ws_bytes", "_dev_index", "_fn")
+                 "_w_ptr", "_packed_ptr", "_scale_ptr", "_shift_ptr", "_status_ptr", "_dev_index", "_fn")
 
     def __init__(self, weight: Tensor, dtype: torch.dtype, scale: Optional[Tensor] = None,
                  shift: Optional[Tensor] = None, relu: bool = False):
@@ -318,7 +298,6 @@ class FusedConvLaunch:
         self._w_ptr, self._packed_ptr = ptr(w), ptr(packed)
         self._scale_ptr, self._shift_ptr = ptr(self.scale), ptr(self.shift)
         self._status_ptr = ptr(device_status(dev))
-        self._ws_bytes = {}
         self._dev_index = dev.index if dev.index is not None else torch.cuda.current_device()
         self._fn = lib().wcn_conv_fwd
 
@@ -328,25 +307,14 @@ class FusedConvLaunch:
             out = torch.empty((num_out, self.c_out), dtype=self.dtype, device=self.device)
         if num_out == 0:
             return out
-        ws = None
-        if self._packed_ptr:
-            nbytes = self._ws_bytes.get(num_out)
-            if nbytes is None:
-                nbytes = self._ws_bytes[num_out] = query_bytes("wcn_conv_workspace_bytes", CONV_AUTO, num_out, self.K,
-                                                               self.c_in, self.c_out, self._dc, self._dc, 0)
-            if nbytes:
-                ws = torch.empty(nbytes, dtype=torch.uint8, device=self.device)
         rc = self._fn(CONV_AUTO, feats.data_ptr(), feats.shape[0], feats.stride(0), self._w_ptr, self._packed_ptr,
                       nbr.data_ptr(), out_rows.data_ptr() if out_rows is not None else None, num_out, self.K,
                       self.c_in, self.c_out, self._dc, self._scale_ptr, self._shift_ptr,
                       residual.data_ptr() if residual is not None else None,
                       residual.stride(0) if residual is not None else 0, self.relu, out.data_ptr(), out.stride(0),
-                      self._dc, 0, ws.data_ptr() if ws is not None else None, nbytes if ws is not None else 0,
-                      self._status_ptr, torch._C._cuda_getCurrentRawStream(self._dev_index))
+                      self._dc, 0, None, 0, self._status_ptr, torch._C._cuda_getCurrentRawStream(self._dev_index))
         if rc != 0:
             check(rc, "wcn_conv_fwd")
-        if ws is not None:
-            LAUNCH_COUNTS["wcn_conv_fwd"] += 1
         return out
 
 
