@@ -284,6 +284,27 @@ int wcn_kmap_tile_order(const int32_t* nbr, int64_t num_out, int32_t num_offsets
 int wcn_kmap_tile_masks(const int32_t* nbr, int64_t num_out, int32_t num_offsets, uint32_t* masks,
                         void* stream);
 
+/* Table of 4x4x4 cells over keys [n, 4] in any order (32-byte aligned buffer of wcn_cells_bytes; 256 bytes per key are
+ * reserved for the rows of a cell, of which as many are touched as there are cells), and windows up to four wide answered
+ * from it: nbr as wcn_kmap_search writes it, repeated keys resolving to the smallest row.  `workspace` (may be NULL)
+ * receives the per-block hit counts wcn_kmap_scan wants.
+ * Replaces the per-offset probes of kernel_map_size_4d (warpconvnet/csrc/discrete_kernels.cu:264-334). */
+int wcn_cells_bytes(int64_t n, int64_t* bytes);
+int wcn_cells_build(const int32_t* keys, int64_t n, void* table, void* stream);
+int wcn_kmap_search_cells(const void* table, int64_t n, const int32_t* queries, int64_t num_queries,
+                          const int32_t* stride, const int32_t* kernel_size, int32_t* nbr, void* workspace, void* stream);
+
+/* wcn_kmap_scan that also leaves the offsets [num_offsets + 1] and the device status word in pinned host memory
+ * (int32 [num_offsets + 2]), valid once the stream has passed it. */
+int wcn_kmap_scan_host(void* workspace, int64_t num_queries, int32_t num_offsets, int32_t* offsets, int32_t* host,
+                       const int32_t* dev_status, void* stream);
+
+/* After wcn_unique_mark / wcn_unique_emit over n rows: host (pinned int32 [items + 3]) = number of distinct rows, device
+ * status word, distinct rows of batch items 0..items-1, rows of any other item.  hist: int32 [items + 1] scratch.
+ * Replaces the bincount behind the output offsets (warpconvnet/geometry/coords/ops/stride.py:48-54). */
+int wcn_unique_counts(const int32_t* rows, int64_t n, const void* workspace, int32_t items, int32_t* hist, int32_t* host,
+                      const int32_t* dev_status, void* stream);
+
 /* ------------------------------------------------------------------ Morton code */
 
 /* codes[i] = 3-D Morton code of (x - min_xyz[0], y - min_xyz[1], z - min_xyz[2]), x in bit

@@ -425,3 +425,33 @@ def test_pyramid_in_one_sync_equals_chained_levels(monkeypatch):
         assert np.array_equal(a.offsets.numpy(), want_off) and np.array_equal(b.offsets.numpy(), want_off)
         assert torch.equal(a.morton_origin, b.morton_origin) and a.bricks.header()["valid"]
     check_device_status(DEV)
+
+
+@pytest.mark.parametrize("n,repeat,batches,low,ksize,stride", [(1, 0, 1, 0, (3, 3, 3), (1, 1, 1)), (255, 40, 2, -30, (3, 3, 3), (1, 1, 1)),
+                                                               (5000, 0, 3, -7, (2, 2, 2), (2, 2, 2)), (5000, 700, 1, 5, (4, 2, 3), (1, 2, 1)),
+                                                               (70000, 9, 2, -(1 << 20), (3, 3, 3), (1, 1, 1)), (3000, 0, 1, 0, (1, 1, 4), (3, 1, 1))])
+def test_cell_table_maps_equal_voxel_table_maps(n, repeat, batches, low, ksize, stride):
+    """Unordered rows, repeated voxels, windows of every width up to four, strides: the dense and the compact form
+    through the cell table equal those through the voxel hash table."""
+    from warpconvnet_b200 import TorchHashTable
+    rng = np.random.default_rng(n + repeat)
+    e = int((n * 7) ** (1 / 3)) + 2
+    c = np.concatenate([rng.integers(0, batches, (n, 1)), rng.integers(0, e, (n, 3)) + low], 1).astype(np.int32)
+    c = np.unique(c, axis=0)
+    c = np.concatenate([c, c[rng.integers(0, len(c), repeat)]])
+    c = dev(c[rng.permutation(len(c))])
+    out = stride_coords(c, stride)[0] if any(s != 1 for s in stride) else c
+    got = generate_kernel_map(c, out, stride, ksize)
+    want = generate_kernel_map(c, out, stride, ksize, hashtable=TorchHashTable.from_keys(c))
+    assert torch.equal(got.neighbor_table(len(out)), want.neighbor_table(len(out)))
+    assert torch.equal(got.offsets, want.offsets) and torch.equal(got.in_maps, want.in_maps)
+    assert torch.equal(got.out_maps, want.out_maps)
+
+
+def test_stride_coords_counts_more_batch_items_than_are_tallied():
+    rng = np.random.default_rng(3)
+    c = np.concatenate([np.sort(rng.integers(0, 3000, (9000, 1)), 0), rng.integers(0, 9, (9000, 3))], 1).astype(np.int32)
+    rows, offsets = stride_coords(dev(c), (2, 2, 2))
+    want, _ = km.stride_coords(c, (2, 2, 2))
+    assert np.array_equal(rows.cpu().numpy(), want)
+    assert offsets.tolist() == [0] + np.cumsum(np.bincount(want[:, 0])).tolist()

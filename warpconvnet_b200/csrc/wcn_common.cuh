@@ -128,6 +128,9 @@ static inline int wcn_num_sms() {
   return cached[dev];
 }
 
+// Where a unique workspace keeps the number of distinct rows (hash_kmap.cu).
+const int* wcn_unique_total(const void* workspace, int64_t n);
+
 // ------------------------------------------------------------------ launches that overlap
 //
 // While it is set (by wcn_net_run, from its second op on), the kernels that take part start as soon as every block of

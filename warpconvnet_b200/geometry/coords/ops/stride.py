@@ -10,6 +10,7 @@ from __future__ import annotations
 import ctypes
 from typing import Optional, Tuple
 
+import numpy as np
 import torch
 from torch import Tensor
 
@@ -79,6 +80,42 @@ def unique_strided_rows(bcoords: Tensor, stride: Tuple[int, int, int] = (1, 1, 1
     return rows[:m], uidx[:m], parent
 
 
+# Batch items whose rows are counted on the device along with the distinct rows.
+COUNTED_ITEMS = 1021
+
+
+def _strided_with_counts(bcoords: Tensor, stride: Tuple[int, int, int], hash_method: HashMethod = HashMethod.CITY):
+    """``(rows, CPU offsets)`` of the distinct rows with one wait of the host: the row count, the rows per batch item and
+    the status word arrive together in pinned memory."""
+    assert bcoords.is_cuda, f"Batched coordinates must be on cuda device, got {bcoords.device}"
+    assert bcoords.dtype == torch.int32 and bcoords.shape[1] == 4
+    dev, c, n = bcoords.device, bcoords.contiguous(), bcoords.shape[0]
+    cap = max(16, 2 * n)
+    table = torch.empty(query_bytes("wcn_hash_table_bytes", cap), dtype=torch.uint8, device=dev)
+    strd = (ctypes.c_int32 * 3)(*[int(s) for s in stride])
+    sp, st, status = ctypes.addressof(strd), stream_ptr(dev), ptr(device_status(dev))
+    check(lib().wcn_hash_build(ptr(c), n, sp, ptr(table), cap, hash_method.value, None, status, st), "wcn_hash_build")
+    ws = torch.empty(query_bytes("wcn_unique_workspace_bytes", n), dtype=torch.uint8, device=dev)
+    count = torch.empty(1, dtype=torch.int64, device=dev)
+    check(lib().wcn_unique_mark(ptr(c), n, sp, ptr(table), cap, hash_method.value, ptr(ws), ptr(count), st),
+          "wcn_unique_mark")
+    rows = torch.empty((n, 4), dtype=torch.int32, device=dev)
+    check(lib().wcn_unique_emit(ptr(c), n, sp, ptr(ws), ptr(rows), None, None, st), "wcn_unique_emit")
+    hist = torch.empty(COUNTED_ITEMS + 1, dtype=torch.int32, device=dev)
+    host = torch.empty(COUNTED_ITEMS + 3, dtype=torch.int32, pin_memory=True)
+    check(lib().wcn_unique_counts(ptr(rows), n, ptr(ws), COUNTED_ITEMS, ptr(hist), ptr(host), status, st),
+          "wcn_unique_counts")
+    torch.cuda.current_stream(dev).synchronize()
+    h = host.numpy()
+    raise_for_status(int(h[1]), dev)
+    rows = rows[:int(h[0])]
+    if h[-1]:  # more batch items than are counted
+        return rows, offsets_from_batch_index(rows[:, 0])
+    offsets = np.zeros(int(np.flatnonzero(h[2:-1])[-1]) + 2, np.int64)
+    np.cumsum(h[2:len(offsets) + 1], out=offsets[1:])
+    return rows, torch.from_numpy(offsets)
+
+
 @torch.no_grad()
 def strided_pyramid(bcoords: Tensor, total_strides, in_offsets: Tensor, hash_method: HashMethod = HashMethod.CITY):
     """Distinct rows of ``floor(bcoords / s)`` for SEVERAL strides ``s`` of the same rows, with ONE
@@ -144,6 +181,8 @@ def stride_coords(batch_indexed_coords: Tensor, stride: Tuple[int, ...], order=N
         rows, _, _, out_offsets = unique_strided_rows(batch_indexed_coords, ntuple(stride, ndim=nd),
                                                       in_offsets=in_offsets)
         return rows, out_offsets
+    if (order is None or order == POINT_ORDERING.RANDOM) and batch_indexed_coords.shape[0] > 0 and nd == 3:
+        return _strided_with_counts(batch_indexed_coords, ntuple(stride, ndim=nd))
     rows, _, _ = unique_strided_rows(batch_indexed_coords, ntuple(stride, ndim=nd))
     if order is not None and order != POINT_ORDERING.RANDOM:
         offsets = offsets_from_batch_index(rows[:, 0])

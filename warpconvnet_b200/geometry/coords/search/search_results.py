@@ -18,7 +18,7 @@ from typing import List, Literal, Optional, Tuple
 import torch
 from torch import Tensor
 
-from ...._native import check, device_status, lib, ptr, query_bytes, raise_for_status, small_to_device, stream_ptr
+from ...._native import check, check_device_status, device_status, lib, ptr, query_bytes, raise_for_status, small_to_device, stream_ptr
 
 
 class IntSearchResult:
@@ -64,6 +64,19 @@ class IntSearchResult:
         self._tiled = (tiled, out_rows)
         return self
 
+    def begin_compact(self) -> None:
+        """Starts the compact form of a map whose hits the search has counted: the counts become write positions and
+        the offsets travel to pinned memory, so that the host finds them there when it asks."""
+        nbr, K, M = self._nbr, self._num_offsets, self._num_out
+        dev = nbr.device
+        offsets = torch.empty(K + 1, dtype=torch.int32, device=dev)
+        host = torch.empty(K + 2, dtype=torch.int32, pin_memory=True)
+        check(lib().wcn_kmap_scan_host(ptr(self._workspace), M, K, ptr(offsets), ptr(host), ptr(device_status(dev)),
+                                       stream_ptr(dev)), "wcn_kmap_scan_host")
+        done = torch.cuda.Event()
+        done.record(torch.cuda.current_stream(dev))
+        self._scanned = (offsets, host, done)
+
     def _plain(self) -> Tensor:
         """The plain neighbour table of a map made dense."""
         if self._nbr is None:
@@ -84,6 +97,13 @@ class IntSearchResult:
         nbr, K, M = self._plain(), self._num_offsets, self._num_out
         dev = nbr.device
         ws = self._workspace
+        scanned = self.__dict__.pop("_scanned", None)
+        if scanned is not None:
+            offsets, host, done = scanned
+            done.synchronize()
+            self._emit_compact(ws, offsets, host[:-1].clone())
+            check_device_status(dev)  # the pairs are being written meanwhile
+            return
         if ws is None:  # searched without hit counts: count now
             ws = torch.empty(query_bytes("wcn_kmap_workspace_bytes", M, K), dtype=torch.uint8, device=dev)
             check(lib().wcn_kmap_count(ptr(nbr), M, K, ptr(ws), stream_ptr(dev)), "wcn_kmap_count")
@@ -92,7 +112,11 @@ class IntSearchResult:
         # the one host synchronisation of a compact map; the device status word is read with it
         both = torch.cat([offsets, device_status(dev)]).cpu()
         raise_for_status(int(both[-1]), dev)
-        offsets_cpu = both[:-1].clone()
+        self._emit_compact(ws, offsets, both[:-1].clone())
+
+    def _emit_compact(self, ws: Tensor, offsets: Tensor, offsets_cpu: Tensor) -> None:
+        nbr, K, M = self._plain(), self._num_offsets, self._num_out
+        dev = nbr.device
         L = int(offsets_cpu[-1])
         in_maps = torch.empty(L, dtype=torch.int32, device=dev)
         out_maps = torch.empty(L, dtype=torch.int32, device=dev)

@@ -483,13 +483,13 @@ def _generate_kernel_map_nd(in_coords: Tensor, out_coords: Tensor, stride, kerne
     """``generate_kernel_map`` for 3 spatial dimensions as is, for 2 through the z = 0 slab."""
     if in_coords.shape[1] == 4:
         return generate_kernel_map(in_coords, out_coords, stride, kernel_size, kernel_dilation, hashtable=hashtable,
-                                   bricks=bricks)
+                                   bricks=bricks, count_hits=False)
     assert in_coords.shape[1] == 3 and out_coords.shape[1] == 3, "coordinates must have 2 or 3 spatial dimensions"
     same = out_coords.data_ptr() == in_coords.data_ptr() and out_coords.shape == in_coords.shape
     in4 = _with_z(in_coords)
     out4 = in4 if same else _with_z(out_coords)
     return generate_kernel_map(in4, out4, tuple(stride) + (1,), tuple(kernel_size) + (1,),
-                               tuple(kernel_dilation) + (1,))
+                               tuple(kernel_dilation) + (1,), count_hits=False)
 
 
 def generate_output_coords_and_kernel_map(input_sparse_tensor: Voxels, kernel_size: Tuple[int, ...],
