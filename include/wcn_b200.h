@@ -339,6 +339,11 @@ int wcn_conv_packed_weight_bytes(int algo, int32_t num_offsets, int32_t c_in, in
 
 /* Re-layout weight[K, c_in, c_out] into the buffer above (K-major tiles for the tensor-core
  * kernel).  No reference counterpart (its kernels read the weights as stored). */
+/* wcn_conv_pack_weight from a weight tensor of another dtype (converted as it is packed), of its transpose per offset
+ * (transposed != 0: weight is [K, c_out, c_in]) and with the offsets in reverse order (reversed != 0): a gradient's
+ * weights in one launch. */
+int wcn_conv_pack_weight_from(const void* weight, int src_dtype, int32_t num_offsets, int32_t c_in, int32_t c_out, int dtype,
+                              int32_t transposed, int32_t reversed, void* packed, void* stream);
 int wcn_conv_pack_weight(int algo, const void* weight, int32_t num_offsets, int32_t c_in,
                          int32_t c_out, int dtype, void* packed, void* stream);
 
@@ -533,6 +538,25 @@ typedef struct { const int32_t* nbr; const int32_t* out_rows; } wcn_net_table;
  * (warpconvnet/nn/modules/sequential.py:14-62, examples/mink_unet.py:212-413). */
 int wcn_net_run(const wcn_net_op* ops, int32_t num_ops, const int64_t* rows, const wcn_net_buffer* buffers,
                 const wcn_net_table* tables, int dtype, int32_t* dev_status, void* stream);
+
+/* ------------------------------------------------------------------ batch normalisation in training */
+
+/* y = relu(batch_norm(x) + residual) of [n, channels] rows (residual, relu optional), rounded to the dtype after the
+ * normalisation and after the addition.  mean / rstd [channels] are left for the backward pass; running_mean / running_var
+ * (may be NULL) and *num_batches (may be NULL) are updated as nn.BatchNorm1d does with a momentum.  eps and momentum are
+ * given as the bits of a float.  `counter`: one zero word, zero again afterwards (one per stream).
+ * backward: dx (may be NULL) and, with a residual behind a ReLU, its gradient; sums [2, channels] = d beta, d gamma;
+ * y: the forward's result where a residual was added, else NULL.
+ * WCN_ERR_UNSUPPORTED_CONFIG: n < 2, more than 1024 channels, or rows that are no whole number of 16-byte pieces.
+ * Stands for the nn.BatchNorm1d / addition / nn.ReLU chain of examples/mink_unet.py:36-47, 129-141. */
+int wcn_batch_norm_workspace_bytes(int64_t n, int32_t channels, int dtype, int64_t* bytes);
+int wcn_batch_norm_train(const void* x, int64_t n, int32_t channels, int dtype, const float* gamma, const float* beta,
+                         uint32_t eps_bits, uint32_t momentum_bits, float* running_mean, float* running_var,
+                         int64_t* num_batches, const void* residual, int relu, void* y, float* mean, float* rstd,
+                         void* workspace, uint32_t* counter, void* stream);
+int wcn_batch_norm_backward(const void* x, const void* dy, const void* y, int64_t n, int32_t channels, int dtype,
+                            const float* gamma, const float* beta, const float* mean, const float* rstd, int relu, void* dx,
+                            void* dresidual, float* sums, void* workspace, uint32_t* counter, void* stream);
 
 /* ------------------------------------------------------------------ self test */
 

@@ -1,0 +1,74 @@
+"""Training-mode BatchNorm + residual + ReLU in the native kernels against the layers they stand for."""
+import pytest
+import torch
+import torch.nn as nn
+
+from warpconvnet_b200 import BatchNorm, Sequential, Voxels
+from warpconvnet_b200.nn.functional.batch_norm import batch_norm_act, can_fuse
+
+from conftest import rel_l2
+
+pytestmark = pytest.mark.gpu
+DEV = "cuda:0"
+TOL = {torch.float32: 4e-6, torch.float16: 2e-3, torch.bfloat16: 1.5e-2}
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.float16, torch.bfloat16])
+@pytest.mark.parametrize("n,c", [(2, 8), (3, 1024), (1000, 24), (4097, 64), (50001, 96), (30000, 256)])
+@pytest.mark.parametrize("relu,with_res", [(False, False), (True, False), (True, True), (False, True)])
+def test_matches_separate_layers(dtype, n, c, relu, with_res):
+    g = torch.Generator().manual_seed(n + c)
+    # means far from zero against the spread: the variance must not cancel
+    x0 = (torch.randn(n, c, generator=g) * 0.5 + torch.randn(c, generator=g) * 3).to(dtype).to(DEV)
+    r0 = torch.randn(n, c, generator=g).to(dtype).to(DEV) if with_res else None
+    dy = torch.randn(n, c, generator=g).to(dtype).to(DEV)
+
+    def build():
+        torch.manual_seed(1)
+        bn = nn.BatchNorm1d(c).to(DEV)
+        with torch.no_grad():
+            bn.weight.copy_(torch.rand(c, generator=torch.Generator().manual_seed(2)) + 0.5)
+            bn.bias.copy_(torch.randn(c, generator=torch.Generator().manual_seed(3)))
+        return bn, x0.clone().requires_grad_(True), r0.clone().requires_grad_(True) if with_res else None
+
+    bn, x, r = build()
+    assert can_fuse(bn, x)
+    y = batch_norm_act(x, bn, relu, r)
+    y.backward(dy)
+    ref, xr, rr = build()
+    if dtype == torch.float32:  # against fp64
+        ref, xr, rr = ref.double(), xr.detach().double().requires_grad_(True), rr.detach().double().requires_grad_(True) if with_res else None
+    z = ref(xr)
+    z = z + rr if with_res else z
+    z = torch.relu(z) if relu else z
+    z.backward(dy.to(z.dtype))
+    tol = TOL[dtype] * (20 if n < 10 else 1)  # a handful of rows: 1 / std amplifies every rounding
+    if relu and dtype == torch.float32:
+        tol = 2e-3  # values within a rounding of zero fall on the other side of the ReLU
+
+    def close(a, b):
+        return rel_l2(a.detach().double().cpu().numpy(), b.detach().double().cpu().numpy()) < tol
+    assert close(y, z) and close(bn.weight.grad, ref.weight.grad) and close(bn.bias.grad, ref.bias.grad)
+    assert n < 10 or close(x.grad, xr.grad)
+    assert not with_res or close(r.grad, rr.grad)
+    assert close(bn.running_mean, ref.running_mean) and close(bn.running_var, ref.running_var)
+    assert int(bn.num_batches_tracked) == 1 and bn.running_mean._version > 0
+    again = batch_norm_act(x0, build()[0], relu, r0)
+    assert torch.equal(again, y)  # the same bits on every run
+
+
+def test_sequential_trains_through_the_fused_layers_and_second_derivatives_work():
+    n, c = 500, 16
+    vox = Voxels(torch.arange(3 * n, dtype=torch.int32, device=DEV).view(n, 3), torch.randn(n, c, device=DEV), offsets=torch.tensor([0, n]))
+    seq = Sequential(BatchNorm(c), nn.ReLU()).to(DEV).train()
+    x = torch.randn(n, c, device=DEV, requires_grad=True)
+    y = seq(vox.replace(batched_features=x)).feature_tensor
+    assert "BatchNormAct" in type(y.grad_fn).__name__
+    (gx,) = torch.autograd.grad((y ** 2).sum(), [x], create_graph=True)
+    (ggx,) = torch.autograd.grad(gx.sum() + (gx ** 2).sum(), [x])
+    xr = x.detach().clone().requires_grad_(True)
+    yr = torch.relu(nn.functional.batch_norm(xr, None, None, seq[0].norm.weight, seq[0].norm.bias, True))
+    (gr,) = torch.autograd.grad((yr ** 2).sum(), [xr], create_graph=True)
+    (ggr,) = torch.autograd.grad(gr.sum() + (gr ** 2).sum(), [xr])
+    assert rel_l2(gx.detach().cpu().numpy(), gr.detach().cpu().numpy()) < 1e-4
+    assert rel_l2(ggx.cpu().numpy(), ggr.cpu().numpy()) < 1e-3

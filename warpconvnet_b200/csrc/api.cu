@@ -29,7 +29,8 @@ int wcn_conv_fp32_fwd(const void* feats, int64_t num_in, int64_t feats_ld, const
 // conv_tcgen05.cu
 bool wcn_conv_tcgen05_supported(int K, int c_in, int c_out, int dtype, int out_dtype);
 int64_t wcn_conv_tcgen05_packed_bytes(int K, int c_in, int c_out);
-int wcn_conv_tcgen05_pack(const void* weight, int K, int c_in, int c_out, void* packed, cudaStream_t st);
+int wcn_conv_tcgen05_pack(const void* weight, int src_dtype, int K, int c_in, int c_out, int dtype, int transposed, int reversed,
+                          void* packed, cudaStream_t st);
 int wcn_conv_tcgen05_fwd(const void* feats, int64_t num_in, int64_t feats_ld, const void* packed, const int32_t* nbr,
                          const int32_t* out_rows, int64_t M, int K, int c_in, int c_out, int dtype,
                          const float* scale, const float* shift, const void* residual, int64_t residual_ld, int relu,
@@ -76,7 +77,14 @@ extern "C" int wcn_conv_pack_weight(int algo, const void* weight, int32_t num_of
   if (!weight || !packed) return WCN_ERR_INVALID_PARAMETERS;
   if (algo == WCN_CONV_SIMT || !wcn_conv_tcgen05_supported(num_offsets, c_in, c_out, dtype, dtype))
     return WCN_ERR_UNSUPPORTED_CONFIG;
-  return wcn_conv_tcgen05_pack(weight, num_offsets, c_in, c_out, packed, wcn_stream(stream));
+  return wcn_conv_tcgen05_pack(weight, dtype, num_offsets, c_in, c_out, dtype, 0, 0, packed, wcn_stream(stream));
+}
+
+extern "C" int wcn_conv_pack_weight_from(const void* weight, int src_dtype, int32_t num_offsets, int32_t c_in, int32_t c_out,
+                                         int dtype, int32_t transposed, int32_t reversed, void* packed, void* stream) {
+  if (!weight || !packed || (reinterpret_cast<uintptr_t>(packed) & 15)) return WCN_ERR_INVALID_PARAMETERS;
+  if (!wcn_conv_tcgen05_supported(num_offsets, c_in, c_out, dtype, dtype)) return WCN_ERR_UNSUPPORTED_CONFIG;
+  return wcn_conv_tcgen05_pack(weight, src_dtype, num_offsets, c_in, c_out, dtype, transposed, reversed, packed, wcn_stream(stream));
 }
 
 static bool conv_takes_tcgen05(int algo, bool tc_ok, const void* packed_weight, const int32_t* dev_status,

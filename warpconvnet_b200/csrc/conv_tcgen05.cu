@@ -748,25 +748,36 @@ conv_tcgen05_kernel(const ConvTcParams p) {
   if (warp == MMA_WARP) tmem_dealloc(tmem_base, tmem_total < 32 ? 32u : tmem_total);
 }
 
-// weight[K, c_in, c_out] -> packed[K][c_in/BK] tiles of [c_out][BK]: every (offset, channel
-// slice) becomes one contiguous K-major tile stored as its swizzled shared-memory image
-// (the layout of tile_offset above), so the kernel moves it with a single bulk copy.
-template <typename T>
-__global__ void pack_weight_kernel(const T* __restrict__ w, T* __restrict__ packed, int K, int c_in, int c_out,
-                                   int bk) {
-  const int64_t total = (int64_t)K * c_in * c_out;
+// weight -> packed[K][c_in/BK] tiles of [c_out][BK]: every (offset, channel slice) becomes one contiguous K-major tile
+// stored as its swizzled shared-memory image (the layout of tile_offset above), so the kernel moves it with a single bulk
+// copy.  A thread makes one 16-byte chunk: eight input channels of one output channel.  The source may have another
+// dtype, be transposed per offset ([K, c_out, c_in]) and hold the offsets in reverse order: what a training step needs
+// of its fp32 weights each time they change, without a cast or a transposed copy in between.
+template <typename TS, typename TD>
+__global__ void pack_weight_kernel(const TS* __restrict__ w, TD* __restrict__ packed, int K, int c_in, int c_out, int bk,
+                                   int transposed, int reversed) {
+  const int64_t total = (int64_t)K * (c_in / 8) * c_out;
   const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= total) return;
-  const int n = (int)(i % c_out);
-  int64_t r = i / c_out;
-  const int cin = (int)(r % c_in);
-  const int k = (int)(r / c_in);
+  // consecutive threads run along the dimension that is contiguous in the source
+  int n, c8;
+  int64_t r;
+  if (transposed) { c8 = (int)(i % (c_in / 8)); r = i / (c_in / 8); n = (int)(r % c_out); r /= c_out; }
+  else { n = (int)(i % c_out); r = i / c_out; c8 = (int)(r % (c_in / 8)); r /= c_in / 8; }
+  const int k = (int)r, cin = c8 * 8;
+  const int64_t ks = reversed ? K - 1 - k : k;
+  __align__(16) TD v[8];
+#pragma unroll
+  for (int u = 0; u < 8; ++u) {
+    const int64_t at = transposed ? (ks * c_out + n) * c_in + cin + u : (ks * c_in + cin + u) * c_out + n;
+    v[u] = wcn_from_float<TD>(wcn_to_float<TS>(w[at]));
+  }
   const int kb = cin / bk, c = cin % bk;
-  const int rb = bk * 2, chunk = c >> 3, within = c & 7, r8 = n & 7;
+  const int rb = bk * 2, chunk = c >> 3, r8 = n & 7;
   const int x = rb == 128 ? r8 : (r8 >> 1);
   const int64_t tile = ((int64_t)k * (c_in / bk) + kb) * c_out * bk;  // elements
   const int64_t off_bytes = (int64_t)(n >> 3) * (8 * rb) + r8 * rb + ((chunk ^ x) << 4);
-  packed[tile + off_bytes / 2 + within] = w[i];
+  *reinterpret_cast<uint4*>(packed + tile + off_bytes / 2) = *reinterpret_cast<const uint4*>(v);
 }
 
 inline int pick_bk(int c_in) { return c_in % 64 == 0 ? 64 : 32; }
@@ -943,12 +954,25 @@ bool wcn_conv_tcgen05_supported(int K, int c_in, int c_out, int dtype, int out_d
 
 int64_t wcn_conv_tcgen05_packed_bytes(int K, int c_in, int c_out) { return (int64_t)K * c_in * c_out * 2; }
 
-int wcn_conv_tcgen05_pack(const void* weight, int K, int c_in, int c_out, void* packed, cudaStream_t st) {
-  const int64_t total = (int64_t)K * c_in * c_out;
+int wcn_conv_tcgen05_pack(const void* weight, int src_dtype, int K, int c_in, int c_out, int dtype, int transposed, int reversed,
+                          void* packed, cudaStream_t st) {
+  const int64_t total = (int64_t)K * (c_in / 8) * c_out;
   if (total == 0) return WCN_OK;
-  pack_weight_kernel<uint16_t><<<(unsigned)((total + 255) / 256), 256, 0, st>>>(
-      (const uint16_t*)weight, (uint16_t*)packed, K, c_in, c_out, pick_bk(c_in));
-  return cudaGetLastError() == cudaSuccess ? WCN_OK : WCN_ERR_EXECUTION;
+  const unsigned grid = (unsigned)((total + 255) / 256);
+#define WCN_PACK_CASE(SD, TS, DD, TD)                                                                                    \
+  if (src_dtype == SD && dtype == DD) {                                                                                  \
+    pack_weight_kernel<TS, TD><<<grid, 256, 0, st>>>((const TS*)weight, (TD*)packed, K, c_in, c_out, pick_bk(c_in),       \
+                                                    transposed, reversed);                                               \
+    return cudaGetLastError() == cudaSuccess ? WCN_OK : WCN_ERR_EXECUTION;                                               \
+  }
+  WCN_PACK_CASE(WCN_F32, float, WCN_F16, __half)
+  WCN_PACK_CASE(WCN_F16, __half, WCN_F16, __half)
+  WCN_PACK_CASE(WCN_BF16, __nv_bfloat16, WCN_F16, __half)
+  WCN_PACK_CASE(WCN_F32, float, WCN_BF16, __nv_bfloat16)
+  WCN_PACK_CASE(WCN_F16, __half, WCN_BF16, __nv_bfloat16)
+  WCN_PACK_CASE(WCN_BF16, __nv_bfloat16, WCN_BF16, __nv_bfloat16)
+#undef WCN_PACK_CASE
+  return WCN_ERR_INVALID_PARAMETERS;
 }
 
 int wcn_conv_tcgen05_fwd(const void* feats, int64_t num_in, int64_t feats_ld, const void* packed, const int32_t* nbr,

@@ -54,7 +54,7 @@ __device__ __forceinline__ float4 load4(const T* row, int c, int limit) {
 template <typename T, int TI, int TJ, bool VEC>
 __global__ void __launch_bounds__(THREADS)
 conv_wgrad_pairs_kernel(const PairsParams p) {
-  constexpr int RI = TI == 8 ? 2 : 8;
+  constexpr int RI = 8;
   constexpr int TY = TI / RI, TX = TJ / 4, G = THREADS / (TX * TY);
   constexpr int XQ = P * TI / 4, YQ = P * TJ / 4;              // four-element pieces of a stage
   constexpr int XN = (XQ + THREADS - 1) / THREADS, YN = (YQ + THREADS - 1) / THREADS;
@@ -141,13 +141,8 @@ conv_wgrad_pairs_kernel(const PairsParams p) {
 #pragma unroll 4
       for (int q = g; q < P; q += G) {
         float x[RI];
-        if constexpr (RI == 8) {
-          *reinterpret_cast<float4*>(x) = *reinterpret_cast<const float4*>(&x_s[buf][q][ty * 4]);
-          *reinterpret_cast<float4*>(x + 4) = *reinterpret_cast<const float4*>(&x_s[buf][q][TI / 2 + ty * 4]);
-        } else {
-          x[0] = x_s[buf][q][ty];
-          x[1] = x_s[buf][q][TI / 2 + ty];
-        }
+        *reinterpret_cast<float4*>(x) = *reinterpret_cast<const float4*>(&x_s[buf][q][ty * 4]);
+        *reinterpret_cast<float4*>(x + 4) = *reinterpret_cast<const float4*>(&x_s[buf][q][TI / 2 + ty * 4]);
         const float4 y = *reinterpret_cast<const float4*>(&y_s[buf][q][tx * 4]);
 #pragma unroll
         for (int r = 0; r < RI; ++r) {
@@ -164,7 +159,7 @@ conv_wgrad_pairs_kernel(const PairsParams p) {
   // ---- add the pair groups in order, then leave the tile
   static_assert(TJ <= 2 * P, "a tile fits the X stages");
   float* sum_s = &x_s[0][0][0];
-  auto row_of = [&](int r) { return RI == 8 ? (r < 4 ? ty * 4 + r : TI / 2 + ty * 4 + r - 4) : (r == 0 ? ty : TI / 2 + ty); };
+  auto row_of = [&](int r) { return r < 4 ? ty * 4 + r : TI / 2 + ty * 4 + r - 4; };
   if constexpr (G > 1) {
     for (int from = 1; from < G; ++from) {  // one group at a time through one tile of shared memory
       __syncthreads();
@@ -197,6 +192,62 @@ conv_wgrad_pairs_kernel(const PairsParams p) {
   if (bad) wcn_report_bounds(p.dev_status);
 }
 
+// Up to CI = 8 input channels (a network's stem): the work is reading one dY row per pair, so a warp takes 32 rows of the
+// table, walks those that have a neighbour and keeps CI sums per output channel (lane); four pairs' rows are in flight.
+// (240 000 rows, 3 -> 32 channels, 27 offsets: the staged tile kernel above took 188 us, bound by shared memory.)
+constexpr int NARROW_THREADS = 256;
+
+template <typename T, int CI>
+__global__ void __launch_bounds__(NARROW_THREADS)
+conv_wgrad_narrow_kernel(const PairsParams p) {
+  __shared__ float part[NARROW_THREADS / 32][CI][32];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int k = blockIdx.y, j = blockIdx.z * 32 + lane;
+  const bool col = j < p.c_out;
+  const T* feats = reinterpret_cast<const T*>(p.feats);
+  const T* gout = reinterpret_cast<const T*>(p.gout) + (col ? j : 0);
+  const int64_t begin = (int64_t)blockIdx.x * p.rows_per_range, end = min(p.M, begin + p.rows_per_range);
+  float acc[CI];
+#pragma unroll
+  for (int c = 0; c < CI; ++c) acc[c] = 0.f;
+  bool bad = false;
+  for (int64_t base = begin + warp * 32; base < end; base += NARROW_THREADS) {
+    const int64_t m = base + lane;
+    int src = m < end ? __ldg(&p.nbr[(int64_t)k * p.M + m]) : -1;
+    if (src >= p.num_in) { src = -1; bad = true; }
+    uint32_t rest = __ballot_sync(0xFFFFFFFFu, src >= 0);
+    int row = (int)m;
+    if (p.out_rows && src >= 0) row = __ldg(&p.out_rows[m]);
+    while (rest) {
+      float g[4], x[4][CI];
+#pragma unroll
+      for (int u = 0; u < 4; ++u) {
+        const bool have = rest != 0;
+        const int b = have ? __ffs(rest) - 1 : 0;
+        rest &= rest - 1;
+        const int s = __shfl_sync(0xFFFFFFFFu, src, b), r = __shfl_sync(0xFFFFFFFFu, row, b);
+        g[u] = have && col ? wcn_to_float<T>(gout[(int64_t)r * p.c_out]) : 0.f;
+#pragma unroll
+        for (int c = 0; c < CI; ++c) x[u][c] = have && c < p.c_in ? wcn_to_float<T>(feats[(int64_t)s * p.c_in + c]) : 0.f;
+      }
+#pragma unroll
+      for (int u = 0; u < 4; ++u)
+#pragma unroll
+        for (int c = 0; c < CI; ++c) acc[c] = fmaf(x[u][c], g[u], acc[c]);
+    }
+  }
+#pragma unroll
+  for (int c = 0; c < CI; ++c) part[warp][c][lane] = acc[c];
+  __syncthreads();
+  for (int i = threadIdx.x; i < CI * 32; i += NARROW_THREADS) {
+    const int c = i / 32, n = blockIdx.z * 32 + (i & 31);
+    float v = part[0][c][i & 31];
+    for (int w = 1; w < NARROW_THREADS / 32; ++w) v += part[w][c][i & 31];
+    if (c < p.c_in && n < p.c_out) p.dst[(((int64_t)blockIdx.x * p.K + k) * p.c_in + c) * p.c_out + n] = v;
+  }
+  if (bad) wcn_report_bounds(p.dev_status);
+}
+
 __global__ void sum_ranges_kernel(const float* __restrict__ partial, int ranges, int64_t n, float* __restrict__ out) {
   const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n) return;
@@ -214,8 +265,8 @@ struct PairsPlan {
 // About eight blocks per multiprocessor, none with fewer than one list of rows.
 PairsPlan plan_pairs(int64_t M, int K, int c_in, int c_out) {
   PairsPlan q;
-  q.ti = c_in <= 8 ? 8 : c_in <= 32 ? 32 : 64;
-  q.tj = c_out <= 32 ? 32 : 64;
+  q.ti = c_in <= 8 ? 8 : c_in <= 32 ? 32 : 64;   // 8: the narrow kernel, 32 columns a block
+  q.tj = c_out <= 32 || q.ti == 8 ? 32 : 64;
   q.tiles_i = (c_in + q.ti - 1) / q.ti;
   q.tiles_j = (c_out + q.tj - 1) / q.tj;
   const int64_t blocks = (int64_t)K * q.tiles_i * q.tiles_j;
@@ -231,12 +282,17 @@ PairsPlan plan_pairs(int64_t M, int K, int c_in, int c_out) {
 template <typename T, bool VEC>
 int launch_pairs(const PairsParams& p, const PairsPlan& q, cudaStream_t st) {
   dim3 grid((unsigned)q.ranges, (unsigned)p.K, (unsigned)(q.tiles_i * q.tiles_j));
+  if (q.ti == 8) {
+    if (p.c_in <= 4) conv_wgrad_narrow_kernel<T, 4><<<grid, NARROW_THREADS, 0, st>>>(p);
+    else conv_wgrad_narrow_kernel<T, 8><<<grid, NARROW_THREADS, 0, st>>>(p);
+    return cudaGetLastError() == cudaSuccess ? WCN_OK : WCN_ERR_EXECUTION;
+  }
 #define WCN_PAIRS_CASE(TI, TJ)                                                                       \
   if (q.ti == TI && q.tj == TJ) {                                                                    \
     conv_wgrad_pairs_kernel<T, TI, TJ, VEC><<<grid, THREADS, 0, st>>>(p);                            \
     return cudaGetLastError() == cudaSuccess ? WCN_OK : WCN_ERR_EXECUTION;                           \
   }
-  WCN_PAIRS_CASE(8, 32) WCN_PAIRS_CASE(8, 64) WCN_PAIRS_CASE(32, 32) WCN_PAIRS_CASE(32, 64) WCN_PAIRS_CASE(64, 32) WCN_PAIRS_CASE(64, 64)
+  WCN_PAIRS_CASE(32, 32) WCN_PAIRS_CASE(32, 64) WCN_PAIRS_CASE(64, 32) WCN_PAIRS_CASE(64, 64)
 #undef WCN_PAIRS_CASE
   return WCN_ERR_UNSUPPORTED_CONFIG;
 }

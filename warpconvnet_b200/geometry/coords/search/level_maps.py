@@ -52,6 +52,7 @@ class PyramidBuild:
         raise_for_status(host[-1], self.device)
         if not host[-2]:
             return None
+        self.ic._shared.setdefault("facts", {})["distinct"] = True
         levels = []
         for l in range(PYRAMID_LEVELS):
             offs = host[l * nb:(l + 1) * nb]
@@ -61,7 +62,7 @@ class PyramidBuild:
             c.offsets.__dict__["_wcn_tuple"] = tuple(offs)  # the form kernel-map cache keys want
             c.batched_tensor = rows[:, 1:]
             c.voxel_size = c.voxel_origin = c.tensor_stride = None
-            c._shared = {"bcoords": rows, "morton_origin": self.counts[8 + 4 * l:11 + 4 * l]}
+            c._shared = {"bcoords": rows, "morton_origin": self.counts[8 + 4 * l:11 + 4 * l], "facts": {"distinct": True}}
             levels.append(c)
         return levels
 

@@ -1,0 +1,103 @@
+"""Training-mode BatchNorm of feature rows with the residual addition and the ReLU that follow it, two native launches
+per direction (``csrc/batch_norm.cu``).  An addition to the reference, whose blocks run ``nn.BatchNorm1d``, the addition
+and ``nn.ReLU`` one after the other (examples/mink_unet.py:36-47, 129-141); values are rounded where those round."""
+from __future__ import annotations
+
+from typing import Optional
+
+import torch
+import torch.nn as nn
+from torch import Tensor
+
+from ..._native import check, dtype_code, lib, ptr, query_bytes, stream_ptr
+
+_DTYPES = (torch.float32, torch.float16, torch.bfloat16)
+_counters: dict = {}
+
+
+def _counter(device: torch.device, stream: int) -> Tensor:
+    """The block counter of the reductions: zero between launches of one stream."""
+    key = (device.index, stream)
+    hit = _counters.get(key)
+    if hit is None:
+        if len(_counters) >= 256:  # streams come and go; a counter is 4 bytes
+            torch.cuda.synchronize(device)
+            _counters.clear()
+        hit = _counters[key] = torch.zeros(1, dtype=torch.int32, device=device)
+    return hit
+
+
+def can_fuse(bn: nn.Module, x: Tensor) -> bool:
+    """Whether ``batch_norm_act`` computes what ``bn(x)`` would (training mode, running statistics kept)."""
+    if type(bn) is not nn.BatchNorm1d or not bn.training or not bn.track_running_stats or bn.momentum is None:
+        return False
+    if not x.is_cuda or x.dtype not in _DTYPES or x.dim() != 2 or not x.is_contiguous() or x.shape[0] < 2:
+        return False
+    if bn._forward_hooks or bn._forward_pre_hooks or bn._backward_hooks or bn._backward_pre_hooks:
+        return False
+    c = x.shape[1]
+    per16 = 16 // x.element_size()
+    return (c == bn.num_features and c % per16 == 0 and c <= 1024 and x.data_ptr() % 16 == 0
+            and bn.running_mean.dtype == torch.float32 and bn.running_mean.device == x.device
+            and (bn.weight is None or bn.weight.dtype == torch.float32) and (bn.bias is None or bn.bias.dtype == torch.float32))
+
+
+class _BatchNormAct(torch.autograd.Function):
+    @staticmethod
+    def forward(ctx, x: Tensor, gamma: Optional[Tensor], beta: Optional[Tensor], residual: Optional[Tensor], bn, relu: bool):
+        n, c = x.shape
+        dev, dc, st = x.device, dtype_code(x.dtype), stream_ptr(x.device)
+        y = torch.empty_like(x)
+        saved = torch.empty((2, c), dtype=torch.float32, device=dev)
+        ws = torch.empty(query_bytes("wcn_batch_norm_workspace_bytes", n, c, dc), dtype=torch.uint8, device=dev)
+        at = saved.data_ptr()
+        check(lib().wcn_batch_norm_train(ptr(x), n, c, dc, ptr(gamma), ptr(beta), _bits(bn.eps), _bits(bn.momentum),
+                                         ptr(bn.running_mean), ptr(bn.running_var), ptr(bn.num_batches_tracked), ptr(residual),
+                                         int(relu), ptr(y), at, at + 4 * c, ptr(ws), ptr(_counter(dev, st)), st),
+              "wcn_batch_norm_train")
+        torch.autograd.graph.increment_version([bn.running_mean, bn.running_var, bn.num_batches_tracked])
+        ctx.relu, ctx.eps = relu, bn.eps
+        ctx.save_for_backward(x, gamma, beta, residual, saved, y if relu and residual is not None else None)
+        return y
+
+    @staticmethod
+    def backward(ctx, dy: Tensor):
+        x, gamma, beta, residual, saved, y = ctx.saved_tensors
+        if torch.is_grad_enabled():  # a graph of the gradient is wanted: the same formulas through torch
+            z = torch.nn.functional.batch_norm(x, None, None, gamma, beta, True, 0.0, ctx.eps)
+            z = z if residual is None else z + residual
+            z = torch.relu(z) if ctx.relu else z
+            wanted = [t for t, need in zip((x, gamma, beta, residual), ctx.needs_input_grad) if need]
+            got = iter(torch.autograd.grad(z, wanted, dy, create_graph=True))
+            return tuple(next(got) if need else None for need in ctx.needs_input_grad[:4]) + (None, None)
+        n, c = x.shape
+        dev, dc, st = x.device, dtype_code(x.dtype), stream_ptr(x.device)
+        dy = dy.contiguous()
+        need_x, _, _, need_res = ctx.needs_input_grad[:4]
+        want_res = need_res and ctx.relu
+        dx = torch.empty_like(x) if need_x or want_res else None
+        dres = torch.empty_like(x) if want_res else None
+        sums = torch.empty((2, c), dtype=torch.float32, device=dev)
+        ws = torch.empty(query_bytes("wcn_batch_norm_workspace_bytes", n, c, dc), dtype=torch.uint8, device=dev)
+        at = saved.data_ptr()
+        check(lib().wcn_batch_norm_backward(ptr(x), ptr(dy), ptr(y), n, c, dc, ptr(gamma), ptr(beta), at, at + 4 * c,
+                                            int(ctx.relu), ptr(dx), ptr(dres), ptr(sums), ptr(ws), ptr(_counter(dev, st)), st),
+              "wcn_batch_norm_backward")
+        return (dx if need_x else None, sums[1] if ctx.needs_input_grad[1] else None,
+                sums[0] if ctx.needs_input_grad[2] else None, (dres if ctx.relu else dy) if need_res else None, None, None)
+
+
+def _bits(value: float) -> int:
+    """A float argument as the 32 bits the C function reinterprets (calls pass integers only)."""
+    import struct
+    return struct.unpack("<I", struct.pack("<f", value))[0]
+
+
+def batch_norm_act(x: Tensor, bn: nn.BatchNorm1d, relu: bool = False, residual: Optional[Tensor] = None) -> Tensor:
+    """``relu(bn(x) + residual)`` of a training step (see :func:`can_fuse`)."""
+    if residual is not None:
+        assert residual.shape == x.shape, f"residual {tuple(residual.shape)} != {tuple(x.shape)}"
+        residual = residual.to(x.dtype).contiguous()
+        if residual.data_ptr() % 16:
+            residual = residual.clone()
+    return _BatchNormAct.apply(x, bn.weight, bn.bias, residual, bn, relu)

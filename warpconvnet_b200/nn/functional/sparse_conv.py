@@ -154,26 +154,46 @@ def _explicit_gemm_forward_logic(in_features: Tensor, weight: Tensor, kernel_map
     return out.to(dtype=in_features.dtype)
 
 
-def _prepared_weight(weight: Tensor, dtype: torch.dtype, algo: int = CONV_AUTO):
-    """(weight in ``dtype``, its re-tiled copy for the tensor-core kernel or None).
+def _cast_weight(weight: Tensor, dtype: torch.dtype, transposed: bool = False, reversed_: bool = False) -> Tensor:
+    """``weight`` (per offset transposed, offsets reversed) as a contiguous tensor of ``dtype``."""
+    w = weight.detach()
+    if transposed:
+        w = w.transpose(1, 2)
+    if reversed_:
+        w = w.flip(0)
+    return w.to(dtype=dtype).contiguous()
 
+
+def _prepared_weight(weight: Tensor, dtype: torch.dtype, algo: int = CONV_AUTO, transposed: bool = False,
+                     reversed_: bool = False):
+    """(weight in ``dtype`` or None, its re-tiled copy for the tensor-core kernel or None): one of the two.
+
+    ``transposed``: of each offset's transpose, ``reversed_``: of the offsets in reverse order (a gradient's weights).
     Both are cached ON the weight tensor object, tagged with its version counter,
     so an inference loop casts and re-tiles a parameter once and a parameter
-    update invalidates the copy."""
+    update invalidates the copy; the re-tiling kernel reads the parameter as it is."""
     store = weight.__dict__.setdefault("_wcn_prepared", {})
-    hit = store.get((dtype, algo))
-    if hit is not None and hit[0] == weight._version and hit[1].device == weight.device:
+    key, tag = (dtype, algo, transposed, reversed_), (weight._version, weight.data_ptr())
+    hit = store.get(key)
+    if hit is not None and hit[0] == tag:
         return hit[1], hit[2]
-    w = weight.detach().to(dtype=dtype).contiguous()
-    K, c_in, c_out = w.shape
-    packed = None
-    if algo != CONV_SIMT and w.is_cuda:
+    K, c_in, c_out = weight.shape
+    if transposed:
+        c_in, c_out = c_out, c_in
+    w = packed = None
+    if algo != CONV_SIMT and weight.is_cuda and dtype in _NATIVE_DTYPES:
         nbytes = query_bytes("wcn_conv_packed_weight_bytes", algo, K, c_in, c_out, dtype_code(dtype))
         if nbytes > 0:
-            packed = torch.empty(nbytes, dtype=torch.uint8, device=w.device)
-            check(lib().wcn_conv_pack_weight(algo, ptr(w), K, c_in, c_out, dtype_code(dtype), ptr(packed),
-                                             stream_ptr(w.device)), "wcn_conv_pack_weight")
-    store[(dtype, algo)] = (weight._version, w, packed)
+            packed = torch.empty(nbytes, dtype=torch.uint8, device=weight.device)
+            src = weight.detach()
+            if src.dtype not in _NATIVE_DTYPES or not src.is_contiguous():
+                src = src.to(dtype=dtype).contiguous()
+            check(lib().wcn_conv_pack_weight_from(ptr(src), dtype_code(src.dtype), K, c_in, c_out, dtype_code(dtype),
+                                                  int(transposed), int(reversed_), ptr(packed), stream_ptr(weight.device)),
+                  "wcn_conv_pack_weight_from")
+    if packed is None:
+        w = _cast_weight(weight, dtype, transposed, reversed_)
+    store[key] = (tag, w, packed)
     return w, packed
 
 
@@ -198,17 +218,19 @@ def _row_view(t: Tensor) -> Tensor:
 
 def sparse_conv_fused(in_features: Tensor, weight: Tensor, kernel_map: IntSearchResult, num_out_coords: int,
                       epilogue: Optional[ConvEpilogue] = None, out_dtype: Optional[torch.dtype] = None,
-                      algo: int = CONV_AUTO, tile_order: Optional[bool] = None, split_k: int = 0) -> Tensor:
+                      algo: int = CONV_AUTO, tile_order: Optional[bool] = None, split_k: int = 0,
+                      transpose_weight: bool = False, reverse_weight: bool = False) -> Tensor:
     """One launch: all kernel offsets + epilogue.  The weight is used in the
     feature dtype (fp32, fp16 or bf16); accumulation is fp32.  ``tile_order`` runs the
     output rows grouped by neighbour pattern (``IntSearchResult.tiled_neighbor_table``;
     same numbers, fewer (tile, offset) pairs to compute); None = by size.  ``split_k``
     (the reference's ``split_k_slices``): 0 lets the library divide the kernel offsets of
     small problems among CTAs, 1 forbids it, 2 and more ask for that many slices (at most 8).  Features,
-    residual and ``epilogue.out`` may be column blocks of wider matrices."""
+    residual and ``epilogue.out`` may be column blocks of wider matrices.  ``transpose_weight`` / ``reverse_weight``: run
+    with each offset's weight transposed / with the offsets in reverse order (the input gradient's weights)."""
     require_cuda(in_features, "in_features")
     x = _row_view(in_features)
-    if algo == CONV_AUTO and split_k == 0 and not tile_order and num_out_coords > 0:
+    if algo == CONV_AUTO and split_k == 0 and not tile_order and num_out_coords > 0 and not reverse_weight:
         # one (input row, offset) pair per output row: the input-side kernel, when it takes the call
         ep0 = epilogue or ConvEpilogue()
         done = None
@@ -218,14 +240,18 @@ def sparse_conv_fused(in_features: Tensor, weight: Tensor, kernel_map: IntSearch
                 dst = ep0.out_rows.to(device=x.device, dtype=torch.int32).view(1, -1).contiguous()
                 ep0 = ConvEpilogue(ep0.scale, ep0.shift, None, ep0.relu, None, ep0.out)
             if ep0.out_rows is None:
-                done = sparse_conv_rows_fused(x, weight, dst, num_out_coords, ep0, out_dtype)
+                done = sparse_conv_rows_fused(x, weight, dst, num_out_coords, ep0, out_dtype, transpose_weight)
         elif getattr(kernel_map, "_one_pair", False) and ep0.out_rows is None and kernel_map._forward is not None:
             done = sparse_conv_rows_fused(x, weight, kernel_map._forward.neighbor_table(x.shape[0]), num_out_coords,
-                                          ep0, out_dtype)
+                                          ep0, out_dtype, transpose_weight)
         if done is not None:
             return done
-    w, packed = _prepared_weight(weight, x.dtype, algo)
-    K, c_in, c_out = w.shape
+    w, packed = _prepared_weight(weight, x.dtype, algo, transpose_weight, reverse_weight)
+    if w is None and x.shape[0] == 0:  # no row to multiply: the kernel for that case reads plain weights
+        w = _cast_weight(weight, x.dtype, transpose_weight, reverse_weight)
+    K, c_in, c_out = weight.shape
+    if transpose_weight:
+        c_in, c_out = c_out, c_in
     assert x.shape[1] == c_in, f"features have {x.shape[1]} channels, weight expects {c_in}"
     dev = x.device
     ep = epilogue or ConvEpilogue()
@@ -289,11 +315,11 @@ class FusedConvLaunch:
     def __init__(self, weight: Tensor, dtype: torch.dtype, scale: Optional[Tensor] = None,
                  shift: Optional[Tensor] = None, relu: bool = False):
         w, packed = _prepared_weight(weight, dtype, CONV_AUTO)
-        dev = w.device
+        dev = weight.device
         self.weight, self.packed = w, packed
         self.scale, self.shift = _as_f32_on(scale, dev), _as_f32_on(shift, dev)
         self.relu = int(bool(relu))
-        self.K, self.c_in, self.c_out = (int(v) for v in w.shape)
+        self.K, self.c_in, self.c_out = (int(v) for v in weight.shape)
         self.dtype, self.device, self._dc = dtype, dev, dtype_code(dtype)
         self._w_ptr, self._packed_ptr = ptr(w), ptr(packed)
         self._scale_ptr, self._shift_ptr = ptr(self.scale), ptr(self.shift)
@@ -307,7 +333,10 @@ class FusedConvLaunch:
             out = torch.empty((num_out, self.c_out), dtype=self.dtype, device=self.device)
         if num_out == 0:
             return out
-        rc = self._fn(CONV_AUTO, feats.data_ptr(), feats.shape[0], feats.stride(0), self._w_ptr, self._packed_ptr,
+        w_ptr = self._w_ptr
+        if w_ptr is None and feats.shape[0] == 0:
+            raise ValueError("a launch record needs at least one input row")
+        rc = self._fn(CONV_AUTO, feats.data_ptr(), feats.shape[0], feats.stride(0), w_ptr, self._packed_ptr,
                       nbr.data_ptr(), out_rows.data_ptr() if out_rows is not None else None, num_out, self.K,
                       self.c_in, self.c_out, self._dc, self._scale_ptr, self._shift_ptr,
                       residual.data_ptr() if residual is not None else None,
@@ -318,32 +347,36 @@ class FusedConvLaunch:
         return out
 
 
-def _prepared_rows_weight(weight: Tensor, dtype: torch.dtype):
+def _prepared_rows_weight(weight: Tensor, dtype: torch.dtype, transposed: bool = False):
     """``(packed, c_out_packed)``: the weight re-tiled for the input-side kernel at a width padded to a
     multiple of 16 columns (extra columns zero), or ``(None, 0)`` when that kernel does not take the
     shape.  Cached on the weight tensor like :func:`_prepared_weight`."""
     store = weight.__dict__.setdefault("_wcn_prepared", {})
-    hit = store.get((dtype, "rows"))
-    if hit is not None and hit[0] == weight._version and hit[3] == weight.device:
+    key, tag = (dtype, "rows", transposed), (weight._version, weight.data_ptr())
+    hit = store.get(key)
+    if hit is not None and hit[0] == tag:
         return hit[1], hit[2]
     packed, c_pack = None, 0
     if weight.is_cuda and dtype in (torch.float16, torch.bfloat16):
         K, c_in, c_out = (int(v) for v in weight.shape)
+        if transposed:
+            c_in, c_out = c_out, c_in
         width = -(-c_out // 16) * 16
         dc = dtype_code(dtype)
         yes = ctypes.c_int32(0)
         check(lib().wcn_conv_rows_supported(K, c_in, width, dc, dc, ctypes.addressof(yes)), "wcn_conv_rows_supported")
         if yes.value:
-            w = weight.detach().to(dtype=dtype)
+            w = weight.detach()
             if width != c_out:
-                w = torch.nn.functional.pad(w, (0, width - c_out))
-            w = w.contiguous()
+                w, transposed = torch.nn.functional.pad(_cast_weight(w, dtype, transposed), (0, width - c_out)), False
+            elif w.dtype not in _NATIVE_DTYPES or not w.is_contiguous():
+                w = w.to(dtype=dtype).contiguous()
             nbytes = query_bytes("wcn_conv_packed_weight_bytes", CONV_AUTO, K, c_in, width, dc)
             if nbytes > 0:
                 packed, c_pack = torch.empty(nbytes, dtype=torch.uint8, device=w.device), width
-                check(lib().wcn_conv_pack_weight(CONV_AUTO, ptr(w), K, c_in, width, dc, ptr(packed), stream_ptr(w.device)),
-                      "wcn_conv_pack_weight")
-    store[(dtype, "rows")] = (weight._version, packed, c_pack, weight.device)
+                check(lib().wcn_conv_pack_weight_from(ptr(w), dtype_code(w.dtype), K, c_in, width, dc, int(transposed), 0,
+                                                      ptr(packed), stream_ptr(w.device)), "wcn_conv_pack_weight_from")
+    store[key] = (tag, packed, c_pack)
     return packed, c_pack
 
 
@@ -356,7 +389,7 @@ def _tma_rows_ok(x: Tensor) -> bool:
 
 def sparse_conv_rows_fused(in_features: Tensor, weight: Tensor, dst_rows: Optional[Tensor], num_out_coords: int,
                            epilogue: Optional[ConvEpilogue] = None,
-                           out_dtype: Optional[torch.dtype] = None) -> Optional[Tensor]:
+                           out_dtype: Optional[torch.dtype] = None, transpose_weight: bool = False) -> Optional[Tensor]:
     """A convolution in which every output row has exactly one (input row, offset) pair, run from
     the input side (``wcn_conv_rows_fwd``): ``out[dst_rows[k, j]] = epilogue(in_features[j] @ weight[k])``.
     ``dst_rows`` is int32 ``[K, N_in]`` (entries < 0: no such pair) — for a 2x2x2 stride-2 transposed
@@ -369,10 +402,12 @@ def sparse_conv_rows_fused(in_features: Tensor, weight: Tensor, dst_rows: Option
     ep = epilogue or ConvEpilogue()
     if x.dtype not in (torch.float16, torch.bfloat16) or not _tma_rows_ok(x) or ep.out_rows is not None:
         return None
-    packed, c_pack = _prepared_rows_weight(weight, x.dtype)
+    packed, c_pack = _prepared_rows_weight(weight, x.dtype, transpose_weight)
     if packed is None:
         return None
     K, c_in, c_out = (int(v) for v in weight.shape)
+    if transpose_weight:
+        c_in, c_out = c_out, c_in
     assert x.shape[1] == c_in, f"features have {x.shape[1]} channels, weight expects {c_in}"
     dev = x.device
     out_dtype = out_dtype or (ep.out.dtype if ep.out is not None else x.dtype)
@@ -568,6 +603,12 @@ def generate_output_coords_and_kernel_map(input_sparse_tensor: Voxels, kernel_si
                                                  hashtable=_cached_table(input_sparse_tensor, in_coords),
                                                  bricks=_cached_bricks(input_sparse_tensor, in_coords))
 
+        if not generative and output_spatially_sparse_tensor is None and order == POINT_ORDERING.RANDOM:
+            if all(s == 1 for s in stride):
+                kernel_map._onto_itself = all(k % 2 == 1 for k in kernel_size)
+                kernel_map._facts = input_sparse_tensor.batched_coordinates._shared.setdefault("facts", {})
+            else:
+                kernel_map._one_parent = tuple(kernel_size) == tuple(stride) and all(int(d) == 1 for d in kernel_dilation)
     if input_sparse_tensor.cache is None:
         input_sparse_tensor._extra_attributes["_cache"] = IntSearchCache()
     input_sparse_tensor.cache.put(key, kernel_map)
@@ -737,6 +778,24 @@ def sparse_conv_wgrad(in_features: Tensor, grad_output: Tensor, kernel_map: IntS
     return gw
 
 
+def _input_gradient(grad_output: Tensor, weight: Tensor, kernel_map: IntSearchResult, num_in: int) -> Tensor:
+    """``dX[in_k] += dY[out_k] @ W_k^T``: the forward kernels over the exchanged map with the weights transposed.
+
+    A stride-1 map of distinct rows onto themselves is its own exchange with the offsets reversed (row m sees row i at
+    offset k exactly when i sees m at K - 1 - k), so its gradient runs over the forward table and its tile order.  A
+    stride-2 map whose every input row has one output row and offset runs from the output side's rows: its gradient is
+    the one-pair convolution."""
+    facts = getattr(kernel_map, "_facts", None)
+    if getattr(kernel_map, "_onto_itself", False) and facts is not None and facts.get("distinct"):
+        return sparse_conv_fused(grad_output, weight, kernel_map, num_in, transpose_weight=True, reverse_weight=True)
+    if getattr(kernel_map, "_one_parent", False):
+        done = sparse_conv_rows_fused(grad_output, weight, kernel_map.neighbor_table(grad_output.shape[0]), num_in,
+                                      transpose_weight=True)
+        if done is not None:
+            return done
+    return sparse_conv_fused(grad_output, weight, kernel_map.swapped(num_in=num_in), num_in, transpose_weight=True)
+
+
 def _normalize_bwd_algo(algo) -> SPARSE_CONV_BWD_ALGO_MODE:
     """Enum | str | list of either -> one algorithm; with a list the first native entry wins
     (no tuner), as for the forward algorithm."""
@@ -773,7 +832,7 @@ class _SparseConvFunction(torch.autograd.Function):
         x, w = ctx.saved_tensors
         km = ctx.kernel_map
         dt = ctx.compute_dtype if ctx.compute_dtype is not None else x.dtype
-        xc, wc, gc = x.to(dt), w.to(dt), grad_output.contiguous().to(dt)
+        xc, gc = x.to(dt), grad_output.contiguous().to(dt)
         need_gx, need_gw = ctx.needs_input_grad[0], ctx.needs_input_grad[1]
         native = (ctx.bwd_algo != SPARSE_CONV_BWD_ALGO_MODE.EXPLICIT_GEMM and gc.is_cuda and dt in _NATIVE_DTYPES
                   and x.shape[0] > 0)
@@ -781,8 +840,7 @@ class _SparseConvFunction(torch.autograd.Function):
         gx = None
         if native_dx:
             with torch.no_grad():
-                wt = wc.detach().transpose(1, 2).contiguous()  # [K, C_out, C_in]
-                gx = sparse_conv_fused(gc.detach(), wt, km.swapped(num_in=x.shape[0]), x.shape[0])
+                gx = _input_gradient(gc.detach(), w, km, x.shape[0])
         elif need_gx:
             gx = torch.zeros_like(xc)
         gw = None
@@ -791,10 +849,11 @@ class _SparseConvFunction(torch.autograd.Function):
                 gw = sparse_conv_wgrad(xc.detach(), gc.detach(), km, gc.shape[0])
         native_dw = gw is not None
         if need_gw and not native_dw:
-            gw = torch.zeros_like(wc)
+            gw = torch.zeros_like(w, dtype=dt)
         need_gw = need_gw and not native_dw
         if need_gw or (need_gx and not native_dx):
             offsets, in_maps, out_maps = km.offsets, km.in_maps, km.out_maps
+            wc = w.to(dt)
             for k in range(len(km)):
                 s, e = int(offsets[k]), int(offsets[k + 1])
                 if e == s:
@@ -806,6 +865,32 @@ class _SparseConvFunction(torch.autograd.Function):
                     gw[k] = torch.matmul(_gather_rows(xc, in_maps[s:e]).T, go)
         return (gx.to(x.dtype) if gx is not None else None, gw.to(w.dtype) if gw is not None else None,
                 None, None, None, None, None, None)
+
+
+class _PointwiseFunction(torch.autograd.Function):
+    """The 1x1x1 convolution in training: a dense GEMM whose weight gradient - a short matrix reduced over all rows -
+    runs through the weight-gradient kernels over the identity map (64 -> 20 channels over 240 000 rows: 130 us as a
+    library GEMM)."""
+
+    @staticmethod
+    def forward(ctx, x, weight):
+        ctx.save_for_backward(x, weight)
+        return x @ (weight[0] if weight.dtype == x.dtype else weight[0].to(x.dtype))
+
+    @staticmethod
+    def backward(ctx, g):
+        x, weight = ctx.saved_tensors
+        w = weight[0].to(x.dtype)
+        g = g.to(x.dtype)
+        gx = g @ w.T if ctx.needs_input_grad[0] else None
+        gw = None
+        if ctx.needs_input_grad[1]:
+            if not torch.is_grad_enabled():
+                gw = sparse_conv_wgrad(x, g, _identity_map(x.shape[0], x.device), x.shape[0])
+            if gw is None:
+                gw = (x.T @ g).unsqueeze(0)
+            gw = gw.to(weight.dtype)
+        return gx, gw
 
 
 # --------------------------------------------------------------------------- entry point
@@ -855,6 +940,11 @@ def spatially_sparse_conv(
 
     if all(k == 1 for k in _kernel_size) and all(s == 1 for s in _stride):
         native = feats.is_cuda and feats.dtype in (torch.float32, torch.float16, torch.bfloat16)
+        if epilogue is None and needs_grad and native and _normalize_bwd_algo(bwd_algo) != SPARSE_CONV_BWD_ALGO_MODE.EXPLICIT_GEMM:
+            out = _PointwiseFunction.apply(feats, weight)
+            if bias is not None:
+                out = out + bias.to(out.dtype)
+            return input_sparse_tensor.replace(batched_features=out)
         if epilogue is None and (needs_grad or not native):
             out = feats @ weight[0].to(feats.dtype) if weight.dtype != feats.dtype else feats @ weight[0]
             if bias is not None:

@@ -16,6 +16,6 @@ def cat(*inputs: Geometry, dim: int = -1):
     if len(inputs) == 1 and isinstance(inputs[0], Sequence):
         inputs = inputs[0]
     assert all(isinstance(i, Geometry) for i in inputs), f"Expected all inputs to be Geometry, got {type(inputs)}"
-    assert all(torch.equal(i.offsets.long(), inputs[0].offsets.long()) for i in inputs), \
+    assert all(i.offsets is inputs[0].offsets or torch.equal(i.offsets.long(), inputs[0].offsets.long()) for i in inputs), \
         "All inputs must have the same offsets"
     return inputs[0].replace(batched_features=torch.cat([i.feature_tensor for i in inputs], dim=dim))

@@ -13,6 +13,8 @@ import torch.nn as nn
 from torch import Tensor
 
 from ...geometry.base.geometry import Geometry
+from ...geometry.types.voxels import Voxels
+from ..functional import batch_norm
 from ..functional.sparse_conv import ConvEpilogue
 from .activations import ReLU as GeometryReLU
 from .base_module import BaseSpatialModule
@@ -102,10 +104,29 @@ class Sequential(nn.Sequential, BaseSpatialModule):
                 x = m(x, epilogue=ep)
                 i = j
                 continue
+            bn = _as_bn(m)
+            if bn is not None and bn.training:
+                feats = x if isinstance(x, Tensor) else x.feature_tensor
+                if batch_norm.can_fuse(bn, feats):
+                    # training: normalisation, residual and ReLU as one function
+                    if isinstance(x, Geometry):
+                        in_sf = x
+                    j = i + 1
+                    relu = j < len(mods) and _is_relu(mods[j])
+                    if relu or (j < len(mods) and isinstance(mods[j], nn.Identity)):
+                        j += 1
+                    res = None
+                    if j == len(mods) and (residual is not None or final_relu) and not relu \
+                            and (residual is None or residual.dtype == feats.dtype):
+                        res, relu, fused_tail = residual, final_relu, True
+                    x = batch_norm.batch_norm_act(feats, bn, relu, res)
+                    i = j
+                    continue
             x, in_sf = run_forward(m, x, in_sf)
             i += 1
         if isinstance(x, Tensor):
-            x = in_sf.replace(batched_features=x)
+            same = type(in_sf) is Voxels and x.dim() == 2 and x.shape[0] == len(in_sf)
+            x = in_sf._derive(x) if same else in_sf.replace(batched_features=x)
         if not fused_tail and (residual is not None or final_relu):
             f = x.feature_tensor
             if residual is not None:
