@@ -631,3 +631,23 @@ def test_pair_weight_gradient_matches_definition(dtype, ksize, n, c_in, c_out):
         want[k] = x[i.long()].double().T @ dy[o.long()].double()
     check_device_status(DEV)
     assert rel_l2(got.cpu().numpy(), want.cpu().numpy()) < 1e-6
+
+
+@pytest.mark.parametrize("ksize,n,c_in,c_out", [(3, 1, 64, 16), (3, 129, 256, 256), (3, 2100, 256, 128), (3, 75649, 32, 48),
+                                                (3, 151297, 64, 32), (3, 151297, 128, 16), (2, 151553, 96, 96), (1, 152000, 32, 32)])
+def test_tensor_core_units_at_the_edges(ksize, n, c_in, c_out):
+    """One unit and less than one, offsets divided among a cluster, one and two 128-row tiles a unit, units taken in
+    fixed strides (up to 151 296 rows on 148 multiprocessors) and claimed (from there), kernels of 1, 8 and 27 offsets:
+    against the FP32-pipe kernel, twice the same bits, with rows in tile order and without."""
+    coords, x, w = _layer_case(n, c_in, c_out, 5 + n, "raster_crop")
+    c = torch.from_numpy(coords).to(DEV)
+    kmap = generate_kernel_map(c, c, (1, 1, 1), (ksize,) * 3)
+    g = torch.Generator().manual_seed(n)
+    x = torch.randn(n, c_in, generator=g).half().to(DEV)
+    w = (torch.randn(ksize ** 3, c_in, c_out, generator=g) * 0.1).half().to(DEV)
+    for ep in (ConvEpilogue(), ConvEpilogue(residual=torch.randn(n, c_out, generator=g).half().to(DEV), relu=True)):
+        ref = sparse_conv_fused(x, w, kmap, n, epilogue=ep, algo=CONV_SIMT)
+        got = [sparse_conv_fused(x, w, kmap, n, epilogue=ep, algo=CONV_TCGEN05, tile_order=t) for t in (False, False, True)]
+        check_device_status(DEV)
+        assert torch.equal(got[0], got[1]) and torch.equal(got[0], got[2])
+        assert rel_l2(got[0].float().cpu().numpy(), ref.float().cpu().numpy()) < 2e-3

@@ -220,7 +220,7 @@ conv_rows_tcgen05_kernel(const __grid_constant__ CUtensorMap feats_map, const Ro
   bool ok = true;
   if (warp == PRODUCER_WARP) {
     // ================================================================ copies: weights and row tiles
-    if (lane == 0) {
+    if (elect_one()) {
       Ring ra{0, 0, p.stages};
       int bbuf = 0, bphase = 0, cur_chunk = -1;
       bool waited = false;
@@ -263,7 +263,7 @@ conv_rows_tcgen05_kernel(const __grid_constant__ CUtensorMap feats_map, const Ro
     __syncwarp();
   } else if (warp == MMA_WARP) {
     // ================================================================ MMA issuer
-    if (lane == 0) {
+    if (elect_one()) {
       Ring ra{0, 0, p.stages};
       int bbuf = 0, bphase = 0, cur_chunk = -1, ab = 0, aphase = 0;
       uint32_t idesc = 0;

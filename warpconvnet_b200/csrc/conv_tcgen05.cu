@@ -1,25 +1,28 @@
 // Output-stationary sparse convolution on the 5th-generation tensor cores.
 //
-// A persistent CTA (one per SM) walks "supertiles" of G x 128 consecutive output
-// rows.  Each 128-row sub-tile owns one fp32 accumulator in tensor memory (the
-// 128 TMEM lanes of an M=128 tcgen05.mma); the accumulators are double-buffered
-// when they fit, so the epilogue of one supertile overlaps the main loop of the
-// next.  Five warp roles, connected by mbarrier rings:
-//  * index warps read the neighbour table of the NEXT supertile (which input row
-//    feeds each output row at each kernel offset), stage it in shared memory and
-//    derive, per sub-tile, the set of offsets that have any neighbour;
-//  * all roles then walk  offsets with a neighbour x channel slices x sub-tiles :
-//    one thread fetches the weight slice of (offset, channel slice) ONCE per
-//    supertile with a bulk copy (the packed weights hold the swizzled shared-memory
-//    image), and eight gather warps copy, for every sub-tile with a neighbour at
-//    that offset, the 128 neighbour rows of the feature matrix into a K-major
-//    swizzled tile (16-byte cp.async, whole row segments per request, absent rows
-//    zero-filled); the copies signal the ring's mbarrier themselves when they land;
-//  * one thread issues tcgen05.mma (weight slice shared by the G sub-tiles) and
-//    releases ring slots with tcgen05.commit;
-//  * epilogue warps read the accumulators with tcgen05.ld, apply scale/shift
-//    (folded BatchNorm or bias), residual add and ReLU, convert and store every
-//    output row exactly once.  No atomics, bit-reproducible.
+// A CTA (one per SM) works through units of G x 128 consecutive output rows.  Each 128-row sub-tile owns one fp32
+// accumulator in tensor memory (the 128 TMEM lanes of an M = 128 tcgen05.mma); the accumulators are double-buffered when
+// they fit, so the epilogue of one unit overlaps the main loop of the next.  Five warp roles, connected by mbarrier rings:
+//  * eight index warps choose the NEXT unit (fixed strides, or claimed from the hardware's queue of CTAs not yet started),
+//    read its neighbour table and stage, for every sub-tile and every offset at which it has any neighbour, the list of
+//    128 input rows;
+//  * all roles then walk  offsets with a neighbour x channel slices : one thread fetches the weight slice of (offset,
+//    channel slice) ONCE per unit with a bulk copy (the packed weights hold the swizzled shared-memory image), and four
+//    gather warps per sub-tile copy the 128 neighbour rows of the feature matrix into a K-major swizzled tile of that
+//    sub-tile's own ring (16-byte cp.async, whole row segments per request, absent rows zero-filled); the copies signal
+//    the ring's mbarrier themselves when they land;
+//  * one thread per sub-tile issues tcgen05.mma and releases ring slots with tcgen05.commit;
+//  * four epilogue warps per sub-tile read the accumulators with tcgen05.ld, apply scale/shift (folded BatchNorm or bias),
+//    residual add and ReLU, convert and store every output row exactly once.  No atomics, bit-reproducible.
+//
+// What bounds it, and what the layout buys (B200, 500 000 rows of a 1 cm room, 9.2 neighbours a row, L2 flushed).  The
+// tensor cores are far from busy below 256 channels: a slot passes through four single-thread or single-warp streams, a
+// barrier round trip costs 350 to 450 clocks, and with one ring for both sub-tiles and both issuers in step the streams
+// waited for each other (no copies, no instructions and no stores at all still took 486 of 631 us at C = 256).  A ring and
+// four gather warps per sub-tile, issuing threads that share nothing but the weight slots and look at the next barriers
+// early, instructions issued behind elect.sync, lists of present offsets only (their 27 KB became row slots) and claimed
+// units: C = 32 / 64 / 96 / 128 / 256 from 94 / 133 / 158 / 201 / 636 us to 86 / 118 / 152 / 186 / 520 us (256: 1.17
+// PFLOP/s); outdoor scene, 128 -> 96, 777 777 rows: 418 -> 359 us; MinkUNet-34 over 1.2 M voxels: 4.77 -> 4.50 ms.
 //
 // Problems with fewer 128-row tiles than multiprocessors divide the kernel offsets of a tile among the S CTAs of a
 // cluster ("split-K over kernel offsets": slice s owns the offsets k with k % S == s, which deals the frequent central
@@ -36,6 +39,7 @@
 // normal exit path (tensor memory released).
 #include "wcn_common.cuh"
 #include "tcgen05_common.cuh"
+#include <atomic>
 
 namespace {
 
@@ -44,14 +48,16 @@ constexpr int MAX_G = 2;              // sub-tiles per supertile (one per MMA is
 constexpr int MAX_RING = 12;          // slots per ring
 constexpr int MAX_OFFSETS = 27;
 constexpr int MAX_SLICES = 8;         // CTAs of a (portable) cluster
-constexpr int EPI_THREADS = 128;      // warps 0..3: TMEM lane quarter = warp index
-constexpr int IDX_THREADS = 128;      // warps 4..7: neighbour-table staging
-constexpr int GATHER_WARP0 = 8;       // warps 8..15: row gathers
+constexpr int EPI_THREADS = 256;      // warps 0..7: TMEM lane quarter = warp index & 3, one sub-tile per four warps
+constexpr int IDX_THREADS = 256;      // warps 8..15: neighbour-table staging, four warps per sub-tile
+constexpr int GATHER_WARP0 = 16;      // warps 16..23: row gathers, four per sub-tile
 constexpr int GATHER_THREADS = 256;
-constexpr int MMA_WARP = 16;          // warps 16, 17: MMA issuers (even / odd sub-tiles); warp 16 owns TMEM
+constexpr int MMA_WARP = 24;          // warps 24, 25: MMA issuers, one per sub-tile; warp 24 owns TMEM
 constexpr int MMA_ISSUERS = 2;
-constexpr int WEIGHT_WARP = 18;       // weight bulk copies
-constexpr int THREADS = 608;
+constexpr int WEIGHT_WARP = 26;       // weight bulk copies
+constexpr int THREADS = 864;
+constexpr int SMEM_LIMIT = 226 * 1024;  // dynamic shared memory the kernels opt in to
+constexpr int CLAIMS = 3;             // claimed units on their way or being read
 
 struct ConvTcParams {
   const char* feats;
@@ -73,12 +79,17 @@ struct ConvTcParams {
   int G;            // sub-tiles per supertile: 1, 2 or 4
   int nbuf;         // accumulator sets in TMEM: 1 or 2
   int cols;         // TMEM columns per accumulator (power of two >= block_n)
-  int sa, sb;       // ring depths
+  int sa, sb;       // ring depths (row slots of each sub-tile, weight slots)
   int kbc;          // channel slices per ring slot (a slot holds kbc K-major tiles side by side)
   int64_t supertiles;
   int S;            // offset slices per supertile (split-K over kernel offsets); 1 = none
   int64_t units;    // supertiles * S work units, walked by the persistent CTAs (S > 1: one each)
+  bool claim;       // one CTA per unit was launched: a CTA claims further units from the hardware's queue
 };
+
+// Row lists (128 input rows of one sub-tile at one offset) staged per sub-tile: two units of ordinary density where K is
+// large, two of any density where it is small.
+__host__ __device__ inline int staged_lists(int K) { return K >= 27 ? K : (2 * K < 27 ? 2 * K : 27); }
 
 // Offsets of slice s of S: the k with k % S == s.
 __device__ __forceinline__ uint32_t slice_mask(int s, int S) {
@@ -117,61 +128,33 @@ __device__ __forceinline__ void ld_global_32B(const void* p, uint32_t* v) {
                : "l"(p));
 }
 
-// `wide`: the destination is 32-byte aligned (rows start on 32-byte boundaries).
-template <typename TO> struct OutVec;
-template <> struct OutVec<float> {
-  static __device__ __forceinline__ void store(float* p, const float (&y)[16], bool wide) {
-    if (wide) {
-      st_global_32B(p, reinterpret_cast<const uint32_t*>(y));
-      st_global_32B(p + 8, reinterpret_cast<const uint32_t*>(y) + 8);
-      return;
-    }
+// Sixteen elements; `wide`: the address is 32-byte aligned (rows start on 32-byte boundaries).
+template <typename TO> __device__ __forceinline__ void load_raw16(const TO* p, TO* v, bool wide) {
+  uint32_t* w = reinterpret_cast<uint32_t*>(v);
+  if (wide) {
 #pragma unroll
-    for (int i = 0; i < 4; ++i) reinterpret_cast<float4*>(p)[i] = make_float4(y[4 * i], y[4 * i + 1], y[4 * i + 2], y[4 * i + 3]);
-  }
-  static __device__ __forceinline__ void load(const float* p, float (&y)[16], bool wide) {
-    if (wide) {
-      ld_global_32B(p, reinterpret_cast<uint32_t*>(y));
-      ld_global_32B(p + 8, reinterpret_cast<uint32_t*>(y) + 8);
-      return;
-    }
+    for (int i = 0; i < (int)sizeof(TO) / 2; ++i) ld_global_32B(reinterpret_cast<const char*>(p) + 32 * i, w + 8 * i);
+  } else {
 #pragma unroll
-    for (int i = 0; i < 4; ++i) {
-      float4 v = __ldg(reinterpret_cast<const float4*>(p) + i);
-      y[4 * i] = v.x; y[4 * i + 1] = v.y; y[4 * i + 2] = v.z; y[4 * i + 3] = v.w;
+    for (int i = 0; i < (int)sizeof(TO); ++i) {
+      const uint4 x = __ldg(reinterpret_cast<const uint4*>(p) + i);
+      w[4 * i] = x.x; w[4 * i + 1] = x.y; w[4 * i + 2] = x.z; w[4 * i + 3] = x.w;
     }
   }
-};
-template <typename T16> struct OutVec16 {
-  static __device__ __forceinline__ void store(T16* p, const float (&y)[16], bool wide) {
-    __align__(32) T16 tmp[16];
+}
+template <typename TO> __device__ __forceinline__ void store16(TO* p, const float (&y)[16], bool wide) {
+  __align__(32) TO v[16];
 #pragma unroll
-    for (int i = 0; i < 16; ++i) tmp[i] = wcn_from_float<T16>(y[i]);
-    if (wide) {
-      st_global_32B(p, reinterpret_cast<const uint32_t*>(tmp));
-      return;
-    }
-    reinterpret_cast<uint4*>(p)[0] = reinterpret_cast<uint4*>(tmp)[0];
-    reinterpret_cast<uint4*>(p)[1] = reinterpret_cast<uint4*>(tmp)[1];
-  }
-  static __device__ __forceinline__ void load(const T16* p, float (&y)[16], bool wide) {
-    __align__(32) T16 tmp[16];
-    if (wide) {
-      ld_global_32B(p, reinterpret_cast<uint32_t*>(tmp));
-    } else {
-      reinterpret_cast<uint4*>(tmp)[0] = __ldg(reinterpret_cast<const uint4*>(p));
-      reinterpret_cast<uint4*>(tmp)[1] = __ldg(reinterpret_cast<const uint4*>(p) + 1);
-    }
+  for (int i = 0; i < 16; ++i) v[i] = wcn_from_float<TO>(y[i]);
+  const uint32_t* w = reinterpret_cast<const uint32_t*>(v);
+  if (wide) {
 #pragma unroll
-    for (int i = 0; i < 16; ++i) y[i] = wcn_to_float<T16>(tmp[i]);
+    for (int i = 0; i < (int)sizeof(TO) / 2; ++i) st_global_32B(reinterpret_cast<char*>(p) + 32 * i, w + 8 * i);
+  } else {
+#pragma unroll
+    for (int i = 0; i < (int)sizeof(TO); ++i)
+      reinterpret_cast<uint4*>(p)[i] = make_uint4(w[4 * i], w[4 * i + 1], w[4 * i + 2], w[4 * i + 3]);
   }
-};
-template <> struct OutVec<__half> : OutVec16<__half> {};
-template <> struct OutVec<__nv_bfloat16> : OutVec16<__nv_bfloat16> {};
-
-// Sub-tiles (bit g) that have a neighbour at offset k, from the per-sub-tile offset masks.
-__device__ __forceinline__ uint32_t subtiles_at(uint32_t m0, uint32_t m1, uint32_t m2, uint32_t m3, int k) {
-  return ((m0 >> k) & 1u) | (((m1 >> k) & 1u) << 1) | (((m2 >> k) & 1u) << 2) | (((m3 >> k) & 1u) << 3);
 }
 
 // Up to N active offsets taken from the low end of `rest` (bit k = offset k still to do);
@@ -198,24 +181,50 @@ struct Ring {
   }
 };
 
-// Control block in shared memory.
+// Control block in shared memory.  Everything a unit's roles need to know about it - which unit it is, which offsets its
+// sub-tiles have, where their neighbour rows were staged - is published by the index warps in one of two `info` entries.
 struct Control {
-  uint64_t a_full[MAX_RING], a_empty[MAX_RING];
+  uint64_t a_full[MAX_G][MAX_RING], a_empty[MAX_G][MAX_RING];
   uint64_t b_full[MAX_RING], b_empty[MAX_RING];
-  uint64_t acc_full[2], acc_empty[2];
+  uint64_t acc_full[2][MAX_G], acc_empty[2][MAX_G];
   uint64_t info_full[2], info_empty[2];
   uint64_t idx_sync;              // rendezvous of the index threads (bounded, unlike bar.sync)
-  uint32_t info_mask[2][MAX_G];   // per staged supertile: non-empty offsets of each sub-tile
-  uint32_t mask_acc[2][MAX_G];    // index warps' scratch while building the masks
+  uint64_t claim_full[CLAIMS];    // a claimed unit has arrived in `claim`
+  __align__(16) uint64_t claim[CLAIMS][2];
+  int64_t info_unit[2];           // the unit; < 0: no more units
+  uint32_t info_mask[2][MAX_G];   // non-empty offsets of each sub-tile
+  int info_entry[2][MAX_G];       // first staged row list of each sub-tile
+  uint32_t mask_acc[3][MAX_G];    // index warps' scratch while building the masks
   uint32_t tmem_holder;
   int skip;
-  int failed;                     // S > 1: the status word once every CTA of the cluster is done
+  int32_t out_row[2][MAX_G * BLOCK_M];          // output row of each slot, -1 past the end
   __align__(16) float sc[256], sh[256];         // this CTA's columns of the epilogue scale / shift (1 / 0 when absent)
 };
 
+// The hardware's work queue (cluster launch control): a running CTA claims a CTA of its grid that has not started yet
+// and does that one's unit itself.  Units differ in their number of offsets; dealt in fixed strides they left the
+// multiprocessors idle for about 15 % of a 256-channel layer, claimed one by one they leave only the last unit.
+__device__ __forceinline__ void claim_next(uint32_t dst, uint32_t bar) {
+  mbar_expect_tx(bar, 16u);
+  asm volatile("clusterlaunchcontrol.try_cancel.async.shared::cta.mbarrier::complete_tx::bytes.b128 [%0], [%1];" ::"r"(dst),
+               "r"(bar)
+               : "memory");
+}
+__device__ __forceinline__ int64_t claimed_unit(const uint64_t (&c)[2]) {
+  uint32_t got, x;
+  asm volatile(
+      "{\n\t.reg .b128 h;\n\t.reg .pred p;\n\tmov.b128 h, {%2, %3};\n\t"
+      "clusterlaunchcontrol.query_cancel.is_canceled.pred.b128 p, h;\n\tselp.u32 %0, 1, 0, p;\n\tmov.u32 %1, 0;\n\t"
+      "@p clusterlaunchcontrol.query_cancel.get_first_ctaid::x.b32.b128 %1, h;\n\t}"
+      : "=r"(got), "=r"(x)
+      : "l"(*(volatile const uint64_t*)&c[0]), "l"(*(volatile const uint64_t*)&c[1])
+      : "memory");
+  return got ? (int64_t)x : -1;
+}
+
 // ------------------------------------------------------------------ kernel
 
-template <int BK, int KBC, bool SPAN, bool BF16, typename TO>
+template <int BK, int KBC, bool SPAN, bool BF16, typename TO, bool RES>
 __global__ void __launch_bounds__(THREADS, 1)
 conv_tcgen05_kernel(const ConvTcParams p) {
   constexpr int RB = BK * 2;         // bytes per tile row
@@ -231,21 +240,48 @@ conv_tcgen05_kernel(const ConvTcParams p) {
   const int B_BYTES = BN * RB;         // one weight tile
   constexpr int A_SLOT = KBC * A_BYTES;  // KBC channel slices per ring slot (KBC divides c_in / BK)
   const int B_SLOT = KBC * B_BYTES;
-  const int IDX_INTS = G * K * BLOCK_M;  // one staged neighbour table
+  const int ENTRIES = G * staged_lists(K);
 
   const uint32_t base = (smem_u32(smem_raw) + 1023u) & ~1023u;
   uint8_t* gen = smem_raw + (base - smem_u32(smem_raw));
   const uint32_t a_base = base;
-  const uint32_t b_base = a_base + p.sa * A_SLOT;
+  const uint32_t b_base = a_base + G * p.sa * A_SLOT;
   const uint32_t misc = b_base + p.sb * B_SLOT;
   uint8_t* misc_gen = gen + (misc - base);
   Control* ctl = reinterpret_cast<Control*>(misc_gen);
-  int32_t* rows_idx = reinterpret_cast<int32_t*>(misc_gen + sizeof(Control));  // [2][G][K][128]
+  int32_t* rows_idx = reinterpret_cast<int32_t*>(misc_gen + sizeof(Control));  // [ENTRIES][128]
   auto bar = [](uint64_t* b) { return smem_u32(b); };
 
-  if (tid == 0) ctl->skip = *(volatile int32_t*)p.dev_status;  // an earlier launch on this status word failed
+  // One rendezvous behind the whole set-up (an earlier form, a thread at a time behind two, took 2 000 clocks: a microsecond
+  // of each of the sixty launches of a small network).
+  if (!p.claim) launch_dependents();
+  const uint32_t tmem_total = (uint32_t)(NBUF * G * p.cols);
+  if (warp == 0) {
+    for (int g = 0; g < G; ++g)
+      if (lane < p.sa) { mbar_init(bar(&ctl->a_full[g][lane]), GATHER_THREADS / G); mbar_init(bar(&ctl->a_empty[g][lane]), 1); }
+    if (lane < p.sb) { mbar_init(bar(&ctl->b_full[lane]), 1); mbar_init(bar(&ctl->b_empty[lane]), G); }
+    if (lane < 2) {
+      for (int g = 0; g < G; ++g) { mbar_init(bar(&ctl->acc_full[lane][g]), 1); mbar_init(bar(&ctl->acc_empty[lane][g]), EPI_THREADS / G); }
+      mbar_init(bar(&ctl->info_full[lane]), IDX_THREADS);
+      mbar_init(bar(&ctl->info_empty[lane]), EPI_THREADS / 32 + G + 1 + GATHER_THREADS / 32);  // epilogue warps, MMA threads, weight thread, gather warps
+    }
+    if (lane < CLAIMS) mbar_init(bar(&ctl->claim_full[lane]), 1);
+    if (lane < 3) ctl->mask_acc[lane][0] = ctl->mask_acc[lane][1] = 0;
+    if (lane == 3) mbar_init(bar(&ctl->idx_sync), IDX_THREADS);
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+  } else if (warp == 1) {
+    if (lane == 0) ctl->skip = *(volatile int32_t*)p.dev_status;  // an earlier launch on this status word failed
+  } else if (warp == MMA_WARP) {
+    tmem_alloc(smem_u32(&ctl->tmem_holder), tmem_total < 32 ? 32u : tmem_total);
+  } else if (warp >= GATHER_WARP0 && warp < MMA_WARP) {
+    for (int i = tid - GATHER_WARP0 * 32; i < BN; i += GATHER_THREADS) {
+      ctl->sc[i] = p.scale ? __ldg(&p.scale[n0 + i]) : 1.f;
+      ctl->sh[i] = p.shift ? __ldg(&p.shift[n0 + i]) : 0.f;
+    }
+  }
+  tc_fence_before();
   __syncthreads();
-  launch_dependents();
+  tc_fence_after();
   bool ok = true;
   if (ctl->skip == (int)WCN_ERR_WAIT_EXPIRED) {
     // Nothing is computed after a kernel on this status word gave up.  The rows this CTA would have
@@ -263,103 +299,143 @@ conv_tcgen05_kernel(const ConvTcParams p) {
           reinterpret_cast<TO*>(p.out)[m * p.out_ld + n0 + (int)(i % BN)] = nan;
         }
       }
-      return;
     }
     ok = false;  // no role does any work
   }
-
-  if (tid == 0) {
-    for (int s = 0; s < p.sa; ++s) { mbar_init(bar(&ctl->a_full[s]), GATHER_THREADS); mbar_init(bar(&ctl->a_empty[s]), MMA_ISSUERS); }
-    for (int s = 0; s < p.sb; ++s) { mbar_init(bar(&ctl->b_full[s]), 1); mbar_init(bar(&ctl->b_empty[s]), MMA_ISSUERS); }
-    for (int i = 0; i < 2; ++i) {
-      mbar_init(bar(&ctl->acc_full[i]), MMA_ISSUERS);
-      mbar_init(bar(&ctl->acc_empty[i]), EPI_THREADS);
-      mbar_init(bar(&ctl->info_full[i]), 1);
-      mbar_init(bar(&ctl->info_empty[i]), EPI_THREADS + MMA_ISSUERS + 1 + GATHER_THREADS / 32);  // epilogue threads, MMA threads, weight thread, gather warps
-    }
-    mbar_init(bar(&ctl->idx_sync), IDX_THREADS);
-    for (int g = 0; g < MAX_G; ++g) ctl->mask_acc[0][g] = ctl->mask_acc[1][g] = 0;
-    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-  }
-  for (int i = tid; i < BN; i += THREADS) {
-    ctl->sc[i] = p.scale ? __ldg(&p.scale[n0 + i]) : 1.f;
-    ctl->sh[i] = p.shift ? __ldg(&p.shift[n0 + i]) : 0.f;
-  }
-  const uint32_t tmem_total = (uint32_t)(NBUF * G * p.cols);
-  if (warp == MMA_WARP) tmem_alloc(smem_u32(&ctl->tmem_holder), tmem_total < 32 ? 32u : tmem_total);
-  tc_fence_before();
-  __syncthreads();
-  tc_fence_after();
   const uint32_t tmem_base = ctl->tmem_holder;
 
-  if (warp >= 4 && warp < GATHER_WARP0) {
+  if (warp >= EPI_THREADS / 32 && warp < GATHER_WARP0) {
     // ================================================================ index warps
-    // Stage the neighbour table of a supertile (one supertile ahead of the copies):
-    // rows_idx[ib][g][k][row] = input row, or -1 where there is no neighbour.
-    // Only the offsets of the unit's slice are read; the others are staged as "no neighbour",
-    // so every role downstream sees a supertile that simply has fewer offsets.  An index that
-    // does not name a feature row is treated as absent and reported (WCN_ERR_BOUNDS).
-    const int itid = tid - EPI_THREADS;
+    // Choose the next unit and stage what the other roles need of it, one unit ahead of the copies: the output row of
+    // every slot, the offsets each sub-tile has any neighbour at, and for each of those the 128 input rows (-1 where a row
+    // has none), as row lists in a ring of G * K entries - room for two units of ordinary density, where two complete
+    // tables would take another 27 KB from the row slots.  Only the offsets of the unit's slice are read; the others
+    // are absent for every role.  An index that does not name a feature row is treated as absent and reported
+    // (WCN_ERR_BOUNDS).
+    // This role paces narrow layers (few bytes per unit), and what it waits for is latency: four warps per sub-tile (or,
+    // for a single sub-tile, four for the even and four for the odd offsets), loads before the wait for a free entry, units
+    // claimed two ahead, one vote per warp.  54 loads and 54 votes in four warps took 14 000 clocks per unit, three times
+    // what the copies of a 32-channel layer take.
+    const int itid = tid - EPI_THREADS, row = itid & (BLOCK_M - 1), half = itid >> 7;
+    const int g = G == 2 ? half : 0;
+    const uint32_t mine = G == 2 ? 0xFFFFFFFFu : half ? 0xAAAAAAAAu : 0x55555555u;   // this thread's offsets
     const int num_in = (int)p.num_in;
-    int ib = 0, iphase = 0, sphase = 0;
+    int sphase = 0, entry = 0, before = 0;   // next free entry; entries of the unit before
+    int n = 0, acc = 0;                      // units staged; scratch of this unit's masks
+    int asked = 0, slot = 0, cphase = 0;     // claims not read yet, the next one to read
+    bool refused = false;
     bool bad = false;
-    for (int64_t wu = blockIdx.x; wu < p.units && ok; wu += gridDim.x) {
-      const int64_t st = p.S > 1 ? wu / p.S : wu;
-      const uint32_t kmask = slice_mask((int)(wu - st * p.S), p.S);
-      const int64_t m0 = st * G * BLOCK_M;
-      if (!mbar_wait(bar(&ctl->info_empty[ib]), iphase ^ 1, p.dev_status)) { ok = false; break; }
-      int32_t* dst = rows_idx + ib * IDX_INTS;
-      // The rows of both sub-tiles are requested before either is consumed: a thread's loads are what this
-      // role waits for, so twice as many in flight halve the time a table takes.
-      const int64_t ma = m0 + itid, mb = m0 + BLOCK_M + itid;
-      const bool two = G > 1;
-      int ra[MAX_OFFSETS], rb[MAX_OFFSETS];
-#pragma unroll
-      for (int k = 0; k < MAX_OFFSETS; ++k) {
-        const bool want = k < K && ((kmask >> k) & 1u);
-        ra[k] = (want && ma < p.M) ? __ldg(&p.nbr[(int64_t)k * p.M + ma]) : -1;
-        rb[k] = (want && two && mb < p.M) ? __ldg(&p.nbr[(int64_t)k * p.M + mb]) : -1;
+    int64_t unit = blockIdx.x;
+    auto claim_one = [&](int at) {
+      if (itid == 0) {
+        // (every index thread has read the slot's last content: they met since)
+        asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+        claim_next(bar(&ctl->claim[at][0]), bar(&ctl->claim_full[at]));
       }
-      uint32_t mine_a = 0, mine_b = 0;
-#pragma unroll
-      for (int k = 0; k < MAX_OFFSETS; ++k) {
-        if (k < K) {
-          if (ra[k] >= num_in) { ra[k] = -1; bad = true; }
-          dst[k * BLOCK_M + itid] = ra[k];
-          if (__any_sync(0xFFFFFFFFu, ra[k] >= 0)) mine_a |= 1u << k;
-          if (two) {
-            if (rb[k] >= num_in) { rb[k] = -1; bad = true; }
-            dst[(K + k) * BLOCK_M + itid] = rb[k];
-            if (__any_sync(0xFFFFFFFFu, rb[k] >= 0)) mine_b |= 1u << k;
+      ++asked;
+    };
+    if (p.claim && ok) claim_one(0);
+    while (ok) {
+      const int ib = n & 1;
+      if (n > 0) {  // the unit after the one just staged
+        if (!p.claim) {
+          unit += gridDim.x;
+          if (unit >= p.units) unit = -1;
+        } else {
+          // (after a refusal nothing more is claimed, but a claim already on its way may still have been granted)
+          for (unit = -1; unit < 0 && asked > 0;) {
+            if (!mbar_wait(bar(&ctl->claim_full[slot]), cphase, p.dev_status)) { ok = false; break; }
+            unit = claimed_unit(ctl->claim[slot]);
+            // (not before: the next launch's CTAs would be placed ahead of this grid's that have not started, and wait there
+            // for the few multiprocessors left to it)
+            if (unit < 0 && !refused) { refused = true; launch_dependents(); }
+            if (++slot == CLAIMS) { slot = 0; cphase ^= 1; }
+            --asked;
           }
+          if (!ok) break;
         }
       }
-      if (lane == 0 && mine_a) atomicOr(&ctl->mask_acc[ib][0], mine_a);
-      if (lane == 0 && mine_b) atomicOr(&ctl->mask_acc[ib][1], mine_b);
+      if (unit < 0) {
+        if (!mbar_wait(bar(&ctl->info_empty[ib]), ((n >> 1) & 1) ^ 1, p.dev_status)) { ok = false; break; }
+        if (itid == 0) ctl->info_unit[ib] = -1;
+        mbar_arrive(bar(&ctl->info_full[ib]));
+        break;
+      }
+      if (p.claim && !refused) claim_one(slot == CLAIMS - 1 ? 0 : slot + 1);
+      const int64_t st = p.S > 1 ? unit / p.S : unit;
+      const uint32_t kmask = slice_mask((int)(unit - st * p.S), p.S) & mine;
+      const int64_t m = (st * G + g) * BLOCK_M + row;
+      int r[MAX_OFFSETS];
+#pragma unroll
+      for (int k = 0; k < MAX_OFFSETS; ++k)
+        r[k] = k < K && ((kmask >> k) & 1u) && m < p.M ? __ldg(&p.nbr[(int64_t)k * p.M + m]) : -1;
+      const int32_t out_row = m < p.M ? (p.out_rows ? __ldg(&p.out_rows[m]) : (int32_t)m) : -1;
+      if (!mbar_wait(bar(&ctl->info_empty[ib]), ((n >> 1) & 1) ^ 1, p.dev_status)) { ok = false; break; }
+      uint32_t has = 0;
+#pragma unroll
+      for (int k = 0; k < MAX_OFFSETS; ++k) {
+        if (r[k] >= num_in) { r[k] = -1; bad = true; }
+        has |= r[k] >= 0 ? 1u << k : 0u;
+      }
+      has = __reduce_or_sync(0xFFFFFFFFu, has);
+      if (lane == 0 && has) atomicOr(&ctl->mask_acc[acc][g], has);
+      if (mine & 1u) ctl->out_row[ib][g * BLOCK_M + row] = out_row;
       // all index threads meet (bounded: a thread that gave up does not arrive, the others time out)
       mbar_arrive(bar(&ctl->idx_sync));
       if (!mbar_wait(bar(&ctl->idx_sync), sphase, p.dev_status)) { ok = false; break; }
       sphase ^= 1;
+      const uint32_t m0 = ctl->mask_acc[acc][0], m1 = ctl->mask_acc[acc][1];
+      // The scratch is used in turns of three: what is cleared here was read before this rendezvous and is next added to
+      // after the following one.
+      acc = acc == 2 ? 0 : acc + 1;
+      if (itid == 0) { const int c = acc == 2 ? 0 : acc + 1; ctl->mask_acc[c][0] = ctl->mask_acc[c][1] = 0; }
+      const int need = __popc(m0) + __popc(m1);
+      // the entries of the unit before last are free (info_empty above); those of the last unit only if it has been read
+      if (before + need > ENTRIES && !mbar_wait(bar(&ctl->info_empty[ib ^ 1]), ((n - 1) >> 1) & 1, p.dev_status)) { ok = false; break; }
+      before = need;
+      int second = entry + __popc(m0);
+      if (second >= ENTRIES) second -= ENTRIES;
       if (itid == 0) {
-        for (int g = 0; g < MAX_G; ++g) {
-          ctl->info_mask[ib][g] = g < G ? ctl->mask_acc[ib][g] : 0u;
-          ctl->mask_acc[ib][g] = 0;  // next use of this entry is two supertiles away, behind info_empty
-        }
-        mbar_arrive(bar(&ctl->info_full[ib]));  // publishes the table and the masks
+        ctl->info_unit[ib] = unit;
+        ctl->info_mask[ib][0] = m0;
+        ctl->info_mask[ib][1] = m1;
+        ctl->info_entry[ib][0] = entry;
+        ctl->info_entry[ib][1] = second;
       }
-      if (++ib == 2) { ib = 0; iphase ^= 1; }
+      const uint32_t own = g == 0 ? m0 : m1;
+      int32_t* at = rows_idx + (g == 0 ? entry : second) * BLOCK_M + row;
+      int32_t* const end = rows_idx + ENTRIES * BLOCK_M;
+#pragma unroll
+      for (int k = 0; k < MAX_OFFSETS; ++k) {
+        if ((own >> k) & 1u) {
+          if ((mine >> k) & 1u) *at = r[k];
+          at += BLOCK_M;
+          if (at >= end) at -= ENTRIES * BLOCK_M;
+        }
+      }
+      entry = second + __popc(m1);
+      if (entry >= ENTRIES) entry -= ENTRIES;
+      mbar_arrive(bar(&ctl->info_full[ib]));  // (256 arrivals publish the lists)
+      ++n;
     }
+    // claims on their way write this CTA's shared memory: they have to arrive (bounded waits) before it leaves
+    if (itid == 0 && p.claim)
+      for (; asked > 0; --asked) {
+        (void)mbar_wait(bar(&ctl->claim_full[slot]), cphase, p.dev_status);
+        if (++slot == CLAIMS) { slot = 0; cphase ^= 1; }
+      }
     if (bad) wcn_report_bounds(p.dev_status);
   } else if (warp == WEIGHT_WARP) {
     // ================================================================ weight loader
-    if (lane == 0) {
+    if (elect_one()) {
       Ring rb{0, 0, p.sb};
-      int ib = 0, iphase = 0;
-      for (int64_t wu = blockIdx.x; wu < p.units && ok; wu += gridDim.x) {
-        if (!mbar_wait(bar(&ctl->info_full[ib]), iphase, p.dev_status)) { ok = false; break; }
+      for (int n = 0; ok; ++n) {
+        const int ib = n & 1;
+        if (!mbar_wait(bar(&ctl->info_full[ib]), (n >> 1) & 1, p.dev_status)) { ok = false; break; }
+        const bool last = ctl->info_unit[ib] < 0;
         uint32_t rest = ctl->info_mask[ib][0] | ctl->info_mask[ib][1];
         mbar_arrive(bar(&ctl->info_empty[ib]));  // only the masks were needed
-        if (++ib == 2) { ib = 0; iphase ^= 1; }
+        if (last) break;
         // One channel slice per offset (KB == 1) and KBC > 1: a ring slot spans KBC consecutive
         // ACTIVE OFFSETS instead of KBC channel slices of one offset, so narrow layers get the same
         // fat slots as wide ones.  All roles take the offsets off the mask in the same groups.
@@ -397,315 +473,305 @@ conv_tcgen05_kernel(const ConvTcParams p) {
     __syncwarp();
   } else if (warp >= GATHER_WARP0 && warp < MMA_WARP) {
     // ================================================================ gather warps
+    // Four warps and a ring of row slots per sub-tile (all eight for the one sub-tile of a small problem).
     wait_for_primary();  // the feature rows are the previous launch's
     const int gwarp = warp - GATHER_WARP0;
-    constexpr int ROWS_PER_WARP = BLOCK_M / (GATHER_THREADS / 32);  // 16
-    constexpr int NJ = ROWS_PER_WARP / RPI;                          // copy instructions per warp per A slot
+    const int g = G == 2 ? gwarp >> 2 : 0;
+    const int row0 = G == 2 ? (gwarp & 3) * 32 : gwarp * 16;  // this warp's 32 (16) rows of the tile
+    constexpr int NJ = 16 / RPI;                               // copy instructions per 16 rows and channel slice
     const int sub_row = lane / CH, chunk = lane % CH;
-    uint32_t aoff[NJ];  // this thread's fixed (row, chunk) positions inside an A tile
+    uint32_t aoff[2 * NJ];  // this thread's fixed (row, chunk) positions inside an A tile
 #pragma unroll
-    for (int j = 0; j < NJ; ++j) aoff[j] = tile_offset<RB>(gwarp * ROWS_PER_WARP + j * RPI + sub_row, chunk);
+    for (int j = 0; j < 2 * NJ; ++j) aoff[j] = tile_offset<RB>((row0 + j * RPI + sub_row) & (BLOCK_M - 1), chunk);
+    const char* feats = p.feats + chunk * 16;
     Ring ra{0, 0, p.sa};
-    int ib = 0, iphase = 0;
-    for (int64_t wu = blockIdx.x; wu < p.units && ok; wu += gridDim.x) {
-      if (!mbar_wait(bar(&ctl->info_full[ib]), iphase, p.dev_status)) { ok = false; break; }
-      const uint32_t mk0 = ctl->info_mask[ib][0], mk1 = ctl->info_mask[ib][1];
-      constexpr uint32_t mk2 = 0u, mk3 = 0u;
-      const int32_t* tab = rows_idx + ib * IDX_INTS + gwarp * ROWS_PER_WARP + sub_row;
-      uint32_t rest = mk0 | mk1 | mk2 | mk3;
+    const uint32_t ring = a_base + g * p.sa * A_SLOT;
+    for (int n = 0; ok; ++n) {
+      const int ib = n & 1;
+      if (!mbar_wait(bar(&ctl->info_full[ib]), (n >> 1) & 1, p.dev_status)) { ok = false; break; }
+      if (ctl->info_unit[ib] < 0) break;
+      const uint32_t own = ctl->info_mask[ib][g];
+      uint32_t rest = SPAN ? own | ctl->info_mask[ib][1] | ctl->info_mask[ib][0] : own;
+      int e = ctl->info_entry[ib][g];
+      const int32_t* tab = rows_idx + row0 + sub_row;
+      // the addresses of this thread's rows, and which of them are there
+      auto rows_of = [&](int entry, const char* (&src)[2 * NJ], uint32_t& have) {
+        have = 0;
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+          if (h < G) {
+#pragma unroll
+            for (int j = h * NJ; j < (h + 1) * NJ; ++j) {
+              const int r = tab[entry * BLOCK_M + j * RPI];
+              have |= (r >= 0 ? 1u : 0u) << j;
+              src[j] = feats + (int64_t)max(r, 0) * p.in_ld_bytes;
+            }
+          }
+        }
+      };
+      auto copy = [&](uint32_t dst, const char* const (&src)[2 * NJ], uint32_t have, int64_t at) {
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+          if (h < G) {
+#pragma unroll
+            for (int j = h * NJ; j < (h + 1) * NJ; ++j)
+              cp_async16(dst + aoff[j], src[j] + at, ((have >> j) & 1u) * 16u);
+          }
+        }
+      };
       while (SPAN && rest && ok) {  // slots that span offsets (see the weight loader)
         int ku[KBC];
         pop_offsets<KBC>(rest, ku);
-        uint32_t gbu[KBC], gany = 0;
+        uint32_t used = 0;
+#pragma unroll
+        for (int u = 0; u < KBC; ++u)
+          if (ku[u] >= 0) used |= ((own >> ku[u]) & 1u) << u;
+        if (!used) continue;
+        if (!mbar_wait(bar(&ctl->a_empty[g][ra.slot]), ra.phase ^ 1, p.dev_status)) { ok = false; break; }
+        const uint32_t dst = ring + ra.slot * A_SLOT;
 #pragma unroll
         for (int u = 0; u < KBC; ++u) {
-          gbu[u] = ku[u] >= 0 ? subtiles_at(mk0, mk1, mk2, mk3, ku[u]) : 0u;
-          gany |= gbu[u];
-        }
-        for (uint32_t gb = gany; gb; gb &= gb - 1) {
-          const int g = __ffs(gb) - 1;
-          if (!mbar_wait(bar(&ctl->a_empty[ra.slot]), ra.phase ^ 1, p.dev_status)) { ok = false; break; }
-          const uint32_t a_dst = a_base + ra.slot * A_SLOT;
-          const char* fbase = p.feats + chunk * 16;
-#pragma unroll
-          for (int u = 0; u < KBC; ++u) {
-            if ((gbu[u] >> g) & 1u) {  // sub-tiles of offsets this row block does not have stay unused
-              const int32_t* rk = tab + (g * K + ku[u]) * BLOCK_M;
-              int src[NJ];
-#pragma unroll
-              for (int j = 0; j < NJ; ++j) src[j] = rk[j * RPI];
-#pragma unroll
-              for (int j = 0; j < NJ; ++j) {
-                const bool have = src[j] >= 0;
-                cp_async16(a_dst + u * A_BYTES + aoff[j], have ? fbase + (int64_t)src[j] * p.in_ld_bytes : p.feats,
-                           have ? 16u : 0u);
-              }
-            }
+          if ((used >> u) & 1u) {  // parts of offsets this sub-tile does not have stay unused
+            const char* src[2 * NJ];
+            uint32_t have;
+            rows_of(e, src, have);
+            if (++e == ENTRIES) e = 0;
+            copy(dst + u * A_BYTES, src, have, 0);
           }
-          cp_async_arrive(bar(&ctl->a_full[ra.slot]));
+        }
+        cp_async_arrive(bar(&ctl->a_full[g][ra.slot]));
+        ra.advance();
+      }
+      while (!SPAN && rest && ok) {
+        rest &= rest - 1;
+        const char* src[2 * NJ];
+        uint32_t have;
+        rows_of(e, src, have);
+        if (++e == ENTRIES) e = 0;
+        for (int kb0 = 0; kb0 < KB; kb0 += KBC) {
+          if (!mbar_wait(bar(&ctl->a_empty[g][ra.slot]), ra.phase ^ 1, p.dev_status)) { ok = false; break; }
+          const uint32_t dst = ring + ra.slot * A_SLOT;
+#pragma unroll
+          for (int u = 0; u < KBC; ++u)  // the row's next channel slices are contiguous in memory
+            copy(dst + u * A_BYTES, src, have, (int64_t)(kb0 + u) * RB);
+          cp_async_arrive(bar(&ctl->a_full[g][ra.slot]));  // hardware arrives when this thread's copies land
           ra.advance();
         }
       }
-      while (!SPAN && rest && ok) {
-        const int k = __ffs(rest) - 1;
-        rest &= rest - 1;
-        const uint32_t gbits = subtiles_at(mk0, mk1, mk2, mk3, k);
-        for (int kb0 = 0; kb0 < KB && ok; kb0 += KBC) {
-          for (uint32_t gb = gbits; gb; gb &= gb - 1) {
-            const int g = __ffs(gb) - 1;
-            if (!mbar_wait(bar(&ctl->a_empty[ra.slot]), ra.phase ^ 1, p.dev_status)) { ok = false; break; }
-            const uint32_t a_dst = a_base + ra.slot * A_SLOT;
-            const int32_t* rk = tab + (g * K + k) * BLOCK_M;
-            int src[NJ];  // all index reads first, so the copies below issue back to back
-#pragma unroll
-            for (int j = 0; j < NJ; ++j) src[j] = rk[j * RPI];
-            const char* fbase = p.feats + (int64_t)kb0 * RB + chunk * 16;
-#pragma unroll
-            for (int j = 0; j < NJ; ++j) {
-              const bool have = src[j] >= 0;
-              const char* sp = have ? fbase + (int64_t)src[j] * p.in_ld_bytes : p.feats;
-#pragma unroll
-              for (int u = 0; u < KBC; ++u)  // the row's next channel slices are contiguous in memory
-                cp_async16(a_dst + u * A_BYTES + aoff[j], have ? sp + u * RB : sp, have ? 16u : 0u);
-            }
-            cp_async_arrive(bar(&ctl->a_full[ra.slot]));  // hardware arrives when this thread's copies land
-            ra.advance();
-          }
-        }
-      }
       __syncwarp();
-      if (lane == 0) mbar_arrive(bar(&ctl->info_empty[ib]));  // this warp is done with the staged table
-      if (++ib == 2) { ib = 0; iphase ^= 1; }
+      if (lane == 0) mbar_arrive(bar(&ctl->info_empty[ib]));  // this warp is done with the staged lists
     }
     cp_async_drain();
   } else if (warp >= MMA_WARP && warp < MMA_WARP + MMA_ISSUERS) {
     // ================================================================ MMA issuers
-    // Two threads share the issue work: issuer w takes the sub-tiles with (g & 1) == w.  Both
-    // walk the same slot sequence, both observe and release every row slot and every weight
-    // slot, and both sign off the accumulator set.
-    const uint32_t issuer = (uint32_t)(warp - MMA_WARP);
-    if (lane == 0) {
+    // One thread per sub-tile.  They share the weight slots - both observe and release every one, because a parity wait is
+    // only meaningful for a thread that is never a whole lap away - and nothing else.  A barrier operation costs a single
+    // thread 50 to 100 clocks even when it succeeds at once, so the next slots' barriers are looked at before this slot's
+    // instructions are issued.
+    const int g = warp - MMA_WARP;
+    if (g < G && elect_one()) {
       const uint32_t idesc = (1u << 4) | ((BF16 ? 1u : 0u) << 7) | ((BF16 ? 1u : 0u) << 10) |
                              ((uint32_t)(BN >> 3) << 17) | ((uint32_t)(BLOCK_M >> 4) << 24);
       Ring ra{0, 0, p.sa}, rb{0, 0, p.sb};
-      int ib = 0, iphase = 0, ab = 0, aphase = 0;
-      for (int64_t wu = blockIdx.x; wu < p.units && ok; wu += gridDim.x) {
-        if (!mbar_wait(bar(&ctl->info_full[ib]), iphase, p.dev_status)) { ok = false; break; }
-        const uint32_t mk0 = ctl->info_mask[ib][0], mk1 = ctl->info_mask[ib][1];
-        constexpr uint32_t mk2 = 0u, mk3 = 0u;
-        const uint32_t uni = mk0 | mk1 | mk2 | mk3;
+      const uint32_t ring = a_base + g * p.sa * A_SLOT;
+      bool a_ready = false, b_ready = false;
+      int ab = 0, aphase = 0;
+      for (int n = 0; ok; ++n) {
+        const int ib = n & 1;
+        if (!mbar_wait(bar(&ctl->info_full[ib]), (n >> 1) & 1, p.dev_status)) { ok = false; break; }
+        const bool last = ctl->info_unit[ib] < 0;
+        const uint32_t own = ctl->info_mask[ib][g];
+        uint32_t rest = own | ctl->info_mask[ib][0] | ctl->info_mask[ib][1];
         mbar_arrive(bar(&ctl->info_empty[ib]));  // only the masks were needed
-        if (++ib == 2) { ib = 0; iphase ^= 1; }
-        // the accumulator set must have been read out by the epilogue of its previous use
-        if (!mbar_wait(bar(&ctl->acc_empty[ab]), aphase ^ 1, p.dev_status)) { ok = false; break; }
+        if (last) break;
+        // the accumulator must have been read out by the epilogue of its previous use
+        if (!mbar_wait(bar(&ctl->acc_empty[ab][g]), aphase ^ 1, p.dev_status)) { ok = false; break; }
         tc_fence_after();
-        uint32_t started = 0;
-        uint32_t rest = uni;
-        while (SPAN && rest && ok) {  // slots that span offsets (see the weight loader)
-          int ku[KBC];
-          pop_offsets<KBC>(rest, ku);
-          uint32_t gbu[KBC], gany = 0;
+        const uint32_t d = tmem_base + (uint32_t)((ab * G + g) * p.cols);
+        uint32_t acc = 0;
+        while (rest && ok) {
+          int ku[SPAN ? KBC : 1];
+          uint32_t used = 0;
+          pop_offsets<SPAN ? KBC : 1>(rest, ku);
 #pragma unroll
-          for (int u = 0; u < KBC; ++u) {
-            gbu[u] = ku[u] >= 0 ? subtiles_at(mk0, mk1, mk2, mk3, ku[u]) : 0u;
-            gany |= gbu[u];
-          }
-          if (!mbar_wait(bar(&ctl->b_full[rb.slot]), rb.phase, p.dev_status)) { ok = false; break; }
-          const uint32_t b_slot = b_base + rb.slot * B_SLOT;
-          for (uint32_t gb = gany; gb; gb &= gb - 1) {
-            const int g = __ffs(gb) - 1;
-            if (!mbar_wait(bar(&ctl->a_full[ra.slot]), ra.phase, p.dev_status)) { ok = false; break; }
-            if (((uint32_t)g & 1u) != issuer) {  // the other issuer's slot
-              mbar_arrive(bar(&ctl->a_empty[ra.slot]));
-              ra.advance();
+          for (int u = 0; u < (SPAN ? KBC : 1); ++u)
+            if (ku[u] >= 0) used |= ((own >> ku[u]) & 1u) << u;
+          for (int kb0 = 0; kb0 < (SPAN ? 1 : KB); kb0 += KBC) {
+            if (!b_ready && !mbar_wait(bar(&ctl->b_full[rb.slot]), rb.phase, p.dev_status)) { ok = false; break; }
+            const uint64_t bdesc = smem_desc<RB>(b_base + rb.slot * B_SLOT);
+            const uint32_t b_free = bar(&ctl->b_empty[rb.slot]);
+            rb.advance();
+            if (!used) {  // this sub-tile has none of the slot's offsets
+              mbar_arrive(b_free);
+              b_ready = mbar_test(bar(&ctl->b_full[rb.slot]), rb.phase);
               continue;
             }
+            if (!a_ready && !mbar_wait(bar(&ctl->a_full[g][ra.slot]), ra.phase, p.dev_status)) { ok = false; break; }
             tc_fence_after();
-            const uint32_t a_slot = a_base + ra.slot * A_SLOT;
-            const uint32_t d = tmem_base + (uint32_t)((ab * G + g) * p.cols);
-            uint32_t acc = (started >> g) & 1u;
+            const uint64_t adesc = smem_desc<RB>(ring + ra.slot * A_SLOT);
+            const uint32_t a_free = bar(&ctl->a_empty[g][ra.slot]);
+            ra.advance();
+            a_ready = mbar_test(bar(&ctl->a_full[g][ra.slot]), ra.phase);
+            b_ready = mbar_test(bar(&ctl->b_full[rb.slot]), rb.phase);
 #pragma unroll
             for (int u = 0; u < KBC; ++u) {
-              if ((gbu[u] >> g) & 1u) {
-                const uint64_t adesc = smem_desc<RB>(a_slot + u * A_BYTES);
-                const uint64_t bdesc = smem_desc<RB>(b_slot + u * B_BYTES);
+              if (!SPAN || ((used >> u) & 1u)) {
 #pragma unroll
                 for (int kk = 0; kk < BK / 16; ++kk)
-                  umma_f16(d, adesc + (uint64_t)(kk * 2), bdesc + (uint64_t)(kk * 2), idesc,
-                           (acc | (uint32_t)kk) ? 1u : 0u);
+                  umma_f16(d, adesc + (uint64_t)(u * (A_BYTES >> 4) + kk * 2), bdesc + (uint64_t)(u * (B_BYTES >> 4) + kk * 2),
+                           idesc, acc | (kk > 0 ? 1u : 0u));
                 acc = 1u;
               }
             }
-            started |= 1u << g;
-            umma_commit(bar(&ctl->a_empty[ra.slot]));
-            ra.advance();
-          }
-          umma_commit(bar(&ctl->b_empty[rb.slot]));
-          rb.advance();
-        }
-        while (!SPAN && rest && ok) {
-          const int k = __ffs(rest) - 1;
-          rest &= rest - 1;
-          const uint32_t gbits = subtiles_at(mk0, mk1, mk2, mk3, k);
-          for (int kb0 = 0; kb0 < KB && ok; kb0 += KBC) {
-            if (!mbar_wait(bar(&ctl->b_full[rb.slot]), rb.phase, p.dev_status)) { ok = false; break; }
-            const uint32_t b_slot = b_base + rb.slot * B_SLOT;
-            for (uint32_t gb = gbits; gb; gb &= gb - 1) {
-              const int g = __ffs(gb) - 1;
-              // Both issuers pass every row slot in step: a parity wait is only meaningful for a
-              // thread that is never a whole ring lap away from the slot, so the issuer that does
-              // not consume a slot still observes its fill and signs it off.
-              if (!mbar_wait(bar(&ctl->a_full[ra.slot]), ra.phase, p.dev_status)) { ok = false; break; }
-              if (((uint32_t)g & 1u) != issuer) {  // the other issuer's slot
-                mbar_arrive(bar(&ctl->a_empty[ra.slot]));
-                ra.advance();
-                continue;
-              }
-              tc_fence_after();
-              const uint32_t a_slot = a_base + ra.slot * A_SLOT;
-              const uint32_t d = tmem_base + (uint32_t)((ab * G + g) * p.cols);
-              const uint32_t acc0 = (started >> g) & 1u;
-#pragma unroll
-              for (int u = 0; u < KBC; ++u) {
-                const uint64_t adesc = smem_desc<RB>(a_slot + u * A_BYTES);
-                const uint64_t bdesc = smem_desc<RB>(b_slot + u * B_BYTES);
-#pragma unroll
-                for (int kk = 0; kk < BK / 16; ++kk)
-                  umma_f16(d, adesc + (uint64_t)(kk * 2), bdesc + (uint64_t)(kk * 2), idesc,
-                           (acc0 | (uint32_t)(u | kk)) ? 1u : 0u);
-              }
-              started |= 1u << g;
-              umma_commit(bar(&ctl->a_empty[ra.slot]));  // slot is free once these MMAs have read it
-              ra.advance();
-            }
-            umma_commit(bar(&ctl->b_empty[rb.slot]));
-            rb.advance();
+            umma_commit(a_free);  // the slots are free once these instructions have read them
+            umma_commit(b_free);
           }
         }
-        if (started && ok) umma_commit(bar(&ctl->acc_full[ab]));  // accumulators of this supertile complete
-        else mbar_arrive(bar(&ctl->acc_full[ab]));
+        if (acc && ok) umma_commit(bar(&ctl->acc_full[ab][g]));  // the sub-tile's accumulator is complete
+        else mbar_arrive(bar(&ctl->acc_full[ab][g]));
         if (++ab == NBUF) { ab = 0; aphase ^= 1; }
       }
     }
     __syncwarp();
   } else {
-    // ================================================================ epilogue (warps 0..3)
+    // ================================================================ epilogue (warps 0..7)
+    // Four warps per sub-tile; with a single sub-tile the second four take the upper half of its columns.  A load issued by
+    // these warps waits its turn behind the gather's copies (2 000 to 5 000 clocks), so the residual of 64 columns is
+    // requested at once, the first of them before the wait for the accumulators: one row at a time in four warps, 32
+    // columns by 32, the residual of a 96-channel layer cost a quarter of its time.
     wait_for_primary();
     // (a launch that overlaps the one before it may have started before that one failed)
     const bool poison = *(volatile const int32_t*)p.dev_status == (int)WCN_ERR_WAIT_EXPIRED;
-    int ib = 0, iphase = 0, ab = 0, aphase = 0;
+    const int half = warp >> 2, g = G == 2 ? half : 0, row = tid & (BLOCK_M - 1);
+    const int middle = ((BN / 16 + 1) / 2) * 16;
+    const int c_begin = G == 2 || half == 0 ? 0 : middle, c_end = G == 2 || half == 1 ? BN : middle;
+    constexpr int CHUNK = RES && sizeof(TO) == 2 ? 64 : 32;   // columns per turn (whose residual is held in registers)
+    constexpr int PIECE = RES ? 16 : 32;                       // columns per tensor-memory load
+    int ab = 0, aphase = 0;
     const bool affine = p.scale != nullptr || p.shift != nullptr;
-    // One 16-column piece of this thread's row: affine, residual, ReLU, convert, store.
-    auto finish16 = [&](float (&y)[16], int c0, TO* orow, const TO* rrow) {
-      if (affine) {
-#pragma unroll
-        for (int q = 0; q < 4; ++q) {
-          const float4 s4 = *reinterpret_cast<const float4*>(&ctl->sc[c0 + 4 * q]);
-          const float4 h4 = *reinterpret_cast<const float4*>(&ctl->sh[c0 + 4 * q]);
-          y[4 * q + 0] = fmaf(y[4 * q + 0], s4.x, h4.x);
-          y[4 * q + 1] = fmaf(y[4 * q + 1], s4.y, h4.y);
-          y[4 * q + 2] = fmaf(y[4 * q + 2], s4.z, h4.z);
-          y[4 * q + 3] = fmaf(y[4 * q + 3], s4.w, h4.w);
-        }
-      }
-      if (rrow) {
-        float res[16];
-        OutVec<TO>::load(rrow + c0, res, p.wide_res);
-#pragma unroll
-        for (int i = 0; i < 16; ++i) y[i] += res[i];
-      }
-      if (p.relu) {
-#pragma unroll
-        for (int i = 0; i < 16; ++i) y[i] = fmaxf(y[i], 0.f);
-      }
-      if (poison) {
-#pragma unroll
-        for (int i = 0; i < 16; ++i) y[i] = __int_as_float(0x7FC00000);
-      }
-      OutVec<TO>::store(orow + c0, y, p.wide_out);
-    };
-    const bool sliced = p.S > 1;  // leave raw fp32 sums in shared memory instead of finishing rows
-    // This thread's output rows in the two sub-tiles of a unit.  With rows in tile order they come from
-    // `out_rows`, and a load issued when its value is needed costs the epilogue a full memory latency per
-    // sub-tile (the gather keeps the memory system busy): the rows of the next unit are read while this one
-    // is finished.
-    auto unit_rows = [&](int64_t wu, int32_t (&rows)[MAX_G]) {
-      const int64_t first = (sliced ? wu / p.S : wu) * G * BLOCK_M + tid;
-#pragma unroll
-      for (int g = 0; g < MAX_G; ++g) {
-        const int64_t slot = first + (int64_t)g * BLOCK_M;
-        rows[g] = (g < G && slot < p.M) ? (p.out_rows ? __ldg(&p.out_rows[slot]) : (int32_t)slot) : -1;
-      }
-    };
-    int32_t next_rows[MAX_G];
-    if ((int64_t)blockIdx.x < p.units) unit_rows(blockIdx.x, next_rows);
-    for (int64_t wu = blockIdx.x; wu < p.units && ok; wu += gridDim.x) {
-      const int64_t st = sliced ? wu / p.S : wu;
-      int32_t rows[MAX_G];
-#pragma unroll
-      for (int g = 0; g < MAX_G; ++g) rows[g] = next_rows[g];
-      if (wu + gridDim.x < p.units) unit_rows(wu + gridDim.x, next_rows);
-      if (ok) ok = mbar_wait(bar(&ctl->info_full[ib]), iphase, p.dev_status);
-      const uint32_t gm0 = ok ? ctl->info_mask[ib][0] : 0u, gm1 = ok ? ctl->info_mask[ib][1] : 0u;
-      mbar_arrive(bar(&ctl->info_empty[ib]));  // only the masks were needed
-      if (++ib == 2) { ib = 0; iphase ^= 1; }
-      if (ok) ok = mbar_wait(bar(&ctl->acc_full[ab]), aphase, p.dev_status);
-      // tcgen05.ld is warp-collective, so the decision to read must be warp-uniform
+    for (int n = 0; ok; ++n) {
+      const int ib = n & 1;
+      ok = mbar_wait(bar(&ctl->info_full[ib]), (n >> 1) & 1, p.dev_status);
       if (!__all_sync(0xFFFFFFFFu, ok)) { ok = false; break; }
-      tc_fence_after();
-      const int64_t m0 = st * G * BLOCK_M;
-      // (neither loop is unrolled: the epilogue's code is shared by all sub-tiles and column pieces, which
-      // keeps the kernel's instruction footprint — five roles run side by side on a multiprocessor — small)
+      const bool last = ctl->info_unit[ib] < 0;
+      const bool any = ctl->info_mask[ib][g] != 0;
+      // This thread's output row (-1 past the end), loaded by the index warps: another latency that is not paid here.
+      const int64_t m = ctl->out_row[ib][g * BLOCK_M + row];
+      __syncwarp();
+      if (lane == 0) mbar_arrive(bar(&ctl->info_empty[ib]));
+      if (last) break;
+      if (p.S > 1) continue;  // the slices' sums are finished behind the roles
+      const bool live = m >= 0;
+      const uint32_t trow = tmem_base + ((uint32_t)((warp & 3) * 32) << 16) + (uint32_t)((ab * G + g) * p.cols);
+      TO* orow = reinterpret_cast<TO*>(p.out) + m * p.out_ld + n0;
+      const TO* rrow = RES && live ? reinterpret_cast<const TO*>(p.residual) + m * p.res_ld + n0 : nullptr;
+      bool ready = false;
 #pragma unroll 1
-      for (int g = 0; g < G; ++g) {
-        if (m0 + (int64_t)g * BLOCK_M >= p.M) break;
-        const uint32_t gmask = g == 0 ? gm0 : gm1;
-        const int64_t slot = m0 + (int64_t)g * BLOCK_M + tid;
-        const int64_t m = g == 0 ? rows[0] : rows[1];   // -1 past the end: never stored
-        const bool live = slot < p.M;
-        const uint32_t trow = tmem_base + ((uint32_t)(warp * 32) << 16) + (uint32_t)((ab * G + g) * p.cols);
-        TO* orow = reinterpret_cast<TO*>(p.out) + m * p.out_ld + n0;
-        const TO* rrow = p.residual ? reinterpret_cast<const TO*>(p.residual) + m * p.res_ld + n0 : nullptr;
-        // this slice's sums of the row, where the ring was (every slot has been consumed)
-        float* prow = reinterpret_cast<float*>(gen) + tid * (BN + 4);
-#pragma unroll 1
-        for (int c0 = 0; c0 < BN; c0 += 32) {  // two TMEM loads in flight per wait (BN is a multiple of 16)
-          const bool two = c0 + 16 < BN;
-          float y0[16], y1[16];
-          if (gmask) {
-            uint32_t r0[16], r1[16];
-            tmem_ld16(trow + (uint32_t)c0, r0);  // executed by all lanes of the warp
-            if (two) tmem_ld16(trow + (uint32_t)c0 + 16u, r1);
-            tmem_ld_wait();
+      for (int cb = c_begin; cb < c_end || !ready; cb += CHUNK) {  // (a half without columns waits all the same)
+        __align__(32) TO res[CHUNK];
+        if (rrow) {
 #pragma unroll
-            for (int i = 0; i < 16; ++i) { y0[i] = __uint_as_float(r0[i]); y1[i] = two ? __uint_as_float(r1[i]) : 0.f; }
+          for (int q = 0; q < CHUNK; q += 16)
+            if (cb + q < c_end) load_raw16(rrow + cb + q, res + q, p.wide_res);
+        }
+        if (!ready) {
+          // tcgen05.ld is warp-collective, so the decision to read must be warp-uniform
+          ok = mbar_wait(bar(&ctl->acc_full[ab][g]), aphase, p.dev_status);
+          if (!__all_sync(0xFFFFFFFFu, ok)) { ok = false; break; }
+          tc_fence_after();
+          ready = true;
+        }
+#pragma unroll
+        for (int q = 0; q < CHUNK; q += PIECE) {
+          const int c0 = cb + q;
+          if (c0 >= c_end) break;
+          uint32_t r[PIECE / 16][16];
+          if (any) {
+#pragma unroll
+            for (int h = 0; h < PIECE / 16; ++h)
+              if (h == 0 || c0 + 16 < c_end) tmem_ld16(trow + (uint32_t)(c0 + 16 * h), r[h]);  // executed by all lanes of the warp
+            tmem_ld_wait();
           } else {
 #pragma unroll
-            for (int i = 0; i < 16; ++i) y0[i] = y1[i] = 0.f;
-          }
-          if (sliced) {
+            for (int h = 0; h < PIECE / 16; ++h)
 #pragma unroll
-            for (int q = 0; q < 4; ++q) {
-              *reinterpret_cast<float4*>(prow + c0 + 4 * q) = make_float4(y0[4 * q], y0[4 * q + 1], y0[4 * q + 2], y0[4 * q + 3]);
-              if (two) *reinterpret_cast<float4*>(prow + c0 + 16 + 4 * q) = make_float4(y1[4 * q], y1[4 * q + 1], y1[4 * q + 2], y1[4 * q + 3]);
+              for (int i = 0; i < 16; ++i) r[h][i] = 0u;
+          }
+          if (live) {
+#pragma unroll
+            for (int h = 0; h < PIECE / 16; ++h) {
+              const int c = c0 + 16 * h;
+              if (h > 0 && c >= c_end) break;
+              // affine, residual, ReLU, convert, store
+              float y[16];
+#pragma unroll
+              for (int i = 0; i < 16; ++i) y[i] = __uint_as_float(r[h][i]);
+              if (affine) {
+#pragma unroll
+                for (int i = 0; i < 16; i += 4) {
+                  const float4 s4 = *reinterpret_cast<const float4*>(&ctl->sc[c + i]);
+                  const float4 h4 = *reinterpret_cast<const float4*>(&ctl->sh[c + i]);
+                  y[i + 0] = fmaf(y[i + 0], s4.x, h4.x);
+                  y[i + 1] = fmaf(y[i + 1], s4.y, h4.y);
+                  y[i + 2] = fmaf(y[i + 2], s4.z, h4.z);
+                  y[i + 3] = fmaf(y[i + 3], s4.w, h4.w);
+                }
+              }
+              if (RES) {
+#pragma unroll
+                for (int i = 0; i < 16; ++i) y[i] += wcn_to_float<TO>(res[q + i]);
+              }
+              if (p.relu) {
+#pragma unroll
+                for (int i = 0; i < 16; ++i) y[i] = fmaxf(y[i], 0.f);
+              }
+              if (poison) {
+#pragma unroll
+                for (int i = 0; i < 16; ++i) y[i] = __int_as_float(0x7FC00000);
+              }
+              store16<TO>(orow + c, y, p.wide_out);
             }
-          } else if (live) {
-            finish16(y0, c0, orow, rrow);
-            if (two) finish16(y1, c0 + 16, orow, rrow);
           }
         }
       }
+      if (!ok) break;
       tc_fence_before();
-      mbar_arrive(bar(&ctl->acc_empty[ab]));   // accumulator set may be overwritten
+      mbar_arrive(bar(&ctl->acc_empty[ab][g]));   // the accumulator may be overwritten
       if (++ab == NBUF) { ab = 0; aphase ^= 1; }
     }
   }
   if (p.S > 1) {
     // ================================================================ the cluster adds its slices
+    // Eight warps leave this slice's sums in shared memory, where the ring was (every slot has been consumed); then each CTA
+    // finishes 1 / S of the rows.  Reading 128 x BN sums from the other CTAs is what this costs, so every CTA starts with
+    // its own slice and goes round: all starting with slice 0 made one multiprocessor serve the whole cluster.  They are
+    // added in slice order, whichever CTA finishes the row: the sum does not depend on where the row lies in its tile.
     __syncwarp();
+    if (warp < 8) {
+      bool have = __all_sync(0xFFFFFFFFu, ok);
+      if (have) have = mbar_wait(bar(&ctl->acc_full[0][0]), 0, p.dev_status);
+      if (__all_sync(0xFFFFFFFFu, have)) {
+        tc_fence_after();
+        const bool any = ctl->info_mask[0][0] != 0;
+        const int q = warp & 3;
+        float* prow = reinterpret_cast<float*>(gen) + (q * 32 + lane) * (BN + 4);
+#pragma unroll 1
+        for (int c0 = (warp >> 2) * 16; c0 < BN; c0 += 32) {
+          uint32_t r[16];
+          if (any) {
+            tmem_ld16(tmem_base + ((uint32_t)(q * 32) << 16) + (uint32_t)c0, r);
+            tmem_ld_wait();
+          } else {
+#pragma unroll
+            for (int i = 0; i < 16; ++i) r[i] = 0u;
+          }
+#pragma unroll
+          for (int i = 0; i < 16; i += 4) *reinterpret_cast<uint4*>(prow + c0 + i) = make_uint4(r[i], r[i + 1], r[i + 2], r[i + 3]);
+        }
+      }
+    }
     cluster_meet();  // every slice's sums are in its CTA's shared memory
-    if (tid == 0) ctl->failed = *(volatile const int32_t*)p.dev_status == (int)WCN_ERR_WAIT_EXPIRED;
-    __syncthreads();
+    const int32_t status = *(volatile const int32_t*)p.dev_status;
     const int64_t st = blockIdx.x / p.S;
     const int rank = (int)(blockIdx.x - st * p.S), per_row = BN / 4;
     const int r0 = rank * BLOCK_M / p.S, r1 = (rank + 1) * BLOCK_M / p.S;
@@ -718,7 +784,16 @@ conv_tcgen05_kernel(const ConvTcParams p) {
       float4 v[MAX_SLICES];
 #pragma unroll
       for (int s = 0; s < MAX_SLICES; ++s)
-        if (s < p.S) v[s] = ld_cluster(at, (uint32_t)s);
+        if (s < p.S && s >= rank) v[s] = ld_cluster(at, (uint32_t)s);
+#pragma unroll
+      for (int s = 0; s < MAX_SLICES; ++s)
+        if (s < rank) v[s] = ld_cluster(at, (uint32_t)s);
+      __align__(16) TO o[4], res[4];
+      if (RES) {
+        const TO* rrow = reinterpret_cast<const TO*>(p.residual) + m * p.res_ld + n0 + c;
+        if (sizeof(TO) == 4) *reinterpret_cast<uint4*>(res) = __ldg(reinterpret_cast<const uint4*>(rrow));
+        else *reinterpret_cast<uint2*>(res) = __ldg(reinterpret_cast<const uint2*>(rrow));
+      }
       float y[4] = {v[0].x, v[0].y, v[0].z, v[0].w};
 #pragma unroll
       for (int s = 1; s < MAX_SLICES; ++s) {
@@ -727,14 +802,12 @@ conv_tcgen05_kernel(const ConvTcParams p) {
           y[2] = __fadd_rn(y[2], v[s].z); y[3] = __fadd_rn(y[3], v[s].w);
         }
       }
-      __align__(16) TO o[4];
-      const TO* rrow = p.residual ? reinterpret_cast<const TO*>(p.residual) + m * p.res_ld + n0 + c : nullptr;
 #pragma unroll
       for (int j = 0; j < 4; ++j) {
         y[j] = fmaf(y[j], ctl->sc[c + j], ctl->sh[c + j]);  // (1 and 0 when there is no affine step)
-        if (rrow) y[j] += wcn_to_float<TO>(rrow[j]);
+        if (RES) y[j] += wcn_to_float<TO>(res[j]);
         if (p.relu) y[j] = fmaxf(y[j], 0.f);
-        if (ctl->failed) y[j] = __int_as_float(0x7FC00000);
+        if (status == (int)WCN_ERR_WAIT_EXPIRED) y[j] = __int_as_float(0x7FC00000);
         o[j] = wcn_from_float<TO>(y[j]);
       }
       TO* dst = reinterpret_cast<TO*>(p.out) + m * p.out_ld + n0 + c;
@@ -782,29 +855,59 @@ __global__ void pack_weight_kernel(const TS* __restrict__ w, TD* __restrict__ pa
 
 inline int pick_bk(int c_in) { return c_in % 64 == 0 ? 64 : 32; }
 
+// CTAs that can be resident at once in clusters of S (they stay inside a group of multiprocessors, whose sizes differ).
+int resident_ctas(int S) {
+  static std::atomic<int> known[64][MAX_SLICES + 1];
+  int dev = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return wcn_num_sms();
+  if (S == 1) return wcn_num_sms();
+  int n = known[dev][S].load(std::memory_order_relaxed);
+  if (n == 0) {
+    auto kern = conv_tcgen05_kernel<64, 1, false, false, __half, false>;  // (one CTA per multiprocessor, like every instance)
+    cudaLaunchAttribute attr = {};
+    attr.id = cudaLaunchAttributeClusterDimension;
+    attr.val.clusterDim.x = (unsigned)S;
+    attr.val.clusterDim.y = attr.val.clusterDim.z = 1;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3((unsigned)S);
+    cfg.blockDim = dim3(THREADS);
+    cfg.dynamicSmemBytes = SMEM_LIMIT;
+    cfg.attrs = &attr;
+    cfg.numAttrs = 1;
+    int clusters = 0;
+    if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_LIMIT) != cudaSuccess ||
+        cudaOccupancyMaxActiveClusters(&clusters, kern, &cfg) != cudaSuccess || clusters < 1) {
+      (void)cudaGetLastError();
+      clusters = wcn_num_sms() / (2 * S);
+    }
+    n = clusters * S;
+    known[dev][S].store(n, std::memory_order_relaxed);
+  }
+  return n;
+}
+
 // Launch geometry.  A problem with fewer 128-row tiles than multiprocessors cannot occupy the GPU with one CTA per tile:
 // its kernel offsets are divided among S CTAs of a cluster and its output columns among blocks of their own (which gather
-// the rows again), whichever combination of the two moves the fewest bytes through one multiprocessor (split_k: 0 =
-// decide here, 1 = columns only, >= 2 = that many slices, at most eight; < 0 = -split_k column blocks).
+// the rows again), whichever combination of the two is expected to take least (split_k: 0 = decide here, 1 = columns only,
+// >= 2 = that many slices, at most eight; < 0 = -split_k column blocks).
 //
-// The model: a CTA reads n_off * (A + B) bytes, A = its 128 rows, B = its columns' weights at one offset, from L2 at the
-// ~100 KB/us one multiprocessor sustains; of K offsets about 0.6 K have a neighbour in a tile; adding the slices
-// costs about 1.5 us.  Clusters of S fit 8 * floor(18 / S) times (eight GPCs of at least 18 multiprocessors), and CTAs
-// beyond what fits wait for a second wave.
+// The model: a CTA reads n_off * (A + B) bytes, A = its 128 rows, B = its columns' weights at one offset, at the ~68 KB/us
+// that one multiprocessor sustains; of K offsets about 0.6 K have a neighbour in a tile; adding the slices costs 1.3 us and
+// 0.0165 us per column (128 sums of every column come through the cluster's network).  Within 1.5 us of the best of all
+// combinations for 128 to 9 000 rows and 32 to 256 channels.
 void pick_split(const ConvTcParams& p, int64_t tiles, int split_k, int* slices, int* blocks) {
-  const int sms = wcn_num_sms();
   *slices = *blocks = 1;
   double best = 1e30;
   for (int S = 1; S <= MAX_SLICES && S <= p.K; ++S) {
     if (split_k == 1 && S > 1) break;
-    const int64_t fit = S == 1 ? sms : (int64_t)S * (18 / S) * 8 * sms / 148;
+    const int64_t fit = resident_ctas(S);
     for (int nb = 1; nb <= 8; nb *= 2) {
       if (p.c_out % (16 * nb) != 0 || (nb > 1 && p.c_out / nb < 32)) break;
       const int64_t ctas = tiles * S * nb;
       if (ctas > fit && ctas > tiles) continue;
       const double off = (p.K > 2 ? 0.6 * p.K : p.K) / S;
       const double bytes = (off < 1 ? 1 : off) * 2.0 * p.c_in * (BLOCK_M + p.c_out / nb);
-      const double us = bytes / 100e3 + (S > 1 ? 1.5 : 0.0);
+      const double us = bytes / 68e3 + (S > 1 ? 1.3 + 0.0165 * (p.c_out / nb) : 0.0);
       if (us < best) { best = us; *slices = S; *blocks = nb; }
     }
   }
@@ -834,22 +937,21 @@ bool plan_launch(ConvTcParams& p, int bk, int split_k, size_t* smem, dim3* grid)
   int g = S > 1 ? 1 : 2;
   while (g > 1 && ((tiles + g - 1) / g) * split * S < 2 * (int64_t)sms) g /= 2;
   const size_t a_unit = (size_t)BLOCK_M * bk * 2, b_unit = (size_t)p.block_n * bk * 2;
-  const size_t limit = 226 * 1024;  // the kernels opt in to this much dynamic shared memory
+  const size_t limit = SMEM_LIMIT;
   const int kb_total = p.c_in / bk;
   // Channel slices per ring slot: as many as give a 32 KiB row slot, fewer if the rings would not fit.
   // (with a single slice per offset the slot spans that many active offsets instead)
-  int kbc = (int)((32 * 1024) / a_unit);
+  int kbc = (int)(32 * 1024 / a_unit);
   if (kb_total > 1 && kbc > kb_total) kbc = kb_total;
   if (kb_total == 1 && kbc > p.K) kbc = p.K;
-  if (kbc > 4) kbc = 4;
   if (kbc < 1) kbc = 1;
   while (kb_total > 1 && kb_total % kbc != 0) --kbc;
   size_t fixed = 0, a_stage = 0, b_stage = 0;
-  for (;;) {  // two staged neighbour tables + a few row slots and 2 weight slots must fit
-    fixed = 1024 + sizeof(Control) + 2 * (size_t)g * p.K * BLOCK_M * 4 + 128;
-    a_stage = kbc * a_unit;
+  for (;;) {  // the staged row lists and two slots of every ring must fit
+    fixed = 1024 + sizeof(Control) + (size_t)g * staged_lists(p.K) * BLOCK_M * 4 + 128;
+    a_stage = g * kbc * a_unit;
     b_stage = kbc * b_unit;
-    if (fixed + (kbc > 1 ? 3 : 4) * a_stage + 2 * b_stage <= limit) break;
+    if (fixed + 2 * a_stage + 2 * b_stage <= limit) break;
     if (kbc > 1) {
       do { --kbc; } while (kb_total > 1 && kb_total % kbc != 0);
       continue;
@@ -862,40 +964,54 @@ bool plan_launch(ConvTcParams& p, int bk, int split_k, size_t* smem, dim3* grid)
   p.nbuf = (g * cols * 2 <= 512) ? 2 : 1;
   p.supertiles = (tiles + g - 1) / g;
   p.units = p.supertiles * S;
-  const size_t budget = limit - fixed;
-  int sb = 3;
-  while (sb > 2 && sb * b_stage > budget / 2) --sb;
-  int sa = (int)((budget - sb * b_stage) / a_stage);
-  if (sa > MAX_RING) sa = MAX_RING;
-  if (sa < 2) return false;
-  // leftover room goes to the weight ring
-  while (sb < 6 && fixed + sa * a_stage + (sb + 1) * b_stage <= limit) ++sb;
+  // Row slots first up to three per sub-tile, then a third weight slot (with two, the fetch of one waits for the last
+  // instruction on the other), then whatever still fits.
+  int sa = 2, sb = 2;
+  for (;;) {
+    const size_t used = fixed + sa * a_stage + sb * b_stage;
+    const bool more_a = sa < MAX_RING && used + a_stage <= limit, more_b = sb < 6 && used + b_stage <= limit;
+    if (more_a && (sa < 3 || (sb >= 3 && (sa < 4 || sb >= 4 || !more_b)))) ++sa;
+    else if (more_b) ++sb;
+    else if (more_a) ++sa;
+    else break;
+  }
   p.sa = sa;
   p.sb = sb;
   // the sums of a slice take the place of the rings
   if (S > 1 && sa * a_stage + sb * b_stage < (size_t)BLOCK_M * (p.block_n + 4) * 4) return false;
   *smem = fixed + sa * a_stage + sb * b_stage;
+  // With four units or more per multiprocessor one CTA per unit is launched, and the first to start claim the rest.  With
+  // fewer, claims made two units ahead deal unevenly (the first CTAs take three units, the last one: 36 -> 47 us for 80 000
+  // rows of 64 channels), and fixed strides let the next launch begin while the last units run.  (Column blocks are made of
+  // problems that fit at once; asked for on larger ones, their CTAs keep the strides: a claim could return another block's.)
   int64_t gx = p.units;
   const int64_t cap = sms / split > 0 ? sms / split : 1;
-  if (gx > cap && S == 1) gx = cap;
+  p.claim = S == 1 && split == 1 && gx >= 4 * cap;
+  if (gx > cap && S == 1 && !p.claim) gx = cap;
   *grid = dim3((unsigned)gx, (unsigned)split);
   return true;
 }
 
-template <int BK, int KBC, bool SPAN, bool BF16, typename TO>
-int launch_kbc(const ConvTcParams& p, size_t smem, dim3 grid, cudaStream_t st) {
-  auto kern = conv_tcgen05_kernel<BK, KBC, SPAN, BF16, TO>;
+template <int BK, int KBC, bool SPAN, bool BF16, typename TO, bool RES>
+int launch_kernel(const ConvTcParams& p, size_t smem, dim3 grid, cudaStream_t st) {
+  auto kern = conv_tcgen05_kernel<BK, KBC, SPAN, BF16, TO, RES>;
   static bool configured[64] = {};  // per template instance and device: opt in to large shared memory once
   int dev = 0;
   if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return WCN_ERR_INITIALIZATION;
   if (!configured[dev]) {
-    if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, 226 * 1024) != cudaSuccess) {
+    if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_LIMIT) != cudaSuccess) {
       (void)cudaGetLastError();  // do not leave a sticky error for the caller's next CUDA call
       return WCN_ERR_INITIALIZATION;
     }
     configured[dev] = true;
   }
   return wcn_launch(kern, grid, dim3(THREADS), smem, st, (unsigned)p.S, p);
+}
+
+template <int BK, int KBC, bool SPAN, bool BF16, typename TO>
+int launch_kbc(const ConvTcParams& p, size_t smem, dim3 grid, cudaStream_t st) {
+  return p.residual ? launch_kernel<BK, KBC, SPAN, BF16, TO, true>(p, smem, grid, st)
+                    : launch_kernel<BK, KBC, SPAN, BF16, TO, false>(p, smem, grid, st);
 }
 
 template <int BK, bool BF16, typename TO>
@@ -905,22 +1021,22 @@ int launch_tc(ConvTcParams& p, int split_k, cudaStream_t st) {
   if (!plan_launch(p, BK, split_k, &smem, &grid)) return WCN_ERR_UNSUPPORTED_CONFIG;
   // SPAN: the whole C_in is one slice and a ring slot holds KBC consecutive active offsets; otherwise a
   // slot holds KBC channel slices of one offset.  A compile-time choice, so that every role's loop
-  // carries only the form it runs.
+  // carries only the form it runs.  (A slot holds at most 32 KiB: two slices of 64 channels, four of 32.)
   if (p.kbc > 1 && p.c_in == BK) {
-    switch (p.kbc) {
-      case 2: return launch_kbc<BK, 2, true, BF16, TO>(p, smem, grid, st);
-      case 3: return launch_kbc<BK, 3, true, BF16, TO>(p, smem, grid, st);
-      case 4: return launch_kbc<BK, 4, true, BF16, TO>(p, smem, grid, st);
-      default: return WCN_ERR_UNSUPPORTED_CONFIG;
+    if (p.kbc == 2) return launch_kbc<BK, 2, true, BF16, TO>(p, smem, grid, st);
+    if constexpr (BK == 32) {
+      if (p.kbc == 3) return launch_kbc<BK, 3, true, BF16, TO>(p, smem, grid, st);
+      if (p.kbc == 4) return launch_kbc<BK, 4, true, BF16, TO>(p, smem, grid, st);
     }
+    return WCN_ERR_UNSUPPORTED_CONFIG;
   }
-  switch (p.kbc) {
-    case 1: return launch_kbc<BK, 1, false, BF16, TO>(p, smem, grid, st);
-    case 2: return launch_kbc<BK, 2, false, BF16, TO>(p, smem, grid, st);
-    case 3: return launch_kbc<BK, 3, false, BF16, TO>(p, smem, grid, st);
-    case 4: return launch_kbc<BK, 4, false, BF16, TO>(p, smem, grid, st);
-    default: return WCN_ERR_UNSUPPORTED_CONFIG;
+  if (p.kbc == 1) return launch_kbc<BK, 1, false, BF16, TO>(p, smem, grid, st);
+  if (p.kbc == 2) return launch_kbc<BK, 2, false, BF16, TO>(p, smem, grid, st);
+  if constexpr (BK == 32) {
+    if (p.kbc == 3) return launch_kbc<BK, 3, false, BF16, TO>(p, smem, grid, st);
+    if (p.kbc == 4) return launch_kbc<BK, 4, false, BF16, TO>(p, smem, grid, st);
   }
+  return WCN_ERR_UNSUPPORTED_CONFIG;
 }
 
 // A barrier phase that cannot complete (one arrival of two), waited for with a short limit:

@@ -168,7 +168,7 @@ conv_wgrad_tcgen05_kernel(const WgradParams p) {
     if (bad) wcn_report_bounds(p.dev_status);
   } else if (warp == WG_MMA_WARP) {
     // ================================================================ MMA issuer
-    if (lane == 0) {
+    if (elect_one()) {
       // fp32 accumulate, A and B MN-major (bits 15, 16), N = c_out, M = 128
       const uint32_t idesc = (1u << 4) | ((BF16 ? 1u : 0u) << 7) | ((BF16 ? 1u : 0u) << 10) | (1u << 15) | (1u << 16) |
                              ((uint32_t)(p.c_out >> 3) << 17) | ((uint32_t)(128 >> 4) << 24);

@@ -36,6 +36,18 @@ __device__ __forceinline__ bool mbar_try_wait(uint32_t bar, uint32_t parity) {
       : "memory");
   return done != 0;
 }
+// A look at the barrier without waiting.
+__device__ __forceinline__ bool mbar_test(uint32_t bar, uint32_t parity) {
+  uint32_t done;
+  asm volatile(
+      "{\n\t.reg .pred p;\n\t"
+      "mbarrier.test_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
+      "selp.u32 %0, 1, 0, p;\n\t}"
+      : "=r"(done)
+      : "r"(bar), "r"(parity)
+      : "memory");
+  return done != 0;
+}
 // Bounded wait.  Returns false when the deadline passed or another thread's wait already ran
 // out.  The status word lives in global memory and is looked at about once per millisecond of
 // waiting.  An expired wait overrides whatever the word held (a skipped out-of-range index is
@@ -130,6 +142,16 @@ __device__ __forceinline__ void tmem_alloc(uint32_t holder_smem, uint32_t cols) 
 }
 __device__ __forceinline__ void tmem_dealloc(uint32_t taddr, uint32_t cols) {
   asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(taddr), "r"(cols) : "memory");
+}
+
+// The thread of a (converged) warp that issues tensor-core instructions and bulk copies.  Chosen with elect.sync rather
+// than by lane number: the compiler then knows that one thread executes the branch and keeps descriptors and addresses
+// in uniform registers.  Behind `lane == 0` four M = 128 x N = 64 x K = 16 instructions and a commit took 323 clocks,
+// behind elect.sync 193 (the tensor core's own rate: 48 clocks each; 80 -> 64 at N = 128).
+__device__ __forceinline__ bool elect_one() {
+  uint32_t one;
+  asm volatile("{\n\t.reg .pred P;\n\telect.sync _|P, 0xFFFFFFFF;\n\tselp.u32 %0, 1, 0, P;\n\t}" : "=r"(one));
+  return one != 0;
 }
 
 __device__ __forceinline__ void umma_f16(uint32_t d_tmem, uint64_t a_desc, uint64_t b_desc, uint32_t idesc,
