@@ -22,7 +22,11 @@
 // four gather warps per sub-tile, issuing threads that share nothing but the weight slots and look at the next barriers
 // early, instructions issued behind elect.sync, lists of present offsets only (their 27 KB became row slots) and claimed
 // units: C = 32 / 64 / 96 / 128 / 256 from 94 / 133 / 158 / 201 / 636 us to 86 / 118 / 152 / 186 / 520 us (256: 1.17
-// PFLOP/s); outdoor scene, 128 -> 96, 777 777 rows: 418 -> 359 us; MinkUNet-34 over 1.2 M voxels: 4.77 -> 4.50 ms.
+// PFLOP/s); outdoor scene, 128 -> 96, 777 777 rows: 418 -> 359 us; MinkUNet-34 over 1.2 M voxels: 4.77 -> 4.50 ms.  Then
+// a shorter way to the first copy of a launch - the first unit's neighbour loads issued before the barriers are set up, a
+// single unit's table published without a rendezvous of the index warps, no look at the status word on the way (the epilogue
+// reads it and writes NaN where an earlier launch gave up): C = 32 / 64 / 96 81 / 113 / 144 us, the network over one
+// scene of 20 000 voxels 928 -> 855 us, over 1.2 M 4.41 ms.
 //
 // Problems with fewer 128-row tiles than multiprocessors divide the kernel offsets of a tile among the S CTAs of a
 // cluster ("split-K over kernel offsets": slice s owns the offsets k with k % S == s, which deals the frequent central
@@ -196,7 +200,6 @@ struct Control {
   int info_entry[2][MAX_G];       // first staged row list of each sub-tile
   uint32_t mask_acc[3][MAX_G];    // index warps' scratch while building the masks
   uint32_t tmem_holder;
-  int skip;
   int32_t out_row[2][MAX_G * BLOCK_M];          // output row of each slot, -1 past the end
   __align__(16) float sc[256], sh[256];         // this CTA's columns of the epilogue scale / shift (1 / 0 when absent)
 };
@@ -255,6 +258,25 @@ conv_tcgen05_kernel(const ConvTcParams p) {
   // One rendezvous behind the whole set-up (an earlier form, a thread at a time behind two, took 2 000 clocks: a microsecond
   // of each of the sixty launches of a small network).
   if (!p.claim) launch_dependents();
+  // The index warps' share of a unit: 128 rows of one sub-tile in four warps (for a single sub-tile four take the even and
+  // four the odd offsets).  The first unit's loads are on their way while the barriers are set up.
+  const int itid = tid - EPI_THREADS, irow = itid & (BLOCK_M - 1);
+  const uint32_t mine = G == 2 ? 0xFFFFFFFFu : itid >= BLOCK_M ? 0xAAAAAAAAu : 0x55555555u;   // this thread's offsets
+  const bool single = !p.claim && (int64_t)gridDim.x >= p.units;                               // one unit per CTA
+  int r[MAX_OFFSETS];
+  int32_t out_row = -1;
+  auto load_lists = [&](int64_t unit) {
+    const int64_t st = p.S > 1 ? unit / p.S : unit;
+    const uint32_t kmask = slice_mask((int)(unit - st * p.S), p.S) & mine;
+    const int64_t m = (st * G + (G == 2 ? itid >> 7 : 0)) * BLOCK_M + irow;
+    const int32_t* at = p.nbr + m;
+#pragma unroll
+    for (int k = 0; k < MAX_OFFSETS; ++k)
+      r[k] = k < K && ((kmask >> k) & 1u) && m < p.M ? __ldg(at + (int64_t)k * p.M) : -1;
+    out_row = m < p.M ? (p.out_rows ? __ldg(&p.out_rows[m]) : (int32_t)m) : -1;
+  };
+  const bool indexing = warp >= EPI_THREADS / 32 && warp < GATHER_WARP0;
+  if (indexing) load_lists(blockIdx.x);
   const uint32_t tmem_total = (uint32_t)(NBUF * G * p.cols);
   if (warp == 0) {
     for (int g = 0; g < G; ++g)
@@ -267,10 +289,9 @@ conv_tcgen05_kernel(const ConvTcParams p) {
     }
     if (lane < CLAIMS) mbar_init(bar(&ctl->claim_full[lane]), 1);
     if (lane < 3) ctl->mask_acc[lane][0] = ctl->mask_acc[lane][1] = 0;
+    if (lane < 2) ctl->info_mask[0][lane] = 0;
     if (lane == 3) mbar_init(bar(&ctl->idx_sync), IDX_THREADS);
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-  } else if (warp == 1) {
-    if (lane == 0) ctl->skip = *(volatile int32_t*)p.dev_status;  // an earlier launch on this status word failed
   } else if (warp == MMA_WARP) {
     tmem_alloc(smem_u32(&ctl->tmem_holder), tmem_total < 32 ? 32u : tmem_total);
   } else if (warp >= GATHER_WARP0 && warp < MMA_WARP) {
@@ -283,28 +304,9 @@ conv_tcgen05_kernel(const ConvTcParams p) {
   __syncthreads();
   tc_fence_after();
   bool ok = true;
-  if (ctl->skip == (int)WCN_ERR_WAIT_EXPIRED) {
-    // Nothing is computed after a kernel on this status word gave up.  The rows this CTA would have
-    // produced are filled with NaN so that the failure cannot pass for data (the CTAs of a cluster go on to the
-    // meeting points at the end, which do the same).
-    wait_for_primary();
-    if (p.S == 1) {
-      const TO nan = wcn_from_float<TO>(__int_as_float(0x7FC00000));
-      for (int64_t st = blockIdx.x; st < p.supertiles; st += gridDim.x) {
-        const int64_t m0 = st * G * BLOCK_M;
-        const int64_t rows = min((int64_t)G * BLOCK_M, p.M - m0);
-        for (int64_t i = tid; i < rows * BN; i += THREADS) {
-          const int64_t slot = m0 + i / BN;
-          const int64_t m = p.out_rows ? (int64_t)__ldg(&p.out_rows[slot]) : slot;
-          reinterpret_cast<TO*>(p.out)[m * p.out_ld + n0 + (int)(i % BN)] = nan;
-        }
-      }
-    }
-    ok = false;  // no role does any work
-  }
   const uint32_t tmem_base = ctl->tmem_holder;
 
-  if (warp >= EPI_THREADS / 32 && warp < GATHER_WARP0) {
+  if (indexing) {
     // ================================================================ index warps
     // Choose the next unit and stage what the other roles need of it, one unit ahead of the copies: the output row of
     // every slot, the offsets each sub-tile has any neighbour at, and for each of those the 128 input rows (-1 where a row
@@ -316,9 +318,7 @@ conv_tcgen05_kernel(const ConvTcParams p) {
     // for a single sub-tile, four for the even and four for the odd offsets), loads before the wait for a free entry, units
     // claimed two ahead, one vote per warp.  54 loads and 54 votes in four warps took 14 000 clocks per unit, three times
     // what the copies of a 32-channel layer take.
-    const int itid = tid - EPI_THREADS, row = itid & (BLOCK_M - 1), half = itid >> 7;
-    const int g = G == 2 ? half : 0;
-    const uint32_t mine = G == 2 ? 0xFFFFFFFFu : half ? 0xAAAAAAAAu : 0x55555555u;   // this thread's offsets
+    const int g = G == 2 ? itid >> 7 : 0;
     const int num_in = (int)p.num_in;
     int sphase = 0, entry = 0, before = 0;   // next free entry; entries of the unit before
     int n = 0, acc = 0;                      // units staged; scratch of this unit's masks
@@ -326,6 +326,24 @@ conv_tcgen05_kernel(const ConvTcParams p) {
     bool refused = false;
     bool bad = false;
     int64_t unit = blockIdx.x;
+    if (single) {
+      // A complete table of the one unit: nothing to compact, so the warps need not meet (a microsecond of the few that
+      // such a launch takes).
+      uint32_t has = 0;
+#pragma unroll
+      for (int k = 0; k < MAX_OFFSETS; ++k) {
+        if (r[k] >= num_in) { r[k] = -1; bad = true; }
+        has |= r[k] >= 0 ? 1u << k : 0u;
+        if (k < K && ((mine >> k) & 1u)) rows_idx[(g * K + k) * BLOCK_M + irow] = r[k];
+      }
+      has = __reduce_or_sync(0xFFFFFFFFu, has);
+      if (lane == 0 && has) atomicOr(&ctl->info_mask[0][g], has);
+      if (mine & 1u) ctl->out_row[0][g * BLOCK_M + irow] = out_row;
+      if (itid == 0) { ctl->info_unit[0] = unit; ctl->info_unit[1] = -1; }
+      mbar_arrive(bar(&ctl->info_full[0]));
+      mbar_arrive(bar(&ctl->info_full[1]));
+      unit = -1;
+    }
     auto claim_one = [&](int at) {
       if (itid == 0) {
         // (every index thread has read the slot's last content: they met since)
@@ -334,8 +352,8 @@ conv_tcgen05_kernel(const ConvTcParams p) {
       }
       ++asked;
     };
-    if (p.claim && ok) claim_one(0);
-    while (ok) {
+    if (p.claim) claim_one(0);
+    while (ok && !single) {
       const int ib = n & 1;
       if (n > 0) {  // the unit after the one just staged
         if (!p.claim) {
@@ -362,14 +380,7 @@ conv_tcgen05_kernel(const ConvTcParams p) {
         break;
       }
       if (p.claim && !refused) claim_one(slot == CLAIMS - 1 ? 0 : slot + 1);
-      const int64_t st = p.S > 1 ? unit / p.S : unit;
-      const uint32_t kmask = slice_mask((int)(unit - st * p.S), p.S) & mine;
-      const int64_t m = (st * G + g) * BLOCK_M + row;
-      int r[MAX_OFFSETS];
-#pragma unroll
-      for (int k = 0; k < MAX_OFFSETS; ++k)
-        r[k] = k < K && ((kmask >> k) & 1u) && m < p.M ? __ldg(&p.nbr[(int64_t)k * p.M + m]) : -1;
-      const int32_t out_row = m < p.M ? (p.out_rows ? __ldg(&p.out_rows[m]) : (int32_t)m) : -1;
+      if (n > 0) load_lists(unit);
       if (!mbar_wait(bar(&ctl->info_empty[ib]), ((n >> 1) & 1) ^ 1, p.dev_status)) { ok = false; break; }
       uint32_t has = 0;
 #pragma unroll
@@ -379,7 +390,7 @@ conv_tcgen05_kernel(const ConvTcParams p) {
       }
       has = __reduce_or_sync(0xFFFFFFFFu, has);
       if (lane == 0 && has) atomicOr(&ctl->mask_acc[acc][g], has);
-      if (mine & 1u) ctl->out_row[ib][g * BLOCK_M + row] = out_row;
+      if (mine & 1u) ctl->out_row[ib][g * BLOCK_M + irow] = out_row;
       // all index threads meet (bounded: a thread that gave up does not arrive, the others time out)
       mbar_arrive(bar(&ctl->idx_sync));
       if (!mbar_wait(bar(&ctl->idx_sync), sphase, p.dev_status)) { ok = false; break; }
@@ -403,7 +414,7 @@ conv_tcgen05_kernel(const ConvTcParams p) {
         ctl->info_entry[ib][1] = second;
       }
       const uint32_t own = g == 0 ? m0 : m1;
-      int32_t* at = rows_idx + (g == 0 ? entry : second) * BLOCK_M + row;
+      int32_t* at = rows_idx + (g == 0 ? entry : second) * BLOCK_M + irow;
       int32_t* const end = rows_idx + ENTRIES * BLOCK_M;
 #pragma unroll
       for (int k = 0; k < MAX_OFFSETS; ++k) {
@@ -534,7 +545,7 @@ conv_tcgen05_kernel(const ConvTcParams p) {
           if ((used >> u) & 1u) {  // parts of offsets this sub-tile does not have stay unused
             const char* src[2 * NJ];
             uint32_t have;
-            rows_of(e, src, have);
+            rows_of(single ? g * K + ku[u] : e, src, have);
             if (++e == ENTRIES) e = 0;
             copy(dst + u * A_BYTES, src, have, 0);
           }
@@ -543,10 +554,11 @@ conv_tcgen05_kernel(const ConvTcParams p) {
         ra.advance();
       }
       while (!SPAN && rest && ok) {
+        const int k = __ffs(rest) - 1;
         rest &= rest - 1;
         const char* src[2 * NJ];
         uint32_t have;
-        rows_of(e, src, have);
+        rows_of(single ? g * K + k : e, src, have);
         if (++e == ENTRIES) e = 0;
         for (int kb0 = 0; kb0 < KB; kb0 += KBC) {
           if (!mbar_wait(bar(&ctl->a_empty[g][ra.slot]), ra.phase ^ 1, p.dev_status)) { ok = false; break; }
