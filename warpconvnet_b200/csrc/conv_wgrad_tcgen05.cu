@@ -5,33 +5,43 @@
 //
 // i.e. per kernel offset a tall-skinny GEMM X_k^T (C_in x rows) times dY (rows x C_out) whose
 // reduction runs over the rows.  Both operands are what the forward kernel already knows how
-// to fetch: 128 gathered rows of X and 128 consecutive rows of dY, as swizzled shared-memory
-// tiles whose rows are 128-byte (or 64-byte) channel slices.  Read as MN-major operands those
-// tiles put the channels on the M / N side of tcgen05.mma and the rows on its K side, so a
-// 128-row step is eight K = 16 instructions and nothing is transposed in memory.
+// to fetch: 128 gathered rows of X and 128 rows of dY, as swizzled shared-memory tiles whose
+// rows are 128-byte (or 64-byte) channel slices.  Read as MN-major operands those tiles put the
+// channels on the M / N side of tcgen05.mma and the rows on its K side, so a 128-row step is
+// eight K = 16 instructions and nothing is transposed in memory.
 //
 // The M = 128 side of an instruction holds 128 / CW "units", a unit being the CW = 64 (or 32)
 // channel slice of X gathered through ONE offset; consecutive units (offset-major) form a
-// group, so a group covers two offsets at C_in = 64, half an offset at C_in = 256, and always
-// shares the same dY tile.  A CTA owns (a contiguous range of 128-row steps) x (one group),
-// accumulates its [128 x C_out] block in tensor memory and adds it to the fp32 gradient with
-// red.global.add (the caller zeroes the gradient; the order of the adds is not fixed, as in
-// any split reduction).  Roles: 8 producer warps (cp.async gathers that signal the stage's
-// mbarrier when they land), 1 MMA thread, 4 epilogue warps.  Every wait is bounded and
-// reports through the device status word.
+// group: two offsets at C_in = 64, half an offset at C_in = 256.  A CTA owns every `ranges`-th
+// 128-row step and as many groups as have room for their [128 x C_out] sums in tensor memory
+// (512 / C_out of them): the dY tile of a step is fetched once for all of them, and a group
+// none of whose offsets has a neighbour in the step costs nothing.  In the end the sums are
+// added to the fp32 gradient with red.global.add.v4.f32 (the caller zeroes the gradient; the
+// order of the adds is not fixed, as in any split reduction).
+//
+// What bounds it is the gather of X: 32 KB per step and group at the rate one multiprocessor
+// takes rows from L2 (the matrix instructions of a step and group take 400 clocks at C_out = 64,
+// its copies about 1 000).  An earlier form had one group per CTA (dY read again for each, and a
+// set-up and a tail for each) and loaded the neighbour indices when they were needed, a memory
+// latency in every step of every producer; here the indices of the next group and the masks of
+// the next step are on their way while this group's rows are copied.
+// 240 000 rows of four rooms, 27 offsets, bf16: 96 -> 64 channels 412 -> 276 us, 64 -> 64 277 -> 148 us, 60 000 coarser rows
+// of 128 -> 128 102 -> 54 us.
+//
+// Roles: 8 producer warps (cp.async gathers that signal the stage's mbarrier when they land, and
+// the adds at the end), 1 MMA thread.  Every wait is bounded and reports through the device
+// status word.
 #include "wcn_common.cuh"
 #include "tcgen05_common.cuh"
 
 namespace {
 
 constexpr int WG_ROWS = 128;          // rows per step (K extent of 8 instructions)
-constexpr int WG_MAX_STAGES = 4;
-constexpr int WG_EPI_WARPS = 4;        // warps 0..3
-constexpr int WG_PROD_WARP0 = 4;      // warps 4..11
-constexpr int WG_PROD_THREADS = 256;
-constexpr int WG_MMA_WARP = 12;
-constexpr int WG_THREADS = 416;
-static_assert(WG_PROD_WARP0 == WG_EPI_WARPS && WG_THREADS == (WG_MMA_WARP + 1) * 32, "role layout");
+constexpr int WG_MAX_STAGES = 6;
+constexpr int WG_MAX_GROUPS = 16;     // 512 columns of tensor memory, 32 a group at least
+constexpr int WG_PROD_THREADS = 256;  // warps 0..7
+constexpr int WG_MMA_WARP = 8;
+constexpr int WG_THREADS = 288;
 
 struct WgradParams {
   const char* feats;     // [num_in, c_in]
@@ -43,18 +53,28 @@ struct WgradParams {
   int64_t M, num_in;
   int K, c_in, c_out;
   int32_t* dev_status;
-  int stages;            // ring depth
-  int steps_per_cta;     // 128-row steps per row range
-  int cols;              // TMEM columns (power of two >= c_out)
+  int stages;            // ring depth of the X tiles (the dY ring has two)
+  int groups;            // groups per CTA
+  int cols;              // TMEM columns of a group (power of two >= c_out)
+  int tmem;              // TMEM columns of the CTA
+  bool vec;              // gw is 16-byte aligned
 };
 
 struct WgradControl {
   uint64_t full[WG_MAX_STAGES], empty[WG_MAX_STAGES];
+  uint64_t dy_full[2], dy_empty[2];
   uint64_t acc_full;
+  uint32_t gmask[WG_MAX_GROUPS];   // offsets that a group gathers through
   uint32_t tmem_holder;
   int skip;
-  int any;  // the accumulator received at least one step
+  uint32_t started;                // groups whose sums received at least one step
 };
+
+__device__ __forceinline__ void red_add4(float* p, const uint32_t* v) {
+  asm volatile("red.relaxed.gpu.global.add.v4.f32 [%0], {%1, %2, %3, %4};" ::"l"(p), "f"(__uint_as_float(v[0])),
+               "f"(__uint_as_float(v[1])), "f"(__uint_as_float(v[2])), "f"(__uint_as_float(v[3]))
+               : "memory");
+}
 
 template <int RBA, int RBB, bool BF16>
 __global__ void __launch_bounds__(WG_THREADS, 1)
@@ -64,162 +84,213 @@ conv_wgrad_tcgen05_kernel(const WgradParams p) {
   constexpr int CHA = RBA / 16, CHB = RBB / 16;
   constexpr int A_TILE = WG_ROWS * RBA;     // one unit's tile
   constexpr int B_TILE = WG_ROWS * RBB;     // one dY channel chunk's tile
+  constexpr int A_STAGE = GU * A_TILE;
   extern __shared__ uint8_t smem_raw[];
 
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int UA = p.c_in / CWA;              // units per offset
   const int NB = p.c_out / (RBB / 2);       // dY channel chunks
   const int total_units = p.K * UA;
-  const int unit0 = blockIdx.y * GU;
-  const int A_STAGE = GU * A_TILE, B_STAGE = NB * B_TILE;
-  const int STAGE = A_STAGE + B_STAGE;
+  const int group0 = blockIdx.y * p.groups;
+  const int ng = min(p.groups, (total_units + GU - 1) / GU - group0);
+  const int B_STAGE = NB * B_TILE;
 
   const uint32_t base = (smem_u32(smem_raw) + 1023u) & ~1023u;
   uint8_t* gen = smem_raw + (base - smem_u32(smem_raw));
-  WgradControl* ctl = reinterpret_cast<WgradControl*>(gen + (size_t)p.stages * STAGE);
+  const uint32_t b_base = base + p.stages * A_STAGE;
+  WgradControl* ctl = reinterpret_cast<WgradControl*>(gen + (size_t)p.stages * A_STAGE + 2 * (size_t)B_STAGE);
   auto bar = [](uint64_t* b) { return smem_u32(b); };
 
-  if (tid == 0) ctl->skip = *(volatile int32_t*)p.dev_status;  // an earlier launch on this status word failed
-  __syncthreads();
-  if (ctl->skip == (int)WCN_ERR_WAIT_EXPIRED) return;
-
-  if (tid == 0) {
-    for (int s = 0; s < p.stages; ++s) { mbar_init(bar(&ctl->full[s]), WG_PROD_THREADS); mbar_init(bar(&ctl->empty[s]), 1); }
-    mbar_init(bar(&ctl->acc_full), 2);  // the commit of the last MMAs and the issuer's own arrival
-    ctl->any = 0;
+  if (warp == 0) {
+    if (lane < p.stages) { mbar_init(bar(&ctl->full[lane]), WG_PROD_THREADS); mbar_init(bar(&ctl->empty[lane]), 1); }
+    if (lane < 2) { mbar_init(bar(&ctl->dy_full[lane]), WG_PROD_THREADS); mbar_init(bar(&ctl->dy_empty[lane]), 1); }
+    if (lane == 2) mbar_init(bar(&ctl->acc_full), 2);  // the commit of the last MMAs and the issuer's own arrival
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+  } else if (warp == 1) {
+    if (lane == 0) ctl->skip = *(volatile int32_t*)p.dev_status;  // an earlier launch on this status word failed
+  } else if (warp == 2) {
+    uint32_t m = 0;
+    if (lane < ng && !p.tile_masks) m = 1;  // (any number of offsets)
+    if (lane < ng && p.tile_masks)
+      for (int u = 0; u < GU; ++u) {
+        const int unit = (group0 + lane) * GU + u;
+        if (unit < total_units) m |= 1u << (unit / UA);
+      }
+    if (lane < WG_MAX_GROUPS) ctl->gmask[lane] = m;
+  } else if (warp == WG_MMA_WARP) {
+    tmem_alloc(smem_u32(&ctl->tmem_holder), (uint32_t)p.tmem);
   }
-  if (warp == WG_MMA_WARP) tmem_alloc(smem_u32(&ctl->tmem_holder), (uint32_t)p.cols);
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem_base = ctl->tmem_holder;
+  const bool run = ctl->skip != (int)WCN_ERR_WAIT_EXPIRED;
 
-  const int64_t total_steps = (p.M + WG_ROWS - 1) / WG_ROWS;
-  const int64_t step0 = (int64_t)blockIdx.x * p.steps_per_cta;
-  const int64_t step1 = min(total_steps, step0 + p.steps_per_cta);
-  bool ok = true;
-  // offsets this group gathers through; a step none of whose rows has a neighbour at any of them
-  // contributes nothing and is skipped by every role alike
-  uint32_t gmask = 0;
-  for (int u = 0; u < GU; ++u)
-    if (unit0 + u < total_units) gmask |= 1u << ((unit0 + u) / UA);
+  const int64_t total_steps = (p.M + WG_ROWS - 1) / WG_ROWS, stride = gridDim.x;
+  auto mask_of = [&](int64_t st) { return st >= total_steps ? 0u : p.tile_masks ? __ldg(&p.tile_masks[st]) : 0xFFFFFFFFu; };
+  bool ok = run;
 
-  if (warp >= WG_PROD_WARP0 && warp < WG_MMA_WARP) {
+  if (warp < WG_MMA_WARP) {
     // ================================================================ producers
-    const int pt = tid - WG_PROD_WARP0 * 32, pwarp = warp - WG_PROD_WARP0;
     constexpr int RPI = 32 / CHA;                 // tile rows per warp-wide copy instruction
     constexpr int NJ = 16 / RPI;                  // instructions per warp per unit (16 rows per warp)
     const int sub_row = lane / CHA, chunk = lane % CHA;
     uint32_t aoff[NJ];
 #pragma unroll
-    for (int j = 0; j < NJ; ++j) aoff[j] = tile_offset<RBA>(pwarp * 16 + j * RPI + sub_row, chunk);
+    for (int j = 0; j < NJ; ++j) aoff[j] = tile_offset<RBA>(warp * 16 + j * RPI + sub_row, chunk);
     const int PR = p.c_out * 2 / 16;              // 16-byte pieces of a dY row
-    const int b_iters = WG_ROWS * PR / WG_PROD_THREADS;
-    int slot = 0, phase = 0;
+    const uint32_t mine = ctl->gmask[lane & (WG_MAX_GROUPS - 1)] & (lane < ng ? 0xFFFFFFFFu : 0u);
+    const int num_in = (int)p.num_in;
     bool bad = false;
-    for (int64_t st = step0; st < step1 && ok; ++st) {
-      if (p.tile_masks && !(__ldg(&p.tile_masks[st]) & gmask)) continue;
-      const int64_t m0 = st * WG_ROWS;
-      // the neighbour indices of this thread's rows, for every unit of the group, before the wait
-      int src[GU][NJ];
+    // Items are (step, group) pairs with a neighbour; lane l holds the neighbours of row l % 16 of this warp's sixteen, for
+    // two units of the group (l / 16 and, in a second register, l / 16 + 2).
+    int64_t st = blockIdx.x;
+    uint32_t rest = __ballot_sync(0xFFFFFFFFu, (mask_of(st) & mine) != 0);
+    uint32_t ahead = mask_of(st + stride);
+    auto settle = [&]() {
+      while (!rest && st < total_steps) {
+        st += stride;
+        rest = __ballot_sync(0xFFFFFFFFu, (ahead & mine) != 0);
+        ahead = mask_of(st + stride);
+      }
+    };
+    auto load_rows = [&](int group, int (&idx)[GU / 2]) {
+      const int64_t m = st * WG_ROWS + warp * 16 + (lane & 15);
+#pragma unroll
+      for (int i = 0; i < GU / 2; ++i) {
+        const int unit = (group0 + group) * GU + (lane >> 4) + 2 * i;
+        idx[i] = (unit < total_units && m < p.M) ? __ldg(&p.nbr[(int64_t)(unit / UA) * p.M + m]) : -1;
+      }
+    };
+    auto load_out = [&]() {
+      const int64_t m = st * WG_ROWS + warp * 16 + (lane & 15);
+      return m < p.M ? (p.out_rows ? __ldg(&p.out_rows[m]) : (int32_t)m) : -1;
+    };
+    settle();
+    int idx[GU / 2];
+    int32_t orow = -1;
+    int group = __ffs(rest) - 1;
+    bool fresh = true;    // the item is the first of its step
+    if (st < total_steps) { load_rows(group, idx); orow = load_out(); }
+    int slot = 0, phase = 0, dslot = 0, dphase = 0;
+    while (ok && st < total_steps) {
+      int cur[GU / 2];
+#pragma unroll
+      for (int i = 0; i < GU / 2; ++i) {
+        cur[i] = idx[i];
+        if (cur[i] >= num_in) { cur[i] = -1; bad = true; }  // names no feature row: counts as absent
+      }
+      const int32_t cur_out = orow;
+      const int cur_group = group;
+      const bool cur_fresh = fresh;
+      const int64_t was = st;
+      rest &= rest - 1;
+      settle();
+      fresh = st != was;
+      if (st < total_steps) {
+        group = __ffs(rest) - 1;
+        load_rows(group, idx);
+        if (fresh) orow = load_out();
+      }
+      if (cur_fresh) {
+        if (!mbar_wait(bar(&ctl->dy_empty[dslot]), dphase ^ 1, p.dev_status)) { ok = false; break; }
+        const uint32_t dst = b_base + dslot * B_STAGE;
+        for (int i = lane; i < 16 * PR; i += 32) {
+          const int r = i / PR, piece = i - r * PR;
+          const int32_t row = __shfl_sync(0xFFFFFFFFu, cur_out, r);
+          cp_async16(dst + (piece / CHB) * B_TILE + tile_offset<RBB>(warp * 16 + r, piece % CHB),
+                     row >= 0 ? p.gout + ((int64_t)row * p.c_out) * 2 + piece * 16 : p.gout, row >= 0 ? 16u : 0u);
+        }
+        cp_async_arrive(bar(&ctl->dy_full[dslot]));  // hardware arrives when this thread's copies land
+        dslot ^= 1;
+        if (dslot == 0) dphase ^= 1;
+      }
+      if (!mbar_wait(bar(&ctl->empty[slot]), phase ^ 1, p.dev_status)) { ok = false; break; }
+      const uint32_t dst = base + slot * A_STAGE;
 #pragma unroll
       for (int u = 0; u < GU; ++u) {
-        const int unit = unit0 + u;
-        const int k = unit / UA;
+        const char* from = p.feats + (int64_t)(((group0 + cur_group) * GU + u) % UA) * RBA + chunk * 16;
 #pragma unroll
         for (int j = 0; j < NJ; ++j) {
-          const int64_t m = m0 + pwarp * 16 + j * RPI + sub_row;
-          // (the loads of a step are independent and all in flight together: nothing with a side effect sits
-          // between them — an index that names no feature row only raises a flag here and is reported once)
-          int r = (unit < total_units && m < p.M) ? __ldg(&p.nbr[(int64_t)k * p.M + m]) : -1;
-          if (r >= (int)p.num_in) { r = -1; bad = true; }  // counts as absent
-          src[u][j] = r;
+          const int r = __shfl_sync(0xFFFFFFFFu, cur[u >> 1], (u & 1) * 16 + j * RPI + sub_row);
+          cp_async16(dst + u * A_TILE + aoff[j], r >= 0 ? from + (int64_t)r * p.c_in * 2 : p.feats, r >= 0 ? 16u : 0u);
         }
       }
-      if (!mbar_wait_inline(bar(&ctl->empty[slot]), phase ^ 1, p.dev_status)) { ok = false; break; }
-      const uint32_t a_dst = base + slot * STAGE;
-      const uint32_t b_dst = a_dst + A_STAGE;
-#pragma unroll
-      for (int u = 0; u < GU; ++u) {
-        const int unit = unit0 + u;
-        const int slice = unit % UA;
-        const char* fbase = p.feats + (int64_t)slice * RBA + chunk * 16;
-#pragma unroll
-        for (int j = 0; j < NJ; ++j) {
-          const bool have = src[u][j] >= 0;
-          cp_async16(a_dst + u * A_TILE + aoff[j], have ? fbase + (int64_t)src[u][j] * p.c_in * 2 : p.feats,
-                     have ? 16u : 0u);
-        }
-      }
-      for (int i = 0; i < b_iters; ++i) {
-        const int q = pt + i * WG_PROD_THREADS;
-        const int row = q / PR, piece = q - row * PR;
-        const bool have = m0 + row < p.M;
-        int64_t grow = m0 + row;
-        if (have && p.out_rows) grow = __ldg(&p.out_rows[grow]);
-        cp_async16(b_dst + (piece / CHB) * B_TILE + tile_offset<RBB>(row, piece % CHB),
-                   have ? p.gout + (grow * p.c_out) * 2 + piece * 16 : p.gout, have ? 16u : 0u);
-      }
-      cp_async_arrive(bar(&ctl->full[slot]));  // hardware arrives when this thread's copies land
+      cp_async_arrive(bar(&ctl->full[slot]));
       if (++slot == p.stages) { slot = 0; phase ^= 1; }
     }
     cp_async_drain();
     if (bad) wcn_report_bounds(p.dev_status);
-  } else if (warp == WG_MMA_WARP) {
+    // ================================================================ the sums are added to the gradient
+    __syncwarp();
+    ok = __all_sync(0xFFFFFFFFu, ok);
+    if (ok) ok = mbar_wait(bar(&ctl->acc_full), 0, p.dev_status);
+    if (__all_sync(0xFFFFFFFFu, ok)) {
+      tc_fence_after();
+      const int row = (warp & 3) * 32 + lane;        // TMEM lane = position on the M side
+      for (int g = warp >> 2; g < ng; g += 2) {
+        if (!((ctl->started >> g) & 1u)) continue;
+        const int unit = (group0 + g) * GU + row / CWA;
+        const bool live = unit < total_units;
+        float* dst = p.gw + ((int64_t)(unit / UA) * p.c_in + (unit % UA) * CWA + row % CWA) * p.c_out;
+        const uint32_t trow = tmem_base + ((uint32_t)((warp & 3) * 32) << 16) + (uint32_t)(g * p.cols);
+        for (int c0 = 0; c0 < p.c_out; c0 += 16) {
+          uint32_t r[16];
+          tmem_ld16(trow + (uint32_t)c0, r);  // executed by all lanes of the warp
+          tmem_ld_wait();
+          if (live && p.vec) {
+#pragma unroll
+            for (int i = 0; i < 16; i += 4) red_add4(dst + c0 + i, r + i);
+          } else if (live) {
+#pragma unroll
+            for (int i = 0; i < 16; ++i) atomicAdd(dst + c0 + i, __uint_as_float(r[i]));
+          }
+        }
+      }
+    }
+  } else {
     // ================================================================ MMA issuer
     if (elect_one()) {
       // fp32 accumulate, A and B MN-major (bits 15, 16), N = c_out, M = 128
       const uint32_t idesc = (1u << 4) | ((BF16 ? 1u : 0u) << 7) | ((BF16 ? 1u : 0u) << 10) | (1u << 15) | (1u << 16) |
                              ((uint32_t)(p.c_out >> 3) << 17) | ((uint32_t)(128 >> 4) << 24);
-      int slot = 0, phase = 0;
-      bool any = false;
-      for (int64_t st = step0; st < step1 && ok; ++st) {
-        if (p.tile_masks && !(__ldg(&p.tile_masks[st]) & gmask)) continue;
-        if (!mbar_wait_inline(bar(&ctl->full[slot]), phase, p.dev_status)) { ok = false; break; }
-        tc_fence_after();
-        const uint32_t a_slot = base + slot * STAGE;
-        const uint32_t b_slot = a_slot + A_STAGE;
+      int slot = 0, phase = 0, dslot = 0, dphase = 0;
+      uint32_t started = 0, mask = mask_of(blockIdx.x);
+      for (int64_t st = blockIdx.x; st < total_steps && ok; st += stride) {
+        uint32_t rest = 0;
+        for (int g = 0; g < ng; ++g) rest |= (mask & ctl->gmask[g]) ? 1u << g : 0u;
+        mask = mask_of(st + stride);
+        if (!rest) continue;
+        if (!mbar_wait(bar(&ctl->dy_full[dslot]), dphase, p.dev_status)) { ok = false; break; }
+        const uint32_t b_slot = b_base + dslot * B_STAGE;
+        for (; rest; rest &= rest - 1) {
+          const int g = __ffs(rest) - 1;
+          if (!mbar_wait(bar(&ctl->full[slot]), phase, p.dev_status)) { ok = false; break; }
+          tc_fence_after();
+          const uint64_t adesc = smem_desc_mn<RBA>(base + slot * A_STAGE, (uint32_t)A_TILE);
+          const uint64_t bdesc = smem_desc_mn<RBB>(b_slot, (uint32_t)B_TILE);
+          const uint32_t d = tmem_base + (uint32_t)(g * p.cols), acc = (started >> g) & 1u;
 #pragma unroll
-        for (int ks = 0; ks < WG_ROWS / 16; ++ks) {  // 16 rows = two 8-row atoms further down the tiles
-          const uint64_t adesc = smem_desc_mn<RBA>(a_slot + ks * 16 * RBA, (uint32_t)A_TILE);
-          const uint64_t bdesc = smem_desc_mn<RBB>(b_slot + ks * 16 * RBB, (uint32_t)B_TILE);
-          umma_f16(tmem_base, adesc, bdesc, idesc, (any || ks > 0) ? 1u : 0u);
+          for (int ks = 0; ks < WG_ROWS / 16; ++ks)  // 16 rows = two 8-row atoms further down the tiles
+            umma_f16(d, adesc + (uint64_t)(ks * RBA), bdesc + (uint64_t)(ks * RBB), idesc, acc | (ks > 0 ? 1u : 0u));
+          started |= 1u << g;
+          umma_commit(bar(&ctl->empty[slot]));  // the stage is free once these instructions have read it
+          if (++slot == p.stages) { slot = 0; phase ^= 1; }
         }
-        any = true;
-        umma_commit(bar(&ctl->empty[slot]));  // the stage is free once these MMAs have read it
-        if (++slot == p.stages) { slot = 0; phase ^= 1; }
+        if (!ok) break;
+        umma_commit(bar(&ctl->dy_empty[dslot]));
+        dslot ^= 1;
+        if (dslot == 0) dphase ^= 1;
       }
       umma_commit(bar(&ctl->acc_full));  // arrives when every MMA above has completed (at once if there were none)
-      ctl->any = (any && ok) ? 1 : 0;
-      mbar_arrive(bar(&ctl->acc_full));  // publishes `any`
+      ctl->started = ok ? started : 0u;
+      mbar_arrive(bar(&ctl->acc_full));  // publishes `started`
     }
     __syncwarp();
-  } else {
-    // ================================================================ epilogue (warps 0..3)
-    ok = mbar_wait_inline(bar(&ctl->acc_full), 0, p.dev_status);
-    if (__all_sync(0xFFFFFFFFu, ok) && ctl->any) {
-      tc_fence_after();
-      const int row = warp * 32 + lane;            // TMEM lane = position on the M side
-      const int unit = unit0 + row / CWA;
-      const bool live = unit < total_units;
-      const int k = unit / UA, ci = (unit % UA) * CWA + row % CWA;
-      float* dst = p.gw + ((int64_t)k * p.c_in + ci) * p.c_out;
-      const uint32_t trow = tmem_base + ((uint32_t)(warp * 32) << 16);
-      for (int c0 = 0; c0 < p.c_out; c0 += 16) {
-        uint32_t r[16];
-        tmem_ld16(trow + (uint32_t)c0, r);  // executed by all lanes of the warp
-        tmem_ld_wait();
-        if (live) {
-#pragma unroll
-          for (int i = 0; i < 16; ++i) atomicAdd(dst + c0 + i, __uint_as_float(r[i]));
-        }
-      }
-    }
   }
   tc_fence_before();
   __syncthreads();
-  if (warp == WG_MMA_WARP) tmem_dealloc(tmem_base, (uint32_t)p.cols);
+  if (warp == WG_MMA_WARP) tmem_dealloc(tmem_base, (uint32_t)p.tmem);
 }
 
 template <int RBA, int RBB, bool BF16>
@@ -227,22 +298,28 @@ int launch_wgrad(WgradParams& p, cudaStream_t st) {
   constexpr int CWA = RBA / 2, GU = 128 / CWA;
   const int UA = p.c_in / CWA, NB = p.c_out / (RBB / 2);
   const int groups = (p.K * UA + GU - 1) / GU;
-  const size_t stage = (size_t)GU * WG_ROWS * RBA + (size_t)NB * WG_ROWS * RBB;
+  const size_t a_stage = (size_t)GU * WG_ROWS * RBA, b_stage = (size_t)NB * WG_ROWS * RBB;
   const size_t limit = 226 * 1024, fixed = 1024 + sizeof(WgradControl) + 128;
-  int stages = (int)((limit - fixed) / stage);
+  int stages = (int)((limit - fixed - 2 * b_stage) / a_stage);
   if (stages > WG_MAX_STAGES) stages = WG_MAX_STAGES;
   if (stages < 2) return WCN_ERR_UNSUPPORTED_CONFIG;
   p.stages = stages;
-  int cols = 32;
-  while (cols < p.c_out) cols <<= 1;
-  p.cols = cols;
-  // enough CTAs for a few waves, but at least four steps each so the set-up cost stays small
+  p.cols = 32;
+  while (p.cols < p.c_out) p.cols <<= 1;
+  // One CTA per multiprocessor.  As many groups per CTA as tensor memory holds (they share dY) while every CTA still gets
+  // two steps; then as many CTAs along the rows as fit.
+  const int sms = wcn_num_sms();
   const int64_t total_steps = (p.M + WG_ROWS - 1) / WG_ROWS;
-  int64_t ranges = (4 * (int64_t)wcn_num_sms() + groups - 1) / groups;
-  if (ranges > (total_steps + 3) / 4) ranges = (total_steps + 3) / 4;
+  int per = 512 / p.cols;
+  if (per > groups) per = groups;
+  while (per > 1 && total_steps * ((groups + per - 1) / per) < 2 * (int64_t)sms) per = (per + 1) / 2;
+  const int blocks = (groups + per - 1) / per;
+  p.groups = (groups + blocks - 1) / blocks;   // evenly
+  p.tmem = 32;
+  while (p.tmem < p.groups * p.cols) p.tmem <<= 1;
+  int64_t ranges = sms / blocks;
+  if (ranges > (total_steps + 1) / 2) ranges = (total_steps + 1) / 2;
   if (ranges < 1) ranges = 1;
-  p.steps_per_cta = (int)((total_steps + ranges - 1) / ranges);
-  ranges = (total_steps + p.steps_per_cta - 1) / p.steps_per_cta;
 
   auto kern = conv_wgrad_tcgen05_kernel<RBA, RBB, BF16>;
   static bool configured[64] = {};  // per template instance and device: opt in to large shared memory once
@@ -255,8 +332,8 @@ int launch_wgrad(WgradParams& p, cudaStream_t st) {
     }
     configured[dev] = true;
   }
-  dim3 grid((unsigned)ranges, (unsigned)groups);
-  kern<<<grid, WG_THREADS, fixed + stages * stage, st>>>(p);
+  dim3 grid((unsigned)ranges, (unsigned)blocks);
+  kern<<<grid, WG_THREADS, fixed + stages * a_stage + 2 * b_stage, st>>>(p);
   return cudaGetLastError() == cudaSuccess ? WCN_OK : WCN_ERR_EXECUTION;
 }
 
@@ -277,6 +354,7 @@ int wcn_conv_wgrad_tcgen05(const void* feats, int64_t num_in, const void* grad_o
   WgradParams p;
   p.feats = (const char*)feats; p.gout = (const char*)grad_out; p.nbr = nbr; p.out_rows = out_rows; p.tile_masks = K <= 32 ? tile_masks : nullptr; p.gw = grad_weight;
   p.M = M; p.num_in = num_in; p.K = K; p.c_in = c_in; p.c_out = c_out; p.dev_status = dev_status;
+  p.vec = (reinterpret_cast<uintptr_t>(grad_weight) & 15) == 0;
   const bool a128 = c_in % 64 == 0, b128 = c_out % 64 == 0, bf = dtype == WCN_BF16;
 #define WCN_WG_CASE(A, B, F) if (a128 == (A == 128) && b128 == (B == 128) && bf == F) return launch_wgrad<A, B, F>(p, st);
   WCN_WG_CASE(128, 128, false) WCN_WG_CASE(128, 64, false) WCN_WG_CASE(64, 128, false) WCN_WG_CASE(64, 64, false)
