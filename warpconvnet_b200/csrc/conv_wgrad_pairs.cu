@@ -192,58 +192,88 @@ conv_wgrad_pairs_kernel(const PairsParams p) {
   if (bad) wcn_report_bounds(p.dev_status);
 }
 
-// Up to CI = 8 input channels (a network's stem): the work is reading one dY row per pair, so a warp takes 32 rows of the
-// table, walks those that have a neighbour and keeps CI sums per output channel (lane); four pairs' rows are in flight.
-// (240 000 rows, 3 -> 32 channels, 27 offsets: the staged tile kernel above took 188 us, bound by shared memory.)
+// Up to CI = 8 input channels (a network's stem).  What counts is how often dY is read and how many instructions a (row,
+// offset) takes: a warp holds the dY rows of 32 table rows (lane = output channel) in registers, stages the input rows of
+// KG offsets in shared memory and multiplies them from there, one broadcast load and CI multiply-adds per row and offset.
+// (240 000 rows, 3 -> 32 channels, 27 offsets: 222 us walking the present pairs of one offset at a time, which reads a dY
+// row per pair; MEASURED here.)
 constexpr int NARROW_THREADS = 256;
+__host__ __device__ constexpr int narrow_offsets(int ci) { return 36 / ci; }   // 9 offsets of 4 channels, 4 of 8: 36 and 32 sums a thread
 
 template <typename T, int CI>
-__global__ void __launch_bounds__(NARROW_THREADS)
+__global__ void __launch_bounds__(NARROW_THREADS, 2)
 conv_wgrad_narrow_kernel(const PairsParams p) {
-  __shared__ float part[NARROW_THREADS / 32][CI][32];
+  constexpr int KG = narrow_offsets(CI), WARPS = NARROW_THREADS / 32;
+  __shared__ __align__(16) float xs[WARPS][KG][32][CI];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  const int k = blockIdx.y, j = blockIdx.z * 32 + lane;
+  const int k0 = blockIdx.y * KG, j = blockIdx.z * 32 + lane;
   const bool col = j < p.c_out;
   const T* feats = reinterpret_cast<const T*>(p.feats);
   const T* gout = reinterpret_cast<const T*>(p.gout) + (col ? j : 0);
   const int64_t begin = (int64_t)blockIdx.x * p.rows_per_range, end = min(p.M, begin + p.rows_per_range);
-  float acc[CI];
+  float acc[KG][CI];
 #pragma unroll
-  for (int c = 0; c < CI; ++c) acc[c] = 0.f;
+  for (int q = 0; q < KG; ++q)
+#pragma unroll
+    for (int c = 0; c < CI; ++c) acc[q][c] = 0.f;
   bool bad = false;
   for (int64_t base = begin + warp * 32; base < end; base += NARROW_THREADS) {
     const int64_t m = base + lane;
-    int src = m < end ? __ldg(&p.nbr[(int64_t)k * p.M + m]) : -1;
-    if (src >= p.num_in) { src = -1; bad = true; }
-    uint32_t rest = __ballot_sync(0xFFFFFFFFu, src >= 0);
-    int row = (int)m;
-    if (p.out_rows && src >= 0) row = __ldg(&p.out_rows[m]);
-    while (rest) {
-      float g[4], x[4][CI];
+    int src[KG];
 #pragma unroll
-      for (int u = 0; u < 4; ++u) {
-        const bool have = rest != 0;
-        const int b = have ? __ffs(rest) - 1 : 0;
-        rest &= rest - 1;
-        const int s = __shfl_sync(0xFFFFFFFFu, src, b), r = __shfl_sync(0xFFFFFFFFu, row, b);
-        g[u] = have && col ? wcn_to_float<T>(gout[(int64_t)r * p.c_out]) : 0.f;
+    for (int q = 0; q < KG; ++q) src[q] = (k0 + q < p.K && m < end) ? __ldg(&p.nbr[(int64_t)(k0 + q) * p.M + m]) : -1;
+    const int row = m < end ? (p.out_rows ? __ldg(&p.out_rows[m]) : (int)m) : -1;
+    uint32_t any = 0;
 #pragma unroll
-        for (int c = 0; c < CI; ++c) x[u][c] = have && c < p.c_in ? wcn_to_float<T>(feats[(int64_t)s * p.c_in + c]) : 0.f;
-      }
+    for (int q = 0; q < KG; ++q) {
+      if (src[q] >= p.num_in) { src[q] = -1; bad = true; }
+      any |= __any_sync(0xFFFFFFFFu, src[q] >= 0) ? 1u << q : 0u;
+      float x[CI];
 #pragma unroll
-      for (int u = 0; u < 4; ++u)
+      for (int c = 0; c < CI; ++c) x[c] = src[q] >= 0 && c < p.c_in ? wcn_to_float<T>(feats[(int64_t)src[q] * p.c_in + c]) : 0.f;
 #pragma unroll
-        for (int c = 0; c < CI; ++c) acc[c] = fmaf(x[u][c], g[u], acc[c]);
+      for (int c = 0; c < CI; c += 4) *reinterpret_cast<float4*>(&xs[warp][q][lane][c]) = make_float4(x[c], x[c + 1], x[c + 2], x[c + 3]);
     }
-  }
+    if (!any) continue;
+    float g[32];
 #pragma unroll
-  for (int c = 0; c < CI; ++c) part[warp][c][lane] = acc[c];
+    for (int b = 0; b < 32; ++b) {
+      const int r = __shfl_sync(0xFFFFFFFFu, row, b);
+      g[b] = r >= 0 && col ? wcn_to_float<T>(gout[(int64_t)r * p.c_out]) : 0.f;
+    }
+    __syncwarp();
+#pragma unroll
+    for (int q = 0; q < KG; ++q) {
+      if (!((any >> q) & 1u)) continue;
+#pragma unroll
+      for (int b = 0; b < 32; ++b)
+#pragma unroll
+        for (int c = 0; c < CI; c += 4) {
+          const float4 x = *reinterpret_cast<const float4*>(&xs[warp][q][b][c]);
+          acc[q][c] = fmaf(x.x, g[b], acc[q][c]);
+          acc[q][c + 1] = fmaf(x.y, g[b], acc[q][c + 1]);
+          acc[q][c + 2] = fmaf(x.z, g[b], acc[q][c + 2]);
+          acc[q][c + 3] = fmaf(x.w, g[b], acc[q][c + 3]);
+        }
+    }
+    __syncwarp();
+  }
+  // the block's sums, in warp order
   __syncthreads();
-  for (int i = threadIdx.x; i < CI * 32; i += NARROW_THREADS) {
-    const int c = i / 32, n = blockIdx.z * 32 + (i & 31);
-    float v = part[0][c][i & 31];
-    for (int w = 1; w < NARROW_THREADS / 32; ++w) v += part[w][c][i & 31];
-    if (c < p.c_in && n < p.c_out) p.dst[(((int64_t)blockIdx.x * p.K + k) * p.c_in + c) * p.c_out + n] = v;
+  float* part = &xs[0][0][0][0];   // [KG * CI][WARPS][32] would not fit at once: one offset at a time
+#pragma unroll
+  for (int q = 0; q < KG; ++q) {
+#pragma unroll
+    for (int c = 0; c < CI; ++c) part[(c * WARPS + warp) * 32 + lane] = acc[q][c];
+    __syncthreads();
+    for (int i = threadIdx.x; i < CI * 32; i += NARROW_THREADS) {
+      const int c = i / 32, n = blockIdx.z * 32 + (i & 31);
+      float v = 0.f;
+#pragma unroll
+      for (int w = 0; w < WARPS; ++w) v += part[(c * WARPS + w) * 32 + (i & 31)];
+      if (k0 + q < p.K && c < p.c_in && n < p.c_out) p.dst[(((int64_t)blockIdx.x * p.K + k0 + q) * p.c_in + c) * p.c_out + n] = v;
+    }
+    __syncthreads();
   }
   if (bad) wcn_report_bounds(p.dev_status);
 }
@@ -258,19 +288,22 @@ __global__ void sum_ranges_kernel(const float* __restrict__ partial, int ranges,
 }
 
 struct PairsPlan {
-  int ti, tj, tiles_i, tiles_j, ranges;
+  int ti, tj, tiles_i, tiles_j, ranges, blocks_k;
   int64_t rows_per_range;
 };
 
-// About eight blocks per multiprocessor, none with fewer than one list of rows.
+// About eight blocks per multiprocessor (two of the narrow kernel), none with fewer than one list of rows.
 PairsPlan plan_pairs(int64_t M, int K, int c_in, int c_out) {
   PairsPlan q;
   q.ti = c_in <= 8 ? 8 : c_in <= 32 ? 32 : 64;   // 8: the narrow kernel, 32 columns a block
   q.tj = c_out <= 32 || q.ti == 8 ? 32 : 64;
   q.tiles_i = (c_in + q.ti - 1) / q.ti;
   q.tiles_j = (c_out + q.tj - 1) / q.tj;
-  const int64_t blocks = (int64_t)K * q.tiles_i * q.tiles_j;
-  int64_t ranges = (8 * (int64_t)wcn_num_sms() + blocks - 1) / blocks;
+  const int ks = narrow_offsets(c_in <= 4 ? 4 : 8);
+  q.blocks_k = q.ti == 8 ? (K + ks - 1) / ks : K;
+  const int64_t blocks = (int64_t)q.blocks_k * q.tiles_i * q.tiles_j;
+  // (the narrow kernel's blocks are resident two at a time)
+  int64_t ranges = ((q.ti == 8 ? 2 : 8) * (int64_t)wcn_num_sms() + blocks - 1) / blocks;
   const int64_t most = (M + LIST - 1) / LIST;
   if (ranges > most) ranges = most;
   if (ranges < 1) ranges = 1;
@@ -281,7 +314,7 @@ PairsPlan plan_pairs(int64_t M, int K, int c_in, int c_out) {
 
 template <typename T, bool VEC>
 int launch_pairs(const PairsParams& p, const PairsPlan& q, cudaStream_t st) {
-  dim3 grid((unsigned)q.ranges, (unsigned)p.K, (unsigned)(q.tiles_i * q.tiles_j));
+  dim3 grid((unsigned)q.ranges, (unsigned)q.blocks_k, (unsigned)(q.tiles_i * q.tiles_j));
   if (q.ti == 8) {
     if (p.c_in <= 4) conv_wgrad_narrow_kernel<T, 4><<<grid, NARROW_THREADS, 0, st>>>(p);
     else conv_wgrad_narrow_kernel<T, 8><<<grid, NARROW_THREADS, 0, st>>>(p);

@@ -42,6 +42,7 @@ constexpr int WG_MAX_GROUPS = 16;     // 512 columns of tensor memory, 32 a grou
 constexpr int WG_PROD_THREADS = 256;  // warps 0..7
 constexpr int WG_MMA_WARP = 8;
 constexpr int WG_THREADS = 288;
+constexpr int AHEAD = 3;              // items whose indices are on their way
 
 struct WgradParams {
   const char* feats;     // [num_in, c_in]
@@ -144,54 +145,48 @@ conv_wgrad_tcgen05_kernel(const WgradParams p) {
     bool bad = false;
     // Items are (step, group) pairs with a neighbour; lane l holds the neighbours of row l % 16 of this warp's sixteen, for
     // two units of the group (l / 16 and, in a second register, l / 16 + 2).
-    int64_t st = blockIdx.x;
+    // The loads of an item wait their turn behind the copies already issued (a microsecond and more), so they are made
+    // AHEAD items early.
+    struct Item { int group; bool fresh; int32_t out; int idx[GU / 2]; };   // fresh: the first of its step
+    int64_t st = blockIdx.x, last = -1;
     uint32_t rest = __ballot_sync(0xFFFFFFFFu, (mask_of(st) & mine) != 0);
     uint32_t ahead = mask_of(st + stride);
-    auto settle = [&]() {
+    auto next = [&](Item& it) {
       while (!rest && st < total_steps) {
         st += stride;
         rest = __ballot_sync(0xFFFFFFFFu, (ahead & mine) != 0);
         ahead = mask_of(st + stride);
       }
-    };
-    auto load_rows = [&](int group, int (&idx)[GU / 2]) {
+      it.group = __ffs(rest) - 1;   // -1: no more
+      if (!rest) return;
+      rest &= rest - 1;
       const int64_t m = st * WG_ROWS + warp * 16 + (lane & 15);
 #pragma unroll
       for (int i = 0; i < GU / 2; ++i) {
-        const int unit = (group0 + group) * GU + (lane >> 4) + 2 * i;
-        idx[i] = (unit < total_units && m < p.M) ? __ldg(&p.nbr[(int64_t)(unit / UA) * p.M + m]) : -1;
+        const int unit = (group0 + it.group) * GU + (lane >> 4) + 2 * i;
+        it.idx[i] = (unit < total_units && m < p.M) ? __ldg(&p.nbr[(int64_t)(unit / UA) * p.M + m]) : -1;
       }
+      it.fresh = st != last;
+      last = st;
+      if (it.fresh) it.out = m < p.M ? (p.out_rows ? __ldg(&p.out_rows[m]) : (int32_t)m) : -1;
     };
-    auto load_out = [&]() {
-      const int64_t m = st * WG_ROWS + warp * 16 + (lane & 15);
-      return m < p.M ? (p.out_rows ? __ldg(&p.out_rows[m]) : (int32_t)m) : -1;
-    };
-    settle();
-    int idx[GU / 2];
-    int32_t orow = -1;
-    int group = __ffs(rest) - 1;
-    bool fresh = true;    // the item is the first of its step
-    if (st < total_steps) { load_rows(group, idx); orow = load_out(); }
+    Item q[AHEAD];
+#pragma unroll
+    for (int i = 0; i < AHEAD; ++i) next(q[i]);
     int slot = 0, phase = 0, dslot = 0, dphase = 0;
-    while (ok && st < total_steps) {
+    while (ok && q[0].group >= 0) {
       int cur[GU / 2];
 #pragma unroll
       for (int i = 0; i < GU / 2; ++i) {
-        cur[i] = idx[i];
+        cur[i] = q[0].idx[i];
         if (cur[i] >= num_in) { cur[i] = -1; bad = true; }  // names no feature row: counts as absent
       }
-      const int32_t cur_out = orow;
-      const int cur_group = group;
-      const bool cur_fresh = fresh;
-      const int64_t was = st;
-      rest &= rest - 1;
-      settle();
-      fresh = st != was;
-      if (st < total_steps) {
-        group = __ffs(rest) - 1;
-        load_rows(group, idx);
-        if (fresh) orow = load_out();
-      }
+      const int32_t cur_out = q[0].out;
+      const int cur_group = q[0].group;
+      const bool cur_fresh = q[0].fresh;
+#pragma unroll
+      for (int i = 0; i + 1 < AHEAD; ++i) q[i] = q[i + 1];
+      next(q[AHEAD - 1]);
       if (cur_fresh) {
         if (!mbar_wait(bar(&ctl->dy_empty[dslot]), dphase ^ 1, p.dev_status)) { ok = false; break; }
         const uint32_t dst = b_base + dslot * B_STAGE;
