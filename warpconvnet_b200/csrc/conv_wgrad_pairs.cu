@@ -196,7 +196,7 @@ conv_wgrad_pairs_kernel(const PairsParams p) {
 // offset) takes: a warp holds the dY rows of 32 table rows (lane = output channel) in registers, stages the input rows of
 // KG offsets in shared memory and multiplies them from there, one broadcast load and CI multiply-adds per row and offset.
 // (240 000 rows, 3 -> 32 channels, 27 offsets: 222 us walking the present pairs of one offset at a time, which reads a dY
-// row per pair; MEASURED here.)
+// row per pair; 114 us here.)
 constexpr int NARROW_THREADS = 256;
 __host__ __device__ constexpr int narrow_offsets(int ci) { return 36 / ci; }   // 9 offsets of 4 channels, 4 of 8: 36 and 32 sums a thread
 

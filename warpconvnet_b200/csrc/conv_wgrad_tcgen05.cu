@@ -19,17 +19,14 @@
 // added to the fp32 gradient with red.global.add.v4.f32 (the caller zeroes the gradient; the
 // order of the adds is not fixed, as in any split reduction).
 //
-// What bounds it is the gather of X: 32 KB per step and group at the rate one multiprocessor
-// takes rows from L2 (the matrix instructions of a step and group take 400 clocks at C_out = 64,
-// its copies about 1 000).  An earlier form had one group per CTA (dY read again for each, and a
-// set-up and a tail for each) and loaded the neighbour indices when they were needed, a memory
-// latency in every step of every producer; here the indices of the next group and the masks of
-// the next step are on their way while this group's rows are copied.
-// 240 000 rows of four rooms, 27 offsets, bf16: 96 -> 64 channels 412 -> 276 us, 64 -> 64 277 -> 148 us, 60 000 coarser rows
-// of 128 -> 128 102 -> 54 us.
+// What bounds it: the producers' instruction streams, then the gather of X (32 KB per step and group; the matrix
+// instructions of one take 400 clocks at C_out = 64).  An earlier form had one group per CTA (dY read again for each, and a
+// set-up and a tail for each), all eight producer warps on every tile and the neighbour indices loaded when they were
+// needed.  240 000 rows of a room, 27 offsets, bf16: 96 -> 64 channels 412 -> 179 us, 64 -> 64 277 -> 110 us, 32 -> 32
+// 69 us; 60 000 rows of 128 -> 128 81 us, of 256 -> 256 292 us.
 //
-// Roles: 8 producer warps (cp.async gathers that signal the stage's mbarrier when they land, and
-// the adds at the end), 1 MMA thread.  Every wait is bounded and reports through the device
+// Roles: two teams of 4 producer warps (cp.async gathers that signal the stage's mbarrier when they
+// land, and the adds at the end), 1 MMA thread.  Every wait is bounded and reports through the device
 // status word.
 #include "wcn_common.cuh"
 #include "tcgen05_common.cuh"
@@ -39,10 +36,9 @@ namespace {
 constexpr int WG_ROWS = 128;          // rows per step (K extent of 8 instructions)
 constexpr int WG_MAX_STAGES = 6;
 constexpr int WG_MAX_GROUPS = 16;     // 512 columns of tensor memory, 32 a group at least
-constexpr int WG_PROD_THREADS = 256;  // warps 0..7
+constexpr int WG_PROD_THREADS = 256;  // warps 0..7, two teams of four
 constexpr int WG_MMA_WARP = 8;
 constexpr int WG_THREADS = 288;
-constexpr int AHEAD = 3;              // items whose indices are on their way
 
 struct WgradParams {
   const char* feats;     // [num_in, c_in]
@@ -66,6 +62,8 @@ struct WgradControl {
   uint64_t dy_full[2], dy_empty[2];
   uint64_t acc_full;
   uint32_t gmask[WG_MAX_GROUPS];   // offsets that a group gathers through
+  int unit_k[WG_MAX_GROUPS * 4];   // a unit's offset (-1: none) and the first byte of its channels
+  int unit_at[WG_MAX_GROUPS * 4];
   uint32_t tmem_holder;
   int skip;
   uint32_t started;                // groups whose sums received at least one step
@@ -103,8 +101,8 @@ conv_wgrad_tcgen05_kernel(const WgradParams p) {
   auto bar = [](uint64_t* b) { return smem_u32(b); };
 
   if (warp == 0) {
-    if (lane < p.stages) { mbar_init(bar(&ctl->full[lane]), WG_PROD_THREADS); mbar_init(bar(&ctl->empty[lane]), 1); }
-    if (lane < 2) { mbar_init(bar(&ctl->dy_full[lane]), WG_PROD_THREADS); mbar_init(bar(&ctl->dy_empty[lane]), 1); }
+    if (lane < p.stages) { mbar_init(bar(&ctl->full[lane]), WG_PROD_THREADS / 2); mbar_init(bar(&ctl->empty[lane]), 1); }
+    if (lane < 2) { mbar_init(bar(&ctl->dy_full[lane]), WG_PROD_THREADS / 2); mbar_init(bar(&ctl->dy_empty[lane]), 1); }
     if (lane == 2) mbar_init(bar(&ctl->acc_full), 2);  // the commit of the last MMAs and the issuer's own arrival
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   } else if (warp == 1) {
@@ -118,6 +116,12 @@ conv_wgrad_tcgen05_kernel(const WgradParams p) {
         if (unit < total_units) m |= 1u << (unit / UA);
       }
     if (lane < WG_MAX_GROUPS) ctl->gmask[lane] = m;
+  } else if (warp == 3) {
+    for (int i = lane; i < ng * GU; i += 32) {
+      const int unit = group0 * GU + i;
+      ctl->unit_k[i] = unit < total_units ? unit / UA : -1;
+      ctl->unit_at[i] = (unit % UA) * RBA;
+    }
   } else if (warp == WG_MMA_WARP) {
     tmem_alloc(smem_u32(&ctl->tmem_holder), (uint32_t)p.tmem);
   }
@@ -133,86 +137,96 @@ conv_wgrad_tcgen05_kernel(const WgradParams p) {
 
   if (warp < WG_MMA_WARP) {
     // ================================================================ producers
+    // Two teams of four warps (32 rows of a tile each) take the items - (step, group) pairs with a neighbour - in turns, and
+    // the dY tiles of the steps in turns: what an item costs is the length of a warp's instruction stream (with eight warps
+    // on every item 1 900 to 2 800 clocks, with or without the copies and the matrix instructions).  The loads of an item
+    // wait their turn behind the copies already issued, so they are made an item of this team early.
     constexpr int RPI = 32 / CHA;                 // tile rows per warp-wide copy instruction
-    constexpr int NJ = 16 / RPI;                  // instructions per warp per unit (16 rows per warp)
+    constexpr int NJ = 32 / RPI;                  // instructions per warp per unit
+    const int team = warp >> 2, row0 = (warp & 3) * 32;
     const int sub_row = lane / CHA, chunk = lane % CHA;
     uint32_t aoff[NJ];
 #pragma unroll
-    for (int j = 0; j < NJ; ++j) aoff[j] = tile_offset<RBA>(warp * 16 + j * RPI + sub_row, chunk);
+    for (int j = 0; j < NJ; ++j) aoff[j] = tile_offset<RBA>(row0 + j * RPI + sub_row, chunk);
     const int PR = p.c_out * 2 / 16;              // 16-byte pieces of a dY row
     const uint32_t mine = ctl->gmask[lane & (WG_MAX_GROUPS - 1)] & (lane < ng ? 0xFFFFFFFFu : 0u);
     const int num_in = (int)p.num_in;
+    const int64_t ld = (int64_t)p.c_in * 2;
     bool bad = false;
-    // Items are (step, group) pairs with a neighbour; lane l holds the neighbours of row l % 16 of this warp's sixteen, for
-    // two units of the group (l / 16 and, in a second register, l / 16 + 2).
-    // The loads of an item wait their turn behind the copies already issued (a microsecond and more), so they are made
-    // AHEAD items early.
-    struct Item { int group; bool fresh; int32_t out; int idx[GU / 2]; };   // fresh: the first of its step
-    int64_t st = blockIdx.x, last = -1;
+    int64_t st = blockIdx.x;
     uint32_t rest = __ballot_sync(0xFFFFFFFFu, (mask_of(st) & mine) != 0);
     uint32_t ahead = mask_of(st + stride);
+    bool fresh = true;             // no item of step `st` has been taken
+    int item = 0, step = 0;        // items and steps taken
+    struct Item { int group; int32_t out; bool dy; int idx[GU]; };   // dy: this team fetches the step's dY tile before it
     auto next = [&](Item& it) {
-      while (!rest && st < total_steps) {
-        st += stride;
-        rest = __ballot_sync(0xFFFFFFFFu, (ahead & mine) != 0);
-        ahead = mask_of(st + stride);
-      }
-      it.group = __ffs(rest) - 1;   // -1: no more
-      if (!rest) return;
-      rest &= rest - 1;
-      const int64_t m = st * WG_ROWS + warp * 16 + (lane & 15);
+      it.dy = false;
+      for (;;) {
+        while (!rest && st < total_steps) {
+          st += stride;
+          rest = __ballot_sync(0xFFFFFFFFu, (ahead & mine) != 0);
+          ahead = mask_of(st + stride);
+          fresh = true;
+        }
+        it.group = __ffs(rest) - 1;   // -1: no more
+        if (!rest) return;
+        const int64_t m = st * WG_ROWS + row0 + lane;
+        const bool own = (item & 1) == team;
+        if (fresh) {
+          fresh = false;
+          if ((step++ & 1) == team) {
+            it.out = m < p.M ? (p.out_rows ? __ldg(&p.out_rows[m]) : (int32_t)m) : -1;
+            it.dy = true;
+            if (!own) { it.group = WG_MAX_GROUPS; return; }   // the tile alone: the item is the other team's
+          }
+        }
+        rest &= rest - 1;
+        ++item;
+        if (!own) continue;
 #pragma unroll
-      for (int i = 0; i < GU / 2; ++i) {
-        const int unit = (group0 + it.group) * GU + (lane >> 4) + 2 * i;
-        it.idx[i] = (unit < total_units && m < p.M) ? __ldg(&p.nbr[(int64_t)(unit / UA) * p.M + m]) : -1;
+        for (int u = 0; u < GU; ++u) {
+          const int k = ctl->unit_k[it.group * GU + u];
+          it.idx[u] = (k >= 0 && m < p.M) ? __ldg(&p.nbr[(int64_t)k * p.M + m]) : -1;
+        }
+        return;
       }
-      it.fresh = st != last;
-      last = st;
-      if (it.fresh) it.out = m < p.M ? (p.out_rows ? __ldg(&p.out_rows[m]) : (int32_t)m) : -1;
     };
-    Item q[AHEAD];
-#pragma unroll
-    for (int i = 0; i < AHEAD; ++i) next(q[i]);
-    int slot = 0, phase = 0, dslot = 0, dphase = 0;
-    while (ok && q[0].group >= 0) {
-      int cur[GU / 2];
-#pragma unroll
-      for (int i = 0; i < GU / 2; ++i) {
-        cur[i] = q[0].idx[i];
-        if (cur[i] >= num_in) { cur[i] = -1; bad = true; }  // names no feature row: counts as absent
-      }
-      const int32_t cur_out = q[0].out;
-      const int cur_group = q[0].group;
-      const bool cur_fresh = q[0].fresh;
-#pragma unroll
-      for (int i = 0; i + 1 < AHEAD; ++i) q[i] = q[i + 1];
-      next(q[AHEAD - 1]);
-      if (cur_fresh) {
+    Item q;
+    next(q);
+    int slot = team, phase = 0, dslot = team, dphase = 0;   // (a team uses every other slot of either ring)
+    while (ok && q.group >= 0) {
+      const Item cur = q;
+      next(q);
+      if (cur.dy) {
         if (!mbar_wait(bar(&ctl->dy_empty[dslot]), dphase ^ 1, p.dev_status)) { ok = false; break; }
         const uint32_t dst = b_base + dslot * B_STAGE;
-        for (int i = lane; i < 16 * PR; i += 32) {
+        for (int i = lane; i < 32 * PR; i += 32) {
           const int r = i / PR, piece = i - r * PR;
-          const int32_t row = __shfl_sync(0xFFFFFFFFu, cur_out, r);
-          cp_async16(dst + (piece / CHB) * B_TILE + tile_offset<RBB>(warp * 16 + r, piece % CHB),
+          const int32_t row = __shfl_sync(0xFFFFFFFFu, cur.out, r);
+          cp_async16(dst + (piece / CHB) * B_TILE + tile_offset<RBB>(row0 + r, piece % CHB),
                      row >= 0 ? p.gout + ((int64_t)row * p.c_out) * 2 + piece * 16 : p.gout, row >= 0 ? 16u : 0u);
         }
         cp_async_arrive(bar(&ctl->dy_full[dslot]));  // hardware arrives when this thread's copies land
-        dslot ^= 1;
-        if (dslot == 0) dphase ^= 1;
+        dphase ^= 1;
+        if (cur.group == WG_MAX_GROUPS) continue;
       }
       if (!mbar_wait(bar(&ctl->empty[slot]), phase ^ 1, p.dev_status)) { ok = false; break; }
       const uint32_t dst = base + slot * A_STAGE;
 #pragma unroll
       for (int u = 0; u < GU; ++u) {
-        const char* from = p.feats + (int64_t)(((group0 + cur_group) * GU + u) % UA) * RBA + chunk * 16;
+        const char* from = p.feats + ctl->unit_at[cur.group * GU + u] + chunk * 16;
+        const bool over = cur.idx[u] >= num_in;   // names no feature row: counts as absent
+        bad |= over;
+        const int mine_row = over ? -1 : cur.idx[u];
 #pragma unroll
         for (int j = 0; j < NJ; ++j) {
-          const int r = __shfl_sync(0xFFFFFFFFu, cur[u >> 1], (u & 1) * 16 + j * RPI + sub_row);
-          cp_async16(dst + u * A_TILE + aoff[j], r >= 0 ? from + (int64_t)r * p.c_in * 2 : p.feats, r >= 0 ? 16u : 0u);
+          const int r = __shfl_sync(0xFFFFFFFFu, mine_row, j * RPI + sub_row);
+          cp_async16(dst + u * A_TILE + aoff[j], r >= 0 ? from + r * ld : p.feats, r >= 0 ? 16u : 0u);
         }
       }
       cp_async_arrive(bar(&ctl->full[slot]));
-      if (++slot == p.stages) { slot = 0; phase ^= 1; }
+      slot += 2;
+      if (slot >= p.stages) { slot = team; phase ^= 1; }
     }
     cp_async_drain();
     if (bad) wcn_report_bounds(p.dev_status);
@@ -297,6 +311,7 @@ int launch_wgrad(WgradParams& p, cudaStream_t st) {
   const size_t limit = 226 * 1024, fixed = 1024 + sizeof(WgradControl) + 128;
   int stages = (int)((limit - fixed - 2 * b_stage) / a_stage);
   if (stages > WG_MAX_STAGES) stages = WG_MAX_STAGES;
+  stages &= ~1;   // the two teams take turns
   if (stages < 2) return WCN_ERR_UNSUPPORTED_CONFIG;
   p.stages = stages;
   p.cols = 32;
