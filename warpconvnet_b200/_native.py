@@ -7,6 +7,7 @@ PyTorch is used for device memory and streams only.
 from __future__ import annotations
 
 import ctypes
+import functools
 import importlib.util
 import os
 from collections import Counter
@@ -243,7 +244,9 @@ def check_device_status(device: torch.device) -> None:
     raise_for_status(int(host[0]), device)
 
 
+@functools.lru_cache(maxsize=1024)
 def query_bytes(fn_name: str, *args) -> int:
+    """The size that a ``wcn_*_bytes`` function gives for ``args`` (it depends on them alone)."""
     out = ctypes.c_int64(0)
     check(getattr(lib(), fn_name)(*args, ctypes.byref(out)), fn_name)
     return int(out.value)

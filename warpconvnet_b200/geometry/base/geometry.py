@@ -20,8 +20,8 @@ from .batched import Coords, Features
 def _amp(tensor: Tensor) -> Tensor:
     # geometry.py:17-34: under autocast, features are seen in the autocast dtype
     if torch.is_autocast_enabled():
-        amp_dtype = torch.get_autocast_gpu_dtype()
-        if amp_dtype is not None:
+        amp_dtype = torch.get_autocast_dtype("cuda")
+        if amp_dtype is not None and amp_dtype != tensor.dtype:
             return tensor.to(dtype=amp_dtype)
     return tensor
 

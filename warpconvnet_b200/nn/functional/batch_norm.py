@@ -3,6 +3,8 @@ per direction (``csrc/batch_norm.cu``).  An addition to the reference, whose blo
 and ``nn.ReLU`` one after the other (examples/mink_unet.py:36-47, 129-141); values are rounded where those round."""
 from __future__ import annotations
 
+import functools
+import struct
 from typing import Optional
 
 import torch
@@ -87,9 +89,9 @@ class _BatchNormAct(torch.autograd.Function):
                 sums[0] if ctx.needs_input_grad[2] else None, (dres if ctx.relu else dy) if need_res else None, None, None)
 
 
+@functools.lru_cache(maxsize=64)
 def _bits(value: float) -> int:
     """A float argument as the 32 bits the C function reinterprets (calls pass integers only)."""
-    import struct
     return struct.unpack("<I", struct.pack("<f", value))[0]
 
 

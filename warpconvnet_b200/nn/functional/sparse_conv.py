@@ -1093,22 +1093,69 @@ class _LayerTables:
     one_pair: bool = False
     dst: Optional[Tensor] = None
     coords: Optional[IntCoords] = None  # strided layers: the output coordinates
+    km: Optional[IntSearchResult] = None
 
 
 def _layer_tables(x: Voxels, kernel_size, stride, dilation, transposed: bool, target: Optional[Voxels]) -> _LayerTables:
     n = x.batched_coordinates.batched_tensor.shape[0]
     if all(k == 1 for k in kernel_size) and all(s == 1 for s in stride):
-        return _LayerTables(n, n, _identity_map(n, x.device).neighbor_table(n), None, True)
+        ident = _identity_map(n, x.device)
+        return _LayerTables(n, n, ident.neighbor_table(n), None, True, km=ident)
     out_coords, _, km = generate_output_coords_and_kernel_map(x, kernel_size, dilation, stride, False, transposed, target)
     m = out_coords.shape[0]
     if transposed and getattr(km, "_one_pair", False) and km._forward is not None:
-        return _LayerTables(n, m, None, None, True, km._forward.neighbor_table(n))
+        return _LayerTables(n, m, None, None, True, km._forward.neighbor_table(n), km=km)
     if TILE_ORDER_MIN_OFFSETS <= len(km) <= 32 and m >= TILE_ORDER_MIN_ROWS:
         nbr, out_rows = km.tiled_neighbor_table(m)
     else:
         nbr, out_rows = km.neighbor_table(m), None
     strided = strided_coordinates(x.batched_coordinates, stride) if any(s != 1 for s in stride) and not transposed else None
-    return _LayerTables(n, m, nbr, out_rows, coords=strided)
+    return _LayerTables(n, m, nbr, out_rows, coords=strided, km=km)
+
+
+def _tables_of(layer, x: Voxels, target: Optional[Voxels]):
+    """(the tables of ``layer`` on the coordinates of ``x``, the coordinate set that keeps them), or None when the call
+    is one that only :func:`spatially_sparse_conv` takes."""
+    ic = x.batched_coordinates
+    kernel_size, stride = layer.kernel_size, layer.stride
+    transposed = layer.transposed
+    key = ("layer", kernel_size, stride, layer.dilation, transposed)
+    ones = (1,) * len(kernel_size)
+    if transposed:
+        # only back onto the set these coordinates are the strided ones of: its tables live with that set
+        if target is None:
+            return None
+        holder = target.batched_coordinates
+        parent = holder._shared.get(("strided", stride))
+        if (parent is None or parent._shared is not ic._shared or ic.tensor_stride is None
+                or not any(o < i for o, i in zip(holder.tensor_stride or ones, ic.tensor_stride))):
+            return None
+    elif target is not None:
+        return None
+    else:
+        holder = ic
+    tables = holder._shared.get(key)
+    if tables is None:
+        tables = holder._shared[key] = _layer_tables(x, kernel_size, stride, layer.dilation, transposed, target)
+    return tables, holder
+
+
+def _output_of(layer, x: Voxels, tables: _LayerTables, holder: IntCoords, y: Tensor) -> Voxels:
+    """The result ``y`` of ``layer`` on ``x`` as a geometry."""
+    ic, kernel_size, stride = x.batched_coordinates, layer.kernel_size, layer.stride
+    ones = (1,) * len(kernel_size)
+    if layer.transposed:
+        return x._derive(y, holder)
+    if kernel_size == ones and stride == ones:
+        return x._derive(y)
+    ts = ic.tensor_stride or ones
+    if stride == ones:
+        out_ic, out_ts = ic, ts
+    else:
+        out_ic, out_ts = tables.coords, tuple(o * s for o, s in zip(stride, ts))
+        if out_ic.tensor_stride is None:
+            out_ic.tensor_stride = out_ts  # the cached set is labelled once
+    return x._derive(y, out_ic if out_ic.tensor_stride == out_ts else out_ic.labelled(out_ts))
 
 
 _NATIVE_ALGOS = (SPARSE_CONV_FWD_ALGO_MODE.AUTO, SPARSE_CONV_FWD_ALGO_MODE.IMPLICIT_GEMM,
@@ -1137,26 +1184,10 @@ def run_layer(layer, x: Voxels, target: Optional[Voxels], epilogue: Optional[Con
             return None
     elif layer.fwd_algo not in _NATIVE_ALGOS:
         return None
-    kernel_size, stride = layer.kernel_size, layer.stride
-    transposed = layer.transposed
-    key = ("layer", kernel_size, stride, layer.dilation, transposed)
-    ones = (1,) * len(kernel_size)
-    if transposed:
-        # only back onto the set these coordinates are the strided ones of: its tables live with that set
-        if target is None:
-            return None
-        holder = target.batched_coordinates
-        parent = holder._shared.get(("strided", stride))
-        if (parent is None or parent._shared is not ic._shared or ic.tensor_stride is None
-                or not any(o < i for o, i in zip(holder.tensor_stride or ones, ic.tensor_stride))):
-            return None
-    elif target is not None:
+    found = _tables_of(layer, x, target)
+    if found is None:
         return None
-    else:
-        holder = ic
-    tables = holder._shared.get(key)
-    if tables is None:
-        tables = holder._shared[key] = _layer_tables(x, kernel_size, stride, layer.dilation, transposed, target)
+    tables, holder = found
     m, c_out = tables.num_out, weight.shape[2]
     if m == 0 or tables.num_in != feats.shape[0]:
         return None
@@ -1173,18 +1204,98 @@ def run_layer(layer, x: Voxels, target: Optional[Voxels], epilogue: Optional[Con
         return None
     else:
         y = rec.conv(feats, tables.nbr, tables.out_rows, m, residual, out)
-    if transposed:
-        return x._derive(y, holder)
-    if kernel_size == ones and stride == ones:
-        return x._derive(y)
-    ts = ic.tensor_stride or ones
-    if stride == ones:
-        out_ic, out_ts = ic, ts
+    return _output_of(layer, x, tables, holder, y)
+
+
+class _LayerFunction(torch.autograd.Function):
+    """A layer in training from its tables: what :class:`_SparseConvFunction` does with the implicit algorithms, without
+    deriving the launches from a kernel map's options on every call."""
+
+    @staticmethod
+    def forward(ctx, x: Tensor, weight: Tensor, tables: _LayerTables):
+        ctx.tables = tables
+        ctx.save_for_backward(x, weight)
+        if x.requires_grad:
+            x = x.detach()
+        if tables.nbr is None:
+            return sparse_conv_fused(x, weight, tables.km, tables.num_out)
+        return _launch_layer(x, weight, tables, False, tables.num_out)
+
+    @staticmethod
+    def backward(ctx, g: Tensor):
+        x, weight = ctx.saved_tensors
+        t = ctx.tables
+        gx = gw = None
+        with torch.no_grad():
+            g = g.detach().contiguous()
+            if g.dtype != x.dtype:
+                g = g.to(x.dtype)
+            if ctx.needs_input_grad[0]:
+                facts = getattr(t.km, "_facts", None)
+                if t.nbr is not None and getattr(t.km, "_onto_itself", False) and facts is not None and facts.get("distinct"):
+                    gx = _launch_layer(g, weight, t, True, t.num_in)  # see _input_gradient
+                else:
+                    gx = _input_gradient(g, weight, t.km, t.num_in)
+            if ctx.needs_input_grad[1]:
+                gw = sparse_conv_wgrad(x.detach(), g, t.km, t.num_out, tile_order=t.out_rows is not None)
+                if gw.dtype != weight.dtype:
+                    gw = gw.to(weight.dtype)
+        return gx, gw, None
+
+
+def _launch_layer(x: Tensor, weight: Tensor, t: _LayerTables, gradient: bool, rows: int) -> Tensor:
+    """One launch over the tables of a layer, with its weights or (``gradient``) with each offset's weight transposed
+    and the offsets in reverse order."""
+    if x.stride(1) != 1:
+        x = x.contiguous()
+    w, packed = _prepared_weight(weight, x.dtype, CONV_AUTO, gradient, gradient)
+    K, c_in, c_out = weight.shape
+    if gradient:
+        c_in, c_out = c_out, c_in
+    out = torch.empty((rows, c_out), dtype=x.dtype, device=x.device)
+    dc = dtype_code(x.dtype)
+    rc = lib().wcn_conv_fwd(CONV_AUTO, x.data_ptr(), x.shape[0], x.stride(0), ptr(w), ptr(packed), t.nbr.data_ptr(),
+                            ptr(t.out_rows), rows, K, c_in, c_out, dc, None, None, None, 0, 0, out.data_ptr(), c_out, dc, 0,
+                            None, 0, device_status(x.device).data_ptr(), stream_ptr(x.device))
+    if rc != 0:
+        check(rc, "wcn_conv_fwd")
+    return out
+
+
+def train_layer(layer, x: Voxels, target: Optional[Voxels]) -> Optional[Voxels]:
+    """``layer`` (a :class:`SpatiallySparseConv`) on ``x`` with gradients, from the coordinate set's tables; None when
+    the call is one that only :func:`spatially_sparse_conv` takes."""
+    weight = layer.weight
+    if (type(x) is not Voxels or layer.generative or layer.compute_dtype is not None
+            or layer.order != POINT_ORDERING.RANDOM or layer.stride_mode != STRIDED_CONV_MODE.STRIDE_ONLY
+            or layer.fwd_algo not in _NATIVE_ALGOS or type(layer.bwd_algo) is not SPARSE_CONV_BWD_ALGO_MODE
+            or layer.bwd_algo == SPARSE_CONV_BWD_ALGO_MODE.EXPLICIT_GEMM):
+        return None
+    feats, bias = x.feature_tensor, layer.bias
+    dtype = feats.dtype
+    if (not feats.is_cuda or dtype not in _NATIVE_DTYPES or feats.dim() != 2 or feats.shape[0] == 0
+            or weight.device != feats.device or weight.shape[1] != feats.shape[1]
+            or (weight.dtype != dtype and _min_dtype(dtype, weight.dtype) != dtype)
+            or not (feats.requires_grad or weight.requires_grad or (bias is not None and bias.requires_grad))):
+        return None
+    ones = all(k == 1 for k in layer.kernel_size) and all(s == 1 for s in layer.stride)
+    if ones:
+        if layer.transposed or target is not None:
+            return None
+        y = _PointwiseFunction.apply(feats, weight)
     else:
-        out_ic, out_ts = tables.coords, tuple(o * s for o, s in zip(stride, ts))
-        if out_ic.tensor_stride is None:
-            out_ic.tensor_stride = out_ts  # the cached set is labelled once
-    return x._derive(y, out_ic if out_ic.tensor_stride == out_ts else out_ic.labelled(out_ts))
+        found = _tables_of(layer, x, target)
+        if found is None:
+            return None
+        tables, holder = found
+        if tables.num_out == 0 or tables.num_in != feats.shape[0]:
+            return None
+        if x._extra_attributes.get("_cache") is None:
+            x._extra_attributes["_cache"] = IntSearchCache()  # shared by everything derived from x, as after any convolution
+        y = _LayerFunction.apply(feats, weight, tables)
+    if bias is not None:
+        y = y + bias.to(y.dtype)
+    return x._derive(y) if ones else _output_of(layer, x, tables, holder, y)
 
 
 def _merge_bias(epilogue: Optional[ConvEpilogue], bias: Optional[Tensor]) -> Optional[ConvEpilogue]:

@@ -82,10 +82,14 @@ class Sequential(nn.Sequential, BaseSpatialModule):
         in_sf = x
         i = 0
         fused_tail = False
-        can_fuse = not torch.is_grad_enabled() or not any(p.requires_grad for p in self.parameters())
+        can_fuse = None  # whether a convolution and the BatchNorm behind it may be one launch (looked at when there is one)
         while i < len(mods):
             m = mods[i]
             bn = _as_bn(mods[i + 1]) if i + 1 < len(mods) else None
+            if (isinstance(m, SpatiallySparseConv) and isinstance(x, Geometry) and bn is not None
+                    and not bn.training and bn.track_running_stats and not m.generative):
+                if can_fuse is None:
+                    can_fuse = not torch.is_grad_enabled() or not any(p.requires_grad for p in self.parameters())
             if (can_fuse and isinstance(m, SpatiallySparseConv) and isinstance(x, Geometry) and bn is not None
                     and not bn.training and bn.track_running_stats and not m.generative):
                 j = i + 2

@@ -18,7 +18,7 @@ from ...geometry.coords.ops.serialization import POINT_ORDERING
 from ...geometry.types.voxels import Voxels
 from ...utils.ntuple import ntuple
 from ..functional.sparse_conv import (SPARSE_CONV_BWD_ALGO_MODE, SPARSE_CONV_FWD_ALGO_MODE, STRIDED_CONV_MODE,
-                                      ConvEpilogue, run_layer, spatially_sparse_conv)
+                                      ConvEpilogue, run_layer, train_layer, spatially_sparse_conv)
 from .base_module import BaseSpatialModule
 
 
@@ -89,6 +89,10 @@ class SpatiallySparseConv(BaseSpatialModule):
                 epilogue: Optional[ConvEpilogue] = None):
         if not torch.is_grad_enabled():
             y = run_layer(self, input_sparse_tensor, output_spatially_sparse_tensor, epilogue)
+            if y is not None:
+                return y
+        elif epilogue is None:
+            y = train_layer(self, input_sparse_tensor, output_spatially_sparse_tensor)
             if y is not None:
                 return y
         return spatially_sparse_conv(
