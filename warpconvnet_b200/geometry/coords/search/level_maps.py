@@ -91,7 +91,8 @@ TILE_ORDER_ROWS = 1024
 
 
 class LevelMaps:
-    """Tables of levels 0..4: :meth:`begin` enqueues the pyramid and level 0, :meth:`finish` the other levels."""
+    """Tables of levels 0..4: the constructor enqueues the pyramid and level 0, :meth:`finish` the other levels - or
+    :meth:`attach` leaves this object with the levels' coordinates, whose tables :meth:`ensure` makes as layers ask."""
 
     def __init__(self, ic: IntCoords, tile_order_rows: int = TILE_ORDER_ROWS):
         self.build = PyramidBuild(ic)
@@ -99,8 +100,7 @@ class LevelMaps:
         n = self.build.n
         self.n = [n]
         self.rows = [self.build.rows]
-        self.nbr, self.order, self.child = [], [], []
-        self._bricks = []
+        self.nbr, self.order, self.child, self._bricks = {}, {}, {}, {}
         self._enqueue(range(1))
 
     def _enqueue(self, which) -> None:
@@ -111,22 +111,18 @@ class LevelMaps:
             nbr = torch.empty((27, n), dtype=torch.int32, device=b.device)
             order = torch.empty(n, dtype=torch.int32, device=b.device) if n >= self.min_rows else None
             bricks = torch.empty(query_bytes("wcn_level_brick_bytes", n), dtype=torch.uint8, device=b.device)
-            self.nbr.append(nbr)
-            self.order.append(order)
-            self._bricks.append(bricks)
+            self.nbr[l], self.order[l], self._bricks[l] = nbr, order, bricks
             slot.rows, slot.n, slot.level = self.rows[l].data_ptr(), n, l
             slot.bricks, slot.order, slot.nbr = bricks.data_ptr(), ptr(order), nbr.data_ptr()
             if l:
-                child = torch.empty((8, n), dtype=torch.int32, device=b.device)
-                self.child.append(child)
+                child = self.child[l - 1] = torch.empty((8, n), dtype=torch.int32, device=b.device)
                 slot.child, slot.first_child = child.data_ptr(), b.first[l - 1].data_ptr()
                 slot.rows_below, slot.n_below = self.rows[l - 1].data_ptr(), self.n[l - 1]
         check(lib().wcn_level_maps(ctypes.addressof(levels), len(which), ptr(b.info), ptr(b.counts), stream_ptr(b.device)),
               "wcn_level_maps")
 
-    def finish(self) -> Optional[List[IntCoords]]:
-        """The coordinates of levels 1..4 (None: not usable); their maps are enqueued and every level's maps left with
-        its coordinates, where layers of those geometries find them."""
+    def _levels(self) -> Optional[List[IntCoords]]:
+        """The coordinates of levels 1..4, linked (None: not usable)."""
         b = self.build
         levels = b.finish()
         if levels is None:
@@ -136,13 +132,47 @@ class LevelMaps:
         for c in levels:
             self.rows.append(c._shared["bcoords"])
             self.n.append(self.rows[-1].shape[0])
+        return levels
+
+    def _window3(self, l: int) -> IntSearchResult:
+        if self.order[l] is not None:
+            return IntSearchResult.from_tiled_table(self.nbr[l], self.order[l], self.n[l], 13)
+        return IntSearchResult.from_neighbor_table(self.nbr[l], self.n[l], None, 13)
+
+    def _window2(self, l: int) -> IntSearchResult:
+        return IntSearchResult.from_neighbor_table(self.child[l], self.n[l], None, None)
+
+    def finish(self) -> Optional[List[IntCoords]]:
+        """The coordinates of levels 1..4 (None: not usable); their maps are enqueued and every level's maps left with
+        its coordinates, where layers of those geometries find them."""
+        levels = self._levels()
+        if levels is None:
+            return None
         self._enqueue(range(1, PYRAMID_LEVELS + 1))
         self._bricks = None
-        for l, c in enumerate([b.ic] + levels):
-            if self.order[l] is not None:
-                c._shared[("kmap", (3, 3, 3), (1, 1, 1))] = IntSearchResult.from_tiled_table(self.nbr[l], self.order[l], self.n[l], 13)
-            else:
-                c._shared[("kmap", (3, 3, 3), (1, 1, 1))] = IntSearchResult.from_neighbor_table(self.nbr[l], self.n[l], None, 13)
+        for l, c in enumerate([self.build.ic] + levels):
+            c._shared[("kmap", (3, 3, 3), (1, 1, 1))] = self._window3(l)
             if l < PYRAMID_LEVELS:
-                c._shared[("kmap", (2, 2, 2), (2, 2, 2))] = IntSearchResult.from_neighbor_table(self.child[l], self.n[l], None, None)
+                c._shared[("kmap", (2, 2, 2), (2, 2, 2))] = self._window2(l)
         return levels
+
+    def attach(self) -> bool:
+        """Levels linked, the maps made as layers ask for them (:meth:`kmap`); False: not usable."""
+        levels = self._levels()
+        if levels is None:
+            return False
+        self._bricks = {}
+        for l, c in enumerate([self.build.ic] + levels):
+            c._shared["level_maps"] = (self, l)
+        self.build.ic = None  # (the coordinate sets hold this object, not the other way round)
+        return True
+
+    def kmap(self, l: int, window: int) -> Optional[IntSearchResult]:
+        """The map of level ``l``: 3x3x3 onto itself or 2x2x2 onto the next level."""
+        at = l if window == 3 else l + 1
+        if at > PYRAMID_LEVELS:
+            return None
+        if at not in self.nbr:
+            self._enqueue(range(at, at + 1))
+            self._bricks = {}
+        return self._window3(l) if window == 3 else self._window2(l)

@@ -33,7 +33,7 @@ from ...geometry.coords.integer import IntCoords
 from ...geometry.coords.ops.serialization import POINT_ORDERING, encode
 from ...geometry.coords.ops.expand import expand_coords
 from ...geometry.coords.ops.stride import stride_coords
-from ...geometry.coords.search.level_maps import morton_pyramid
+from ...geometry.coords.search.level_maps import LevelMaps, morton_pyramid
 from ...geometry.coords.search.cache import IntSearchCache, IntSearchCacheKey
 from ...geometry.coords.search.search_results import IntSearchResult
 from ...geometry.coords.search.torch_discrete import generate_kernel_map
@@ -615,12 +615,28 @@ def generate_output_coords_and_kernel_map(input_sparse_tensor: Voxels, kernel_si
     return out_coords, out_offsets, kernel_map
 
 
+_LEVEL_WINDOWS = (((3, 3, 3), (1, 1, 1)), ((2, 2, 2), (2, 2, 2)))
+
+
 def _level_map(fine: Voxels, kernel_size, kernel_dilation, stride, coarse_rows: Tensor) -> Optional[IntSearchResult]:
     """The map of this window that :class:`LevelMaps` left with the coordinates of ``fine`` (from ``fine`` to its own
-    rows or to its strided rows), or None."""
+    rows or to its strided rows), or None.  Natively sorted coordinates get their maps that way: five launches a level
+    where a brick table, a stand-by hash table, a search and a tile order take ten."""
+    if any(d != 1 for d in kernel_dilation):
+        return None
     shared = fine.batched_coordinates._shared
-    km = shared.get(("kmap", tuple(kernel_size), tuple(stride)))
-    if km is None or any(d != 1 for d in kernel_dilation):
+    window = (tuple(kernel_size), tuple(stride))
+    km = shared.get(("kmap",) + window)
+    if km is None and window in _LEVEL_WINDOWS:
+        if "level_maps" not in shared and shared.get("morton_info") is not None and ("strided", (2, 2, 2)) not in shared \
+                and window[0] == (3, 3, 3) and fine.batched_coordinates.batched_tensor.shape[0] > 0:
+            LevelMaps(fine.batched_coordinates, TILE_ORDER_MIN_ROWS).attach()
+        if "level_maps" in shared:
+            maps, level = shared["level_maps"]
+            km = maps.kmap(level, window[0][0])
+            if km is not None:
+                shared[("kmap",) + window] = km
+    if km is None:
         return None
     rows = shared["bcoords"] if all(s == 1 for s in stride) else shared[("strided", tuple(stride))]._shared["bcoords"]
     return km if rows.data_ptr() == coarse_rows.data_ptr() and rows.shape == coarse_rows.shape else None
