@@ -72,3 +72,34 @@ def test_sequential_trains_through_the_fused_layers_and_second_derivatives_work(
     (ggr,) = torch.autograd.grad(gr.sum() + (gr ** 2).sum(), [xr])
     assert rel_l2(gx.detach().cpu().numpy(), gr.detach().cpu().numpy()) < 1e-4
     assert rel_l2(ggx.cpu().numpy(), ggr.cpu().numpy()) < 1e-3
+
+
+@pytest.mark.parametrize("stride,residual,relu", [(1, False, True), (1, True, True), (2, False, False)])
+def test_convolution_and_norm_as_one_function(stride, residual, relu):
+    """A convolution with the BatchNorm, residual and ReLU behind it in training: outputs, running statistics and every
+    gradient as from the layers one by one, and a gradient of the gradient where the layers have one."""
+    from warpconvnet_b200 import Sequential, SparseConv3d, Voxels
+    g = torch.Generator().manual_seed(stride)
+    xyz = torch.unique(torch.randint(0, 24, (4000, 3), generator=g, dtype=torch.int32), dim=0)
+    n = len(xyz)
+    feats = torch.randn(n, 32, generator=g).to(DEV)
+    results = []
+    for together in (True, False):
+        torch.manual_seed(3)
+        seq = Sequential(SparseConv3d(32, 64, 3 if stride == 1 else 2, stride, bias=False), nn.BatchNorm1d(64),
+                         nn.ReLU() if relu and not residual else nn.Identity()).to(DEV).train()
+        x = feats.clone().requires_grad_(True)
+        v = Voxels(xyz.to(DEV), x, offsets=torch.tensor([0, n])).sort()
+        res = torch.linspace(-1, 1, n * 64, device=DEV).view(n, 64).requires_grad_(True) if residual else None
+        if together:
+            y = seq(v, residual=res, final_relu=relu and residual).feature_tensor
+        else:
+            handle = seq[0].register_forward_hook(lambda m, a, out: None)  # a hooked layer runs by itself
+            y = seq(v, residual=res, final_relu=relu and residual).feature_tensor
+            handle.remove()
+        w = torch.linspace(0.5, 1.5, y.numel(), device=DEV).view_as(y)
+        wanted = [x, seq[0].weight, seq[1].weight, seq[1].bias] + ([res] if residual else [])
+        grads = torch.autograd.grad((y * w).sum(), wanted)
+        results.append([y.detach(), seq[1].running_mean.clone(), seq[1].running_var.clone(), *grads])
+    for a, b in zip(*results):
+        assert a.dtype == b.dtype and float((a - b).norm()) <= 1e-5 * max(1.0, float(b.norm()))

@@ -22,7 +22,7 @@ from ..geometry.coords.search.cache import IntSearchCache
 from ..geometry.coords.search.level_maps import LevelMaps
 from ..geometry.coords.search.search_results import IntSearchResult
 from ..nn.functional import sparse_conv
-from ..nn.functional.sparse_conv import (STRIDED_CONV_MODE, TILE_ORDER_MIN_OFFSETS, TILE_ORDER_MIN_ROWS, ConvEpilogue,
+from ..nn.functional.sparse_conv import (STRIDED_CONV_MODE, TILE_ORDER_MIN_OFFSETS, TILE_ORDER_MIN_ROWS, ConvEpilogue, train_layer_norm,
                                          FusedConvLaunch, FusedRowsLaunch, _identity_map, _implicit_gemm_forward_logic, _merge_bias,
                                          generate_output_coords_and_kernel_map, prefetch_strided_coordinates)
 from ..nn.functional.transforms import cat
@@ -60,7 +60,11 @@ class ConvTrBlock(nn.Module):
             scale, shift = fold_batchnorm(bn)
             ep = ConvEpilogue(scale=scale, shift=shift, relu=isinstance(self.norm_act[1], nn.ReLU), out=out)
             return self.conv_tr(x, out_spatial_sparsity, epilogue=ep)
-        res = self.norm_act(self.conv_tr(x, out_spatial_sparsity))
+        res = None
+        if bn.training and torch.is_grad_enabled() and isinstance(self.norm_act[1], (nn.ReLU, nn.Identity)):
+            res = train_layer_norm(self.conv_tr, bn, x, out_spatial_sparsity, isinstance(self.norm_act[1], nn.ReLU), None)
+        if res is None:
+            res = self.norm_act(self.conv_tr(x, out_spatial_sparsity))
         if out is not None:
             out.copy_(res.feature_tensor)
         return res

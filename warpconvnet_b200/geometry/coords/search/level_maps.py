@@ -78,12 +78,7 @@ def morton_pyramid(ic: IntCoords) -> bool:
     """Computes and links the stride-2 levels of a natively sorted set; False when it is none (or not usable)."""
     if ic._shared.get("morton_info") is None:
         return False
-    levels = PyramidBuild(ic).finish()
-    if levels is None:
-        ic._shared["morton_info"] = None
-        return False
-    link_levels(ic, levels)
-    return True
+    return LevelMaps(ic, begin=False).attach()
 
 
 # 3x3x3 tables of at least this many rows are put in tile order.
@@ -91,17 +86,18 @@ TILE_ORDER_ROWS = 1024
 
 
 class LevelMaps:
-    """Tables of levels 0..4: the constructor enqueues the pyramid and level 0, :meth:`finish` the other levels - or
+    """Tables of levels 0..4: the constructor enqueues the pyramid and (``begin``) level 0, :meth:`finish` the other levels - or
     :meth:`attach` leaves this object with the levels' coordinates, whose tables :meth:`ensure` makes as layers ask."""
 
-    def __init__(self, ic: IntCoords, tile_order_rows: int = TILE_ORDER_ROWS):
+    def __init__(self, ic: IntCoords, tile_order_rows: int = TILE_ORDER_ROWS, begin: bool = True):
         self.build = PyramidBuild(ic)
         self.min_rows = tile_order_rows
         n = self.build.n
         self.n = [n]
         self.rows = [self.build.rows]
         self.nbr, self.order, self.child, self._bricks = {}, {}, {}, {}
-        self._enqueue(range(1))
+        if begin:
+            self._enqueue(range(1))
 
     def _enqueue(self, which) -> None:
         b = self.build

@@ -31,33 +31,67 @@ def _counter(device: torch.device, stream: int) -> Tensor:
 
 def can_fuse(bn: nn.Module, x: Tensor) -> bool:
     """Whether ``batch_norm_act`` computes what ``bn(x)`` would (training mode, running statistics kept)."""
+    return (x.is_cuda and x.dim() == 2 and x.is_contiguous() and x.data_ptr() % 16 == 0
+            and fusable(bn, x.shape[0], x.shape[1], x.dtype, x.device))
+
+
+def fusable(bn: nn.Module, n: int, c: int, dtype: torch.dtype, device: torch.device) -> bool:
+    """:func:`can_fuse` for contiguous rows that do not exist yet."""
     if type(bn) is not nn.BatchNorm1d or not bn.training or not bn.track_running_stats or bn.momentum is None:
-        return False
-    if not x.is_cuda or x.dtype not in _DTYPES or x.dim() != 2 or not x.is_contiguous() or x.shape[0] < 2:
         return False
     if bn._forward_hooks or bn._forward_pre_hooks or bn._backward_hooks or bn._backward_pre_hooks:
         return False
-    c = x.shape[1]
-    per16 = 16 // x.element_size()
-    return (c == bn.num_features and c % per16 == 0 and c <= 1024 and x.data_ptr() % 16 == 0
-            and bn.running_mean.dtype == torch.float32 and bn.running_mean.device == x.device
-            and (bn.weight is None or bn.weight.dtype == torch.float32) and (bn.bias is None or bn.bias.dtype == torch.float32))
+    mean, w, b = bn.running_mean, bn.weight, bn.bias
+    return (device.type == "cuda" and dtype in _DTYPES and n >= 2 and c == bn.num_features and c <= 1024
+            and c % (4 if dtype == torch.float32 else 8) == 0 and mean.dtype == torch.float32 and mean.device == device
+            and (w is None or w.dtype == torch.float32) and (b is None or b.dtype == torch.float32))
+
+
+def train_forward(x: Tensor, gamma, beta, residual, bn: nn.BatchNorm1d, relu: bool):
+    """(the rows, mean and 1 / std) of one training step; the running statistics advance."""
+    n, c = x.shape
+    dev, dc, st = x.device, dtype_code(x.dtype), stream_ptr(x.device)
+    y = torch.empty_like(x)
+    saved = torch.empty((2, c), dtype=torch.float32, device=dev)
+    ws = torch.empty(query_bytes("wcn_batch_norm_workspace_bytes", n, c, dc), dtype=torch.uint8, device=dev)
+    at = saved.data_ptr()
+    check(lib().wcn_batch_norm_train(ptr(x), n, c, dc, ptr(gamma), ptr(beta), _bits(bn.eps), _bits(bn.momentum),
+                                     ptr(bn.running_mean), ptr(bn.running_var), ptr(bn.num_batches_tracked), ptr(residual),
+                                     int(relu), ptr(y), at, at + 4 * c, ptr(ws), ptr(_counter(dev, st)), st),
+          "wcn_batch_norm_train")
+    torch.autograd.graph.increment_version([bn.running_mean, bn.running_var, bn.num_batches_tracked])
+    return y, saved
+
+
+def train_backward(dy: Tensor, x: Tensor, gamma, beta, saved: Tensor, y: Optional[Tensor], relu: bool, need_x: bool,
+                   need_res: bool):
+    """(dx, (d beta, d gamma), d residual); ``y`` only with a residual under a ReLU."""
+    n, c = x.shape
+    dev, dc, st = x.device, dtype_code(x.dtype), stream_ptr(x.device)
+    dy = dy.contiguous()
+    want_res = need_res and relu
+    dx = torch.empty_like(x) if need_x or want_res else None
+    dres = torch.empty_like(x) if want_res else None
+    sums = torch.empty((2, c), dtype=torch.float32, device=dev)
+    ws = torch.empty(query_bytes("wcn_batch_norm_workspace_bytes", n, c, dc), dtype=torch.uint8, device=dev)
+    at = saved.data_ptr()
+    check(lib().wcn_batch_norm_backward(ptr(x), ptr(dy), ptr(y), n, c, dc, ptr(gamma), ptr(beta), at, at + 4 * c, int(relu),
+                                        ptr(dx), ptr(dres), ptr(sums), ptr(ws), ptr(_counter(dev, st)), st),
+          "wcn_batch_norm_backward")
+    return dx, sums, (dres if relu else dy) if need_res else None
+
+
+def formula(x: Tensor, gamma, beta, residual, eps: float, relu: bool) -> Tensor:
+    """The same through torch, for a graph of the gradient (running statistics untouched)."""
+    z = torch.nn.functional.batch_norm(x, None, None, gamma, beta, True, 0.0, eps)
+    z = z if residual is None else z + residual
+    return torch.relu(z) if relu else z
 
 
 class _BatchNormAct(torch.autograd.Function):
     @staticmethod
     def forward(ctx, x: Tensor, gamma: Optional[Tensor], beta: Optional[Tensor], residual: Optional[Tensor], bn, relu: bool):
-        n, c = x.shape
-        dev, dc, st = x.device, dtype_code(x.dtype), stream_ptr(x.device)
-        y = torch.empty_like(x)
-        saved = torch.empty((2, c), dtype=torch.float32, device=dev)
-        ws = torch.empty(query_bytes("wcn_batch_norm_workspace_bytes", n, c, dc), dtype=torch.uint8, device=dev)
-        at = saved.data_ptr()
-        check(lib().wcn_batch_norm_train(ptr(x), n, c, dc, ptr(gamma), ptr(beta), _bits(bn.eps), _bits(bn.momentum),
-                                         ptr(bn.running_mean), ptr(bn.running_var), ptr(bn.num_batches_tracked), ptr(residual),
-                                         int(relu), ptr(y), at, at + 4 * c, ptr(ws), ptr(_counter(dev, st)), st),
-              "wcn_batch_norm_train")
-        torch.autograd.graph.increment_version([bn.running_mean, bn.running_var, bn.num_batches_tracked])
+        y, saved = train_forward(x, gamma, beta, residual, bn, relu)
         ctx.relu, ctx.eps = relu, bn.eps
         ctx.save_for_backward(x, gamma, beta, residual, saved, y if relu and residual is not None else None)
         return y
@@ -66,27 +100,13 @@ class _BatchNormAct(torch.autograd.Function):
     def backward(ctx, dy: Tensor):
         x, gamma, beta, residual, saved, y = ctx.saved_tensors
         if torch.is_grad_enabled():  # a graph of the gradient is wanted: the same formulas through torch
-            z = torch.nn.functional.batch_norm(x, None, None, gamma, beta, True, 0.0, ctx.eps)
-            z = z if residual is None else z + residual
-            z = torch.relu(z) if ctx.relu else z
+            z = formula(x, gamma, beta, residual, ctx.eps, ctx.relu)
             wanted = [t for t, need in zip((x, gamma, beta, residual), ctx.needs_input_grad) if need]
             got = iter(torch.autograd.grad(z, wanted, dy, create_graph=True))
             return tuple(next(got) if need else None for need in ctx.needs_input_grad[:4]) + (None, None)
-        n, c = x.shape
-        dev, dc, st = x.device, dtype_code(x.dtype), stream_ptr(x.device)
-        dy = dy.contiguous()
-        need_x, _, _, need_res = ctx.needs_input_grad[:4]
-        want_res = need_res and ctx.relu
-        dx = torch.empty_like(x) if need_x or want_res else None
-        dres = torch.empty_like(x) if want_res else None
-        sums = torch.empty((2, c), dtype=torch.float32, device=dev)
-        ws = torch.empty(query_bytes("wcn_batch_norm_workspace_bytes", n, c, dc), dtype=torch.uint8, device=dev)
-        at = saved.data_ptr()
-        check(lib().wcn_batch_norm_backward(ptr(x), ptr(dy), ptr(y), n, c, dc, ptr(gamma), ptr(beta), at, at + 4 * c,
-                                            int(ctx.relu), ptr(dx), ptr(dres), ptr(sums), ptr(ws), ptr(_counter(dev, st)), st),
-              "wcn_batch_norm_backward")
-        return (dx if need_x else None, sums[1] if ctx.needs_input_grad[1] else None,
-                sums[0] if ctx.needs_input_grad[2] else None, (dres if ctx.relu else dy) if need_res else None, None, None)
+        need_x, need_g, need_b, need_res = ctx.needs_input_grad[:4]
+        dx, sums, dres = train_backward(dy, x, gamma, beta, saved, y, ctx.relu, need_x, need_res)
+        return dx if need_x else None, sums[1] if need_g else None, sums[0] if need_b else None, dres, None, None
 
 
 @functools.lru_cache(maxsize=64)
@@ -95,11 +115,16 @@ def _bits(value: float) -> int:
     return struct.unpack("<I", struct.pack("<f", value))[0]
 
 
-def batch_norm_act(x: Tensor, bn: nn.BatchNorm1d, relu: bool = False, residual: Optional[Tensor] = None) -> Tensor:
-    """``relu(bn(x) + residual)`` of a training step (see :func:`can_fuse`)."""
+def aligned_residual(residual: Optional[Tensor], shape, dtype: torch.dtype) -> Optional[Tensor]:
     if residual is not None:
-        assert residual.shape == x.shape, f"residual {tuple(residual.shape)} != {tuple(x.shape)}"
-        residual = residual.to(x.dtype).contiguous()
+        assert residual.shape == shape, f"residual {tuple(residual.shape)} != {tuple(shape)}"
+        residual = residual.to(dtype).contiguous()
         if residual.data_ptr() % 16:
             residual = residual.clone()
+    return residual
+
+
+def batch_norm_act(x: Tensor, bn: nn.BatchNorm1d, relu: bool = False, residual: Optional[Tensor] = None) -> Tensor:
+    """``relu(bn(x) + residual)`` of a training step (see :func:`can_fuse`)."""
+    residual = aligned_residual(residual, x.shape, x.dtype)
     return _BatchNormAct.apply(x, bn.weight, bn.bias, residual, bn, relu)

@@ -34,6 +34,7 @@ from ...geometry.coords.ops.serialization import POINT_ORDERING, encode
 from ...geometry.coords.ops.expand import expand_coords
 from ...geometry.coords.ops.stride import stride_coords
 from ...geometry.coords.search.level_maps import LevelMaps, morton_pyramid
+from . import batch_norm
 from ...geometry.coords.search.cache import IntSearchCache, IntSearchCacheKey
 from ...geometry.coords.search.search_results import IntSearchResult
 from ...geometry.coords.search.torch_discrete import generate_kernel_map
@@ -1231,32 +1232,64 @@ class _LayerFunction(torch.autograd.Function):
     def forward(ctx, x: Tensor, weight: Tensor, tables: _LayerTables):
         ctx.tables = tables
         ctx.save_for_backward(x, weight)
-        if x.requires_grad:
-            x = x.detach()
-        if tables.nbr is None:
-            return sparse_conv_fused(x, weight, tables.km, tables.num_out)
-        return _launch_layer(x, weight, tables, False, tables.num_out)
+        return _layer_output(x.detach(), weight, tables)
 
     @staticmethod
     def backward(ctx, g: Tensor):
         x, weight = ctx.saved_tensors
-        t = ctx.tables
-        gx = gw = None
-        with torch.no_grad():
-            g = g.detach().contiguous()
-            if g.dtype != x.dtype:
-                g = g.to(x.dtype)
-            if ctx.needs_input_grad[0]:
-                facts = getattr(t.km, "_facts", None)
-                if t.nbr is not None and getattr(t.km, "_onto_itself", False) and facts is not None and facts.get("distinct"):
-                    gx = _launch_layer(g, weight, t, True, t.num_in)  # see _input_gradient
-                else:
-                    gx = _input_gradient(g, weight, t.km, t.num_in)
-            if ctx.needs_input_grad[1]:
-                gw = sparse_conv_wgrad(x.detach(), g, t.km, t.num_out, tile_order=t.out_rows is not None)
-                if gw.dtype != weight.dtype:
-                    gw = gw.to(weight.dtype)
+        gx, gw = _layer_gradients(g, x, weight, ctx.tables, *ctx.needs_input_grad[:2])
         return gx, gw, None
+
+
+class _LayerNormFunction(torch.autograd.Function):
+    """A layer in training with the BatchNorm, residual and ReLU behind it: one node of the graph for what is two
+    otherwise (a node costs the host about 60 us a step, as much as its launches)."""
+
+    @staticmethod
+    def forward(ctx, x: Tensor, weight: Tensor, gamma, beta, residual, tables: _LayerTables, bn, relu: bool):
+        z = _layer_output(x.detach(), weight, tables)
+        y, stats = batch_norm.train_forward(z, gamma, beta, residual, bn, relu)
+        ctx.tables, ctx.relu, ctx.eps = tables, relu, bn.eps
+        ctx.save_for_backward(x, weight, gamma, beta, residual, z, stats, y if relu and residual is not None else None)
+        return y
+
+    @staticmethod
+    def backward(ctx, dy: Tensor):
+        x, weight, gamma, beta, residual, z, stats, y = ctx.saved_tensors
+        need = ctx.needs_input_grad[:5]
+        if torch.is_grad_enabled():  # a graph of the gradient is wanted: the two steps as they are without this function
+            out = batch_norm.formula(_LayerFunction.apply(x, weight, ctx.tables), gamma, beta, residual, ctx.eps, ctx.relu)
+            got = iter(torch.autograd.grad(out, [t for t, n in zip((x, weight, gamma, beta, residual), need) if n], dy,
+                                           create_graph=True))
+            return tuple(next(got) if n else None for n in need) + (None, None, None)
+        dz, sums, dres = batch_norm.train_backward(dy, z, gamma, beta, stats, y, ctx.relu, need[0] or need[1], need[4])
+        gx, gw = _layer_gradients(dz, x, weight, ctx.tables, need[0], need[1]) if need[0] or need[1] else (None, None)
+        return gx, gw, sums[1] if need[2] else None, sums[0] if need[3] else None, dres, None, None, None
+
+
+def _layer_output(x: Tensor, weight: Tensor, t: _LayerTables) -> Tensor:
+    if t.nbr is None:
+        return sparse_conv_fused(x, weight, t.km, t.num_out)
+    return _launch_layer(x, weight, t, False, t.num_out)
+
+
+def _layer_gradients(g: Tensor, x: Tensor, weight: Tensor, t: _LayerTables, need_x: bool, need_w: bool):
+    gx = gw = None
+    with torch.no_grad():
+        g = g.detach().contiguous()
+        if g.dtype != x.dtype:
+            g = g.to(x.dtype)
+        if need_x:
+            facts = getattr(t.km, "_facts", None)
+            if t.nbr is not None and getattr(t.km, "_onto_itself", False) and facts is not None and facts.get("distinct"):
+                gx = _launch_layer(g, weight, t, True, t.num_in)  # see _input_gradient
+            else:
+                gx = _input_gradient(g, weight, t.km, t.num_in)
+        if need_w:
+            gw = sparse_conv_wgrad(x.detach(), g, t.km, t.num_out, tile_order=t.out_rows is not None)
+            if gw.dtype != weight.dtype:
+                gw = gw.to(weight.dtype)
+    return gx, gw
 
 
 def _launch_layer(x: Tensor, weight: Tensor, t: _LayerTables, gradient: bool, rows: int) -> Tensor:
@@ -1278,40 +1311,75 @@ def _launch_layer(x: Tensor, weight: Tensor, t: _LayerTables, gradient: bool, ro
     return out
 
 
+def _trains_natively(layer, x: Voxels) -> bool:
+    """Whether a training call of ``layer`` on ``x`` is one that runs from tables."""
+    feats, weight = x.batched_features.batched_tensor, layer.weight
+    return (type(x) is Voxels and not layer.generative and layer.compute_dtype is None
+            and layer.order == POINT_ORDERING.RANDOM and layer.stride_mode == STRIDED_CONV_MODE.STRIDE_ONLY
+            and layer.fwd_algo in _NATIVE_ALGOS and type(layer.bwd_algo) is SPARSE_CONV_BWD_ALGO_MODE
+            and layer.bwd_algo != SPARSE_CONV_BWD_ALGO_MODE.EXPLICIT_GEMM
+            and feats.is_cuda and feats.dim() == 2 and feats.shape[0] > 0
+            and weight.device == feats.device and weight.shape[1] == feats.shape[1])
+
+
+def _training_tables(layer, x: Voxels, target: Optional[Voxels], feats: Tensor):
+    """(tables, their coordinate set) of a training call, or None."""
+    dtype, weight = feats.dtype, layer.weight
+    if dtype not in _NATIVE_DTYPES or (weight.dtype != dtype and _min_dtype(dtype, weight.dtype) != dtype):
+        return None
+    found = _tables_of(layer, x, target)
+    if found is None or found[0].num_out == 0 or found[0].num_in != feats.shape[0]:
+        return None
+    if x._extra_attributes.get("_cache") is None:
+        x._extra_attributes["_cache"] = IntSearchCache()  # shared by everything derived from x, as after any convolution
+    return found
+
+
+def _is_pointwise(layer) -> bool:
+    return all(k == 1 for k in layer.kernel_size) and all(s == 1 for s in layer.stride)
+
+
 def train_layer(layer, x: Voxels, target: Optional[Voxels]) -> Optional[Voxels]:
     """``layer`` (a :class:`SpatiallySparseConv`) on ``x`` with gradients, from the coordinate set's tables; None when
     the call is one that only :func:`spatially_sparse_conv` takes."""
-    weight = layer.weight
-    if (type(x) is not Voxels or layer.generative or layer.compute_dtype is not None
-            or layer.order != POINT_ORDERING.RANDOM or layer.stride_mode != STRIDED_CONV_MODE.STRIDE_ONLY
-            or layer.fwd_algo not in _NATIVE_ALGOS or type(layer.bwd_algo) is not SPARSE_CONV_BWD_ALGO_MODE
-            or layer.bwd_algo == SPARSE_CONV_BWD_ALGO_MODE.EXPLICIT_GEMM):
+    if type(x) is not Voxels or not _trains_natively(layer, x):
         return None
-    feats, bias = x.feature_tensor, layer.bias
-    dtype = feats.dtype
-    if (not feats.is_cuda or dtype not in _NATIVE_DTYPES or feats.dim() != 2 or feats.shape[0] == 0
-            or weight.device != feats.device or weight.shape[1] != feats.shape[1]
-            or (weight.dtype != dtype and _min_dtype(dtype, weight.dtype) != dtype)
-            or not (feats.requires_grad or weight.requires_grad or (bias is not None and bias.requires_grad))):
+    weight, bias, feats = layer.weight, layer.bias, x.feature_tensor
+    if not (feats.requires_grad or weight.requires_grad or (bias is not None and bias.requires_grad)):
         return None
-    ones = all(k == 1 for k in layer.kernel_size) and all(s == 1 for s in layer.stride)
-    if ones:
-        if layer.transposed or target is not None:
+    pointwise = _is_pointwise(layer)
+    if pointwise:
+        if layer.transposed or target is not None or feats.dtype not in _NATIVE_DTYPES:
             return None
         y = _PointwiseFunction.apply(feats, weight)
     else:
-        found = _tables_of(layer, x, target)
+        found = _training_tables(layer, x, target, feats)
         if found is None:
             return None
-        tables, holder = found
-        if tables.num_out == 0 or tables.num_in != feats.shape[0]:
-            return None
-        if x._extra_attributes.get("_cache") is None:
-            x._extra_attributes["_cache"] = IntSearchCache()  # shared by everything derived from x, as after any convolution
-        y = _LayerFunction.apply(feats, weight, tables)
+        y = _LayerFunction.apply(feats, weight, found[0])
     if bias is not None:
         y = y + bias.to(y.dtype)
-    return x._derive(y) if ones else _output_of(layer, x, tables, holder, y)
+    return x._derive(y) if pointwise else _output_of(layer, x, *found, y)
+
+
+def train_layer_norm(layer, bn, x: Voxels, target: Optional[Voxels], relu: bool, residual: Optional[Tensor]) -> Optional[Voxels]:
+    """:func:`train_layer` with ``relu(bn(.) + residual)`` behind it; None when one of them does not take the call."""
+    if (type(x) is not Voxels or layer.bias is not None or not _trains_natively(layer, x) or _is_pointwise(layer)
+            or layer._forward_hooks or layer._forward_pre_hooks or layer._backward_hooks or layer._backward_pre_hooks):
+        return None
+    feats, weight = x.feature_tensor, layer.weight
+    if not (feats.requires_grad or weight.requires_grad) or (residual is not None and residual.dtype != feats.dtype):
+        return None
+    found = _training_tables(layer, x, target, feats)
+    if found is None:
+        return None
+    tables, holder = found
+    m, c = tables.num_out, weight.shape[2]
+    if not batch_norm.fusable(bn, m, c, feats.dtype, feats.device):
+        return None
+    y = _LayerNormFunction.apply(feats, weight, bn.weight, bn.bias, batch_norm.aligned_residual(residual, (m, c), feats.dtype),
+                                 tables, bn, relu)
+    return _output_of(layer, x, tables, holder, y)
 
 
 def _merge_bias(epilogue: Optional[ConvEpilogue], bias: Optional[Tensor]) -> Optional[ConvEpilogue]:

@@ -15,7 +15,7 @@ from torch import Tensor
 from ...geometry.base.geometry import Geometry
 from ...geometry.types.voxels import Voxels
 from ..functional import batch_norm
-from ..functional.sparse_conv import ConvEpilogue
+from ..functional.sparse_conv import ConvEpilogue, train_layer_norm
 from .activations import ReLU as GeometryReLU
 from .base_module import BaseSpatialModule
 from .normalizations import BatchNorm as GeometryBatchNorm
@@ -70,6 +70,17 @@ def _is_relu(m) -> bool:
 
 
 class Sequential(nn.Sequential, BaseSpatialModule):
+    @staticmethod
+    def _behind_norm(mods, j: int, residual: Optional[Tensor], final_relu: bool):
+        """What a BatchNorm before position ``j`` can take along: (position behind it, ReLU, residual, whether the
+        sequence's ``residual`` / ``final_relu`` are in it)."""
+        relu = j < len(mods) and _is_relu(mods[j])
+        if relu or (j < len(mods) and isinstance(mods[j], nn.Identity)):
+            j += 1
+        if j == len(mods) and (residual is not None or final_relu) and not relu:
+            return j, final_relu, residual, True
+        return j, relu, None, False
+
     def forward(self, x: Geometry, residual: Optional[Tensor] = None, final_relu: bool = False,
                 out: Optional[Tensor] = None):
         """``residual`` / ``final_relu`` (additions to the reference signature) are
@@ -108,6 +119,14 @@ class Sequential(nn.Sequential, BaseSpatialModule):
                 x = m(x, epilogue=ep)
                 i = j
                 continue
+            if bn is not None and bn.training and isinstance(m, SpatiallySparseConv) and torch.is_grad_enabled():
+                # training: the convolution with its normalisation, residual and ReLU as one function
+                j, relu, res, tail = self._behind_norm(mods, i + 2, residual, final_relu)
+                y = train_layer_norm(m, bn, x, None, relu, res)
+                if y is not None:
+                    x, i = y, j
+                    fused_tail |= tail
+                    continue
             bn = _as_bn(m)
             if bn is not None and bn.training:
                 feats = x if isinstance(x, Tensor) else x.feature_tensor
@@ -115,14 +134,10 @@ class Sequential(nn.Sequential, BaseSpatialModule):
                     # training: normalisation, residual and ReLU as one function
                     if isinstance(x, Geometry):
                         in_sf = x
-                    j = i + 1
-                    relu = j < len(mods) and _is_relu(mods[j])
-                    if relu or (j < len(mods) and isinstance(mods[j], nn.Identity)):
-                        j += 1
-                    res = None
-                    if j == len(mods) and (residual is not None or final_relu) and not relu \
-                            and (residual is None or residual.dtype == feats.dtype):
-                        res, relu, fused_tail = residual, final_relu, True
+                    j, relu, res, tail = self._behind_norm(mods, i + 1, residual, final_relu)
+                    if tail and residual is not None and residual.dtype != feats.dtype:
+                        relu, res, tail = False, None, False
+                    fused_tail |= tail
                     x = batch_norm.batch_norm_act(feats, bn, relu, res)
                     i = j
                     continue
