@@ -368,7 +368,7 @@ int wcn_conv_workspace_bytes(int algo, int64_t num_out, int32_t num_offsets, int
  * one (a skip connection's half of a concatenated buffer); rows must start on 16-byte boundaries
  * for the tensor-core kernel.  nbr entries >= num_in count as absent and raise WCN_ERR_BOUNDS.
  * num_in and M are below 2^31 (row numbers are 32-bit); larger values return WCN_ERR_INVALID_PARAMETERS.
- * algo WCN_CONV_TCGEN05 needs dtype f16/bf16, c_in % 32 == 0, c_out % 16 == 0, 16 <= c_out <= 256
+ * algo WCN_CONV_TCGEN05 needs dtype f16/bf16, c_in >= 16, c_in % 8 == 0, c_out % 16 == 0, 16 <= c_out <= 256
  * and `packed_weight` from wcn_conv_pack_weight; WCN_CONV_AUTO picks it when those hold and
  * packed_weight is not NULL, else the SIMT kernel.
  * split_k: the tensor-core kernel may divide the kernel offsets of a 128-row block among the S CTAs of a cluster (slice s
@@ -441,7 +441,7 @@ int wcn_conv_rows_fwd(const void* feats, int64_t num_in, int64_t feats_ld, const
  *   grad_weight[k] += feats[nbr[k*M + m], :]^T (outer) grad_out[m, :]   over rows m with nbr >= 0
  * feats / grad_out share `dtype` (f16 or bf16), fp32 accumulation on the tensor cores; the partial
  * sums of different row ranges are added with atomics, so the last bits vary from run to run.
- * Needs c_in % 32 == 0, c_out % 32 == 0, c_out <= 256; else WCN_ERR_UNSUPPORTED_CONFIG (callers
+ * Needs c_in >= 16, c_in % 8 == 0, c_out % 16 == 0, c_out <= 256; else WCN_ERR_UNSUPPORTED_CONFIG (callers
  * take wcn_conv_wgrad_pairs).  (`nbr`, `out_rows`) is the pair wcn_conv_fwd takes: the plain table
  * with out_rows NULL, or the tiled one with its row order (grad_out is then read at out_rows[s]);
  * `tile_masks` (from wcn_kmap_tile_masks on the same table, or NULL) lets the kernel skip the 128-row

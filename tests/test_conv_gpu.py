@@ -651,3 +651,30 @@ def test_tensor_core_units_at_the_edges(ksize, n, c_in, c_out):
         check_device_status(DEV)
         assert torch.equal(got[0], got[1]) and torch.equal(got[0], got[2])
         assert rel_l2(got[0].float().cpu().numpy(), ref.float().cpu().numpy()) < 2e-3
+
+
+@pytest.mark.parametrize("dtype", [torch.float16, torch.bfloat16])
+@pytest.mark.parametrize("ksize,n,c_in,c_out", [(3, 3000, 48, 64), (3, 700, 16, 16), (3, 5001, 40, 48), (3, 90000, 24, 112),
+                                                (2, 4000, 112, 80), (3, 2000, 200, 208), (1, 600, 72, 32)])
+def test_widths_between_the_channel_slices(dtype, ksize, n, c_in, c_out):
+    """Input widths that are multiples of 8 but not of 32 run on the tensor cores with zeros behind their channels: forward
+    and weight gradient against the FP32-pipe kernels and a GEMM per offset; features that start at any address."""
+    from warpconvnet_b200.nn.functional.sparse_conv import sparse_conv_wgrad
+    coords, _, _ = _layer_case(n, 8, 8, n, "raster_crop")
+    c = torch.from_numpy(coords).to(DEV)
+    kmap = generate_kernel_map(c, c, (1, 1, 1), (ksize,) * 3)
+    g = torch.Generator().manual_seed(n)
+    wide = torch.randn(n, c_in + 1, generator=g).to(dtype).to(DEV)
+    dy = torch.randn(n, c_out, generator=g).to(dtype).to(DEV)
+    w = (torch.randn(ksize ** 3, c_in, c_out, generator=g) * 0.1).to(dtype).to(DEV)
+    x = wide[:, 1:].contiguous()
+    ref = sparse_conv_fused(x, w, kmap, n, algo=CONV_SIMT).float()
+    for got in (sparse_conv_fused(x, w, kmap, n, algo=CONV_TCGEN05), sparse_conv_fused(x, w, kmap, n),
+                sparse_conv_fused(wide[:, 1:], w, kmap, n)):
+        check_device_status(DEV)
+        assert rel_l2(got.float().cpu().numpy(), ref.cpu().numpy()) < (2e-3 if dtype == torch.float16 else 1.2e-2)
+    nbr = kmap.neighbor_table(n)
+    want = torch.stack([x.float()[nbr[k].clamp(min=0).long()].mul((nbr[k] >= 0)[:, None]).T @ dy.float() for k in range(len(nbr))])
+    got = sparse_conv_wgrad(x, dy, kmap, n)
+    check_device_status(DEV)
+    assert rel_l2(got.cpu().numpy(), want.cpu().numpy()) < 1e-3

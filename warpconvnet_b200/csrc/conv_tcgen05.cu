@@ -72,7 +72,8 @@ struct ConvTcParams {
   int64_t M, num_in;
   int64_t in_ld_bytes;      // distance between consecutive feature rows, bytes
   int64_t out_ld, res_ld;   // distance between consecutive output / residual rows, elements
-  int K, c_in, c_out;
+  int K, c_in, c_out;       // c_in: padded to the packed weights' channel slices
+  int row_bytes;            // bytes of a feature row (the channels beyond are filled with zeros)
   const float* scale;
   const float* shift;
   const void* residual;
@@ -495,6 +496,7 @@ conv_tcgen05_kernel(const ConvTcParams p) {
 #pragma unroll
     for (int j = 0; j < 2 * NJ; ++j) aoff[j] = tile_offset<RB>((row0 + j * RPI + sub_row) & (BLOCK_M - 1), chunk);
     const char* feats = p.feats + chunk * 16;
+    const int valid = p.row_bytes - chunk * 16;   // a slice that starts at or beyond it has no channels for this thread
     Ring ra{0, 0, p.sa};
     const uint32_t ring = a_base + g * p.sa * A_SLOT;
     for (int n = 0; ok; ++n) {
@@ -520,7 +522,8 @@ conv_tcgen05_kernel(const ConvTcParams p) {
           }
         }
       };
-      auto copy = [&](uint32_t dst, const char* const (&src)[2 * NJ], uint32_t have, int64_t at) {
+      auto copy = [&](uint32_t dst, const char* const (&src)[2 * NJ], uint32_t have, int at) {
+        if (BK == 32 && at >= valid) { have = 0; at = 0; }   // (rows that fill their slices to the end run with BK = 64 too)
 #pragma unroll
         for (int h = 0; h < 2; ++h) {
           if (h < G) {
@@ -565,7 +568,7 @@ conv_tcgen05_kernel(const ConvTcParams p) {
           const uint32_t dst = ring + ra.slot * A_SLOT;
 #pragma unroll
           for (int u = 0; u < KBC; ++u)  // the row's next channel slices are contiguous in memory
-            copy(dst + u * A_BYTES, src, have, (int64_t)(kb0 + u) * RB);
+            copy(dst + u * A_BYTES, src, have, (kb0 + u) * RB);
           cp_async_arrive(bar(&ctl->a_full[g][ra.slot]));  // hardware arrives when this thread's copies land
           ra.advance();
         }
@@ -841,30 +844,33 @@ conv_tcgen05_kernel(const ConvTcParams p) {
 template <typename TS, typename TD>
 __global__ void pack_weight_kernel(const TS* __restrict__ w, TD* __restrict__ packed, int K, int c_in, int c_out, int bk,
                                    int transposed, int reversed) {
-  const int64_t total = (int64_t)K * (c_in / 8) * c_out;
+  const int pad = (c_in + 31) / 32 * 32;   // channels c_in .. pad - 1 are zeros
+  const int64_t total = (int64_t)K * (pad / 8) * c_out;
   const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= total) return;
   // consecutive threads run along the dimension that is contiguous in the source
   int n, c8;
   int64_t r;
-  if (transposed) { c8 = (int)(i % (c_in / 8)); r = i / (c_in / 8); n = (int)(r % c_out); r /= c_out; }
-  else { n = (int)(i % c_out); r = i / c_out; c8 = (int)(r % (c_in / 8)); r /= c_in / 8; }
+  if (transposed) { c8 = (int)(i % (pad / 8)); r = i / (pad / 8); n = (int)(r % c_out); r /= c_out; }
+  else { n = (int)(i % c_out); r = i / c_out; c8 = (int)(r % (pad / 8)); r /= pad / 8; }
   const int k = (int)r, cin = c8 * 8;
   const int64_t ks = reversed ? K - 1 - k : k;
   __align__(16) TD v[8];
 #pragma unroll
   for (int u = 0; u < 8; ++u) {
     const int64_t at = transposed ? (ks * c_out + n) * c_in + cin + u : (ks * c_in + cin + u) * c_out + n;
-    v[u] = wcn_from_float<TD>(wcn_to_float<TS>(w[at]));
+    v[u] = wcn_from_float<TD>(cin + u < c_in ? wcn_to_float<TS>(w[at]) : 0.f);
   }
   const int kb = cin / bk, c = cin % bk;
   const int rb = bk * 2, chunk = c >> 3, r8 = n & 7;
   const int x = rb == 128 ? r8 : (r8 >> 1);
-  const int64_t tile = ((int64_t)k * (c_in / bk) + kb) * c_out * bk;  // elements
+  const int64_t tile = ((int64_t)k * (pad / bk) + kb) * c_out * bk;  // elements
   const int64_t off_bytes = (int64_t)(n >> 3) * (8 * rb) + r8 * rb + ((chunk ^ x) << 4);
   *reinterpret_cast<uint4*>(packed + tile + off_bytes / 2) = *reinterpret_cast<const uint4*>(v);
 }
 
+inline int padded(int c_in) { return (c_in + 31) / 32 * 32; }
+// (the check for channels beyond the row cost the BK = 64 form 2 % of a 256-channel layer: it has none)
 inline int pick_bk(int c_in) { return c_in % 64 == 0 ? 64 : 32; }
 
 // CTAs that can be resident at once in clusters of S (they stay inside a group of multiprocessors, whose sizes differ).
@@ -1077,14 +1083,14 @@ extern "C" int wcn_selftest_bounded_wait(int64_t limit_cycles, int32_t* dev_stat
 
 bool wcn_conv_tcgen05_supported(int K, int c_in, int c_out, int dtype, int out_dtype) {
   return (dtype == WCN_F16 || dtype == WCN_BF16) && (out_dtype == dtype || out_dtype == WCN_F32) && K >= 1 &&
-         K <= MAX_OFFSETS && c_in >= 32 && c_in % 32 == 0 && c_out >= 16 && c_out <= 256 && c_out % 16 == 0;
+         K <= MAX_OFFSETS && c_in >= 16 && c_in % 8 == 0 && c_out >= 16 && c_out <= 256 && c_out % 16 == 0;
 }
 
-int64_t wcn_conv_tcgen05_packed_bytes(int K, int c_in, int c_out) { return (int64_t)K * c_in * c_out * 2; }
+int64_t wcn_conv_tcgen05_packed_bytes(int K, int c_in, int c_out) { return (int64_t)K * padded(c_in) * c_out * 2; }
 
 int wcn_conv_tcgen05_pack(const void* weight, int src_dtype, int K, int c_in, int c_out, int dtype, int transposed, int reversed,
                           void* packed, cudaStream_t st) {
-  const int64_t total = (int64_t)K * (c_in / 8) * c_out;
+  const int64_t total = (int64_t)K * (padded(c_in) / 8) * c_out;
   if (total == 0) return WCN_OK;
   const unsigned grid = (unsigned)((total + 255) / 256);
 #define WCN_PACK_CASE(SD, TS, DD, TD)                                                                                    \
@@ -1117,7 +1123,7 @@ int wcn_conv_tcgen05_fwd(const void* feats, int64_t num_in, int64_t feats_ld, co
     return WCN_ERR_INVALID_PARAMETERS;
   ConvTcParams p = {};
   p.feats = (const char*)feats; p.wpacked = (const char*)packed; p.nbr = nbr; p.out_rows = out_rows;
-  p.M = M; p.num_in = num_in; p.K = K; p.c_in = c_in; p.c_out = c_out;
+  p.M = M; p.num_in = num_in; p.K = K; p.c_in = padded(c_in); p.row_bytes = c_in * 2; p.c_out = c_out;
   p.in_ld_bytes = feats_ld * 2; p.out_ld = out_ld; p.res_ld = residual_ld;
   p.scale = scale; p.shift = shift; p.residual = residual; p.relu = relu; p.out = out;
   p.dev_status = dev_status;

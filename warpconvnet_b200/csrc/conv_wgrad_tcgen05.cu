@@ -87,8 +87,8 @@ conv_wgrad_tcgen05_kernel(const WgradParams p) {
   extern __shared__ uint8_t smem_raw[];
 
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  const int UA = p.c_in / CWA;              // units per offset
-  const int NB = p.c_out / (RBB / 2);       // dY channel chunks
+  const int UA = (p.c_in + CWA - 1) / CWA;               // units per offset
+  const int NB = (p.c_out + RBB / 2 - 1) / (RBB / 2);    // dY channel chunks (N = c_out: what lies beyond is not read)
   const int total_units = p.K * UA;
   const int group0 = blockIdx.y * p.groups;
   const int ng = min(p.groups, (total_units + GU - 1) / GU - group0);
@@ -218,10 +218,12 @@ conv_wgrad_tcgen05_kernel(const WgradParams p) {
         const bool over = cur.idx[u] >= num_in;   // names no feature row: counts as absent
         bad |= over;
         const int mine_row = over ? -1 : cur.idx[u];
+        const bool valid = ctl->unit_at[cur.group * GU + u] + chunk * 16 < p.c_in * 2;   // (the last slice may be narrower)
 #pragma unroll
         for (int j = 0; j < NJ; ++j) {
           const int r = __shfl_sync(0xFFFFFFFFu, mine_row, j * RPI + sub_row);
-          cp_async16(dst + u * A_TILE + aoff[j], r >= 0 ? from + r * ld : p.feats, r >= 0 ? 16u : 0u);
+          const bool have = r >= 0 && valid;
+          cp_async16(dst + u * A_TILE + aoff[j], have ? from + r * ld : p.feats, have ? 16u : 0u);
         }
       }
       cp_async_arrive(bar(&ctl->full[slot]));
@@ -240,7 +242,7 @@ conv_wgrad_tcgen05_kernel(const WgradParams p) {
       for (int g = warp >> 2; g < ng; g += 2) {
         if (!((ctl->started >> g) & 1u)) continue;
         const int unit = (group0 + g) * GU + row / CWA;
-        const bool live = unit < total_units;
+        const bool live = unit < total_units && (unit % UA) * CWA + row % CWA < p.c_in;
         float* dst = p.gw + ((int64_t)(unit / UA) * p.c_in + (unit % UA) * CWA + row % CWA) * p.c_out;
         const uint32_t trow = tmem_base + ((uint32_t)((warp & 3) * 32) << 16) + (uint32_t)(g * p.cols);
         for (int c0 = 0; c0 < p.c_out; c0 += 16) {
@@ -305,7 +307,7 @@ conv_wgrad_tcgen05_kernel(const WgradParams p) {
 template <int RBA, int RBB, bool BF16>
 int launch_wgrad(WgradParams& p, cudaStream_t st) {
   constexpr int CWA = RBA / 2, GU = 128 / CWA;
-  const int UA = p.c_in / CWA, NB = p.c_out / (RBB / 2);
+  const int UA = (p.c_in + CWA - 1) / CWA, NB = (p.c_out + RBB / 2 - 1) / (RBB / 2);
   const int groups = (p.K * UA + GU - 1) / GU;
   const size_t a_stage = (size_t)GU * WG_ROWS * RBA, b_stage = (size_t)NB * WG_ROWS * RBB;
   const size_t limit = 226 * 1024, fixed = 1024 + sizeof(WgradControl) + 128;
@@ -350,8 +352,8 @@ int launch_wgrad(WgradParams& p, cudaStream_t st) {
 }  // namespace
 
 bool wcn_conv_wgrad_tcgen05_supported(int K, int c_in, int c_out, int dtype) {
-  return (dtype == WCN_F16 || dtype == WCN_BF16) && K >= 1 && c_in >= 32 && c_in % 32 == 0 && c_out >= 32 &&
-         c_out % 32 == 0 && c_out <= 256 && (int64_t)K * c_in <= 65535ll * 32;
+  return (dtype == WCN_F16 || dtype == WCN_BF16) && K >= 1 && c_in >= 16 && c_in % 8 == 0 && c_out >= 16 &&
+         c_out % 16 == 0 && c_out <= 256 && (int64_t)K * c_in <= 65535ll * 32;
 }
 
 int wcn_conv_wgrad_tcgen05(const void* feats, int64_t num_in, const void* grad_out, const int32_t* nbr,

@@ -311,6 +311,7 @@ constexpr int PYR_THREADS = 256;
 constexpr int PYR_SHIFTS = 6;   // cells of 2, 4, .., 64 voxels are counted
 
 struct PyramidParams {
+  int groups, per_block;   // groups of PYR_THREADS rows, and how many of them a block of the second kernel takes
   const int4* rows;         // [n] sorted
   const int32_t* info;      // of the sort: corner, ...
   int64_t n;
@@ -351,55 +352,66 @@ pyramid_count_kernel(const PyramidParams p) {
   if (i < p.n && d == 0) p.counts[7] = 1;  // equal to the row before
 }
 
+// Every block adds up the counts of all groups of rows before its own, so large sets give a block several groups
+// (`per_block`): 1.2 M rows, a group each: 64 us, four: 41, sixteen: MEASURED us.
 __global__ void __launch_bounds__(PYR_THREADS)
 pyramid_emit_kernel(const PyramidParams p) {
+  constexpr int WARPS = PYR_THREADS / 32, PARTS = WARPS / PYR_SHIFTS > 0 ? WARPS / PYR_SHIFTS : 1;
   __shared__ int32_t before_s[PYR_SHIFTS], all_s[PYR_SHIFTS];
-  __shared__ int32_t warp_c[PYR_SHIFTS][PYR_THREADS / 32];
+  __shared__ int32_t warp_c[PYR_SHIFTS][WARPS];
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  const int64_t i = (int64_t)blockIdx.x * PYR_THREADS + tid;
   const int ox = __ldg(&p.info[0]), oy = __ldg(&p.info[1]), oz = __ldg(&p.info[2]);
+  const int group0 = (int)blockIdx.x * p.per_block;
   if (tid < PYR_SHIFTS) before_s[tid] = all_s[tid] = 0;
   __syncthreads();
-  for (int s = warp; s < PYR_SHIFTS; s += PYR_THREADS / 32) {
+  for (int w = warp; w < PYR_SHIFTS * PARTS; w += WARPS) {
+    const int s = w / PARTS, part = w % PARTS;
     int before = 0, all = 0;
 #pragma unroll 4
-    for (int b = lane; b < (int)gridDim.x; b += 32) {
-      const int v = __ldg(&p.block_counts[s * gridDim.x + b]);
+    for (int b = part * 32 + lane; b < p.groups; b += 32 * PARTS) {
+      const int v = __ldg(&p.block_counts[s * p.groups + b]);
       all += v;
-      if (b < (int)blockIdx.x) before += v;
+      if (b < group0) before += v;
     }
     before = __reduce_add_sync(0xFFFFFFFFu, before);
     all = __reduce_add_sync(0xFFFFFFFFu, all);
-    if (lane == 0) { before_s[s] = before; all_s[s] = all; }
+    if (lane == 0) { atomicAdd(&before_s[s], before); atomicAdd(&all_s[s], all); }
   }
-  int4 row = make_int4(0, 0, 0, 0);
-  const bool live = i < p.n;
-  const uint32_t d = live ? step_bits(p, i, ox, oy, oz, &row) : 0u;
-  uint32_t heads[PYR_SHIFTS];
+  for (int q = 0; q < p.per_block && group0 + q < p.groups; ++q) {
+    const int64_t i = (int64_t)(group0 + q) * PYR_THREADS + tid;
+    int4 row = make_int4(0, 0, 0, 0);
+    const bool live = i < p.n;
+    const uint32_t d = live ? step_bits(p, i, ox, oy, oz, &row) : 0u;
+    uint32_t heads[PYR_SHIFTS];
 #pragma unroll
-  for (int s = 0; s < PYR_SHIFTS; ++s) {
-    heads[s] = __ballot_sync(0xFFFFFFFFu, (d >> (s + 1)) != 0);
-    if (lane == 0) warp_c[s][warp] = __popc(heads[s]);
-  }
-  __syncthreads();
-  int rank_below = (int)i;
+    for (int s = 0; s < PYR_SHIFTS; ++s) {
+      heads[s] = __ballot_sync(0xFFFFFFFFu, (d >> (s + 1)) != 0);
+      if (lane == 0) warp_c[s][warp] = __popc(heads[s]);
+    }
+    __syncthreads();
+    int rank_below = (int)i;
 #pragma unroll
-  for (int l = 0; l < 4; ++l) {
-    if (l >= p.levels) break;
-    int rank = before_s[l] + __popc(heads[l] & ((1u << lane) - 1u));
-    for (int w = 0; w < warp; ++w) rank += warp_c[l][w];
-    if (live && ((d >> (l + 1)) != 0)) {
-      const int s = l + 1;
-      p.out[l][rank] = make_int4(row.x, row.y >> s, row.z >> s, row.w >> s);
-      p.first[l][rank] = rank_below;
-      rank_below = rank;
+    for (int l = 0; l < 4; ++l) {
+      if (l >= p.levels) break;
+      int rank = before_s[l] + __popc(heads[l] & ((1u << lane) - 1u));
+      for (int w = 0; w < warp; ++w) rank += warp_c[l][w];
+      if (live && ((d >> (l + 1)) != 0)) {
+        const int s = l + 1;
+        p.out[l][rank] = make_int4(row.x, row.y >> s, row.z >> s, row.w >> s);
+        p.first[l][rank] = rank_below;
+        rank_below = rank;
+      }
+      if (live) {  // batch items start where their first row does (an empty one where the next does)
+        const bool start = i == 0 || d == 0xFFFFFFFFu;
+        if (start)
+          for (int b = 0; b <= p.batches; ++b)
+            if (p.offsets[b] == (int32_t)i) p.host[(int64_t)l * (p.batches + 1) + b] = rank;
+      }
     }
-    if (live) {  // batch items start where their first row does (an empty one where the next does)
-      const bool start = i == 0 || d == 0xFFFFFFFFu;
-      if (start)
-        for (int b = 0; b <= p.batches; ++b)
-          if (p.offsets[b] == (int32_t)i) p.host[(int64_t)l * (p.batches + 1) + b] = rank;
-    }
+    __syncthreads();
+    if (tid < PYR_SHIFTS)
+      for (int w = 0; w < WARPS; ++w) before_s[tid] += warp_c[tid][w];
+    __syncthreads();
   }
   if (blockIdx.x == 0 && tid == 0) {
     p.counts[0] = (int32_t)p.n;
@@ -491,7 +503,9 @@ extern "C" int wcn_pyramid(const int32_t* rows, int64_t n, const int32_t* info, 
   if (cudaMemsetAsync(counts, 0, 8 * sizeof(int32_t), st) != cudaSuccess) return WCN_ERR_EXECUTION;
   const unsigned blocks = (unsigned)((n + PYR_THREADS - 1) / PYR_THREADS);
   pyramid_count_kernel<<<blocks, PYR_THREADS, 0, st>>>(p);
-  pyramid_emit_kernel<<<blocks, PYR_THREADS, 0, st>>>(p);
+  p.groups = (int)blocks;
+  p.per_block = blocks <= 592 ? 1 : (int)((blocks + 295) / 296);   // two blocks a multiprocessor
+  pyramid_emit_kernel<<<(blocks + p.per_block - 1) / p.per_block, PYR_THREADS, 0, st>>>(p);
   WCN_CHECK_LAUNCH();
   return WCN_OK;
 }

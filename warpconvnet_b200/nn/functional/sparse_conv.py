@@ -212,6 +212,11 @@ TILE_ORDER_MIN_ROWS = 1024
 TILE_ORDER_MIN_OFFSETS = 9
 
 
+def _aligned(t: Tensor) -> bool:
+    """Whether the rows of ``t`` start on 16-byte boundaries."""
+    return t.data_ptr() % 16 == 0 and t.stride(0) * t.element_size() % 16 == 0
+
+
 def _row_view(t: Tensor) -> Tensor:
     """``t`` as a matrix whose rows are contiguous (any row stride), copying only if they are not."""
     return t if t.dim() == 2 and t.stride(1) == 1 and t.stride(0) >= t.shape[1] else t.contiguous()
@@ -247,6 +252,9 @@ def sparse_conv_fused(in_features: Tensor, weight: Tensor, kernel_map: IntSearch
                                           ep0, out_dtype, transpose_weight)
         if done is not None:
             return done
+    if algo == CONV_AUTO and x.shape[1] % 32 and x.dtype != torch.float32 and x.shape[0] > 0 \
+            and not all(_aligned(t) for t in (x, epilogue and epilogue.out, epilogue and epilogue.residual) if t is not None):
+        algo = CONV_SIMT  # the tensor-core kernel takes these widths, but not rows at any address
     w, packed = _prepared_weight(weight, x.dtype, algo, transpose_weight, reverse_weight)
     if w is None and x.shape[0] == 0:  # no row to multiply: the kernel for that case reads plain weights
         w = _cast_weight(weight, x.dtype, transpose_weight, reverse_weight)
@@ -764,7 +772,7 @@ def _cached_bricks(voxels: Optional[Voxels], coords: Tensor):
 def sparse_conv_wgrad(in_features: Tensor, grad_output: Tensor, kernel_map: IntSearchResult,
                       num_out_coords: int, tile_order: bool = False) -> Optional[Tensor]:
     """``dW[k] = X[in_k]^T @ dY[out_k]`` for every kernel offset, fp32 result ``[K, C_in, C_out]``: one launch on the
-    tensor cores for fp16 / bf16 widths that are multiples of 32 (output width at most 256), the pair kernel on the FP32
+    tensor cores for fp16 / bf16 widths of 16 and more that are multiples of 8 (input) and 16 (output, at most 256), the pair kernel on the FP32
     pipes for fp32 and all other widths.  None when the operands are in no native dtype (the caller then uses a
     GEMM per offset)."""
     require_cuda(in_features, "in_features")
@@ -778,7 +786,7 @@ def sparse_conv_wgrad(in_features: Tensor, grad_output: Tensor, kernel_map: IntS
         nbr, out_rows = kernel_map.tiled_neighbor_table(num_out_coords)
     else:
         nbr, out_rows = kernel_map.neighbor_table(num_out_coords), None
-    if x.dtype == torch.float32 or c_in % 32 or c_out % 32 or c_out > 256 or K > 32:
+    if x.dtype == torch.float32 or c_in < 16 or c_in % 8 or c_out % 16 or c_out > 256 or K > 32:
         gw = torch.empty((K, c_in, c_out), dtype=torch.float32, device=dev)
         nbytes = query_bytes("wcn_conv_wgrad_pairs_workspace_bytes", num_out_coords, K, c_in, c_out)
         ws = torch.empty(nbytes, dtype=torch.uint8, device=dev) if nbytes else None
@@ -786,6 +794,7 @@ def sparse_conv_wgrad(in_features: Tensor, grad_output: Tensor, kernel_map: IntS
                                          c_out, dtype_code(x.dtype), ptr(gw), ptr(ws), nbytes, ptr(device_status(dev)),
                                          stream_ptr(dev)), "wcn_conv_wgrad_pairs")
         return gw
+    x, g = (t if t.data_ptr() % 16 == 0 else t.clone() for t in (x, g))
     masks = kernel_map.tile_masks(num_out_coords, tiled) if K > 1 else None  # steps without neighbours are skipped
     gw = torch.zeros((K, c_in, c_out), dtype=torch.float32, device=dev)
     check(lib().wcn_conv_wgrad(ptr(x), x.shape[0], ptr(g), ptr(nbr), ptr(out_rows), ptr(masks), num_out_coords, K,
@@ -1217,7 +1226,8 @@ def run_layer(layer, x: Voxels, target: Optional[Voxels], epilogue: Optional[Con
         x._extra_attributes["_cache"] = IntSearchCache()  # shared by everything derived from x, as after any convolution
     if tables.one_pair and rec.rows_launch(weight).takes(feats):
         y = rec.rows(feats, tables.dst, m, residual, out)
-    elif tables.nbr is None:
+    elif tables.nbr is None or (weight.shape[1] % 32 and rec.conv.packed is not None
+                                and not all(_aligned(t) for t in (feats, residual, out) if t is not None)):
         return None
     else:
         y = rec.conv(feats, tables.nbr, tables.out_rows, m, residual, out)
@@ -1297,6 +1307,8 @@ def _launch_layer(x: Tensor, weight: Tensor, t: _LayerTables, gradient: bool, ro
     and the offsets in reverse order."""
     if x.stride(1) != 1:
         x = x.contiguous()
+    if not _aligned(x):
+        x = x.clone(memory_format=torch.contiguous_format)
     w, packed = _prepared_weight(weight, x.dtype, CONV_AUTO, gradient, gradient)
     K, c_in, c_out = weight.shape
     if gradient:
