@@ -510,9 +510,12 @@ typedef struct {
 /* 3x3x3 maps in tile order and children tables of up to five levels, a launch per stage for all of them.  The rows must
  * be what wcn_pyramid called usable.  (nbr, order) is a pair for wcn_conv_fwd, child the [8, n] table of the 2x2x2
  * stride-2 convolution and of wcn_conv_rows_fwd on the way back up.
+ * Tables of up to small_window_rows rows are ordered in windows of 4 096 rows, larger ones in windows of 16 384 (which
+ * leave about 7 % fewer (tile, offset) pairs; one keeps a block busy for 25 us, a small one for 9).
  * Replaces generate_kernel_map per layer geometry (warpconvnet/geometry/coords/search/torch_discrete.py:365-466). */
 int wcn_level_brick_bytes(int64_t n, int64_t* bytes);
-int wcn_level_maps(const wcn_level* levels, int32_t num_levels, const int32_t* info, const int32_t* counts, void* stream);
+int wcn_level_maps(const wcn_level* levels, int32_t num_levels, const int32_t* info, const int32_t* counts,
+                   int32_t small_window_rows, void* stream);
 
 /* ------------------------------------------------------------------ a network as one call */
 

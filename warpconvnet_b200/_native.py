@@ -80,7 +80,7 @@ SIGNATURES = {
     "wcn_pyramid_workspace_bytes": [_c_i64, _p_i64],
     "wcn_pyramid": [_c_vp, _c_i64, _c_vp, _c_vp, _c_i32, _c_i32, _c_vp, _c_vp, _c_vp, _c_vp, _c_vp, _c_vp, _c_vp],
     "wcn_level_brick_bytes": [_c_i64, _p_i64],
-    "wcn_level_maps": [_c_vp, _c_i32, _c_vp, _c_vp, _c_vp],
+    "wcn_level_maps": [_c_vp, _c_i32, _c_vp, _c_vp, _c_i32, _c_vp],
     "wcn_net_run": [_c_vp, _c_i32, _c_vp, _c_vp, _c_vp, _c_i32, _c_vp, _c_vp],
     "wcn_selftest_bounded_wait": [_c_i64, _c_vp, _c_vp, _c_vp],
     "wcn_conv_rows_supported": [_c_i32, _c_i32, _c_i32, _c_i32, _c_i32, _c_vp],

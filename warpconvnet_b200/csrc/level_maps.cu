@@ -258,10 +258,6 @@ template <int W> int launch_sort(const LevelsParams& p, int levels, int lo, int 
   return cudaGetLastError() == cudaSuccess ? WCN_OK : WCN_ERR_EXECUTION;
 }
 
-// Tables of up to this many rows are sorted in the small windows: a large one keeps one block busy for 25 us, a small
-// one for 9, and layers over tables this size are bound by latency, not by the 7 % more (tile, offset) pairs.
-constexpr int kSmallWindowRows = 65536;
-
 }  // namespace
 
 extern "C" int wcn_level_brick_bytes(int64_t n, int64_t* bytes) {
@@ -270,8 +266,9 @@ extern "C" int wcn_level_brick_bytes(int64_t n, int64_t* bytes) {
   return WCN_OK;
 }
 
-extern "C" int wcn_level_maps(const wcn_level* levels, int32_t num_levels, const int32_t* info, const int32_t* counts, void* stream) {
-  if (!levels || num_levels < 1 || num_levels > MAX_LEVELS || !info || !counts) return WCN_ERR_INVALID_PARAMETERS;
+extern "C" int wcn_level_maps(const wcn_level* levels, int32_t num_levels, const int32_t* info, const int32_t* counts,
+                              int32_t small_window_rows, void* stream) {
+  if (!levels || num_levels < 1 || num_levels > MAX_LEVELS || !info || !counts || small_window_rows < 0) return WCN_ERR_INVALID_PARAMETERS;
   LevelsParams p = {};
   p.info = info; p.counts = counts;
   int64_t most = 0, small_windows = 0, large_windows = 0;
@@ -290,7 +287,7 @@ extern "C" int wcn_level_maps(const wcn_level* levels, int32_t num_levels, const
     most = q.n > most ? q.n : most;
     if (q.order) {
       tiled = true;
-      if (q.n <= kSmallWindowRows) small_windows = small_windows > (q.n + kTileWindowSmall - 1) / kTileWindowSmall ? small_windows : (q.n + kTileWindowSmall - 1) / kTileWindowSmall;
+      if (q.n <= small_window_rows) small_windows = small_windows > (q.n + kTileWindowSmall - 1) / kTileWindowSmall ? small_windows : (q.n + kTileWindowSmall - 1) / kTileWindowSmall;
       else large_windows = large_windows > (q.n + kTileWindowLarge - 1) / kTileWindowLarge ? large_windows : (q.n + kTileWindowLarge - 1) / kTileWindowLarge;
     }
     children |= q.child != nullptr;
@@ -302,8 +299,8 @@ extern "C" int wcn_level_maps(const wcn_level* levels, int32_t num_levels, const
   if (tiled) {
     level_key_kernel<<<grid, THREADS, 0, st>>>(p);
     int rc = WCN_OK;
-    if (large_windows) rc = launch_sort<kTileWindowLarge>(p, num_levels, kSmallWindowRows + 1, INT_MAX, (int)large_windows, st);
-    if (rc == WCN_OK && small_windows) rc = launch_sort<kTileWindowSmall>(p, num_levels, 0, kSmallWindowRows, (int)small_windows, st);
+    if (large_windows) rc = launch_sort<kTileWindowLarge>(p, num_levels, small_window_rows + 1, INT_MAX, (int)large_windows, st);
+    if (rc == WCN_OK && small_windows) rc = launch_sort<kTileWindowSmall>(p, num_levels, 0, small_window_rows, (int)small_windows, st);
     if (rc != WCN_OK) return rc;
   }
   level_search_kernel<<<grid, THREADS, 0, st>>>(p);

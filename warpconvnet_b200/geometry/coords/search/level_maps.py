@@ -78,20 +78,27 @@ def morton_pyramid(ic: IntCoords) -> bool:
     """Computes and links the stride-2 levels of a natively sorted set; False when it is none (or not usable)."""
     if ic._shared.get("morton_info") is None:
         return False
-    return LevelMaps(ic, begin=False).attach()
+    return LevelMaps(ic, begin=False, small_window_rows=LAYER_SMALL_WINDOW_ROWS).attach()
 
 
 # 3x3x3 tables of at least this many rows are put in tile order.
 TILE_ORDER_ROWS = 1024
+# Tables of up to this many rows are ordered in small windows: for the forward of a network, whose layers over so few rows
+# are bound by latency.  Tables that layers ask for one by one (their gradients use them too) get the large windows: the
+# fp32 layers of a 60 000-row room took 195 us in them and 216 in small ones.
+SMALL_WINDOW_ROWS = 65536
+LAYER_SMALL_WINDOW_ROWS = 4096
 
 
 class LevelMaps:
     """Tables of levels 0..4: the constructor enqueues the pyramid and (``begin``) level 0, :meth:`finish` the other levels - or
     :meth:`attach` leaves this object with the levels' coordinates, whose tables :meth:`ensure` makes as layers ask."""
 
-    def __init__(self, ic: IntCoords, tile_order_rows: int = TILE_ORDER_ROWS, begin: bool = True):
+    def __init__(self, ic: IntCoords, tile_order_rows: int = TILE_ORDER_ROWS, begin: bool = True,
+                 small_window_rows: int = SMALL_WINDOW_ROWS):
         self.build = PyramidBuild(ic)
         self.min_rows = tile_order_rows
+        self.small_window_rows = small_window_rows
         n = self.build.n
         self.n = [n]
         self.rows = [self.build.rows]
@@ -114,8 +121,8 @@ class LevelMaps:
                 child = self.child[l - 1] = torch.empty((8, n), dtype=torch.int32, device=b.device)
                 slot.child, slot.first_child = child.data_ptr(), b.first[l - 1].data_ptr()
                 slot.rows_below, slot.n_below = self.rows[l - 1].data_ptr(), self.n[l - 1]
-        check(lib().wcn_level_maps(ctypes.addressof(levels), len(which), ptr(b.info), ptr(b.counts), stream_ptr(b.device)),
-              "wcn_level_maps")
+        check(lib().wcn_level_maps(ctypes.addressof(levels), len(which), ptr(b.info), ptr(b.counts),
+                                   self.small_window_rows, stream_ptr(b.device)), "wcn_level_maps")
 
     def _levels(self) -> Optional[List[IntCoords]]:
         """The coordinates of levels 1..4, linked (None: not usable)."""

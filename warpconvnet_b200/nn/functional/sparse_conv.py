@@ -33,7 +33,7 @@ from ...geometry.coords.integer import IntCoords
 from ...geometry.coords.ops.serialization import POINT_ORDERING, encode
 from ...geometry.coords.ops.expand import expand_coords
 from ...geometry.coords.ops.stride import stride_coords
-from ...geometry.coords.search.level_maps import LevelMaps, morton_pyramid
+from ...geometry.coords.search.level_maps import LAYER_SMALL_WINDOW_ROWS, LevelMaps, morton_pyramid
 from . import batch_norm
 from ...geometry.coords.search.cache import IntSearchCache, IntSearchCacheKey
 from ...geometry.coords.search.search_results import IntSearchResult
@@ -639,7 +639,7 @@ def _level_map(fine: Voxels, kernel_size, kernel_dilation, stride, coarse_rows: 
     if km is None and window in _LEVEL_WINDOWS:
         if "level_maps" not in shared and shared.get("morton_info") is not None and ("strided", (2, 2, 2)) not in shared \
                 and window[0] == (3, 3, 3) and fine.batched_coordinates.batched_tensor.shape[0] > 0:
-            LevelMaps(fine.batched_coordinates, TILE_ORDER_MIN_ROWS).attach()
+            LevelMaps(fine.batched_coordinates, TILE_ORDER_MIN_ROWS, True, LAYER_SMALL_WINDOW_ROWS).attach()
         if "level_maps" in shared:
             maps, level = shared["level_maps"]
             km = maps.kmap(level, window[0][0])
