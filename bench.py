@@ -291,8 +291,8 @@ def install_conv_profiler(profile):
     orig_launch = F.FusedConvLaunch.__call__
     orig_rows = F.FusedRowsLaunch.__call__
 
-    def rows_launch(self, feats, dst_rows, num_out, residual=None, out=None):
-        res = orig_rows(self, feats, dst_rows, num_out, residual, out)
+    def rows_launch(self, feats, dst_rows, num_out, residual=None, out=None, every_row=True):
+        res = orig_rows(self, feats, dst_rows, num_out, residual, out, every_row)
         profile.calls.append((lambda: orig_rows(self, feats, dst_rows, num_out, residual, res),
                               (num_out, num_out, self.K), self.c_in, self.c_out, "tcgen05"))
         return res

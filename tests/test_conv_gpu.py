@@ -7,7 +7,7 @@ import torch.nn as nn
 
 from oracle import kernel_map as km
 from oracle import sparse_conv as osc
-from warpconvnet_b200 import (SPARSE_CONV_FWD_ALGO_MODE as ALGO, ConvEpilogue, IntSearchResult, Sequential,
+from warpconvnet_b200 import (SPARSE_CONV_BWD_ALGO_MODE as BWD, SPARSE_CONV_FWD_ALGO_MODE as ALGO, ConvEpilogue, IntSearchResult, Sequential,
                               SparseConv3d, Voxels, generate_kernel_map, spatially_sparse_conv, stride_coords)
 from warpconvnet_b200._native import CONV_SIMT, CONV_TCGEN05, check_device_status
 from warpconvnet_b200.datasets import synthetic
@@ -19,6 +19,13 @@ from conftest import rel_l2
 pytestmark = pytest.mark.gpu
 DEV = "cuda:0"
 TOL = {torch.float32: 1e-4, torch.float16: 1e-2, torch.bfloat16: 1e-2}
+
+
+def room_rows(n):
+    """Room voxels about a corner that is no multiple of 2 or 3, in random order: ``[N, 4]`` with batch index 0."""
+    xyz = synthetic.room_scene(n, 0.04, 29, "raster_crop") - 7
+    xyz = xyz[np.random.default_rng(0).permutation(len(xyz))]
+    return np.ascontiguousarray(np.concatenate([np.zeros((len(xyz), 1), np.int32), xyz.astype(np.int32)], 1))
 
 
 def make_voxels(coords_b, feats, **kw):
@@ -528,6 +535,79 @@ def test_backward_native_dx_strided_and_transposed_fp16():
         ref2.index_add_(0, torch.from_numpy(o[s:e]).long(), gu.float()[torch.from_numpy(i[s:e]).long()] @ wt.float()[k].T)
     assert rel_l2(cg.grad.float().cpu().numpy(), ref2.numpy()) < 1e-2
     check_device_status(DEV)
+
+
+def _stale(*shapes):
+    """Leaves NaN in the allocator's free blocks of these fp16 shapes: what an uninitialised result would show."""
+    blocks = [torch.full(s, float("nan"), dtype=torch.float16, device=DEV) for s in shapes for _ in range(3)]
+    torch.cuda.synchronize()
+    del blocks
+
+
+@pytest.mark.parametrize("sort", [False, True])
+@pytest.mark.parametrize("ksize,repeated", [(3, False), (2, True), (2, False)])
+def test_rows_that_no_pair_names_are_not_left_uninitialised(sort, ksize, repeated):
+    """Window = stride layers run from the input side, which writes the rows that the table names.  Repeated voxels
+    (the table holds the smallest row) and the last rows of centred odd windows are in no pair: their input gradient is
+    zero and their transposed output the bias alone."""
+    g = torch.Generator().manual_seed(ksize)
+    coords = room_rows(6000)
+    if repeated:
+        coords = np.concatenate([coords, coords[::7]])
+    n, c_in, c_out = len(coords), 32, 64
+    vox = make_voxels(coords, torch.randn(n, c_in, generator=g).half())
+    vox = vox.sort() if sort else vox
+    xg = vox.feature_tensor.clone().requires_grad_(True)
+    w = (torch.randn(ksize ** 3, c_in, c_out, generator=g) * 0.1).half().to(DEV)
+    wu = (torch.randn(ksize ** 3, c_out, c_in, generator=g) * 0.1).half().to(DEV)
+    bias = torch.randn(c_in, generator=g).half().to(DEV)
+    fine = vox.replace(batched_features=xg)
+    down = spatially_sparse_conv(fine, w, ksize, stride=ksize, fwd_algo=ALGO.IMPLICIT_GEMM, bwd_algo=BWD.IMPLICIT_GEMM)
+    go = torch.randn(down.feature_tensor.shape, generator=g).half().to(DEV)
+    _stale((n, c_in))
+    (gx,) = torch.autograd.grad(down.feature_tensor, [xg], go)
+    _stale((n, c_in))
+    coarse = down.replace(batched_features=down.feature_tensor.detach())
+    with torch.no_grad():
+        up = spatially_sparse_conv(coarse, wu, ksize, stride=ksize, transposed=True, bias=bias,
+                                   output_spatially_sparse_tensor=fine, fwd_algo=ALGO.IMPLICIT_GEMM).feature_tensor
+        layer = SparseConv3d(c_out, c_in, ksize, stride=ksize, transposed=True, bias=True).to(DEV).half()
+        layer.weight.copy_(wu)
+        layer.bias.copy_(bias)
+        _stale((n, c_in))
+        up_layer = layer(coarse, fine).feature_tensor
+    nbr = generate_kernel_map(fine.batch_indexed_coordinates, coarse.batch_indexed_coordinates, (ksize,) * 3,
+                              (ksize,) * 3).neighbor_table(len(coarse))
+    want_gx = torch.zeros(n, c_in, dtype=torch.float64, device=DEV)
+    want_up = bias.double().repeat(n, 1)
+    unnamed = torch.ones(n, dtype=torch.bool, device=DEV)
+    for k in range(ksize ** 3):
+        m = (nbr[k] >= 0).nonzero()[:, 0]
+        rows = nbr[k, m].long()
+        want_gx[rows] += go[m].double() @ w[k].double().T
+        want_up[rows] += coarse.feature_tensor[m].double() @ wu[k].double()
+        unnamed[rows] = False
+    assert bool(unnamed.any()) == (repeated or ksize == 3)
+    for got, want in ((gx, want_gx), (up, want_up), (up_layer, want_up)):
+        assert torch.isfinite(got).all()
+        assert rel_l2(got.double().cpu().numpy(), want.cpu().numpy()) < 2e-3   # fp16 results
+        assert torch.equal(got[unnamed].double(), want[unnamed])
+    check_device_status(DEV)
+
+
+def test_network_over_repeated_voxels_has_no_uninitialised_rows():
+    coords = room_rows(6000)
+    coords = np.concatenate([coords, coords[::7]])
+    torch.manual_seed(0)
+    model = MinkUNet18(3, 20).to(DEV).half().eval()
+    x = torch.rand(len(coords), 3, generator=torch.Generator().manual_seed(1)).half()
+    ys = []
+    for fill in (float("nan"), 0.0):
+        arena = torch.full((64 << 20,), fill, dtype=torch.float16, device=DEV)
+        del arena
+        with torch.no_grad():
+            ys.append(model(make_voxels(coords, x)).feature_tensor)
+    assert torch.isfinite(ys[0]).all() and torch.equal(*ys)
 
 
 def test_surface_errors_and_shortcuts():

@@ -361,7 +361,8 @@ class _LaunchPlan:
             if up_rows.takes(cur):
                 # every fine voxel has one parent (the coarse set is the strided fine set): the parents'
                 # rows are streamed once and each offset's block written at its child
-                up_rows(cur, children[level], n[level], out=left)
+                facts = ics[level]._shared.get("facts", {})   # repeated voxels of the finest level are nobody's child
+                up_rows(cur, children[level], n[level], out=left, every_row=bool(facts.get("distinct") or facts.get("unique")))
             else:
                 up(cur, up_table(level), None, n[level], out=left)
             if tables[level] is None:

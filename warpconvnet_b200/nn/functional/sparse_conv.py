@@ -249,7 +249,7 @@ def sparse_conv_fused(in_features: Tensor, weight: Tensor, kernel_map: IntSearch
                 done = sparse_conv_rows_fused(x, weight, dst, num_out_coords, ep0, out_dtype, transpose_weight)
         elif getattr(kernel_map, "_one_pair", False) and ep0.out_rows is None and kernel_map._forward is not None:
             done = sparse_conv_rows_fused(x, weight, kernel_map._forward.neighbor_table(x.shape[0]), num_out_coords,
-                                          ep0, out_dtype, transpose_weight)
+                                          ep0, out_dtype, transpose_weight, every_row=_names_every_row(kernel_map))
         if done is not None:
             return done
     if algo == CONV_AUTO and x.shape[1] % 32 and x.dtype != torch.float32 and x.shape[0] > 0 \
@@ -398,14 +398,16 @@ def _tma_rows_ok(x: Tensor) -> bool:
 
 def sparse_conv_rows_fused(in_features: Tensor, weight: Tensor, dst_rows: Optional[Tensor], num_out_coords: int,
                            epilogue: Optional[ConvEpilogue] = None,
-                           out_dtype: Optional[torch.dtype] = None, transpose_weight: bool = False) -> Optional[Tensor]:
+                           out_dtype: Optional[torch.dtype] = None, transpose_weight: bool = False,
+                           every_row: bool = True) -> Optional[Tensor]:
     """A convolution in which every output row has exactly one (input row, offset) pair, run from
     the input side (``wcn_conv_rows_fwd``): ``out[dst_rows[k, j]] = epilogue(in_features[j] @ weight[k])``.
     ``dst_rows`` is int32 ``[K, N_in]`` (entries < 0: no such pair) — for a 2x2x2 stride-2 transposed
     convolution the neighbour table of the matching strided convolution — or None for a 1x1x1
     convolution (``K == 1``, output row = input row).  Returns None when the kernel does not take the
     call (dtype, shape or alignment), so the caller can use the output-side kernels.  Output rows
-    that no pair names are left as they were (in a fresh result: uninitialised)."""
+    that no pair names are left as they were (in a fresh result: uninitialised), unless ``every_row`` is
+    False: the caller cannot say that there are none, and they receive the epilogue of a zero."""
     require_cuda(in_features, "in_features")
     x = _row_view(in_features)
     ep = epilogue or ConvEpilogue()
@@ -440,12 +442,40 @@ def sparse_conv_rows_fused(in_features: Tensor, weight: Tensor, dst_rows: Option
         residual = _row_view(residual)
         assert tuple(residual.shape) == (num_out_coords, c_out)
     scale, shift = _as_f32_on(ep.scale, dev), _as_f32_on(ep.shift, dev)
+    if not every_row:
+        _fill_unnamed_rows(out[:num_out_coords], shift, residual, ep.relu)
     check(lib().wcn_conv_rows_fwd(ptr(x), x.shape[0], x.stride(0), ptr(packed), ptr(dst_rows), num_out_coords, K,
                                   c_in, c_pack, c_out, dtype_code(x.dtype), ptr(scale), ptr(shift), ptr(residual),
                                   residual.stride(0) if residual is not None else 0, int(ep.relu), ptr(out),
                                   out.stride(0), dtype_code(out_dtype), ptr(device_status(dev)), stream_ptr(dev)),
           "wcn_conv_rows_fwd")
     return out
+
+
+def _fill_unnamed_rows(out: Tensor, shift: Optional[Tensor], residual: Optional[Tensor], relu) -> None:
+    """The epilogue of a zero in every row of ``out``, in the kernel's steps: rows that the input-side kernel does not
+    write are then what the output-side kernels make of a row without neighbours."""
+    if shift is None and residual is None:
+        out.zero_()
+        return
+    y = shift if residual is None else residual.float() if shift is None else residual.float() + shift
+    out.copy_(y.clamp(min=0) if relu else y)
+
+
+def _names_every_row(kernel_map: IntSearchResult) -> bool:
+    """Whether the (input row, offset) pairs of a map whose window is its stride name every row of the finer side: the
+    finer rows are known to be distinct (a table holds one row per voxel, so a repeated one is in no pair) and the
+    windows start at the multiples of the stride (odd ones are centred: 3p + 2 belongs to the window of p + 1, which
+    need not be there)."""
+    facts = getattr(kernel_map, "_finer_rows", None)
+    return facts is not None and bool(facts.get("distinct") or facts.get("unique"))
+
+
+def _finer_rows(fine: IntCoords, kernel_size) -> Optional[dict]:
+    """What :func:`_names_every_row` looks at (the facts may become known after the map was made)."""
+    if any(int(k) % 2 and int(k) != 1 for k in kernel_size):
+        return None
+    return fine._shared.setdefault("facts", {})
 
 
 class FusedRowsLaunch:
@@ -476,11 +506,13 @@ class FusedRowsLaunch:
         return self.usable and _tma_rows_ok(feats)
 
     def __call__(self, feats: Tensor, dst_rows: Optional[Tensor], num_out: int, residual: Optional[Tensor] = None,
-                 out: Optional[Tensor] = None) -> Tensor:
+                 out: Optional[Tensor] = None, every_row: bool = True) -> Tensor:
         if out is None:
             out = torch.empty((num_out, self.c_out), dtype=self.dtype, device=self.device)
         if num_out == 0 or feats.shape[0] == 0:
             return out
+        if not every_row:  # see sparse_conv_rows_fused
+            _fill_unnamed_rows(out[:num_out], self.shift, residual, self.relu)
         rc = self._fn(feats.data_ptr(), feats.shape[0], feats.stride(0), self._packed_ptr,
                       dst_rows.data_ptr() if dst_rows is not None else None, num_out, self.K, self.c_in, self.c_pack,
                       self.c_out, self._dc, self._scale_ptr, self._shift_ptr,
@@ -605,6 +637,8 @@ def generate_output_coords_and_kernel_map(input_sparse_tensor: Voxels, kernel_si
         kernel_map._one_pair = (tuple(kernel_size) == tuple(stride) and all(int(d) == 1 for d in kernel_dilation)
                                 and parent is not None
                                 and parent._shared is input_sparse_tensor.batched_coordinates._shared)
+        if kernel_map._one_pair:
+            kernel_map._finer_rows = _finer_rows(fine, kernel_size)
     else:
         kernel_map = _level_map(input_sparse_tensor, kernel_size, kernel_dilation, stride, out_coords)
         if kernel_map is None:
@@ -618,6 +652,8 @@ def generate_output_coords_and_kernel_map(input_sparse_tensor: Voxels, kernel_si
                 kernel_map._facts = input_sparse_tensor.batched_coordinates._shared.setdefault("facts", {})
             else:
                 kernel_map._one_parent = tuple(kernel_size) == tuple(stride) and all(int(d) == 1 for d in kernel_dilation)
+                if kernel_map._one_parent:
+                    kernel_map._finer_rows = _finer_rows(input_sparse_tensor.batched_coordinates, kernel_size)
     if input_sparse_tensor.cache is None:
         input_sparse_tensor._extra_attributes["_cache"] = IntSearchCache()
     input_sparse_tensor.cache.put(key, kernel_map)
@@ -672,6 +708,7 @@ def strided_coordinates(coords: IntCoords, stride: Tuple[int, ...]) -> IntCoords
             out_coords, out_offsets = stride_coords(bc, stride, in_offsets=coords.offsets)
         hit = IntCoords(out_coords[:, 1:], offsets=out_offsets)
         hit._bcoords = out_coords
+        hit._shared["facts"] = {"unique": True}
         origin = coords.morton_origin
         if origin is not None and bc.shape[1] == 4:
             # First occurrences of floor(c / s) in Morton order are themselves in Morton order about
@@ -740,6 +777,7 @@ def _pyramid_in_one_sync(level: IntCoords, steps) -> None:
     for s, total, (rows, offsets) in zip(steps, totals, results):
         hit = IntCoords(rows[:, 1:], offsets=offsets)
         hit._bcoords = rows
+        hit._shared["facts"] = {"unique": True}
         if origin is not None:
             t = total[0] if len(set(total)) == 1 else torch.tensor(total, dtype=torch.int32, device=origin.device)
             hit.morton_origin = torch.div(origin, t, rounding_mode="floor").to(torch.int32)
@@ -816,7 +854,7 @@ def _input_gradient(grad_output: Tensor, weight: Tensor, kernel_map: IntSearchRe
         return sparse_conv_fused(grad_output, weight, kernel_map, num_in, transpose_weight=True, reverse_weight=True)
     if getattr(kernel_map, "_one_parent", False):
         done = sparse_conv_rows_fused(grad_output, weight, kernel_map.neighbor_table(grad_output.shape[0]), num_in,
-                                      transpose_weight=True)
+                                      transpose_weight=True, every_row=_names_every_row(kernel_map))
         if done is not None:
             return done
     return sparse_conv_fused(grad_output, weight, kernel_map.swapped(num_in=num_in), num_in, transpose_weight=True)
@@ -1225,7 +1263,7 @@ def run_layer(layer, x: Voxels, target: Optional[Voxels], epilogue: Optional[Con
     if x._extra_attributes.get("_cache") is None:
         x._extra_attributes["_cache"] = IntSearchCache()  # shared by everything derived from x, as after any convolution
     if tables.one_pair and rec.rows_launch(weight).takes(feats):
-        y = rec.rows(feats, tables.dst, m, residual, out)
+        y = rec.rows(feats, tables.dst, m, residual, out, every_row=tables.dst is None or _names_every_row(tables.km))
     elif tables.nbr is None or (weight.shape[1] % 32 and rec.conv.packed is not None
                                 and not all(_aligned(t) for t in (feats, residual, out) if t is not None)):
         return None
