@@ -610,6 +610,28 @@ def test_network_over_repeated_voxels_has_no_uninitialised_rows():
     assert torch.isfinite(ys[0]).all() and torch.equal(*ys)
 
 
+@pytest.mark.parametrize("dtype", [torch.float32, torch.float16])
+def test_layers_run_under_inference_mode(dtype):
+    """The vectors an eval-mode BatchNorm is folded to inside ``torch.inference_mode`` have no version counter."""
+    from warpconvnet_b200.examples.mink_unet import BasicBlock
+    coords = room_rows(2000)
+    x = torch.randn(len(coords), 32, generator=torch.Generator().manual_seed(0)).to(dtype)
+    for make in (lambda: Sequential(SparseConv3d(32, 32, 3, bias=True), nn.BatchNorm1d(32), nn.ReLU()), lambda: BasicBlock(32, 64)):
+        torch.manual_seed(0)
+        m = make().to(DEV)
+        randomize_batchnorm_(m, 1)
+        m = m.to(dtype).eval()
+        vox = make_voxels(coords, x)
+        with torch.inference_mode():
+            first = [m(vox).feature_tensor.clone() for _ in range(2)]
+        with torch.no_grad():
+            m(vox)
+            for mod in m.modules():
+                mod.__dict__.pop("_wcn_folded", None)
+            want = m(vox).feature_tensor
+        assert torch.equal(first[0], want) and torch.equal(first[1], want)
+
+
 def test_surface_errors_and_shortcuts():
     n = 2000
     coords, x, w = _layer_case(n, 8, 12, 5, "sample")

@@ -1109,6 +1109,12 @@ def spatially_sparse_conv(
 # coordinate set (where the coordinate set's other derived data lives).
 
 
+def _version_of(t: Optional[Tensor]) -> int:
+    """The version counter of ``t``; tensors made under ``torch.inference_mode`` have none (nor can they be written
+    outside of it), such as the vectors a BatchNorm is folded to there."""
+    return 0 if t is None or t.is_inference() else t._version
+
+
 class _LayerRecord:
     """The launch records of one (weight, bias, epilogue vectors, dtype), current while none of them is written.
     (It is kept with the weight tensor, so it holds none itself.)"""
@@ -1119,7 +1125,7 @@ class _LayerRecord:
         ep = _merge_bias(ConvEpilogue(scale=scale, shift=shift), bias)
         self.w_version, self.w_ptr = weight._version, weight.data_ptr()
         self.vectors = (bias, scale, shift)
-        self.versions = tuple(t._version if t is not None else 0 for t in self.vectors)
+        self.versions = tuple(map(_version_of, self.vectors))
         self.conv = FusedConvLaunch(weight, dtype, ep.scale, ep.shift, relu=relu)
         self.rows = None  # FusedRowsLaunch, made by the first layer call that can use one
 
@@ -1127,8 +1133,8 @@ class _LayerRecord:
         b, sc, sh = self.vectors
         v = self.versions
         return (b is bias and sc is scale and sh is shift and weight._version == self.w_version
-                and weight.data_ptr() == self.w_ptr and (b is None or b._version == v[0])
-                and (sc is None or sc._version == v[1]) and (sh is None or sh._version == v[2]))
+                and weight.data_ptr() == self.w_ptr and _version_of(b) == v[0] and _version_of(sc) == v[1]
+                and _version_of(sh) == v[2])
 
     def rows_launch(self, weight) -> "FusedRowsLaunch":
         if self.rows is None:
