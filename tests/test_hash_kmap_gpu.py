@@ -455,3 +455,28 @@ def test_stride_coords_counts_more_batch_items_than_are_tallied():
     want, _ = km.stride_coords(c, (2, 2, 2))
     assert np.array_equal(rows.cpu().numpy(), want)
     assert offsets.tolist() == [0] + np.cumsum(np.bincount(want[:, 0])).tolist()
+
+
+@pytest.mark.parametrize("what", ["map", "pyramid"])
+def test_results_on_their_way_to_the_host_keep_their_memory(what):
+    """A map (or a pyramid) dropped while the kernel that writes its sizes is still queued: the next small pinned
+    allocation must not be the memory that kernel writes."""
+    from warpconvnet_b200 import Voxels
+    from warpconvnet_b200.geometry.coords.search.level_maps import PYRAMID_LEVELS, PyramidBuild
+    xyz = torch.from_numpy(synthetic.room_scene(3000, 0.04, 3, "raster_crop")).to(DEV)
+    n = len(xyz)
+    coords = torch.cat([torch.zeros((n, 1), dtype=torch.int32, device=DEV), xyz], 1).contiguous()
+    ic = Voxels(xyz, torch.zeros(n, 1, device=DEV), offsets=torch.tensor([0, n])).sort().batched_coordinates
+    words, dtype = (29, torch.int32) if what == "map" else (2 * PYRAMID_LEVELS + 2, torch.int64)
+    for warm in (True, False):  # (the first pass leaves the allocator's blocks behind)
+        torch.cuda.synchronize()
+        if not warm:
+            torch.cuda._sleep(50_000_000)  # some 25 ms in front of the kernels
+        if what == "map":
+            generate_kernel_map(coords, coords, (1, 1, 1), (3, 3, 3)).neighbor_table(n)
+        else:
+            PyramidBuild(ic)
+        mine = [torch.full((words,), 7, dtype=dtype, pin_memory=True) for _ in range(8)]
+        torch.cuda.synchronize()
+        assert all(bool((t == 7).all()) for t in mine)
+    check_device_status(torch.device(DEV))

@@ -10,6 +10,7 @@ import ctypes
 import functools
 import importlib.util
 import os
+import threading
 from collections import Counter
 from typing import Optional
 
@@ -242,6 +243,27 @@ def check_device_status(device: torch.device) -> None:
     host.copy_(word, non_blocking=True)
     torch.cuda.current_stream(device).synchronize()
     raise_for_status(int(host[0]), device)
+
+
+_written: list = []   # (event, pinned tensor): results of kernels that may still be running
+_written_lock = threading.Lock()
+
+
+def pinned_result(words: int, dtype: torch.dtype, device: torch.device, launch):
+    """(pinned tensor of ``words``, event after the kernels that write it): ``launch(tensor)`` enqueues those on the
+    current stream.  Torch's pinned allocator knows of copies, not of kernels, and would hand the memory to the next
+    caller as soon as the tensor is dropped; so it is kept here until the event has passed, whether or not the caller
+    waits for it.  (Not inside a stream capture: a graph's kernels write at every replay.)"""
+    host = torch.empty(words, dtype=dtype, pin_memory=True)
+    done = torch.cuda.Event()
+    try:
+        launch(host)
+    finally:
+        done.record(torch.cuda.current_stream(device))
+        with _written_lock:
+            _written[:] = [w for w in _written if not w[0].query()]
+            _written.append((done, host))
+    return host, done
 
 
 @functools.lru_cache(maxsize=1024)

@@ -14,7 +14,7 @@ from typing import List, Optional
 import torch
 from torch import Tensor
 
-from ...._native import Level, check, device_status, lib, ptr, query_bytes, raise_for_status, stream_ptr
+from ...._native import Level, check, device_status, lib, pinned_result, ptr, query_bytes, raise_for_status, stream_ptr
 from ..integer import IntCoords
 from .search_results import IntSearchResult
 
@@ -35,13 +35,13 @@ class PyramidBuild:
         self.out = torch.empty((PYRAMID_LEVELS, n, 4), dtype=torch.int32, device=dev)
         self.first = torch.empty((PYRAMID_LEVELS, n), dtype=torch.int32, device=dev)
         self.counts = torch.empty(24, dtype=torch.int32, device=dev)
-        self.host = torch.empty(PYRAMID_LEVELS * (self.batches + 1) + 2, dtype=torch.int64, pin_memory=True)
         ws = torch.empty(query_bytes("wcn_pyramid_workspace_bytes", n), dtype=torch.uint8, device=dev)
-        check(lib().wcn_pyramid(ptr(rows), n, ptr(info), ptr(offsets), self.batches, PYRAMID_LEVELS, ptr(self.out),
-                                ptr(self.first), ptr(self.counts), ptr(self.host), ptr(ws), ptr(device_status(dev)),
-                                stream_ptr(dev)), "wcn_pyramid")
-        self._done = torch.cuda.Event()
-        self._done.record(torch.cuda.current_stream(dev))
+
+        def launch(host: Tensor) -> None:
+            check(lib().wcn_pyramid(ptr(rows), n, ptr(info), ptr(offsets), self.batches, PYRAMID_LEVELS, ptr(self.out),
+                                    ptr(self.first), ptr(self.counts), ptr(host), ptr(ws), ptr(device_status(dev)),
+                                    stream_ptr(dev)), "wcn_pyramid")
+        self.host, self._done = pinned_result(PYRAMID_LEVELS * (self.batches + 1) + 2, torch.int64, dev, launch)
 
     def finish(self) -> Optional[List[IntCoords]]:
         """Waits for the counts; the levels' coordinates, or None when the rows are not what the pyramid needs

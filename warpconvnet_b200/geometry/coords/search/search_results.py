@@ -18,7 +18,7 @@ from typing import List, Literal, Optional, Tuple
 import torch
 from torch import Tensor
 
-from ...._native import check, check_device_status, device_status, lib, ptr, query_bytes, raise_for_status, small_to_device, stream_ptr
+from ...._native import check, check_device_status, device_status, lib, pinned_result, ptr, query_bytes, raise_for_status, small_to_device, stream_ptr
 
 
 class IntSearchResult:
@@ -70,12 +70,11 @@ class IntSearchResult:
         nbr, K, M = self._nbr, self._num_offsets, self._num_out
         dev = nbr.device
         offsets = torch.empty(K + 1, dtype=torch.int32, device=dev)
-        host = torch.empty(K + 2, dtype=torch.int32, pin_memory=True)
-        check(lib().wcn_kmap_scan_host(ptr(self._workspace), M, K, ptr(offsets), ptr(host), ptr(device_status(dev)),
-                                       stream_ptr(dev)), "wcn_kmap_scan_host")
-        done = torch.cuda.Event()
-        done.record(torch.cuda.current_stream(dev))
-        self._scanned = (offsets, host, done)
+
+        def scan(host: Tensor) -> None:
+            check(lib().wcn_kmap_scan_host(ptr(self._workspace), M, K, ptr(offsets), ptr(host), ptr(device_status(dev)),
+                                           stream_ptr(dev)), "wcn_kmap_scan_host")
+        self._scanned = (offsets, *pinned_result(K + 2, torch.int32, dev, scan))
 
     def _plain(self) -> Tensor:
         """The plain neighbour table of a map made dense."""

@@ -131,7 +131,7 @@ def _kernel_map_from_cells(in_coords: Tensor, out_coords: Tensor, stride, kernel
     check(lib().wcn_kmap_search_cells(ptr(table), n, ptr(q), M, ctypes.addressof(strd), ctypes.addressof(ksz), ptr(nbr),
                                       ptr(ws), st), "wcn_kmap_search_cells")
     out = IntSearchResult.from_neighbor_table(nbr, n, ws, identity_map_index)
-    if count_hits:
+    if count_hits and not torch.cuda.is_current_stream_capturing():  # (nothing can wait for the sizes inside a capture)
         out.begin_compact()
     return out
 
