@@ -103,3 +103,25 @@ def test_convolution_and_norm_as_one_function(stride, residual, relu):
         results.append([y.detach(), seq[1].running_mean.clone(), seq[1].running_var.clone(), *grads])
     for a, b in zip(*results):
         assert a.dtype == b.dtype and float((a - b).norm()) <= 1e-5 * max(1.0, float(b.norm()))
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.float16])
+def test_gradients_and_saved_tensors_at_any_address(dtype):
+    """A gradient that is a view at an odd element of a flat buffer, and saved tensors that a hook returns as such views."""
+    n, c = 300, 16
+    g = torch.Generator().manual_seed(0)
+    x0, r0, dy = (torch.randn(n, c, generator=g).to(dtype).to(DEV) for _ in range(3))
+
+    def odd(t):
+        return torch.cat([t.new_zeros(1), t.flatten()])[1:].view(t.shape)
+
+    def grads(gradient, hooks):
+        bn = nn.BatchNorm1d(c).to(DEV)
+        x, r = x0.clone().requires_grad_(True), r0.clone().requires_grad_(True)
+        with torch.autograd.graph.saved_tensors_hooks(lambda t: t, odd if hooks else lambda t: t):
+            y = batch_norm_act(x, bn, True, r)
+            return torch.autograd.grad(y, [x, r, bn.weight, bn.bias], gradient)
+    want = grads(dy, False)
+    assert odd(dy).data_ptr() % 16
+    for gradient, hooks in ((odd(dy), False), (dy, True), (odd(dy), True)):
+        assert all(torch.equal(a, b) for a, b in zip(grads(gradient, hooks), want))

@@ -63,12 +63,22 @@ def train_forward(x: Tensor, gamma, beta, residual, bn: nn.BatchNorm1d, relu: bo
     return y, saved
 
 
+def _aligned_rows(t: Optional[Tensor]) -> Optional[Tensor]:
+    """``t`` contiguous on a 16-byte boundary (a gradient may be a view into a flat buffer, a saved tensor whatever a
+    saved-tensor hook made of it)."""
+    if t is not None:
+        t = t.contiguous()
+        if t.data_ptr() % 16:
+            t = t.clone()
+    return t
+
+
 def train_backward(dy: Tensor, x: Tensor, gamma, beta, saved: Tensor, y: Optional[Tensor], relu: bool, need_x: bool,
                    need_res: bool):
     """(dx, (d beta, d gamma), d residual); ``y`` only with a residual under a ReLU."""
+    x, dy, y = _aligned_rows(x), _aligned_rows(dy), _aligned_rows(y)
     n, c = x.shape
     dev, dc, st = x.device, dtype_code(x.dtype), stream_ptr(x.device)
-    dy = dy.contiguous()
     want_res = need_res and relu
     dx = torch.empty_like(x) if need_x or want_res else None
     dres = torch.empty_like(x) if want_res else None
@@ -118,9 +128,7 @@ def _bits(value: float) -> int:
 def aligned_residual(residual: Optional[Tensor], shape, dtype: torch.dtype) -> Optional[Tensor]:
     if residual is not None:
         assert residual.shape == shape, f"residual {tuple(residual.shape)} != {tuple(shape)}"
-        residual = residual.to(dtype).contiguous()
-        if residual.data_ptr() % 16:
-            residual = residual.clone()
+        residual = _aligned_rows(residual.to(dtype))
     return residual
 
 
