@@ -632,6 +632,31 @@ def test_layers_run_under_inference_mode(dtype):
         assert torch.equal(first[0], want) and torch.equal(first[1], want)
 
 
+@pytest.mark.parametrize("sort", [False, True])
+@pytest.mark.parametrize("c_in", [16, 24, 32])
+def test_network_takes_feature_rows_at_any_address(sort, c_in):
+    """Features that are a column block one element into a wider matrix: no row starts on a 16-byte boundary."""
+    coords = room_rows(3000)
+    torch.manual_seed(0)
+    model = MinkUNet18(c_in, 20).to(DEV)
+    randomize_batchnorm_(model, 1)
+    model = model.half().eval()
+    wide = torch.rand(len(coords), c_in + 8, generator=torch.Generator().manual_seed(1)).half().to(DEV)
+    x = wide[:, 1:1 + c_in]
+    vox = make_voxels(coords, x)
+    if sort:
+        vox = vox.sort()
+        x = x[vox.extra_attributes["perm"]]
+        wide[:, 1:1 + c_in] = x
+        vox = vox.replace(batched_features=wide[:, 1:1 + c_in])
+    assert vox.feature_tensor.data_ptr() % 16
+    with torch.no_grad():
+        got = model(vox).feature_tensor
+        want = model(vox.replace(batched_features=x.contiguous())).feature_tensor
+    assert torch.equal(got, want)
+    check_device_status(DEV)
+
+
 def test_surface_errors_and_shortcuts():
     n = 2000
     coords, x, w = _layer_case(n, 8, 12, 5, "sample")

@@ -23,7 +23,7 @@ from ..geometry.coords.search.level_maps import LevelMaps
 from ..geometry.coords.search.search_results import IntSearchResult
 from ..nn.functional import sparse_conv
 from ..nn.functional.sparse_conv import (STRIDED_CONV_MODE, TILE_ORDER_MIN_OFFSETS, TILE_ORDER_MIN_ROWS, ConvEpilogue, train_layer_norm,
-                                         FusedConvLaunch, FusedRowsLaunch, _identity_map, _implicit_gemm_forward_logic, _merge_bias,
+                                         FusedConvLaunch, FusedRowsLaunch, _aligned, _identity_map, _implicit_gemm_forward_logic, _merge_bias,
                                          generate_output_coords_and_kernel_map, prefetch_strided_coordinates)
 from ..nn.functional.transforms import cat
 from ..nn.modules.activations import ReLU
@@ -285,6 +285,14 @@ class _LaunchPlan:
         return (list(map(_tensor_version, self._tensors)) == self._versions
                 and list(map(torch.Tensor.data_ptr, self._tensors)) == self._ptrs)
 
+    def stem_rows(self, feats: torch.Tensor) -> torch.Tensor:
+        """The features as rows that the stem takes: contiguous, for the tensor-core kernel on 16-byte boundaries."""
+        if feats.stride(1) != 1:
+            feats = feats.contiguous()
+        if self.stem.packed is not None and not _aligned(feats):
+            feats = feats.clone(memory_format=torch.contiguous_format)
+        return feats
+
     @staticmethod
     def _blocks(stage, x: torch.Tensor, nbr, rows, n: int, out: Optional[torch.Tensor] = None) -> torch.Tensor:
         last = len(stage) - 1
@@ -339,9 +347,7 @@ class _LaunchPlan:
             buf = torch.empty((rows, c_up + c_skip), dtype=dtype, device=dev)
             return buf, buf[:, :c_up], buf[:, c_up:]
 
-        feats = x.feature_tensor
-        if feats.stride(1) != 1:
-            feats = feats.contiguous()
+        feats = self.stem_rows(x.feature_tensor)
         # encoder: every stage writes its result into the right-hand block of its level's skip buffer
         bufs = [joined(n[0], P[7], self.init_dim), joined(n[1], P[6], P[0]), joined(n[2], P[5], P[1]),
                 joined(n[3], P[4], P[2])]
@@ -397,7 +403,7 @@ class _Program:
 
     def __init__(self, plan: "_LaunchPlan"):
         P, init = plan.planes, plan.init_dim
-        self.dtype, self.device = plan.dtype, plan.device
+        self.dtype, self.device, self.stem_rows = plan.dtype, plan.device, plan.stem_rows
         self.joined_width = [P[7] + init, P[6] + P[0], P[5] + P[1], P[4] + P[2]]
         skip_col = [P[7], P[6], P[5], P[4]]
         ops, width = [], {}
@@ -463,9 +469,7 @@ class _Program:
 
     def run(self, x: Voxels, restore_order: bool):
         dev, dtype = self.device, self.dtype
-        feats = x.feature_tensor
-        if feats.stride(1) != 1:
-            feats = feats.contiguous()
+        feats = self.stem_rows(x.feature_tensor)
         ic = x.batched_coordinates
         perm = x.extra_attributes.get("perm") if restore_order else None
         assert not restore_order or perm is not None, "restore_order needs the permutation that Voxels.sort records"
