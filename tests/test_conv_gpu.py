@@ -657,6 +657,32 @@ def test_network_takes_feature_rows_at_any_address(sort, c_in):
     check_device_status(DEV)
 
 
+@pytest.mark.parametrize("sort", [False, True])
+def test_a_layer_from_raw_coordinates_can_be_captured(sort):
+    """Sort, kernel map and a 3x3x3 layer in one CUDA graph: nothing on the way may wait on the host."""
+    coords = room_rows(5000)
+    xyz, x = torch.from_numpy(coords[:, 1:].copy()).to(DEV), torch.randn(len(coords), 32, device=DEV).half()
+    conv = SparseConv3d(32, 32, 3, bias=False).to(DEV).half()
+
+    def layer():
+        v = Voxels(xyz, x, offsets=torch.tensor([0, len(coords)]))
+        with torch.no_grad():
+            return conv(v.sort() if sort else v).feature_tensor
+    side = torch.cuda.Stream()
+    with torch.cuda.stream(side):
+        layer()
+    torch.cuda.synchronize()
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        got = layer()
+    for _ in range(2):
+        x.normal_()
+        xyz.copy_(xyz.flip(0))
+        graph.replay()
+        assert torch.equal(got, layer())
+    check_device_status(DEV)
+
+
 def test_surface_errors_and_shortcuts():
     n = 2000
     coords, x, w = _layer_case(n, 8, 12, 5, "sample")

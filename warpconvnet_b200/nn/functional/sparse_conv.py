@@ -674,7 +674,8 @@ def _level_map(fine: Voxels, kernel_size, kernel_dilation, stride, coarse_rows: 
     km = shared.get(("kmap",) + window)
     if km is None and window in _LEVEL_WINDOWS:
         if "level_maps" not in shared and shared.get("morton_info") is not None and ("strided", (2, 2, 2)) not in shared \
-                and window[0] == (3, 3, 3) and fine.batched_coordinates.batched_tensor.shape[0] > 0:
+                and window[0] == (3, 3, 3) and fine.batched_coordinates.batched_tensor.shape[0] > 0 \
+                and not torch.cuda.is_current_stream_capturing():  # (the host waits for the sizes of the levels)
             LevelMaps(fine.batched_coordinates, TILE_ORDER_MIN_ROWS, True, LAYER_SMALL_WINDOW_ROWS).attach()
         if "level_maps" in shared:
             maps, level = shared["level_maps"]
