@@ -125,3 +125,55 @@ def test_gradients_and_saved_tensors_at_any_address(dtype):
     assert odd(dy).data_ptr() % 16
     for gradient, hooks in ((odd(dy), False), (dy, True), (odd(dy), True)):
         assert all(torch.equal(a, b) for a, b in zip(grads(gradient, hooks), want))
+
+
+def test_modules_that_do_something_of_their_own_are_called_in_training():
+    """Hooks on the activation, on a geometry BatchNorm or on all modules, and classes with a forward of their own."""
+    from torch.nn.modules.module import register_module_forward_hook
+    from warpconvnet_b200 import ReLU, SparseConv3d
+    from warpconvnet_b200.examples.mink_unet import ConvTrBlock
+
+    class Halved(SparseConv3d):
+        def forward(self, *a, **kw):
+            y = super().forward(*a, **kw)
+            return y.replace(batched_features=y.feature_tensor * 0.5)
+
+    class Leaky(nn.ReLU):
+        def forward(self, x):
+            return torch.nn.functional.leaky_relu(x, 0.1)
+
+    g = torch.Generator().manual_seed(0)
+    xyz = torch.unique(torch.randint(0, 16, (2000, 3), generator=g, dtype=torch.int32), dim=0)
+    n = len(xyz)
+    vox = Voxels(xyz.to(DEV), torch.randn(n, 16, generator=g).to(DEV), offsets=torch.tensor([0, n])).sort()
+    for norm, act in ((nn.BatchNorm1d(16), nn.ReLU()), (BatchNorm(16), ReLU()), (BatchNorm(16), nn.Identity())):
+        seq = Sequential(SparseConv3d(16, 16, 3, bias=False), norm, act).to(DEV).train()
+        want = seq(vox).feature_tensor.detach()
+        modules = [seq[0], norm, act, *norm.children(), *act.children()]
+        for m in modules:
+            seen = []
+            handle = m.register_forward_hook(lambda *a: seen.append(1))
+            got = seq(vox).feature_tensor
+            handle.remove()
+            assert seen == [1], type(m)
+            assert rel_l2(got.detach().cpu().numpy(), want.cpu().numpy()) < 1e-5
+        seen = []
+        handle = register_module_forward_hook(lambda m, *a: seen.append(m))
+        try:
+            seq(vox)
+        finally:
+            handle.remove()
+        assert all(m in seen for m in modules)
+    up = ConvTrBlock(16, 16, kernel_size=2, stride=2).to(DEV).train()
+    coarse = SparseConv3d(16, 16, 2, stride=2).to(DEV)(vox)
+    for m in (up.conv_tr, up.norm_act, up.norm_act[0], up.norm_act[1]):
+        seen = []
+        handle = m.register_forward_hook(lambda *a: seen.append(1))
+        up(coarse, vox)
+        handle.remove()
+        assert seen == [1], type(m)
+    torch.manual_seed(0)
+    a = Sequential(Halved(16, 16, 3, bias=False), nn.BatchNorm1d(16, eps=1.0), Leaky()).to(DEV).train()
+    y = a(vox).feature_tensor
+    z = nn.functional.batch_norm(a[0](vox).feature_tensor, None, None, None, None, True, 0.0, 1.0)
+    assert rel_l2(y.detach().cpu().numpy(), nn.functional.leaky_relu(z, 0.1).detach().cpu().numpy()) < 1e-5

@@ -25,6 +25,7 @@ from ..nn.functional import sparse_conv
 from ..nn.functional.sparse_conv import (STRIDED_CONV_MODE, TILE_ORDER_MIN_OFFSETS, TILE_ORDER_MIN_ROWS, ConvEpilogue, train_layer_norm,
                                          FusedConvLaunch, FusedRowsLaunch, _aligned, _identity_map, _implicit_gemm_forward_logic, _merge_bias,
                                          generate_output_coords_and_kernel_map, prefetch_strided_coordinates)
+from ..nn.functional.batch_norm import bare
 from ..nn.functional.transforms import cat
 from ..nn.modules.activations import ReLU
 from ..nn.modules.sequential import Sequential, fold_batchnorm
@@ -61,7 +62,8 @@ class ConvTrBlock(nn.Module):
             ep = ConvEpilogue(scale=scale, shift=shift, relu=isinstance(self.norm_act[1], nn.ReLU), out=out)
             return self.conv_tr(x, out_spatial_sparsity, epilogue=ep)
         res = None
-        if bn.training and torch.is_grad_enabled() and isinstance(self.norm_act[1], (nn.ReLU, nn.Identity)):
+        if (bn.training and torch.is_grad_enabled() and type(self.norm_act[1]) in (nn.ReLU, nn.Identity)
+                and bare(self.norm_act, *self.norm_act)):
             res = train_layer_norm(self.conv_tr, bn, x, out_spatial_sparsity, isinstance(self.norm_act[1], nn.ReLU), None)
         if res is None:
             res = self.norm_act(self.conv_tr(x, out_spatial_sparsity))

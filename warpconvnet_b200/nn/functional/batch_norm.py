@@ -9,6 +9,7 @@ from typing import Optional
 
 import torch
 import torch.nn as nn
+import torch.nn.modules.module as _module
 from torch import Tensor
 
 from ..._native import check, dtype_code, lib, ptr, query_bytes, stream_ptr
@@ -29,6 +30,16 @@ def _counter(device: torch.device, stream: int) -> Tensor:
     return hit
 
 
+def bare(*modules: nn.Module) -> bool:
+    """Whether calling these modules runs their class's ``forward`` and nothing else: no hooks, on them or on all modules,
+    and no ``forward`` of the instance's own."""
+    if (_module._global_forward_hooks or _module._global_forward_pre_hooks or _module._global_backward_hooks
+            or _module._global_backward_pre_hooks):
+        return False
+    return not any(m._forward_hooks or m._forward_pre_hooks or m._backward_hooks or m._backward_pre_hooks or "forward" in m.__dict__
+                   for m in modules)
+
+
 def can_fuse(bn: nn.Module, x: Tensor) -> bool:
     """Whether ``batch_norm_act`` computes what ``bn(x)`` would (training mode, running statistics kept)."""
     return (x.is_cuda and x.dim() == 2 and x.is_contiguous() and x.data_ptr() % 16 == 0
@@ -39,7 +50,7 @@ def fusable(bn: nn.Module, n: int, c: int, dtype: torch.dtype, device: torch.dev
     """:func:`can_fuse` for contiguous rows that do not exist yet."""
     if type(bn) is not nn.BatchNorm1d or not bn.training or not bn.track_running_stats or bn.momentum is None:
         return False
-    if bn._forward_hooks or bn._forward_pre_hooks or bn._backward_hooks or bn._backward_pre_hooks:
+    if not bare(bn):
         return False
     mean, w, b = bn.running_mean, bn.weight, bn.bias
     return (device.type == "cuda" and dtype in _DTYPES and n >= 2 and c == bn.num_features and c <= 1024

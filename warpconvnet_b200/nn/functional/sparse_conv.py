@@ -1422,7 +1422,7 @@ def train_layer(layer, x: Voxels, target: Optional[Voxels]) -> Optional[Voxels]:
 def train_layer_norm(layer, bn, x: Voxels, target: Optional[Voxels], relu: bool, residual: Optional[Tensor]) -> Optional[Voxels]:
     """:func:`train_layer` with ``relu(bn(.) + residual)`` behind it; None when one of them does not take the call."""
     if (type(x) is not Voxels or layer.bias is not None or not _trains_natively(layer, x) or _is_pointwise(layer)
-            or layer._forward_hooks or layer._forward_pre_hooks or layer._backward_hooks or layer._backward_pre_hooks):
+            or not batch_norm.bare(layer)):
         return None
     feats, weight = x.feature_tensor, layer.weight
     if not (feats.requires_grad or weight.requires_grad) or (residual is not None and residual.dtype != feats.dtype):

@@ -69,13 +69,19 @@ def _is_relu(m) -> bool:
     return isinstance(m, (nn.ReLU, GeometryReLU))
 
 
+def _swallowed(m, *classes) -> bool:
+    """Whether ``m`` is exactly one of ``classes`` and nobody would notice that it is not called itself: in training other
+    functions stand for it, and hooks on it (or on the layer that a geometry module wraps) have to fire."""
+    return type(m) in classes and batch_norm.bare(m, *m.children())
+
+
 class Sequential(nn.Sequential, BaseSpatialModule):
     @staticmethod
     def _behind_norm(mods, j: int, residual: Optional[Tensor], final_relu: bool):
         """What a BatchNorm before position ``j`` can take along: (position behind it, ReLU, residual, whether the
         sequence's ``residual`` / ``final_relu`` are in it)."""
-        relu = j < len(mods) and _is_relu(mods[j])
-        if relu or (j < len(mods) and isinstance(mods[j], nn.Identity)):
+        relu = j < len(mods) and _swallowed(mods[j], nn.ReLU, GeometryReLU)
+        if relu or (j < len(mods) and _swallowed(mods[j], nn.Identity)):
             j += 1
         if j == len(mods) and (residual is not None or final_relu) and not relu:
             return j, final_relu, residual, True
@@ -119,7 +125,8 @@ class Sequential(nn.Sequential, BaseSpatialModule):
                 x = m(x, epilogue=ep)
                 i = j
                 continue
-            if bn is not None and bn.training and isinstance(m, SpatiallySparseConv) and torch.is_grad_enabled():
+            if (bn is not None and bn.training and isinstance(m, SpatiallySparseConv) and torch.is_grad_enabled()
+                    and type(m).forward is SpatiallySparseConv.forward and _swallowed(mods[i + 1], nn.BatchNorm1d, GeometryBatchNorm)):
                 # training: the convolution with its normalisation, residual and ReLU as one function
                 j, relu, res, tail = self._behind_norm(mods, i + 2, residual, final_relu)
                 y = train_layer_norm(m, bn, x, None, relu, res)
@@ -128,7 +135,7 @@ class Sequential(nn.Sequential, BaseSpatialModule):
                     fused_tail |= tail
                     continue
             bn = _as_bn(m)
-            if bn is not None and bn.training:
+            if bn is not None and bn.training and _swallowed(m, nn.BatchNorm1d, GeometryBatchNorm):
                 feats = x if isinstance(x, Tensor) else x.feature_tensor
                 if batch_norm.can_fuse(bn, feats):
                     # training: normalisation, residual and ReLU as one function
