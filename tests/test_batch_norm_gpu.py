@@ -177,3 +177,20 @@ def test_modules_that_do_something_of_their_own_are_called_in_training():
     y = a(vox).feature_tensor
     z = nn.functional.batch_norm(a[0](vox).feature_tensor, None, None, None, None, True, 0.0, 1.0)
     assert rel_l2(y.detach().cpu().numpy(), nn.functional.leaky_relu(z, 0.1).detach().cpu().numpy()) < 1e-5
+
+
+@pytest.mark.parametrize("shape", [(1, 16), (16,), ("n", 1)])
+def test_residuals_that_are_broadcast_train(shape):
+    from warpconvnet_b200 import SparseConv3d
+    g = torch.Generator().manual_seed(0)
+    xyz = torch.unique(torch.randint(0, 16, (2000, 3), generator=g, dtype=torch.int32), dim=0)
+    n = len(xyz)
+    vox = Voxels(xyz.to(DEV), torch.randn(n, 16, generator=g).to(DEV), offsets=torch.tensor([0, n]))
+    res = torch.randn([n if s == "n" else s for s in shape], generator=g).to(DEV).requires_grad_(True)
+    for seq in (Sequential(SparseConv3d(16, 16, 3, bias=False), nn.BatchNorm1d(16)), Sequential(nn.BatchNorm1d(16))):
+        seq = seq.to(DEV).train()
+        y = seq(vox, residual=res, final_relu=True).feature_tensor
+        want = torch.relu(seq(vox).feature_tensor + res)
+        assert rel_l2(y.detach().cpu().numpy(), want.detach().cpu().numpy()) < 1e-6
+        (a,), (b,) = torch.autograd.grad(y.sum(), [res]), torch.autograd.grad(want.sum(), [res])
+        assert a.shape == res.shape and rel_l2(a.cpu().numpy(), b.cpu().numpy()) < 1e-5

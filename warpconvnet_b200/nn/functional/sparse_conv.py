@@ -1432,7 +1432,7 @@ def train_layer_norm(layer, bn, x: Voxels, target: Optional[Voxels], relu: bool,
         return None
     tables, holder = found
     m, c = tables.num_out, weight.shape[2]
-    if not batch_norm.fusable(bn, m, c, feats.dtype, feats.device):
+    if not batch_norm.fusable(bn, m, c, feats.dtype, feats.device) or (residual is not None and residual.shape != (m, c)):
         return None
     y = _LayerNormFunction.apply(feats, weight, bn.weight, bn.bias, batch_norm.aligned_residual(residual, (m, c), feats.dtype),
                                  tables, bn, relu)

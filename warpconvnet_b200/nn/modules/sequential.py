@@ -142,7 +142,7 @@ class Sequential(nn.Sequential, BaseSpatialModule):
                     if isinstance(x, Geometry):
                         in_sf = x
                     j, relu, res, tail = self._behind_norm(mods, i + 1, residual, final_relu)
-                    if tail and residual is not None and residual.dtype != feats.dtype:
+                    if tail and residual is not None and (residual.dtype != feats.dtype or residual.shape != feats.shape):
                         relu, res, tail = False, None, False
                     fused_tail |= tail
                     x = batch_norm.batch_norm_act(feats, bn, relu, res)
