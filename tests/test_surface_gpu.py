@@ -218,3 +218,44 @@ def test_custom_kernel_center_matches_reference_fixture(golden):
     dils = generate_kernel_map(c, coarse, (2, 2, 2), (3, 3, 3), kernel_dilation=tuple(int(v) for v in g["dilation"]))
     assert np.array_equal(dils.neighbor_table(len(g["coarse"])).cpu().numpy(), g["found_ds"])
     check_device_status(DEV)
+
+
+def test_copies_and_pickles_of_what_has_run():
+    """Layers, networks, maps and voxels after their first use: nothing kept with them (launch records, plans, sizes still
+    on their way to the host) stands in the way of a copy or is carried over stale."""
+    import copy
+    import io
+    from warpconvnet_b200 import SparseConv3d, generate_kernel_map
+    from warpconvnet_b200.examples.mink_unet import MinkUNet18, randomize_batchnorm_
+    from warpconvnet_b200.datasets import synthetic
+    dev = "cuda:0"
+    xyz = torch.from_numpy(synthetic.room_scene(3000, 0.04, 3, "raster_crop")).to(dev)
+    n = len(xyz)
+    torch.manual_seed(0)
+    vox = Voxels(xyz, torch.randn(n, 3, device=dev).half(), offsets=torch.tensor([0, n])).sort()
+    wide = vox.replace(batched_features=torch.randn(n, 32, device=dev).half())
+    model = MinkUNet18(3, 20).to(dev)
+    randomize_batchnorm_(model, 1)
+    model = model.half().eval()
+    layer = SparseConv3d(32, 32, 3).to(dev).half()
+
+    def through_file(obj):
+        f = io.BytesIO()
+        torch.save(obj, f)
+        f.seek(0)
+        return torch.load(f, weights_only=False)
+    with torch.no_grad():
+        for net, x in ((layer, wide), (model, vox)):
+            want = net(x).feature_tensor
+            for clone in (copy.deepcopy(net), through_file(net)):
+                assert torch.equal(clone(x).feature_tensor, want)
+                for p in clone.parameters():
+                    p.zero_()
+                assert not clone(x).feature_tensor.any() and torch.equal(net(x).feature_tensor, want)
+            assert torch.equal(net(copy.deepcopy(x)).feature_tensor, want)
+    coords = torch.cat([torch.zeros((n, 1), dtype=torch.int32, device=dev), xyz], 1).contiguous()
+    torch.cuda.synchronize()
+    torch.cuda._sleep(20_000_000)
+    m = generate_kernel_map(coords, coords, (1, 1, 1), (3, 3, 3))
+    twin = copy.deepcopy(m)
+    assert torch.equal(twin.offsets, m.offsets) and torch.equal(twin.in_maps, m.in_maps) and torch.equal(twin.out_maps, m.out_maps)

@@ -279,6 +279,9 @@ class _LaunchPlan:
         self.head_rows = FusedRowsLaunch(head.weight, dtype, None, head_shift)
         self._program = None
 
+    def __reduce_ex__(self, protocol):
+        return type(None), ()   # a copy or a pickle of the model makes its own
+
     def current(self, dtype, device) -> bool:
         """True while no parameter or buffer has been written or re-allocated since the plan was made
         (version counters and data pointers compared in C loops: this runs on every forward)."""

@@ -48,6 +48,7 @@ class PyramidBuild:
         (repeated voxels, an extent of 2^21 or more)."""
         self._done.synchronize()
         host = self.host.tolist()
+        self.host = self._done = None  # (an event cannot be copied, and coordinates that hold this object can)
         nb = self.batches + 1
         raise_for_status(host[-1], self.device)
         if not host[-2]:

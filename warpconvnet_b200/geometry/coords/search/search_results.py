@@ -76,6 +76,12 @@ class IntSearchResult:
                                            stream_ptr(dev)), "wcn_kmap_scan_host")
         self._scanned = (offsets, *pinned_result(K + 2, torch.int32, dev, scan))
 
+    def __getstate__(self) -> dict:
+        state = self.__dict__.copy()
+        if state.pop("_scanned", None) is not None:
+            state["_workspace"] = None  # write positions by now; the sizes may not have arrived: a copy counts again
+        return state
+
     def _plain(self) -> Tensor:
         """The plain neighbour table of a map made dense."""
         if self._nbr is None:

@@ -165,6 +165,14 @@ def _cast_weight(weight: Tensor, dtype: torch.dtype, transposed: bool = False, r
     return w.to(dtype=dtype).contiguous()
 
 
+class _Kept(dict):
+    """What is derived from a weight and kept with it (packed copies, launch records with raw pointers): a copy or a
+    pickle of the weight starts without any."""
+
+    def __reduce_ex__(self, protocol):
+        return _Kept, ()
+
+
 def _prepared_weight(weight: Tensor, dtype: torch.dtype, algo: int = CONV_AUTO, transposed: bool = False,
                      reversed_: bool = False):
     """(weight in ``dtype`` or None, its re-tiled copy for the tensor-core kernel or None): one of the two.
@@ -173,7 +181,7 @@ def _prepared_weight(weight: Tensor, dtype: torch.dtype, algo: int = CONV_AUTO, 
     Both are cached ON the weight tensor object, tagged with its version counter,
     so an inference loop casts and re-tiles a parameter once and a parameter
     update invalidates the copy; the re-tiling kernel reads the parameter as it is."""
-    store = weight.__dict__.setdefault("_wcn_prepared", {})
+    store = weight.__dict__.setdefault("_wcn_prepared", _Kept())
     key, tag = (dtype, algo, transposed, reversed_), (weight._version, weight.data_ptr())
     hit = store.get(key)
     if hit is not None and hit[0] == tag:
@@ -360,7 +368,7 @@ def _prepared_rows_weight(weight: Tensor, dtype: torch.dtype, transposed: bool =
     """``(packed, c_out_packed)``: the weight re-tiled for the input-side kernel at a width padded to a
     multiple of 16 columns (extra columns zero), or ``(None, 0)`` when that kernel does not take the
     shape.  Cached on the weight tensor like :func:`_prepared_weight`."""
-    store = weight.__dict__.setdefault("_wcn_prepared", {})
+    store = weight.__dict__.setdefault("_wcn_prepared", _Kept())
     key, tag = (dtype, "rows", transposed), (weight._version, weight.data_ptr())
     hit = store.get(key)
     if hit is not None and hit[0] == tag:
@@ -1145,7 +1153,7 @@ class _LayerRecord:
 
 
 def _layer_record(weight, bias, scale, shift, relu, dtype) -> _LayerRecord:
-    store = weight.__dict__.setdefault("_wcn_layer", {})
+    store = weight.__dict__.setdefault("_wcn_layer", _Kept())
     rec = store.get((dtype, relu))
     if rec is None or not rec.current(weight, bias, scale, shift):
         rec = store[(dtype, relu)] = _LayerRecord(weight, bias, scale, shift, relu, dtype)
