@@ -194,3 +194,29 @@ def test_residuals_that_are_broadcast_train(shape):
         assert rel_l2(y.detach().cpu().numpy(), want.detach().cpu().numpy()) < 1e-6
         (a,), (b,) = torch.autograd.grad(y.sum(), [res]), torch.autograd.grad(want.sum(), [res])
         assert a.shape == res.shape and rel_l2(a.cpu().numpy(), b.cpu().numpy()) < 1e-5
+
+
+def test_captured_steps_do_not_depend_on_one_another():
+    """Of two graphs over the same memory pool the one captured last is replayed first (and the other never): nothing it
+    reads may be left to the first one to initialise."""
+    n, c = 5000, 32
+    x = torch.randn(n, c, device=DEV)
+    bn = nn.BatchNorm1d(c).to(DEV)
+    want = batch_norm_act(x, bn, True)
+    pool = torch.cuda.graph_pool_handle()
+
+    def captured(fn):
+        graph = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(graph, pool=pool):
+            out = fn()
+        return graph, out
+    junk, blocks = captured(lambda: [torch.full((131072,), 12345, dtype=torch.int32, device=DEV) for _ in range(16)])
+    junk.replay()
+    torch.cuda.synchronize()
+    del blocks
+    first = captured(lambda: batch_norm_act(x, bn, True))
+    second = captured(lambda: batch_norm_act(x, bn, True))
+    for _ in range(2):
+        second[0].replay()
+        assert torch.equal(second[1], want)
+    del first, second, junk

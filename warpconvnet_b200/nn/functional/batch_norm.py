@@ -19,13 +19,15 @@ _counters: dict = {}
 
 
 def _counter(device: torch.device, stream: int) -> Tensor:
-    """The block counter of the reductions: zero between launches of one stream."""
+    """The block counter of the reductions: zero between launches of one stream.  A launch that is being captured gets one
+    of its own, zeroed by the graph: graphs replay in any order and on any stream, and the capture's memory is theirs."""
+    if torch.cuda.is_current_stream_capturing():
+        return torch.zeros(1, dtype=torch.int32, device=device)
     key = (device.index, stream)
     hit = _counters.get(key)
     if hit is None:
-        if len(_counters) >= 256:  # streams come and go; a counter is 4 bytes
-            torch.cuda.synchronize(device)
-            _counters.clear()
+        if len(_counters) >= 256:  # streams come and go; the memory of a counter returns to its own stream
+            _counters.pop(next(iter(_counters)), None)
         hit = _counters[key] = torch.zeros(1, dtype=torch.int32, device=device)
     return hit
 
@@ -65,10 +67,10 @@ def train_forward(x: Tensor, gamma, beta, residual, bn: nn.BatchNorm1d, relu: bo
     y = torch.empty_like(x)
     saved = torch.empty((2, c), dtype=torch.float32, device=dev)
     ws = torch.empty(query_bytes("wcn_batch_norm_workspace_bytes", n, c, dc), dtype=torch.uint8, device=dev)
-    at = saved.data_ptr()
+    at, counter = saved.data_ptr(), _counter(dev, st)
     check(lib().wcn_batch_norm_train(ptr(x), n, c, dc, ptr(gamma), ptr(beta), _bits(bn.eps), _bits(bn.momentum),
                                      ptr(bn.running_mean), ptr(bn.running_var), ptr(bn.num_batches_tracked), ptr(residual),
-                                     int(relu), ptr(y), at, at + 4 * c, ptr(ws), ptr(_counter(dev, st)), st),
+                                     int(relu), ptr(y), at, at + 4 * c, ptr(ws), ptr(counter), st),
           "wcn_batch_norm_train")
     torch.autograd.graph.increment_version([bn.running_mean, bn.running_var, bn.num_batches_tracked])
     return y, saved
@@ -95,9 +97,9 @@ def train_backward(dy: Tensor, x: Tensor, gamma, beta, saved: Tensor, y: Optiona
     dres = torch.empty_like(x) if want_res else None
     sums = torch.empty((2, c), dtype=torch.float32, device=dev)
     ws = torch.empty(query_bytes("wcn_batch_norm_workspace_bytes", n, c, dc), dtype=torch.uint8, device=dev)
-    at = saved.data_ptr()
+    at, counter = saved.data_ptr(), _counter(dev, st)
     check(lib().wcn_batch_norm_backward(ptr(x), ptr(dy), ptr(y), n, c, dc, ptr(gamma), ptr(beta), at, at + 4 * c, int(relu),
-                                        ptr(dx), ptr(dres), ptr(sums), ptr(ws), ptr(_counter(dev, st)), st),
+                                        ptr(dx), ptr(dres), ptr(sums), ptr(ws), ptr(counter), st),
           "wcn_batch_norm_backward")
     return dx, sums, (dres if relu else dy) if need_res else None
 
