@@ -220,3 +220,32 @@ def test_captured_steps_do_not_depend_on_one_another():
         second[0].replay()
         assert torch.equal(second[1], want)
     del first, second, junk
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.float16])
+@pytest.mark.parametrize("n,c", [(2, 8), (7, 24), (50001, 64), (18945, 96), (200000, 16), (30000, 1024)])
+@pytest.mark.parametrize("at", [0, -1])
+def test_variance_keeps_its_precision_beside_a_large_value(dtype, n, c, at):
+    """One row far from all others, the first or the last one: the variance within a few dozen fp32 roundings,
+    the mean within as many of the spread."""
+    x = torch.randn(n, c, generator=torch.Generator().manual_seed(c)).to(dtype)
+    x[at] = 1000.0
+    bn = nn.BatchNorm1d(c, momentum=1.0).to(DEV)
+    with torch.no_grad():
+        batch_norm_act(x.to(DEV), bn)
+    xd = x.double()
+    mean, var = xd.mean(0), xd.var(0)
+    assert float((bn.running_mean.cpu().double() - mean).abs().max()) < 1e-6 * float(var.sqrt().min())
+    assert rel_l2(bn.running_var.cpu().numpy(), var.numpy()) < 2e-6
+
+
+def test_infinite_and_missing_values_reach_the_statistics():
+    """A channel with an infinity or a NaN has no variance; the others are untouched (as with nn.BatchNorm1d)."""
+    n, c = 1000, 16
+    x = torch.randn(n, c, device=DEV)
+    clean = batch_norm_act(x, nn.BatchNorm1d(c).to(DEV)).detach()
+    x[n // 2, 3], x[0, 5], x[n - 1, 7] = float("inf"), float("-inf"), float("nan")
+    y = batch_norm_act(x, nn.BatchNorm1d(c).to(DEV)).detach()
+    bad = torch.zeros(c, dtype=torch.bool, device=DEV)
+    bad[[3, 5, 7]] = True
+    assert torch.isnan(y[:, bad]).all() and torch.equal(y[:, ~bad], clean[:, ~bad])
