@@ -249,3 +249,31 @@ def test_infinite_and_missing_values_reach_the_statistics():
     bad = torch.zeros(c, dtype=torch.bool, device=DEV)
     bad[[3, 5, 7]] = True
     assert torch.isnan(y[:, bad]).all() and torch.equal(y[:, ~bad], clean[:, ~bad])
+
+
+@pytest.mark.parametrize("which", ["running_mean", "running_var", "weight", "bias", "num_batches_tracked"])
+def test_parameters_that_the_kernel_does_not_read_take_the_module(which):
+    """Every second element of a wider buffer, or a counter of another type: computed by nn.BatchNorm1d as before."""
+    n, c = 200, 16
+    x = torch.randn(n, c, device=DEV)
+
+    def build(strided):
+        g = torch.Generator().manual_seed(0)
+        bn = nn.BatchNorm1d(c).to(DEV)
+        for name in ("running_mean", "running_var", "weight", "bias"):
+            v = torch.rand(c, generator=g).to(DEV) + 0.5
+            if strided and name == which:
+                wide = torch.zeros(2 * c, device=DEV)
+                wide[::2] = v
+                v = wide[::2]
+            getattr(bn, name).data = v
+        if strided and which == "num_batches_tracked":
+            bn.num_batches_tracked = bn.num_batches_tracked.cpu()
+        return Sequential(bn).train()
+    vox = Voxels(torch.arange(3 * n, dtype=torch.int32, device=DEV).view(n, 3), x, offsets=torch.tensor([0, n]))
+    a, b = build(True), build(False)
+    assert not can_fuse(a[0], x) and can_fuse(b[0], x)
+    ya, yb = a(vox).feature_tensor, b(vox).feature_tensor
+    assert rel_l2(ya.detach().cpu().numpy(), yb.detach().cpu().numpy()) < 1e-6
+    for p, q in zip(a[0].buffers(), b[0].buffers()):
+        assert rel_l2(p.cpu().numpy(), q.cpu().numpy()) < 1e-6

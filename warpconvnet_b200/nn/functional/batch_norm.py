@@ -54,10 +54,12 @@ def fusable(bn: nn.Module, n: int, c: int, dtype: torch.dtype, device: torch.dev
         return False
     if not bare(bn):
         return False
-    mean, w, b = bn.running_mean, bn.weight, bn.bias
+    tracked = bn.num_batches_tracked
     return (device.type == "cuda" and dtype in _DTYPES and n >= 2 and c == bn.num_features and c <= 1024
-            and c % (4 if dtype == torch.float32 else 8) == 0 and mean.dtype == torch.float32 and mean.device == device
-            and (w is None or w.dtype == torch.float32) and (b is None or b.dtype == torch.float32))
+            and c % (4 if dtype == torch.float32 else 8) == 0 and tracked is not None and tracked.device == device
+            and tracked.dtype == torch.int64
+            and all(t is None or (t.dtype == torch.float32 and t.device == device and t.is_contiguous() and t.numel() == c)
+                    for t in (bn.running_mean, bn.running_var, bn.weight, bn.bias)))
 
 
 def train_forward(x: Tensor, gamma, beta, residual, bn: nn.BatchNorm1d, relu: bool):
