@@ -133,3 +133,33 @@ def test_pooling_gradients_of_every_width(reduction, dtype, c, ksize):
         np.add.at(want, i, gs[o] / (count[o][:, None] if reduction == "mean" else 1.0))
     check_device_status(DEV)
     assert rel_l2(got.double().cpu().numpy(), want) < {torch.float32: 1e-6, torch.float16: 1e-3, torch.bfloat16: 8e-3}[dtype]
+
+
+@pytest.mark.parametrize("reduction", ["max", "min", "mean", "sum"])
+@pytest.mark.parametrize("ksize", [2, 3])
+def test_pooling_has_second_derivatives(reduction, ksize):
+    """The gradient of a gradient, through the definition over the kernel map in fp64."""
+    coords, x, vox = _scene(800, 5, 67)
+    x = vox.feature_tensor.clone().requires_grad_(True)
+    out = sparse_reduce(vox.replace(batched_features=x), kernel_size=ksize, stride=2, reduction=reduction)
+    from warpconvnet_b200 import generate_kernel_map
+    nbr = generate_kernel_map(vox.batch_indexed_coordinates.contiguous(), out.batch_indexed_coordinates.contiguous(), (2, 2, 2),
+                              (ksize,) * 3).neighbor_table(len(out)).long()
+    xd = x.detach().double().requires_grad_(True)
+    have = (nbr >= 0).unsqueeze(2)
+    rows = xd[nbr.clamp(min=0)]
+    if reduction in ("max", "min"):
+        s = 1.0 if reduction == "max" else -1.0
+        window = torch.where(have, s * rows, -torch.inf)
+        want = s * window.gather(0, window.argmax(0, keepdim=True))[0]
+    else:
+        want = torch.where(have, rows, 0.0).sum(0)
+        want = want / have.sum(0) if reduction == "mean" else want
+
+    def second(y, x0):
+        (gx,) = torch.autograd.grad((y ** 3).sum(), [x0], create_graph=True)
+        (ggx,) = torch.autograd.grad((gx ** 2).sum(), [x0])
+        return gx.detach(), ggx
+    for a, b in zip(second(out.feature_tensor, x), second(want, xd)):
+        assert rel_l2(a.double().cpu().numpy(), b.cpu().numpy()) < 1e-5
+    check_device_status(DEV)

@@ -76,6 +76,13 @@ class _RowReduce(torch.autograd.Function):
         return _RowReduceBackward.apply(grad_out, ctx.kernel_map, ctx.num_in, arg, count), None, None, None
 
 
+def _attained(nbr: Tensor, arg: Tensor):
+    """(input row, whether there is one) per element ``[M, C]`` of the outputs, from the offset that attained its extremum."""
+    at = arg.long() & (255 if arg.dtype == torch.uint8 else 65535)
+    rows = nbr.t().gather(1, at.clamp(max=nbr.shape[0] - 1)).long()
+    return rows.clamp(min=0), (at < nbr.shape[0]) & (rows >= 0)
+
+
 class _RowReduceBackward(torch.autograd.Function):
     """The gradient of :class:`_RowReduce`, linear in the output gradient and differentiable with respect to it."""
 
@@ -100,10 +107,8 @@ class _RowReduceBackward(torch.autograd.Function):
         if arg is None:
             total = _native_reduce(gg.contiguous(), nbr, _NATIVE_OP[REDUCTIONS.SUM])
             return (total if count is None else (total / count.unsqueeze(1)).to(gg.dtype)), None, None, None, None
-        at = arg.long() & (255 if arg.dtype == torch.uint8 else 65535)
-        rows = nbr.long().gather(0, at.clamp(max=nbr.shape[0] - 1))
-        live = (at < nbr.shape[0]) & (rows >= 0)
-        return gg.gather(0, rows.clamp(min=0)) * live, None, None, None, None
+        rows, live = _attained(nbr, arg)
+        return torch.where(live, gg.gather(0, rows), torch.zeros((), dtype=gg.dtype, device=gg.device)), None, None, None, None
 
 
 def neighbor_reduction(features: Tensor, kernel_map: IntSearchResult, num_out: int,
