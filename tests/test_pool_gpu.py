@@ -163,3 +163,30 @@ def test_pooling_has_second_derivatives(reduction, ksize):
     for a, b in zip(second(out.feature_tensor, x), second(want, xd)):
         assert rel_l2(a.double().cpu().numpy(), b.cpu().numpy()) < 1e-5
     check_device_status(DEV)
+
+
+@pytest.mark.parametrize("reduction", ["max", "min"])
+@pytest.mark.parametrize("dtype", [torch.float32, torch.float16])
+def test_extremum_gradients_over_repeated_voxels(reduction, dtype):
+    """Pooling at stride 1 over repeated voxels: the outputs of a voxel's copies all take the same input row, whose
+    gradient is the sum of theirs."""
+    coords, x, _ = _scene(1500, 8, 65, dtype)
+    coords = np.concatenate([coords[coords[:, 0] == 0], coords[coords[:, 0] == 0][::3]])
+    n = len(coords)
+    g = torch.Generator().manual_seed(66)
+    x = torch.randn(n, 8, generator=g).to(dtype).to(DEV).requires_grad_(True)
+    vox = Voxels(torch.from_numpy(coords[:, 1:].copy()).to(DEV), x, offsets=torch.tensor([0, n]))
+    out = sparse_reduce(vox, kernel_size=3, stride=1, reduction=reduction).feature_tensor
+    dy = torch.randn(out.shape, generator=g).to(dtype).to(DEV)
+    (got,) = torch.autograd.grad(out, [x], dy)
+    from warpconvnet_b200 import generate_kernel_map
+    rows = vox.batch_indexed_coordinates.contiguous()
+    nbr = generate_kernel_map(rows, rows, (1, 1, 1), (3, 3, 3)).neighbor_table(n).long()
+    xd = x.detach().double().requires_grad_(True)
+    s = 1.0 if reduction == "max" else -1.0
+    window = torch.where((nbr >= 0).unsqueeze(2), s * xd[nbr.clamp(min=0)], -torch.inf)
+    want = s * window.gather(0, window.argmax(0, keepdim=True))[0]   # (the first of equal values)
+    (ref,) = torch.autograd.grad(want, [xd], dy.double())
+    assert torch.equal(out.detach().double(), want.detach())
+    assert rel_l2(got.double().cpu().numpy(), ref.cpu().numpy()) < (1e-6 if dtype == torch.float32 else 1e-3)
+    check_device_status(DEV)

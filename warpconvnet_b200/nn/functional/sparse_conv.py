@@ -655,6 +655,8 @@ def generate_output_coords_and_kernel_map(input_sparse_tensor: Voxels, kernel_si
                                                  bricks=_cached_bricks(input_sparse_tensor, in_coords))
 
         if not generative and output_spatially_sparse_tensor is None and order == POINT_ORDERING.RANDOM:
+            kernel_map._output_rows = (input_sparse_tensor.batched_coordinates._shared.setdefault("facts", {})
+                                       if all(s == 1 for s in stride) else {"unique": True})
             if all(s == 1 for s in stride):
                 kernel_map._onto_itself = all(k % 2 == 1 for k in kernel_size)
                 kernel_map._facts = input_sparse_tensor.batched_coordinates._shared.setdefault("facts", {})

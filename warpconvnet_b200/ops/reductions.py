@@ -90,14 +90,21 @@ class _RowReduceBackward(torch.autograd.Function):
     def forward(ctx, grad_out: Tensor, kernel_map: IntSearchResult, num_in: int, arg, count) -> Tensor:
         g = grad_out.contiguous()
         M, C, dev = g.shape[0], g.shape[1], g.device
+        ctx.kernel_map, ctx.num_out = kernel_map, M
+        ctx.save_for_backward(arg, count)
+        facts = getattr(kernel_map, "_output_rows", {})
+        if arg is not None and not (facts.get("distinct") or facts.get("unique")):
+            # Output rows with the same coordinates (or a caller's own map): an input row may have several at one offset,
+            # of which a transposed table holds one.  Added up where the extremum was instead.
+            rows, live = _attained(kernel_map.neighbor_table(M), arg)
+            gx = torch.zeros((num_in, C), dtype=torch.float32, device=dev)
+            return gx.scatter_add_(0, rows, torch.where(live, g.float(), 0.0)).to(g.dtype)
         nbr_t = kernel_map.swapped(num_in=num_in).neighbor_table(num_in)
         gx = torch.empty((num_in, C), dtype=g.dtype, device=dev)
         check(lib().wcn_row_reduce_backward(ptr(g), M, ptr(nbr_t), num_in, nbr_t.shape[0], C, dtype_code(g.dtype),
                                             ptr(arg), arg.element_size() if arg is not None else 0, ptr(count),
                                             ptr(gx), ptr(device_status(dev)), stream_ptr(dev)),
               "wcn_row_reduce_backward")
-        ctx.kernel_map, ctx.num_out = kernel_map, M
-        ctx.save_for_backward(arg, count)
         return gx
 
     @staticmethod
