@@ -119,16 +119,31 @@ KERNELS_PER_CALL = {
 LAUNCH_COUNTS: Counter = Counter()
 
 
+def _counted(raw, name: str, kernels: Optional[int]):
+    """``raw`` through ctypes, counting the kernels it launches."""
+    if not kernels:
+        return raw
+
+    def fn(*args):
+        LAUNCH_COUNTS[name] += kernels
+        return raw(*args)
+    return fn
+
+
 class _Library:
     """The C functions as attributes.  Those that take only integers and pointers go through the ``_fastcall``
     extension (csrc/fastcall.c): a 26-argument call costs 0.3 us there and 3.5 us through ctypes, which for a small
-    layer is as much as its launch.  It also counts the kernels they launch."""
+    layer is as much as its launch.  It also counts the kernels they launch.  The extension is a way of calling and no
+    more: where it cannot be built (it knows the argument passing of x86-64 Linux and needs Python 3.12 with its headers)
+    ``bind`` is None and ctypes makes the same calls."""
 
     def __init__(self, handle, bind):
         for name, argtypes in SIGNATURES.items():
             fn = getattr(handle, name)
             fn.argtypes, fn.restype = argtypes, ctypes.c_int
-            if all(t in (_c_i32, _c_i64, _c_vp) for t in argtypes):
+            if bind is None:
+                fn = _counted(fn, name, KERNELS_PER_CALL.get(name))
+            elif all(t in (_c_i32, _c_i64, _c_vp) for t in argtypes):
                 fn = bind(ctypes.cast(fn, ctypes.c_void_p).value, len(argtypes), name, LAUNCH_COUNTS,
                           KERNELS_PER_CALL.get(name))
             setattr(self, name, fn)
@@ -149,20 +164,29 @@ def lib():
     """The loaded library; raises NativeLibraryError when it is not built."""
     global _lib
     if _lib is None:
-        for path in (LIB_PATH, FASTCALL_PATH):
-            if not os.path.isfile(path):
-                raise NativeLibraryError(
-                    f"{path} is missing: build it with `python -m warpconvnet_b200.csrc.build` "
-                    "(nvcc, sm_100a). This package has no fallback path.")
+        if not os.path.isfile(LIB_PATH):
+            raise NativeLibraryError(
+                f"{LIB_PATH} is missing: build it with `python -m warpconvnet_b200.csrc.build` "
+                "(nvcc, sm_100a). This package has no fallback path.")
         try:
             handle = ctypes.CDLL(LIB_PATH)
-            spec = importlib.util.spec_from_file_location("_fastcall", FASTCALL_PATH)
-            fastcall = importlib.util.module_from_spec(spec)
-            spec.loader.exec_module(fastcall)
-        except (OSError, ImportError) as e:  # pragma: no cover
-            raise NativeLibraryError(f"cannot load the native library: {e}") from e
-        _lib = _Library(handle, fastcall.bind)
+        except OSError as e:  # pragma: no cover
+            raise NativeLibraryError(f"cannot load {LIB_PATH}: {e}") from e
+        _lib = _Library(handle, _fastcall_bind())
     return _lib
+
+
+def _fastcall_bind():
+    """``bind`` of the extension, or None where it was not built or does not load."""
+    if not os.path.isfile(FASTCALL_PATH):
+        return None
+    try:
+        spec = importlib.util.spec_from_file_location("_fastcall", FASTCALL_PATH)
+        fastcall = importlib.util.module_from_spec(spec)
+        spec.loader.exec_module(fastcall)
+    except ImportError:
+        return None
+    return fastcall.bind
 
 
 def status_string(status: int) -> str:

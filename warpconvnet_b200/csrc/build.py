@@ -1,5 +1,5 @@
 """Build libwcn_b200.so in this folder with nvcc for sm_100a (no other architecture), and the _fastcall.so extension
-through which Python calls it.
+through which Python calls it where that can be built (ctypes makes the calls elsewhere).
 
 Usage: ``python -m warpconvnet_b200.csrc.build [--force] [--verbose]``
 """
@@ -35,8 +35,14 @@ def needs_build():
 
 def build_fastcall(force=False):
     if force or not os.path.isfile(FASTCALL) or os.path.getmtime(FASTCALL_SOURCE) > os.path.getmtime(FASTCALL):
-        subprocess.check_call([os.environ.get("CC", "gcc"), "-O2", "-shared", "-fPIC", "-I" + sysconfig.get_paths()["include"],
-                               FASTCALL_SOURCE, "-o", FASTCALL])
+        cmd = [os.environ.get("CC", "gcc"), "-O2", "-shared", "-fPIC", "-I" + sysconfig.get_paths()["include"],
+               FASTCALL_SOURCE, "-o", FASTCALL]
+        try:
+            subprocess.check_call(cmd)
+        except (OSError, subprocess.CalledProcessError) as e:  # another machine, an older Python, no headers
+            if os.path.isfile(FASTCALL):
+                os.remove(FASTCALL)  # (of an earlier source)
+            print(f"_fastcall.so was not built ({e}): calls go through ctypes")
 
 
 def build(force=False, verbose=False, ptxas_info=False):
