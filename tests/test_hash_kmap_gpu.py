@@ -480,3 +480,26 @@ def test_results_on_their_way_to_the_host_keep_their_memory(what):
         torch.cuda.synchronize()
         assert all(bool((t == 7).all()) for t in mine)
     check_device_status(torch.device(DEV))
+
+
+def test_maps_are_made_where_the_cell_table_does_not_fit():
+    """With less memory free than the table of 4x4x4 cells takes, the voxel table makes the same map."""
+    dev = torch.device(DEV)
+    g = torch.Generator().manual_seed(0)
+    xyz = torch.unique(torch.randint(0, 160, (900000, 3), generator=g, dtype=torch.int32), dim=0)
+    xyz = xyz[torch.randperm(len(xyz), generator=g)]
+    n = len(xyz)
+    coords = torch.cat([torch.zeros((n, 1), dtype=torch.int32), xyz], 1).contiguous().to(dev)
+    want = generate_kernel_map(coords, coords, (1, 1, 1), (2, 2, 2))
+    want = [want.neighbor_table(n).clone(), want.in_maps.clone(), want.out_maps.clone(), want.offsets.clone()]
+    torch.cuda.synchronize()
+    torch.cuda.empty_cache()
+    total = torch.cuda.get_device_properties(dev).total_memory
+    torch.cuda.set_per_process_memory_fraction((torch.cuda.memory_reserved(dev) + 320 * n * 0.8) / total, dev)
+    try:
+        got = generate_kernel_map(coords, coords, (1, 1, 1), (2, 2, 2))
+        got = [got.neighbor_table(n), got.in_maps, got.out_maps, got.offsets]
+    finally:
+        torch.cuda.set_per_process_memory_fraction(1.0, dev)
+    assert all(torch.equal(a, b) for a, b in zip(got, want))
+    check_device_status(dev)

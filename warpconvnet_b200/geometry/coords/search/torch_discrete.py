@@ -112,22 +112,27 @@ def _kernel_map_from_size(hashtable: TorchHashTable, batched_query_coords: Tenso
     return IntSearchResult.from_neighbor_table(nbr, n_in, ws, identity_map_index)
 
 
-# The cell table reserves 288 bytes per key (the rows of up to one 4x4x4 cell per key): up to 4.6 GB; larger sets go
-# through the voxel table (40 bytes per key).
+# The cell table reserves 320 bytes per key (two 32-byte entries and the 64 rows of up to one 4x4x4 cell per key) while the
+# map is made: up to 5.4 GB.  Larger sets, and sets for which that much is not free, go through the voxel table (40 bytes
+# per key).
 CELL_TABLE_MAX_ROWS = 1 << 24
 
 
 def _kernel_map_from_cells(in_coords: Tensor, out_coords: Tensor, stride, kernel_size, identity_map_index, count_hits):
-    """A map of unordered coordinates for which the caller has no table: through a table of 4x4x4 cells."""
+    """A map of unordered coordinates for which the caller has no table: through a table of 4x4x4 cells.  None when there
+    is no memory for that."""
     dev, n, M, K = in_coords.device, in_coords.shape[0], out_coords.shape[0], int(np.prod(kernel_size))
     keys, q = in_coords.contiguous(), out_coords.contiguous()
     st = stream_ptr(dev)
-    table = torch.empty(query_bytes("wcn_cells_bytes", n), dtype=torch.uint8, device=dev)
+    try:
+        nbr = torch.empty((K, M), dtype=torch.int32, device=dev)
+        ws = torch.empty(query_bytes("wcn_kmap_workspace_bytes", M, K), dtype=torch.uint8, device=dev) if count_hits else None
+        table = torch.empty(query_bytes("wcn_cells_bytes", n), dtype=torch.uint8, device=dev)
+    except torch.OutOfMemoryError:
+        return None
     check(lib().wcn_cells_build(ptr(keys), n, ptr(table), st), "wcn_cells_build")
-    nbr = torch.empty((K, M), dtype=torch.int32, device=dev)
     ksz = (ctypes.c_int32 * 3)(*[int(k) for k in kernel_size])
     strd = (ctypes.c_int32 * 3)(*[int(s) for s in stride])
-    ws = torch.empty(query_bytes("wcn_kmap_workspace_bytes", M, K), dtype=torch.uint8, device=dev) if count_hits else None
     check(lib().wcn_kmap_search_cells(ptr(table), n, ptr(q), M, ctypes.addressof(strd), ctypes.addressof(ksz), ptr(nbr),
                                       ptr(ws), st), "wcn_kmap_search_cells")
     out = IntSearchResult.from_neighbor_table(nbr, n, ws, identity_map_index)
@@ -187,8 +192,10 @@ def generate_kernel_map(batch_indexed_in_coords: Tensor, batch_indexed_out_coord
             and batch_indexed_in_coords.is_cuda and batch_indexed_in_coords.shape[1] == 4
             and all(1 <= int(k) <= 4 for k in kernel_size) and (kernel_dilation is None or all(int(d) == 1 for d in kernel_dilation))
             and batch_indexed_in_coords.shape[0] <= CELL_TABLE_MAX_ROWS):
-        return _kernel_map_from_cells(batch_indexed_in_coords, batch_indexed_out_coords, stride, tuple(kernel_size),
+        done = _kernel_map_from_cells(batch_indexed_in_coords, batch_indexed_out_coords, stride, tuple(kernel_size),
                                       identity_map_index, count_hits)
+        if done is not None:
+            return done
     if hashtable is None or hashtable.hash_method != hash_method:
         hashtable = TorchHashTable.from_keys(batch_indexed_in_coords, hash_method=hash_method, device=dev)
     else:
