@@ -90,3 +90,28 @@ def test_repeated_voxels_and_huge_extents_are_not_usable():
     v = Voxels(coords, torch.zeros(50, 1, device=DEV), offsets=offsets).sort()
     assert PyramidBuild(v.batched_coordinates).finish() is None
     check_device_status(DEV)
+
+
+def test_large_pyramids_keep_no_more_than_their_rows(monkeypatch):
+    from warpconvnet_b200.geometry.coords.search import level_maps
+    from warpconvnet_b200.nn.functional.sparse_conv import strided_coordinates
+    g = torch.Generator(device="cuda").manual_seed(0)
+    n = 300000
+    cell = torch.randperm(128 ** 3, generator=g, device="cuda")[:n].int()
+    xyz = torch.stack([cell // (128 * 128), cell // 128 % 128, cell % 128], dim=1).int().contiguous()
+    tables = []
+    for limit in (n + 1, n):
+        monkeypatch.setattr(level_maps, "TRIMMED_ROWS", limit)
+        ic = Voxels(xyz, torch.zeros(n, 1, device="cuda"), offsets=torch.tensor([0, n])).sort().batched_coordinates
+        torch.cuda.synchronize()
+        before = torch.cuda.memory_allocated()
+        level, rows = ic, 0
+        for _ in range(4):
+            level = strided_coordinates(level, (2, 2, 2))
+            rows += len(level)
+        kept = torch.cuda.memory_allocated() - before
+        assert kept > 80 * n if limit > n else kept < 20 * rows + (64 << 10)
+        maps, _ = ic._shared["level_maps"]
+        tables.append([maps.kmap(l, w).neighbor_table(maps.n[l if w == 3 else l + 1]).clone() for l in range(4) for w in (3, 2)])
+    assert all(torch.equal(a, b) for a, b in zip(*tables))
+    check_device_status(torch.device("cuda:0"))

@@ -19,6 +19,10 @@ from ..integer import IntCoords
 from .search_results import IntSearchResult
 
 PYRAMID_LEVELS = 4
+# The levels are written into buffers for as many rows as the finest one (their sizes are not known before): 80 bytes per
+# fine row, of which a room's levels use about 7.  From this many rows on what is there is copied out; below it the eight
+# copies are not worth the at most 168 MB that stay with the coordinates.
+TRIMMED_ROWS = 1 << 21
 
 
 class PyramidBuild:
@@ -55,9 +59,15 @@ class PyramidBuild:
             return None
         self.ic._shared.setdefault("facts", {})["distinct"] = True
         levels = []
+        sizes = [host[(l + 1) * nb - 1] for l in range(PYRAMID_LEVELS)]
+        outs = [self.out[l, :m] for l, m in enumerate(sizes)]
+        if self.n >= TRIMMED_ROWS:
+            outs = [o.clone() for o in outs]
+            self.first = [self.first[l, :m].clone() for l, m in enumerate(sizes)]
+        self.out = None
         for l in range(PYRAMID_LEVELS):
             offs = host[l * nb:(l + 1) * nb]
-            rows = self.out[l, :offs[-1]]
+            rows = outs[l]
             c = object.__new__(IntCoords)
             c.offsets = torch.tensor(offs, dtype=torch.int64)
             c.offsets.__dict__["_wcn_tuple"] = tuple(offs)  # the form kernel-map cache keys want
