@@ -8,7 +8,7 @@ import torch
 
 from oracle import kernel_map as km
 from oracle import sparse_conv as osc
-from warpconvnet_b200 import (POINT_ORDERING, SPARSE_CONV_FWD_ALGO_MODE as ALGO, SparseConv2d, SparseConv3d, Voxels,
+from warpconvnet_b200 import (POINT_ORDERING, SPARSE_CONV_FWD_ALGO_MODE as ALGO, BatchNorm, Sequential, SparseConv2d, SparseConv3d, Voxels,
                               generate_kernel_map, spatially_sparse_conv)
 from warpconvnet_b200._native import check_device_status
 from warpconvnet_b200.geometry.coords.ops.batch_index import batch_indexed_coordinates
@@ -259,3 +259,29 @@ def test_copies_and_pickles_of_what_has_run():
     m = generate_kernel_map(coords, coords, (1, 1, 1), (3, 3, 3))
     twin = copy.deepcopy(m)
     assert torch.equal(twin.offsets, m.offsets) and torch.equal(twin.in_maps, m.in_maps) and torch.equal(twin.out_maps, m.out_maps)
+
+
+def test_pointwise_layers_take_part_in_forward_mode_and_function_transforms():
+    from torch.autograd import forward_ad as fwd
+    n = 100
+    coords = torch.arange(3 * n, dtype=torch.int32, device=DEV).view(n, 3)
+    layer = SparseConv3d(8, 4, 1).to(DEV)
+    x, t = torch.randn(n, 8, device=DEV), torch.randn(n, 8, device=DEV)
+
+    def f(feats):
+        return layer(Voxels(coords, feats, offsets=torch.tensor([0, n]))).feature_tensor
+    want = t @ layer.weight[0]
+    with fwd.dual_level():
+        tangent = fwd.unpack_dual(f(fwd.make_dual(x, t))).tangent
+        assert rel_l2(tangent.detach().cpu().numpy(), want.detach().cpu().numpy()) < 1e-5
+        block = Sequential(layer, BatchNorm(4), torch.nn.ReLU()).to(DEV).train()
+        y = block(Voxels(coords, fwd.make_dual(x, t), offsets=torch.tensor([0, n]))).feature_tensor
+        z = torch.relu(torch.nn.functional.batch_norm(fwd.make_dual(x, t) @ layer.weight[0] + layer.bias, None, None, training=True))
+        got, ref = fwd.unpack_dual(y).tangent, fwd.unpack_dual(z).tangent
+        assert rel_l2(got.detach().cpu().numpy(), ref.detach().cpu().numpy()) < 1e-4
+    _, tangent = torch.func.jvp(f, (x,), (t,))
+    assert rel_l2(tangent.detach().cpu().numpy(), want.detach().cpu().numpy()) < 1e-5
+    grad = torch.func.grad(lambda v: (f(v) ** 2).sum())(x)
+    xr = x.clone().requires_grad_(True)
+    (ref,) = torch.autograd.grad((f(xr) ** 2).sum(), [xr])
+    assert rel_l2(grad.detach().cpu().numpy(), ref.cpu().numpy()) < 1e-5

@@ -11,6 +11,7 @@ import torch
 import torch.nn as nn
 import torch.nn.modules.module as _module
 from torch import Tensor
+from torch.autograd import forward_ad
 
 from ..._native import check, dtype_code, lib, ptr, query_bytes, stream_ptr
 
@@ -30,6 +31,12 @@ def _counter(device: torch.device, stream: int) -> Tensor:
             _counters.pop(next(iter(_counters)), None)
         hit = _counters[key] = torch.zeros(1, dtype=torch.int32, device=device)
     return hit
+
+
+def reverse_mode_only() -> bool:
+    """Whether neither forward-mode differentiation nor a function transform is on: autograd functions take part in plain
+    backward passes only, torch's own operations in all of them."""
+    return forward_ad._current_level < 0 and not torch._C._are_functorch_transforms_active()
 
 
 def bare(*modules: nn.Module) -> bool:
@@ -52,7 +59,7 @@ def fusable(bn: nn.Module, n: int, c: int, dtype: torch.dtype, device: torch.dev
     """:func:`can_fuse` for contiguous rows that do not exist yet."""
     if type(bn) is not nn.BatchNorm1d or not bn.training or not bn.track_running_stats or bn.momentum is None:
         return False
-    if not bare(bn):
+    if not bare(bn) or not reverse_mode_only():
         return False
     tracked = bn.num_batches_tracked
     return (device.type == "cuda" and dtype in _DTYPES and n >= 2 and c == bn.num_features and c <= 1024

@@ -1015,7 +1015,8 @@ def spatially_sparse_conv(
 
     if all(k == 1 for k in _kernel_size) and all(s == 1 for s in _stride):
         native = feats.is_cuda and feats.dtype in (torch.float32, torch.float16, torch.bfloat16)
-        if epilogue is None and needs_grad and native and _normalize_bwd_algo(bwd_algo) != SPARSE_CONV_BWD_ALGO_MODE.EXPLICIT_GEMM:
+        if (epilogue is None and needs_grad and native and batch_norm.reverse_mode_only()
+                and _normalize_bwd_algo(bwd_algo) != SPARSE_CONV_BWD_ALGO_MODE.EXPLICIT_GEMM):
             out = _PointwiseFunction.apply(feats, weight)
             if bias is not None:
                 out = out + bias.to(out.dtype)
@@ -1416,7 +1417,7 @@ def train_layer(layer, x: Voxels, target: Optional[Voxels]) -> Optional[Voxels]:
         return None
     pointwise = _is_pointwise(layer)
     if pointwise:
-        if layer.transposed or target is not None or feats.dtype not in _NATIVE_DTYPES:
+        if layer.transposed or target is not None or feats.dtype not in _NATIVE_DTYPES or not batch_norm.reverse_mode_only():
             return None
         y = _PointwiseFunction.apply(feats, weight)
     else:
