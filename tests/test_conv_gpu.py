@@ -683,6 +683,19 @@ def test_a_layer_from_raw_coordinates_can_be_captured(sort):
     check_device_status(DEV)
 
 
+@pytest.mark.parametrize("dtype", [torch.float32, torch.float16])
+def test_launch_record_without_input_rows(dtype):
+    from warpconvnet_b200.nn.functional.sparse_conv import FusedConvLaunch
+    g = torch.Generator().manual_seed(0)
+    w, scale, shift = torch.randn(27, 32, 48, generator=g).to(dtype).to(DEV), torch.rand(48, device=DEV), torch.randn(48, device=DEV)
+    res = torch.randn(70, 48, generator=g).to(dtype).to(DEV)
+    nbr = torch.full((27, 70), -1, dtype=torch.int32, device=DEV)
+    none = torch.empty((0, 32), dtype=dtype, device=DEV)
+    got = FusedConvLaunch(w, dtype, scale, shift, relu=True)(none, nbr, None, 70, residual=res)
+    assert torch.equal(got, torch.relu(res.float() + shift).to(dtype))
+    assert not FusedConvLaunch(w, dtype)(none, nbr, None, 70).any()
+
+
 def test_surface_errors_and_shortcuts():
     n = 2000
     coords, x, w = _layer_case(n, 8, 12, 5, "sample")

@@ -351,8 +351,9 @@ class FusedConvLaunch:
         if num_out == 0:
             return out
         w_ptr = self._w_ptr
-        if w_ptr is None and feats.shape[0] == 0:
-            raise ValueError("a launch record needs at least one input row")
+        if w_ptr is None and feats.shape[0] == 0:  # no row to multiply, and no plain weights for the kernel of that case
+            _fill_unnamed_rows(out[:num_out], self.shift, residual, self.relu)
+            return out
         rc = self._fn(CONV_AUTO, feats.data_ptr(), feats.shape[0], feats.stride(0), w_ptr, self._packed_ptr,
                       nbr.data_ptr(), out_rows.data_ptr() if out_rows is not None else None, num_out, self.K,
                       self.c_in, self.c_out, self._dc, self._scale_ptr, self._shift_ptr,
