@@ -696,6 +696,19 @@ def test_launch_record_without_input_rows(dtype):
     assert not FusedConvLaunch(w, dtype)(none, nbr, None, 70).any()
 
 
+@pytest.mark.parametrize("dtype", [torch.float32, torch.float16])
+def test_a_bias_given_other_memory_is_seen(dtype):
+    """``bias.data = ...`` moves a parameter without a new version (flat-parameter optimisers and averaged models do)."""
+    coords = room_rows(500)
+    vox = make_voxels(coords, torch.randn(len(coords), 32, generator=torch.Generator().manual_seed(0)).to(dtype))
+    layer = SparseConv3d(32, 32, 3, bias=True).to(DEV).to(dtype)
+    with torch.no_grad():
+        before = layer(vox).feature_tensor.clone()
+        layer.bias.data = layer.bias.data + 4
+        after = layer(vox).feature_tensor
+    assert rel_l2((after - before).float().cpu().numpy(), np.full(before.shape, 4.0)) < 1e-2
+
+
 def test_surface_errors_and_shortcuts():
     n = 2000
     coords, x, w = _layer_case(n, 8, 12, 5, "sample")

@@ -1122,10 +1122,10 @@ def spatially_sparse_conv(
 # coordinate set (where the coordinate set's other derived data lives).
 
 
-def _version_of(t: Optional[Tensor]) -> int:
-    """The version counter of ``t``; tensors made under ``torch.inference_mode`` have none (nor can they be written
+def _written(t: Optional[Tensor]):
+    """What changes when ``t`` is written or given other memory: its address and its version counter; tensors made under ``torch.inference_mode`` have none (nor can they be written
     outside of it), such as the vectors a BatchNorm is folded to there."""
-    return 0 if t is None or t.is_inference() else t._version
+    return None if t is None else (t.data_ptr(), 0 if t.is_inference() else t._version)
 
 
 class _LayerRecord:
@@ -1138,7 +1138,7 @@ class _LayerRecord:
         ep = _merge_bias(ConvEpilogue(scale=scale, shift=shift), bias)
         self.w_version, self.w_ptr = weight._version, weight.data_ptr()
         self.vectors = (bias, scale, shift)
-        self.versions = tuple(map(_version_of, self.vectors))
+        self.versions = tuple(map(_written, self.vectors))
         self.conv = FusedConvLaunch(weight, dtype, ep.scale, ep.shift, relu=relu)
         self.rows = None  # FusedRowsLaunch, made by the first layer call that can use one
 
@@ -1146,8 +1146,8 @@ class _LayerRecord:
         b, sc, sh = self.vectors
         v = self.versions
         return (b is bias and sc is scale and sh is shift and weight._version == self.w_version
-                and weight.data_ptr() == self.w_ptr and _version_of(b) == v[0] and _version_of(sc) == v[1]
-                and _version_of(sh) == v[2])
+                and weight.data_ptr() == self.w_ptr and _written(b) == v[0] and _written(sc) == v[1]
+                and _written(sh) == v[2])
 
     def rows_launch(self, weight) -> "FusedRowsLaunch":
         if self.rows is None:
