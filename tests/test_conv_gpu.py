@@ -709,6 +709,28 @@ def test_a_bias_given_other_memory_is_seen(dtype):
     assert rel_l2((after - before).float().cpu().numpy(), np.full(before.shape, 4.0)) < 1e-2
 
 
+@pytest.mark.parametrize("c_in,c_out", [(24, 32), (48, 48), (64, 64)])
+def test_c_call_with_both_weights_takes_rows_at_any_address(c_in, c_out):
+    """The C function with plain and packed weights over rows that do not start on 16-byte boundaries: any kernel will do,
+    and one takes them."""
+    from warpconvnet_b200._native import CONV_AUTO, WCN_F16, check, device_status, lib, ptr, query_bytes, stream_ptr
+    dev, n = torch.device(DEV), 600
+    g = torch.Generator().manual_seed(c_in)
+    nbr = torch.where(torch.rand(8, n, generator=g) < 0.4, torch.randint(0, n, (8, n), generator=g), -1).int().to(dev)
+    w = (torch.randn(8, c_in, c_out, generator=g) * 0.1).half().to(dev)
+    wide = torch.randn(n, c_in + 8, generator=g).half().to(dev)
+    x = wide[:, 1:1 + c_in]
+    packed = torch.empty(query_bytes("wcn_conv_packed_weight_bytes", CONV_AUTO, 8, c_in, c_out, WCN_F16), dtype=torch.uint8, device=dev)
+    check(lib().wcn_conv_pack_weight(CONV_AUTO, ptr(w), 8, c_in, c_out, WCN_F16, ptr(packed), stream_ptr(dev)), "pack")
+    out = torch.empty(n, c_out, dtype=torch.float16, device=dev)
+    check(lib().wcn_conv_fwd(CONV_AUTO, x.data_ptr(), n, x.stride(0), ptr(w), ptr(packed), ptr(nbr), None, n, 8, c_in, c_out,
+                             WCN_F16, None, None, None, 0, 0, ptr(out), c_out, WCN_F16, 0, None, 0, ptr(device_status(dev)),
+                             stream_ptr(dev)), "wcn_conv_fwd")
+    want = sum(torch.where((nbr[k] >= 0)[:, None], x[nbr[k].clamp(min=0).long()].double(), 0.0) @ w[k].double() for k in range(8))
+    assert rel_l2(out.double().cpu().numpy(), want.cpu().numpy()) < 1e-3
+    check_device_status(dev)
+
+
 def test_surface_errors_and_shortcuts():
     n = 2000
     coords, x, w = _layer_case(n, 8, 12, 5, "sample")

@@ -118,7 +118,13 @@ extern "C" int wcn_conv_fwd(int algo, const void* feats, int64_t num_in, int64_t
   if (!nbr || !out || (num_in > 0 && !feats)) return WCN_ERR_INVALID_PARAMETERS;
   (void)workspace; (void)workspace_bytes;
   cudaStream_t st = wcn_stream(stream);
-  const bool tc_ok = wcn_conv_tcgen05_supported(num_offsets, c_in, c_out, dtype, out_dtype);
+  bool tc_ok = wcn_conv_tcgen05_supported(num_offsets, c_in, c_out, dtype, out_dtype);
+  if (algo == WCN_CONV_AUTO && weight && tc_ok) {
+    // rows that the tensor-core kernel does not read or write (16 bytes at a time): the other kernels take any address
+    const int64_t es = wcn_dtype_size(out_dtype);
+    auto odd = [](const void* p, int64_t row_bytes) { return ((reinterpret_cast<uintptr_t>(p) | (uintptr_t)row_bytes) & 15) != 0; };
+    if (odd(feats, feats_ld * 2) || odd(out, out_ld * es) || (residual && odd(residual, residual_ld * es))) tc_ok = false;
+  }
   if (conv_takes_tcgen05(algo, tc_ok, packed_weight, dev_status, num_in)) {
     if (!tc_ok) return WCN_ERR_UNSUPPORTED_CONFIG;
     return wcn_conv_tcgen05_fwd(feats, num_in, feats_ld, packed_weight, nbr, out_rows, num_out, num_offsets, c_in,

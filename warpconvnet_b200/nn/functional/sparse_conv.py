@@ -1123,8 +1123,9 @@ def spatially_sparse_conv(
 
 
 def _written(t: Optional[Tensor]):
-    """What changes when ``t`` is written or given other memory: its address and its version counter; tensors made under ``torch.inference_mode`` have none (nor can they be written
-    outside of it), such as the vectors a BatchNorm is folded to there."""
+    """What changes when ``t`` is written or given other memory: its address and its version counter.  Tensors made under
+    ``torch.inference_mode`` have none (nor can they be written outside of it), such as the vectors a BatchNorm is folded
+    to there."""
     return None if t is None else (t.data_ptr(), 0 if t.is_inference() else t._version)
 
 
