@@ -731,6 +731,31 @@ def test_c_call_with_both_weights_takes_rows_at_any_address(c_in, c_out):
     check_device_status(dev)
 
 
+@pytest.mark.parametrize("dtype", [torch.float32, torch.float16])
+@pytest.mark.parametrize("c_in", [3, 8, 33])
+def test_weight_gradient_of_gradients_that_are_not_finite(dtype, c_in):
+    """An overflown row of dY reaches the offsets at which that row has a neighbour, and no others."""
+    from warpconvnet_b200.nn.functional.sparse_conv import sparse_conv_wgrad
+    coords = room_rows(3000)
+    n, c_out = len(coords), 20
+    g = torch.Generator().manual_seed(c_in)
+    rows = torch.from_numpy(coords).to(DEV)
+    kmap = generate_kernel_map(rows, rows, (1, 1, 1), (3, 3, 3))
+    x, dy = (torch.randn(n, c, generator=g).to(dtype).to(DEV) for c in (c_in, c_out))
+    dy[17, 3], dy[1001, 5], dy[n - 1, 19] = float("inf"), float("nan"), float("-inf")
+    nbr = kmap.neighbor_table(n).long()
+    for tiled in (False, True):
+        got = sparse_conv_wgrad(x, dy, kmap, n, tile_order=tiled).double()
+        for k in range(27):
+            m = (nbr[k] >= 0).nonzero()[:, 0]
+            want = x[nbr[k, m]].double().T @ dy[m].double()
+            fine = torch.isfinite(want)
+            assert torch.equal(fine, torch.isfinite(got[k]))
+            assert not fine.any() or rel_l2(got[k][fine].cpu().numpy(), want[fine].cpu().numpy()) < 1e-5
+    assert not torch.isfinite(got).all() and torch.isfinite(got[:, :, 4]).all()
+    check_device_status(DEV)
+
+
 def test_surface_errors_and_shortcuts():
     n = 2000
     coords, x, w = _layer_case(n, 8, 12, 5, "sample")

@@ -200,11 +200,26 @@ conv_wgrad_pairs_kernel(const PairsParams p) {
 constexpr int NARROW_THREADS = 256;
 __host__ __device__ constexpr int narrow_offsets(int ci) { return 36 / ci; }   // 9 offsets of 4 channels, 4 of 8: 36 and 32 sums a thread
 
+// One element of dW over the rows begin .. end - 1, present pairs only.
+template <typename T>
+__device__ __noinline__ float present_sum(const PairsParams& p, int k, int c, int n, int64_t begin, int64_t end) {
+  float v = 0.f;
+  for (int64_t m = begin; m < end; ++m) {
+    const int r = __ldg(&p.nbr[(int64_t)k * p.M + m]);
+    if (r < 0 || r >= p.num_in) continue;
+    const int64_t row = p.out_rows ? (int64_t)__ldg(&p.out_rows[m]) : m;
+    v = fmaf(wcn_to_float<T>(reinterpret_cast<const T*>(p.feats)[(int64_t)r * p.c_in + c]),
+             wcn_to_float<T>(reinterpret_cast<const T*>(p.gout)[row * p.c_out + n]), v);
+  }
+  return v;
+}
+
 template <typename T, int CI>
 __global__ void __launch_bounds__(NARROW_THREADS, 2)
 conv_wgrad_narrow_kernel(const PairsParams p) {
   constexpr int KG = narrow_offsets(CI), WARPS = NARROW_THREADS / 32;
   __shared__ __align__(16) float xs[WARPS][KG][32][CI];
+  __shared__ int again;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int k0 = blockIdx.y * KG, j = blockIdx.z * 32 + lane;
   const bool col = j < p.c_out;
@@ -259,6 +274,7 @@ conv_wgrad_narrow_kernel(const PairsParams p) {
     __syncwarp();
   }
   // the block's sums, in warp order
+  if (threadIdx.x == 0) again = 0;
   __syncthreads();
   float* part = &xs[0][0][0][0];   // [KG * CI][WARPS][32] would not fit at once: one offset at a time
 #pragma unroll
@@ -272,9 +288,21 @@ conv_wgrad_narrow_kernel(const PairsParams p) {
 #pragma unroll
       for (int w = 0; w < WARPS; ++w) v += part[(c * WARPS + w) * 32 + (i & 31)];
       if (k0 + q < p.K && c < p.c_in && n < p.c_out) p.dst[(((int64_t)blockIdx.x * p.K + k0 + q) * p.c_in + c) * p.c_out + n] = v;
+      if (!isfinite(v)) again = 1;
     }
     __syncthreads();
   }
+  // Absent neighbours were multiplied as zeros: an infinity or NaN in dY made sums out of pairs that do not exist.  The sums
+  // that are not finite are taken once more, by themselves (kept in registers for a second pass of the warps they cost the
+  // finite case its registers: 3 channels bf16, 240 000 rows, 107 -> 120 us).
+  if (again)
+    for (int q = 0; q < KG; ++q)
+      for (int i = threadIdx.x; i < CI * 32; i += NARROW_THREADS) {
+        const int c = i / 32, n = blockIdx.z * 32 + (i & 31);
+        if (k0 + q >= p.K || c >= p.c_in || n >= p.c_out) continue;
+        float* dst = &p.dst[(((int64_t)blockIdx.x * p.K + k0 + q) * p.c_in + c) * p.c_out + n];
+        if (!isfinite(*dst)) *dst = present_sum<T>(p, k0 + q, c, n, begin, end);
+      }
   if (bad) wcn_report_bounds(p.dev_status);
 }
 
