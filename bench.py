@@ -6,11 +6,12 @@
     python bench.py --impl reference --steps K --warmup W  # the reference's CPU path
 
 Besides the headline (MinkUNet-34 voxels/s) the line carries, measured outside the timed
-regions: ``kmap`` (kernel-map build alone over 4 x 250 000-voxel rooms, both generators:
-Mcoords/s, algorithmic GB/s and fraction of the HBM copy bandwidth per stage), ``layers`` (single
-layers on a 500 000-voxel room: 3x3x3 / stride-2 down / transposed up, widths 32..256, fp16 and
-bf16), ``strong`` (the SAME 8-room batch divided among the ranks) and, with two or more ranks,
-``config5`` (one 8 M-voxel LiDAR scene split by Morton range with a halo exchange).
+regions, ``strong`` (the SAME 8-room batch divided among the ranks) and, with two or more ranks,
+``config5`` (one 8 M-voxel LiDAR scene split by Morton range with a halo exchange).  Tables, measured
+there too, are JSON lines on stderr: ``kmap`` (kernel-map build alone over 4 x 250 000-voxel rooms,
+both generators: Mcoords/s, algorithmic GB/s and fraction of the HBM copy bandwidth per stage),
+``layers`` (single layers on a 500 000-voxel room: 3x3x3 / stride-2 down / transposed up, widths
+32..256, fp16 and bf16) and ``roofline.by_shape``.
 
 One step = one pass of the whole path over one batch held by a rank: Morton
 ordering of the voxels, coordinate hashing, kernel-map generation for every
@@ -164,6 +165,27 @@ def cpu_forward_timed(args, repeats):
         osc.minkunet_forward(sd, coords, feats)
         times.append(time.perf_counter() - t0)
     return n, times
+
+
+def rounded(value):
+    """``value`` with its floats at six significant digits."""
+    if isinstance(value, float):
+        return float(f"{value:.6g}")
+    if isinstance(value, dict):
+        return {k: rounded(v) for k, v in value.items()}
+    return [rounded(v) for v in value] if isinstance(value, (list, tuple)) else value
+
+
+def print_result(line):
+    """The result as one line on stdout, short enough to be kept whole by whoever reads its tail; the tables (every kernel
+    map, every layer, every convolution shape) go to stderr, a JSON line each."""
+    line = rounded(line)
+    tables = {k: line.pop(k, None) for k in ("kmap", "layers")}
+    tables["roofline.by_shape"] = line["roofline"].pop("by_shape", None)
+    for name, table in tables.items():
+        if table is not None:
+            print(json.dumps({name: table}), file=sys.stderr, flush=True)
+    print(json.dumps(line), flush=True)
 
 
 def run_reference_arm(args):
@@ -623,7 +645,7 @@ def run_gpu_arm(args):
             "gpu_launches": int(launches), "clocks": clocks, "roofline": roofline, "cpu_baseline": cpu,
             "voxels_per_gpu": n_vox, "strong": strong, "kmap": kmap, "layers": layers, "config5": config5,
         }
-        print(json.dumps(line), flush=True)
+        print_result(line)
     if world > 1:
         dist.destroy_process_group()
 
