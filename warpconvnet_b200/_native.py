@@ -285,7 +285,8 @@ def pinned_result(words: int, dtype: torch.dtype, device: torch.device, launch):
     finally:
         done.record(torch.cuda.current_stream(device))
         with _written_lock:
-            _written[:] = [w for w in _written if not w[0].query()]
+            if len(_written) >= 16:
+                _written[:] = [w for w in _written if not w[0].query()]
             _written.append((done, host))
     return host, done
 

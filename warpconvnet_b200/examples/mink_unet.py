@@ -63,7 +63,7 @@ class ConvTrBlock(nn.Module):
             return self.conv_tr(x, out_spatial_sparsity, epilogue=ep)
         res = None
         if (bn.training and torch.is_grad_enabled() and type(self.norm_act[1]) in (nn.ReLU, nn.Identity)
-                and bare(self.norm_act, *self.norm_act)):
+                and bare(self.norm_act, *self.norm_act._modules.values())):
             res = train_layer_norm(self.conv_tr, bn, x, out_spatial_sparsity, isinstance(self.norm_act[1], nn.ReLU), None)
         if res is None:
             res = self.norm_act(self.conv_tr(x, out_spatial_sparsity))

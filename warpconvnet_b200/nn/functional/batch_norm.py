@@ -45,8 +45,12 @@ def bare(*modules: nn.Module) -> bool:
     if (_module._global_forward_hooks or _module._global_forward_pre_hooks or _module._global_backward_hooks
             or _module._global_backward_pre_hooks):
         return False
-    return not any(m._forward_hooks or m._forward_pre_hooks or m._backward_hooks or m._backward_pre_hooks or "forward" in m.__dict__
-                   for m in modules)
+    for m in modules:
+        d = m.__dict__  # (a training step asks this of every block: no attribute protocol)
+        if (d["_forward_hooks"] or d["_forward_pre_hooks"] or d["_backward_hooks"] or d["_backward_pre_hooks"]
+                or "forward" in d):
+            return False
+    return True
 
 
 def can_fuse(bn: nn.Module, x: Tensor) -> bool:
@@ -61,12 +65,17 @@ def fusable(bn: nn.Module, n: int, c: int, dtype: torch.dtype, device: torch.dev
         return False
     if not bare(bn) or not reverse_mode_only():
         return False
-    tracked = bn.num_batches_tracked
-    return (device.type == "cuda" and dtype in _DTYPES and n >= 2 and c == bn.num_features and c <= 1024
-            and c % (4 if dtype == torch.float32 else 8) == 0 and tracked is not None and tracked.device == device
-            and tracked.dtype == torch.int64
-            and all(t is None or (t.dtype == torch.float32 and t.device == device and t.is_contiguous() and t.numel() == c)
-                    for t in (bn.running_mean, bn.running_var, bn.weight, bn.bias)))
+    if (device.type != "cuda" or dtype not in _DTYPES or n < 2 or c != bn.num_features or c > 1024
+            or c % (4 if dtype == torch.float32 else 8)):
+        return False
+    buffers, params = bn._buffers, bn._parameters
+    tracked = buffers["num_batches_tracked"]
+    if tracked is None or tracked.device != device or tracked.dtype != torch.int64:
+        return False
+    for t in (buffers["running_mean"], buffers["running_var"], params["weight"], params["bias"]):
+        if t is not None and (t.dtype != torch.float32 or t.device != device or not t.is_contiguous() or t.numel() != c):
+            return False
+    return buffers["running_mean"] is not None
 
 
 def train_forward(x: Tensor, gamma, beta, residual, bn: nn.BatchNorm1d, relu: bool):

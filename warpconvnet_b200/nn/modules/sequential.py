@@ -72,7 +72,7 @@ def _is_relu(m) -> bool:
 def _swallowed(m, *classes) -> bool:
     """Whether ``m`` is exactly one of ``classes`` and nobody would notice that it is not called itself: in training other
     functions stand for it, and hooks on it (or on the layer that a geometry module wraps) have to fire."""
-    return type(m) in classes and batch_norm.bare(m, *m.children())
+    return type(m) in classes and batch_norm.bare(m, *m._modules.values())
 
 
 class Sequential(nn.Sequential, BaseSpatialModule):
@@ -126,7 +126,8 @@ class Sequential(nn.Sequential, BaseSpatialModule):
                 i = j
                 continue
             if (bn is not None and bn.training and isinstance(m, SpatiallySparseConv) and torch.is_grad_enabled()
-                    and type(m).forward is SpatiallySparseConv.forward and _swallowed(mods[i + 1], nn.BatchNorm1d, GeometryBatchNorm)):
+                    and type(m).forward is SpatiallySparseConv.forward
+                    and (mods[i + 1] is bn or _swallowed(mods[i + 1], GeometryBatchNorm))):   # (bn itself: fusable)
                 # training: the convolution with its normalisation, residual and ReLU as one function
                 j, relu, res, tail = self._behind_norm(mods, i + 2, residual, final_relu)
                 y = train_layer_norm(m, bn, x, None, relu, res)
@@ -135,7 +136,7 @@ class Sequential(nn.Sequential, BaseSpatialModule):
                     fused_tail |= tail
                     continue
             bn = _as_bn(m)
-            if bn is not None and bn.training and _swallowed(m, nn.BatchNorm1d, GeometryBatchNorm):
+            if bn is not None and bn.training and (m is bn or _swallowed(m, GeometryBatchNorm)):
                 feats = x if isinstance(x, Tensor) else x.feature_tensor
                 if batch_norm.can_fuse(bn, feats):
                     # training: normalisation, residual and ReLU as one function
