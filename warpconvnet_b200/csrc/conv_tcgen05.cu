@@ -81,7 +81,7 @@ struct ConvTcParams {
   void* out;
   int32_t* dev_status;
   int block_n;      // output columns per CTA (blockIdx.y selects the column block)
-  int G;            // sub-tiles per supertile: 1, 2 or 4
+  int G;            // sub-tiles per supertile: 1 or 2
   int nbuf;         // accumulator sets in TMEM: 1 or 2
   int cols;         // TMEM columns per accumulator (power of two >= block_n)
   int sa, sb;       // ring depths (row slots of each sub-tile, weight slots)
