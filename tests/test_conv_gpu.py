@@ -879,6 +879,26 @@ def test_tensor_core_units_at_the_edges(ksize, n, c_in, c_out):
         assert rel_l2(got[0].float().cpu().numpy(), ref.float().cpu().numpy()) < 2e-3
 
 
+@pytest.mark.parametrize("n", [18944, 18945, 37889, 65536, 65537, 12 * 16384, 13 * 16384 + 129])
+def test_every_unit_comes_once_whatever_their_order(n):
+    """Rows in tile order are worked through dense supertiles first, the last windows of a launch together: one unit per
+    multiprocessor, one more than that, small and large windows, whole and partial windows before the launch's tail.  The
+    sum of a row runs over the same offsets either way, so that the results are those of the plain order bit for bit."""
+    g = torch.Generator(device=DEV).manual_seed(n)
+    present = torch.rand(27, n, generator=g, device=DEV) < torch.rand(n, generator=g, device=DEV) ** 3
+    nbr = torch.where(present, torch.randint(0, n, (27, n), generator=g, device=DEV, dtype=torch.int32), torch.full((), -1, dtype=torch.int32, device=DEV))
+    kmap = IntSearchResult.from_neighbor_table(nbr, n)
+    x = torch.randn(n, 32, generator=g, device=DEV).half()
+    w = (torch.randn(27, 32, 32, generator=g, device=DEV) * 0.1).half()
+    got = []
+    for tiled in (False, True):
+        out = torch.full((n, 32), float("nan"), dtype=torch.float16, device=DEV)
+        got.append(sparse_conv_fused(x, w, kmap, n, epilogue=ConvEpilogue(out=out), algo=CONV_TCGEN05, tile_order=tiled))
+    check_device_status(DEV)
+    want = sparse_conv_fused(x, w, kmap, n, algo=CONV_SIMT)
+    assert torch.equal(*got) and rel_l2(got[0].float().cpu().numpy(), want.float().cpu().numpy()) < 2e-3
+
+
 @pytest.mark.parametrize("dtype", [torch.float16, torch.bfloat16])
 @pytest.mark.parametrize("ksize,n,c_in,c_out", [(3, 3000, 48, 64), (3, 700, 16, 16), (3, 5001, 40, 48), (3, 90000, 24, 112),
                                                 (2, 4000, 112, 80), (3, 2000, 200, 208), (1, 600, 72, 32)])

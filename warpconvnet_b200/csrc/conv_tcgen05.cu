@@ -26,7 +26,9 @@
 // MinkUNet-34 over 1.2 M voxels: 4.77 -> 4.50 ms.  Then a shorter way to the first copy of a launch - the first unit's neighbour loads issued before the barriers are set up, a
 // single unit's table published without a rendezvous of the index warps, no look at the status word on the way (the epilogue
 // reads it and writes NaN where an earlier launch gave up): C = 32 / 64 / 96 81 / 113 / 144 us, the network over one
-// scene of 20 000 voxels 928 -> 855 us, over 1.2 M 4.41 ms.
+// scene of 20 000 voxels 928 -> 855 us, over 1.2 M 4.41 ms.  Then the order of the units (supertile_of) and claims that wait
+// until the unit before last is done: a multiprocessor was idle for 15 to 17 % of a layer, 500 000 rows of 64 / 128 / 256
+// channels 113 / 187 / 547 -> 104 / 170 / 499 us, the network over 150 000 / 1.2 M voxels 1 318 / 4 589 -> 1 273 / 4 449.
 //
 // Problems with fewer 128-row tiles than multiprocessors divide the kernel offsets of a tile among the S CTAs of a
 // cluster ("split-K over kernel offsets": slice s owns the offsets k with k % S == s, which deals the frequent central
@@ -43,6 +45,7 @@
 // normal exit path (tensor memory released).
 #include "wcn_common.cuh"
 #include "tcgen05_common.cuh"
+#include "tile_order.cuh"
 #include <atomic>
 
 namespace {
@@ -61,7 +64,7 @@ constexpr int MMA_ISSUERS = 2;
 constexpr int WEIGHT_WARP = 26;       // weight bulk copies
 constexpr int THREADS = 864;
 constexpr int SMEM_LIMIT = 226 * 1024;  // dynamic shared memory the kernels opt in to
-constexpr int CLAIMS = 3;             // claimed units on their way or being read
+constexpr int TAIL_WINDOWS = 12;      // windows of the tile order that are begun together, at the end of a launch
 
 struct ConvTcParams {
   const char* feats;
@@ -90,11 +93,26 @@ struct ConvTcParams {
   int S;            // offset slices per supertile (split-K over kernel offsets); 1 = none
   int64_t units;    // supertiles * S work units, walked by the persistent CTAs (S > 1: one each)
   bool claim;       // one CTA per unit was launched: a CTA claims further units from the hardware's queue
+  int window, tail; // supertiles of a window of the tile order (0: rows in no such order), windows of the launch's tail
 };
 
 // Row lists (128 input rows of one sub-tile at one offset) staged per sub-tile: two units of ordinary density where K is
 // large, two of any density where it is small.
 __host__ __device__ inline int staged_lists(int K) { return K >= 27 ? K : (2 * K < 27 ? 2 * K : 27); }
+
+// The supertile that comes `turn`-th.  The tile order puts the rows with the fewest neighbours first in a window and those
+// with the most last, so that a supertile takes between a fifth of the mean time and three times as long.  Taken as they
+// lie, the last to begin were the longest: one multiprocessor finished while the others had been idle for 15 to 17 % of a
+// layer of 500 000 rows.  So every window is begun with its last supertile, windows from the last to the first, and the first
+// `tail` windows come together at the end, the longest supertiles of all of them first: what begins last is short.  (All
+// windows together would gather from the whole feature matrix at once.)
+__device__ __forceinline__ int64_t supertile_of(const ConvTcParams& p, int64_t turn) {
+  if (p.window == 0) return turn;
+  const int64_t head = p.supertiles - (int64_t)p.tail * p.window;
+  if (turn < head) return p.supertiles - 1 - turn;
+  const int j = (int)(turn - head), place = j / p.tail, w = j - place * p.tail;
+  return (int64_t)w * p.window + (p.window - 1 - place);
+}
 
 // Offsets of slice s of S: the k with k % S == s.
 __device__ __forceinline__ uint32_t slice_mask(int s, int S) {
@@ -194,8 +212,8 @@ struct Control {
   uint64_t acc_full[2][MAX_G], acc_empty[2][MAX_G];
   uint64_t info_full[2], info_empty[2];
   uint64_t idx_sync;              // rendezvous of the index threads (bounded, unlike bar.sync)
-  uint64_t claim_full[CLAIMS];    // a claimed unit has arrived in `claim`
-  __align__(16) uint64_t claim[CLAIMS][2];
+  uint64_t claim_full;            // a claimed unit has arrived in `claim`
+  __align__(16) uint64_t claim[2];
   int64_t info_unit[2];           // the unit; < 0: no more units
   uint32_t info_mask[2][MAX_G];   // non-empty offsets of each sub-tile
   int info_entry[2][MAX_G];       // first staged row list of each sub-tile
@@ -277,7 +295,8 @@ conv_tcgen05_kernel(const ConvTcParams p) {
     out_row = m < p.M ? (p.out_rows ? __ldg(&p.out_rows[m]) : (int32_t)m) : -1;
   };
   const bool indexing = warp >= EPI_THREADS / 32 && warp < GATHER_WARP0;
-  if (indexing) load_lists(blockIdx.x);
+  const int64_t first = p.S > 1 ? (int64_t)blockIdx.x : supertile_of(p, blockIdx.x);
+  if (indexing) load_lists(first);
   const uint32_t tmem_total = (uint32_t)(NBUF * G * p.cols);
   if (warp == 0) {
     for (int g = 0; g < G; ++g)
@@ -288,7 +307,7 @@ conv_tcgen05_kernel(const ConvTcParams p) {
       mbar_init(bar(&ctl->info_full[lane]), IDX_THREADS);
       mbar_init(bar(&ctl->info_empty[lane]), EPI_THREADS / 32 + G + 1 + GATHER_THREADS / 32);  // epilogue warps, MMA threads, weight thread, gather warps
     }
-    if (lane < CLAIMS) mbar_init(bar(&ctl->claim_full[lane]), 1);
+    if (lane == 2) mbar_init(bar(&ctl->claim_full), 1);
     if (lane < 3) ctl->mask_acc[lane][0] = ctl->mask_acc[lane][1] = 0;
     if (lane < 2) ctl->info_mask[0][lane] = 0;
     if (lane == 3) mbar_init(bar(&ctl->idx_sync), IDX_THREADS);
@@ -323,10 +342,9 @@ conv_tcgen05_kernel(const ConvTcParams p) {
     const int num_in = (int)p.num_in;
     int sphase = 0, entry = 0, before = 0;   // next free entry; entries of the unit before
     int n = 0, acc = 0;                      // units staged; scratch of this unit's masks
-    int asked = 0, slot = 0, cphase = 0;     // claims not read yet, the next one to read
-    bool refused = false;
+    int cphase = 0;
     bool bad = false;
-    int64_t unit = blockIdx.x;
+    int64_t unit = first, turn = blockIdx.x;
     if (single) {
       // A complete table of the one unit: nothing to compact, so the warps need not meet (a microsecond of the few that
       // such a launch takes).
@@ -345,33 +363,35 @@ conv_tcgen05_kernel(const ConvTcParams p) {
       mbar_arrive(bar(&ctl->info_full[1]));
       unit = -1;
     }
-    auto claim_one = [&](int at) {
-      if (itid == 0) {
-        // (every index thread has read the slot's last content: they met since)
-        asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-        claim_next(bar(&ctl->claim[at][0]), bar(&ctl->claim_full[at]));
-      }
-      ++asked;
-    };
-    if (p.claim) claim_one(0);
     while (ok && !single) {
       const int ib = n & 1;
       if (n > 0) {  // the unit after the one just staged
         if (!p.claim) {
-          unit += gridDim.x;
-          if (unit >= p.units) unit = -1;
+          turn += gridDim.x;
+          unit = turn < p.units ? supertile_of(p, turn) : -1;
         } else {
-          // (after a refusal nothing more is claimed, but a claim already on its way may still have been granted)
-          for (unit = -1; unit < 0 && asked > 0;) {
-            if (!mbar_wait(bar(&ctl->claim_full[slot]), cphase, p.dev_status)) { ok = false; break; }
-            unit = claimed_unit(ctl->claim[slot]);
-            // (not before: the next launch's CTAs would be placed ahead of this grid's that have not started, and wait there
-            // for the few multiprocessors left to it)
-            if (unit < 0 && !refused) { refused = true; launch_dependents(); }
-            if (++slot == CLAIMS) { slot = 0; cphase ^= 1; }
-            --asked;
+          // Not before the unit before last is done: a multiprocessor then holds the unit it works on and the next one, and
+          // those that are left go to whoever is free.  (Claimed two ahead, the last units waited in the queues of busy
+          // multiprocessors: with the order of the supertiles, 500 000 rows of 96 / 128 / 256 channels 143 / 187 / 547 -> 130 /
+          // 170 / 499 us, 80 000 rows of 64 channels 38 -> 34.)
+          if (!mbar_wait(bar(&ctl->info_empty[ib]), ((n >> 1) & 1) ^ 1, p.dev_status)) { ok = false; break; }
+          if (itid == 0) {
+            // (every index thread has read the last claim: they met since)
+            asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+            claim_next(bar(&ctl->claim[0]), bar(&ctl->claim_full));
           }
-          if (!ok) break;
+          // (a claim on its way writes this CTA's shared memory: it has to arrive before the CTA leaves)
+          if (!mbar_wait(bar(&ctl->claim_full), cphase, p.dev_status)) {
+            (void)mbar_wait(bar(&ctl->claim_full), cphase, p.dev_status);
+            ok = false;
+            break;
+          }
+          cphase ^= 1;
+          unit = claimed_unit(ctl->claim);
+          // (not before: the next launch's CTAs would be placed ahead of this grid's that have not started, and wait there
+          // for the few multiprocessors left to it)
+          if (unit < 0) launch_dependents();
+          else unit = supertile_of(p, unit);
         }
       }
       if (unit < 0) {
@@ -380,7 +400,6 @@ conv_tcgen05_kernel(const ConvTcParams p) {
         mbar_arrive(bar(&ctl->info_full[ib]));
         break;
       }
-      if (p.claim && !refused) claim_one(slot == CLAIMS - 1 ? 0 : slot + 1);
       if (n > 0) load_lists(unit);
       if (!mbar_wait(bar(&ctl->info_empty[ib]), ((n >> 1) & 1) ^ 1, p.dev_status)) { ok = false; break; }
       uint32_t has = 0;
@@ -430,12 +449,6 @@ conv_tcgen05_kernel(const ConvTcParams p) {
       mbar_arrive(bar(&ctl->info_full[ib]));  // (256 arrivals publish the lists)
       ++n;
     }
-    // claims on their way write this CTA's shared memory: they have to arrive (bounded waits) before it leaves
-    if (itid == 0 && p.claim)
-      for (; asked > 0; --asked) {
-        (void)mbar_wait(bar(&ctl->claim_full[slot]), cphase, p.dev_status);
-        if (++slot == CLAIMS) { slot = 0; cphase ^= 1; }
-      }
     if (bad) wcn_report_bounds(p.dev_status);
   } else if (warp == WEIGHT_WARP) {
     // ================================================================ weight loader
@@ -998,14 +1011,23 @@ bool plan_launch(ConvTcParams& p, int bk, int split_k, size_t* smem, dim3* grid)
   // the sums of a slice take the place of the rings
   if (S > 1 && sa * a_stage + sb * b_stage < (size_t)BLOCK_M * (p.block_n + 4) * 4) return false;
   *smem = fixed + sa * a_stage + sb * b_stage;
-  // With four units or more per multiprocessor one CTA per unit is launched, and the first to start claim the rest.  With
-  // fewer, claims made two units ahead deal unevenly (the first CTAs take three units, the last one: 36 -> 47 us for 80 000
-  // rows of 64 channels), and fixed strides let the next launch begin while the last units run.  (Column blocks are made of
-  // problems that fit at once; asked for on larger ones, their CTAs keep the strides: a claim could return another block's.)
+  // Where there are more units than multiprocessors one CTA per unit is launched, and the first to start claim the rest (the
+  // network over 2 x 100 000 voxels 1 701 -> 1 602 us against fixed strides below four units per multiprocessor and claims
+  // two ahead above).  Few units of rows in no tile order take much the same time and keep the fixed strides (2x2x2 down
+  // and up of 300 000 rows 60.9 us, 61.4 with claims).  Column blocks are made of problems that fit at once; asked for on
+  // larger ones, their CTAs keep the strides: a claim could return another block's.
   int64_t gx = p.units;
   const int64_t cap = sms / split > 0 ? sms / split : 1;
-  p.claim = S == 1 && split == 1 && gx >= 4 * cap;
+  p.claim = S == 1 && split == 1 && (p.out_rows ? gx > cap : gx >= 4 * cap);
   if (gx > cap && S == 1 && !p.claim) gx = cap;
+  // The windows of the tile order: 4096 rows up to 65 536 rows in a network.  (Whatever a caller's table has, every supertile
+  // comes once; only the order depends on it.)
+  p.window = p.out_rows && S == 1 ? (p.M > 65536 ? kTileWindowLarge : kTileWindowSmall) / (g * BLOCK_M) : 0;
+  p.tail = 0;
+  if (p.window > 0) {
+    const int64_t whole = p.supertiles / p.window;
+    p.tail = (int)(whole < TAIL_WINDOWS ? whole : TAIL_WINDOWS);
+  }
   *grid = dim3((unsigned)gx, (unsigned)split);
   return true;
 }
