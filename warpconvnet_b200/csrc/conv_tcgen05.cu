@@ -1020,9 +1020,7 @@ bool plan_launch(ConvTcParams& p, int bk, int split_k, size_t* smem, dim3* grid)
   const int64_t cap = sms / split > 0 ? sms / split : 1;
   p.claim = S == 1 && split == 1 && (p.out_rows ? gx > cap : gx >= 4 * cap);
   if (gx > cap && S == 1 && !p.claim) gx = cap;
-  // The windows of the tile order: 4096 rows up to 65 536 rows in a network.  (Whatever a caller's table has, every supertile
-  // comes once; only the order depends on it.)
-  p.window = p.out_rows && S == 1 ? (p.M > 65536 ? kTileWindowLarge : kTileWindowSmall) / (g * BLOCK_M) : 0;
+  p.window = p.out_rows && S == 1 ? tile_window(p.M, wcn_overlap_launches) / (g * BLOCK_M) : 0;
   p.tail = 0;
   if (p.window > 0) {
     const int64_t whole = p.supertiles / p.window;

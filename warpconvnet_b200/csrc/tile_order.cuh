@@ -8,6 +8,10 @@ namespace {
 constexpr int kTileWindowSmall = 4096, kTileWindowLarge = 16384;
 constexpr int kTileOrderThreads = 1024;
 
+// Rows of a window of a table of M rows in tile order: the large window above 4096 rows, in a network above 65 536.  (For the
+// order in which a convolution begins its tiles; a table with other windows gives the same results.)
+inline int tile_window(int64_t M, bool network) { return M > (network ? 65536 : 4096) ? kTileWindowLarge : kTileWindowSmall; }
+
 // Sort key of a row from which of its K offsets have a neighbour (bit k of `present`).  For a 3x3x3 window the centre
 // comes in bit 0, then the 6 face, 12 edge and 8 corner offsets, so that the rarest offsets are the most significant
 // bits and rows that share them end up in the same tiles (2-4 % fewer (tile, offset) pairs than offsets in index
