@@ -353,6 +353,12 @@ int wcn_conv_pack_weight(int algo, const void* weight, int32_t num_offsets, int3
 int wcn_conv_workspace_bytes(int algo, int64_t num_out, int32_t num_offsets, int32_t c_in, int32_t c_out,
                              int dtype, int out_dtype, int32_t split_k, int64_t* bytes);
 
+/* Bytes of `workspace` with which wcn_conv_fwd runs an fp32 problem on the tensor cores, every number as the exact sum of
+ * three bf16 numbers (csrc/conv_split_tcgen05.cu; its results are closer to exact sums than those of the FP32 pipes); 0
+ * where it does not.  Any 16-byte aligned device memory, used from the first launch of the call to its last.
+ * No reference counterpart. */
+int wcn_conv_f32_workspace_bytes(int64_t num_in, int64_t num_out, int32_t num_offsets, int32_t c_in, int32_t c_out, int64_t* bytes);
+
 /* Output-stationary sparse convolution with a fused epilogue:
  *   acc[s, :] = sum_k feats[nbr[k*M + s], :] @ weight[k]      (rows with nbr < 0 skipped, fp32 accumulation)
  *   m = out_rows[s]           (out_rows NULL: m = s; else a permutation of 0..M-1, see
@@ -375,7 +381,8 @@ int wcn_conv_workspace_bytes(int algo, int64_t num_out, int32_t num_offsets, int
  * owns the offsets k with k % S == s), whose fp32 sums are added in slice order before the epilogue: for problems with
  * fewer row blocks than multiprocessors.  0 = the library decides, 1 = never, 2.. = that many slices (at most 8); a
  * negative value divides the OUTPUT COLUMNS into -split_k blocks instead (a tuning aid).  `workspace` must hold
- * wcn_conv_workspace_bytes(...) for the same arguments (NULL / 0 when that is 0).  Results are the same bits on every run
+ * wcn_conv_workspace_bytes(...) for the same arguments (NULL / 0 when that is 0); fp32 problems under WCN_CONV_AUTO take one
+ * of wcn_conv_f32_workspace_bytes(...), with the same meaning of split_k > 0, and run on the FP32 pipes without.  Results are the same bits on every run
  * for a given S; different S round differently (fp32 sums are grouped by slice).
  * Replaces implicit_gemm (warpconvnet/csrc/warpconvnet_pybind.cpp:732-837,
  * warpconvnet/csrc/implicit_gemm.cu:44-267) and cutlass_gemm_AD_gather_scatter with its

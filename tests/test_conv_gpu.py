@@ -834,6 +834,66 @@ def test_fp32_kernel_matches_the_fp32_pipe_kernel(ksize, n, c_in, c_out):
     check_device_status(DEV)
 
 
+def _random_map(K, n, num_in, g):
+    present = torch.rand(K, n, generator=g, device=DEV) < torch.rand(n, generator=g, device=DEV) ** 2
+    nbr = torch.randint(0, num_in, (K, n), generator=g, device=DEV, dtype=torch.int32)
+    return IntSearchResult.from_neighbor_table(torch.where(present, nbr, torch.full((), -1, dtype=torch.int32, device=DEV)), num_in)
+
+
+@pytest.mark.parametrize("K,n,num_in,c_in,c_out", [(27, 1, 1, 64, 32), (27, 129, 500, 52, 48), (8, 2000, 4000, 36, 144), (8, 700, 700, 32, 32), (1, 13000, 13000, 128, 96), (27, 300, 300, 64, 64), (27, 14000, 14000, 20, 16),
+                                                   (27, 9472, 9000, 32, 128), (27, 9473, 9473, 96, 112), (27, 18945, 18945, 32, 32),
+                                                   (27, 70000, 70000, 64, 64), (3, 700, 600, 160, 256)])
+def test_fp32_on_the_tensor_cores_is_closer_to_exact_sums(K, n, num_in, c_in, c_out):
+    """Offsets divided among a cluster and not, whole and partial row tiles, column blocks, channels that do not fill a
+    slice, rows apart, every part of the epilogue: against sums in 64 bits.  What is dropped of a product is below 2^-25
+    of it and an accumulator adds 32 channels before it is rounded: 3e-7 is twice the largest error measured."""
+    g = torch.Generator(device=DEV).manual_seed(n)
+    kmap = _random_map(K, n, num_in, g)
+    nbr = kmap.neighbor_table(n)
+    wide = torch.randn(num_in, c_in + 4, generator=g, device=DEV)
+    x = wide[:, 4:]
+    w = torch.randn(K, c_in, c_out, generator=g, device=DEV) * (K * c_in) ** -0.5
+    res, scale, shift = torch.randn(n, c_out, generator=g, device=DEV), torch.rand(c_out, generator=g, device=DEV) + 0.5, torch.randn(c_out, generator=g, device=DEV)
+    want = torch.zeros(n, c_out, dtype=torch.float64, device=DEV)
+    for k in range(K):
+        m = (nbr[k] >= 0).nonzero()[:, 0]
+        want[m] += x[nbr[k, m].long()].double() @ w[k].double()
+    got = sparse_conv_fused(x, w, kmap, n)
+    again = sparse_conv_fused(x, w, kmap, n, tile_order=True)
+    simt = sparse_conv_fused(x, w, kmap, n, algo=CONV_SIMT)
+    check_device_status(DEV)
+    error = lambda y: float((y.double() - want).norm() / want.norm().clamp(min=1e-30))
+    assert error(got) < 3e-7 and error(again) < 3e-7
+    if n * c_out > 30000:
+        assert error(got) <= error(simt)
+    full = sparse_conv_fused(x, w, kmap, n, epilogue=ConvEpilogue(scale=scale, shift=shift, residual=res, relu=True))
+    want = (want * scale.double() + shift.double() + res.double()).clamp(min=0)
+    assert error(full) < 3e-7
+    check_device_status(DEV)
+
+
+@pytest.mark.parametrize("n", [12000, 19000])
+@pytest.mark.parametrize("where,value", [("x", float("inf")), ("x", float("nan")), ("x", 3.4e38), ("w", float("-inf")), ("w", 2.0 ** 64)])
+def test_fp32_numbers_without_three_parts(n, where, value, monkeypatch):
+    """Infinities, NaN and numbers whose partial products could overflow give what the FP32 pipes make of them."""
+    g = torch.Generator(device=DEV).manual_seed(n)
+    kmap = _random_map(27, n, n, g)
+    x = torch.randn(n, 32, generator=g, device=DEV)
+    w = torch.randn(27, 32, 32, generator=g, device=DEV)
+    if where == "x":
+        x[n // 2, 5] = value
+    else:
+        w[13, 7, 3] = value
+    got = sparse_conv_fused(x, w, kmap, n)
+    monkeypatch.setattr("warpconvnet_b200.nn.functional.sparse_conv._f32_workspace", lambda *a: (None, 0))
+    want = sparse_conv_fused(x, w, kmap, n)
+    check_device_status(DEV)
+    assert torch.equal(torch.isnan(got), torch.isnan(want)) and torch.equal(torch.isinf(got), torch.isinf(want))
+    fine = torch.isfinite(want)
+    assert torch.equal(got[~fine & ~torch.isnan(want)], want[~fine & ~torch.isnan(want)])
+    assert float((got[fine].double() - want[fine].double()).norm() / want[fine].double().norm()) < 1e-6
+
+
 @pytest.mark.parametrize("dtype", [torch.float32, torch.float16, torch.bfloat16])
 @pytest.mark.parametrize("ksize,n,c_in,c_out", [(3, 5000, 3, 32), (3, 1025, 8, 64), (2, 4000, 48, 20), (3, 3000, 64, 64),
                                                 (3, 700, 33, 31), (5, 600, 5, 96), (1, 40, 130, 70)])

@@ -63,6 +63,7 @@ SIGNATURES = {
     "wcn_conv_wgrad_pairs_workspace_bytes": [_c_i64, _c_i32, _c_i32, _c_i32, _p_i64],
     "wcn_conv_wgrad_pairs": [_c_vp, _c_i64, _c_vp, _c_vp, _c_vp, _c_i64, _c_i32, _c_i32, _c_i32, _c_i32, _c_vp, _c_vp, _c_i64, _c_vp, _c_vp],
     "wcn_conv_workspace_bytes": [_c_i32, _c_i64, _c_i32, _c_i32, _c_i32, _c_i32, _c_i32, _c_i32, _p_i64],
+    "wcn_conv_f32_workspace_bytes": [_c_i64, _c_i64, _c_i32, _c_i32, _c_i32, _p_i64],
     "wcn_conv_fwd": [_c_i32, _c_vp, _c_i64, _c_i64, _c_vp, _c_vp, _c_vp, _c_vp, _c_i64, _c_i32, _c_i32, _c_i32, _c_i32,
                      _c_vp, _c_vp, _c_vp, _c_i64, _c_i32, _c_vp, _c_i64, _c_i32, _c_i32, _c_vp, _c_i64, _c_vp, _c_vp],
     "wcn_batch_norm_workspace_bytes": [_c_i64, _c_i32, _c_i32, _p_i64],

@@ -26,6 +26,13 @@ int wcn_conv_fp32_fwd(const void* feats, int64_t num_in, int64_t feats_ld, const
                       const int32_t* out_rows, int64_t M, int K, int c_in, int c_out, const float* scale,
                       const float* shift, const void* residual, int64_t residual_ld, int relu, void* out,
                       int64_t out_ld, int sms, int32_t* dev_status, cudaStream_t st);
+// conv_split_tcgen05.cu
+bool wcn_conv_split_supported(int K, int c_in, int c_out);
+int64_t wcn_conv_split_workspace(int64_t num_in, int K, int c_in, int c_out);
+int wcn_conv_split_fwd(const void* feats, int64_t num_in, int64_t feats_ld, const void* weight, const int32_t* nbr,
+                       const int32_t* out_rows, int64_t M, int K, int c_in, int c_out, const float* scale, const float* shift,
+                       const void* residual, int64_t residual_ld, int relu, void* out, int64_t out_ld, int split_k, void* workspace,
+                       int32_t* dev_status, cudaStream_t st);
 // conv_tcgen05.cu
 bool wcn_conv_tcgen05_supported(int K, int c_in, int c_out, int dtype, int out_dtype);
 int64_t wcn_conv_tcgen05_packed_bytes(int K, int c_in, int c_out);
@@ -100,6 +107,22 @@ extern "C" int wcn_conv_workspace_bytes(int algo, int64_t num_out, int32_t num_o
   return WCN_OK;
 }
 
+extern "C" int wcn_conv_f32_workspace_bytes(int64_t num_in, int64_t num_out, int32_t num_offsets, int32_t c_in, int32_t c_out,
+                                            int64_t* bytes) {
+  if (!bytes || num_in < 0 || num_out < 0 || num_offsets <= 0 || c_in <= 0 || c_out <= 0) return WCN_ERR_INVALID_PARAMETERS;
+  // Few rows of narrow layers stay on the FP32 pipes, which are done before two launches are (us, FP32 pipes / tensor cores;
+  // 32 -> 32: 5 000 room voxels 22 / 20, random cells 17 / 20, outdoor 12 / 17, 10 000: 37 / 28, 25 / 28, 23 / 26, 20 000: 55 / 34,
+  // 43 / 30, 33 / 28; 64 -> 64, 2 000: 41 / 21, 33 / 22, 23 / 20).
+  // A single offset is one pass over the rows, which the planes double (20 000 rows: 64 -> 64 16 / 22, 128 -> 128 43 / 30); a few
+  // offsets of narrow layers run one thread per output row without (8 offsets, 32 -> 32: 59 / 18 for 5 000 rows).
+  const int64_t area = (int64_t)c_in * c_out;
+  const bool row_per_thread = wcn_conv_narrow_out_supported(num_offsets, c_in, c_out, WCN_F32, nullptr, c_in);
+  const bool few = num_offsets == 1 ? area < 12288 || num_out < 12000 : area < 2048 && num_out < 12000 && !row_per_thread;
+  *bytes = num_in > 0 && num_out > 0 && !few && wcn_conv_split_supported(num_offsets, c_in, c_out)
+               ? wcn_conv_split_workspace(num_in, num_offsets, c_in, c_out) : 0;
+  return WCN_OK;
+}
+
 extern "C" int wcn_conv_fwd(int algo, const void* feats, int64_t num_in, int64_t feats_ld, const void* weight,
                             const void* packed_weight, const int32_t* nbr, const int32_t* out_rows,
                             int64_t num_out, int32_t num_offsets, int32_t c_in, int32_t c_out, int dtype,
@@ -116,7 +139,6 @@ extern "C" int wcn_conv_fwd(int algo, const void* feats, int64_t num_in, int64_t
   if (feats_ld < c_in || out_ld < c_out || residual_ld < c_out) return WCN_ERR_INVALID_PARAMETERS;
   if (num_out == 0) return WCN_OK;
   if (!nbr || !out || (num_in > 0 && !feats)) return WCN_ERR_INVALID_PARAMETERS;
-  (void)workspace; (void)workspace_bytes;
   cudaStream_t st = wcn_stream(stream);
   bool tc_ok = wcn_conv_tcgen05_supported(num_offsets, c_in, c_out, dtype, out_dtype);
   if (algo == WCN_CONV_AUTO && weight && tc_ok) {
@@ -140,6 +162,13 @@ extern "C" int wcn_conv_fwd(int algo, const void* feats, int64_t num_in, int64_t
                                        out_dtype, dev_status, st);
     if (rc != WCN_ERR_UNSUPPORTED_CONFIG) return rc;
   }
+  const bool fp32 = algo == WCN_CONV_AUTO && num_in > 0 &&
+                    wcn_conv_fp32_supported(c_in, c_out, dtype, out_dtype, feats, feats_ld, weight, out, out_ld, residual, residual_ld);
+  if (fp32 && workspace && dev_status && (reinterpret_cast<uintptr_t>(workspace) & 15) == 0 &&
+      wcn_conv_split_supported(num_offsets, c_in, c_out) &&
+      workspace_bytes >= wcn_conv_split_workspace(num_in, num_offsets, c_in, c_out))
+    return wcn_conv_split_fwd(feats, num_in, feats_ld, weight, nbr, out_rows, num_out, num_offsets, c_in, c_out, scale, shift,
+                              residual, residual_ld, relu, out, out_ld, split_k, workspace, dev_status, st);
   if (algo == WCN_CONV_AUTO && num_in > 0 && wcn_conv_narrow_out_supported(num_offsets, c_in, c_out, dtype, feats, feats_ld)) {
     // a few output channels (a classification head): one thread per output row
     const int rc = wcn_conv_narrow_out_fwd(feats, num_in, feats_ld, weight, nbr, out_rows, num_out, num_offsets, c_in,
@@ -147,10 +176,10 @@ extern "C" int wcn_conv_fwd(int algo, const void* feats, int64_t num_in, int64_t
                                            out_dtype, dev_status, st);
     if (rc != WCN_ERR_UNSUPPORTED_CONFIG) return rc;
   }
-  if (algo == WCN_CONV_AUTO && num_in > 0 &&
-      wcn_conv_fp32_supported(c_in, c_out, dtype, out_dtype, feats, feats_ld, weight, out, out_ld, residual, residual_ld))
+  if (fp32) {
     return wcn_conv_fp32_fwd(feats, num_in, feats_ld, weight, nbr, out_rows, num_out, num_offsets, c_in, c_out, scale, shift,
                              residual, residual_ld, relu, out, out_ld, wcn_num_sms(), dev_status, st);
+  }
   return wcn_conv_simt_fwd(feats, num_in, feats_ld, weight, nbr, out_rows, num_out, num_offsets, c_in, c_out, dtype,
                            scale, shift, residual, residual_ld, relu, out, out_ld, out_dtype, dev_status, st);
 }

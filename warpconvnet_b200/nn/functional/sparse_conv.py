@@ -230,6 +230,19 @@ def _row_view(t: Tensor) -> Tensor:
     return t if t.dim() == 2 and t.stride(1) == 1 and t.stride(0) >= t.shape[1] else t.contiguous()
 
 
+def _f32_workspace(x: Tensor, num_out: int, K: int, c_in: int, c_out: int) -> Tuple[Optional[Tensor], int]:
+    """(memory with which an fp32 layer runs on the tensor cores, its bytes): ``(None, 0)`` where it does not."""
+    if x.dtype != torch.float32:
+        return None, 0
+    nbytes = query_bytes("wcn_conv_f32_workspace_bytes", x.shape[0], num_out, K, c_in, c_out)
+    if nbytes:
+        try:
+            return torch.empty(nbytes, dtype=torch.uint8, device=x.device), nbytes
+        except torch.cuda.OutOfMemoryError:  # one and a half times the features: the FP32 pipes need none
+            pass
+    return None, 0
+
+
 def sparse_conv_fused(in_features: Tensor, weight: Tensor, kernel_map: IntSearchResult, num_out_coords: int,
                       epilogue: Optional[ConvEpilogue] = None, out_dtype: Optional[torch.dtype] = None,
                       algo: int = CONV_AUTO, tile_order: Optional[bool] = None, split_k: int = 0,
@@ -306,10 +319,12 @@ def sparse_conv_fused(in_features: Tensor, weight: Tensor, kernel_map: IntSearch
         assert tuple(residual.shape) == (num_out_coords, c_out), \
             f"residual {tuple(residual.shape)} != output {(num_out_coords, c_out)}"
     dc, odc = dtype_code(x.dtype), dtype_code(out_dtype)
+    workspace, workspace_bytes = _f32_workspace(x, num_out_coords, K, c_in, c_out) if algo == CONV_AUTO and odc == dc else (None, 0)
     check(lib().wcn_conv_fwd(algo, ptr(x), x.shape[0], x.stride(0), ptr(w), ptr(packed), ptr(nbr), ptr(out_rows),
                              num_out_coords, K, c_in, c_out, dc, ptr(scale), ptr(shift), ptr(residual),
                              residual.stride(0) if residual is not None else 0, int(ep.relu), ptr(out),
-                             out.stride(0), odc, split_k, None, 0, ptr(device_status(dev)), stream_ptr(dev)),
+                             out.stride(0), odc, split_k, ptr(workspace), workspace_bytes, ptr(device_status(dev)),
+                             stream_ptr(dev)),
           "wcn_conv_fwd")
     return out
 
@@ -354,12 +369,14 @@ class FusedConvLaunch:
         if w_ptr is None and feats.shape[0] == 0:  # no row to multiply, and no plain weights for the kernel of that case
             _fill_unnamed_rows(out[:num_out], self.shift, residual, self.relu)
             return out
+        workspace, workspace_bytes = _f32_workspace(feats, num_out, self.K, self.c_in, self.c_out)
         rc = self._fn(CONV_AUTO, feats.data_ptr(), feats.shape[0], feats.stride(0), w_ptr, self._packed_ptr,
                       nbr.data_ptr(), out_rows.data_ptr() if out_rows is not None else None, num_out, self.K,
                       self.c_in, self.c_out, self._dc, self._scale_ptr, self._shift_ptr,
                       residual.data_ptr() if residual is not None else None,
                       residual.stride(0) if residual is not None else 0, self.relu, out.data_ptr(), out.stride(0),
-                      self._dc, 0, None, 0, self._status_ptr, torch._C._cuda_getCurrentRawStream(self._dev_index))
+                      self._dc, 0, ptr(workspace), workspace_bytes, self._status_ptr,
+                      torch._C._cuda_getCurrentRawStream(self._dev_index))
         if rc != 0:
             check(rc, "wcn_conv_fwd")
         return out
@@ -1373,9 +1390,10 @@ def _launch_layer(x: Tensor, weight: Tensor, t: _LayerTables, gradient: bool, ro
         c_in, c_out = c_out, c_in
     out = torch.empty((rows, c_out), dtype=x.dtype, device=x.device)
     dc = dtype_code(x.dtype)
+    workspace, workspace_bytes = _f32_workspace(x, rows, K, c_in, c_out)
     rc = lib().wcn_conv_fwd(CONV_AUTO, x.data_ptr(), x.shape[0], x.stride(0), ptr(w), ptr(packed), t.nbr.data_ptr(),
                             ptr(t.out_rows), rows, K, c_in, c_out, dc, None, None, None, 0, 0, out.data_ptr(), c_out, dc, 0,
-                            None, 0, device_status(x.device).data_ptr(), stream_ptr(x.device))
+                            ptr(workspace), workspace_bytes, device_status(x.device).data_ptr(), stream_ptr(x.device))
     if rc != 0:
         check(rc, "wcn_conv_fwd")
     return out
