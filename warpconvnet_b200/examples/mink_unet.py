@@ -497,13 +497,18 @@ class _Program:
             LAUNCH_COUNTS["wcn_net_run"] += n
 
         enqueue(0, 1)  # the stem runs while the host waits for the sizes of the coarser levels
-        if maps.finish() is None:
+        out = torch.empty((n0, self.classes), dtype=dtype, device=dev)
+        buffers[2 * self.OUT], buffers[2 * self.OUT + 1] = out.data_ptr(), self.classes
+        dst = perm.to(torch.int32) if restore_order else None
+        # from here to the last launch the device waits for the host: what can be done before or after is
+        if not maps.launch():
             return None
         for l in range(5):
             rows[l] = maps.n[l]
-            tables[2 * l], tables[2 * l + 1] = maps.nbr[l].data_ptr(), ptr(maps.order[l]) or 0
-            if l < 4:
-                tables[2 * (self.CHILD + l)] = maps.child[l].data_ptr()
+            nbr, order, child = maps.at[l]
+            tables[2 * l], tables[2 * l + 1] = nbr, order or 0
+            if l:
+                tables[2 * (self.CHILD + l - 1)] = child
         total, places = 0, []
         for b, level, w in self.arena:
             places.append((b, w, total))
@@ -512,18 +517,17 @@ class _Program:
         base = arena.data_ptr()
         for b, w, at in places:
             buffers[2 * b], buffers[2 * b + 1] = base + at, w
-        out = torch.empty((n0, self.classes), dtype=dtype, device=dev)
-        buffers[2 * self.OUT], buffers[2 * self.OUT + 1] = out.data_ptr(), self.classes
         if restore_order:  # sorted row j is original row perm[j]: each row of logits is written at its original place
-            dst = perm.to(torch.int32)
             tables[2 * self.PERM] = dst.data_ptr()
             enqueue(1, count - 2)
             last = NetOp.from_buffer_copy(self.ops[count - 1])
             last.table = self.PERM
             ops, count = ctypes.addressof(last), 1
             enqueue(0, 1)
+            maps.keep()
             return out
         enqueue(1, count - 1)
+        maps.keep()
         return x._derive(out)
 
 

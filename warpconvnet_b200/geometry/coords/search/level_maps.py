@@ -45,29 +45,42 @@ class PyramidBuild:
             check(lib().wcn_pyramid(ptr(rows), n, ptr(info), ptr(offsets), self.batches, PYRAMID_LEVELS, ptr(self.out),
                                     ptr(self.first), ptr(self.counts), ptr(host), ptr(ws), ptr(device_status(dev)),
                                     stream_ptr(dev)), "wcn_pyramid")
+        self.out_ptr = self.first_ptr = self.counted = None
         self.host, self._done = pinned_result(PYRAMID_LEVELS * (self.batches + 1) + 2, torch.int64, dev, launch)
 
-    def finish(self) -> Optional[List[IntCoords]]:
-        """Waits for the counts; the levels' coordinates, or None when the rows are not what the pyramid needs
+    def sizes(self) -> Optional[List[int]]:
+        """Waits for the counts; the levels' row counts, or None when the rows are not what the pyramid needs
         (repeated voxels, an extent of 2^21 or more)."""
         self._done.synchronize()
-        host = self.host.tolist()
+        host = self.counted = self.host.tolist()
         self.host = self._done = None  # (an event cannot be copied, and coordinates that hold this object can)
         nb = self.batches + 1
         raise_for_status(host[-1], self.device)
         if not host[-2]:
             return None
-        self.ic._shared.setdefault("facts", {})["distinct"] = True
-        levels = []
         sizes = [host[(l + 1) * nb - 1] for l in range(PYRAMID_LEVELS)]
-        outs = [self.out[l, :m] for l, m in enumerate(sizes)]
         if self.n >= TRIMMED_ROWS:
-            outs = [o.clone() for o in outs]
+            self.out = [self.out[l, :m].clone() for l, m in enumerate(sizes)]
             self.first = [self.first[l, :m].clone() for l, m in enumerate(sizes)]
-        self.out = None
+        # where each level's rows and first children start
+        trimmed = isinstance(self.out, list)
+        self.out_ptr = [self.out[l].data_ptr() if trimmed else self.out.data_ptr() + 16 * l * self.n for l in range(PYRAMID_LEVELS)]
+        self.first_ptr = [self.first[l].data_ptr() if trimmed else self.first.data_ptr() + 4 * l * self.n for l in range(PYRAMID_LEVELS)]
+        return sizes
+
+    def finish(self) -> Optional[List[IntCoords]]:
+        """The levels' coordinates, or None (see :meth:`sizes`)."""
+        return None if self.sizes() is None else self.coordinates()
+
+    def coordinates(self) -> List[IntCoords]:
+        """The levels' coordinates, once their sizes are known."""
+        host, nb = self.counted, self.batches + 1
+        self.ic._shared.setdefault("facts", {})["distinct"] = True
+        levels, outs = [], self.out
+        self.out = self.counted = self.out_ptr = self.first_ptr = None   # (addresses would be wrong in a copy)
         for l in range(PYRAMID_LEVELS):
             offs = host[l * nb:(l + 1) * nb]
-            rows = outs[l]
+            rows = outs[l] if isinstance(outs, list) else outs[l, :offs[-1]]
             c = object.__new__(IntCoords)
             c.offsets = torch.tensor(offs, dtype=torch.int64)
             c.offsets.__dict__["_wcn_tuple"] = tuple(offs)  # the form kernel-map cache keys want
@@ -115,39 +128,67 @@ class LevelMaps:
         n = self.build.n
         self.n = [n]
         self.rows = [self.build.rows]
-        self.nbr, self.order, self.child, self._bricks = {}, {}, {}, {}
+        self.nbr, self.order, self.child, self._bricks = {}, {}, {}, None
+        self.at, self._made = {}, []   # (nbr, order, child) addresses of a level; tables whose tensors have not been made
         if begin:
             self._enqueue(range(1))
 
     def _enqueue(self, which) -> None:
+        """The maps of some levels, all in one piece of memory (an allocation costs the host 2 us, a view as much)."""
         b = self.build
         levels = (Level * len(which))()
-        for slot, l in zip(levels, which):
+        total = bricks = 0
+        places = []
+        for l in which:
             n = self.n[l]
-            nbr = torch.empty((27, n), dtype=torch.int32, device=b.device)
-            order = torch.empty(n, dtype=torch.int32, device=b.device) if n >= self.min_rows else None
-            bricks = torch.empty(query_bytes("wcn_level_brick_bytes", n), dtype=torch.uint8, device=b.device)
-            self.nbr[l], self.order[l], self._bricks[l] = nbr, order, bricks
-            slot.rows, slot.n, slot.level = self.rows[l].data_ptr(), n, l
-            slot.bricks, slot.order, slot.nbr = bricks.data_ptr(), ptr(order), nbr.data_ptr()
+            words = -(-n // 64) * 64   # every table starts on a 256-byte boundary
+            tiled = n >= self.min_rows
+            places.append((l, n, total, total + 27 * words if tiled else None, total + 28 * words if l else None, bricks))
+            total += (28 + (8 if l else 0)) * words
+            bricks += -(-query_bytes("wcn_level_brick_bytes", n) // 256) * 256
+        memory = torch.empty(total, dtype=torch.int32, device=b.device)
+        scratch = self._bricks = torch.empty(bricks, dtype=torch.uint8, device=b.device)
+        base, brick_base = memory.data_ptr(), scratch.data_ptr()
+        for slot, (l, n, nbr, order, child, brick) in zip(levels, places):
+            at = self.at[l] = (base + 4 * nbr, None if order is None else base + 4 * order, None if child is None else base + 4 * child)
+            slot.rows, slot.n, slot.level = self._row_ptr(l), n, l
+            slot.bricks, slot.order, slot.nbr = brick_base + brick, at[1], at[0]
             if l:
-                child = self.child[l - 1] = torch.empty((8, n), dtype=torch.int32, device=b.device)
-                slot.child, slot.first_child = child.data_ptr(), b.first[l - 1].data_ptr()
-                slot.rows_below, slot.n_below = self.rows[l - 1].data_ptr(), self.n[l - 1]
+                slot.child = at[2]
+                slot.first_child = b.first_ptr[l - 1] if b.first_ptr else b.first[l - 1].data_ptr()
+                slot.rows_below, slot.n_below = self._row_ptr(l - 1), self.n[l - 1]
         check(lib().wcn_level_maps(ctypes.addressof(levels), len(which), ptr(b.info), ptr(b.counts),
                                    self.small_window_rows, stream_ptr(b.device)), "wcn_level_maps")
+        self._made.append((memory, places))
 
-    def _levels(self) -> Optional[List[IntCoords]]:
-        """The coordinates of levels 1..4, linked (None: not usable)."""
-        b = self.build
-        levels = b.finish()
-        if levels is None:
-            b.ic._shared["morton_info"] = None
-            return None
-        link_levels(b.ic, levels)
-        for c in levels:
-            self.rows.append(c._shared["bcoords"])
-            self.n.append(self.rows[-1].shape[0])
+    def _row_ptr(self, l: int) -> int:
+        return self.rows[l].data_ptr() if l < len(self.rows) else self.build.out_ptr[l - 1]
+
+    def _tensors(self) -> None:
+        """The tables that have been enqueued as tensors."""
+        self.at = {}   # (addresses would be wrong in a copy)
+        for memory, places in self._made:
+            for l, n, nbr, order, child, _ in places:
+                self.nbr[l] = memory[nbr:nbr + 27 * n].view(27, n)
+                self.order[l] = None if order is None else memory[order:order + n]
+                if child is not None:
+                    self.child[l - 1] = memory[child:child + 8 * n].view(8, n)
+        self._made = []
+
+    def _sizes(self) -> bool:
+        """Waits for the sizes of the levels; False: not usable."""
+        sizes = self.build.sizes()
+        if sizes is None:
+            self.build.ic._shared["morton_info"] = None
+            return False
+        self.n += sizes
+        return True
+
+    def _levels(self) -> List[IntCoords]:
+        """The coordinates of levels 1..4, linked."""
+        levels = self.build.coordinates()
+        link_levels(self.build.ic, levels)
+        self.rows += [c._shared["bcoords"] for c in levels]
         return levels
 
     def _window3(self, l: int) -> IntSearchResult:
@@ -158,14 +199,24 @@ class LevelMaps:
     def _window2(self, l: int) -> IntSearchResult:
         return IntSearchResult.from_neighbor_table(self.child[l], self.n[l], None, None)
 
-    def finish(self) -> Optional[List[IntCoords]]:
-        """The coordinates of levels 1..4 (None: not usable); their maps are enqueued and every level's maps left with
-        its coordinates, where layers of those geometries find them."""
-        levels = self._levels()
-        if levels is None:
-            return None
+    def launch(self) -> bool:
+        """Waits for the sizes of the levels and enqueues the maps of levels 1..4 (False: not usable): their addresses are in
+        ``at``.  :meth:`keep` does the rest, for which the device need not wait."""
+        if not self._sizes():
+            return False
         self._enqueue(range(1, PYRAMID_LEVELS + 1))
         self._bricks = None
+        return True
+
+    def finish(self) -> Optional[List[IntCoords]]:
+        """:meth:`launch` and :meth:`keep` (None: not usable)."""
+        return self.keep() if self.launch() else None
+
+    def keep(self) -> List[IntCoords]:
+        """The coordinates of levels 1..4, with every level's maps left with its coordinates, where layers of those
+        geometries find them."""
+        levels = self._levels()
+        self._tensors()
         for l, c in enumerate([self.build.ic] + levels):
             c._shared[("kmap", (3, 3, 3), (1, 1, 1))] = self._window3(l)
             if l < PYRAMID_LEVELS:
@@ -174,10 +225,11 @@ class LevelMaps:
 
     def attach(self) -> bool:
         """Levels linked, the maps made as layers ask for them (:meth:`kmap`); False: not usable."""
-        levels = self._levels()
-        if levels is None:
+        if not self._sizes():
             return False
-        self._bricks = {}
+        levels = self._levels()
+        self._bricks = None
+        self._tensors()
         for l, c in enumerate([self.build.ic] + levels):
             c._shared["level_maps"] = (self, l)
         self.build.ic = None  # (the coordinate sets hold this object, not the other way round)
@@ -190,5 +242,6 @@ class LevelMaps:
             return None
         if at not in self.nbr:
             self._enqueue(range(at, at + 1))
-            self._bricks = {}
+            self._bricks = None
+            self._tensors()
         return self._window3(l) if window == 3 else self._window2(l)
