@@ -460,6 +460,14 @@ int wcn_conv_wgrad(const void* feats, int64_t num_in, const void* grad_out, cons
                    const int32_t* out_rows, const uint32_t* tile_masks, int64_t num_out, int32_t num_offsets, int32_t c_in, int32_t c_out, int dtype,
                    float* grad_weight, int32_t* dev_status, void* stream);
 
+/* The same gradient of fp32 tensors on the tensor cores, every number as the exact sum of three bf16 numbers: grad_weight
+ * (16-byte aligned, like the other matrices and the workspace) is written, the same bits on every run.  c_in and c_out are
+ * multiples of 4 from 16 on, num_offsets at most 32, tile_masks must be given; 0 bytes: not taken. */
+int wcn_conv_wgrad_f32_workspace_bytes(int64_t num_in, int64_t num_out, int32_t num_offsets, int32_t c_in, int32_t c_out, int64_t* bytes);
+int wcn_conv_wgrad_f32(const float* feats, int64_t num_in, const float* grad_out, const int32_t* nbr, const int32_t* out_rows,
+                       const uint32_t* tile_masks, int64_t num_out, int32_t num_offsets, int32_t c_in, int32_t c_out,
+                       float* grad_weight, void* workspace, int64_t workspace_bytes, int32_t* dev_status, void* stream);
+
 /* The same gradient on the FP32 pipes, for any dtype and widths (fp32 tensors, a 3-channel stem): grad_weight is
  * written, not accumulated into, from partial sums of row ranges added in order (the same bits on every run).
  * `workspace`: wcn_conv_wgrad_pairs_workspace_bytes bytes (0: none needed). */

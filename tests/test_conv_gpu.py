@@ -872,6 +872,40 @@ def test_fp32_on_the_tensor_cores_is_closer_to_exact_sums(K, n, num_in, c_in, c_
     check_device_status(DEV)
 
 
+@pytest.mark.parametrize("K,n,num_in,c_in,c_out", [(27, 1, 1, 64, 32), (27, 129, 90, 52, 48), (16, 4000, 6000, 36, 132), (32, 700, 700, 160, 16),
+                                                   (27, 5000, 5000, 96, 64), (27, 70000, 70000, 64, 64), (27, 66000, 66000, 128, 256)])
+def test_fp32_weight_gradient_on_the_tensor_cores(K, n, num_in, c_in, c_out):
+    """Groups that end inside an offset and past the last, partial tiles, one range and many, column blocks: against sums
+    in 64 bits (4e-7 is twice the largest error measured), closer to them than the FP32 pipes, twice the same bits."""
+    from warpconvnet_b200.nn.functional import sparse_conv as sc
+    g = torch.Generator(device=DEV).manual_seed(n)
+    kmap = _random_map(K, n, num_in, g)
+    nbr = kmap.neighbor_table(n)
+    x, dy = torch.randn(num_in, c_in, generator=g, device=DEV), torch.randn(n, c_out, generator=g, device=DEV)
+    want = torch.stack([x[nbr[k].clamp(min=0).long()].double().mul((nbr[k] >= 0)[:, None]).T @ dy.double() for k in range(K)])
+    error = lambda y: float((y.double() - want).norm() / want.norm().clamp(min=1e-30))
+    for tiled in (False, K <= 27):
+        got = [sc.sparse_conv_wgrad(x, dy, kmap, n, tile_order=tiled) for _ in range(2)]
+        check_device_status(DEV)
+        assert torch.equal(*got) and error(got[0]) < 4e-7
+    with pytest.MonkeyPatch.context() as m:
+        query = sc.query_bytes
+        m.setattr(sc, "query_bytes", lambda name, *a: 0 if name == "wcn_conv_wgrad_f32_workspace_bytes" else query(name, *a))
+        pipes = sc.sparse_conv_wgrad(x, dy, kmap, n)
+        assert n < 1000 or error(got[0]) <= error(pipes)
+        for value, row in ((float("inf"), 0), (float("nan"), n // 2), (1e30, n - 1)):
+            bad = dy.clone()
+            bad[row, 3] = value
+            want_bad = sc.sparse_conv_wgrad(x, bad, kmap, n)
+            with pytest.MonkeyPatch.context() as back:
+                back.setattr(sc, "query_bytes", query)
+                got_bad = sc.sparse_conv_wgrad(x, bad, kmap, n)
+            assert torch.equal(torch.isfinite(got_bad), torch.isfinite(want_bad))
+            fine = torch.isfinite(want_bad)
+            assert not fine.any() or rel_l2(got_bad[fine].cpu().numpy(), want_bad[fine].cpu().numpy()) < 1e-5
+    check_device_status(DEV)
+
+
 @pytest.mark.parametrize("n", [12000, 19000])
 @pytest.mark.parametrize("where,value", [("x", float("inf")), ("x", float("nan")), ("x", 3.4e38), ("w", float("-inf")), ("w", 2.0 ** 64)])
 def test_fp32_numbers_without_three_parts(n, where, value, monkeypatch):

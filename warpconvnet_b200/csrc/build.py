@@ -10,8 +10,8 @@ import sysconfig
 
 HERE = os.path.dirname(os.path.abspath(__file__))
 SOURCES = ["api.cu", "hash_kmap.cu", "brick_kmap.cu", "cell_kmap.cu", "morton_sort.cu", "level_maps.cu", "net_run.cu", "conv_explicit.cu", "row_reduce.cu", "batch_norm.cu", "conv_simt.cu", "conv_fp32.cu", "conv_split_tcgen05.cu", "conv_tcgen05.cu",
-           "conv_wgrad_tcgen05.cu", "conv_wgrad_pairs.cu", "conv_rows_tcgen05.cu"]
-HEADERS = ["wcn_common.cuh", "tile_order.cuh", "tcgen05_common.cuh", os.path.join("..", "..", "include", "wcn_b200.h")]
+           "conv_wgrad_tcgen05.cu", "conv_wgrad_split_tcgen05.cu", "conv_wgrad_pairs.cu", "conv_rows_tcgen05.cu"]
+HEADERS = ["wcn_common.cuh", "tile_order.cuh", "tcgen05_common.cuh", "split_bf16.cuh", os.path.join("..", "..", "include", "wcn_b200.h")]
 LIB = os.path.join(HERE, "libwcn_b200.so")
 FASTCALL_SOURCE, FASTCALL = os.path.join(HERE, "fastcall.c"), os.path.join(HERE, "_fastcall.so")
 NVCC_FLAGS = ["-gencode", "arch=compute_100a,code=sm_100a", "-lineinfo", "-O3", "-std=c++17",

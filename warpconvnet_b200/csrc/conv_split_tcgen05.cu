@@ -29,6 +29,7 @@
 // 64 channels 40, of 128 69 instead of 30.
 #include "wcn_common.cuh"
 #include "tcgen05_common.cuh"
+#include "split_bf16.cuh"
 #include "tile_order.cuh"
 #include <atomic>
 
@@ -115,15 +116,6 @@ __device__ __forceinline__ float finish(const SplitParams& p, float y, int64_t m
 
 // ------------------------------------------------------------------ planes
 
-// x = h + m + l exactly (round to nearest twice; the rest has eight bits).
-__device__ __forceinline__ void split3(float x, __nv_bfloat16& h, __nv_bfloat16& m, __nv_bfloat16& l) {
-  h = __float2bfloat16_rn(x);
-  const float r = __fsub_rn(x, __bfloat162float(h));
-  m = __float2bfloat16_rn(r);
-  l = __float2bfloat16_rn(__fsub_rn(r, __bfloat162float(m)));
-}
-__device__ __forceinline__ bool unsplittable(float x) { return !(fabsf(x) < 9.223372e18f); }
-
 // Bound by memory (4 bytes in, 6 out per channel): a thread makes eight channels of a row, or of a column of the weights.
 __global__ void __launch_bounds__(256)
 split_planes_kernel(const float* __restrict__ feats, int64_t num_in, int64_t in_ld, const float* __restrict__ weight, int K, int c_in,
@@ -139,10 +131,7 @@ split_planes_kernel(const float* __restrict__ feats, int64_t num_in, int64_t in_
     if (i < rows) {
       const int64_t r = i / per_row;
       const int c = (int)(i - r * per_row) * 8;
-      const float* src = feats + r * in_ld + c;
-      const float4 a = c < c_in ? __ldg(reinterpret_cast<const float4*>(src)) : make_float4(0, 0, 0, 0);
-      const float4 b = c + 4 < c_in ? __ldg(reinterpret_cast<const float4*>(src + 4)) : make_float4(0, 0, 0, 0);
-      v[0] = a.x; v[1] = a.y; v[2] = a.z; v[3] = a.w; v[4] = b.x; v[5] = b.y; v[6] = b.z; v[7] = b.w;
+      load_eight(feats + r * in_ld, c, c_in, v);
       apart = (int64_t)cp * 2;
       dst = planes + r * 3 * apart + c * 2;
     } else {
@@ -155,14 +144,7 @@ split_planes_kernel(const float* __restrict__ feats, int64_t num_in, int64_t in_
       apart = (int64_t)c_out * SP_RB;
       dst = wplanes + ((int64_t)k * (cp / SP_BK) + c / SP_BK) * 3 * apart + tile_offset<SP_RB>(n, (c % SP_BK) / 8);
     }
-    __align__(16) __nv_bfloat16 part[3][8];
-#pragma unroll
-    for (int u = 0; u < 8; ++u) {
-      special |= unsplittable(v[u]);
-      split3(v[u], part[0][u], part[1][u], part[2][u]);
-    }
-#pragma unroll
-    for (int s = 0; s < 3; ++s) *reinterpret_cast<uint4*>(dst + s * apart) = *reinterpret_cast<const uint4*>(part[s]);
+    special |= store_parts(v, dst, apart);
   }
   const int any = __syncthreads_or(special);
   if (threadIdx.x == 0) flags[blockIdx.x] = any;
@@ -376,13 +358,11 @@ conv_split_kernel(const SplitParams p) {
             tc_fence_after();
             const uint64_t a = smem_desc<SP_RB>(base + slot * slot_bytes), b = smem_desc<SP_RB>(base + slot * slot_bytes + 3 * SP_PLANE);
             const uint32_t d = tmem + ab * SP_MAX_N;
-            // (plane of the rows, plane of the weights): small products first
-            constexpr int kA[6] = {2, 0, 1, 1, 0, 0}, kB[6] = {0, 2, 1, 0, 1, 0};
 #pragma unroll
             for (int q = 0; q < 6; ++q)
 #pragma unroll
               for (int kk = 0; kk < SP_BK / 16; ++kk)
-                umma_f16(d, a + (uint64_t)(kA[q] * (SP_PLANE >> 4) + kk * 2), b + (uint64_t)(kB[q] * (b_bytes >> 4) + kk * 2), idesc,
+                umma_f16(d, a + (uint64_t)(split_a(q) * (SP_PLANE >> 4) + kk * 2), b + (uint64_t)(split_b(q) * (b_bytes >> 4) + kk * 2), idesc,
                          q + kk > 0 ? 1u : 0u);
             umma_commit(bar(&ctl->empty[slot]));
             umma_commit(bar(&ctl->acc_full[ab]));

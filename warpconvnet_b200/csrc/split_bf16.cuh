@@ -1,0 +1,43 @@
+// fp32 numbers as sums of three bf16 numbers: what the kernels that multiply them on the tensor cores share.  Everything is
+// in an unnamed namespace: each translation unit gets its own copy.
+#pragma once
+#include "wcn_common.cuh"
+
+namespace {
+
+// The six products that are kept (first part of the one factor, of the other; 0 = h, 1 = m, 2 = l), small ones first: the
+// tensor core's accumulator drops what is below its last place.
+__host__ __device__ constexpr int split_a(int q) { return (0x001102 >> (4 * q)) & 15; }
+__host__ __device__ constexpr int split_b(int q) { return (0x010120 >> (4 * q)) & 15; }
+
+// x = h + m + l exactly (round to nearest twice; the rest has eight bits).
+__device__ __forceinline__ void split3(float x, __nv_bfloat16& h, __nv_bfloat16& m, __nv_bfloat16& l) {
+  h = __float2bfloat16_rn(x);
+  const float r = __fsub_rn(x, __bfloat162float(h));
+  m = __float2bfloat16_rn(r);
+  l = __float2bfloat16_rn(__fsub_rn(r, __bfloat162float(m)));
+}
+// Infinities, NaN, and numbers whose parts could have an infinite product where the numbers have none.
+__device__ __forceinline__ bool unsplittable(float x) { return !(fabsf(x) < 9.223372e18f); }
+
+// The parts of eight numbers, 16 bytes each, `apart` bytes from one another.
+__device__ __forceinline__ bool store_parts(const float (&v)[8], char* dst, int64_t apart) {
+  __align__(16) __nv_bfloat16 part[3][8];
+  bool special = false;
+#pragma unroll
+  for (int u = 0; u < 8; ++u) {
+    special |= unsplittable(v[u]);
+    split3(v[u], part[0][u], part[1][u], part[2][u]);
+  }
+#pragma unroll
+  for (int s = 0; s < 3; ++s) *reinterpret_cast<uint4*>(dst + s * apart) = *reinterpret_cast<const uint4*>(part[s]);
+  return special;
+}
+// Eight consecutive numbers of a row, zeros from `limit` on (a multiple of four; rows start on 16-byte boundaries).
+__device__ __forceinline__ void load_eight(const float* row, int c, int limit, float (&v)[8]) {
+  const float4 a = c < limit ? __ldg(reinterpret_cast<const float4*>(row + c)) : make_float4(0, 0, 0, 0);
+  const float4 b = c + 4 < limit ? __ldg(reinterpret_cast<const float4*>(row + c + 4)) : make_float4(0, 0, 0, 0);
+  v[0] = a.x; v[1] = a.y; v[2] = a.z; v[3] = a.w; v[4] = b.x; v[5] = b.y; v[6] = b.z; v[7] = b.w;
+}
+
+}  // namespace

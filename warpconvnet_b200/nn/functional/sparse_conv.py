@@ -839,8 +839,8 @@ def _cached_bricks(voxels: Optional[Voxels], coords: Tensor):
 def sparse_conv_wgrad(in_features: Tensor, grad_output: Tensor, kernel_map: IntSearchResult,
                       num_out_coords: int, tile_order: bool = False) -> Optional[Tensor]:
     """``dW[k] = X[in_k]^T @ dY[out_k]`` for every kernel offset, fp32 result ``[K, C_in, C_out]``: one launch on the
-    tensor cores for fp16 / bf16 widths of 16 and more that are multiples of 8 (input) and 16 (output, at most 256), the pair kernel on the FP32
-    pipes for fp32 and all other widths.  None when the operands are in no native dtype (the caller then uses a
+    tensor cores for fp16 / bf16 widths of 16 and more that are multiples of 8 (input) and 16 (output, at most 256) and for
+    fp32 over many offsets (as sums of three bf16 numbers), the pair kernel on the FP32 pipes for everything else.  None when the operands are in no native dtype (the caller then uses a
     GEMM per offset)."""
     require_cuda(in_features, "in_features")
     x, g = in_features.contiguous(), grad_output.contiguous()
@@ -853,6 +853,21 @@ def sparse_conv_wgrad(in_features: Tensor, grad_output: Tensor, kernel_map: IntS
         nbr, out_rows = kernel_map.tiled_neighbor_table(num_out_coords)
     else:
         nbr, out_rows = kernel_map.neighbor_table(num_out_coords), None
+    if x.dtype == torch.float32 and x.data_ptr() % 16 == 0 and g.data_ptr() % 16 == 0:
+        nbytes = query_bytes("wcn_conv_wgrad_f32_workspace_bytes", x.shape[0], num_out_coords, K, c_in, c_out)
+        ws = None
+        if nbytes:
+            try:
+                ws = torch.empty(nbytes, dtype=torch.uint8, device=dev)
+            except torch.cuda.OutOfMemoryError:  # three times the features: the FP32 pipes need less
+                pass
+        if ws is not None:
+            masks = kernel_map.tile_masks(num_out_coords, tiled)
+            gw = torch.empty((K, c_in, c_out), dtype=torch.float32, device=dev)
+            check(lib().wcn_conv_wgrad_f32(ptr(x), x.shape[0], ptr(g), ptr(nbr), ptr(out_rows), ptr(masks), num_out_coords, K, c_in,
+                                           c_out, ptr(gw), ptr(ws), nbytes, ptr(device_status(dev)), stream_ptr(dev)),
+                  "wcn_conv_wgrad_f32")
+            return gw
     if x.dtype == torch.float32 or c_in < 16 or c_in % 8 or c_out % 16 or c_out > 256 or K > 32:
         gw = torch.empty((K, c_in, c_out), dtype=torch.float32, device=dev)
         nbytes = query_bytes("wcn_conv_wgrad_pairs_workspace_bytes", num_out_coords, K, c_in, c_out)
