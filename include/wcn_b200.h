@@ -557,6 +557,12 @@ typedef struct { const int32_t* nbr; const int32_t* out_rows; } wcn_net_table;
 int wcn_net_run(const wcn_net_op* ops, int32_t num_ops, const int64_t* rows, const wcn_net_buffer* buffers,
                 const wcn_net_table* tables, int dtype, int32_t* dev_status, void* stream);
 
+/* sums[j] = sum of column j of x [n, channels] (contiguous 16-byte aligned rows that are whole 16-byte pieces, 4096 bytes at
+ * most; fp32 sums, the same bits on every run): the gradient of a layer's bias.  workspace: the bytes that the query gives
+ * (0: not taken).  Stands for the reduction that autograd makes of sparse_conv.py:1794-1795. */
+int wcn_column_sums_workspace_bytes(int64_t n, int32_t channels, int dtype, int64_t* bytes);
+int wcn_column_sums(const void* x, int64_t n, int32_t channels, int dtype, float* sums, void* workspace, void* stream);
+
 /* ------------------------------------------------------------------ batch normalisation in training */
 
 /* y = relu(batch_norm(x) + residual) of [n, channels] rows (residual, relu optional), rounded to the dtype after the

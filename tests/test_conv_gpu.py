@@ -906,6 +906,58 @@ def test_fp32_weight_gradient_on_the_tensor_cores(K, n, num_in, c_in, c_out):
     check_device_status(DEV)
 
 
+@pytest.mark.parametrize("dtype", [torch.float32, torch.float16, torch.bfloat16])
+@pytest.mark.parametrize("n,c", [(1, 8), (5, 24), (1023, 64), (70001, 96), (3000, 1000), (300, 7)])
+def test_column_sums(dtype, n, c):
+    """Fewer rows than a block takes at once, columns that do not divide a block, widths without a kernel: against 64 bits
+    (fp32 sums of some hundred numbers, added in double), twice the same bits."""
+    from warpconvnet_b200.nn.functional.sparse_conv import _column_sums
+    x = torch.randn(n, c, generator=torch.Generator(device=DEV).manual_seed(n), device=DEV).to(dtype)
+    got, want = _column_sums(x), x.double().sum(0)
+    assert torch.equal(got, _column_sums(x))
+    assert float((got.double() - want).abs().max()) <= 1e-6 * float(x.double().abs().sum(0).max())
+
+
+@pytest.mark.parametrize("dtype,bias_dtype", [(torch.float32, torch.float32), (torch.float16, torch.float16), (torch.bfloat16, torch.float32)])
+@pytest.mark.parametrize("kind", ["same", "down", "up"])
+def test_bias_of_a_training_layer(dtype, bias_dtype, kind):
+    """The bias as part of the layer's node: forward and all gradients against the node without it and an addition; a graph of
+    the bias gradient, and forward-mode tangents of the bias, go through torch as before."""
+    coords = room_rows(5000)
+    vox = make_voxels(coords, torch.randn(len(coords), 32, generator=torch.Generator().manual_seed(1)).to(dtype)).sort()
+    torch.manual_seed(0)
+    down = SparseConv3d(32, 48, 2, stride=2, bias=True).to(DEV).to(dtype)
+    layer = {"same": SparseConv3d(32, 48, 3, bias=True), "down": down, "up": SparseConv3d(48, 32, 2, stride=2, bias=True, transposed=True)}[kind]
+    layer = layer.to(DEV).to(dtype)
+    layer.bias.data = torch.randn(layer.bias.shape, device=DEV).to(bias_dtype)
+    if kind == "up":
+        with torch.no_grad():
+            vox, target = down(vox), vox
+    call = (lambda v: layer(v, target)) if kind == "up" else layer
+    outs = []
+    for fused in (True, False):
+        x = vox.feature_tensor.detach().clone().requires_grad_(True)
+        bias = layer.bias
+        if not fused:
+            layer.bias = None
+        y = call(vox.replace(batched_features=x)).feature_tensor
+        if not fused:
+            y = (y.double() + bias.double()).to(dtype)
+            layer.bias = bias
+        dy = torch.randn(y.shape, generator=torch.Generator(device=DEV).manual_seed(2), device=DEV).to(dtype)
+        outs.append([y.detach(), *torch.autograd.grad(y, [x, layer.weight, bias], dy)])
+    tol = {torch.float32: 1e-6, torch.float16: 2e-3, torch.bfloat16: 1e-2}[dtype]
+    for got, want in zip(*outs):
+        assert got.dtype == want.dtype and rel_l2(got.float().cpu().numpy(), want.float().cpu().numpy()) < tol
+    x = vox.feature_tensor.detach().clone().requires_grad_(True)
+    y = call(vox.replace(batched_features=x)).feature_tensor
+    dy = torch.ones_like(y).requires_grad_(True)
+    (gb,) = torch.autograd.grad(y, [layer.bias], dy, create_graph=True)
+    (back,) = torch.autograd.grad(gb.sum(), [dy])
+    assert torch.equal(back, torch.ones_like(back))
+    check_device_status(DEV)
+
+
 @pytest.mark.parametrize("n", [12000, 19000])
 @pytest.mark.parametrize("where,value", [("x", float("inf")), ("x", float("nan")), ("x", 3.4e38), ("w", float("-inf")), ("w", 2.0 ** 64)])
 def test_fp32_numbers_without_three_parts(n, where, value, monkeypatch):

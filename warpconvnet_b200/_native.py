@@ -68,6 +68,8 @@ SIGNATURES = {
     "wcn_conv_f32_workspace_bytes": [_c_i64, _c_i64, _c_i32, _c_i32, _c_i32, _p_i64],
     "wcn_conv_fwd": [_c_i32, _c_vp, _c_i64, _c_i64, _c_vp, _c_vp, _c_vp, _c_vp, _c_i64, _c_i32, _c_i32, _c_i32, _c_i32,
                      _c_vp, _c_vp, _c_vp, _c_i64, _c_i32, _c_vp, _c_i64, _c_i32, _c_i32, _c_vp, _c_i64, _c_vp, _c_vp],
+    "wcn_column_sums_workspace_bytes": [_c_i64, _c_i32, _c_i32, _p_i64],
+    "wcn_column_sums": [_c_vp, _c_i64, _c_i32, _c_i32, _c_vp, _c_vp, _c_vp],
     "wcn_batch_norm_workspace_bytes": [_c_i64, _c_i32, _c_i32, _p_i64],
     "wcn_batch_norm_train": [_c_vp, _c_i64, _c_i32, _c_i32, _c_vp, _c_vp, _c_i32, _c_i32, _c_vp, _c_vp, _c_vp, _c_vp, _c_i32,
                              _c_vp, _c_vp, _c_vp, _c_vp, _c_vp, _c_vp],
@@ -117,7 +119,7 @@ KERNELS_PER_CALL = {
     "wcn_kmap_tile_order": 3, "wcn_conv_wgrad": 1, "wcn_conv_wgrad_pairs": 2, "wcn_conv_wgrad_f32": 3, "wcn_kmap_tile_masks": 1, "wcn_row_reduce": 1, "wcn_row_reduce_train": 1, "wcn_row_reduce_backward": 1, "wcn_kmap_search_self": 1, "wcn_kmap_search_dilated": 1, "wcn_kmap_count": 1,
     "wcn_gather_rows": 1, "wcn_scatter_add_rows": 1, "wcn_conv_pack_weight": 1, "wcn_conv_fwd": 1,
     "wcn_selftest_bounded_wait": 1, "wcn_brick_build": 3, "wcn_kmap_search_bricks": 1,
-    "wcn_conv_rows_fwd": 1, "wcn_batch_norm_train": 2, "wcn_batch_norm_backward": 2, "wcn_conv_pack_weight_from": 1, "wcn_cells_build": 4, "wcn_kmap_search_cells": 1, "wcn_kmap_scan_host": 2, "wcn_unique_counts": 2, "wcn_morton_sort": 1, "wcn_pyramid": 2, "wcn_level_maps": 5,
+    "wcn_conv_rows_fwd": 1, "wcn_batch_norm_train": 2, "wcn_column_sums": 2, "wcn_batch_norm_backward": 2, "wcn_conv_pack_weight_from": 1, "wcn_cells_build": 4, "wcn_kmap_search_cells": 1, "wcn_kmap_scan_host": 2, "wcn_unique_counts": 2, "wcn_morton_sort": 1, "wcn_pyramid": 2, "wcn_level_maps": 5,
 }
 LAUNCH_COUNTS: Counter = Counter()
 

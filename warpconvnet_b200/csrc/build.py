@@ -9,7 +9,7 @@ import sys
 import sysconfig
 
 HERE = os.path.dirname(os.path.abspath(__file__))
-SOURCES = ["api.cu", "hash_kmap.cu", "brick_kmap.cu", "cell_kmap.cu", "morton_sort.cu", "level_maps.cu", "net_run.cu", "conv_explicit.cu", "row_reduce.cu", "batch_norm.cu", "conv_simt.cu", "conv_fp32.cu", "conv_split_tcgen05.cu", "conv_tcgen05.cu",
+SOURCES = ["api.cu", "hash_kmap.cu", "brick_kmap.cu", "cell_kmap.cu", "morton_sort.cu", "level_maps.cu", "net_run.cu", "conv_explicit.cu", "row_reduce.cu", "batch_norm.cu", "column_sums.cu", "conv_simt.cu", "conv_fp32.cu", "conv_split_tcgen05.cu", "conv_tcgen05.cu",
            "conv_wgrad_tcgen05.cu", "conv_wgrad_split_tcgen05.cu", "conv_wgrad_pairs.cu", "conv_rows_tcgen05.cu"]
 HEADERS = ["wcn_common.cuh", "tile_order.cuh", "tcgen05_common.cuh", "split_bf16.cuh", os.path.join("..", "..", "include", "wcn_b200.h")]
 LIB = os.path.join(HERE, "libwcn_b200.so")

@@ -1341,6 +1341,41 @@ class _LayerFunction(torch.autograd.Function):
         return gx, gw, None
 
 
+def _column_sums(g: Tensor) -> Tensor:
+    """``g.sum(0)`` in fp32 of contiguous rows."""
+    n, c = g.shape
+    nbytes = query_bytes("wcn_column_sums_workspace_bytes", n, c, dtype_code(g.dtype)) if g.data_ptr() % 16 == 0 else 0
+    if not nbytes:
+        return g.sum(0, dtype=torch.float32)
+    sums = torch.empty(c, dtype=torch.float32, device=g.device)
+    ws = torch.empty(nbytes, dtype=torch.uint8, device=g.device)
+    check(lib().wcn_column_sums(g.data_ptr(), n, c, dtype_code(g.dtype), sums.data_ptr(), ws.data_ptr(), stream_ptr(g.device)),
+          "wcn_column_sums")
+    return sums
+
+
+class _LayerBiasFunction(torch.autograd.Function):
+    """A layer in training with its bias, which the convolution's epilogue adds: beside :class:`_LayerFunction` that was an
+    addition and a reduction through torch, 38 us of the 270 that a layer of 60 000 fp32 rows of 64 channels takes."""
+
+    @staticmethod
+    def forward(ctx, x: Tensor, weight: Tensor, bias: Tensor, tables: _LayerTables):
+        ctx.tables, ctx.bias_dtype = tables, bias.dtype
+        ctx.save_for_backward(x, weight)
+        return _layer_output(x.detach(), weight, tables, bias.detach())
+
+    @staticmethod
+    def backward(ctx, g: Tensor):
+        x, weight = ctx.saved_tensors
+        need_x, need_w, need_b = ctx.needs_input_grad[:3]
+        gx, gw = _layer_gradients(g, x, weight, ctx.tables, need_x, need_w) if need_x or need_w else (None, None)
+        gb = None
+        if need_b:  # (through torch where a graph of the gradient is wanted)
+            gb = g.sum(0, dtype=torch.float32) if torch.is_grad_enabled() else _column_sums(g.contiguous())
+            gb = gb.to(ctx.bias_dtype)
+        return gx, gw, gb, None
+
+
 class _LayerNormFunction(torch.autograd.Function):
     """A layer in training with the BatchNorm, residual and ReLU behind it: one node of the graph for what is two
     otherwise (a node costs the host about 60 us a step, as much as its launches)."""
@@ -1367,10 +1402,10 @@ class _LayerNormFunction(torch.autograd.Function):
         return gx, gw, sums[1] if need[2] else None, sums[0] if need[3] else None, dres, None, None, None
 
 
-def _layer_output(x: Tensor, weight: Tensor, t: _LayerTables) -> Tensor:
+def _layer_output(x: Tensor, weight: Tensor, t: _LayerTables, bias: Optional[Tensor] = None) -> Tensor:
     if t.nbr is None:
-        return sparse_conv_fused(x, weight, t.km, t.num_out)
-    return _launch_layer(x, weight, t, False, t.num_out)
+        return sparse_conv_fused(x, weight, t.km, t.num_out, None if bias is None else ConvEpilogue(shift=bias))
+    return _launch_layer(x, weight, t, False, t.num_out, bias)
 
 
 def _layer_gradients(g: Tensor, x: Tensor, weight: Tensor, t: _LayerTables, need_x: bool, need_w: bool):
@@ -1392,8 +1427,8 @@ def _layer_gradients(g: Tensor, x: Tensor, weight: Tensor, t: _LayerTables, need
     return gx, gw
 
 
-def _launch_layer(x: Tensor, weight: Tensor, t: _LayerTables, gradient: bool, rows: int) -> Tensor:
-    """One launch over the tables of a layer, with its weights or (``gradient``) with each offset's weight transposed
+def _launch_layer(x: Tensor, weight: Tensor, t: _LayerTables, gradient: bool, rows: int, bias: Optional[Tensor] = None) -> Tensor:
+    """One launch over the tables of a layer (``bias`` added), with its weights or (``gradient``) with each offset's weight transposed
     and the offsets in reverse order."""
     if x.stride(1) != 1:
         x = x.contiguous()
@@ -1406,8 +1441,9 @@ def _launch_layer(x: Tensor, weight: Tensor, t: _LayerTables, gradient: bool, ro
     out = torch.empty((rows, c_out), dtype=x.dtype, device=x.device)
     dc = dtype_code(x.dtype)
     workspace, workspace_bytes = _f32_workspace(x, rows, K, c_in, c_out)
+    shift = _as_f32_on(bias, x.device)
     rc = lib().wcn_conv_fwd(CONV_AUTO, x.data_ptr(), x.shape[0], x.stride(0), ptr(w), ptr(packed), t.nbr.data_ptr(),
-                            ptr(t.out_rows), rows, K, c_in, c_out, dc, None, None, None, 0, 0, out.data_ptr(), c_out, dc, 0,
+                            ptr(t.out_rows), rows, K, c_in, c_out, dc, None, ptr(shift), None, 0, 0, out.data_ptr(), c_out, dc, 0,
                             ptr(workspace), workspace_bytes, device_status(x.device).data_ptr(), stream_ptr(x.device))
     if rc != 0:
         check(rc, "wcn_conv_fwd")
@@ -1459,7 +1495,11 @@ def train_layer(layer, x: Voxels, target: Optional[Voxels]) -> Optional[Voxels]:
         found = _training_tables(layer, x, target, feats)
         if found is None:
             return None
-        y = _LayerFunction.apply(feats, weight, found[0])
+        if (bias is not None and bias.dim() == 1 and bias.shape[0] == weight.shape[2] and bias.device == feats.device
+                and bias.dtype in _NATIVE_DTYPES and batch_norm.reverse_mode_only()):
+            y, bias = _LayerBiasFunction.apply(feats, weight, bias, found[0]), None
+        else:
+            y = _LayerFunction.apply(feats, weight, found[0])
     if bias is not None:
         y = y + bias.to(y.dtype)
     return x._derive(y) if pointwise else _output_of(layer, x, *found, y)
