@@ -11,15 +11,18 @@
 // pair does not exist).  So
 //   * the rows of X arrive as 128 x BK tiles through TMA (cp.async.bulk.tensor, hardware swizzle),
 //     each row read once per weight chunk instead of once per output row that needs it;
-//   * the weights of a chunk of offsets (up to 256 output columns) stay in shared memory across
+//   * the weights of a chunk of offsets (up to 128 output columns, or one offset) stay in shared memory across
 //     all row tiles a CTA processes; the chunk of the next unit is loaded behind the current one;
 //   * accumulators are two to four sets of up to 256 TMEM columns, so the epilogues of the previous
 //     tiles (whose latency is a table lookup, a TMEM load and scattered stores) overlap the MMAs of
 //     the next ones;
-//   * eight epilogue warps read TMEM, apply scale / shift / residual / ReLU and store each
+//   * twelve epilogue warps read TMEM, apply scale / shift / residual / ReLU and store each
 //     C_out-wide block at its destination row.
 // Work unit = (chunk of offsets, row tile); units are numbered chunk-major and dealt round-robin to
 // a persistent grid, so a CTA changes its weight chunk only a few times on large inputs.
+//
+// What bounds it is the latency of the epilogue's steps: with eight warps and chunks of up to 256 columns the transposed layer
+// 96 -> 96 from 75 000 to 300 000 rows took 32.0 us, with twelve and 128 28.8 (eight and 128: 31.8; sixteen: 38).
 //
 // Every wait is bounded (tcgen05_common.cuh); a kernel that gives up sets the status word, drains
 // its copies and frees its tensor memory.
@@ -33,9 +36,10 @@ constexpr int BLOCK_M = 128;
 constexpr int MAX_STAGES = 24;         // row-tile ring: up to 192 KB in flight per multiprocessor
 constexpr int MAX_Q = 8;               // offsets per chunk
 constexpr int MAX_ACC = 4;             // accumulator sets in tensor memory
-constexpr int PRODUCER_WARP = 0, MMA_WARP = 1, EPI_WARP0 = 2, EPI_WARPS = 8;
+constexpr int PRODUCER_WARP = 0, MMA_WARP = 1, EPI_WARP0 = 2, EPI_WARPS = 12;
 constexpr int THREADS = (EPI_WARP0 + EPI_WARPS) * 32;
-constexpr int MAX_COLS = 256;          // output columns of one chunk (one MMA's N)
+constexpr int MAX_COLS = 256;          // output columns of one offset (one MMA's N)
+constexpr int CHUNK_COLS = 128;        // output columns of a chunk of several: four accumulator sets fit in tensor memory
 constexpr int SMEM_BUDGET = 220 * 1024;
 
 struct RowsParams {
@@ -202,7 +206,7 @@ conv_rows_tcgen05_kernel(const __grid_constant__ CUtensorMap feats_map, const Ro
     }
     for (int i = 0; i < MAX_ACC; ++i) {
       mbar_init(bar(&ctl->acc_full[i]), 1);
-      mbar_init(bar(&ctl->acc_empty[i]), EPI_WARPS / 2);   // the four warps that finish a given unit
+      mbar_init(bar(&ctl->acc_empty[i]), 4);   // the four warps that finish a given unit
     }
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     asm volatile("prefetch.tensormap [%0];" ::"l"(reinterpret_cast<uint64_t>(&feats_map)) : "memory");
@@ -307,14 +311,15 @@ conv_rows_tcgen05_kernel(const __grid_constant__ CUtensorMap feats_map, const Ro
     }
     __syncwarp();
   } else {
-    // ================================================================ epilogue (8 warps)
-    // TMEM lanes 32*(warp % 4).. belong to this warp.  The two warps of a lane quarter take
-    // alternate units: what an epilogue pays per unit besides the data (barrier round trip, table
-    // lookup, loop control) then overlaps between the two, and four accumulator sets keep both fed.
+    // ================================================================ epilogue (12 warps)
+    // TMEM lanes 32*(warp % 4).. belong to this warp.  The three warps of a lane quarter take
+    // units in turns: what an epilogue pays per unit besides the data (barrier round trip, table
+    // lookup, loop control) then overlaps between them, and four accumulator sets keep them fed (where
+    // only two fit, two of the warps take part: a wait may be one phase ahead, not two).
     wait_for_primary();
     // (a launch that overlaps the one before it may have started before that one failed: looked at again when done)
     if (tid == EPI_WARP0 * 32) ctl->skip = *(volatile const int32_t*)p.dev_status;
-    const int ew = warp - EPI_WARP0, quarter = warp & 3, half = ew >> 2;
+    const int ew = warp - EPI_WARP0, quarter = warp & 3, team = ew >> 2, teams = min(EPI_WARPS / 4, p.nacc);
     const bool affine = p.scale != nullptr || p.shift != nullptr;
     const int pieces = p.c_out >> 4;
     bool bad = false;
@@ -338,8 +343,9 @@ conv_rows_tcgen05_kernel(const __grid_constant__ CUtensorMap feats_map, const Ro
     // ahead: the table comes from DRAM and its latency would otherwise sit between every
     // accumulator set and its stores.
     UnitCursor cur = first;
-    if (half) cur.advance(grid, tiles);
-    int ab = half % p.nacc, aphase = 0;   // local unit n uses set n % nacc in phase (n / nacc) & 1
+    cur.advance(team * grid, tiles);
+    if (team >= teams) cur.chunk = p.nchunks;
+    int ab = team, aphase = 0;   // local unit n uses set n % nacc in phase (n / nacc) & 1
     int dnext[MAX_Q];
 #pragma unroll
     for (int o = 0; o < MAX_Q; ++o) dnext[o] = -1;
@@ -359,7 +365,7 @@ conv_rows_tcgen05_kernel(const __grid_constant__ CUtensorMap feats_map, const Ro
 #pragma unroll
       for (int o = 0; o < MAX_Q; ++o) dsts[o] = dnext[o];
       UnitCursor nxt = cur;
-      nxt.advance(2 * grid, tiles);
+      nxt.advance(teams * grid, tiles);
       if (nxt.chunk < p.nchunks) load_dsts(nxt);
       if (ok) ok = mbar_wait(bar(&ctl->acc_full[ab]), aphase, p.dev_status);
       if (!__all_sync(0xFFFFFFFFu, ok)) { ok = false; break; }  // tcgen05.ld is warp-collective
@@ -390,7 +396,7 @@ conv_rows_tcgen05_kernel(const __grid_constant__ CUtensorMap feats_map, const Ro
       tc_fence_before();
       __syncwarp();
       if (lane == 0) mbar_arrive(bar(&ctl->acc_empty[ab]));
-      ab += 2;
+      ab += teams;
       while (ab >= p.nacc) { ab -= p.nacc; aphase ^= 1; }
       cur = nxt;
     }
@@ -413,7 +419,8 @@ bool plan_rows(int K, int c_in, int c_out, RowsParams* p, size_t* smem) {
   const int a_bytes = BLOCK_M * bk * 2;
   const int64_t per_offset = (int64_t)c_in * c_out * 2;
   const int fixed = (int)sizeof(RowsControl) + 1024;
-  int q = MAX_COLS / c_out < K ? MAX_COLS / c_out : K, nbuf = 0;
+  int q = CHUNK_COLS / c_out < K ? CHUNK_COLS / c_out : K, nbuf = 0;
+  if (q < 1) q = 1;
   if (q > MAX_Q) q = MAX_Q;
   for (; q >= 1; --q) {
     const int nchunks = (K + q - 1) / q;
