@@ -60,8 +60,9 @@ class PyramidBuild:
             return None
         sizes = [host[(l + 1) * nb - 1] for l in range(PYRAMID_LEVELS)]
         if self.n >= TRIMMED_ROWS:
-            self.out = [self.out[l, :m].clone() for l, m in enumerate(sizes)]
+            outs = [self.out[l, :m].clone() for l, m in enumerate(sizes)]
             self.first = [self.first[l, :m].clone() for l, m in enumerate(sizes)]
+            self.out = outs
         # where each level's rows and first children start
         trimmed = isinstance(self.out, list)
         self.out_ptr = [self.out[l].data_ptr() if trimmed else self.out.data_ptr() + 16 * l * self.n for l in range(PYRAMID_LEVELS)]
@@ -134,32 +135,46 @@ class LevelMaps:
             self._enqueue(range(1))
 
     def _enqueue(self, which) -> None:
-        """The maps of some levels, all in one piece of memory (an allocation costs the host 2 us, a view as much)."""
-        b = self.build
+        """The maps of some levels: of one level as tensors of their own, of several in one piece of memory (an allocation
+        costs the host 2 us, a view as much), of which :meth:`_tensors` makes views."""
+        b, dev = self.build, self.build.device
         levels = (Level * len(which))()
-        total = bricks = 0
-        places = []
-        for l in which:
-            n = self.n[l]
-            words = -(-n // 64) * 64   # every table starts on a 256-byte boundary
-            tiled = n >= self.min_rows
-            places.append((l, n, total, total + 27 * words if tiled else None, total + 28 * words if l else None, bricks))
-            total += (28 + (8 if l else 0)) * words
-            bricks += -(-query_bytes("wcn_level_brick_bytes", n) // 256) * 256
-        memory = torch.empty(total, dtype=torch.int32, device=b.device)
-        scratch = self._bricks = torch.empty(bricks, dtype=torch.uint8, device=b.device)
-        base, brick_base = memory.data_ptr(), scratch.data_ptr()
-        for slot, (l, n, nbr, order, child, brick) in zip(levels, places):
-            at = self.at[l] = (base + 4 * nbr, None if order is None else base + 4 * order, None if child is None else base + 4 * child)
-            slot.rows, slot.n, slot.level = self._row_ptr(l), n, l
-            slot.bricks, slot.order, slot.nbr = brick_base + brick, at[1], at[0]
+        if len(which) == 1:
+            l, n = which[0], self.n[which[0]]
+            nbr = self.nbr[l] = torch.empty((27, n), dtype=torch.int32, device=dev)
+            order = self.order[l] = torch.empty(n, dtype=torch.int32, device=dev) if n >= self.min_rows else None
+            bricks = self._bricks = torch.empty(query_bytes("wcn_level_brick_bytes", n), dtype=torch.uint8, device=dev)
+            child = None
             if l:
-                slot.child = at[2]
+                child = self.child[l - 1] = torch.empty((8, n), dtype=torch.int32, device=dev)
+            self.at[l] = (nbr.data_ptr(), ptr(order), ptr(child))
+            brick_at = [bricks.data_ptr()]
+        else:
+            total = bytes_ = 0
+            places, brick_at = [], []
+            for l in which:
+                n = self.n[l]
+                words = -(-n // 64) * 64   # every table starts on a 256-byte boundary
+                places.append((l, n, total, total + 27 * words if n >= self.min_rows else None, total + 28 * words if l else None))
+                total += (28 + (8 if l else 0)) * words
+                brick_at.append(bytes_)
+                bytes_ += -(-query_bytes("wcn_level_brick_bytes", n) // 256) * 256
+            memory = torch.empty(total, dtype=torch.int32, device=dev)
+            bricks = self._bricks = torch.empty(bytes_, dtype=torch.uint8, device=dev)
+            base = memory.data_ptr()
+            brick_at = [bricks.data_ptr() + v for v in brick_at]
+            for l, _, *tables in places:
+                self.at[l] = tuple(None if v is None else base + 4 * v for v in tables)
+            self._made.append((memory, places))
+        for slot, l, brick in zip(levels, which, brick_at):
+            slot.rows, slot.n, slot.level = self._row_ptr(l), self.n[l], l
+            slot.nbr, slot.order, slot.child = self.at[l]
+            slot.bricks = brick
+            if l:
                 slot.first_child = b.first_ptr[l - 1] if b.first_ptr else b.first[l - 1].data_ptr()
                 slot.rows_below, slot.n_below = self._row_ptr(l - 1), self.n[l - 1]
         check(lib().wcn_level_maps(ctypes.addressof(levels), len(which), ptr(b.info), ptr(b.counts),
-                                   self.small_window_rows, stream_ptr(b.device)), "wcn_level_maps")
-        self._made.append((memory, places))
+                                   self.small_window_rows, stream_ptr(dev)), "wcn_level_maps")
 
     def _row_ptr(self, l: int) -> int:
         return self.rows[l].data_ptr() if l < len(self.rows) else self.build.out_ptr[l - 1]
@@ -168,7 +183,7 @@ class LevelMaps:
         """The tables that have been enqueued as tensors."""
         self.at = {}   # (addresses would be wrong in a copy)
         for memory, places in self._made:
-            for l, n, nbr, order, child, _ in places:
+            for l, n, nbr, order, child in places:
                 self.nbr[l] = memory[nbr:nbr + 27 * n].view(27, n)
                 self.order[l] = None if order is None else memory[order:order + n]
                 if child is not None:
