@@ -1,5 +1,6 @@
 // Output-stationary sparse convolution of fp32 tensors: gathered rows times weights on the FP32 pipes, with the
-// absent neighbours left out.
+// absent neighbours left out.  For widths that conv_split_tcgen05.cu does not take, more than 27 offsets, calls without
+// workspace, and the problems that are done here before that kernel's two launches are (few rows of narrow layers, one offset).
 //
 // Bound by FMA issue where neighbours are dense and by latency where they are few.  A block owns TM output rows x TN
 // columns.  Per kernel offset the rows of the tile that have a neighbour are listed (ballots over the table column),

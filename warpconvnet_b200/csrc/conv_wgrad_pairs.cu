@@ -1,5 +1,5 @@
-// Weight gradient of the sparse convolution on the FP32 pipes, for fp32 tensors and for widths the tensor-core kernel
-// does not take (a 3-channel stem, odd widths):
+// Weight gradient of the sparse convolution on the FP32 pipes, for fp32 tensors that conv_wgrad_split_tcgen05.cu does not take
+// (few offsets, narrow layers) and for widths the tensor-core kernels do not take (a 3-channel stem, odd widths):
 //     dW[k][ci][co] = sum over rows m with a neighbour at offset k of X[nbr[k][m]][ci] * dY[m][co].
 //
 // Bound by FMA issue.  A block owns one offset, a TI x TJ tile of its matrix and a range of rows.  It lists the rows
