@@ -1,0 +1,180 @@
+"""GPU tests of the fp32 layers' tensor-core kernels, of a training layer's bias and of the order in which the
+half-precision convolution takes its units."""
+import pytest
+import torch
+
+from warpconvnet_b200 import ConvEpilogue, IntSearchResult, SparseConv3d
+from warpconvnet_b200._native import CONV_SIMT, CONV_TCGEN05, check_device_status
+from warpconvnet_b200.nn.functional.sparse_conv import sparse_conv_fused
+
+from conftest import rel_l2
+from test_conv_gpu import make_voxels, room_rows
+
+pytestmark = pytest.mark.gpu
+DEV = "cuda:0"
+
+
+def _random_map(K, n, num_in, g):
+    present = torch.rand(K, n, generator=g, device=DEV) < torch.rand(n, generator=g, device=DEV) ** 2
+    nbr = torch.randint(0, num_in, (K, n), generator=g, device=DEV, dtype=torch.int32)
+    return IntSearchResult.from_neighbor_table(torch.where(present, nbr, torch.full((), -1, dtype=torch.int32, device=DEV)), num_in)
+
+
+@pytest.mark.parametrize("K,n,num_in,c_in,c_out", [(27, 1, 1, 64, 32), (27, 129, 500, 52, 48), (8, 2000, 4000, 36, 144), (8, 700, 700, 32, 32), (1, 13000, 13000, 128, 96), (27, 300, 300, 64, 64), (27, 14000, 14000, 20, 16),
+                                                   (27, 9472, 9000, 32, 128), (27, 9473, 9473, 96, 112), (27, 18945, 18945, 32, 32),
+                                                   (27, 70000, 70000, 64, 64), (3, 700, 600, 160, 256)])
+def test_fp32_on_the_tensor_cores_is_closer_to_exact_sums(K, n, num_in, c_in, c_out):
+    """Offsets divided among a cluster and not, whole and partial row tiles, column blocks, channels that do not fill a
+    slice, rows apart, every part of the epilogue: against sums in 64 bits.  What is dropped of a product is below 2^-25
+    of it and an accumulator adds 32 channels before it is rounded: 3e-7 is twice the largest error measured."""
+    g = torch.Generator(device=DEV).manual_seed(n)
+    kmap = _random_map(K, n, num_in, g)
+    nbr = kmap.neighbor_table(n)
+    wide = torch.randn(num_in, c_in + 4, generator=g, device=DEV)
+    x = wide[:, 4:]
+    w = torch.randn(K, c_in, c_out, generator=g, device=DEV) * (K * c_in) ** -0.5
+    res, scale, shift = torch.randn(n, c_out, generator=g, device=DEV), torch.rand(c_out, generator=g, device=DEV) + 0.5, torch.randn(c_out, generator=g, device=DEV)
+    want = torch.zeros(n, c_out, dtype=torch.float64, device=DEV)
+    for k in range(K):
+        m = (nbr[k] >= 0).nonzero()[:, 0]
+        want[m] += x[nbr[k, m].long()].double() @ w[k].double()
+    got = sparse_conv_fused(x, w, kmap, n)
+    again = sparse_conv_fused(x, w, kmap, n, tile_order=True)
+    simt = sparse_conv_fused(x, w, kmap, n, algo=CONV_SIMT)
+    check_device_status(DEV)
+    error = lambda y: float((y.double() - want).norm() / want.norm().clamp(min=1e-30))
+    assert error(got) < 3e-7 and error(again) < 3e-7
+    if n * c_out > 30000:
+        assert error(got) <= error(simt)
+    full = sparse_conv_fused(x, w, kmap, n, epilogue=ConvEpilogue(scale=scale, shift=shift, residual=res, relu=True))
+    want = (want * scale.double() + shift.double() + res.double()).clamp(min=0)
+    assert error(full) < 3e-7
+    check_device_status(DEV)
+
+
+@pytest.mark.parametrize("K,n,num_in,c_in,c_out", [(27, 1, 1, 64, 32), (27, 129, 90, 52, 48), (16, 4000, 6000, 36, 132), (32, 700, 700, 160, 16),
+                                                   (27, 5000, 5000, 96, 64), (27, 70000, 70000, 64, 64), (27, 66000, 66000, 128, 256)])
+def test_fp32_weight_gradient_on_the_tensor_cores(K, n, num_in, c_in, c_out):
+    """Groups that end inside an offset and past the last, partial tiles, one range and many, column blocks: against sums
+    in 64 bits (4e-7 is twice the largest error measured), closer to them than the FP32 pipes, twice the same bits."""
+    from warpconvnet_b200.nn.functional import sparse_conv as sc
+    g = torch.Generator(device=DEV).manual_seed(n)
+    kmap = _random_map(K, n, num_in, g)
+    nbr = kmap.neighbor_table(n)
+    x, dy = torch.randn(num_in, c_in, generator=g, device=DEV), torch.randn(n, c_out, generator=g, device=DEV)
+    want = torch.stack([x[nbr[k].clamp(min=0).long()].double().mul((nbr[k] >= 0)[:, None]).T @ dy.double() for k in range(K)])
+    error = lambda y: float((y.double() - want).norm() / want.norm().clamp(min=1e-30))
+    for tiled in (False, K <= 27):
+        got = [sc.sparse_conv_wgrad(x, dy, kmap, n, tile_order=tiled) for _ in range(2)]
+        check_device_status(DEV)
+        assert torch.equal(*got) and error(got[0]) < 4e-7
+    with pytest.MonkeyPatch.context() as m:
+        query = sc.query_bytes
+        m.setattr(sc, "query_bytes", lambda name, *a: 0 if name == "wcn_conv_wgrad_f32_workspace_bytes" else query(name, *a))
+        pipes = sc.sparse_conv_wgrad(x, dy, kmap, n)
+        assert n < 1000 or error(got[0]) <= error(pipes)
+        for value, row in ((float("inf"), 0), (float("nan"), n // 2), (1e30, n - 1)):
+            bad = dy.clone()
+            bad[row, 3] = value
+            want_bad = sc.sparse_conv_wgrad(x, bad, kmap, n)
+            with pytest.MonkeyPatch.context() as back:
+                back.setattr(sc, "query_bytes", query)
+                got_bad = sc.sparse_conv_wgrad(x, bad, kmap, n)
+            assert torch.equal(torch.isfinite(got_bad), torch.isfinite(want_bad))
+            fine = torch.isfinite(want_bad)
+            assert not fine.any() or rel_l2(got_bad[fine].cpu().numpy(), want_bad[fine].cpu().numpy()) < 1e-5
+    check_device_status(DEV)
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.float16, torch.bfloat16])
+@pytest.mark.parametrize("n,c", [(1, 8), (5, 24), (1023, 64), (70001, 96), (3000, 1000), (300, 7)])
+def test_column_sums(dtype, n, c):
+    """Fewer rows than a block takes at once, columns that do not divide a block, widths without a kernel: against 64 bits
+    (fp32 sums of some hundred numbers, added in double), twice the same bits."""
+    from warpconvnet_b200.nn.functional.sparse_conv import _column_sums
+    x = torch.randn(n, c, generator=torch.Generator(device=DEV).manual_seed(n), device=DEV).to(dtype)
+    got, want = _column_sums(x), x.double().sum(0)
+    assert torch.equal(got, _column_sums(x))
+    assert float((got.double() - want).abs().max()) <= 1e-6 * float(x.double().abs().sum(0).max())
+
+
+@pytest.mark.parametrize("dtype,bias_dtype", [(torch.float32, torch.float32), (torch.float16, torch.float16), (torch.bfloat16, torch.float32)])
+@pytest.mark.parametrize("kind", ["same", "down", "up"])
+def test_bias_of_a_training_layer(dtype, bias_dtype, kind):
+    """The bias as part of the layer's node: forward and all gradients against the node without it and an addition; a graph of
+    the bias gradient, and forward-mode tangents of the bias, go through torch as before."""
+    coords = room_rows(5000)
+    vox = make_voxels(coords, torch.randn(len(coords), 32, generator=torch.Generator().manual_seed(1)).to(dtype)).sort()
+    torch.manual_seed(0)
+    down = SparseConv3d(32, 48, 2, stride=2, bias=True).to(DEV).to(dtype)
+    layer = {"same": SparseConv3d(32, 48, 3, bias=True), "down": down, "up": SparseConv3d(48, 32, 2, stride=2, bias=True, transposed=True)}[kind]
+    layer = layer.to(DEV).to(dtype)
+    layer.bias.data = torch.randn(layer.bias.shape, device=DEV).to(bias_dtype)
+    if kind == "up":
+        with torch.no_grad():
+            vox, target = down(vox), vox
+    call = (lambda v: layer(v, target)) if kind == "up" else layer
+    outs = []
+    for fused in (True, False):
+        x = vox.feature_tensor.detach().clone().requires_grad_(True)
+        bias = layer.bias
+        if not fused:
+            layer.bias = None
+        y = call(vox.replace(batched_features=x)).feature_tensor
+        if not fused:
+            y = (y.double() + bias.double()).to(dtype)
+            layer.bias = bias
+        dy = torch.randn(y.shape, generator=torch.Generator(device=DEV).manual_seed(2), device=DEV).to(dtype)
+        outs.append([y.detach(), *torch.autograd.grad(y, [x, layer.weight, bias], dy)])
+    tol = {torch.float32: 1e-6, torch.float16: 2e-3, torch.bfloat16: 1e-2}[dtype]
+    for got, want in zip(*outs):
+        assert got.dtype == want.dtype and rel_l2(got.float().cpu().numpy(), want.float().cpu().numpy()) < tol
+    x = vox.feature_tensor.detach().clone().requires_grad_(True)
+    y = call(vox.replace(batched_features=x)).feature_tensor
+    dy = torch.ones_like(y).requires_grad_(True)
+    (gb,) = torch.autograd.grad(y, [layer.bias], dy, create_graph=True)
+    (back,) = torch.autograd.grad(gb.sum(), [dy])
+    assert torch.equal(back, torch.ones_like(back))
+    check_device_status(DEV)
+
+
+@pytest.mark.parametrize("n", [12000, 19000])
+@pytest.mark.parametrize("where,value", [("x", float("inf")), ("x", float("nan")), ("x", 3.4e38), ("w", float("-inf")), ("w", 2.0 ** 64)])
+def test_fp32_numbers_without_three_parts(n, where, value, monkeypatch):
+    """Infinities, NaN and numbers whose partial products could overflow give what the FP32 pipes make of them."""
+    g = torch.Generator(device=DEV).manual_seed(n)
+    kmap = _random_map(27, n, n, g)
+    x = torch.randn(n, 32, generator=g, device=DEV)
+    w = torch.randn(27, 32, 32, generator=g, device=DEV)
+    if where == "x":
+        x[n // 2, 5] = value
+    else:
+        w[13, 7, 3] = value
+    got = sparse_conv_fused(x, w, kmap, n)
+    monkeypatch.setattr("warpconvnet_b200.nn.functional.sparse_conv._f32_workspace", lambda *a: (None, 0))
+    want = sparse_conv_fused(x, w, kmap, n)
+    check_device_status(DEV)
+    assert torch.equal(torch.isnan(got), torch.isnan(want)) and torch.equal(torch.isinf(got), torch.isinf(want))
+    fine = torch.isfinite(want)
+    assert torch.equal(got[~fine & ~torch.isnan(want)], want[~fine & ~torch.isnan(want)])
+    assert float((got[fine].double() - want[fine].double()).norm() / want[fine].double().norm()) < 1e-6
+
+
+@pytest.mark.parametrize("n", [18944, 18945, 37889, 65536, 65537, 12 * 16384, 13 * 16384 + 129])
+def test_every_unit_comes_once_whatever_their_order(n):
+    """Rows in tile order are worked through dense supertiles first, the last windows of a launch together: one unit per
+    multiprocessor, one more than that, small and large windows, whole and partial windows before the launch's tail.  The
+    sum of a row runs over the same offsets either way, so that the results are those of the plain order bit for bit."""
+    g = torch.Generator(device=DEV).manual_seed(n)
+    present = torch.rand(27, n, generator=g, device=DEV) < torch.rand(n, generator=g, device=DEV) ** 3
+    nbr = torch.where(present, torch.randint(0, n, (27, n), generator=g, device=DEV, dtype=torch.int32), torch.full((), -1, dtype=torch.int32, device=DEV))
+    kmap = IntSearchResult.from_neighbor_table(nbr, n)
+    x = torch.randn(n, 32, generator=g, device=DEV).half()
+    w = (torch.randn(27, 32, 32, generator=g, device=DEV) * 0.1).half()
+    got = []
+    for tiled in (False, True):
+        out = torch.full((n, 32), float("nan"), dtype=torch.float16, device=DEV)
+        got.append(sparse_conv_fused(x, w, kmap, n, epilogue=ConvEpilogue(out=out), algo=CONV_TCGEN05, tile_order=tiled))
+    check_device_status(DEV)
+    want = sparse_conv_fused(x, w, kmap, n, algo=CONV_SIMT)
+    assert torch.equal(*got) and rel_l2(got[0].float().cpu().numpy(), want.float().cpu().numpy()) < 2e-3
