@@ -178,3 +178,31 @@ def test_every_unit_comes_once_whatever_their_order(n):
     check_device_status(DEV)
     want = sparse_conv_fused(x, w, kmap, n, algo=CONV_SIMT)
     assert torch.equal(*got) and rel_l2(got[0].float().cpu().numpy(), want.float().cpu().numpy()) < 2e-3
+
+
+@pytest.mark.parametrize("n", [700, 19000])
+@pytest.mark.parametrize("ex,ew", [(-116, 0), (-124, 0), (-140, 0), (0, -118), (-20, -100), (-64, -64), (-75, -68)])
+def test_fp32_small_numbers_keep_their_bits(n, ex, ew):
+    """Numbers whose third or second part would lie below bf16's range, subnormal ones, and pairs whose product is subnormal:
+    layer and weight gradient as close to sums in 64 bits as the FP32 pipes, and (3e-7, 4e-7: see above) where the result
+    itself is not subnormal."""
+    from warpconvnet_b200.nn.functional import sparse_conv as sc
+    g = torch.Generator(device=DEV).manual_seed(n)
+    kmap = _random_map(27, n, n, g)
+    nbr = kmap.neighbor_table(n)
+    # (in two steps: 2 ** -140 times an fp32 number would be rounded before the multiplication)
+    x = (torch.randn(n, 48, generator=g, device=DEV).double() * 2.0 ** ex).float()
+    w = (torch.randn(27, 48, 64, generator=g, device=DEV).double() * 2.0 ** ew).float()
+    dy = (torch.randn(n, 64, generator=g, device=DEV).double() * 2.0 ** ew).float()
+    rows = [x[nbr[k].clamp(min=0).long()].double().mul((nbr[k] >= 0)[:, None]) for k in range(27)]
+    want = sum(rows[k] @ w[k].double() for k in range(27)), torch.stack([r.T @ dy.double() for r in rows])
+    error = lambda y, e: float((y.double() - e).norm() / e.norm())
+    with pytest.MonkeyPatch.context() as m:
+        got = sparse_conv_fused(x, w, kmap, n), sc.sparse_conv_wgrad(x, dy, kmap, n)
+        query = sc.query_bytes
+        m.setattr(sc, "query_bytes", lambda name, *a: 0 if "f32" in name else query(name, *a))
+        pipes = sparse_conv_fused(x, w, kmap, n), sc.sparse_conv_wgrad(x, dy, kmap, n)
+    check_device_status(DEV)
+    for y, f, e, limit in zip(got, pipes, want, (3e-7, 4e-7)):
+        assert error(y, e) <= 1.02 * error(f, e)
+        assert error(y, e) < limit or ex + ew < -125

@@ -9,7 +9,7 @@
 // nearest: 9.7e-8 (C = 128: 1.3e-7 against 6.4e-7; 20 000 random cells, C = 32: 6.8e-8 against 1.3e-7).
 //
 // Two launches.  The first writes the three bf16 planes of every feature row and of the weights (as swizzled shared-memory
-// images) to the caller's workspace, and whether any number is infinite, NaN or above 2^63 (a product of two parts could
+// images) to the caller's workspace, and whether any number is infinite, NaN or above 2^39 (a product of two parts could
 // then be infinite where the number's is not): with such a number every block of the second launch multiplies its rows on
 // the FMA pipes instead.  The second is the convolution.  A CTA works through units of 128 output rows x BN columns, claimed
 // one ahead from the hardware's queue, dense rows first:
@@ -433,7 +433,7 @@ conv_split_kernel(const SplitParams p) {
           if (c < cols) {
             float y[4];
 #pragma unroll
-            for (int j = 0; j < 4; ++j) y[j] = poison ? __int_as_float(0x7FC00000) : finish(p, sum[c + j], m, n0 + c + j);
+            for (int j = 0; j < 4; ++j) y[j] = poison ? __int_as_float(0x7FC00000) : finish(p, sum[c + j] * kSumScale, m, n0 + c + j);
             *reinterpret_cast<float4*>(dst + c) = make_float4(y[0], y[1], y[2], y[3]);
           }
         }
@@ -463,7 +463,7 @@ conv_split_kernel(const SplitParams p) {
       const float y[4] = {v[0].x, v[0].y, v[0].z, v[0].w};
       float o[4];
 #pragma unroll
-      for (int j = 0; j < 4; ++j) o[j] = poison ? __int_as_float(0x7FC00000) : finish(p, y[j], m, n0 + c + j);
+      for (int j = 0; j < 4; ++j) o[j] = poison ? __int_as_float(0x7FC00000) : finish(p, y[j] * kSumScale, m, n0 + c + j);
       *reinterpret_cast<float4*>(p.out + m * p.out_ld + n0 + c) = make_float4(o[0], o[1], o[2], o[3]);
     }
     cluster_meet();   // no CTA leaves while another may read its sums

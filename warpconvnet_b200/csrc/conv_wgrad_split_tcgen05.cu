@@ -289,7 +289,7 @@ conv_wgrad_split_kernel(const WsParams p) {
       for (int c = 0; c < 64; c += 4)
         if (c < cols && n0 + c < p.c_out) {
           const float nan = __int_as_float(0x7FC00000);
-          *reinterpret_cast<float4*>(dst + c) = poison || !ok ? make_float4(nan, nan, nan, nan) : make_float4(sum[c], sum[c + 1], sum[c + 2], sum[c + 3]);
+          *reinterpret_cast<float4*>(dst + c) = poison || !ok ? make_float4(nan, nan, nan, nan) : make_float4(sum[c] * kSumScale, sum[c + 1] * kSumScale, sum[c + 2] * kSumScale, sum[c + 3] * kSumScale);
         }
     }
   }

@@ -10,6 +10,11 @@ namespace {
 __host__ __device__ constexpr int split_a(int q) { return (0x001102 >> (4 * q)) & 15; }
 __host__ __device__ constexpr int split_b(int q) { return (0x010120 >> (4 * q)) & 15; }
 
+// bf16 ends at 2^-133, the last bit of a small fp32 number lies at 2^-149.  So every number is multiplied by 2^24 before it is
+// split, which brings all of them, the subnormal ones too, and the products of their parts into range; sums of products are
+// taken back by 2^-48.  Both are exact.  (Split as they were, numbers lost bits from 2^-110 downwards: 6e-5 at 2^-120.)
+constexpr float kSplitScale = 16777216.f, kSumScale = 1.f / (16777216.f * 16777216.f);
+
 // x = h + m + l exactly (round to nearest twice; the rest has eight bits).
 __device__ __forceinline__ void split3(float x, __nv_bfloat16& h, __nv_bfloat16& m, __nv_bfloat16& l) {
   h = __float2bfloat16_rn(x);
@@ -17,17 +22,18 @@ __device__ __forceinline__ void split3(float x, __nv_bfloat16& h, __nv_bfloat16&
   m = __float2bfloat16_rn(r);
   l = __float2bfloat16_rn(__fsub_rn(r, __bfloat162float(m)));
 }
-// Infinities, NaN, and numbers whose parts could have an infinite product where the numbers have none.
+// Infinities, NaN, and (scaled) numbers whose parts could have an infinite product where the numbers have none.
 __device__ __forceinline__ bool unsplittable(float x) { return !(fabsf(x) < 9.223372e18f); }
 
-// The parts of eight numbers, 16 bytes each, `apart` bytes from one another.
+// The parts of eight numbers times kSplitScale, 16 bytes each, `apart` bytes from one another.
 __device__ __forceinline__ bool store_parts(const float (&v)[8], char* dst, int64_t apart) {
   __align__(16) __nv_bfloat16 part[3][8];
   bool special = false;
 #pragma unroll
   for (int u = 0; u < 8; ++u) {
-    special |= unsplittable(v[u]);
-    split3(v[u], part[0][u], part[1][u], part[2][u]);
+    const float x = v[u] * kSplitScale;
+    special |= unsplittable(x);
+    split3(x, part[0][u], part[1][u], part[2][u]);
   }
 #pragma unroll
   for (int s = 0; s < 3; ++s) *reinterpret_cast<uint4*>(dst + s * apart) = *reinterpret_cast<const uint4*>(part[s]);
