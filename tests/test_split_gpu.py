@@ -206,3 +206,30 @@ def test_fp32_small_numbers_keep_their_bits(n, ex, ew):
     for y, f, e, limit in zip(got, pipes, want, (3e-7, 4e-7)):
         assert error(y, e) <= 1.02 * error(f, e)
         assert error(y, e) < limit or ex + ew < -125
+
+
+@pytest.mark.parametrize("n,c_out", [(300, 64), (5000, 144), (19000, 16), (19000, 160), (70000, 64)])
+def test_fp32_special_numbers_stay_with_their_rows(n, c_out, monkeypatch):
+    """A number that has no three parts changes the rows that name its row, as the FP32 pipes have them, and no bit of the
+    others, however the offsets and columns of a tile are divided; in a row that no pair names it changes nothing."""
+    g = torch.Generator(device=DEV).manual_seed(n)
+    kmap = _random_map(27, n, n - 1, g)
+    nbr = kmap.neighbor_table(n)
+    x = torch.randn(n, 64, generator=g, device=DEV)
+    w = torch.randn(27, 64, c_out, generator=g, device=DEV)
+    clean = sparse_conv_fused(x, w, kmap, n)
+    bad = x.clone()
+    bad[n - 1] = float("nan")
+    for row, value in ((0, float("inf")), (n // 3, float("nan")), (n // 2, -3e30), (n - 2, 6e11)):
+        bad[row, row % 64] = value
+    for tiled in (False, True):
+        got = sparse_conv_fused(bad, w, kmap, n, tile_order=tiled)
+        with monkeypatch.context() as m:
+            m.setattr("warpconvnet_b200.nn.functional.sparse_conv._f32_workspace", lambda *a: (None, 0))
+            want = sparse_conv_fused(bad, w, kmap, n, tile_order=tiled)
+        check_device_status(DEV)
+        named = torch.isin(nbr, torch.tensor([0, n // 3, n // 2, n - 2], device=DEV, dtype=nbr.dtype)).any(0)
+        assert named.any() and torch.equal(got[~named], clean[~named])
+        fine = torch.isfinite(want)
+        assert torch.equal(got[~fine].nan_to_num(1.0), want[~fine].nan_to_num(1.0)) and (named[:, None] & fine).any()
+        assert rel_l2(got[fine].cpu().numpy(), want[fine].cpu().numpy()) < 1e-6

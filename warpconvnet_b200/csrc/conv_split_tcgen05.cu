@@ -9,9 +9,11 @@
 // nearest: 9.7e-8 (C = 128: 1.3e-7 against 6.4e-7; 20 000 random cells, C = 32: 6.8e-8 against 1.3e-7).
 //
 // Two launches.  The first writes the three bf16 planes of every feature row and of the weights (as swizzled shared-memory
-// images) to the caller's workspace, and whether any number is infinite, NaN or above 2^39 (a product of two parts could
-// then be infinite where the number's is not): with such a number every block of the second launch multiplies its rows on
-// the FMA pipes instead.  The second is the convolution.  A CTA works through units of 128 output rows x BN columns, claimed
+// images) to the caller's workspace.  A number that is infinite, NaN or above 2^39 (a product of two parts could then be
+// infinite where the numbers' is not) becomes NaN there, and an output row whose sums are not finite is multiplied again on
+// the FMA pipes from the numbers as they came: other rows do not notice (60 000 rows of 64 channels: 71 us, with one NaN 142,
+// with one in every hundredth row 378, in every row 910; conv_fp32.cu 205.  As a second form of the whole launch, taken for
+// any such number anywhere: 1 840).  The second is the convolution.  A CTA works through units of 128 output rows x BN columns, claimed
 // one ahead from the hardware's queue, dense rows first:
 //  * four gather warps read the unit's neighbour table (32 rows each), agree on the offsets present, and copy for every
 //    (offset, 32 channels) the three planes of the listed rows into a slot of a ring (cp.async, absent rows zero-filled);
@@ -46,15 +48,13 @@ constexpr int SP_MAX_SLICES = 8;                      // CTAs of a (portable) cl
 constexpr int SP_EPI = 256, SP_GATHER = 128;          // warps 0..7 and 8..11
 constexpr int SP_MMA_WARP = 12, SP_ISSUERS = 2, SP_WEIGHT_WARP = 14, SP_THREADS = 480;
 constexpr size_t SP_SMEM = 226 * 1024;
-constexpr int SP_FLAGS = 1024;                        // blocks of the first launch at most
+constexpr int SP_PLANE_BLOCKS = 1024;                 // of the first launch at most
 
 struct SplitParams {
   const char* planes;      // [num_in][3][cp] bf16
   const char* wplanes;     // [K][cp / 32][3] images of [c_out][32] bf16
-  const int32_t* flags;    // what the blocks of the first launch found
-  int num_flags;
   const float* feats;
-  const float* weight;     // (the two as they came, for numbers that cannot be split)
+  const float* weight;     // (the two as they came, for rows with numbers that cannot be split)
   const int32_t* nbr;
   const int32_t* out_rows;
   int64_t M, in_ld, out_ld, res_ld;
@@ -114,16 +114,51 @@ __device__ __forceinline__ float finish(const SplitParams& p, float y, int64_t m
   return p.relu ? fmaxf(y, 0.f) : y;
 }
 
+// Whether any of `cols` sums is infinite or NaN (0 times it is no zero).
+__device__ __forceinline__ bool not_finite(const float (&sum)[64], int cols) {
+  float t[4] = {0.f, 0.f, 0.f, 0.f};
+#pragma unroll
+  for (int c = 0; c < 64; ++c)
+    if (c < cols) t[c & 3] = fmaf(sum[c], 0.f, t[c & 3]);
+  return !((t[0] + t[1]) + (t[2] + t[3]) == 0.f);
+}
+
+// Four columns of a table row on the FMA pipes, offsets and channels in order: what a number without three parts (its first
+// part is NaN) or a sum past the end of fp32 asks for.
+__device__ __forceinline__ void fma_four(const SplitParams& p, int64_t slot, int n, float (&y)[4]) {
+  y[0] = y[1] = y[2] = y[3] = 0.f;
+  int next = __ldg(&p.nbr[slot]);
+  for (int k = 0; k < p.K; ++k) {
+    const int r = next;
+    if (k + 1 < p.K) next = __ldg(&p.nbr[(int64_t)(k + 1) * p.M + slot]);
+    if (r < 0 || r >= p.num_in) continue;   // (reported by the gather warps)
+    const float* x = p.feats + (int64_t)r * p.in_ld;
+    const float* w = p.weight + (int64_t)k * p.c_in * p.c_out + n;
+#pragma unroll 4   // (loads in flight are what this takes its time for)
+    for (int c = 0; c < p.c_in; c += 4) {
+      const float4 a = __ldg(reinterpret_cast<const float4*>(x + c));
+      const float v[4] = {a.x, a.y, a.z, a.w};
+#pragma unroll
+      for (int u = 0; u < 4; ++u) {
+        const float4 b = __ldg(reinterpret_cast<const float4*>(w + (int64_t)(c + u) * p.c_out));
+        y[0] = fmaf(v[u], b.x, y[0]);
+        y[1] = fmaf(v[u], b.y, y[1]);
+        y[2] = fmaf(v[u], b.z, y[2]);
+        y[3] = fmaf(v[u], b.w, y[3]);
+      }
+    }
+  }
+}
+
 // ------------------------------------------------------------------ planes
 
 // Bound by memory (4 bytes in, 6 out per channel): a thread makes eight channels of a row, or of a column of the weights.
 __global__ void __launch_bounds__(256)
 split_planes_kernel(const float* __restrict__ feats, int64_t num_in, int64_t in_ld, const float* __restrict__ weight, int K, int c_in,
-                    int cp, int c_out, char* __restrict__ planes, char* __restrict__ wplanes, int32_t* __restrict__ flags) {
+                    int cp, int c_out, char* __restrict__ planes, char* __restrict__ wplanes) {
   launch_dependents();
   const int per_row = cp / 8;
   const int64_t rows = num_in * per_row, total = rows + (int64_t)K * per_row * c_out;
-  bool special = false;
   for (int64_t i = (int64_t)blockIdx.x * 256 + threadIdx.x; i < total; i += (int64_t)gridDim.x * 256) {
     float v[8];
     char* dst;
@@ -144,10 +179,8 @@ split_planes_kernel(const float* __restrict__ feats, int64_t num_in, int64_t in_
       apart = (int64_t)c_out * SP_RB;
       dst = wplanes + ((int64_t)k * (cp / SP_BK) + c / SP_BK) * 3 * apart + tile_offset<SP_RB>(n, (c % SP_BK) / 8);
     }
-    special |= store_parts(v, dst, apart);
+    store_parts(v, dst, apart);
   }
-  const int any = __syncthreads_or(special);
-  if (threadIdx.x == 0) flags[blockIdx.x] = any;
 }
 
 // ------------------------------------------------------------------ convolution
@@ -173,34 +206,9 @@ conv_split_kernel(const SplitParams p) {
     if (lane < 3) ctl->mask_acc[lane] = 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
+  if (warp == SP_MMA_WARP) tmem_alloc(smem_u32(&ctl->tmem), 512);
   // (everything above runs while the planes are written; tables, weights and rows are older than that launch)
   wait_for_primary();
-  int special = 0;
-  for (int i = tid; i < p.num_flags; i += SP_THREADS) special |= __ldcg(&p.flags[i]);
-  special = __syncthreads_or(special);
-  if (special) {
-    // A number that has no three parts: the FMA pipes, one sum per thread at a time (one unit per CTA: none are claimed).
-    const int block = first % p.blocks;
-    const int64_t m0 = (int64_t)tile_of(p, first / p.blocks) * SP_M;
-    for (int i = rank * SP_THREADS + tid; i < SP_M * BN; i += p.S * SP_THREADS) {
-      const int64_t slot = m0 + i / BN;
-      const int n = block * BN + i % BN;
-      if (slot >= p.M) break;
-      float y = 0.f;
-      for (int k = 0; k < p.K; ++k) {
-        const int r = __ldg(&p.nbr[(int64_t)k * p.M + slot]);
-        if (r >= p.num_in) wcn_report_bounds(p.dev_status);
-        if (r < 0 || r >= p.num_in) continue;
-        const float* x = p.feats + (int64_t)r * p.in_ld;
-        const float* w = p.weight + (int64_t)k * p.c_in * p.c_out + n;
-        for (int c = 0; c < p.c_in; ++c) y = fmaf(__ldg(x + c), __ldg(w + (int64_t)c * p.c_out), y);
-      }
-      const int64_t m = p.out_rows ? (int64_t)__ldg(&p.out_rows[slot]) : slot;
-      p.out[m * p.out_ld + n] = finish(p, y, m, n);
-    }
-    return;
-  }
-  if (warp == SP_MMA_WARP) tmem_alloc(smem_u32(&ctl->tmem), 512);
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
@@ -424,18 +432,38 @@ conv_split_kernel(const SplitParams p) {
 #pragma unroll
         for (int c = 0; c < 64; c += 4)
           if (c < cols) *reinterpret_cast<float4*>(dst + c) = make_float4(sum[c], sum[c + 1], sum[c + 2], sum[c + 3]);
-      } else if (m >= 0) {
+      } else {
         const bool poison = *(volatile const int32_t*)p.dev_status == (int)WCN_ERR_WAIT_EXPIRED;
         const int n0 = (unit % p.blocks) * BN + c_begin;
-        float* dst = p.out + m * p.out_ld + n0;
+        const bool again = m >= 0 && !poison && not_finite(sum, cols);
+        if (m >= 0 && !again) {
+          float* dst = p.out + m * p.out_ld + n0;
 #pragma unroll
-        for (int c = 0; c < 64; c += 4) {
-          if (c < cols) {
-            float y[4];
+          for (int c = 0; c < 64; c += 4) {
+            if (c < cols) {
+              float y[4];
 #pragma unroll
-            for (int j = 0; j < 4; ++j) y[j] = poison ? __int_as_float(0x7FC00000) : finish(p, sum[c + j] * kSumScale, m, n0 + c + j);
-            *reinterpret_cast<float4*>(dst + c) = make_float4(y[0], y[1], y[2], y[3]);
+              for (int j = 0; j < 4; ++j) y[j] = poison ? __int_as_float(0x7FC00000) : finish(p, sum[c + j] * kSumScale, m, n0 + c + j);
+              *reinterpret_cast<float4*>(dst + c) = make_float4(y[0], y[1], y[2], y[3]);
+            }
           }
+        }
+        // rows with such sums: four columns a lane, as many rows at once as the warp has room for
+        for (uint32_t rest = __ballot_sync(0xFFFFFFFFu, again); rest;) {
+          const int per = cols >> 2, at_once = 32 / per, turn = lane / per, c = (lane - turn * per) * 4;
+          int r = -1;
+          for (int i = 0; i < at_once && rest; ++i, rest &= rest - 1)
+            if (i == turn) r = __ffs(rest) - 1;
+          if (r >= 0) {
+            const int64_t slot = (int64_t)tile_of(p, unit / p.blocks) * SP_M + (warp & 3) * 32 + r;
+            const int64_t at = p.out_rows ? (int64_t)__ldg(&p.out_rows[slot]) : slot;
+            float y[4];
+            fma_four(p, slot, n0 + c, y);
+#pragma unroll
+            for (int j = 0; j < 4; ++j) y[j] = finish(p, y[j], at, n0 + c + j);
+            *reinterpret_cast<float4*>(p.out + at * p.out_ld + n0 + c) = make_float4(y[0], y[1], y[2], y[3]);
+          }
+          __syncwarp();
         }
       }
     }
@@ -460,10 +488,11 @@ conv_split_kernel(const SplitParams p) {
       for (int q = 1; q < SP_MAX_SLICES; ++q)
         if (q < p.S) { v[0].x += v[q].x; v[0].y += v[q].y; v[0].z += v[q].z; v[0].w += v[q].w; }
       const int64_t m = p.out_rows ? (int64_t)__ldg(&p.out_rows[m0 + r]) : m0 + r;
-      const float y[4] = {v[0].x, v[0].y, v[0].z, v[0].w};
+      float y[4] = {v[0].x * kSumScale, v[0].y * kSumScale, v[0].z * kSumScale, v[0].w * kSumScale};
+      if (!poison && !(fmaf(v[0].x, 0.f, v[0].y * 0.f) + fmaf(v[0].z, 0.f, v[0].w * 0.f) == 0.f)) fma_four(p, m0 + r, n0 + c, y);
       float o[4];
 #pragma unroll
-      for (int j = 0; j < 4; ++j) o[j] = poison ? __int_as_float(0x7FC00000) : finish(p, y[j] * kSumScale, m, n0 + c + j);
+      for (int j = 0; j < 4; ++j) o[j] = poison ? __int_as_float(0x7FC00000) : finish(p, y[j], m, n0 + c + j);
       *reinterpret_cast<float4*>(p.out + m * p.out_ld + n0 + c) = make_float4(o[0], o[1], o[2], o[3]);
     }
     cluster_meet();   // no CTA leaves while another may read its sums
@@ -475,7 +504,7 @@ conv_split_kernel(const SplitParams p) {
 
 struct SplitPlan {
   int cp, block_n, blocks;
-  size_t flags, weights, rows;   // bytes of the parts of the workspace
+  size_t weights, rows;   // bytes of the parts of the workspace
 };
 
 SplitPlan plan_split(int64_t num_in, int K, int c_in, int c_out) {
@@ -484,7 +513,6 @@ SplitPlan plan_split(int64_t num_in, int K, int c_in, int c_out) {
   q.blocks = (c_out + SP_MAX_N - 1) / SP_MAX_N;
   while (c_out % (16 * q.blocks) != 0) ++q.blocks;   // (c_out is a multiple of 16)
   q.block_n = c_out / q.blocks;
-  q.flags = SP_FLAGS * sizeof(int32_t);
   q.weights = (size_t)K * q.cp * c_out * 6;
   q.rows = (size_t)num_in * q.cp * 6;
   return q;
@@ -523,7 +551,7 @@ bool wcn_conv_split_supported(int K, int c_in, int c_out) {
 
 int64_t wcn_conv_split_workspace(int64_t num_in, int K, int c_in, int c_out) {
   const SplitPlan q = plan_split(num_in, K, c_in, c_out);
-  return (int64_t)(q.flags + q.weights + q.rows);
+  return (int64_t)(q.weights + q.rows);
 }
 
 // (rows and weights that wcn_conv_fp32_supported takes; `workspace` on a 16-byte boundary)
@@ -544,7 +572,7 @@ int wcn_conv_split_fwd(const void* feats, int64_t num_in, int64_t feats_ld, cons
   const SplitPlan q = plan_split(num_in, K, c_in, c_out);
   char* ws = (char*)workspace;
   SplitParams p = {};
-  p.flags = (const int32_t*)ws; p.wplanes = ws + q.flags; p.planes = ws + q.flags + q.weights;
+  p.wplanes = ws; p.planes = ws + q.weights;
   p.feats = (const float*)feats; p.weight = (const float*)weight; p.nbr = nbr; p.out_rows = out_rows;
   p.M = M; p.in_ld = feats_ld; p.out_ld = out_ld; p.res_ld = residual_ld;
   p.K = K; p.c_in = c_in; p.cp = q.cp; p.c_out = c_out; p.num_in = (int)num_in;
@@ -573,10 +601,8 @@ int wcn_conv_split_fwd(const void* feats, int64_t num_in, int64_t feats_ld, cons
   if (p.slots < 2) return WCN_ERR_UNSUPPORTED_CONFIG;
   const int64_t items = (num_in + (int64_t)K * c_out) * (q.cp / 8);
   int64_t blocks = (items + 511) / 512;
-  if (blocks > SP_FLAGS) blocks = SP_FLAGS;
-  p.num_flags = (int)blocks;
-  split_planes_kernel<<<(unsigned)blocks, 256, 0, st>>>(p.feats, num_in, feats_ld, p.weight, K, c_in, q.cp, c_out, ws + q.flags + q.weights,
-                                                        ws + q.flags, (int32_t*)ws);
+  if (blocks > SP_PLANE_BLOCKS) blocks = SP_PLANE_BLOCKS;
+  split_planes_kernel<<<(unsigned)blocks, 256, 0, st>>>(p.feats, num_in, feats_ld, p.weight, K, c_in, q.cp, c_out, ws + q.weights, ws);
   WCN_CHECK_LAUNCH();
   cudaLaunchAttribute attr[2] = {};
   attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;

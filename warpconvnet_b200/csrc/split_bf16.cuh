@@ -22,7 +22,8 @@ __device__ __forceinline__ void split3(float x, __nv_bfloat16& h, __nv_bfloat16&
   m = __float2bfloat16_rn(r);
   l = __float2bfloat16_rn(__fsub_rn(r, __bfloat162float(m)));
 }
-// Infinities, NaN, and (scaled) numbers whose parts could have an infinite product where the numbers have none.
+// Infinities, NaN, and (scaled) numbers whose parts could have an infinite product where the numbers have none: their first
+// part is NaN, which makes NaN of every sum that they are in, and such a sum is made again from the numbers themselves.
 __device__ __forceinline__ bool unsplittable(float x) { return !(fabsf(x) < 9.223372e18f); }
 
 // The parts of eight numbers times kSplitScale, 16 bytes each, `apart` bytes from one another.
@@ -34,6 +35,7 @@ __device__ __forceinline__ bool store_parts(const float (&v)[8], char* dst, int6
     const float x = v[u] * kSplitScale;
     special |= unsplittable(x);
     split3(x, part[0][u], part[1][u], part[2][u]);
+    if (unsplittable(x)) part[0][u] = __ushort_as_bfloat16(0x7FC0);
   }
 #pragma unroll
   for (int s = 0; s < 3; ++s) *reinterpret_cast<uint4*>(dst + s * apart) = *reinterpret_cast<const uint4*>(part[s]);
