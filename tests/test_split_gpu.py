@@ -233,3 +233,41 @@ def test_fp32_special_numbers_stay_with_their_rows(n, c_out, monkeypatch):
         fine = torch.isfinite(want)
         assert torch.equal(got[~fine].nan_to_num(1.0), want[~fine].nan_to_num(1.0)) and (named[:, None] & fine).any()
         assert rel_l2(got[fine].cpu().numpy(), want[fine].cpu().numpy()) < 1e-6
+
+
+@pytest.mark.parametrize("n,c_in,c_out", [(500, 64, 64), (9000, 36, 128), (20000, 160, 16), (70000, 64, 96)])
+def test_fp32_special_numbers_stay_with_their_weights(n, c_in, c_out, monkeypatch):
+    """A number that has no three parts changes the weight gradients that it belongs to, as the FP32 pipes have them, and no bit
+    of the others: a row of every offset's matrix for one of X (none where no pair names it), a column for one of dY, to the
+    present pairs only."""
+    from warpconvnet_b200.nn.functional import sparse_conv as sc
+    g = torch.Generator(device=DEV).manual_seed(n)
+    kmap = _random_map(27, n, n - 1, g)
+    x, dy = torch.randn(n, c_in, generator=g, device=DEV), torch.randn(n, c_out, generator=g, device=DEV)
+    clean = sc.sparse_conv_wgrad(x, dy, kmap, n)
+    query = sc.query_bytes
+    for value in (float("inf"), float("nan"), -1e30):
+        for rows, cols in (([n - 1], []), ([3], []), ([], [n // 2]), ([n // 4, n // 3], [0])):
+            bad, bad_dy = x.clone(), dy.clone()
+            for r in rows:
+                bad[r, 5] = value
+            for r in cols:
+                bad_dy[r, c_out - 3] = value
+            got = sc.sparse_conv_wgrad(bad, bad_dy, kmap, n, tile_order=True)
+            with monkeypatch.context() as m:
+                m.setattr(sc, "query_bytes", lambda name, *a: 0 if name == "wcn_conv_wgrad_f32_workspace_bytes" else query(name, *a))
+                want = sc.sparse_conv_wgrad(bad, bad_dy, kmap, n)
+            check_device_status(DEV)
+            same = torch.ones(27, c_in, c_out, dtype=torch.bool, device=DEV)
+            if rows and rows != [n - 1]:
+                same[:, 5] = False
+            if cols:
+                same[:, :, (c_out - 3) // 4 * 4:(c_out - 3) // 4 * 4 + 4] = False
+            ordered = sc.sparse_conv_wgrad(x, dy, kmap, n, tile_order=True)
+            assert torch.equal(got[same], ordered[same]) and rel_l2(ordered.cpu().numpy(), clean.cpu().numpy()) < 1e-6
+            fine = torch.isfinite(want)
+            assert torch.equal(got[~fine].nan_to_num(1.0), want[~fine].nan_to_num(1.0))
+            fine &= ~same
+            # (sums of N = n / 3 products one after the other: N roundings of 2^-24 of partial sums that grow as their square
+            # root, 2^-25 (N / 6)^1/2 = 2e-6 of the total for the longest, on both sides)
+            assert not fine.any() or rel_l2(got[fine].cpu().numpy(), want[fine].cpu().numpy()) < 1e-5

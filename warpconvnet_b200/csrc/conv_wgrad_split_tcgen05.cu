@@ -32,14 +32,12 @@ constexpr int WS_MAX_TILES = 512;                     // 128-row tiles of a rang
 constexpr int WS_EPI = 256, WS_GATHER = 128;          // warps 0..7 and 8..11
 constexpr int WS_MMA_WARP = 12, WS_ISSUERS = 2, WS_DY_WARP = 14, WS_THREADS = 480;
 constexpr size_t WS_SMEM = 226 * 1024;
-constexpr int WS_FLAGS = 1024;
+constexpr int WS_PLANE_BLOCKS = 1024;                 // of the first launch at most
 
 struct WsParams {
   const char* planes;       // [num_in][3][cp] bf16
   const char* images;       // [tiles][4][3][gchunks] images of 32 rows x 32 channels
-  const int32_t* flags;
-  int num_flags;
-  const float* feats;
+  const float* feats;       // (these two for sums that are not finite)
   const float* gout;
   const int32_t* nbr;
   const int32_t* out_rows;
@@ -57,23 +55,23 @@ struct WsControl {
   uint32_t tmem;
   int32_t count;
   int32_t tile[WS_MAX_TILES];   // tiles of the range that the group has anything in
+  uint32_t again[2][WS_CHUNKS]; // fours of columns (of the two halves) of a chunk with sums that are not finite
+  uint32_t odd[2][128];         // those of a row
 };
 
 __global__ void __launch_bounds__(256)
 wgrad_planes_kernel(const float* __restrict__ feats, int64_t num_in, int c_in, int cp, const float* __restrict__ gout, int64_t M, int c_out,
-                    int gchunks, int tiles, const int32_t* __restrict__ out_rows, char* __restrict__ planes, char* __restrict__ images,
-                    int32_t* __restrict__ flags) {
+                    int gchunks, int tiles, const int32_t* __restrict__ out_rows, char* __restrict__ planes, char* __restrict__ images) {
   launch_dependents();
   const int per_x = cp / 8, per_g = gchunks * 4;
   const int64_t x_items = num_in * per_x, total = x_items + (int64_t)tiles * 128 * per_g;
-  bool special = false;
   for (int64_t i = (int64_t)blockIdx.x * 256 + threadIdx.x; i < total; i += (int64_t)gridDim.x * 256) {
     float v[8];
     if (i < x_items) {
       const int64_t r = i / per_x;
       const int c = (int)(i - r * per_x) * 8;
       load_eight(feats + r * c_in, c, c_in, v);
-      special |= store_parts(v, planes + r * 6 * cp + c * 2, (int64_t)cp * 2);
+      store_parts(v, planes + r * 6 * cp + c * 2, (int64_t)cp * 2);
     } else {
       const int64_t q = i - x_items, m = q / per_g;
       const int c = (int)(q - m * per_g) * 8;
@@ -85,11 +83,9 @@ wgrad_planes_kernel(const float* __restrict__ feats, int64_t num_in, int c_in, i
         for (int u = 0; u < 8; ++u) v[u] = 0.f;
       }
       const int64_t apart = (int64_t)gchunks * WS_CHUNK;
-      special |= store_parts(v, images + (m / WS_ROWS) * 3 * apart + (c / 32) * WS_CHUNK + tile_offset<64>((int)(m % WS_ROWS), (c % 32) / 8), apart);
+      store_parts(v, images + (m / WS_ROWS) * 3 * apart + (c / 32) * WS_CHUNK + tile_offset<64>((int)(m % WS_ROWS), (c % 32) / 8), apart);
     }
   }
-  const int any = __syncthreads_or(special);
-  if (threadIdx.x == 0) flags[blockIdx.x] = any;
 }
 
 __global__ void __launch_bounds__(WS_THREADS, 1)
@@ -123,37 +119,20 @@ conv_wgrad_split_kernel(const WsParams p) {
       n += __popc(b);
     }
     if (lane == 0) ctl->count = n;
+    if (lane < 2 * WS_CHUNKS) ctl->again[lane / WS_CHUNKS][lane % WS_CHUNKS] = 0;
   } else if (warp == WS_MMA_WARP) {
     tmem_alloc(smem_u32(&ctl->tmem), 512);
   }
   // (everything above runs while the parts are written; tables, masks and rows are older than that launch)
   wait_for_primary();
-  int special = 0;
-  for (int i = tid; i < p.num_flags; i += WS_THREADS) special |= __ldcg(&p.flags[i]);
   tc_fence_before();
-  special = __syncthreads_or(special);
+  __syncthreads();
   tc_fence_after();
   const uint32_t tmem = ctl->tmem;
-  const int steps = special ? 0 : ctl->count * 4;
+  const int steps = ctl->count * 4;
   bool ok = true;
 
-  if (special) {
-    // A number that has no three parts: the FMA pipes, present pairs only, one sum per thread at a time.
-    const int64_t m1 = min(p.M, (int64_t)t1 * 128);
-    for (int i = tid; i < 128 * BN; i += WS_THREADS) {
-      const int q = group * WS_CHUNKS + (i / BN) / 32, k = q / cpc, ci = (q % cpc) * 32 + (i / BN) % 32, co = block * BN + i % BN;
-      if (q >= chunks || ci >= p.c_in || co >= p.c_out) continue;
-      float v = 0.f;
-      for (int64_t m = (int64_t)t0 * 128; m < m1; ++m) {
-        const int r = __ldg(&p.nbr[(int64_t)k * p.M + m]);
-        if (r >= p.num_in) wcn_report_bounds(p.dev_status);
-        if (r < 0 || r >= p.num_in) continue;
-        const int64_t row = p.out_rows ? (int64_t)__ldg(&p.out_rows[m]) : m;
-        v = fmaf(__ldg(&p.feats[(int64_t)r * p.c_in + ci]), __ldg(&p.gout[row * p.c_out + co]), v);
-      }
-      p.dst[(((int64_t)range * p.K + k) * p.c_in + ci) * p.c_out + co] = v;
-    }
-  } else if (warp >= 8 && warp < WS_MMA_WARP) {
+  if (warp >= 8 && warp < WS_MMA_WARP) {
     // ================================================================ gather: a chunk per warp
     const int w = warp - 8, q = group * WS_CHUNKS + w;
     const bool mine = q < chunks;
@@ -281,20 +260,97 @@ conv_wgrad_split_kernel(const WsParams p) {
       if (++ab == WS_ACCS) { ab = 0; aphase ^= 1; }
     }
     const int q = group * WS_CHUNKS + (warp & 3), k = q / cpc, ci = (q % cpc) * 32 + lane;
+    const int n0 = block * BN + c_begin;
+    float* dst = p.dst + (((int64_t)range * p.K + k) * p.c_in + ci) * p.c_out + n0;
+    uint32_t mine = 0;   // fours of columns with a sum that is not finite
     if (q < chunks && ci < p.c_in) {
-      const bool poison = *(volatile const int32_t*)p.dev_status == (int)WCN_ERR_WAIT_EXPIRED;
-      const int n0 = block * BN + c_begin;
-      float* dst = p.dst + (((int64_t)range * p.K + k) * p.c_in + ci) * p.c_out + n0;
+      const bool poison = !ok || *(volatile const int32_t*)p.dev_status == (int)WCN_ERR_WAIT_EXPIRED;
 #pragma unroll
       for (int c = 0; c < 64; c += 4)
         if (c < cols && n0 + c < p.c_out) {
           const float nan = __int_as_float(0x7FC00000);
-          *reinterpret_cast<float4*>(dst + c) = poison || !ok ? make_float4(nan, nan, nan, nan) : make_float4(sum[c] * kSumScale, sum[c + 1] * kSumScale, sum[c + 2] * kSumScale, sum[c + 3] * kSumScale);
+          if (poison) *reinterpret_cast<float4*>(dst + c) = make_float4(nan, nan, nan, nan);
+          else if (!(fmaf(sum[c], 0.f, sum[c + 1] * 0.f) + fmaf(sum[c + 2], 0.f, sum[c + 3] * 0.f) == 0.f)) mine |= 1u << (c / 4);
+          else *reinterpret_cast<float4*>(dst + c) = make_float4(sum[c] * kSumScale, sum[c + 1] * kSumScale, sum[c + 2] * kSumScale, sum[c + 3] * kSumScale);
         }
+    }
+    const uint32_t any = __reduce_or_sync(0xFFFFFFFFu, mine);
+    if (any) {
+      ctl->odd[half][tid & 127] = mine;
+      if (lane == 0) ctl->again[half][warp & 3] = any;
     }
   }
   tc_fence_before();
   __syncthreads();
+  // A number without three parts, or one beside an absent row (0 times infinity): such sums are made again on the FMA pipes
+  // from the present pairs, up to eight fours of a chunk at a time.  All warps take slots of 32 rows in turns, their sums
+  // are added in order through the ring, which nothing uses any more (60 000 room voxels, 64 -> 64, 101 us: 357 with a NaN in
+  // a row of X and one of dY, 930 with nothing else, 175 in conv_wgrad_pairs.cu; one thread per sum walking all rows took
+  // 20 000, an epilogue warp on its own 808 and 1 629).
+  float* part = reinterpret_cast<float*>(smem_raw + (base - smem_u32(smem_raw)));
+  for (int i = 0; i < 2 * WS_CHUNKS; ++i) {
+    const int half = i / WS_CHUNKS, w = i % WS_CHUNKS, q = group * WS_CHUNKS + w, k = q / cpc, ci = (q % cpc) * 32 + lane;
+    const int n0 = block * BN + (half ? ((BN / 16 + 1) / 2) * 16 : 0);
+    for (uint32_t rest = ctl->again[half][w]; rest;) {
+      int col[8], fours = 0;
+#pragma unroll
+      for (int j = 0; j < 8; ++j) {
+        col[j] = rest ? (__ffs(rest) - 1) * 4 : 0;
+        fours += rest ? 1 : 0;
+        rest &= rest - 1;
+      }
+      float4 acc[8];
+#pragma unroll
+      for (int j = 0; j < 8; ++j) acc[j] = make_float4(0.f, 0.f, 0.f, 0.f);
+      for (int t = warp; t < steps; t += WS_THREADS / 32) {
+        const int64_t m = (int64_t)ctl->tile[t >> 2] * 128 + (t & 3) * WS_ROWS + lane;
+        const int r = m < p.M ? __ldg(&p.nbr[(int64_t)k * p.M + m]) : -1;
+        const int64_t at = m < p.M && p.out_rows ? (int64_t)__ldg(&p.out_rows[m]) : m;
+        for (uint32_t have = __ballot_sync(0xFFFFFFFFu, r >= 0 && r < p.num_in); have;) {   // (others are reported by the gather warps)
+          float x[4];
+          const float* g[4];
+#pragma unroll
+          for (int u = 0; u < 4; ++u) {
+            const int row = have ? __ffs(have) - 1 : -1;
+            have &= have - 1;
+            const int64_t from = __shfl_sync(0xFFFFFFFFu, r, max(row, 0)), to = __shfl_sync(0xFFFFFFFFu, at, max(row, 0));
+            x[u] = row >= 0 && ci < p.c_in ? __ldg(&p.feats[from * p.c_in + ci]) : 0.f;
+            g[u] = row >= 0 ? p.gout + to * p.c_out + n0 : nullptr;
+          }
+#pragma unroll
+          for (int j = 0; j < 8; ++j) {
+            if (j >= fours) break;
+            float4 v[4];
+#pragma unroll
+            for (int u = 0; u < 4; ++u) v[u] = g[u] ? __ldg(reinterpret_cast<const float4*>(g[u] + col[j])) : make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll
+            for (int u = 0; u < 4; ++u) {
+              acc[j].x = fmaf(x[u], v[u].x, acc[j].x);
+              acc[j].y = fmaf(x[u], v[u].y, acc[j].y);
+              acc[j].z = fmaf(x[u], v[u].z, acc[j].z);
+              acc[j].w = fmaf(x[u], v[u].w, acc[j].w);
+            }
+          }
+        }
+      }
+#pragma unroll
+      for (int j = 0; j < 8; ++j)
+        if (j < fours) reinterpret_cast<float4*>(part)[(warp * 8 + j) * 32 + lane] = acc[j];
+      __syncthreads();
+      int c = 0;
+#pragma unroll
+      for (int j = 0; j < 8; ++j) c = warp == j ? col[j] : c;
+      if (warp < fours && ((ctl->odd[half][w * 32 + lane] >> (c / 4)) & 1u)) {
+        float4 y = make_float4(0.f, 0.f, 0.f, 0.f);
+        for (int from = 0; from < WS_THREADS / 32; ++from) {
+          const float4 v = reinterpret_cast<const float4*>(part)[(from * 8 + warp) * 32 + lane];
+          y.x += v.x; y.y += v.y; y.z += v.z; y.w += v.w;
+        }
+        *reinterpret_cast<float4*>(p.dst + (((int64_t)range * p.K + k) * p.c_in + ci) * p.c_out + n0 + c) = y;
+      }
+      __syncthreads();
+    }
+  }
   if (warp == WS_MMA_WARP) tmem_dealloc(tmem, 512);
 }
 
@@ -354,7 +410,7 @@ extern "C" int wcn_conv_wgrad_f32_workspace_bytes(int64_t num_in, int64_t num_ou
   // 27 offsets, 60 000 rows: 79 / 69, outdoors 58 / 64).
   if (num_offsets < 16 || (int64_t)c_in * c_out < 2048 || !wgrad_split_supported(num_in, num_out, num_offsets, c_in, c_out)) return WCN_OK;
   const WsPlan q = plan_ws(num_in, num_out, num_offsets, c_in, c_out);
-  *bytes = (int64_t)(WS_FLAGS * sizeof(int32_t) + q.planes + q.images + q.partial);
+  *bytes = (int64_t)(q.planes + q.images + q.partial);
   return WCN_OK;
 }
 
@@ -367,7 +423,7 @@ extern "C" int wcn_conv_wgrad_f32(const float* feats, int64_t num_in, const floa
       odd(grad_weight) || odd(workspace))
     return WCN_ERR_INVALID_PARAMETERS;
   const WsPlan q = plan_ws(num_in, num_out, num_offsets, c_in, c_out);
-  if (workspace_bytes < (int64_t)(WS_FLAGS * sizeof(int32_t) + q.planes + q.images + q.partial)) return WCN_ERR_INVALID_PARAMETERS;
+  if (workspace_bytes < (int64_t)(q.planes + q.images + q.partial)) return WCN_ERR_INVALID_PARAMETERS;
   static bool configured[64] = {};
   int dev = 0;
   if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return WCN_ERR_INITIALIZATION;
@@ -381,11 +437,11 @@ extern "C" int wcn_conv_wgrad_f32(const float* feats, int64_t num_in, const floa
   cudaStream_t st = wcn_stream(stream);
   char* ws = (char*)workspace;
   WsParams p = {};
-  p.flags = (const int32_t*)ws; p.planes = ws + WS_FLAGS * sizeof(int32_t); p.images = p.planes + q.planes;
+  p.planes = ws; p.images = p.planes + q.planes;
   p.feats = feats; p.gout = grad_out; p.nbr = nbr; p.out_rows = out_rows; p.masks = tile_masks;
   p.M = num_out; p.K = num_offsets; p.c_in = c_in; p.cp = q.cp; p.c_out = c_out; p.num_in = (int)num_in; p.gchunks = q.gchunks;
   p.groups = q.groups; p.blocks = q.blocks; p.block_n = q.block_n; p.tiles = q.tiles; p.per_range = q.per_range;
-  p.dst = q.ranges > 1 ? (float*)(ws + WS_FLAGS * sizeof(int32_t) + q.planes + q.images) : grad_weight;
+  p.dst = q.ranges > 1 ? (float*)(ws + q.planes + q.images) : grad_weight;
   p.dev_status = dev_status;
   const size_t slot = WS_A + 3 * (size_t)q.block_n * 64, fixed = 1024 + sizeof(WsControl) + 64;
   p.slots = (int)((WS_SMEM - fixed) / slot);
@@ -394,10 +450,9 @@ extern "C" int wcn_conv_wgrad_f32(const float* feats, int64_t num_in, const floa
   if (ctas > 0x7FFFFFFFll) return WCN_ERR_UNSUPPORTED_CONFIG;
   const int64_t items = num_in * (q.cp / 8) + (int64_t)q.tiles * 128 * q.gchunks * 4;
   int64_t blocks = (items + 511) / 512;
-  if (blocks > WS_FLAGS) blocks = WS_FLAGS;
-  p.num_flags = (int)blocks;
+  if (blocks > WS_PLANE_BLOCKS) blocks = WS_PLANE_BLOCKS;
   wgrad_planes_kernel<<<(unsigned)blocks, 256, 0, st>>>(feats, num_in, c_in, q.cp, grad_out, num_out, c_out, q.gchunks, q.tiles, out_rows,
-                                                        (char*)p.planes, (char*)p.images, (int32_t*)ws);
+                                                        (char*)p.planes, (char*)p.images);
   WCN_CHECK_LAUNCH();
   cudaLaunchAttribute attr = {};
   attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;

@@ -27,19 +27,16 @@ __device__ __forceinline__ void split3(float x, __nv_bfloat16& h, __nv_bfloat16&
 __device__ __forceinline__ bool unsplittable(float x) { return !(fabsf(x) < 9.223372e18f); }
 
 // The parts of eight numbers times kSplitScale, 16 bytes each, `apart` bytes from one another.
-__device__ __forceinline__ bool store_parts(const float (&v)[8], char* dst, int64_t apart) {
+__device__ __forceinline__ void store_parts(const float (&v)[8], char* dst, int64_t apart) {
   __align__(16) __nv_bfloat16 part[3][8];
-  bool special = false;
 #pragma unroll
   for (int u = 0; u < 8; ++u) {
     const float x = v[u] * kSplitScale;
-    special |= unsplittable(x);
     split3(x, part[0][u], part[1][u], part[2][u]);
     if (unsplittable(x)) part[0][u] = __ushort_as_bfloat16(0x7FC0);
   }
 #pragma unroll
   for (int s = 0; s < 3; ++s) *reinterpret_cast<uint4*>(dst + s * apart) = *reinterpret_cast<const uint4*>(part[s]);
-  return special;
 }
 // Eight consecutive numbers of a row, zeros from `limit` on (a multiple of four; rows start on 16-byte boundaries).
 __device__ __forceinline__ void load_eight(const float* row, int c, int limit, float (&v)[8]) {
