@@ -271,3 +271,22 @@ def test_fp32_special_numbers_stay_with_their_weights(n, c_in, c_out, monkeypatc
             # (sums of N = n / 3 products one after the other: N roundings of 2^-24 of partial sums that grow as their square
             # root, 2^-25 (N / 6)^1/2 = 2e-6 of the total for the longest, on both sides)
             assert not fine.any() or rel_l2(got[fine].cpu().numpy(), want[fine].cpu().numpy()) < 1e-5
+
+
+@pytest.mark.parametrize("c_in,c_out", [(32, 32), (64, 64), (36, 36), (128, 144)])
+def test_fp32_rows_do_not_depend_on_their_launch(c_in, c_out):
+    """What a scene divided among GPUs relies on (interior rows, boundary rows, all rows at once; halo rows that have not
+    arrived yet hold anything): with ``split_k=1`` a row's bits are those of the launch over all rows."""
+    g = torch.Generator(device=DEV).manual_seed(c_in)
+    n = 45000
+    kmap = _random_map(27, n, n, g)
+    nbr = kmap.neighbor_table(n)
+    x = torch.randn(n + 50, c_in, generator=g, device=DEV)
+    w = torch.randn(27, c_in, c_out, generator=g, device=DEV)
+    whole = sparse_conv_fused(x, w, kmap, n, split_k=1)
+    x[n:] = float("nan")
+    for rows in (slice(0, 90), slice(17000, 18000), slice(5000, 45000)):
+        part = IntSearchResult.from_neighbor_table(nbr[:, rows].contiguous(), n + 50)
+        got = sparse_conv_fused(x, w, part, len(range(n)[rows]), split_k=1)
+        check_device_status(DEV)
+        assert torch.equal(got, whole[rows])

@@ -25,7 +25,7 @@ bool wcn_conv_fp32_supported(int c_in, int c_out, int dtype, int out_dtype, cons
 int wcn_conv_fp32_fwd(const void* feats, int64_t num_in, int64_t feats_ld, const void* weight, const int32_t* nbr,
                       const int32_t* out_rows, int64_t M, int K, int c_in, int c_out, const float* scale,
                       const float* shift, const void* residual, int64_t residual_ld, int relu, void* out,
-                      int64_t out_ld, int sms, int32_t* dev_status, cudaStream_t st);
+                      int64_t out_ld, int sms, int split_k, int32_t* dev_status, cudaStream_t st);
 // conv_split_tcgen05.cu
 bool wcn_conv_split_supported(int K, int c_in, int c_out);
 int64_t wcn_conv_split_workspace(int64_t num_in, int K, int c_in, int c_out);
@@ -178,7 +178,7 @@ extern "C" int wcn_conv_fwd(int algo, const void* feats, int64_t num_in, int64_t
   }
   if (fp32) {
     return wcn_conv_fp32_fwd(feats, num_in, feats_ld, weight, nbr, out_rows, num_out, num_offsets, c_in, c_out, scale, shift,
-                             residual, residual_ld, relu, out, out_ld, wcn_num_sms(), dev_status, st);
+                             residual, residual_ld, relu, out, out_ld, wcn_num_sms(), split_k, dev_status, st);
   }
   return wcn_conv_simt_fwd(feats, num_in, feats_ld, weight, nbr, out_rows, num_out, num_offsets, c_in, c_out, dtype,
                            scale, shift, residual, residual_ld, relu, out, out_ld, out_dtype, dev_status, st);

@@ -277,7 +277,7 @@ bool wcn_conv_fp32_supported(int c_in, int c_out, int dtype, int out_dtype, cons
 int wcn_conv_fp32_fwd(const void* feats, int64_t num_in, int64_t feats_ld, const void* weight, const int32_t* nbr,
                       const int32_t* out_rows, int64_t M, int K, int c_in, int c_out, const float* scale,
                       const float* shift, const void* residual, int64_t residual_ld, int relu, void* out,
-                      int64_t out_ld, int sms, int32_t* dev_status, cudaStream_t st) {
+                      int64_t out_ld, int sms, int split_k, int32_t* dev_status, cudaStream_t st) {
   F32Params p;
   p.feats = (const float*)feats; p.weight = (const float*)weight; p.nbr = nbr; p.out_rows = out_rows;
   p.M = M; p.in_ld = feats_ld; p.out_ld = out_ld; p.res_ld = residual_ld;
@@ -293,10 +293,11 @@ int wcn_conv_fp32_fwd(const void* feats, int64_t num_in, int64_t feats_ld, const
   }
   // Row tile: 64 rows while they give every multiprocessor a block, else 16 (more blocks, each re-reading the weights).
   // With fewer than four blocks per multiprocessor a block's own chain of steps is what takes the time, not the
-  // arithmetic: its offsets are dealt to groups of threads (20 000 cells, C = 32: 47 -> 30 us).
+  // arithmetic: its offsets are dealt to groups of threads (20 000 cells, C = 32: 47 -> 30 us), unless the caller wants sums
+  // that do not depend on how many rows a launch has (split_k = 1).
   const int blocks_n = (c_out + tn - 1) / tn;
   const bool small = ((M + 63) / 64) * blocks_n < sms;
-  const bool grouped = K >= 8 && ((M + 63) / 64) * blocks_n < 4 * (int64_t)sms;
+  const bool grouped = split_k != 1 && K >= 8 && ((M + 63) / 64) * blocks_n < 4 * (int64_t)sms;
   p.tiles_per_window = out_rows ? (M > 4096 ? 16384 : 4096) / (small ? 16 : 64) : 0;
 #define WCN_F32_CASE(TN, GN)                                                               \
   if (tn == TN) {                                                                          \

@@ -230,10 +230,13 @@ def _row_view(t: Tensor) -> Tensor:
     return t if t.dim() == 2 and t.stride(1) == 1 and t.stride(0) >= t.shape[1] else t.contiguous()
 
 
-def _f32_workspace(x: Tensor, num_out: int, K: int, c_in: int, c_out: int) -> Tuple[Optional[Tensor], int]:
-    """(memory with which an fp32 layer runs on the tensor cores, its bytes): ``(None, 0)`` where it does not."""
+def _f32_workspace(x: Tensor, num_out: int, K: int, c_in: int, c_out: int, split_k: int = 0) -> Tuple[Optional[Tensor], int]:
+    """(memory with which an fp32 layer runs on the tensor cores, its bytes): ``(None, 0)`` where it does not.  With
+    ``split_k=1`` that does not depend on the number of rows, so that launches over parts of the rows compute the same."""
     if x.dtype != torch.float32:
         return None, 0
+    if split_k == 1 and num_out > 0:
+        num_out = 1 << 40  # more rows than any rule asks for
     nbytes = query_bytes("wcn_conv_f32_workspace_bytes", x.shape[0], num_out, K, c_in, c_out)
     if nbytes:
         try:
@@ -319,7 +322,7 @@ def sparse_conv_fused(in_features: Tensor, weight: Tensor, kernel_map: IntSearch
         assert tuple(residual.shape) == (num_out_coords, c_out), \
             f"residual {tuple(residual.shape)} != output {(num_out_coords, c_out)}"
     dc, odc = dtype_code(x.dtype), dtype_code(out_dtype)
-    workspace, workspace_bytes = _f32_workspace(x, num_out_coords, K, c_in, c_out) if algo == CONV_AUTO and odc == dc else (None, 0)
+    workspace, workspace_bytes = _f32_workspace(x, num_out_coords, K, c_in, c_out, split_k) if algo == CONV_AUTO and odc == dc else (None, 0)
     check(lib().wcn_conv_fwd(algo, ptr(x), x.shape[0], x.stride(0), ptr(w), ptr(packed), ptr(nbr), ptr(out_rows),
                              num_out_coords, K, c_in, c_out, dc, ptr(scale), ptr(shift), ptr(residual),
                              residual.stride(0) if residual is not None else 0, int(ep.relu), ptr(out),
