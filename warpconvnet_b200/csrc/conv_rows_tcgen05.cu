@@ -18,8 +18,8 @@
 //     the next ones;
 //   * twelve epilogue warps read TMEM, apply scale / shift / residual / ReLU and store each
 //     C_out-wide block at its destination row.
-// Work unit = (chunk of offsets, row tile); units are numbered chunk-major and dealt round-robin to
-// a persistent grid, so a CTA changes its weight chunk only a few times on large inputs.
+// Work unit = (chunk of offsets, row tile); units are numbered chunk-major (in groups of tiles where the rows do not stay in L2)
+// and dealt round-robin to a persistent grid, so a CTA changes its weight chunk only a few times on large inputs.
 //
 // What bounds it is the latency of the epilogue's steps: with eight warps and chunks of up to 256 columns the transposed layer
 // 96 -> 96 from 75 000 to 300 000 rows took 32.0 us, with twelve and 128 28.8 (eight and 128: 31.8; sixteen: 38).
@@ -41,6 +41,7 @@ constexpr int THREADS = (EPI_WARP0 + EPI_WARPS) * 32;
 constexpr int MAX_COLS = 256;          // output columns of one offset (one MMA's N)
 constexpr int CHUNK_COLS = 128;        // output columns of a chunk of several: four accumulator sets fit in tensor memory
 constexpr int SMEM_BUDGET = 220 * 1024;
+constexpr int64_t GROUP_BYTES = 24ll << 20;   // rows of a group of tiles
 
 struct RowsParams {
   const char* wpacked;       // packed weights: [K][c_in/BK] swizzled tiles of [c_out][BK]
@@ -50,6 +51,7 @@ struct RowsParams {
   int q, nchunks, nbuf, stages; // offsets per chunk, chunks, weight buffers, row-tile ring depth
   int nacc;                     // accumulator sets (2..4, as many as fit in 512 columns)
   int64_t tiles, units;
+  int group;                 // row tiles that all chunks are done for before the next ones are read
   const float* scale;
   const float* shift;
   const void* residual;
@@ -143,17 +145,31 @@ __device__ __forceinline__ void add_residual(const TO* rrow, int c0, float (&y)[
   }
 }
 
-// Position in the unit sequence of a CTA: units are numbered chunk-major, a CTA takes every
-// grid-th one.  Kept as (chunk, tile) and advanced by additions only.
-struct UnitCursor {
-  int chunk, tile;
-  __device__ __forceinline__ void advance(int step, int tiles) {
+// Position in the unit sequence of a CTA: units are numbered chunk-major inside groups of row tiles (GROUPED, else over all of
+// them), a CTA takes every grid-th one.  Kept as (chunk, tile, the group's tiles) and advanced by additions only; chunk >=
+// nchunks behind the last unit.  (One form for both costs the kernels with a single group 3 to 8 %.)
+template <bool GROUPED> struct UnitCursor {
+  int chunk, tile, base, end;
+  __device__ __forceinline__ void advance(int step, const RowsParams& p) {
     tile += step;
-    while (tile >= tiles) { tile -= tiles; ++chunk; }
+    if (!GROUPED) {
+      while (tile >= (int)p.tiles) { tile -= (int)p.tiles; ++chunk; }
+      return;
+    }
+    while (tile >= end) {
+      tile -= end - base;
+      ++chunk;
+      if (chunk == p.nchunks && end < (int)p.tiles) {
+        tile += end - base;
+        base = end;
+        end = min(end + p.group, (int)p.tiles);
+        chunk = 0;
+      }
+    }
   }
 };
 
-template <int BK, bool BF16, typename TO>
+template <int BK, bool BF16, typename TO, bool GROUPED>
 __global__ void __launch_bounds__(THREADS, 1)
 conv_rows_tcgen05_kernel(const __grid_constant__ CUtensorMap feats_map, const RowsParams p) {
   extern __shared__ uint8_t smem_raw[];
@@ -164,7 +180,7 @@ conv_rows_tcgen05_kernel(const __grid_constant__ CUtensorMap feats_map, const Ro
   const int B_TILE = p.c_out * RB;          // one (offset, channel slice) weight tile
   const int B_SLICE = p.q * B_TILE;         // the chunk's tiles of one channel slice, stacked along N
   const int B_BUF = KB * B_SLICE;
-  const int tiles = (int)p.tiles, grid = (int)gridDim.x;
+  const int grid = (int)gridDim.x;
 
   const uint32_t base = (smem_u32(smem_raw) + 1023u) & ~1023u;
   uint8_t* gen = smem_raw + (base - smem_u32(smem_raw));
@@ -172,8 +188,8 @@ conv_rows_tcgen05_kernel(const __grid_constant__ CUtensorMap feats_map, const Ro
   const uint32_t a_base = b_base + (uint32_t)(p.nbuf * B_BUF);
   RowsControl* ctl = reinterpret_cast<RowsControl*>(gen + p.nbuf * B_BUF + p.stages * A_BYTES);
   auto bar = [](uint64_t* b) { return smem_u32(b); };
-  UnitCursor first{0, 0};
-  first.advance((int)blockIdx.x, tiles);
+  UnitCursor<GROUPED> first{0, 0, 0, min(p.group, (int)p.tiles)};
+  first.advance((int)blockIdx.x, p);
 
   if (tid == 0) ctl->skip = *(volatile int32_t*)p.dev_status;
   __syncthreads();
@@ -181,7 +197,7 @@ conv_rows_tcgen05_kernel(const __grid_constant__ CUtensorMap feats_map, const Ro
   // NaN in the rows of this CTA's units.
   auto mark_rows = [&]() {
     const TO nan = wcn_from_float<TO>(__int_as_float(0x7FC00000));
-    for (UnitCursor c = first; c.chunk < p.nchunks; c.advance(grid, tiles)) {
+    for (UnitCursor<GROUPED> c = first; c.chunk < p.nchunks; c.advance(grid, p)) {
       const int k0 = c.chunk * p.q, qc = min(p.q, p.K - k0);
       for (int i = tid; i < qc * BLOCK_M; i += THREADS) {
         const int64_t row = (int64_t)c.tile * BLOCK_M + (i % BLOCK_M);
@@ -232,7 +248,7 @@ conv_rows_tcgen05_kernel(const __grid_constant__ CUtensorMap feats_map, const Ro
       int bbuf = 0, bphase = 0, cur_chunk = -1;
       bool waited = false;
       int issued = 0;  // row-tile copies issued (for the drain below)
-      for (UnitCursor c = first; c.chunk < p.nchunks && ok; c.advance(grid, tiles)) {
+      for (UnitCursor<GROUPED> c = first; c.chunk < p.nchunks && ok; c.advance(grid, p)) {
         if (c.chunk != cur_chunk) {
           if (cur_chunk >= 0 && ++bbuf == p.nbuf) { bbuf = 0; bphase ^= 1; }
           cur_chunk = c.chunk;
@@ -276,7 +292,7 @@ conv_rows_tcgen05_kernel(const __grid_constant__ CUtensorMap feats_map, const Ro
       uint32_t idesc = 0;
       const uint64_t adesc0 = smem_desc<RB>(a_base), bdesc0 = smem_desc<RB>(b_base);
       uint64_t bdesc_buf = bdesc0;
-      for (UnitCursor c = first; c.chunk < p.nchunks && ok; c.advance(grid, tiles)) {
+      for (UnitCursor<GROUPED> c = first; c.chunk < p.nchunks && ok; c.advance(grid, p)) {
         if (c.chunk != cur_chunk) {
           if (cur_chunk >= 0) {
             umma_commit(bar(&ctl->b_empty[bbuf]));  // the previous chunk's weights may be overwritten
@@ -342,14 +358,14 @@ conv_rows_tcgen05_kernel(const __grid_constant__ CUtensorMap feats_map, const Ro
     // Destination rows of this thread's row in a unit.  They are requested one unit of this warp
     // ahead: the table comes from DRAM and its latency would otherwise sit between every
     // accumulator set and its stores.
-    UnitCursor cur = first;
-    cur.advance(team * grid, tiles);
+    UnitCursor<GROUPED> cur = first;
+    cur.advance(team * grid, p);
     if (team >= teams) cur.chunk = p.nchunks;
     int ab = team, aphase = 0;   // local unit n uses set n % nacc in phase (n / nacc) & 1
     int dnext[MAX_Q];
 #pragma unroll
     for (int o = 0; o < MAX_Q; ++o) dnext[o] = -1;
-    auto load_dsts = [&](const UnitCursor& c) {
+    auto load_dsts = [&](const UnitCursor<GROUPED>& c) {
       const int row = c.tile * BLOCK_M + quarter * 32 + lane;
       const int k0 = c.chunk * p.q, qc = min(p.q, p.K - k0);
 #pragma unroll
@@ -364,8 +380,8 @@ conv_rows_tcgen05_kernel(const __grid_constant__ CUtensorMap feats_map, const Ro
       int dsts[MAX_Q];
 #pragma unroll
       for (int o = 0; o < MAX_Q; ++o) dsts[o] = dnext[o];
-      UnitCursor nxt = cur;
-      nxt.advance(teams * grid, tiles);
+      UnitCursor<GROUPED> nxt = cur;
+      nxt.advance(teams * grid, p);
       if (nxt.chunk < p.nchunks) load_dsts(nxt);
       if (ok) ok = mbar_wait(bar(&ctl->acc_full[ab]), aphase, p.dev_status);
       if (!__all_sync(0xFFFFFFFFu, ok)) { ok = false; break; }  // tcgen05.ld is warp-collective
@@ -456,9 +472,9 @@ EncodeTiledFn encode_tiled() {
   return fn;
 }
 
-template <int BK, bool BF16, typename TO>
+template <int BK, bool BF16, typename TO, bool GROUPED>
 int launch_rows(const CUtensorMap& map, const RowsParams& p, size_t smem, unsigned grid, cudaStream_t st) {
-  auto kern = conv_rows_tcgen05_kernel<BK, BF16, TO>;
+  auto kern = conv_rows_tcgen05_kernel<BK, BF16, TO, GROUPED>;
   static bool configured[64] = {};
   int dev = 0;
   cudaGetDevice(&dev);
@@ -509,6 +525,18 @@ int wcn_conv_rows_tcgen05_fwd(const void* feats, int64_t num_in, int64_t feats_l
   p.K = K; p.c_in = c_in; p.c_out = c_out_packed; p.c_store = c_out;
   p.tiles = (num_in + BLOCK_M - 1) / BLOCK_M;
   p.units = p.tiles * p.nchunks;
+  const int sms = wcn_num_sms();
+  // Every chunk reads all rows, so what is much larger than L2 is worked through in groups of tiles that stay there (whole
+  // rounds of the grid, as the weights change with every chunk of a group).  us, chunks over all rows / in groups of 24 MB (chunks
+  // of up to 256 columns over all rows): 256 -> 96 from 201 000 rows (103 MB, eight chunks) 162 / 107 (111), 256 -> 48 (four) 90 / 68
+  // (84), 128 -> 128 from 424 000 (109 MB) 178 / 171 (207), 96 -> 96 from 300 000 (58 MB) 119 / 102 (111).  Below the line the rows come
+  // from L2 anyway, and the changes of weights and the longer cursor cost 4 to 9 %: 128 -> 64 from 150 000 (38 MB, four) 45 / 49,
+  // 96 -> 64 from 576 000 (111 MB) 131 / 137, 192 -> 32 from 424 000 (163 MB, two) 78 / 85, 256 -> 192 from 74 000 (38 MB) 76 / 80.
+  // Groups of 16 MB are too short for 256 channels (256 -> 192 from 150 000 rows 172, 147 with 24 MB), 32 and 48 MB within 2 %.
+  const int64_t matrix = num_in * c_in * 2, round = (int64_t)sms * BLOCK_M * c_in * 2;
+  const int64_t line = c_in >= 192 && p.nchunks >= 4 ? 350000000ll : 450000000ll;
+  const bool grouped = p.nchunks > 1 && matrix * p.nchunks > line;
+  p.group = (int)(grouped ? sms * (GROUP_BYTES > round ? GROUP_BYTES / round : 1) : p.tiles);
   p.scale = scale; p.shift = shift; p.residual = residual; p.res_ld = residual_ld; p.relu = relu;
   p.out = out; p.out_ld = out_ld; p.dev_status = dev_status;
 
@@ -524,10 +552,11 @@ int wcn_conv_rows_tcgen05_fwd(const void* feats, int64_t num_in, int64_t feats_l
                              CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
   if (rc != CUDA_SUCCESS) return WCN_ERR_UNSUPPORTED_CONFIG;
 
-  const int sms = wcn_num_sms();
   const unsigned grid = (unsigned)(p.units < sms ? p.units : sms);
   const bool bf = dtype == WCN_BF16;
-#define WCN_ROWS_CASE(BKV, BFV, TOV) return launch_rows<BKV, BFV, TOV>(map, p, smem, grid, st)
+#define WCN_ROWS_CASE(BKV, BFV, TOV)                                                   \
+  return p.group < p.tiles ? launch_rows<BKV, BFV, TOV, true>(map, p, smem, grid, st) \
+                           : launch_rows<BKV, BFV, TOV, false>(map, p, smem, grid, st)
   if (out_dtype == WCN_F32) {
     if (bk == 64) { if (bf) WCN_ROWS_CASE(64, true, float); else WCN_ROWS_CASE(64, false, float); }
     else          { if (bf) WCN_ROWS_CASE(32, true, float); else WCN_ROWS_CASE(32, false, float); }
