@@ -290,3 +290,49 @@ def test_fp32_rows_do_not_depend_on_their_launch(c_in, c_out):
         got = sparse_conv_fused(x, w, part, len(range(n)[rows]), split_k=1)
         check_device_status(DEV)
         assert torch.equal(got, whole[rows])
+
+
+def _fastest(f):
+    times = []
+    for _ in range(9):
+        torch.cuda._sleep(400000)   # (the launches are there before the first one starts)
+        start, end = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
+        start.record()
+        f()
+        end.record()
+        torch.cuda.synchronize()
+        times.append(start.elapsed_time(end))
+    return sorted(times)[2]
+
+
+@pytest.mark.parametrize("n,c_out", [(300, 176), (19000, 208), (2000, 272), (20000, 400)])
+def test_fp32_column_blocks_of_different_widths(n, c_out):
+    """Widths above 128 columns that equal blocks of sixteens do not divide well, with offsets divided among a cluster and not:
+    against sums in 64 bits, forward and weight gradient (the bounds above)."""
+    from warpconvnet_b200.nn.functional import sparse_conv as sc
+    g = torch.Generator(device=DEV).manual_seed(c_out)
+    kmap = _random_map(27, n, n, g)
+    nbr = kmap.neighbor_table(n)
+    x, dy = torch.randn(n, 48, generator=g, device=DEV), torch.randn(n, c_out - 12, generator=g, device=DEV)
+    w = torch.randn(27, 48, c_out, generator=g, device=DEV)
+    rows = [x[nbr[k].clamp(min=0).long()].double().mul((nbr[k] >= 0)[:, None]) for k in range(27)]
+    want = sum(rows[k] @ w[k].double() for k in range(27)), torch.stack([r.T @ dy.double() for r in rows])
+    got = sparse_conv_fused(x, w, kmap, n), sc.sparse_conv_wgrad(x, dy, kmap, n)
+    check_device_status(DEV)
+    for y, e, limit in zip(got, want, (3e-7, 4e-7)):
+        assert float((y.double() - e).norm() / e.norm()) < limit
+
+
+def test_fp32_column_blocks_are_few():
+    """A layer gathers its rows once per column block: 208 columns take two blocks, not thirteen of sixteen, and a gradient of
+    160 two, not five (5.1 and 3.3 times a layer of 112 and a gradient of 80 columns before, 1.6 and 1.7 times with two)."""
+    from warpconvnet_b200.nn.functional import sparse_conv as sc
+    g = torch.Generator(device=DEV).manual_seed(0)
+    n = 40000
+    kmap = _random_map(27, n, n, g)
+    x = torch.randn(n, 64, generator=g, device=DEV)
+    layer = lambda c: _fastest(lambda w=torch.randn(27, 64, c, generator=g, device=DEV): sparse_conv_fused(x, w, kmap, n))
+    grad = lambda c: _fastest(lambda dy=torch.randn(n, c, generator=g, device=DEV): sc.sparse_conv_wgrad(x, dy, kmap, n))
+    ratio = layer(208) / layer(112), grad(160) / grad(80)
+    assert ratio[0] < 3 and ratio[1] < 2.6
+    check_device_status(DEV)

@@ -59,7 +59,7 @@ struct SplitParams {
   const int32_t* out_rows;
   int64_t M, in_ld, out_ld, res_ld;
   int K, c_in, cp, c_out, num_in;
-  int block_n, blocks;     // columns of a unit, column blocks
+  int block_n, blocks;     // columns of a unit (of the last column block: what is left), column blocks
   int tiles, window, tail; // row tiles; see tile_of
   int S;                   // CTAs of a cluster that divide the offsets of a unit: slice s has those with k % S == s
   int slots;
@@ -195,6 +195,7 @@ conv_split_kernel(const SplitParams p) {
   SplitControl* ctl = reinterpret_cast<SplitControl*>(smem_raw + (base - smem_u32(smem_raw)) + p.slots * slot_bytes);
   auto bar = [](uint64_t* b) { return smem_u32(b); };
   const int units = p.tiles * p.blocks;
+  auto columns_of = [&](int unit) { return min(BN, p.c_out - unit % p.blocks * BN); };
   const int first = p.S > 1 ? (int)blockIdx.x / p.S : (int)blockIdx.x, rank = p.S > 1 ? (int)blockIdx.x % p.S : 0;
 
   if (warp == 0) {
@@ -329,15 +330,16 @@ conv_split_kernel(const SplitParams p) {
         mbar_arrive(bar(&ctl->info_empty[ib]));
         if (unit < 0) break;
         const int n0 = (unit % p.blocks) * BN;
+        const uint32_t bytes = (uint32_t)(columns_of(unit) * SP_RB);
         for (; rest && ok; rest &= rest - 1) {
           const char* src = p.wplanes + ((int64_t)(__ffs(rest) - 1) * KB * 3 * p.c_out + n0) * SP_RB;
           for (int kb = 0; kb < KB; ++kb) {
             if (!mbar_wait(bar(&ctl->empty[slot]), phase ^ 1, p.dev_status)) { ok = false; break; }
             const uint32_t dst = base + slot * slot_bytes + 3 * SP_PLANE, full = bar(&ctl->full[slot]);
-            mbar_expect_tx(full, (uint32_t)(3 * b_bytes));
+            mbar_expect_tx(full, 3 * bytes);
 #pragma unroll
             for (int s = 0; s < 3; ++s)
-              bulk_copy_g2s(dst + s * b_bytes, src + (int64_t)(kb * 3 + s) * p.c_out * SP_RB, (uint32_t)b_bytes, full);
+              bulk_copy_g2s(dst + s * b_bytes, src + (int64_t)(kb * 3 + s) * p.c_out * SP_RB, bytes, full);
             if (++slot == p.slots) { slot = 0; phase ^= 1; }
           }
         }
@@ -349,7 +351,7 @@ conv_split_kernel(const SplitParams p) {
     // Two threads take the slots in turns: what one of them waits and signals between its instructions (some 250 clocks a
     // slot, of 690) the other's fill.
     if (elect_one()) {
-      const uint32_t idesc = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(BN >> 3) << 17) | ((uint32_t)(SP_M >> 4) << 24);
+      const uint32_t idesc0 = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(SP_M >> 4) << 24);
       const int mine = warp - SP_MMA_WARP;
       int slot = 0, phase = 0, ab = 0, aphase = 0, turn = 0;
       for (int n = 0; ok; ++n) {
@@ -359,6 +361,7 @@ conv_split_kernel(const SplitParams p) {
         const int steps = __popc(ctl->info_mask[ib]) * KB;
         mbar_arrive(bar(&ctl->info_empty[ib]));
         if (unit < 0) break;
+        const uint32_t idesc = idesc0 | ((uint32_t)(columns_of(unit) >> 3) << 17);
         for (int i = 0; i < steps; ++i) {
           if (turn == mine) {
             if (!mbar_wait(bar(&ctl->acc_empty[ab]), aphase ^ 1, p.dev_status) ||
@@ -385,8 +388,6 @@ conv_split_kernel(const SplitParams p) {
   } else {
     // ================================================================ sums and epilogue
     const int half = warp >> 2, row = tid & (SP_M - 1);
-    const int middle = ((BN / 16 + 1) / 2) * 16;
-    const int c_begin = half ? middle : 0, cols = half ? BN - middle : middle;   // at most 64 columns a thread
     int ab = 0, aphase = 0;
     for (int n = 0; ok; ++n) {
       const int ib = n & 1;
@@ -398,6 +399,8 @@ conv_split_kernel(const SplitParams p) {
       __syncwarp();
       if (lane == 0) mbar_arrive(bar(&ctl->info_empty[ib]));
       if (unit < 0) break;
+      const int bn = columns_of(unit), middle = ((bn / 16 + 1) / 2) * 16;
+      const int c_begin = half ? middle : 0, cols = half ? bn - middle : middle;   // at most 64 columns a thread
       float sum[64];
 #pragma unroll
       for (int i = 0; i < 64; ++i) sum[i] = 0.f;
@@ -474,7 +477,7 @@ conv_split_kernel(const SplitParams p) {
     cluster_meet();
     const bool poison = *(volatile const int32_t*)p.dev_status == (int)WCN_ERR_WAIT_EXPIRED;
     const int64_t m0 = (int64_t)tile_of(p, first / p.blocks) * SP_M;
-    const int n0 = (first % p.blocks) * BN, per_row = BN / 4;
+    const int n0 = (first % p.blocks) * BN, per_row = columns_of(first) / 4;
     const int r0 = rank * SP_M / p.S, r1 = (rank + 1) * SP_M / p.S;
     for (int i = tid; i < (r1 - r0) * per_row; i += SP_THREADS) {
       const int r = r0 + i / per_row, c = (i % per_row) * 4;
@@ -510,9 +513,11 @@ struct SplitPlan {
 SplitPlan plan_split(int64_t num_in, int K, int c_in, int c_out) {
   SplitPlan q;
   q.cp = (c_in + SP_BK - 1) / SP_BK * SP_BK;
+  // As few column blocks as there can be (each gathers all rows again), about equally wide; c_out is a multiple of 16.  (Blocks
+  // of one width: 64 -> 208 columns were thirteen, 100 000 room / outdoor voxels 632 / 644 us, two take 206 / 198.)
   q.blocks = (c_out + SP_MAX_N - 1) / SP_MAX_N;
-  while (c_out % (16 * q.blocks) != 0) ++q.blocks;   // (c_out is a multiple of 16)
-  q.block_n = c_out / q.blocks;
+  q.block_n = (c_out / 16 + q.blocks - 1) / q.blocks * 16;
+  q.blocks = (c_out + q.block_n - 1) / q.block_n;
   q.weights = (size_t)K * q.cp * c_out * 6;
   q.rows = (size_t)num_in * q.cp * 6;
   return q;

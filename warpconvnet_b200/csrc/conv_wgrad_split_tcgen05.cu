@@ -100,6 +100,7 @@ conv_wgrad_split_kernel(const WsParams p) {
   const int block = (int)blockIdx.x % p.blocks, turn = ((int)blockIdx.x / p.blocks) % p.groups, range = (int)blockIdx.x / (p.blocks * p.groups);
   const int middle = (p.groups - 1) / 2;
   const int group = (turn & 1) ? middle + (turn + 1) / 2 : middle - turn / 2;
+  const int bn = min(BN, p.gchunks * 32 - block * BN);   // (the last column block may be narrower)
   const int cpc = p.cp / 32, chunks = p.K * cpc;
   const int t0 = range * p.per_range, t1 = min(p.tiles, t0 + p.per_range);
   uint32_t offsets = 0;
@@ -130,7 +131,7 @@ conv_wgrad_split_kernel(const WsParams p) {
   tc_fence_after();
   const uint32_t tmem = ctl->tmem;
   const int steps = ctl->count * 4;
-  bool ok = true;
+  bool ok = true, redo = false;
 
   if (warp >= 8 && warp < WS_MMA_WARP) {
     // ================================================================ gather: a chunk per warp
@@ -192,9 +193,9 @@ conv_wgrad_split_kernel(const WsParams p) {
         if (!mbar_wait(bar(&ctl->empty[slot]), phase ^ 1, p.dev_status)) { ok = false; break; }
         const uint32_t dst = base + slot * slot_bytes + WS_A, full = bar(&ctl->full[slot]);
         const char* src = p.images + ((int64_t)ctl->tile[i >> 2] * 4 + (i & 3)) * 3 * part + (int64_t)block * b_bytes;
-        mbar_expect_tx(full, (uint32_t)(3 * b_bytes));
+        mbar_expect_tx(full, (uint32_t)(3 * bn * 64));
 #pragma unroll
-        for (int s = 0; s < 3; ++s) bulk_copy_g2s(dst + s * b_bytes, src + s * part, (uint32_t)b_bytes, full);
+        for (int s = 0; s < 3; ++s) bulk_copy_g2s(dst + s * b_bytes, src + s * part, (uint32_t)(bn * 64), full);
         if (++slot == p.slots) { slot = 0; phase ^= 1; }
       }
     }
@@ -202,8 +203,8 @@ conv_wgrad_split_kernel(const WsParams p) {
   } else if (warp == WS_MMA_WARP || warp == WS_MMA_WARP + 1) {
     // ================================================================ tensor-core instructions, slots in turns
     if (elect_one()) {
-      // fp32 accumulate, bf16, A and B MN-major (bits 15, 16), N = BN, M = 128
-      const uint32_t idesc = (1u << 4) | (1u << 7) | (1u << 10) | (1u << 15) | (1u << 16) | ((uint32_t)(BN >> 3) << 17) | (8u << 24);
+      // fp32 accumulate, bf16, A and B MN-major (bits 15, 16), N = bn, M = 128
+      const uint32_t idesc = (1u << 4) | (1u << 7) | (1u << 10) | (1u << 15) | (1u << 16) | ((uint32_t)(bn >> 3) << 17) | (8u << 24);
       int slot = 0, phase = 0, ab = 0, aphase = 0;
       for (int i = 0; i < steps; ++i) {
         if ((i & 1) == warp - WS_MMA_WARP) {
@@ -228,8 +229,8 @@ conv_wgrad_split_kernel(const WsParams p) {
     __syncwarp();
   } else if (warp < 8) {
     // ================================================================ sums: a row of the group per thread, half of its columns
-    const int half = warp >> 2, mid = ((BN / 16 + 1) / 2) * 16;
-    const int c_begin = half ? mid : 0, cols = half ? BN - mid : mid;   // at most 64 columns a thread
+    const int half = warp >> 2, mid = ((bn / 16 + 1) / 2) * 16;
+    const int c_begin = half ? mid : 0, cols = half ? bn - mid : mid;   // at most 64 columns a thread
     float sum[64];
 #pragma unroll
     for (int i = 0; i < 64; ++i) sum[i] = 0.f;
@@ -275,22 +276,23 @@ conv_wgrad_split_kernel(const WsParams p) {
         }
     }
     const uint32_t any = __reduce_or_sync(0xFFFFFFFFu, mine);
-    if (any) {
+    redo = any != 0;
+    if (redo) {
       ctl->odd[half][tid & 127] = mine;
       if (lane == 0) ctl->again[half][warp & 3] = any;
     }
   }
   tc_fence_before();
-  __syncthreads();
+  redo = __syncthreads_or(redo);
   // A number without three parts, or one beside an absent row (0 times infinity): such sums are made again on the FMA pipes
   // from the present pairs, up to eight fours of a chunk at a time.  All warps take slots of 32 rows in turns, their sums
   // are added in order through the ring, which nothing uses any more (60 000 room voxels, 64 -> 64, 101 us: 357 with a NaN in
   // a row of X and one of dY, 930 with nothing else, 175 in conv_wgrad_pairs.cu; one thread per sum walking all rows took
   // 20 000, an epilogue warp on its own 808 and 1 629).
   float* part = reinterpret_cast<float*>(smem_raw + (base - smem_u32(smem_raw)));
-  for (int i = 0; i < 2 * WS_CHUNKS; ++i) {
+  for (int i = 0; redo && i < 2 * WS_CHUNKS; ++i) {
     const int half = i / WS_CHUNKS, w = i % WS_CHUNKS, q = group * WS_CHUNKS + w, k = q / cpc, ci = (q % cpc) * 32 + lane;
-    const int n0 = block * BN + (half ? ((BN / 16 + 1) / 2) * 16 : 0);
+    const int n0 = block * BN + (half ? ((bn / 16 + 1) / 2) * 16 : 0);
     for (uint32_t rest = ctl->again[half][w]; rest;) {
       int col[8], fours = 0;
 #pragma unroll
@@ -376,9 +378,9 @@ WsPlan plan_ws(int64_t num_in, int64_t M, int K, int c_in, int c_out) {
   q.cp = (c_in + 31) / 32 * 32;
   q.gchunks = (c_out + 31) / 32;
   q.groups = (K * (q.cp / 32) + WS_CHUNKS - 1) / WS_CHUNKS;
-  q.blocks = (q.gchunks + 3) / 4;
-  while (q.gchunks % q.blocks) ++q.blocks;
-  q.block_n = q.gchunks / q.blocks * 32;
+  q.blocks = (q.gchunks + 3) / 4;   // as few as there can be: each gathers all rows of X again (64 -> 160 columns in five: 435 us, two 263)
+  q.block_n = (q.gchunks + q.blocks - 1) / q.blocks * 32;
+  q.blocks = (q.gchunks * 32 + q.block_n - 1) / q.block_n;
   q.tiles = (int)((M + 127) / 128);
   // Three CTAs a multiprocessor or more (they differ in what they have to do), of at least four tiles each.
   const int64_t work = (int64_t)q.groups * q.blocks;
