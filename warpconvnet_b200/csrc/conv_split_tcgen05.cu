@@ -256,14 +256,6 @@ conv_split_kernel(const SplitParams p) {
         ctl->mask_acc[acc == 2 ? 0 : acc + 1] = 0;
         ctl->info_unit[ib] = unit;
         ctl->info_mask[ib] = mask;
-        if (p.S == 1) {
-          // (every gather thread has read the last claim: they met since)
-          asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-          mbar_expect_tx(bar(&ctl->claim_full), 16u);
-          asm volatile("clusterlaunchcontrol.try_cancel.async.shared::cta.mbarrier::complete_tx::bytes.b128 [%0], [%1];" ::"r"(
-                           smem_u32(&ctl->claim[0])), "r"(bar(&ctl->claim_full))
-                       : "memory");
-        }
       }
       __syncwarp();
       mbar_arrive(bar(&ctl->info_full[ib]));
@@ -288,7 +280,18 @@ conv_split_kernel(const SplitParams p) {
           if (++slot == p.slots) { slot = 0; phase ^= 1; }
         }
       }
-      // the next unit (the claim has had this unit's copies to arrive; on failure it still has to, it writes shared memory)
+      // The next unit is claimed when this one's copies have been issued: a multiprocessor with a long unit leaves those that are
+      // left to others (asked for before the copies, by whoever started first: 20 000 / 25 000 / 60 000 room voxels, 128 -> 128, 128,
+      // 96 channels 93 / 98 / 116 us, now 69 / 72 / 111; 20 000 cells, 32 -> 32 25.0 / 22.8).
+      if (p.S == 1 && gtid == 0) {
+        // (every gather thread has read the last claim: they met since)
+        asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+        mbar_expect_tx(bar(&ctl->claim_full), 16u);
+        asm volatile("clusterlaunchcontrol.try_cancel.async.shared::cta.mbarrier::complete_tx::bytes.b128 [%0], [%1];" ::"r"(
+                         smem_u32(&ctl->claim[0])), "r"(bar(&ctl->claim_full))
+                     : "memory");
+      }
+      // (on failure the claim still has to arrive: it writes shared memory)
       uint32_t got = 0, x = 0;
       if (p.S == 1) {
         if (!mbar_wait(bar(&ctl->claim_full), claim_phase, p.dev_status)) {
