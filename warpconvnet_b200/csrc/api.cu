@@ -118,7 +118,18 @@ extern "C" int wcn_conv_f32_workspace_bytes(int64_t num_in, int64_t num_out, int
   const int64_t area = (int64_t)c_in * c_out;
   const bool row_per_thread = wcn_conv_narrow_out_supported(num_offsets, c_in, c_out, WCN_F32, nullptr, c_in);
   const bool few = num_offsets == 1 ? area < 12288 || num_out < 12000 : area < 2048 && num_out < 12000 && !row_per_thread;
-  *bytes = num_in > 0 && num_out > 0 && !few && wcn_conv_split_supported(num_offsets, c_in, c_out)
+  // The other way round for the narrowest: rows of 16 channels become planes of 32, written and read, while one thread per row
+  // or few offsets are little work (8 offsets, 16 -> 16: 100 000 rows 37 / 42, 1 000 000 150 / 271, 16 -> 32 up to 150 000 rows alike,
+  // 250 000 108 / 128; 27 offsets, 16 -> 16: 100 000 100 / 56, 300 000 127 / 132, outdoors 140 / 161).
+  const bool narrow = area <= 1024 && (c_in < 32 || c_out < 32) && (row_per_thread || num_offsets <= 8) &&
+                      num_out >= (num_offsets <= 8 ? 150000 : 250000);
+  // Planes are made of all input rows, so that a launch over a small part of the output rows (a boundary, a crop) may be done
+  // sooner without them: 2 ns per 1 000 input numbers against what an output row gains (us, 27 offsets, from 1 000 000 rows: 64 -> 64
+  // for 15 625 rows 70 / 148, for 62 500 202 / 173, outdoors 44 / 146 and 123 / 161; 128 -> 128 208 / 288, 650 / 343).
+  const double planes = 2e-6 * (double)num_in * ((c_in + 31) / 32 * 32);
+  const bool part = num_in > 8 * num_out &&
+                    planes > (1e-3 + 2.7e-7 * (double)area) * num_offsets / 27 * (double)num_out + 3.7e-3 * (double)area;
+  *bytes = num_in > 0 && num_out > 0 && !few && !narrow && !part && wcn_conv_split_supported(num_offsets, c_in, c_out)
                ? wcn_conv_split_workspace(num_in, num_offsets, c_in, c_out) : 0;
   return WCN_OK;
 }

@@ -410,7 +410,10 @@ extern "C" int wcn_conv_wgrad_f32_workspace_bytes(int64_t num_in, int64_t num_ou
   // Few offsets stay on the FP32 pipes (8 of them, 60 000 rows of 64 -> 64: 50 us / 42 in a room, 32 / 74 outdoors: the three
   // parts are as much to write as the gradient is to read), and narrow layers, where the two take the same time (32 -> 32,
   // 27 offsets, 60 000 rows: 79 / 69, outdoors 58 / 64).
-  if (num_offsets < 16 || (int64_t)c_in * c_out < 2048 || !wgrad_split_supported(num_in, num_out, num_offsets, c_in, c_out)) return WCN_OK;
+  // So do a few rows of a large matrix, all of whose rows would be split (see wcn_conv_f32_workspace_bytes).
+  const double area = (double)c_in * c_out;
+  if (num_in > 8 * num_out && 2e-6 * (double)num_in * ((c_in + 31) / 32 * 32) > 25. + 3.7e-7 * area * (double)num_out) return WCN_OK;
+  if (num_offsets < 16 || area < 2048 || !wgrad_split_supported(num_in, num_out, num_offsets, c_in, c_out)) return WCN_OK;
   const WsPlan q = plan_ws(num_in, num_out, num_offsets, c_in, c_out);
   *bytes = (int64_t)(q.planes + q.images + q.partial);
   return WCN_OK;
