@@ -336,3 +336,13 @@ def test_fp32_column_blocks_are_few():
     ratio = layer(208) / layer(112), grad(160) / grad(80)
     assert ratio[0] < 3 and ratio[1] < 2.6
     check_device_status(DEV)
+
+
+@pytest.mark.parametrize("n,c", [(300000, 1024), (800000, 256), (1000000, 16)])
+def test_column_sums_of_many_rows(n, c):
+    """A thread adds hundreds to thousands of rows of these.  Trees of eight numbers in fp32 (three additions deep, each half a
+    unit of 2^-24 off at most) and a result rounded once, everything else in double: below 1e-7 of the sums' 2-norm."""
+    from warpconvnet_b200.nn.functional.sparse_conv import _column_sums
+    x = torch.randn(n, c, generator=torch.Generator(device=DEV).manual_seed(c), device=DEV)
+    want = x.sum(0, dtype=torch.float64)
+    assert float((_column_sums(x).double() - want).norm() / want.norm()) < 1e-7
