@@ -346,3 +346,38 @@ def test_column_sums_of_many_rows(n, c):
     x = torch.randn(n, c, generator=torch.Generator(device=DEV).manual_seed(c), device=DEV)
     want = x.sum(0, dtype=torch.float64)
     assert float((_column_sums(x).double() - want).norm() / want.norm()) < 1e-7
+
+
+@pytest.mark.parametrize("frozen", [True, False])
+@pytest.mark.parametrize("dtype", [torch.float32, torch.float16])
+def test_gradient_of_a_bias_alone(dtype, frozen):
+    """A layer of which only the bias trains keeps nothing for the backward pass; the gradient of a bias alone does not run the
+    layer's, one by one, in batches (``is_grads_batched``) and, as a tangent, in forward mode."""
+    import torch.autograd.forward_ad as fwd
+    from warpconvnet_b200._native import LAUNCH_COUNTS
+    coords = room_rows(3000)
+    vox = make_voxels(coords, torch.randn(len(coords), 32, generator=torch.Generator().manual_seed(1)).to(dtype)).sort()
+    torch.manual_seed(0)
+    layer = SparseConv3d(32, 48, 3, bias=True).to(DEV).to(dtype)
+    layer.weight.requires_grad_(not frozen)
+    kept = []
+    with torch.autograd.graph.saved_tensors_hooks(lambda t: (kept.append(t), t)[1], lambda t: t):
+        y = layer(vox).feature_tensor
+    assert type(y.grad_fn).__name__ == "_BiasFunctionBackward" and len(kept) == (0 if frozen else 2)
+    dys = torch.randn(3, *y.shape, generator=torch.Generator(device=DEV).manual_seed(2), device=DEV).to(dtype)
+    want = dys.double().sum(1)
+    close = lambda a, b: rel_l2(a.double().cpu().numpy(), b.cpu().numpy()) < (1e-6 if dtype == torch.float32 else 1e-3)
+    LAUNCH_COUNTS.clear()
+    for dy, w in zip(dys, want):
+        assert close(torch.autograd.grad(y, [layer.bias], dy, retain_graph=True)[0], w)
+    assert LAUNCH_COUNTS["wcn_column_sums"] == 3 * 2 and not any(c for k, c in LAUNCH_COUNTS.items() if "conv" in k)
+    assert close(torch.autograd.grad(y, [layer.bias], dys, is_grads_batched=True)[0], want)
+    if frozen:  # (without a parameter that trains a call is one of inference)
+        return
+    with fwd.dual_level():
+        bias = layer.bias
+        del layer.bias
+        layer.bias = fwd.make_dual(bias.detach(), torch.full_like(bias.detach(), 0.5))
+        tangent = fwd.unpack_dual(layer(vox).feature_tensor).tangent
+        assert tangent is not None and torch.equal(tangent, torch.full_like(y, 0.5))
+    check_device_status(DEV)

@@ -1332,16 +1332,16 @@ class _LayerFunction(torch.autograd.Function):
     deriving the launches from a kernel map's options on every call."""
 
     @staticmethod
-    def forward(ctx, x: Tensor, weight: Tensor, tables: _LayerTables):
+    def forward(ctx, x: Tensor, weight: Tensor, tables: _LayerTables, bias: Optional[Tensor]):
         ctx.tables = tables
         ctx.save_for_backward(x, weight)
-        return _layer_output(x.detach(), weight, tables)
+        return _layer_output(x.detach(), weight, tables, bias)
 
     @staticmethod
     def backward(ctx, g: Tensor):
         x, weight = ctx.saved_tensors
         gx, gw = _layer_gradients(g, x, weight, ctx.tables, *ctx.needs_input_grad[:2])
-        return gx, gw, None
+        return gx, gw, None, None
 
 
 def _column_sums(g: Tensor) -> Tensor:
@@ -1357,26 +1357,25 @@ def _column_sums(g: Tensor) -> Tensor:
     return sums
 
 
-class _LayerBiasFunction(torch.autograd.Function):
-    """A layer in training with its bias, which the convolution's epilogue adds: beside :class:`_LayerFunction` that was an
-    addition and a reduction through torch, 38 us of the 270 that a layer of 60 000 fp32 rows of 64 channels takes."""
+class _BiasFunction(torch.autograd.Function):
+    """The bias that a convolution's epilogue has added to ``y`` already, as a node of its own: beside it stood an addition and
+    a reduction through torch, 38 us of the 270 that a layer of 60 000 fp32 rows of 64 channels takes.  (Part of the layer's node,
+    a gradient of the bias alone ran the layer's own gradients too, and a layer of which only the bias trains kept its input.)"""
 
     @staticmethod
-    def forward(ctx, x: Tensor, weight: Tensor, bias: Tensor, tables: _LayerTables):
-        ctx.tables, ctx.bias_dtype = tables, bias.dtype
-        ctx.save_for_backward(x, weight)
-        return _layer_output(x.detach(), weight, tables, bias.detach())
+    def forward(ctx, y: Tensor, bias: Tensor):
+        ctx.bias_dtype = bias.dtype
+        ctx.mark_dirty(y)
+        return y
 
     @staticmethod
     def backward(ctx, g: Tensor):
-        x, weight = ctx.saved_tensors
-        need_x, need_w, need_b = ctx.needs_input_grad[:3]
-        gx, gw = _layer_gradients(g, x, weight, ctx.tables, need_x, need_w) if need_x or need_w else (None, None)
         gb = None
-        if need_b:  # (through torch where a graph of the gradient is wanted)
-            gb = g.sum(0, dtype=torch.float32) if torch.is_grad_enabled() else _column_sums(g.contiguous())
-            gb = gb.to(ctx.bias_dtype)
-        return gx, gw, gb, None
+        if ctx.needs_input_grad[1]:
+            # (through torch where a graph of the gradient is wanted, and for batches of gradients, which have no memory of their own)
+            native = not torch.is_grad_enabled() and torch._C._has_storage(g)
+            gb = (_column_sums(g.contiguous()) if native else g.sum(0, dtype=torch.float32)).to(ctx.bias_dtype)
+        return g if ctx.needs_input_grad[0] else None, gb
 
 
 class _LayerNormFunction(torch.autograd.Function):
@@ -1396,7 +1395,7 @@ class _LayerNormFunction(torch.autograd.Function):
         x, weight, gamma, beta, residual, z, stats, y = ctx.saved_tensors
         need = ctx.needs_input_grad[:5]
         if torch.is_grad_enabled():  # a graph of the gradient is wanted: the two steps as they are without this function
-            out = batch_norm.formula(_LayerFunction.apply(x, weight, ctx.tables), gamma, beta, residual, ctx.eps, ctx.relu)
+            out = batch_norm.formula(_LayerFunction.apply(x, weight, ctx.tables, None), gamma, beta, residual, ctx.eps, ctx.relu)
             got = iter(torch.autograd.grad(out, [t for t, n in zip((x, weight, gamma, beta, residual), need) if n], dy,
                                            create_graph=True))
             return tuple(next(got) if n else None for n in need) + (None, None, None)
@@ -1500,9 +1499,9 @@ def train_layer(layer, x: Voxels, target: Optional[Voxels]) -> Optional[Voxels]:
             return None
         if (bias is not None and bias.dim() == 1 and bias.shape[0] == weight.shape[2] and bias.device == feats.device
                 and bias.dtype in _NATIVE_DTYPES and batch_norm.reverse_mode_only()):
-            y, bias = _LayerBiasFunction.apply(feats, weight, bias, found[0]), None
+            y, bias = _BiasFunction.apply(_LayerFunction.apply(feats, weight, found[0], bias.detach()), bias), None
         else:
-            y = _LayerFunction.apply(feats, weight, found[0])
+            y = _LayerFunction.apply(feats, weight, found[0], None)
     if bias is not None:
         y = y + bias.to(y.dtype)
     return x._derive(y) if pointwise else _output_of(layer, x, *found, y)
