@@ -358,6 +358,8 @@ int wcn_conv_workspace_bytes(int algo, int64_t num_out, int32_t num_offsets, int
  * where it does not.  Any 16-byte aligned device memory, used from the first launch of the call to its last.
  * No reference counterpart. */
 int wcn_conv_f32_workspace_bytes(int64_t num_in, int64_t num_out, int32_t num_offsets, int32_t c_in, int32_t c_out, int64_t* bytes);
+/* Kernels that this thread's last wcn_conv_fwd or wcn_conv_wgrad_f32 launched (with a workspace or partial sums more than one). */
+int wcn_conv_f32_launches(void);
 
 /* Output-stationary sparse convolution with a fused epilogue:
  *   acc[s, :] = sum_k feats[nbr[k*M + s], :] @ weight[k]      (rows with nbr < 0 skipped, fp32 accumulation)

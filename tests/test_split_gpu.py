@@ -381,3 +381,45 @@ def test_gradient_of_a_bias_alone(dtype, frozen):
         tangent = fwd.unpack_dual(layer(vox).feature_tensor).tangent
         assert tangent is not None and torch.equal(tangent, torch.full_like(y, 0.5))
     check_device_status(DEV)
+
+
+def test_fp32_launches_are_counted():
+    """Planes and convolution are two kernels, the FP32 pipes one; the weight gradient has a third where there are partial sums."""
+    from warpconvnet_b200._native import LAUNCH_COUNTS
+    from warpconvnet_b200.nn.functional import sparse_conv as sc
+    g = torch.Generator(device=DEV).manual_seed(0)
+
+    def counted(n, c, name, f):
+        kmap = _random_map(27, n, n, g)
+        kmap.tile_masks(n)
+        x, y, w = (torch.randn(*shape, generator=g, device=DEV) for shape in ((n, c), (n, c), (27, c, c)))
+        LAUNCH_COUNTS.clear()
+        f(x, y, w, kmap, n)
+        return LAUNCH_COUNTS[name]
+
+    forward, gradient = lambda x, y, w, kmap, n: sparse_conv_fused(x, w, kmap, n), lambda x, y, w, kmap, n: sc.sparse_conv_wgrad(x, y, kmap, n)
+    assert counted(3000, 64, "wcn_conv_fwd", forward) == 2 and counted(3000, 36, "wcn_conv_fwd", forward) == 1
+    assert counted(400, 64, "wcn_conv_wgrad_f32", gradient) == 2 and counted(20000, 64, "wcn_conv_wgrad_f32", gradient) == 3
+    check_device_status(DEV)
+
+
+def test_fp32_kernels_are_loud_after_an_expired_wait():
+    """While the status word holds an expired wait the fp32 kernels write NaN, sums that are made again among them."""
+    from warpconvnet_b200._native import device_status, lib, ptr, stream_ptr
+    from warpconvnet_b200.nn.functional import sparse_conv as sc
+    g = torch.Generator(device=DEV).manual_seed(0)
+    n, dev = 6000, torch.device(DEV)
+    kmap = _random_map(27, n, n, g)
+    x, dy, w = (torch.randn(*shape, generator=g, device=DEV) for shape in ((n, 64), (n, 64), (27, 64, 64)))
+    calls = [lambda s=s: sparse_conv_fused(x, w, kmap, n, split_k=s) for s in (1, 4)] + [lambda: sc.sparse_conv_wgrad(x, dy, kmap, n)]
+    x[5, 5] = float("inf")
+    right = [f() for f in calls]
+    check_device_status(DEV)
+    assert lib().wcn_selftest_bounded_wait(200_000, ptr(device_status(dev)), None, stream_ptr(dev)) == 0
+    loud = [f() for f in calls]
+    torch.cuda.synchronize()
+    with pytest.raises(RuntimeError, match="expired"):
+        check_device_status(DEV)
+    assert all(bool(torch.isnan(y).all()) for y in loud)
+    assert all(torch.equal(a.nan_to_num(1.0), f().nan_to_num(1.0)) for a, f in zip(right, calls))
+    check_device_status(DEV)

@@ -65,6 +65,7 @@ SIGNATURES = {
     "wcn_conv_wgrad_pairs_workspace_bytes": [_c_i64, _c_i32, _c_i32, _c_i32, _p_i64],
     "wcn_conv_wgrad_pairs": [_c_vp, _c_i64, _c_vp, _c_vp, _c_vp, _c_i64, _c_i32, _c_i32, _c_i32, _c_i32, _c_vp, _c_vp, _c_i64, _c_vp, _c_vp],
     "wcn_conv_workspace_bytes": [_c_i32, _c_i64, _c_i32, _c_i32, _c_i32, _c_i32, _c_i32, _c_i32, _p_i64],
+    "wcn_conv_f32_launches": [],
     "wcn_conv_f32_workspace_bytes": [_c_i64, _c_i64, _c_i32, _c_i32, _c_i32, _p_i64],
     "wcn_conv_fwd": [_c_i32, _c_vp, _c_i64, _c_i64, _c_vp, _c_vp, _c_vp, _c_vp, _c_i64, _c_i32, _c_i32, _c_i32, _c_i32,
                      _c_vp, _c_vp, _c_vp, _c_i64, _c_i32, _c_vp, _c_i64, _c_i32, _c_i32, _c_vp, _c_i64, _c_vp, _c_vp],
@@ -155,6 +156,12 @@ class _Library:
         handle.wcn_status_string.argtypes, handle.wcn_status_string.restype = [ctypes.c_int], ctypes.c_char_p
         handle.wcn_brick_usable_flag.argtypes, handle.wcn_brick_usable_flag.restype = [ctypes.c_void_p], ctypes.c_void_p
         self.wcn_status_string, self.wcn_brick_usable_flag = handle.wcn_status_string, handle.wcn_brick_usable_flag
+
+
+def count_f32_launches(name: str) -> None:
+    """Corrects what the call just made was counted as: with a workspace ``wcn_conv_fwd`` launches one or two kernels,
+    ``wcn_conv_wgrad_f32`` two or three."""
+    LAUNCH_COUNTS[name] += lib().wcn_conv_f32_launches() - KERNELS_PER_CALL[name]
 
 
 def launches_total() -> int:

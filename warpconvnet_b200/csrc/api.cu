@@ -28,6 +28,7 @@ int wcn_conv_fp32_fwd(const void* feats, int64_t num_in, int64_t feats_ld, const
                       int64_t out_ld, int sms, int split_k, int32_t* dev_status, cudaStream_t st);
 // conv_split_tcgen05.cu
 bool wcn_conv_split_supported(int K, int c_in, int c_out);
+thread_local int wcn_f32_launches = 0;   // see wcn_conv_f32_launches
 int64_t wcn_conv_split_workspace(int64_t num_in, int K, int c_in, int c_out);
 int wcn_conv_split_fwd(const void* feats, int64_t num_in, int64_t feats_ld, const void* weight, const int32_t* nbr,
                        const int32_t* out_rows, int64_t M, int K, int c_in, int c_out, const float* scale, const float* shift,
@@ -134,6 +135,8 @@ extern "C" int wcn_conv_f32_workspace_bytes(int64_t num_in, int64_t num_out, int
   return WCN_OK;
 }
 
+extern "C" int wcn_conv_f32_launches(void) { return wcn_f32_launches; }
+
 extern "C" int wcn_conv_fwd(int algo, const void* feats, int64_t num_in, int64_t feats_ld, const void* weight,
                             const void* packed_weight, const int32_t* nbr, const int32_t* out_rows,
                             int64_t num_out, int32_t num_offsets, int32_t c_in, int32_t c_out, int dtype,
@@ -150,6 +153,7 @@ extern "C" int wcn_conv_fwd(int algo, const void* feats, int64_t num_in, int64_t
   if (feats_ld < c_in || out_ld < c_out || residual_ld < c_out) return WCN_ERR_INVALID_PARAMETERS;
   if (num_out == 0) return WCN_OK;
   if (!nbr || !out || (num_in > 0 && !feats)) return WCN_ERR_INVALID_PARAMETERS;
+  wcn_f32_launches = 1;
   cudaStream_t st = wcn_stream(stream);
   bool tc_ok = wcn_conv_tcgen05_supported(num_offsets, c_in, c_out, dtype, out_dtype);
   if (algo == WCN_CONV_AUTO && weight && tc_ok) {
@@ -177,9 +181,11 @@ extern "C" int wcn_conv_fwd(int algo, const void* feats, int64_t num_in, int64_t
                     wcn_conv_fp32_supported(c_in, c_out, dtype, out_dtype, feats, feats_ld, weight, out, out_ld, residual, residual_ld);
   if (fp32 && workspace && dev_status && (reinterpret_cast<uintptr_t>(workspace) & 15) == 0 &&
       wcn_conv_split_supported(num_offsets, c_in, c_out) &&
-      workspace_bytes >= wcn_conv_split_workspace(num_in, num_offsets, c_in, c_out))
+      workspace_bytes >= wcn_conv_split_workspace(num_in, num_offsets, c_in, c_out)) {
+    wcn_f32_launches = 2;
     return wcn_conv_split_fwd(feats, num_in, feats_ld, weight, nbr, out_rows, num_out, num_offsets, c_in, c_out, scale, shift,
                               residual, residual_ld, relu, out, out_ld, split_k, workspace, dev_status, st);
+  }
   if (algo == WCN_CONV_AUTO && num_in > 0 && wcn_conv_narrow_out_supported(num_offsets, c_in, c_out, dtype, feats, feats_ld)) {
     // a few output channels (a classification head): one thread per output row
     const int rc = wcn_conv_narrow_out_fwd(feats, num_in, feats_ld, weight, nbr, out_rows, num_out, num_offsets, c_in,

@@ -21,6 +21,8 @@
 #include "tcgen05_common.cuh"
 #include "split_bf16.cuh"
 
+extern thread_local int wcn_f32_launches;   // api.cu
+
 namespace {
 
 constexpr int WS_ROWS = 32;                           // rows of a slot
@@ -469,6 +471,7 @@ extern "C" int wcn_conv_wgrad_f32(const float* feats, int64_t num_in, const floa
     (void)cudaGetLastError();
     return WCN_ERR_EXECUTION;
   }
+  wcn_f32_launches = q.ranges == 1 ? 2 : 3;
   if (q.ranges == 1) return WCN_OK;
   const int64_t n = (int64_t)num_offsets * c_in * c_out / 4;
   wgrad_sum_kernel<<<(unsigned)((n + 127) / 128), 128, 0, st>>>((const float4*)p.dst, q.ranges, n, (float4*)grad_weight);

@@ -27,7 +27,7 @@ import numpy as np
 import torch
 from torch import Tensor
 
-from ..._native import (CONV_AUTO, CONV_SIMT, CONV_TCGEN05, check, device_status, dtype_code, lib, ptr,
+from ..._native import (CONV_AUTO, CONV_SIMT, CONV_TCGEN05, check, count_f32_launches, device_status, dtype_code, lib, ptr,
                         query_bytes, require_cuda, stream_ptr)
 from ...geometry.coords.integer import IntCoords
 from ...geometry.coords.ops.serialization import POINT_ORDERING, encode
@@ -329,6 +329,8 @@ def sparse_conv_fused(in_features: Tensor, weight: Tensor, kernel_map: IntSearch
                              out.stride(0), odc, split_k, ptr(workspace), workspace_bytes, ptr(device_status(dev)),
                              stream_ptr(dev)),
           "wcn_conv_fwd")
+    if workspace is not None:
+        count_f32_launches("wcn_conv_fwd")
     return out
 
 
@@ -382,6 +384,8 @@ class FusedConvLaunch:
                       torch._C._cuda_getCurrentRawStream(self._dev_index))
         if rc != 0:
             check(rc, "wcn_conv_fwd")
+        if workspace is not None:
+            count_f32_launches("wcn_conv_fwd")
         return out
 
 
@@ -870,6 +874,7 @@ def sparse_conv_wgrad(in_features: Tensor, grad_output: Tensor, kernel_map: IntS
             check(lib().wcn_conv_wgrad_f32(ptr(x), x.shape[0], ptr(g), ptr(nbr), ptr(out_rows), ptr(masks), num_out_coords, K, c_in,
                                            c_out, ptr(gw), ptr(ws), nbytes, ptr(device_status(dev)), stream_ptr(dev)),
                   "wcn_conv_wgrad_f32")
+            count_f32_launches("wcn_conv_wgrad_f32")
             return gw
     if x.dtype == torch.float32 or c_in < 16 or c_in % 8 or c_out % 16 or c_out > 256 or K > 32:
         gw = torch.empty((K, c_in, c_out), dtype=torch.float32, device=dev)
@@ -1449,6 +1454,8 @@ def _launch_layer(x: Tensor, weight: Tensor, t: _LayerTables, gradient: bool, ro
                             ptr(workspace), workspace_bytes, device_status(x.device).data_ptr(), stream_ptr(x.device))
     if rc != 0:
         check(rc, "wcn_conv_fwd")
+    if workspace is not None:
+        count_f32_launches("wcn_conv_fwd")
     return out
 
 
