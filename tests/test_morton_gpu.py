@@ -115,3 +115,25 @@ def test_large_pyramids_keep_no_more_than_their_rows(monkeypatch):
         tables.append([maps.kmap(l, w).neighbor_table(maps.n[l if w == 3 else l + 1]).clone() for l in range(4) for w in (3, 2)])
     assert all(torch.equal(a, b) for a, b in zip(*tables))
     check_device_status(torch.device("cuda:0"))
+
+
+def test_a_coordinate_set_keeps_its_own_tables_only():
+    """The maps of a network's levels: the memory behind the tables of one coordinate set (neighbours and row order of its
+    level, children of the next) is not that of another's."""
+    coords, offsets = _scene(60000, [20000, 40000], 150, 5)
+    key = torch.unique(torch.cat([torch.repeat_interleave(torch.arange(2), torch.tensor([20000, 40000]))[:, None], coords.cpu().long()], 1), dim=0)
+    offsets = torch.tensor([0, int((key[:, 0] == 0).sum()), len(key)])
+    v = Voxels(key[:, 1:].int().to(DEV), torch.zeros(len(key), 1, device=DEV), offsets=offsets).sort()
+    maps = LevelMaps(v.batched_coordinates)
+    assert maps.finish() is not None
+    storages = []
+    for l in range(1, 5):
+        held = [maps.nbr[l]] + ([] if maps.order[l] is None else [maps.order[l]]) + ([maps.child[l]] if l < 4 else [])
+        assert len({t.untyped_storage().data_ptr() for t in held}) == 1
+        words = -(-maps.n[l] // 64) * 64, -(-maps.n[l + 1] // 64) * 64 if l < 4 else 0
+        size = held[0].untyped_storage().nbytes()   # (beside the assertion, whose message would print the storage)
+        assert size <= 4 * (28 * words[0] + 8 * words[1])
+        storages.append(held[0].untyped_storage().data_ptr())
+    storages += [maps.child[0].untyped_storage().data_ptr(), maps.nbr[0].untyped_storage().data_ptr()]
+    assert len(set(storages)) == 6
+    check_device_status(DEV)

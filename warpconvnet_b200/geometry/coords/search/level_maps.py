@@ -135,8 +135,9 @@ class LevelMaps:
             self._enqueue(range(1))
 
     def _enqueue(self, which) -> None:
-        """The maps of some levels: of one level as tensors of their own, of several in one piece of memory (an allocation
-        costs the host 2 us, a view as much), of which :meth:`_tensors` makes views."""
+        """The maps of some levels: of one level as tensors of their own, of several in a piece of memory for each
+        coordinate set (an allocation costs the host 2 us, a view as much), of which :meth:`_tensors` makes views: who keeps
+        one set keeps its tables and no others.  The table of the children between two levels is the finer set's."""
         b, dev = self.build, self.build.device
         levels = (Level * len(which))()
         if len(which) == 1:
@@ -150,22 +151,30 @@ class LevelMaps:
             self.at[l] = (nbr.data_ptr(), ptr(order), ptr(child))
             brick_at = [bricks.data_ptr()]
         else:
-            total = bytes_ = 0
-            places, brick_at = [], []
+            words, want, brick_at, bytes_ = {}, dict.fromkeys(range(max(which[0] - 1, 0), which[-1] + 1), 0), [], 0
             for l in which:
                 n = self.n[l]
-                words = -(-n // 64) * 64   # every table starts on a 256-byte boundary
-                places.append((l, n, total, total + 27 * words if n >= self.min_rows else None, total + 28 * words if l else None))
-                total += (28 + (8 if l else 0)) * words
+                words[l] = -(-n // 64) * 64   # every table starts on a 256-byte boundary
+                want[l] += (28 if n >= self.min_rows else 27) * words[l]
+                if l:
+                    want[l - 1] += 8 * words[l]
                 brick_at.append(bytes_)
                 bytes_ += -(-query_bytes("wcn_level_brick_bytes", n) // 256) * 256
-            memory = torch.empty(total, dtype=torch.int32, device=dev)
+            memory = {l: torch.empty(w, dtype=torch.int32, device=dev) for l, w in want.items()}
+            base, used = {l: m.data_ptr() for l, m in memory.items()}, dict.fromkeys(want, 0)
             bricks = self._bricks = torch.empty(bytes_, dtype=torch.uint8, device=dev)
-            base = memory.data_ptr()
             brick_at = [bricks.data_ptr() + v for v in brick_at]
-            for l, _, *tables in places:
-                self.at[l] = tuple(None if v is None else base + 4 * v for v in tables)
-            self._made.append((memory, places))
+
+            def take(l: int, rows: int, of: int) -> int:
+                used[l] += rows * words[of]
+                return used[l] - rows * words[of]
+
+            for l in which:
+                nbr, order = take(l, 27, l), take(l, 1, l) if self.n[l] >= self.min_rows else None
+                child = take(l - 1, 8, l) if l else None
+                self.at[l] = (base[l] + 4 * nbr, None if order is None else base[l] + 4 * order,
+                              None if child is None else base[l - 1] + 4 * child)
+                self._made.append((l, memory[l], nbr, order, memory.get(l - 1), child))
         for slot, l, brick in zip(levels, which, brick_at):
             slot.rows, slot.n, slot.level = self._row_ptr(l), self.n[l], l
             slot.nbr, slot.order, slot.child = self.at[l]
@@ -182,12 +191,12 @@ class LevelMaps:
     def _tensors(self) -> None:
         """The tables that have been enqueued as tensors."""
         self.at = {}   # (addresses would be wrong in a copy)
-        for memory, places in self._made:
-            for l, n, nbr, order, child in places:
-                self.nbr[l] = memory[nbr:nbr + 27 * n].view(27, n)
-                self.order[l] = None if order is None else memory[order:order + n]
-                if child is not None:
-                    self.child[l - 1] = memory[child:child + 8 * n].view(8, n)
+        for l, memory, nbr, order, finer, child in self._made:
+            n = self.n[l]
+            self.nbr[l] = memory[nbr:nbr + 27 * n].view(27, n)
+            self.order[l] = None if order is None else memory[order:order + n]
+            if child is not None:
+                self.child[l - 1] = finer[child:child + 8 * n].view(8, n)
         self._made = []
 
     def _sizes(self) -> bool:
