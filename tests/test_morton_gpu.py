@@ -137,3 +137,28 @@ def test_a_coordinate_set_keeps_its_own_tables_only():
     storages += [maps.child[0].untyped_storage().data_ptr(), maps.nbr[0].untyped_storage().data_ptr()]
     assert len(set(storages)) == 6
     check_device_status(DEV)
+
+
+def test_the_storages_of_large_pyramids_are_those_of_their_rows(monkeypatch):
+    """What a pyramid keeps as the sum of the storages that are held (16 bytes of coordinates and 4 of first children a row):
+    ``torch.cuda.memory_allocated`` also depends on which blocks the allocator has left."""
+    from warpconvnet_b200.geometry.coords.search import level_maps
+    from warpconvnet_b200.nn.functional.sparse_conv import strided_coordinates
+    n = 300000
+    cell = torch.randperm(128 ** 3, generator=torch.Generator().manual_seed(1))[:n].int()
+    xyz = torch.stack([cell // (128 * 128), cell // 128 % 128, cell % 128], dim=1).contiguous().to(DEV)
+    for limit in (n + 1, n):
+        monkeypatch.setattr(level_maps, "TRIMMED_ROWS", limit)
+        ic = Voxels(xyz, torch.zeros(n, 1, device=DEV), offsets=torch.tensor([0, n])).sort().batched_coordinates
+        level, rows, held = ic, 0, []
+        for _ in range(4):
+            level = strided_coordinates(level, (2, 2, 2))
+            rows += len(level)
+            held.append(level._shared["bcoords"])
+        maps, _ = ic._shared["level_maps"]
+        first = maps.build.first
+        held += list(first) if isinstance(first, list) else [first]
+        assert maps.build.out is None
+        kept = sum({t.untyped_storage().data_ptr(): t.untyped_storage().nbytes() for t in held}.values())
+        assert kept >= 80 * n if limit > n else kept <= 20 * rows
+    check_device_status(DEV)
