@@ -384,9 +384,11 @@ int wcn_conv_f32_launches(void);
  * fewer row blocks than multiprocessors.  0 = the library decides, 1 = never, 2.. = that many slices (at most 8); a
  * negative value divides the OUTPUT COLUMNS into -split_k blocks instead (a tuning aid).  `workspace` must hold
  * wcn_conv_workspace_bytes(...) for the same arguments (NULL / 0 when that is 0); fp32 problems under WCN_CONV_AUTO take one
- * of wcn_conv_f32_workspace_bytes(...), with the same meaning of split_k > 0, and run on the FP32 pipes without.  With split_k = 1 a row's sums
- * do not depend on which other rows a launch has (asked with the same num_out, that query gives the same answer for all of them).  Results are the same bits on every run
- * for a given S; different S round differently (fp32 sums are grouped by slice).
+ * of wcn_conv_f32_workspace_bytes(...), with the same meaning of split_k > 0, and run on the FP32 pipes without.
+ * With split_k = 1 a row's sums do not depend on which other rows a launch has (asked with the same num_out, that query gives
+ * the same answer for all of them).  Results are the same bits on every run for a given S and, in fp32, with the workspace
+ * given or not given each time (the two round differently: a caller that goes on without one for want of memory gets the
+ * FP32 pipes' bits); different S round differently (fp32 sums are grouped by slice).
  * Replaces implicit_gemm (warpconvnet/csrc/warpconvnet_pybind.cpp:732-837,
  * warpconvnet/csrc/implicit_gemm.cu:44-267) and cutlass_gemm_AD_gather_scatter with its
  * split_k_slices argument (warpconvnet_pybind.cpp:396-509,

@@ -1,7 +1,7 @@
 // Sparse convolution of fp32 tensors on the 5th-generation tensor cores, without giving up fp32.
 //
 // An fp32 number is the exact sum of three bf16 numbers (24 bits of significand, eight in each): x = h + m + l, w likewise.
-// Of the nine products six are kept, h h, h m, m h, m m, h l, l h (what is left out is below 2^-25 of a product), each exact
+// Of the nine products six are kept, h h, h m, m h, m m, h l, l h (what is left out, m l, l m and l l, is below 2^-24 of a product), each exact
 // in fp32.  What the tensor core does not do as fp32 arithmetic does is add: its accumulator drops the bits below its last
 // place instead of rounding them, and over the some 640 additions of a 64-channel layer that bias alone was nine times the
 // error of the FMA kernel (4.1e-6 against 4.5e-7 of the result's 2-norm, 60 000 room voxels).  So an accumulator is only
@@ -23,8 +23,9 @@
 //    apply scale / shift, residual and ReLU and store the row.  No atomics, the same bits on every run.
 // Few row tiles divide the offsets of a tile among the CTAs of a cluster, which add their sums through distributed shared memory.
 //
-// Bound by the tensor cores: 12 instructions of M = 128, K = 16 (57 clocks each at N = 64, where reading A from shared memory
-// takes as long as the arithmetic) per 128 rows, offset and 32 channels, and by the last tiles of a launch.  Measured (us, the
+// Bound by the rate at which narrow instructions are issued: 12 of M = 128, K = 16 per 128 rows, offset and 32 channels, each of
+// which takes as long as A takes to be read from shared memory (57 clocks at N = 64, 61 at 96, 67 at 128; the tensor pipe itself
+// is busy for 29 to 34 % of the time), and by the last tiles of a launch.  Measured (us, the
 // FMA kernel of conv_fp32.cu / both launches here, L2 flushed): room voxels, 60 000: 64 -> 64 201 / 71, 128 -> 128 652 / 136,
 // 100 000: 64 -> 64 320 / 97, 2 000: 64 -> 64 41 / 21; 20 000 random cells, 32 -> 32 42 / 30.  One issuing thread instead of two:
 // 60 000 rows of 64 channels 75; eight gather warps of 16 rows cost the epilogue its registers; without clusters 2 000 rows of

@@ -335,8 +335,9 @@ conv_tcgen05_kernel(const ConvTcParams p) {
     // are absent for every role.  An index that does not name a feature row is treated as absent and reported
     // (WCN_ERR_BOUNDS).
     // This role paces narrow layers (few bytes per unit), and what it waits for is latency: four warps per sub-tile (or,
-    // for a single sub-tile, four for the even and four for the odd offsets), loads before the wait for a free entry, units
-    // claimed two ahead, one vote per warp.  54 loads and 54 votes in four warps took 14 000 clocks per unit, three times
+    // for a single sub-tile, four for the even and four for the odd offsets), one vote per warp.  A CTA's first
+    // unit and those of fixed strides are loaded before the wait for a free entry; a claimed unit waits for the entry, then for
+    // the claim, then loads (see below what claims further ahead cost).  54 loads and 54 votes in four warps took 14 000 clocks per unit, three times
     // what the copies of a 32-channel layer take.
     const int g = G == 2 ? itid >> 7 : 0;
     const int num_in = (int)p.num_in;

@@ -12,9 +12,9 @@
 // rows in turns into one of four accumulators, and eight warps add every accumulator to the sums in their registers.  The
 // ranges leave partial sums, which the third launch adds in order: the same bits on every run.
 //
-// Bound by the tensor cores (12 instructions of 57 clocks at N = 64 per slot) and the spread of the groups: an inner offset is
-// in every tile, a corner in few; the inner ones start first.  Measured (us, conv_wgrad_pairs.cu / all three
-// launches, L2 flushed): 60 000 room voxels, 64 -> 64 177 / 101, 128 -> 128 673 / 165, 96 -> 48 337 / 126; 2 000: 64 -> 64 52 / 24;
+// Bound by the rate of narrow instructions (12 of 57 clocks at N = 64 per slot; the tensor pipe is busy for 37 % of the time) and
+// the spread of the groups: an inner offset is in every tile, a corner in few; the inner ones start first.  Measured (us,
+// conv_wgrad_pairs.cu / all three launches, L2 flushed): 60 000 room voxels, 64 -> 64 177 / 101, 128 -> 128 673 / 165, 96 -> 48 337 / 126; 2 000: 64 -> 64 52 / 24;
 // outdoors, 60 000: 64 -> 64 128 / 95, 128 -> 128 415 / 150.  Distance from sums in 64 bits: 1.7e-7 against 6.2e-7, 2.0e-7 against
 // 1.1e-6.  Table entries asked for one slot ahead instead of a tile ahead: 126 us instead of 79 for the second launch.
 #include "wcn_common.cuh"

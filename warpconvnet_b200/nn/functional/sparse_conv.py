@@ -241,7 +241,7 @@ def _f32_workspace(x: Tensor, num_out: int, K: int, c_in: int, c_out: int, split
     if nbytes:
         try:
             return torch.empty(nbytes, dtype=torch.uint8, device=x.device), nbytes
-        except torch.cuda.OutOfMemoryError:  # one and a half times the features: the FP32 pipes need none
+        except torch.cuda.OutOfMemoryError:  # one and a half times the features: the FP32 pipes need none (and round differently)
             pass
     return None, 0
 
@@ -866,7 +866,7 @@ def sparse_conv_wgrad(in_features: Tensor, grad_output: Tensor, kernel_map: IntS
         if nbytes:
             try:
                 ws = torch.empty(nbytes, dtype=torch.uint8, device=dev)
-            except torch.cuda.OutOfMemoryError:  # three times the features: the FP32 pipes need less
+            except torch.cuda.OutOfMemoryError:  # three times the features: the FP32 pipes need less (and round differently)
                 pass
         if ws is not None:
             masks = kernel_map.tile_masks(num_out_coords, tiled)
