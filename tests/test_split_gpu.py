@@ -423,3 +423,28 @@ def test_fp32_kernels_are_loud_after_an_expired_wait():
     assert all(bool(torch.isnan(y).all()) for y in loud)
     assert all(torch.equal(a.nan_to_num(1.0), f().nan_to_num(1.0)) for a, f in zip(right, calls))
     check_device_status(DEV)
+
+
+def test_gradients_of_an_input_and_a_bias_in_parts():
+    """Whichever of a layer's three gradients are asked for, together or one by one, they have the same bits, behind an input that is a
+    leaf and one that is not; batches of bias gradients do not run the layer's either way."""
+    coords = room_rows(3000)
+    vox = make_voxels(coords, torch.randn(len(coords), 64, generator=torch.Generator().manual_seed(1))).sort()
+    torch.manual_seed(0)
+    layer = SparseConv3d(64, 48, 3, bias=True).to(DEV)
+    x = vox.feature_tensor.detach().clone().requires_grad_(True)
+    for feats in (x, x * 1.0):
+        y = layer(vox.replace(batched_features=feats)).feature_tensor
+        dy = torch.randn(y.shape, generator=torch.Generator(device=DEV).manual_seed(2), device=DEV)
+        asked = {"x": x, "w": layer.weight, "b": layer.bias}
+        want = dict(zip(asked, torch.autograd.grad(y, list(asked.values()), dy, retain_graph=True)))
+        for names in ("x", "w", "b", "xw", "xb", "wb"):
+            got = torch.autograd.grad(y, [asked[k] for k in names], dy, retain_graph=True)
+            assert all(torch.equal(a, want[k]) for a, k in zip(got, names))
+        batch = torch.stack([dy, -dy])
+        (gb,) = torch.autograd.grad(y, [layer.bias], batch, retain_graph=True, is_grads_batched=True)
+        assert rel_l2(gb[0].cpu().numpy(), want["b"].cpu().numpy()) < 1e-6 and torch.equal(gb[0], -gb[1])
+        y.backward(dy, inputs=[layer.bias])
+        assert torch.equal(layer.bias.grad, want["b"]) and layer.weight.grad is None and x.grad is None
+        layer.bias.grad = None
+    check_device_status(DEV)

@@ -1337,16 +1337,16 @@ class _LayerFunction(torch.autograd.Function):
     deriving the launches from a kernel map's options on every call."""
 
     @staticmethod
-    def forward(ctx, x: Tensor, weight: Tensor, tables: _LayerTables, bias: Optional[Tensor]):
+    def forward(ctx, x: Tensor, weight: Tensor, tables: _LayerTables):
         ctx.tables = tables
         ctx.save_for_backward(x, weight)
-        return _layer_output(x.detach(), weight, tables, bias)
+        return _layer_output(x.detach(), weight, tables)
 
     @staticmethod
     def backward(ctx, g: Tensor):
         x, weight = ctx.saved_tensors
         gx, gw = _layer_gradients(g, x, weight, ctx.tables, *ctx.needs_input_grad[:2])
-        return gx, gw, None, None
+        return gx, gw, None
 
 
 def _column_sums(g: Tensor) -> Tensor:
@@ -1362,25 +1362,43 @@ def _column_sums(g: Tensor) -> Tensor:
     return sums
 
 
+def _asked_for(nodes) -> bool:
+    """Whether the backward pass under way wants a gradient of any of these nodes of the graph (``needs_input_grad`` only says which
+    inputs could have one)."""
+    for node, _ in nodes:
+        try:
+            if node is not None and torch._C._will_engine_execute_node(node):
+                return True
+        except RuntimeError:  # what it says of a leaf that torch.autograd.grad was given (13 us)
+            return True
+    return False
+
+
 class _BiasFunction(torch.autograd.Function):
-    """The bias that a convolution's epilogue has added to ``y`` already, as a node of its own: beside it stood an addition and
-    a reduction through torch, 38 us of the 270 that a layer of 60 000 fp32 rows of 64 channels takes.  (Part of the layer's node,
-    a gradient of the bias alone ran the layer's own gradients too, and a layer of which only the bias trains kept its input.)"""
+    """A layer in training with its bias, which the convolution's epilogue adds: beside :class:`_LayerFunction` that was an
+    addition and a reduction through torch, 38 us of the 270 that a layer of 60 000 fp32 rows of 64 channels takes, and as a
+    node of its own behind the layer's 22 us of the 228 that the host needs for a 16-bit layer, forward and all gradients.  A layer of which
+    only the bias trains keeps nothing, and a gradient of the bias alone does not run the layer's unless the input is a leaf that requires
+    a gradient: whoever asked that of an input wants it, and the answer would be an exception (13 us)."""
 
     @staticmethod
-    def forward(ctx, y: Tensor, bias: Tensor):
-        ctx.bias_dtype = bias.dtype
-        ctx.mark_dirty(y)
-        return y
+    def forward(ctx, x: Tensor, weight: Tensor, bias: Tensor, tables: _LayerTables):
+        ctx.tables, ctx.bias_dtype, ctx.of_leaf = tables, bias.dtype, ctx.needs_input_grad[0] and x.is_leaf
+        if ctx.needs_input_grad[0] or ctx.needs_input_grad[1]:
+            ctx.save_for_backward(x, weight)
+        return _layer_output(x.detach(), weight, tables, bias)
 
     @staticmethod
     def backward(ctx, g: Tensor):
-        gb = None
-        if ctx.needs_input_grad[1]:
-            # (through torch where a graph of the gradient is wanted, and for batches of gradients, which have no memory of their own)
-            native = not torch.is_grad_enabled() and torch._C._has_storage(g)
+        need_x, need_w, need_b = ctx.needs_input_grad[:3]
+        gx = gw = gb = None
+        plain = torch._C._has_storage(g)   # (batches of gradients have no memory of their own)
+        if (need_x or need_w) and (not need_b or (ctx.of_leaf and plain) or _asked_for(ctx.next_functions[:2])):
+            gx, gw = _layer_gradients(g, *ctx.saved_tensors, ctx.tables, need_x, need_w)
+        if need_b:
+            native = plain and not torch.is_grad_enabled()   # (through torch where a graph of the gradient is wanted)
             gb = (_column_sums(g.contiguous()) if native else g.sum(0, dtype=torch.float32)).to(ctx.bias_dtype)
-        return g if ctx.needs_input_grad[0] else None, gb
+        return gx, gw, gb, None
 
 
 class _LayerNormFunction(torch.autograd.Function):
@@ -1400,7 +1418,7 @@ class _LayerNormFunction(torch.autograd.Function):
         x, weight, gamma, beta, residual, z, stats, y = ctx.saved_tensors
         need = ctx.needs_input_grad[:5]
         if torch.is_grad_enabled():  # a graph of the gradient is wanted: the two steps as they are without this function
-            out = batch_norm.formula(_LayerFunction.apply(x, weight, ctx.tables, None), gamma, beta, residual, ctx.eps, ctx.relu)
+            out = batch_norm.formula(_LayerFunction.apply(x, weight, ctx.tables), gamma, beta, residual, ctx.eps, ctx.relu)
             got = iter(torch.autograd.grad(out, [t for t, n in zip((x, weight, gamma, beta, residual), need) if n], dy,
                                            create_graph=True))
             return tuple(next(got) if n else None for n in need) + (None, None, None)
@@ -1506,9 +1524,9 @@ def train_layer(layer, x: Voxels, target: Optional[Voxels]) -> Optional[Voxels]:
             return None
         if (bias is not None and bias.dim() == 1 and bias.shape[0] == weight.shape[2] and bias.device == feats.device
                 and bias.dtype in _NATIVE_DTYPES and batch_norm.reverse_mode_only()):
-            y, bias = _BiasFunction.apply(_LayerFunction.apply(feats, weight, found[0], bias.detach()), bias), None
+            y, bias = _BiasFunction.apply(feats, weight, bias, found[0]), None
         else:
-            y = _LayerFunction.apply(feats, weight, found[0], None)
+            y = _LayerFunction.apply(feats, weight, found[0])
     if bias is not None:
         y = y + bias.to(y.dtype)
     return x._derive(y) if pointwise else _output_of(layer, x, *found, y)
