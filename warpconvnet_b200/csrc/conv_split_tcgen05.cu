@@ -26,8 +26,8 @@
 // Bound by the rate at which narrow instructions are issued: 12 of M = 128, K = 16 per 128 rows, offset and 32 channels, each of
 // which takes as long as A takes to be read from shared memory (57 clocks at N = 64, 61 at 96, 67 at 128; the tensor pipe itself
 // is busy for 29 to 34 % of the time), and by the last tiles of a launch.  Measured (us, the
-// FMA kernel of conv_fp32.cu / both launches here, L2 flushed): room voxels, 60 000: 64 -> 64 201 / 71, 128 -> 128 652 / 136,
-// 100 000: 64 -> 64 320 / 97, 2 000: 64 -> 64 41 / 21; 20 000 random cells, 32 -> 32 42 / 30.  One issuing thread instead of two:
+// FMA kernel of conv_fp32.cu / both launches here, L2 flushed): room voxels, 60 000: 64 -> 64 207 / 69, 128 -> 128 672 / 134,
+// 100 000: 64 -> 64 320 / 105, 2 000: 64 -> 64 40 / 20; 20 000 random cells, 32 -> 32 41 / 28.  One issuing thread instead of two:
 // 60 000 rows of 64 channels 75; eight gather warps of 16 rows cost the epilogue its registers; without clusters 2 000 rows of
 // 64 channels 40, of 128 69 instead of 30.
 #include "wcn_common.cuh"

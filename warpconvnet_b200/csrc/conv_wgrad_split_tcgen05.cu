@@ -14,8 +14,8 @@
 //
 // Bound by the rate of narrow instructions (12 of 57 clocks at N = 64 per slot; the tensor pipe is busy for 37 % of the time) and
 // the spread of the groups: an inner offset is in every tile, a corner in few; the inner ones start first.  Measured (us,
-// conv_wgrad_pairs.cu / all three launches, L2 flushed): 60 000 room voxels, 64 -> 64 177 / 101, 128 -> 128 673 / 165, 96 -> 48 337 / 126; 2 000: 64 -> 64 52 / 24;
-// outdoors, 60 000: 64 -> 64 128 / 95, 128 -> 128 415 / 150.  Distance from sums in 64 bits: 1.7e-7 against 6.2e-7, 2.0e-7 against
+// conv_wgrad_pairs.cu / all three launches, L2 flushed): 60 000 room voxels, 64 -> 64 181 / 107, 128 -> 128 681 / 165, 96 -> 48 339 / 144; 2 000: 64 -> 64 52 / 26;
+// outdoors, 60 000: 64 -> 64 118 / 93, 128 -> 128 525 / 149.  Distance from sums in 64 bits: 1.7e-7 against 6.2e-7, 2.0e-7 against
 // 1.1e-6.  Table entries asked for one slot ahead instead of a tile ahead: 126 us instead of 79 for the second launch.
 #include "wcn_common.cuh"
 #include "tcgen05_common.cuh"
