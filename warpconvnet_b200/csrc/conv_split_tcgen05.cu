@@ -115,7 +115,8 @@ __device__ __forceinline__ float finish(const SplitParams& p, float y, int64_t m
   return p.relu ? fmaxf(y, 0.f) : y;
 }
 
-// Whether any of `cols` sums is infinite or NaN (0 times it is no zero).
+// Whether any of `cols` sums is infinite or NaN (0 times it is no zero).  0.4 us a unit of a narrow layer: 32 -> 48, 95 702 outdoor voxels
+// 57.2 us without, 60.4 with it.  A branch for sixteen columns, or two numbers an instruction, take as long.
 __device__ __forceinline__ bool not_finite(const float (&sum)[64], int cols) {
   float t[4] = {0.f, 0.f, 0.f, 0.f};
 #pragma unroll
